@@ -149,16 +149,21 @@ struct nvmoe_plan {
     uint32_t launches = 0;
     long long wait_cycles = 4000000000ll;  // limit of the bounded in-kernel waits of the tensor path (about 2 s)
     uint32_t debug_flags = 0;
-    // dense linears run as one always-selected resource of a plan of their own shape (nvmoe_dense_linear)
+    // dense linears run as one always-selected resource of a plan of their own shape (nvmoe_dense_linear); the
+    // matrices of one shape share that plan's scratch and have an address table each, so that a block whose gate and
+    // up projections have the same shape resolves each of them once and not on every call
+    struct DenseMatrix {
+        nvmoe_buffer* addresses = nullptr;
+        const void* weights = nullptr;
+        const void* scales = nullptr;
+        uint64_t weights_uid = 0, scales_uid = 0, weights_version = 0, scales_version = 0, last_use = 0;
+    };
     struct DenseLinear {
         uint32_t rows = 0, cols = 0;
         nvmoe_plan* plan = nullptr;
-        nvmoe_buffer* addresses = nullptr;
         nvmoe_buffer* slots = nullptr;
         DeviceArray unit_routes;
-        const void* weights = nullptr;
-        const void* scales = nullptr;
-        uint64_t weights_version = 0, scales_version = 0;
+        std::vector<DenseMatrix> matrices;  // at most kMaxExpertSets, least recently used replaced
     };
     std::vector<DenseLinear> dense;
 };
@@ -547,7 +552,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
     cudaStreamSynchronize(p->device->stream);
     for (auto& dl : p->dense) {
         nvmoe_plan_destroy(dl.plan);
-        nvmoe_buffer_destroy(dl.addresses);
+        for (auto& matrix : dl.matrices) nvmoe_buffer_destroy(matrix.addresses);
         nvmoe_buffer_destroy(dl.slots);
         dl.unit_routes.release();
     }
@@ -1204,8 +1209,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         g.max_tokens = p->g.max_tokens;
         NVMOE_TRY(nvmoe_plan_create(d, &g, &fresh.plan));
         fresh.plan->expert_path = p->expert_path;
-        int rc = nvmoe_buffer_create(d, 64u, &fresh.addresses);
-        if (rc == NVMOE_OK) rc = nvmoe_buffer_create(d, 8u, &fresh.slots);
+        int rc = nvmoe_buffer_create(d, 8u, &fresh.slots);
         const uint32_t slot_words[2] = {0u, 1u};
         if (rc == NVMOE_OK) rc = nvmoe_buffer_write(fresh.slots, 0, slot_words, 8u);
         if (rc == NVMOE_OK && fresh.unit_routes.ensure((size_t)g.max_tokens * 4u) != cudaSuccess)
@@ -1217,7 +1221,6 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         }
         if (rc != NVMOE_OK) {
             nvmoe_plan_destroy(fresh.plan);
-            nvmoe_buffer_destroy(fresh.addresses);
             nvmoe_buffer_destroy(fresh.slots);
             fresh.unit_routes.release();
             return rc;
@@ -1228,21 +1231,41 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     nvmoe_plan* sub = dl->plan;
     sub->expert_path = p->expert_path;
     sub->wait_cycles = p->wait_cycles;
-    if (dl->weights != weights->ptr || dl->scales != scales->ptr || dl->weights_version != weights->version ||
-        dl->scales_version != scales->version) {
-        // the two address records of the one resource: {address, byte count, generation, resident, representation}
-        uint64_t records[8] = {(uint64_t)(uintptr_t)weights->ptr, (uint64_t)rows * (cols / 2u), 1u + weights->version, 1u,
-                               (uint64_t)(uintptr_t)scales->ptr,  (uint64_t)rows * (cols / 32u), 1u + scales->version, 1u};
-        NVMOE_TRY(nvmoe_buffer_write(dl->addresses, 0, records, sizeof records));
-        dl->weights = weights->ptr;
-        dl->scales = scales->ptr;
-        dl->weights_version = weights->version;
-        dl->scales_version = scales->version;
+    nvmoe_plan::DenseMatrix* m = nullptr;
+    for (auto& entry : dl->matrices)
+        if (entry.weights == weights->ptr && entry.scales == scales->ptr) m = &entry;
+    if (!m) {
+        if (dl->matrices.size() < kMaxExpertSets) {
+            nvmoe_plan::DenseMatrix fresh;
+            NVMOE_TRY(nvmoe_buffer_create(d, 64u, &fresh.addresses));
+            dl->matrices.push_back(fresh);
+            m = &dl->matrices.back();
+        } else {
+            m = &dl->matrices[0];
+            for (auto& entry : dl->matrices)
+                if (entry.last_use < m->last_use) m = &entry;
+        }
+    }
+    m->last_use = ++sub->use_clock;
+    if (m->weights != weights->ptr || m->scales != scales->ptr || m->weights_uid != weights->uid || m->scales_uid != scales->uid ||
+        m->weights_version != weights->version || m->scales_version != scales->version) {
+        // the two address records of the one resource: {address, byte count, generation, resident, representation}; the
+        // generation keys the re-tiled scales, so no two contents of one scale address may share it
+        const uint64_t generation = ++sub->use_clock;
+        uint64_t records[8] = {(uint64_t)(uintptr_t)weights->ptr, (uint64_t)rows * (cols / 2u), generation, 1u,
+                               (uint64_t)(uintptr_t)scales->ptr,  (uint64_t)rows * (cols / 32u), generation, 1u};
+        NVMOE_TRY(nvmoe_buffer_write(m->addresses, 0, records, sizeof records));
+        m->weights = weights->ptr;
+        m->scales = scales->ptr;
+        m->weights_uid = weights->uid;
+        m->scales_uid = scales->uid;
+        m->weights_version = weights->version;
+        m->scales_version = scales->version;
     }
     cudaStream_t st = d->stream;
     const bool tensor = use_tensor_path(sub);
     ExpertSet* es = nullptr;
-    NVMOE_TRY(prepare_expert_set(sub, false, dl->addresses, dl->slots, tensor, &es));
+    NVMOE_TRY(prepare_expert_set(sub, false, m->addresses, dl->slots, tensor, &es));
     uint32_t* region = sub->tile_list.as<uint32_t>() + tile_region_words(sub);
     launch_dense_schedule(T, tc_token_tile_for(T, 1u, 1u, false), sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(),
                           sub->position[1].as<uint32_t>(), tensor ? region + 64 : nullptr, tensor ? region : nullptr, st);

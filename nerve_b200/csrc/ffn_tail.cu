@@ -59,6 +59,63 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const uint32_t* __restric
     }
 }
 
+// The same norm with a block per row, for rows of whole 16-byte pieces that fit in shared memory. A warp that walks
+// its row from global memory pays a memory round trip every few steps, twice (777 rows of 7168: 41 us, 22 MB moved);
+// here 128 threads fetch the whole row at once, one warp runs the pinned sums out of shared memory and all of them
+// write the row. Bound by the latency of the three phases, hidden across the blocks of an SM.
+constexpr uint32_t kNormThreads = 128u;
+__global__ void __launch_bounds__(kNormThreads) rms_norm_row_kernel(const uint4* __restrict__ input, const uint4* __restrict__ weight,
+                                                                    uint4* __restrict__ output, uint32_t hidden, float eps,
+                                                                    float weight_offset) {
+    extern __shared__ __align__(16) uint32_t row_words[];
+    __shared__ float inv_shared;
+    grid_dependency_sync();
+    const uint32_t vecs = hidden / 8u, words = hidden / 2u;
+    uint4* row = reinterpret_cast<uint4*>(row_words);
+    const uint4* x = input + (size_t)blockIdx.x * vecs;
+    constexpr uint32_t kDepth = 8u;
+    for (uint32_t i0 = threadIdx.x; i0 < vecs; i0 += kNormThreads * kDepth) {
+        uint4 v[kDepth];
+#pragma unroll
+        for (uint32_t u = 0; u < kDepth; u++)
+            if (i0 + kNormThreads * u < vecs) v[u] = __ldg(x + i0 + kNormThreads * u);
+#pragma unroll
+        for (uint32_t u = 0; u < kDepth; u++)
+            if (i0 + kNormThreads * u < vecs) row[i0 + kNormThreads * u] = v[u];
+    }
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        float lo = 0.0f, hi = 0.0f;
+#pragma unroll 8
+        for (uint32_t w = threadIdx.x; w < words; w += 32u) {
+            const uint32_t v = row_words[w];
+            const float a = nvmoe_bf16_to_f32(v), b = nvmoe_bf16_to_f32(v >> 16);
+            lo = __fmaf_rn(a, a, lo);
+            hi = __fmaf_rn(b, b, hi);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = __fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = __fadd_rn(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        const float total = __fadd_rn(lo, hi);
+        if (threadIdx.x == 0u) inv_shared = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)hidden), eps)));
+    }
+    __syncthreads();
+    const float inv_rms = inv_shared;
+    auto scaled = [&](uint32_t xv, uint32_t wv) {
+        const float a = __fmul_rn(__fmul_rn(nvmoe_bf16_to_f32(xv), inv_rms), __fadd_rn(nvmoe_bf16_to_f32(wv), weight_offset));
+        const float b = __fmul_rn(__fmul_rn(nvmoe_bf16_to_f32(xv >> 16), inv_rms), __fadd_rn(nvmoe_bf16_to_f32(wv >> 16), weight_offset));
+        return pack_bf16x2(a, b);
+    };
+    uint4* y = output + (size_t)blockIdx.x * vecs;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < vecs; i += kNormThreads) {
+        const uint4 xv = row[i], wv = __ldg(weight + i);
+        y[i] = make_uint4(scaled(xv.x, wv.x), scaled(xv.y, wv.y), scaled(xv.z, wv.z), scaled(xv.w, wv.w));
+    }
+}
+
 __device__ __forceinline__ float silu_times(float g, float u, float limit) {
     if (limit > 0.0f) {
         g = fminf(g, limit);
@@ -231,6 +288,12 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 void launch_rms_norm(const uint16_t* input, const uint16_t* weight, uint16_t* output, uint32_t rows, uint32_t hidden, float eps,
                      float weight_offset, cudaStream_t stream) {
+    if (hidden % 8u == 0u && hidden * 2u <= 48u * 1024u - 64u && aligned16(input) && aligned16(weight) && aligned16(output)) {
+        launch_chained(rms_norm_row_kernel, dim3(rows), dim3(kNormThreads), (size_t)hidden * 2u, stream, reinterpret_cast<const uint4*>(input),
+                       reinterpret_cast<const uint4*>(weight), reinterpret_cast<uint4*>(output), hidden, eps, weight_offset);
+        return;
+    }
+    // rows of odd length or alignment, and rows beyond 48 KB
     launch_chained(rms_norm_kernel, dim3((rows + 7u) / 8u), dim3(256), 0, stream, reinterpret_cast<const uint32_t*>(input),
                    reinterpret_cast<const uint32_t*>(weight), reinterpret_cast<uint32_t*>(output), rows, hidden, eps, weight_offset);
 }

@@ -1,0 +1,66 @@
+"""Sizes at which the launch rules change kernels, and the remainders inside them: every case against the CPU checker."""
+import numpy as np
+import pytest
+
+from nerve_b200 import synthetic
+from nerve_b200.backend import CudaComputeDevice, MoePlan, geometry_from_config
+from oracle import moe_oracle as mo
+from tests.helpers import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    dev = CudaComputeDevice(0)
+    yield dev
+    dev.close()
+
+
+def bf16(x):
+    return synthetic.f32_to_bf16(np.asarray(x, dtype=np.float32))
+
+
+def plan_of(device, **kw):
+    fields = {"hidden": 256, "intermediate": 384, "experts": 8, "k": 2, "act_block": 32} | kw
+    tokens = fields.pop("tokens", 64)
+    return MoePlan(device, geometry_from_config(synthetic.MoeConfig("edges", **fields), tokens))
+
+
+# one vector, a partial pass of the block, the longest row a block keeps, the first that it does not
+@pytest.mark.parametrize("rows,hidden", [(3, 8), (2, 8200), (150, 1032), (2, 24544), (2, 24552)])
+def test_rms_norm_rows(device, rows, hidden):
+    rng = np.random.default_rng(hidden)
+    x, w = bf16(rng.standard_normal((rows, hidden))), bf16(1.0 + 0.1 * rng.standard_normal(hidden))
+    plan = plan_of(device)
+    xb, wb, ob = device.resident_buffer_from(x), device.resident_buffer_from(w), device.create_resident_buffer(x.nbytes)
+    plan.rms_norm(rows, hidden, xb, ob, wb, 1e-6, 0.0)
+    np.testing.assert_array_equal(ob.read(np.uint16).reshape(x.shape), mo.rms_norm(x, w, 1e-6, 0.0))
+    plan.destroy()
+
+
+def test_dense_linears_of_one_shape_keep_their_own_tables(device):
+    """Two matrices of one shape in turn, then one of them with new contents, then more matrices than are kept."""
+    rng = np.random.default_rng(5)
+    rows, cols, tokens = 128, 256, 9
+    plan = plan_of(device)
+    x = bf16(rng.standard_normal((tokens, cols)))
+    xb, ob = device.resident_buffer_from(x), device.create_resident_buffer(tokens * rows * 2)
+    mats = []
+    for _ in range(67):
+        w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(121, 128, (rows, cols // 32), dtype=np.uint8)
+        mats.append([w, s, device.resident_buffer_from(w), device.resident_buffer_from(s)])
+
+    def check(i):
+        ob.fill(0)
+        plan.dense_linear(tokens, xb, ob, mats[i][2], mats[i][3], rows, cols)
+        assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, mats[i][0], mats[i][1], 32, tier=1))
+
+    for i in (0, 1, 0, 1):
+        check(i)
+    mats[1][1] = rng.integers(121, 128, (rows, cols // 32), dtype=np.uint8)
+    mats[1][3].write_bytes(mats[1][1])
+    for i in (1, 0, *range(2, 67), 0, 1, 66):
+        check(i)
+    assert plan.status() == 0
+    plan.destroy()
