@@ -126,7 +126,7 @@ struct nvmoe_plan {
     uint32_t frame_words = 0;
     int expert_path = 0;
     // scratch every expert call needs
-    DeviceArray status, grouped[2], offsets[2], block_hist, bucket_base;
+    DeviceArray status, grouped[2], offsets[2], block_hist, bucket_totals;
     std::vector<std::unique_ptr<ExpertSet>> sets[2];  // [gate/up, down], least recently used replaced
     uint64_t use_clock = 0;
     DeviceArray xq, x_scales, x_e8m0, iq, i_scales, i_e8m0, tile_list, ep_source;
@@ -179,7 +179,7 @@ size_t tile_region_words(const nvmoe_plan* p) {
 size_t scratch_blocks(const nvmoe_plan* p) { return ((size_t)p->g.max_tokens * p->K + kSortChunk - 1u) / kSortChunk; }
 
 SortScratch sort_scratch(const nvmoe_plan* p) {
-    return SortScratch{p->block_hist.as<uint32_t>(), p->bucket_base.as<uint32_t>(), (uint32_t)scratch_blocks(p),
+    return SortScratch{p->block_hist.as<uint32_t>(), p->bucket_totals.as<uint32_t>(), (uint32_t)scratch_blocks(p),
                        p->experts + 1u};
 }
 
@@ -487,7 +487,7 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         want(p->offsets[i], sizeof(uint32_t) * (p->experts + 2u));
     }
     want(p->block_hist, sizeof(uint32_t) * scratch_blocks(p) * (p->experts + 1u));
-    want(p->bucket_base, sizeof(uint32_t) * (p->experts + 2u));
+    want(p->bucket_totals, sizeof(uint32_t) * (p->experts + 2u));
     want(p->xq, T * H);
     want(p->x_scales, sizeof(float) * T * (H / g.act_block));
     want(p->x_e8m0, sizeof(uint32_t) * T * ((H + 127u) / 128u));
@@ -559,7 +559,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
     for (auto& stage_sets : p->sets)
         for (auto& es : stage_sets) es->release();
     DeviceArray* all[] = {&p->status, &p->grouped[0], &p->grouped[1], &p->offsets[0],
-                          &p->offsets[1], &p->block_hist, &p->bucket_base, &p->xq, &p->x_scales, &p->x_e8m0, &p->iq,
+                          &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->x_e8m0, &p->iq,
                           &p->i_scales, &p->i_e8m0, &p->tile_list, &p->ep_source, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
                           &p->controls, &p->hidden_dev, &p->output_dev};
@@ -1417,7 +1417,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     ExpertSet* sets[2] = {nullptr, nullptr};
     NVMOE_TRY(prepare_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
     NVMOE_TRY(prepare_expert_set(p, false, a->down_addresses, a->down_slots, tensor, &sets[1]));
-    if (layer_schedule_is_small(T, p->K, p->experts)) {
+    if (layer_schedule_is_fused(T, p->K, p->experts, a->expert_count != 0u)) {
         LayerSchedule ls{};
         ls.routes = (const uint32_t*)routes->ptr;
         ls.intermediates = (uint32_t*)frames.ptr;
@@ -1446,8 +1446,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         ls.num_experts = p->experts;
         ls.n_tile[0] = tc_token_tile_for(T, p->K, p->experts, true);
         ls.n_tile[1] = tc_token_tile_for(T, p->K, p->experts, false);
-        launch_layer_schedule_small(ls, st);
-        p->launches++;
+        p->launches += launch_layer_schedule(ls, sort_scratch(p), st);
         NVMOE_TRY(post_launch(p, "layer schedule"));
     } else {
         write_control_kernel<<<1, 32, 0, st>>>((uint32_t*)gate_control.ptr, T, a->expert_start, a->expert_count);

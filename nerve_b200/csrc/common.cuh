@@ -109,7 +109,7 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
 
 struct SortScratch {  // schedule.cu: scratch of the counting sort, sized for max_tokens
     uint32_t* block_hist;      // [blocks][buckets]
-    uint32_t* bucket_base;     // [buckets + 1]
+    uint32_t* bucket_totals;   // [buckets]
     uint32_t blocks_capacity;
     uint32_t buckets_capacity;
 };
@@ -125,7 +125,7 @@ void launch_route_count(const uint32_t* routes, const uint32_t* slots, uint32_t 
 // (expert, token tile) list of the tensor-core expert kernels from the expert offsets
 void launch_build_tiles(const uint32_t* expert_offsets, uint32_t num_experts, uint32_t n_tile, uint32_t* tiles,
                         uint32_t* count, cudaStream_t stream);
-// One-launch schedule of a whole layer call for small T*K (layer_schedule_is_small): control words,
+// Schedule of a whole layer call in one launch, or three for large T*K (layer_schedule_is_fused): control words,
 // compact list, owned count, and per expert stage [gate/up, down] the grouped routes, expert offsets
 // and (when tiles[stage] is set) the tile list. experts[stage] must already be resolved.
 struct LayerSchedule {
@@ -143,8 +143,8 @@ struct LayerSchedule {
     uint32_t* status;
     uint32_t tokens, expert_start, expert_count, K, I, tiles_per_route[2], num_experts, n_tile[2];
 };
-bool layer_schedule_is_small(uint32_t tokens, uint32_t K, uint32_t num_experts);
-void launch_layer_schedule_small(const LayerSchedule& s, cudaStream_t stream);
+bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned);
+uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream);  // returns its launches
 // validates the address/slot tables of every expert once per call
 // (rows, cols: logical shape of one matrix; experts from native_start on hold native FP8; with
 // whole_blocks_only an FP8-form matrix whose columns are not whole 128-blocks is treated as not resident:

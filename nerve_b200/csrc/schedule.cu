@@ -228,57 +228,72 @@ __device__ void phase_hist(uint32_t count, uint32_t buckets, uint32_t* block_his
     for (uint32_t b = threadIdx.x; b < buckets; b += blockDim.x) block_hist[(size_t)blockIdx.x * buckets + b] = hist[b];
 }
 
-// phase 2 (one block): block_hist[blk][b] <- rank of the first item of bucket b in block blk;
-// bucket_base[b] <- exclusive scan of bucket totals, total at [buckets].
-__global__ void __launch_bounds__(1024) phase_scan_kernel(uint32_t* block_hist, uint32_t* bucket_base,
-                                                         uint32_t blocks, uint32_t buckets) {
-    extern __shared__ uint32_t totals[];
-    // a warp per bucket: thirty-two blocks' counts are scanned at a time with shuffles
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    for (uint32_t b = warp; b < buckets; b += warps) {
-        uint32_t run = 0u;
-        for (uint32_t blk0 = 0; blk0 < blocks; blk0 += 32u) {
-            const uint32_t blk = blk0 + lane;
-            const uint32_t v = blk < blocks ? block_hist[(size_t)blk * buckets + b] : 0u;
-            uint32_t incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += n;
-            }
-            if (blk < blocks) block_hist[(size_t)blk * buckets + b] = run + incl - v;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0u) totals[b] = run;
+// phase 2: block_hist[blk][b] <- rank, within bucket b, of the first item of block blk; totals[b] <- items of bucket b.
+// A block of 32 warps owns 32 buckets: a lane is a bucket (a warp reads 128 neighbouring bytes of a row of counts), a
+// warp is a run of rows, which it sums, and writes back once it knows what the runs before it hold. Bound by the latency
+// of the few dependent loads. One block for all buckets with a warp walking each column read every count from a sector
+// of its own: 576 x 257 counts took 120 us.
+__global__ void __launch_bounds__(1024) phase_scan_kernel(uint32_t* block_hist, uint32_t* totals, uint32_t blocks, uint32_t buckets) {
+    __shared__ uint32_t part[32][32];
+    grid_dependency_sync();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t b = blockIdx.x * 32u + lane;
+    const uint32_t per = (blocks + 31u) / 32u;
+    const uint32_t begin = min_u32(warp * per, blocks), end = min_u32(begin + per, blocks);
+    uint32_t sum = 0u;
+    if (b < buckets) {
+#pragma unroll 8
+        for (uint32_t r = begin; r < end; r++) sum += block_hist[(size_t)r * buckets + b];
     }
+    part[warp][lane] = sum;
     __syncthreads();
-    if (threadIdx.x < 32u) {
-        uint32_t carry = 0u;
-        for (uint32_t b0 = 0; b0 < buckets; b0 += 32u) {
-            uint32_t b = b0 + threadIdx.x;
-            uint32_t v = b < buckets ? totals[b] : 0u;
-            uint32_t incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)threadIdx.x >= o) incl += n;
-            }
-            if (b < buckets) bucket_base[b] = carry + incl - v;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (threadIdx.x == 0u) bucket_base[buckets] = carry;
+    uint32_t running = 0u;
+    for (uint32_t w = 0; w < warp; w++) running += part[w][lane];
+    if (b >= buckets) return;
+    if (warp == 31u) totals[b] = running + sum;
+#pragma unroll 8
+    for (uint32_t r = begin; r < end; r++) {
+        const uint32_t here = block_hist[(size_t)r * buckets + b];
+        block_hist[(size_t)r * buckets + b] = running;
+        running += here;
     }
 }
 
+// out[b] <- sum of value(0 .. b-1) for b <= buckets, by one warp
+template <class ValueFn>
+__device__ __forceinline__ void warp_exclusive_scan(uint32_t buckets, uint32_t* out, ValueFn value) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t carry = 0u;
+    for (uint32_t b0 = 0; b0 < buckets; b0 += 32u) {
+        const uint32_t b = b0 + lane;
+        const uint32_t v = b < buckets ? value(b) : 0u;
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += n;
+        }
+        if (b < buckets) out[b] = carry + incl - v;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0u) out[buckets] = carry;
+}
+
+// phase 3: every block scans the bucket totals itself (`bases`, if given, receives the scan, total at [buckets]) and
+// places its items. Needs buckets + 1 words of dynamic shared memory.
 template <class KeyFn, class EmitFn>
-__device__ void phase_scatter(uint32_t count, uint32_t buckets, const uint32_t* block_hist,
-                              const uint32_t* bucket_base, KeyFn key, EmitFn emit) {
+__device__ void phase_scatter(uint32_t count, uint32_t buckets, const uint32_t* block_hist, const uint32_t* totals,
+                              KeyFn key, EmitFn emit, uint32_t* bases = nullptr) {
     extern __shared__ uint32_t running[];
+    if (threadIdx.x < 32u) warp_exclusive_scan(buckets, running, [&](uint32_t b) { return totals[b]; });
+    __syncthreads();
+    if (bases && blockIdx.x == 0u)
+        for (uint32_t b = threadIdx.x; b <= buckets; b += blockDim.x) bases[b] = running[b];
     uint32_t begin = blockIdx.x * kSortChunk;
     if (begin >= count) return;
     uint32_t end = min_u32(begin + kSortChunk, count);
-    for (uint32_t b = threadIdx.x; b < buckets; b += blockDim.x)
-        running[b] = bucket_base[b] + block_hist[(size_t)blockIdx.x * buckets + b];
+    if (bases) __syncthreads();
+    for (uint32_t b = threadIdx.x; b < buckets; b += blockDim.x) running[b] += block_hist[(size_t)blockIdx.x * buckets + b];
     __syncthreads();
     block_stable_scatter(begin, end, running, key, emit);
 }
@@ -302,7 +317,7 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const uint32_t* ro
                                                              uint32_t params, uint32_t* control,
                                                              uint32_t max_tokens, uint32_t K, uint32_t I,
                                                              uint32_t tiles_per_route, uint32_t num_experts,
-                                                             const uint32_t* block_hist, const uint32_t* bucket_base) {
+                                                             const uint32_t* block_hist, const uint32_t* totals) {
     const uint32_t T = min_u32(control[0], max_tokens);
     const uint32_t count = T * K;
     const uint32_t data_words = K * (I / 2u);
@@ -311,9 +326,9 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const uint32_t* ro
     // every block has read what it needs from control[0..2]; block 0 publishes the command words
     if (partitioned) {
         OwnedKey key{routes, slots, slot_words, params, control[1], control[1] + control[2]};
-        phase_scatter(count, num_experts + 1u, block_hist, bucket_base, key, emit);
+        phase_scatter(count, num_experts + 1u, block_hist, totals, key, emit);
         if (blockIdx.x == 0u && threadIdx.x == 0u) {
-            uint32_t owned = bucket_base[1];
+            uint32_t owned = totals[0];
             control[3] = owned;
             control[4] = owned * tiles_per_route;
             control[5] = 1u;
@@ -321,7 +336,7 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const uint32_t* ro
         }
     } else {
         RouteKey key{routes, num_experts};
-        phase_scatter(count, num_experts + 1u, block_hist, bucket_base, key, emit);
+        phase_scatter(count, num_experts + 1u, block_hist, totals, key, emit);
         if (blockIdx.x == 0u && threadIdx.x == 0u) {
             control[3] = count;
             control[4] = K * tiles_per_route;
@@ -574,6 +589,7 @@ __global__ void __launch_bounds__(1024) layer_schedule_small_kernel(LayerSchedul
 // counts them per warp), and its down stage visits the first owned-by-the-down-table-count of them.
 // One round trip to global memory, five block barriers.
 constexpr uint32_t kRankChunks = 16u;  // routes per thread at most (count <= 16 * blockDim); the kernel is built for 1, 4 and 16
+constexpr uint32_t kWideScheduleRoutes = 1024u;
 constexpr uint32_t kNotListed = 0xffffu;  // bucket field of a route that is in no list
 
 __host__ __device__ inline uint32_t layer_schedule_rank_threads(uint32_t count) { return count <= 256u ? 256u : 1024u; }
@@ -754,6 +770,104 @@ __global__ void __launch_bounds__(1024) layer_schedule_rank_kernel(LayerSchedule
     }
 }
 
+// The same schedule for more routes than one block ranks well: 256 routes a block, in three launches. As above, one
+// stable sort of the routes by expert id serves all lists: the counts per (block, bucket) are taken once (a histogram
+// launch, then phase_scan_kernel), and the last launch turns them into places in the compact list and in both
+// groupings at once. Every block scans the bucket totals itself; block 0 also writes what is per call. Unpartitioned
+// calls only: the owned-route form lists routes in source order, which is another sort.
+// Bound by the latency of three short dependent kernels. The thirteen launches of one sort per list took 413 us for
+// 147456 routes of 257 experts, and the one-block form 44 us for 16384 of 32.
+__global__ void __launch_bounds__(256) layer_schedule_hist_kernel(LayerSchedule s, uint32_t* block_hist) {
+    grid_dependency_sync();
+    phase_hist(s.tokens * s.K, s.num_experts + 1u, block_hist, RouteKey{s.routes, s.num_experts});
+}
+
+__host__ __device__ inline size_t layer_schedule_wide_smem_bytes(uint32_t num_experts) {
+    // the compact list's, two groupings' and two tile lists' bases; ranks of this block; [warp][bucket] counts (u16); kept[2]
+    const size_t buckets = (size_t)num_experts + 1u;
+    return (5u * (buckets + 1u) + buckets) * sizeof(uint32_t) + (8u * buckets + 1u) / 2u * 4u + 2u * buckets;
+}
+
+__global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedule s, const uint32_t* __restrict__ block_hist,
+                                                                    const uint32_t* __restrict__ totals) {
+    extern __shared__ uint32_t smem_words[];
+    const uint32_t count = s.tokens * s.K, E = s.num_experts, B = E + 1u;  // bucket E collects out-of-range expert ids
+    uint32_t* base_all = smem_words;
+    uint32_t* gbase[2] = {base_all + (B + 1u), base_all + 2u * (B + 1u)};
+    uint32_t* tile_base[2] = {base_all + 3u * (B + 1u), base_all + 4u * (B + 1u)};
+    uint32_t* first = base_all + 5u * (B + 1u);
+    uint32_t* table_words = first + B;
+    uint16_t* table = reinterpret_cast<uint16_t*>(table_words);
+    uint8_t* kept = reinterpret_cast<uint8_t*>(table_words + (8u * B + 1u) / 2u);  // [2][B]: the stage keeps routes of this bucket
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    for (uint32_t w = threadIdx.x; w < (8u * B + 1u) / 2u; w += blockDim.x) table_words[w] = 0u;
+    grid_dependency_sync();
+    const uint32_t i = blockIdx.x * kSortChunk + threadIdx.x;
+    uint32_t bucket = kNotListed;
+    if (i < count) bucket = min_u32(__ldg(s.routes + i) & 0xffffu, E);
+    for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) {
+        first[b] = __ldg(block_hist + (size_t)blockIdx.x * B + b);
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++) kept[stage * B + b] = (b < E && s.experts[stage][b].w[0] != nullptr) ? 1u : 0u;
+    }
+    __syncthreads();
+    const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
+    const uint32_t before = __popc(peers & ((1u << lane) - 1u));
+    if (bucket != kNotListed && before == 0u) table[warp * B + bucket] = (uint16_t)__popc(peers);
+    if (warp < 5u) {  // five scans, a warp each
+        const uint32_t stage = warp == 0u ? 0u : (warp - 1u) & 1u;
+        uint32_t* out = warp == 0u ? base_all : warp >= 3u ? tile_base[stage] : gbase[stage];
+        warp_exclusive_scan(B, out, [&](uint32_t b) {
+            const uint32_t v = __ldg(totals + b);
+            if (warp == 0u) return v;
+            if (!kept[stage * B + b]) return 0u;
+            return warp >= 3u ? (v + s.n_tile[stage] - 1u) / s.n_tile[stage] : v;
+        });
+    }
+    __syncthreads();
+    if (i < count) {
+        uint32_t rank = first[bucket] + before;
+        for (uint32_t w = 0; w < warp; w++) rank += table[w * B + bucket];
+        const uint32_t at = base_all[bucket] + rank;
+        const uint32_t data_words = s.K * (s.I / 2u);
+        s.intermediates[(size_t)(at / s.K) * (data_words + s.K) + data_words + at % s.K] = i;
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++) {
+            uint32_t place = kUnboundSlot;
+            if (kept[stage * B + bucket]) {
+                place = gbase[stage][bucket] + rank;
+                s.grouped[stage][place] = i;
+            } else {
+                raise_status(s.status, bucket == E ? NVMOE_STATUS_ROUTE_OUT_OF_RANGE : NVMOE_STATUS_EXPERT_NOT_RESIDENT);
+            }
+            if (s.position[stage]) s.position[stage][i] = place;
+        }
+    }
+    if (blockIdx.x != 0u) return;
+    if (threadIdx.x < 14u) {
+        const uint32_t stage = threadIdx.x / 7u, j = threadIdx.x % 7u;
+        uint32_t value = 1u;  // word 6
+        if (j == 0u || j == 5u) value = s.tokens;
+        if (j == 1u) value = s.expert_start;
+        if (j == 2u) value = 0u;
+        if (j == 3u) value = count;
+        if (j == 4u) value = s.K * s.tiles_per_route[stage];
+        s.control[stage][j] = value;
+    }
+    for (uint32_t x = threadIdx.x; x < 2u * B; x += blockDim.x) {
+        const uint32_t stage = x / B, b = x % B;
+        s.offsets[stage][b] = gbase[stage][b];  // bucket E is never kept: gbase[stage][E] is the total
+        if (s.tiles[stage] && b == E) *s.tile_count[stage] = tile_base[stage][E];
+    }
+    // tile lists: a warp per (stage, expert), its tiles side by side
+    for (uint32_t x = warp; x < 2u * E; x += blockDim.x >> 5) {
+        const uint32_t stage = x / E, b = x % E;
+        if (!s.tiles[stage]) continue;
+        const uint32_t at = tile_base[stage][b], n = tile_base[stage][b + 1u] - at;
+        for (uint32_t j = lane; j < n; j += 32u) s.tiles[stage][at + j] = (b << 16) | j;
+    }
+}
+
 __global__ void __launch_bounds__(256) group_hist_kernel(SlotKey key, const uint32_t* control,
                                                         uint32_t max_tokens, uint32_t* block_hist, uint32_t* position) {
     key.capacity = min_u32(control[0], max_tokens) * key.K;
@@ -767,12 +881,10 @@ __global__ void __launch_bounds__(256) group_hist_kernel(SlotKey key, const uint
 __global__ void __launch_bounds__(256) group_scatter_kernel(SlotKey key, const uint32_t* control,
                                                            uint32_t max_tokens, uint32_t* grouped,
                                                            uint32_t* expert_offsets, const uint32_t* block_hist,
-                                                           const uint32_t* bucket_base, uint32_t* position) {
+                                                           const uint32_t* totals, uint32_t* position) {
     key.capacity = min_u32(control[0], max_tokens) * key.K;
     GroupEmit emit{key, grouped, position};
-    phase_scatter(slot_count(control, max_tokens, key.K), key.num_experts, block_hist, bucket_base, key, emit);
-    if (blockIdx.x == 0u)
-        for (uint32_t b = threadIdx.x; b <= key.num_experts; b += blockDim.x) expert_offsets[b] = bucket_base[b];
+    phase_scatter(slot_count(control, max_tokens, key.K), key.num_experts, block_hist, totals, key, emit, expert_offsets);
 }
 
 // ---- expert-parallel dispatch: group routes by the rank that owns their expert ------------------
@@ -821,11 +933,11 @@ __global__ void __launch_bounds__(256) ep_pack_hist_kernel(DestKey key, uint32_t
 }
 
 __global__ void __launch_bounds__(256) ep_pack_scatter_kernel(DestKey key, PackEmit emit, uint32_t count,
-                                                             const uint32_t* block_hist, const uint32_t* bucket_base,
+                                                             const uint32_t* block_hist, const uint32_t* totals,
                                                              uint32_t* dest_counts) {
-    phase_scatter(count, key.world, block_hist, bucket_base, key, emit);
+    phase_scatter(count, key.world, block_hist, totals, key, emit);
     if (blockIdx.x == 0u)
-        for (uint32_t b = threadIdx.x; b < key.world; b += blockDim.x) dest_counts[b] = bucket_base[b + 1u] - bucket_base[b];
+        for (uint32_t b = threadIdx.x; b < key.world; b += blockDim.x) dest_counts[b] = totals[b];
 }
 
 // send_rows[p] = hidden[token of route send_source[p]]; one warp per row, 16-byte pieces
@@ -912,6 +1024,11 @@ __global__ void sum_counts_kernel(const uint32_t* counts, uint32_t n, uint32_t* 
 
 constexpr uint32_t kSmallSortLimit = 4096u;
 
+void launch_phase_scan(const SortScratch& scratch, uint32_t blocks, uint32_t buckets, cudaStream_t stream) {
+    launch_chained(phase_scan_kernel, dim3((buckets + 31u) / 32u), dim3(1024), 0, stream, scratch.block_hist, scratch.bucket_totals,
+                   blocks, buckets);
+}
+
 }  // namespace
 
 void launch_ep_pack(const uint16_t* hidden, const uint32_t* routes, const uint32_t* owner, uint32_t tokens,
@@ -929,9 +1046,9 @@ void launch_ep_pack(const uint16_t* hidden, const uint32_t* routes, const uint32
     } else {
         const uint32_t blocks = (count + kSortChunk - 1u) / kSortChunk;
         ep_pack_hist_kernel<<<blocks, 256, world * sizeof(uint32_t), stream>>>(key, count, scratch.block_hist, send_index);
-        phase_scan_kernel<<<1, 1024, world * sizeof(uint32_t), stream>>>(scratch.block_hist, scratch.bucket_base, blocks, world);
-        ep_pack_scatter_kernel<<<blocks, 256, world * sizeof(uint32_t), stream>>>(key, emit, count, scratch.block_hist,
-                                                                                 scratch.bucket_base, dest_counts);
+        launch_phase_scan(scratch, blocks, world, stream);
+        ep_pack_scatter_kernel<<<blocks, 256, (world + 1u) * sizeof(uint32_t), stream>>>(key, emit, count, scratch.block_hist,
+                                                                                        scratch.bucket_totals, dest_counts);
     }
     const uint32_t row_vec = hidden_size / 8u;  // uint4 per bf16 row
     if (segment_rows) {
@@ -977,11 +1094,10 @@ void launch_route_compact(const uint32_t* routes, uint32_t* intermediates, const
     compact_hist_kernel<<<blocks, 256, buckets * sizeof(uint32_t), stream>>>(
         routes, slots, slot_words, params_per_resource, control, max_tokens, K, num_experts, scratch.block_hist);
     // the partitioned form uses one bucket; scanning all of them costs nothing and needs no host read
-    phase_scan_kernel<<<1, 1024, buckets * sizeof(uint32_t), stream>>>(scratch.block_hist, scratch.bucket_base,
-                                                                        blocks, buckets);
-    compact_scatter_kernel<<<blocks, 256, buckets * sizeof(uint32_t), stream>>>(
+    launch_phase_scan(scratch, blocks, buckets, stream);
+    compact_scatter_kernel<<<blocks, 256, (buckets + 1u) * sizeof(uint32_t), stream>>>(
         routes, intermediates, slots, slot_words, params_per_resource, control, max_tokens, K,
-        intermediate_size, tiles_per_route, num_experts, scratch.block_hist, scratch.bucket_base);
+        intermediate_size, tiles_per_route, num_experts, scratch.block_hist, scratch.bucket_totals);
 }
 
 static bool rank_schedule_fits(uint64_t count, uint32_t num_experts) {
@@ -993,13 +1109,29 @@ static bool three_sort_schedule_fits(uint64_t count, uint32_t num_experts) {
     return count <= kSmallSortLimit && layer_schedule_smem_bytes((uint32_t)count, num_experts) <= 48u * 1024u;
 }
 
-bool layer_schedule_is_small(uint32_t tokens, uint32_t K, uint32_t num_experts) {
-    const uint64_t count = (uint64_t)tokens * K;
-    return rank_schedule_fits(count, num_experts) || three_sort_schedule_fits(count, num_experts);
+// More routes than one pass of a 1024-thread block go to the three-launch form, unless it is a partitioned call or the
+// tables of that many experts do not fit.
+static bool wide_schedule_fits(uint64_t count, uint32_t num_experts, bool partitioned) {
+    return count > kWideScheduleRoutes && !partitioned && num_experts < kNotListed - 1u &&
+           layer_schedule_wide_smem_bytes(num_experts) <= 48u * 1024u;
 }
 
-void launch_layer_schedule_small(const LayerSchedule& s, cudaStream_t stream) {
+bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned) {
+    const uint64_t count = (uint64_t)tokens * K;
+    return wide_schedule_fits(count, num_experts, partitioned) || rank_schedule_fits(count, num_experts) ||
+           three_sort_schedule_fits(count, num_experts);
+}
+
+uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream) {
     const uint32_t count = s.tokens * s.K;
+    if (wide_schedule_fits(count, s.num_experts, s.expert_count != 0u)) {
+        const uint32_t blocks = (count + kSortChunk - 1u) / kSortChunk, buckets = s.num_experts + 1u;
+        launch_chained(layer_schedule_hist_kernel, dim3(blocks), dim3(256), buckets * sizeof(uint32_t), stream, s, scratch.block_hist);
+        launch_phase_scan(scratch, blocks, buckets, stream);
+        launch_chained(layer_schedule_scatter_kernel, dim3(blocks), dim3(256), layer_schedule_wide_smem_bytes(s.num_experts), stream, s,
+                       scratch.block_hist, scratch.bucket_totals);
+        return 3u;
+    }
     if (rank_schedule_fits(count, s.num_experts)) {
         const uint32_t threads = layer_schedule_rank_threads(count);
         const uint32_t chunks = (count + threads - 1u) / threads;
@@ -1007,10 +1139,11 @@ void launch_layer_schedule_small(const LayerSchedule& s, cudaStream_t stream) {
                                                                                   : layer_schedule_rank_kernel<kRankChunks>;
         launch_chained(kernel, dim3(1), dim3(threads),
                        layer_schedule_rank_smem_bytes(count, s.num_experts), stream, s);
-        return;
+        return 1u;
     }
     launch_chained(layer_schedule_small_kernel, dim3(1), dim3(count <= 256u ? 256u : 1024u),
                    layer_schedule_smem_bytes(count, s.num_experts), stream, s);
+    return 1u;
 }
 
 void launch_build_tiles(const uint32_t* expert_offsets, uint32_t num_experts, uint32_t n_tile, uint32_t* tiles,
@@ -1051,10 +1184,9 @@ void launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, c
     const uint32_t blocks = (count + kSortChunk - 1u) / kSortChunk;
     group_hist_kernel<<<blocks, 256, num_experts * sizeof(uint32_t), stream>>>(key, control, max_tokens,
                                                                                scratch.block_hist, position);
-    phase_scan_kernel<<<1, 1024, num_experts * sizeof(uint32_t), stream>>>(scratch.block_hist, scratch.bucket_base,
-                                                                            blocks, num_experts);
-    group_scatter_kernel<<<blocks, 256, num_experts * sizeof(uint32_t), stream>>>(
-        key, control, max_tokens, grouped_routes, expert_offsets, scratch.block_hist, scratch.bucket_base, position);
+    launch_phase_scan(scratch, blocks, num_experts, stream);
+    group_scatter_kernel<<<blocks, 256, (num_experts + 1u) * sizeof(uint32_t), stream>>>(
+        key, control, max_tokens, grouped_routes, expert_offsets, scratch.block_hist, scratch.bucket_totals, position);
 }
 
 }  // namespace nvmoe

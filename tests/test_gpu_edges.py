@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, MoePlan, geometry_from_config
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, geometry_from_config
 from oracle import moe_oracle as mo
 from tests.helpers import assert_close
 
@@ -63,4 +63,44 @@ def test_dense_linears_of_one_shape_keep_their_own_tables(device):
     for i in (1, 0, *range(2, 67), 0, 1, 66):
         check(i)
     assert plan.status() == 0
+    plan.destroy()
+
+
+# routes on either side of the one-block schedule's limit (1024), whole and ragged blocks of 256 routes, both scale
+# blocks, a K tail (352 = 2.75 x 128), an expert that is not resident
+@pytest.mark.parametrize("name,shape,tokens,absent", [
+    ("gpt-oss-20b", (256, 384, 16), 256, None), ("gpt-oss-20b", (352, 160, 33), 257, 5), ("gpt-oss-20b", (1056, 320, 16), 1100, 0),
+    ("deepseek-v3", (512, 256, 24), 113, None), ("deepseek-v3", (384, 640, 24), 114, 24), ("deepseek-v3", (1024, 256, 256), 512, 7)])
+def test_layer_call_equals_its_nodes(device, name, shape, tokens, absent):
+    """The layer call schedules, quantises and fuses in its own way; the node operators are the plain one."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS[name], *shape)
+    case = synthetic.make_case(cfg, tokens, seed=3)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    if absent is not None:
+        for slots, params in ((bank.gate_up_slots, 4), (bank.down_slots, 2)):
+            words = slots.read(np.uint32).copy()
+            words[absent * params:(absent + 1) * params] = 0xffffffff
+            slots.write_bytes(words)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    rb = device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None
+    sb = device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None
+    K, H = cfg.total_k, cfg.hidden
+    make = device.create_resident_buffer
+    out, want, routes = make(tokens * H * 2), make(tokens * H * 2), make(tokens * K * 4)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw, router_bias=rb, bias=sb, routes_out=routes)
+    missed = plan.status()
+    frames, outputs, gate, down = make(tokens * plan.frame_words * 4), make(tokens * K * H * 2), make(28), make(28)
+    frames.fill(0)
+    outputs.fill(0)
+    control = np.array([tokens, 0, 0, 0, 0, 0, 0], dtype=np.uint32)
+    gate.write_bytes(control)
+    down.write_bytes(control)
+    plan.moe_route_compact(tokens, routes, frames, gate, bank.gate_up_slots)
+    plan.independent_sparse_moe_gate_up(tokens, hidden, routes, frames, bank.gate_up_addresses, bank.gate_up_slots, gate)
+    plan.moe_route_count(tokens, routes, down, bank.down_slots)
+    plan.independent_sparse_moe_down(tokens, frames, routes, outputs, bank.down_addresses, bank.down_slots, down)
+    plan.moe_reduce(tokens, outputs, want)
+    np.testing.assert_array_equal(out.read(np.uint16), want.read(np.uint16))
+    assert missed == plan.status() and (missed == 0) == (absent is None)
     plan.destroy()
