@@ -828,12 +828,16 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
 // Quantises the activations of one expert stage into the form its kernels read: expert-grouped rows
 // with E8M0 scales for the tensor path (after the stage has been scheduled), token- or route-ordered
 // rows with f32 scales for the CUDA-core path. `source` is the bf16 hidden matrix (gate/up) or the
-// intermediates frames (down).
-static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void* source, bool tensor) {
+// intermediates frames (down). `whole_call`: the stage's position table covers every route of the T tokens (it does
+// not when the caller's control words may name fewer tokens), so the hidden rows can be made token by token.
+static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void* source, bool tensor, bool whole_call) {
     const nvmoe_geometry& g = p->g;
     const int set = gate_up ? 0 : 1;
     cudaStream_t st = p->device->stream;
-    if (tensor) {
+    if (tensor && gate_up && whole_call &&
+        launch_quantize_tokens(source, p->position[0].as<uint32_t>(), T, p->K, g.hidden_size, g.act_block, p->grouped_q[0].as<uint8_t>(),
+                               p->grouped_e8m0[0].as<uint32_t>(), st)) {
+    } else if (tensor) {
         launch_quantize_grouped(source, !gate_up, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), p->experts,
                                 T * p->K, p->K, gate_up ? g.hidden_size : g.intermediate_size, g.intermediate_size,
                                 g.act_block, p->grouped_q[set].as<uint8_t>(), p->grouped_e8m0[set].as<uint32_t>(), st);
@@ -878,7 +882,7 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     ExpertSet* es = c.prepared;
     if (!es) NVMOE_TRY(prepare_expert_set(p, gate_up, c.addresses, c.slots, tensor, &es));
     if (!c.scheduled) NVMOE_TRY(schedule_stage(p, gate_up, es, T, c.routes, c.intermediates, c.control, tensor));
-    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor));
+    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor, false));
     ExpertLaunch el{};
     el.work = GroupedWork{p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), es->ptrs.as<ExpertPtrs>(), p->experts};
     if (tensor) {
@@ -1272,8 +1276,10 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     sub->launches++;
     NVMOE_TRY(post_launch(sub, "dense linear schedule"));
     if (tensor) {
-        launch_quantize_grouped(input->ptr, false, sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(), 1u, T, 1u, cols, cols,
-                                sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st);
+        if (!launch_quantize_tokens(input->ptr, sub->position[1].as<uint32_t>(), T, 1u, cols, sub->g.act_block,
+                                    sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st))
+            launch_quantize_grouped(input->ptr, false, sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(), 1u, T, 1u, cols, cols,
+                                    sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st);
     } else {
         launch_quantize((const uint16_t*)input->ptr, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(),
                         sub->i_e8m0.as<uint32_t>(), st);
@@ -1462,7 +1468,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
                                  (const uint32_t*)down_control.ptr, tensor));
     }
     mark(kStageQuantX);
-    NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor));
+    NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true));
     mark(kStageGateUp);
     ExpertCall call;
     call.T = T;
@@ -1477,7 +1483,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     call.fuse_quantise = fused_quantise;
     NVMOE_TRY(run_experts(p, call));
     mark(kStageQuantI);
-    if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor));
+    if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true));
     mark(kStageDown);
     // routes that are skipped (owned by another device, expert not resident) leave their rows untouched:
     // the combine below reads the down stage's position table and counts them as zeros; rows handed to

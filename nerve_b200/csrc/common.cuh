@@ -187,6 +187,11 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
                              const uint32_t* expert_offsets, uint32_t num_experts, uint32_t max_routes, uint32_t K,
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
                              uint32_t* scales_e8m0, cudaStream_t stream);
+// The same gate/up operands from the inverse list: position[token * K + r] = row of that route (0xffffffff: skipped),
+// valid for every route of the call. False when the shape needs the form above (blocks other than 32 or 128 columns,
+// input not 16-byte aligned).
+bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
+                            uint8_t* q, uint32_t* scales_e8m0, cudaStream_t stream);
 // the same for the K rows of every intermediates frame (skips the schedule words)
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K,
                             uint32_t intermediate_size, uint32_t block, uint8_t* q, float* scales_f32,

@@ -159,6 +159,58 @@ __global__ void __launch_bounds__(256) quantize_grouped_rows_kernel(const uint16
     }
 }
 
+// The same operands made token by token, for calls whose place of every route is known (`position`, route -> row): a
+// token's row is read and quantised once and stored to each of its routes' rows, where the form above reads and
+// quantises it again for every route. A warp takes 512 columns of one token, sixteen a lane (two 16-byte loads, one
+// 16-byte store per route); LANES = block / 16 lanes share a scale and eight lanes fill one word of scale bytes.
+// Bound by the stores: 16384 tokens x 7168 columns to 9 rows each are 1.06 GB (684 us in the form above).
+template <uint32_t LANES>
+__global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __restrict__ input, const uint32_t* __restrict__ position,
+                                                             uint32_t tokens, uint32_t K, uint32_t cols, uint32_t chunks,
+                                                             uint8_t* __restrict__ q, uint32_t* __restrict__ scales_e8m0) {
+    grid_dependency_sync();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t item = blockIdx.x * 4u + (threadIdx.x >> 5);
+    const uint32_t token = item / chunks, col = (item % chunks) * 512u + lane * 16u;
+    if (token >= tokens) return;
+    const bool active = col < cols;  // (columns come in whole blocks: the lanes of a block agree)
+    uint32_t mine = lane < K ? __ldg(position + (size_t)token * K + lane) : kUnboundSlot;
+    uint4 v[2] = {};
+    if (active) {
+        const uint4* src = reinterpret_cast<const uint4*>(input + (size_t)token * cols + col);
+        v[0] = __ldg(src);
+        v[1] = __ldg(src + 1);
+    }
+    const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) m = fmaxf(m, fmaxf(fabsf(nvmoe_bf16_to_f32(w[i])), fabsf(nvmoe_bf16_to_f32(w[i] >> 16))));
+#pragma unroll
+    for (uint32_t o = 1u; o < LANES; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float scale = nvmoe_rounded_fp8_scale(m);
+    const float inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
+    uint32_t out[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        out[i] = to_e4m3x4(nvmoe_bf16_to_f32(w[2 * i]) * inv, nvmoe_bf16_to_f32(w[2 * i] >> 16) * inv,
+                           nvmoe_bf16_to_f32(w[2 * i + 1]) * inv, nvmoe_bf16_to_f32(w[2 * i + 1] >> 16) * inv);
+    // two lanes hold 32 columns: byte (lane % 8) / 2 of the word of their 128
+    uint32_t word = active ? (nvmoe_f32_bits(scale) >> 23) << (8u * ((lane & 7u) >> 1)) : 0u;
+    word |= __shfl_xor_sync(0xffffffffu, word, 2);
+    word |= __shfl_xor_sync(0xffffffffu, word, 4);
+    const uint32_t words128 = (cols + 127u) / 128u;
+    for (uint32_t r0 = 0; r0 < K; r0 += 32u) {
+        if (r0 != 0u) mine = r0 + lane < K ? __ldg(position + (size_t)token * K + r0 + lane) : kUnboundSlot;
+        const uint32_t here = min(32u, K - r0);
+        for (uint32_t r = 0; r < here; r++) {
+            const uint32_t row = __shfl_sync(0xffffffffu, mine, r);
+            if (row == kUnboundSlot || !active) continue;  // a route that the stage skips
+            *reinterpret_cast<uint4*>(q + (size_t)row * cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
+            if ((lane & 7u) == 0u) scales_e8m0[(size_t)row * words128 + col / 128u] = word;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256) scales_to_e8m0_kernel(const float* scales, uint32_t rows, uint32_t cols,
                                                             uint32_t block, uint32_t* scales_e8m0, uint32_t* status) {
     const uint32_t blocks_per_row = cols / block;
@@ -217,6 +269,19 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
     launch_chained(quantize_grouped_kernel, dim3(grid_for((uint64_t)max_routes * (cols / block))), dim3(256), 0, stream, input,
                    frames, grouped_routes, expert_offsets, num_experts, max_routes, K, cols, intermediate_size, block, q,
                    scales_e8m0);
+}
+
+bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
+                            uint8_t* q, uint32_t* scales_e8m0, cudaStream_t stream) {
+    if ((block != 32u && block != 128u) || cols % block != 0u || (reinterpret_cast<uintptr_t>(input) & 15u) != 0u) return false;
+    const uint32_t chunks = (cols + 511u) / 512u;
+    const uint64_t warps = (uint64_t)tokens * chunks;
+    if (warps == 0u) return true;
+    if (warps > 0x7fffffffull) return false;
+    const auto kernel = block == 32u ? quantize_tokens_kernel<2u> : quantize_tokens_kernel<8u>;
+    launch_chained(kernel, dim3((uint32_t)((warps + 3u) / 4u)), dim3(128), 0, stream, static_cast<const uint16_t*>(input), position, tokens,
+                   K, cols, chunks, q, scales_e8m0);
+    return true;
 }
 
 void launch_scales_to_e8m0(const float* scales, uint32_t rows, uint32_t cols, uint32_t block,
