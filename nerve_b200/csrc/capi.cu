@@ -830,13 +830,16 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
 // rows with f32 scales for the CUDA-core path. `source` is the bf16 hidden matrix (gate/up) or the
 // intermediates frames (down). `whole_call`: the stage's position table covers every route of the T tokens (it does
 // not when the caller's control words may name fewer tokens), so the hidden rows can be made token by token.
-static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void* source, bool tensor, bool whole_call) {
+// `fused`: gate/up will write the down stage's operands itself.
+static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void* source, bool tensor, bool whole_call, bool fused) {
     const nvmoe_geometry& g = p->g;
     const int set = gate_up ? 0 : 1;
     cudaStream_t st = p->device->stream;
+    const DownRows down{fused ? p->position[1].as<uint32_t>() : nullptr, p->grouped_q[1].as<uint8_t>(), p->grouped_e8m0[1].as<uint32_t>(),
+                        g.intermediate_size};
     if (tensor && gate_up && whole_call &&
         launch_quantize_tokens(source, p->position[0].as<uint32_t>(), T, p->K, g.hidden_size, g.act_block, p->grouped_q[0].as<uint8_t>(),
-                               p->grouped_e8m0[0].as<uint32_t>(), st)) {
+                               p->grouped_e8m0[0].as<uint32_t>(), down, st)) {
     } else if (tensor) {
         launch_quantize_grouped(source, !gate_up, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), p->experts,
                                 T * p->K, p->K, gate_up ? g.hidden_size : g.intermediate_size, g.intermediate_size,
@@ -882,7 +885,7 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     ExpertSet* es = c.prepared;
     if (!es) NVMOE_TRY(prepare_expert_set(p, gate_up, c.addresses, c.slots, tensor, &es));
     if (!c.scheduled) NVMOE_TRY(schedule_stage(p, gate_up, es, T, c.routes, c.intermediates, c.control, tensor));
-    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor, false));
+    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor, false, false));
     ExpertLaunch el{};
     el.work = GroupedWork{p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), es->ptrs.as<ExpertPtrs>(), p->experts};
     if (tensor) {
@@ -917,6 +920,7 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
             el.q_out = p->grouped_q[1].as<uint8_t>();
             el.q_e8m0 = p->grouped_e8m0[1].as<uint32_t>();
             el.down_position = p->position[1].as<uint32_t>();
+            el.intermediates = nullptr;  // the down stage reads the codes only
         }
     }
     if (p->profile_stages) cudaEventRecord(p->kernel_ev[set][0], st);
@@ -1277,7 +1281,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     NVMOE_TRY(post_launch(sub, "dense linear schedule"));
     if (tensor) {
         if (!launch_quantize_tokens(input->ptr, sub->position[1].as<uint32_t>(), T, 1u, cols, sub->g.act_block,
-                                    sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st))
+                                    sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), DownRows{}, st))
             launch_quantize_grouped(input->ptr, false, sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(), 1u, T, 1u, cols, cols,
                                     sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st);
     } else {
@@ -1418,8 +1422,10 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     if (!a->routes_in) NVMOE_TRY(nvmoe_route(p, T, logits, routes, a->bias, a->telemetry));
     mark(kStageSchedule);
     const bool tensor = use_tensor_path(p);
-    // with 32-wide scale blocks the tensor-path gate/up epilogue quantises its own output for the down stage
-    const bool fused_quantise = tensor && g.act_block == 32u;
+    // with scale blocks of 32 or 128 (what a warp, or the four warps of an epilogue group, hold of a token) the tensor-path
+    // gate/up epilogue quantises its own output for the down stage
+    const bool fused_quantise = tensor && (g.act_block == 32u || g.act_block == 128u) &&
+                                (reinterpret_cast<uintptr_t>(a->hidden->ptr) & 15u) == 0u;  // (as launch_quantize_tokens wants it)
     ExpertSet* sets[2] = {nullptr, nullptr};
     NVMOE_TRY(prepare_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
     NVMOE_TRY(prepare_expert_set(p, false, a->down_addresses, a->down_slots, tensor, &sets[1]));
@@ -1468,7 +1474,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
                                  (const uint32_t*)down_control.ptr, tensor));
     }
     mark(kStageQuantX);
-    NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true));
+    NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true, fused_quantise));
     mark(kStageGateUp);
     ExpertCall call;
     call.T = T;
@@ -1483,7 +1489,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     call.fuse_quantise = fused_quantise;
     NVMOE_TRY(run_experts(p, call));
     mark(kStageQuantI);
-    if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true));
+    if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true, false));
     mark(kStageDown);
     // routes that are skipped (owned by another device, expert not resident) leave their rows untouched:
     // the combine below reads the down stage's position table and counts them as zeros; rows handed to

@@ -188,10 +188,17 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
                              uint32_t* scales_e8m0, cudaStream_t stream);
 // The same gate/up operands from the inverse list: position[token * K + r] = row of that route (0xffffffff: skipped),
-// valid for every route of the call. False when the shape needs the form above (blocks other than 32 or 128 columns,
-// input not 16-byte aligned).
+// valid for every route of the call. `down` (position null: nothing) names the down stage's operand rows, of which those
+// of routes that only the down stage keeps are set to zero. False when the shape needs the form above (blocks other than
+// 32 or 128 columns, input not 16-byte aligned).
+struct DownRows {
+    const uint32_t* position;
+    uint8_t* q;
+    uint32_t* scales_e8m0;
+    uint32_t cols;
+};
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
-                            uint8_t* q, uint32_t* scales_e8m0, cudaStream_t stream);
+                            uint8_t* q, uint32_t* scales_e8m0, const DownRows& down, cudaStream_t stream);
 // the same for the K rows of every intermediates frame (skips the schedule words)
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K,
                             uint32_t intermediate_size, uint32_t block, uint8_t* q, float* scales_f32,
@@ -206,7 +213,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     const float* act_scales;     // [rows][K_dim/act_block] f32
     const uint32_t* act_e8m0;    // [rows][ceil(K_dim/128)] packed E8M0 (tensor path)
     const uint32_t* routes;      // route words (down: weights)
-    uint32_t* intermediates;     // gate/up output frames
+    uint32_t* intermediates;     // gate/up output frames (tensor path with q_out: may be null)
     uint16_t* outputs;           // down output [T][K][H]
     float* partial_outputs;      // down, tensor-parallel form: raw f32 sums [T][K][H] instead of `outputs` (no route weight, no rounding)
     uint32_t* status;
@@ -217,7 +224,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     // tensor path, gate/up only: where the down stage's grouping puts each route (its operand row)
     const uint32_t* down_position;
     // tensor path, gate/up only, optional: the down stage's activation quantisation done in the epilogue
-    // (E4M3 bytes [down_position][I], E8M0 bytes [down_position][ceil(I/128)] words); needs act_block 32
+    // (E4M3 bytes [down_position][I], E8M0 bytes [down_position][ceil(I/128)] words); needs act_block 32 or 128
     uint8_t* q_out;
     uint32_t* q_e8m0;
     uint64_t* cta_trace;         // tensor path diagnostics: [2][grid][4] words per CTA, or null

@@ -103,7 +103,7 @@ struct Config {
     // that do not exist.
     static constexpr uint32_t kSfBytes = kMatrices * kScaleBlockBytes + (N_TILE <= 16u ? kScaleBlockBytes / 2u : kScaleBlockBytes);
     static constexpr uint32_t kStageBytes = kSub * (kABytes + kBTileBytes + kSfBytes);
-    static constexpr uint32_t kBarrierBytes = 256u;
+    static constexpr uint32_t kBarrierBytes = 256u + (GATE_UP ? 64u * kEpilogueGroups : 0u);  // barriers, then the block maxima
     // The arrays start at the first 1024-byte boundary of the dynamic shared memory. Room for that round-up is set
     // aside unless leaving it out buys another slot; the kernel then insists on a base that is aligned already
     // (it is when the kernel has no static shared memory) and does nothing, with NVMOE_STATUS_INTERNAL, otherwise.
@@ -157,6 +157,10 @@ struct Barriers {
     uint32_t acc_ready[2];        // the verdict of the epilogue warp that watches acc_full, for the others
 };
 
+// Block maxima of the fused quantisation with 128-row scale blocks: [set of four tokens, alternating][lane quadrant]
+// [token] of each epilogue group, as the bf16 bits of the magnitude
+using BlockMaxima = uint16_t[2][4][4];
+
 // TRACE compiles the diagnostics in (cycle counters of CTA 0, per-CTA global-timer stamps): the
 // instantiation that runs unless a plan's trace was armed has none of them in its loops.
 template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR, bool TRACE>
@@ -169,7 +173,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     // operand tiles need 1024-byte alignment for the 128-byte swizzle
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
     Barriers* bars = reinterpret_cast<Barriers*>(smem + C::kStages * C::kStageBytes);
-    static_assert(sizeof(Barriers) <= C::kBarrierBytes, "barrier block");
+    static_assert(sizeof(Barriers) <= 256u && sizeof(BlockMaxima) == 64u, "barrier block");
+    BlockMaxima* maxima = reinterpret_cast<BlockMaxima*>(reinterpret_cast<unsigned char*>(bars) + 256u);
     volatile uint32_t* abort_flag = &bars->abort;
     if (C::kNeedsAlignedBase && smem != smem_raw) {  // (uniform) no room was set aside for the round-up
         grid_dependency_sync();
@@ -597,7 +602,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         const uint32_t quad = warp & 3u;  // the quadrant of tensor-memory lanes this warp may read
         const uint32_t epilogue_group = warp < 4u ? 0u : (warp - C::kFirstExtraEpilogueWarp) / 4u + 1u;
         const uint32_t frame_words = K * (I / 2u) + K;
-        uint32_t acc_it = 0u;
+        uint32_t acc_it = 0u, set_it = 0u;
+        const bool whole_block = GATE_UP && p.g.act_block == 128u;  // the scale block of the fused quantisation is the tile's 128 rows
         long long trace_epi_wait = 0;
         const long long trace_begin = TRACE ? clock64() : 0;
         for (uint32_t tile = blockIdx.x; tile < tile_count; tile += gridDim.x, acc_it++) {
@@ -654,7 +660,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                     // the row of the down stage's operand matrix that this route's activations go to
                     my_route = (GATE_UP && p.q_out != nullptr) ? __ldg(p.down_position + ri) : kUnboundSlot;
                     if (GATE_UP) {
-                        my_row = reinterpret_cast<uint64_t>(reinterpret_cast<uint16_t*>(p.intermediates + (size_t)(ri / K) * frame_words) +
+                        if (p.intermediates != nullptr) my_row = reinterpret_cast<uint64_t>(reinterpret_cast<uint16_t*>(p.intermediates + (size_t)(ri / K) * frame_words) +
                                                             (size_t)(ri % K) * I);
                     } else if (p.partial_outputs != nullptr) {
                         my_row = reinterpret_cast<uint64_t>(p.partial_outputs + (size_t)ri * H);
@@ -664,7 +670,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                     }
                 }
                 tmem_ld_wait();
-                const bool quantise = GATE_UP && p.q_out != nullptr;  // host: only with 32-row scale blocks
+                const bool quantise = GATE_UP && p.q_out != nullptr;  // host: only with scale blocks of 32 or 128 rows
+                const bool store_rows = !GATE_UP || p.intermediates != nullptr;  // (uniform) a caller's rows; a layer only needs their codes
                 // Four tokens at a time go through each step together, with no branch between them, so that
                 // their instruction latencies overlap (the activation math is one long dependent chain per
                 // value); columns past `valid` hold zeros and are only not stored.
@@ -695,6 +702,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         }
                         continue;
                     }
+                    if (store_rows) {
 #pragma unroll
                     for (uint32_t t = 0; t < 4u; t++) {
                         uint16_t* out = reinterpret_cast<uint16_t*>(__shfl_sync(0xffffffffu, my_row, g0 + t));
@@ -706,9 +714,12 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                             if (c0 + g0 + t < valid && row + kBlockM < out_rows) out[row + kBlockM] = (uint16_t)second;
                         }
                     }
+                    }
                     if (quantise) {
                         // the activation quantisation of the down stage, on the values just rounded to bf16: one
-                        // power-of-two scale per 32 rows, which is exactly this warp's share of the tile
+                        // power-of-two scale per 32 rows, which is exactly this warp's share of the tile, or per 128
+                        // rows, the share of the four warps of the group, which then hand their maxima round (a pass
+                        // over the frames instead took 744 us for 147456 rows of 2048)
                         float m[4];
 #pragma unroll
                         for (uint32_t t = 0; t < 4u; t++) m[t] = row_ok ? fabsf(nvmoe_bf16_to_f32(bits[t])) : 0.0f;
@@ -716,6 +727,18 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
                             for (uint32_t t = 0; t < 4u; t++) m[t] = fmaxf(m[t], __shfl_xor_sync(0xffffffffu, m[t], o));
+                        }
+                        if (whole_block) {
+                            // (the four warps of a group run through the same tokens; a set's maxima are overwritten two
+                            // sets later, when every warp has passed the barrier of the set between)
+                            uint16_t(&quad_max)[4][4] = maxima[epilogue_group][set_it++ & 1u];
+                            if (lane < 4u)
+                                quad_max[quad][lane] = (uint16_t)(__float_as_uint(lane == 0u ? m[0] : lane == 1u ? m[1] : lane == 2u ? m[2] : m[3]) >> 16);
+                            named_barrier(2u + epilogue_group, 128u);
+#pragma unroll
+                            for (uint32_t t = 0; t < 4u; t++)
+                                m[t] = fmaxf(fmaxf(fmaxf(0.0f, nvmoe_bf16_to_f32(quad_max[0][t])), nvmoe_bf16_to_f32(quad_max[1][t])),
+                                             fmaxf(nvmoe_bf16_to_f32(quad_max[2][t]), nvmoe_bf16_to_f32(quad_max[3][t])));
                         }
                         const uint32_t first_row = m_tile * C::kTileRows + quad * 32u;
                         const bool writes_scale = lane == 0u && first_row < out_rows;

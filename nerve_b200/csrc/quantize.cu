@@ -164,10 +164,13 @@ __global__ void __launch_bounds__(256) quantize_grouped_rows_kernel(const uint16
 // quantises it again for every route. A warp takes 512 columns of one token, sixteen a lane (two 16-byte loads, one
 // 16-byte store per route); LANES = block / 16 lanes share a scale and eight lanes fill one word of scale bytes.
 // Bound by the stores: 16384 tokens x 7168 columns to 9 rows each are 1.06 GB (684 us in the form above).
+// When gate/up writes the down stage's operands itself (`down`), a route that only the down stage keeps would find
+// whatever lies in its row: it gets zeros here, as if the gate/up frame had never been written.
 template <uint32_t LANES>
 __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __restrict__ input, const uint32_t* __restrict__ position,
                                                              uint32_t tokens, uint32_t K, uint32_t cols, uint32_t chunks,
-                                                             uint8_t* __restrict__ q, uint32_t* __restrict__ scales_e8m0) {
+                                                             uint8_t* __restrict__ q, uint32_t* __restrict__ scales_e8m0,
+                                                             DownRows down) {
     grid_dependency_sync();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t item = blockIdx.x * 4u + (threadIdx.x >> 5);
@@ -204,7 +207,17 @@ __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __
         const uint32_t here = min(32u, K - r0);
         for (uint32_t r = 0; r < here; r++) {
             const uint32_t row = __shfl_sync(0xffffffffu, mine, r);
-            if (row == kUnboundSlot || !active) continue;  // a route that the stage skips
+            if (row == kUnboundSlot) {  // a route that the stage skips
+                const uint32_t down_row = down.position && item % chunks == 0u ? __ldg(down.position + (size_t)token * K + r0 + r) : kUnboundSlot;
+                if (down_row != kUnboundSlot) {
+                    for (uint32_t c = lane * 16u; c < down.cols; c += 512u)
+                        *reinterpret_cast<uint4*>(down.q + (size_t)down_row * down.cols + c) = make_uint4(0u, 0u, 0u, 0u);
+                    const uint32_t down_words = (down.cols + 127u) / 128u;
+                    for (uint32_t c = lane; c < down_words; c += 32u) down.scales_e8m0[(size_t)down_row * down_words + c] = 0x7f7f7f7fu;
+                }
+                continue;
+            }
+            if (!active) continue;
             *reinterpret_cast<uint4*>(q + (size_t)row * cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
             if ((lane & 7u) == 0u) scales_e8m0[(size_t)row * words128 + col / 128u] = word;
         }
@@ -272,7 +285,7 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
 }
 
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
-                            uint8_t* q, uint32_t* scales_e8m0, cudaStream_t stream) {
+                            uint8_t* q, uint32_t* scales_e8m0, const DownRows& down, cudaStream_t stream) {
     if ((block != 32u && block != 128u) || cols % block != 0u || (reinterpret_cast<uintptr_t>(input) & 15u) != 0u) return false;
     const uint32_t chunks = (cols + 511u) / 512u;
     const uint64_t warps = (uint64_t)tokens * chunks;
@@ -280,7 +293,7 @@ bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_
     if (warps > 0x7fffffffull) return false;
     const auto kernel = block == 32u ? quantize_tokens_kernel<2u> : quantize_tokens_kernel<8u>;
     launch_chained(kernel, dim3((uint32_t)((warps + 3u) / 4u)), dim3(128), 0, stream, static_cast<const uint16_t*>(input), position, tokens,
-                   K, cols, chunks, q, scales_e8m0);
+                   K, cols, chunks, q, scales_e8m0, down);
     return true;
 }
 
