@@ -48,6 +48,7 @@ constexpr uint32_t kTmaBoxBytes = kBlockM * 64u;   // global bytes of one 128 x 
 constexpr uint32_t kATileBytes = kBlockM * 128u;   // one byte slot per element
 constexpr uint32_t kScaleBlockBytes = 512u;        // 128 rows x 4 scale bytes
 constexpr uint32_t kMaxStages = 8u;
+constexpr uint32_t kRowPairRounds = 6u;  // tiles an SM goes through at least before narrow down tiles pair their rows
 constexpr uint32_t kWatchWarp = 2u;     // the epilogue warp that polls for a finished accumulator (not on the MMA or TMA warp's scheduler)
 
 struct TileList {
@@ -58,8 +59,8 @@ struct TileList {
 // ROW_PAIR (down only): a tile covers two 128-row tiles of the one weight matrix, handled as the two
 // "matrices" of a stage exactly as gate and up are: two accumulators alternate (one MMA cannot follow
 // another into the same accumulator at full rate) and the token tile is fetched once for 256 rows. Used
-// for the wide token tiles of large batches; small batches keep 128-row tiles, which spread better
-// over the SMs.
+// for the wide token tiles of large batches and for narrow ones when there are many (takes_row_pairs);
+// small batches keep 128-row tiles, which spread better over the SMs.
 template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR>
 struct Config {
     static_assert(!(GATE_UP && ROW_PAIR), "gate/up already holds two matrices a stage");
@@ -842,56 +843,80 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 
 int g_sm_count[16] = {0};
 
-// wide token tiles of the down stage take two row tiles at a time
-template <bool GATE_UP, uint32_t N_TILE>
-constexpr bool row_pair() { return !GATE_UP && N_TILE >= 64u; }
-
-template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA>
-void launch_n(const ExpertLaunch& p, cudaStream_t stream) {
-    using C = Config<GATE_UP, N_TILE, USE_TMA, row_pair<GATE_UP, N_TILE>()>;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (g_sm_count[dev & 15] == 0) cudaDeviceGetAttribute(&g_sm_count[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR>
+void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
+    using C = Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>;
     // the traced instantiation only when a plan's trace was armed (and only for the TMA form)
     if (USE_TMA && p.cta_trace != nullptr) {
-        launch_chained(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, row_pair<GATE_UP, N_TILE>(), USE_TMA>, dim3(g_sm_count[dev & 15]),
-                       dim3(C::kThreads), C::kSmemBytes, stream, p, TileList{p.tile_list, p.tile_count});
+        launch_chained(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, ROW_PAIR, USE_TMA>, dim3(sms), dim3(C::kThreads), C::kSmemBytes, stream, p,
+                       TileList{p.tile_list, p.tile_count});
     } else {
-        launch_chained(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, row_pair<GATE_UP, N_TILE>(), false>, dim3(g_sm_count[dev & 15]),
-                       dim3(C::kThreads), C::kSmemBytes, stream, p, TileList{p.tile_list, p.tile_count});
+        launch_chained(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, ROW_PAIR, false>, dim3(sms), dim3(C::kThreads), C::kSmemBytes, stream, p,
+                       TileList{p.tile_list, p.tile_count});
     }
+}
+
+// Whether a down launch takes two row tiles at a time: always with wide token tiles, and with narrow ones (TMA form)
+// when that leaves every SM several tiles to go through. A stage of a row pair is one K block of two weight boxes, one
+// token box and two scale copies, where a single row tile needs six copies for the same bytes (0.42 against 0.49 us per
+// stage); single row tiles spread over the SMs in finer steps, which is worth more when there are only a few rounds.
+bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) {
+    if (n_tile >= 64u) return true;
+    if (!tma) return false;
+    const uint64_t routes = (uint64_t)p.tokens * (p.g.routed_k + p.g.always_count);
+    const uint64_t lists = routes < p.work.num_experts ? routes : p.work.num_experts;
+    return lists * ((p.g.hidden_size + 2u * kBlockM - 1u) / (2u * kBlockM)) >= (uint64_t)kRowPairRounds * (uint64_t)sms;
 }
 
 template <bool GATE_UP>
 void launch(const ExpertLaunch& p, cudaStream_t stream) {
     constexpr uint32_t kWide = 96u;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (g_sm_count[dev & 15] == 0) cudaDeviceGetAttribute(&g_sm_count[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+    const int sms = g_sm_count[dev & 15];
     const uint32_t n = tc_token_tile_for(p.tokens, p.g.routed_k + p.g.always_count, p.work.num_experts, GATE_UP);
-    if (p.tmaps != nullptr) {
+    const bool tma = p.tmaps != nullptr;
+    const bool pairs = !GATE_UP && takes_row_pairs(p, n, tma, sms);
+    if (tma && pairs) {
         switch (n) {
-            case 16u: launch_n<GATE_UP, 16u, true>(p, stream); break;
-            case 32u: launch_n<GATE_UP, 32u, true>(p, stream); break;
-            case 64u: launch_n<GATE_UP, 64u, true>(p, stream); break;
-            default: launch_n<GATE_UP, kWide, true>(p, stream); break;
+            case 16u: launch_n<GATE_UP, 16u, true, !GATE_UP>(p, sms, stream); break;
+            case 32u: launch_n<GATE_UP, 32u, true, !GATE_UP>(p, sms, stream); break;
+            case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, kWide, true, !GATE_UP>(p, sms, stream); break;
+        }
+    } else if (tma) {
+        switch (n) {
+            case 16u: launch_n<GATE_UP, 16u, true, false>(p, sms, stream); break;
+            case 32u: launch_n<GATE_UP, 32u, true, false>(p, sms, stream); break;
+            case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, kWide, true, !GATE_UP>(p, sms, stream); break;
         }
     } else {
         switch (n) {
-            case 16u: launch_n<GATE_UP, 16u, false>(p, stream); break;
-            case 32u: launch_n<GATE_UP, 32u, false>(p, stream); break;
-            case 64u: launch_n<GATE_UP, 64u, false>(p, stream); break;
-            default: launch_n<GATE_UP, kWide, false>(p, stream); break;
+            case 16u: launch_n<GATE_UP, 16u, false, false>(p, sms, stream); break;
+            case 32u: launch_n<GATE_UP, 32u, false, false>(p, sms, stream); break;
+            case 64u: launch_n<GATE_UP, 64u, false, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, kWide, false, !GATE_UP>(p, sms, stream); break;
         }
     }
 }
 
-template <bool GATE_UP, uint32_t N_TILE>
+template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR>
 void configure_one() {
-    constexpr bool kPair = row_pair<GATE_UP, N_TILE>();
-    cudaFuncSetAttribute(experts_tc_kernel<GATE_UP, N_TILE, true, kPair, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Config<GATE_UP, N_TILE, true, kPair>::kSmemBytes);
-    cudaFuncSetAttribute(experts_tc_kernel<GATE_UP, N_TILE, true, kPair, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Config<GATE_UP, N_TILE, true, kPair>::kSmemBytes);
-    cudaFuncSetAttribute(experts_tc_kernel<GATE_UP, N_TILE, false, kPair, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Config<GATE_UP, N_TILE, false, kPair>::kSmemBytes);
+    constexpr int kBytes = (int)Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::kSmemBytes;
+    cudaFuncSetAttribute(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, ROW_PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (USE_TMA)
+        cudaFuncSetAttribute(experts_tc_kernel<GATE_UP, N_TILE, USE_TMA, ROW_PAIR, USE_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+}
+
+template <uint32_t N_TILE>
+void configure_tile() {
+    configure_one<true, N_TILE, true, false>();
+    configure_one<true, N_TILE, false, false>();
+    configure_one<false, N_TILE, true, true>();
+    configure_one<false, N_TILE, false, (N_TILE >= 64u)>();
+    if (N_TILE < 64u) configure_one<false, N_TILE, true, (N_TILE >= 64u)>();
 }
 
 }  // namespace
@@ -1012,14 +1037,10 @@ void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8
 
 
 void tc_configure_kernels() {
-    configure_one<true, 16u>();
-    configure_one<true, 32u>();
-    configure_one<true, 64u>();
-    configure_one<true, 96u>();
-    configure_one<false, 16u>();
-    configure_one<false, 32u>();
-    configure_one<false, 64u>();
-    configure_one<false, 96u>();
+    configure_tile<16u>();
+    configure_tile<32u>();
+    configure_tile<64u>();
+    configure_tile<96u>();
 }
 
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<true>(p, stream); }
