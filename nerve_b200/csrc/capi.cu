@@ -502,14 +502,15 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         want(p->grouped_q[1], R * I);
         want(p->grouped_e8m0[0], sizeof(uint32_t) * R * ((H + 127u) / 128u));
         want(p->grouped_e8m0[1], sizeof(uint32_t) * R * ((I + 127u) / 128u));
-        want(p->act_maps, 8u * 128u);
+        want(p->act_maps, 10u * 128u);
         if (err == cudaSuccess) {
-            unsigned char maps[8 * 128];
+            unsigned char maps[10 * 128];
+            const uint32_t token_tiles[5] = {16u, 32u, 64u, 96u, 128u};
             bool ok = true;
             for (uint32_t set = 0; set < 2u && ok; set++)
-                for (uint32_t i = 0; i < 4u && ok; i++)
-                    ok = tc_encode_activation_map(maps + (set * 4u + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R,
-                                                  (uint32_t)(set == 0u ? H : I), i < 3u ? 16u << i : 96u);
+                for (uint32_t i = 0; i < 5u && ok; i++)
+                    ok = tc_encode_activation_map(maps + (set * 5u + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R,
+                                                  (uint32_t)(set == 0u ? H : I), token_tiles[i]);
             if (ok) {
                 err = cudaMemcpyAsync(p->act_maps.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
                 if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
@@ -818,7 +819,8 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
     p->launches += (size_t)T * p->K <= 4096u ? 1u : 3u;
     if (tensor) {
         uint32_t* region = p->tile_list.as<uint32_t>() + set * tile_region_words(p);
-        launch_build_tiles(p->offsets[set].as<uint32_t>(), p->experts, tc_token_tile_for(T, p->K, p->experts, gate_up), region + 64,
+        const uint32_t rows = gate_up ? p->g.intermediate_size : p->g.hidden_size;
+        launch_build_tiles(p->offsets[set].as<uint32_t>(), p->experts, tc_token_tile_for(T, p->K, p->experts, rows, gate_up), region + 64,
                            region, st);
         p->launches++;
     }
@@ -914,8 +916,9 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     el.wait_cycles = p->wait_cycles;
     el.debug_flags = p->debug_flags;
     if (tensor) {
-        const uint32_t size_index = tc_token_tile_index(tc_token_tile_for(T, p->K, p->experts, gate_up));
-        el.act_tmap = el.tmaps ? p->act_maps.as<uint8_t>() + (set * 4u + size_index) * 128u : nullptr;
+        const uint32_t size_index = tc_token_tile_index(
+            tc_token_tile_for(T, p->K, p->experts, gate_up ? g.intermediate_size : g.hidden_size, gate_up));
+        el.act_tmap = el.tmaps ? p->act_maps.as<uint8_t>() + (set * 5u + size_index) * 128u : nullptr;
         if (c.fuse_quantise && gate_up) {
             el.q_out = p->grouped_q[1].as<uint8_t>();
             el.q_e8m0 = p->grouped_e8m0[1].as<uint32_t>();
@@ -1275,7 +1278,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     ExpertSet* es = nullptr;
     NVMOE_TRY(prepare_expert_set(sub, false, m->addresses, dl->slots, tensor, &es));
     uint32_t* region = sub->tile_list.as<uint32_t>() + tile_region_words(sub);
-    launch_dense_schedule(T, tc_token_tile_for(T, 1u, 1u, false), sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(),
+    launch_dense_schedule(T, tc_token_tile_for(T, 1u, 1u, rows, false), sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(),
                           sub->position[1].as<uint32_t>(), tensor ? region + 64 : nullptr, tensor ? region : nullptr, st);
     sub->launches++;
     NVMOE_TRY(post_launch(sub, "dense linear schedule"));
@@ -1456,8 +1459,8 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         ls.tiles_per_route[0] = (g.intermediate_size + g.gate_tile_rows - 1u) / g.gate_tile_rows;
         ls.tiles_per_route[1] = (g.hidden_size + g.down_tile_rows - 1u) / g.down_tile_rows;
         ls.num_experts = p->experts;
-        ls.n_tile[0] = tc_token_tile_for(T, p->K, p->experts, true);
-        ls.n_tile[1] = tc_token_tile_for(T, p->K, p->experts, false);
+        ls.n_tile[0] = tc_token_tile_for(T, p->K, p->experts, g.intermediate_size, true);
+        ls.n_tile[1] = tc_token_tile_for(T, p->K, p->experts, g.hidden_size, false);
         p->launches += launch_layer_schedule(ls, sort_scratch(p), st);
         NVMOE_TRY(post_launch(p, "layer schedule"));
     } else {

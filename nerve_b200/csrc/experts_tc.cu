@@ -48,6 +48,7 @@ constexpr uint32_t kTmaBoxBytes = kBlockM * 64u;   // global bytes of one 128 x 
 constexpr uint32_t kATileBytes = kBlockM * 128u;   // one byte slot per element
 constexpr uint32_t kScaleBlockBytes = 512u;        // 128 rows x 4 scale bytes
 constexpr uint32_t kMaxStages = 8u;
+constexpr uint32_t kTargetSms = 148u;
 constexpr uint32_t kRowPairRounds = 6u;  // tiles an SM goes through at least before narrow down tiles pair their rows
 constexpr uint32_t kWatchWarp = 2u;     // the epilogue warp that polls for a finished accumulator (not on the MMA or TMA warp's scheduler)
 
@@ -119,9 +120,19 @@ struct Config {
     static constexpr uint32_t kBRegion = kBlocks * kABytes;                    // offset of the token tiles
     static constexpr uint32_t kSfRegion = kBRegion + kBlocks * kBTileBytes;    // offset of the scale blocks
     static constexpr uint32_t kAccColumns = kMatrices * N_TILE;
-    static constexpr uint32_t kAccStages = (2u * kAccColumns + 16u <= 512u) ? 2u : 1u;
+    static constexpr uint32_t kAccStages = 2u;
     static constexpr uint32_t kScaleColumns = 4u * (kMatrices + 1u);
-    static constexpr uint32_t kColumnsUsed = kAccStages * kAccColumns + kScaleColumns;
+    // Two accumulators of 128 tokens and two matrices would be all of tensor memory, with no columns left for the
+    // scales. They share 16 columns instead: the last tokens' second matrix of the first accumulator lies where the
+    // second accumulator keeps the first tokens' first matrix. The epilogue reads that chunk before all others and
+    // says so (acc_head), and the MMAs of the next tile wait for it: about a microsecond per tile, during which the
+    // ring fills. Wider tiles fetch fewer weight bytes per token, and the MMA itself is bound by its operand reads
+    // from shared memory below 128 columns (64.8 cycles at 96 columns, 68.5 at 128).
+    static constexpr bool kOverlap = 2u * kAccColumns + kScaleColumns > 512u;
+    static constexpr uint32_t kAccStride = kOverlap ? kAccColumns - 16u : kAccColumns;
+    static constexpr uint32_t kScaleColumn0 = (kAccStages - 1u) * kAccStride + kAccColumns;
+    static constexpr uint32_t kColumnsUsed = kScaleColumn0 + kScaleColumns;
+    static_assert(kColumnsUsed <= 512u, "tensor memory");
     static constexpr uint32_t kTmemColumns = kColumnsUsed <= 32u ? 32u : kColumnsUsed <= 64u ? 64u : kColumnsUsed <= 128u ? 128u : kColumnsUsed <= 256u ? 256u : 512u;
     static constexpr uint32_t kSmemBytes = kStages * kStageBytes + (kNeedsAlignedBase ? 0u : 1024u) + kBarrierBytes;
     static_assert(N_TILE % 16u == 0u && N_TILE >= 16u && N_TILE <= 128u, "token tile");
@@ -151,6 +162,7 @@ struct Barriers {
     uint64_t empty[kMaxStages];
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
+    uint64_t acc_head[2];         // overlapping accumulators: the shared chunk of this one has been read
     uint64_t drain;
     uint32_t tmem_base;
     uint32_t abort;
@@ -211,6 +223,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         for (uint32_t a = 0; a < 2u; a++) {
             mbar_init(&bars->acc_full[a], 1u);
             mbar_init(&bars->acc_empty[a], C::kEpilogueThreads);
+            mbar_init(&bars->acc_head[a], 128u);
         }
         mbar_init(&bars->drain, 1u);
         bars->abort = 0u;
@@ -229,7 +242,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
-    const uint32_t tmem_scales = tmem_base + C::kAccStages * C::kAccColumns;
+    const uint32_t tmem_scales = tmem_base + C::kScaleColumn0;
     // everything above touched only this CTA's shared and tensor memory; what follows reads what the
     // kernels before this one wrote
     grid_dependency_sync();
@@ -529,9 +542,12 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 const uint32_t acc = acc_it % C::kAccStages;
                 const long long a0 = TRACE ? clock64() : 0;
                 if (!mbar_wait(&bars->acc_empty[acc], ((acc_it / C::kAccStages) & 1u) ^ 1u, abort_flag, wait_limit)) break;
+                if (C::kOverlap && acc_it != 0u &&
+                    !mbar_wait(&bars->acc_head[acc ^ 1u], ((acc_it - 1u) / C::kAccStages) & 1u, abort_flag, wait_limit))
+                    break;
                 if (TRACE) trace_acc += clock64() - a0;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * C::kAccColumns;
+                const uint32_t d_tmem = tmem_base + acc * C::kAccStride;
                 for (uint32_t ks = 0; ks < k_stages; ks++, it++) {
                     const long long f0 = TRACE ? clock64() : 0;
                     if (!mbar_wait(&bars->full[slot], full_parity, abort_flag, wait_limit)) {
@@ -632,14 +648,23 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             tc_fence_after();
             const uint32_t row = m_tile * C::kTileRows + quad * 32u + lane;  // (with row pairs: of the first half)
             const bool row_ok = row < out_rows;
-            const uint32_t lane_addr = tmem_base + ((quad * 32u) << 16) + acc * C::kAccColumns;
+            const uint32_t lane_addr = tmem_base + ((quad * 32u) << 16) + acc * C::kAccStride;
             // The epilogue groups share out a wide tile by 16-column chunks. A narrow tile (one or two chunks)
             // is shared out by sets of four tokens instead, every group reading the chunk: a tile of eight
             // tokens is then two groups' work side by side, not one group's in turn.
             constexpr bool kShareByFours = N_TILE <= 32u && C::kEpilogueGroups > 1u;
-            for (uint32_t c0 = kShareByFours ? 0u : 16u * epilogue_group; c0 < N_TILE;
-                 c0 += kShareByFours ? 16u : 16u * C::kEpilogueGroups) {
-                if (c0 >= valid) break;  // uniform: no token of this tile lives in the remaining columns
+            for (uint32_t n0 = kShareByFours ? 0u : 16u * epilogue_group; n0 < N_TILE;
+                 n0 += kShareByFours ? 16u : 16u * C::kEpilogueGroups) {
+                // the chunk that overlapping accumulators share comes first: the last of the first one, the first of the second
+                const uint32_t c0 = C::kOverlap && acc == 0u ? N_TILE - 16u - n0 : n0;
+                const bool head = C::kOverlap && n0 == 0u;  // (group 0's)
+                if (c0 >= valid) {  // uniform: no token of this tile lives in these columns
+                    if (head) {
+                        tc_fence_before();
+                        mbar_arrive(&bars->acc_head[acc]);
+                    }
+                    continue;
+                }
                 if (kShareByFours) {
                     // does any of this chunk's sets of four fall to this group? (uniform)
                     bool mine = false;
@@ -671,6 +696,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                     }
                 }
                 tmem_ld_wait();
+                if (head) {
+                    tc_fence_before();
+                    mbar_arrive(&bars->acc_head[acc]);
+                }
                 const bool quantise = GATE_UP && p.q_out != nullptr;  // host: only with scale blocks of 32 or 128 rows
                 const bool store_rows = !GATE_UP || p.intermediates != nullptr;  // (uniform) a caller's rows; a layer only needs their codes
                 // Four tokens at a time go through each step together, with no branch between them, so that
@@ -870,12 +899,12 @@ bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) 
 
 template <bool GATE_UP>
 void launch(const ExpertLaunch& p, cudaStream_t stream) {
-    constexpr uint32_t kWide = 96u;
     int dev = 0;
     cudaGetDevice(&dev);
     if (g_sm_count[dev & 15] == 0) cudaDeviceGetAttribute(&g_sm_count[dev & 15], cudaDevAttrMultiProcessorCount, dev);
     const int sms = g_sm_count[dev & 15];
-    const uint32_t n = tc_token_tile_for(p.tokens, p.g.routed_k + p.g.always_count, p.work.num_experts, GATE_UP);
+    const uint32_t n = tc_token_tile_for(p.tokens, p.g.routed_k + p.g.always_count, p.work.num_experts,
+                                         GATE_UP ? p.g.intermediate_size : p.g.hidden_size, GATE_UP);
     const bool tma = p.tmaps != nullptr;
     const bool pairs = !GATE_UP && takes_row_pairs(p, n, tma, sms);
     if (tma && pairs) {
@@ -883,21 +912,24 @@ void launch(const ExpertLaunch& p, cudaStream_t stream) {
             case 16u: launch_n<GATE_UP, 16u, true, !GATE_UP>(p, sms, stream); break;
             case 32u: launch_n<GATE_UP, 32u, true, !GATE_UP>(p, sms, stream); break;
             case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
-            default: launch_n<GATE_UP, kWide, true, !GATE_UP>(p, sms, stream); break;
+            case 96u: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, 128u, true, !GATE_UP>(p, sms, stream); break;
         }
     } else if (tma) {
         switch (n) {
             case 16u: launch_n<GATE_UP, 16u, true, false>(p, sms, stream); break;
             case 32u: launch_n<GATE_UP, 32u, true, false>(p, sms, stream); break;
             case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
-            default: launch_n<GATE_UP, kWide, true, !GATE_UP>(p, sms, stream); break;
+            case 96u: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, 128u, true, !GATE_UP>(p, sms, stream); break;
         }
     } else {
         switch (n) {
             case 16u: launch_n<GATE_UP, 16u, false, false>(p, sms, stream); break;
             case 32u: launch_n<GATE_UP, 32u, false, false>(p, sms, stream); break;
             case 64u: launch_n<GATE_UP, 64u, false, !GATE_UP>(p, sms, stream); break;
-            default: launch_n<GATE_UP, kWide, false, !GATE_UP>(p, sms, stream); break;
+            case 96u: launch_n<GATE_UP, 96u, false, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, 128u, false, !GATE_UP>(p, sms, stream); break;
         }
     }
 }
@@ -927,18 +959,37 @@ bool tc_shape_supported(const nvmoe_geometry& g) {
 
 bool tc_enabled_by_default() { return true; }
 
-uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, bool gate_up) {
+uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up) {
     // tokens per expert if routing were uniform; skew only adds token tiles
     const uint32_t routes = tokens * routes_per_token;
     const uint32_t per_expert = (routes + num_experts - 1u) / num_experts;
-    // wide tiles hold two accumulators per token column (gate and up, or two row tiles of down): 96 columns
-    // is the widest tile that still leaves tensor memory for a second pair, so that the epilogue of one
-    // tile overlaps the MMAs of the next
-    (void)gate_up;
-    return per_expert <= 12u ? 16u : per_expert <= 24u ? 32u : per_expert <= 48u ? 64u : 96u;
+    // the narrowest tile that holds an expert's tokens (with some room for skew: a second tile reads the weights again)
+    if (per_expert <= 12u) return 16u;
+    if (per_expert <= 24u) return 32u;
+    if (per_expert <= 48u) return 64u;
+    if (per_expert <= 96u) return 96u;
+    // Beyond that an expert takes several tiles and the wide ones are the cheapest per token (a stage of 128 columns
+    // takes about 56/50 of the time of one of 96: 16384 tokens x 7168 x 2048 in 256 experts 9.98 against 10.48 ms), unless
+    // a wave of the SMs goes half empty with them (777 x 7168 x 2048 dense: 115 us with 128 columns, 109 with 96): the
+    // fewest rounds x stage time wins.
+    const uint32_t row_tiles = gate_up ? (out_rows + kBlockM - 1u) / kBlockM : (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM);
+    const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {56u, 50u};
+    uint32_t best = 0u;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t i = 0; i < 2u; i++) {
+        const uint64_t tiles = (uint64_t)num_experts * ((per_expert + widths[i] - 1u) / widths[i]) * row_tiles;
+        const uint64_t cost = (tiles + kTargetSms - 1u) / kTargetSms * stage_time[i];
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = widths[i];
+        }
+    }
+    return best;
 }
 
-uint32_t tc_token_tile_index(uint32_t n_tile) { return n_tile == 16u ? 0u : n_tile == 32u ? 1u : n_tile == 64u ? 2u : 3u; }
+uint32_t tc_token_tile_index(uint32_t n_tile) {
+    return n_tile == 16u ? 0u : n_tile == 32u ? 1u : n_tile == 64u ? 2u : n_tile == 96u ? 3u : 4u;
+}
 
 size_t tc_derived_scale_bytes(uint32_t rows, uint32_t cols) {
     return (size_t)((rows + kBlockM - 1u) / kBlockM) * ((cols + kBlockK - 1u) / kBlockK) * kScaleBlockBytes;
@@ -1041,6 +1092,7 @@ void tc_configure_kernels() {
     configure_tile<32u>();
     configure_tile<64u>();
     configure_tile<96u>();
+    configure_tile<128u>();
 }
 
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<true>(p, stream); }
