@@ -783,9 +783,9 @@ __global__ void __launch_bounds__(256) layer_schedule_hist_kernel(LayerSchedule 
 }
 
 __host__ __device__ inline size_t layer_schedule_wide_smem_bytes(uint32_t num_experts) {
-    // the compact list's, two groupings' and two tile lists' bases; ranks of this block; [warp][bucket] counts (u16); kept[2]
+    // the compact list's, two groupings' and two tile lists' bases; ranks of this block; totals; [warp][bucket] counts (u16); kept[2]
     const size_t buckets = (size_t)num_experts + 1u;
-    return (5u * (buckets + 1u) + buckets) * sizeof(uint32_t) + (8u * buckets + 1u) / 2u * 4u + 2u * buckets;
+    return (5u * (buckets + 1u) + 2u * buckets) * sizeof(uint32_t) + (8u * buckets + 1u) / 2u * 4u + 2u * buckets;
 }
 
 __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedule s, const uint32_t* __restrict__ block_hist,
@@ -796,7 +796,8 @@ __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedu
     uint32_t* gbase[2] = {base_all + (B + 1u), base_all + 2u * (B + 1u)};
     uint32_t* tile_base[2] = {base_all + 3u * (B + 1u), base_all + 4u * (B + 1u)};
     uint32_t* first = base_all + 5u * (B + 1u);
-    uint32_t* table_words = first + B;
+    uint32_t* total = first + B;
+    uint32_t* table_words = total + B;
     uint16_t* table = reinterpret_cast<uint16_t*>(table_words);
     uint8_t* kept = reinterpret_cast<uint8_t*>(table_words + (8u * B + 1u) / 2u);  // [2][B]: the stage keeps routes of this bucket
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -807,6 +808,7 @@ __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedu
     if (i < count) bucket = min_u32(__ldg(s.routes + i) & 0xffffu, E);
     for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) {
         first[b] = __ldg(block_hist + (size_t)blockIdx.x * B + b);
+        total[b] = __ldg(totals + b);
 #pragma unroll
         for (uint32_t stage = 0; stage < 2u; stage++) kept[stage * B + b] = (b < E && s.experts[stage][b].w[0] != nullptr) ? 1u : 0u;
     }
@@ -816,12 +818,12 @@ __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedu
     if (bucket != kNotListed && before == 0u) table[warp * B + bucket] = (uint16_t)__popc(peers);
     if (warp < 5u) {  // five scans, a warp each
         const uint32_t stage = warp == 0u ? 0u : (warp - 1u) & 1u;
-        uint32_t* out = warp == 0u ? base_all : warp >= 3u ? tile_base[stage] : gbase[stage];
-        warp_exclusive_scan(B, out, [&](uint32_t b) {
-            const uint32_t v = __ldg(totals + b);
+        const uint32_t n_tile = stage == 0u ? s.n_tile[0] : s.n_tile[1];
+        warp_exclusive_scan(B, base_all + warp * (B + 1u), [&](uint32_t b) {  // (the arrays lie in the warps' order)
+            const uint32_t v = total[b];
             if (warp == 0u) return v;
             if (!kept[stage * B + b]) return 0u;
-            return warp >= 3u ? (v + s.n_tile[stage] - 1u) / s.n_tile[stage] : v;
+            return warp >= 3u ? (v + n_tile - 1u) / n_tile : v;
         });
     }
     __syncthreads();
@@ -843,28 +845,25 @@ __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedu
             if (s.position[stage]) s.position[stage][i] = place;
         }
     }
-    if (blockIdx.x != 0u) return;
-    if (threadIdx.x < 14u) {
-        const uint32_t stage = threadIdx.x / 7u, j = threadIdx.x % 7u;
-        uint32_t value = 1u;  // word 6
-        if (j == 0u || j == 5u) value = s.tokens;
-        if (j == 1u) value = s.expert_start;
-        if (j == 2u) value = 0u;
-        if (j == 3u) value = count;
-        if (j == 4u) value = s.K * s.tiles_per_route[stage];
-        s.control[stage][j] = value;
-    }
-    for (uint32_t x = threadIdx.x; x < 2u * B; x += blockDim.x) {
-        const uint32_t stage = x / B, b = x % B;
-        s.offsets[stage][b] = gbase[stage][b];  // bucket E is never kept: gbase[stage][E] is the total
-        if (s.tiles[stage] && b == E) *s.tile_count[stage] = tile_base[stage][E];
-    }
-    // tile lists: a warp per (stage, expert), its tiles side by side
-    for (uint32_t x = warp; x < 2u * E; x += blockDim.x >> 5) {
-        const uint32_t stage = x / E, b = x % E;
+    // tile lists: a warp per expert, its tiles side by side, the experts shared out over the blocks (by block 0 alone the
+    // lists of 257 experts took 20 us)
+#pragma unroll
+    for (uint32_t stage = 0; stage < 2u; stage++) {
         if (!s.tiles[stage]) continue;
-        const uint32_t at = tile_base[stage][b], n = tile_base[stage][b + 1u] - at;
-        for (uint32_t j = lane; j < n; j += 32u) s.tiles[stage][at + j] = (b << 16) | j;
+        for (uint32_t b = blockIdx.x * 8u + warp; b < E; b += gridDim.x * 8u) {
+            const uint32_t at = tile_base[stage][b], n = tile_base[stage][b + 1u] - at;
+            for (uint32_t j = lane; j < n; j += 32u) s.tiles[stage][at + j] = (b << 16) | j;
+        }
+    }
+    if (blockIdx.x != 0u) return;
+#pragma unroll
+    for (uint32_t stage = 0; stage < 2u; stage++) {
+        const uint32_t j = threadIdx.x;
+        if (j < 7u)
+            s.control[stage][j] = j == 0u || j == 5u ? s.tokens : j == 1u ? s.expert_start : j == 2u ? 0u : j == 3u ? count
+                                  : j == 4u ? s.K * s.tiles_per_route[stage] : 1u;
+        for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) s.offsets[stage][b] = gbase[stage][b];  // bucket E is never kept: the total
+        if (s.tiles[stage] && threadIdx.x == 0u) *s.tile_count[stage] = tile_base[stage][E];
     }
 }
 
