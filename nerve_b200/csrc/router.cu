@@ -271,12 +271,13 @@ __global__ void __launch_bounds__(128) router_kernel(RouterLaunch p, uint32_t wa
 }
 
 // ---- the same router with a token's experts in registers ------------------------------------------
-// For up to 32 * EPL experts and at most 32 selections a token, without group-limited masking: lane l keeps the
+// For up to 32 * EPL experts and at most 32 selections a token; GROUPS: with group-limited masking, for groups of a
+// power of two of experts up to 32, which are then a run of lanes: lane l keeps the
 // experts l, l + 32, .. in registers, lane r keeps selection r once it is made, and everything the kernel above
 // does through shared memory by one lane (the weights, the ascending order, packing, telemetry) is done by the
 // lanes side by side. Every sum that has an order keeps it (values travel by shuffle and are added in the same
 // sequence); the results are bit for bit those of router_kernel, which remains for the other cases.
-template <int EPL>
+template <int EPL, bool GROUPS>
 __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
     grid_dependency_sync();
     constexpr uint32_t kFull = 0xffffffffu;
@@ -344,6 +345,35 @@ __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
 
     // ---- k rounds of arg-max: lane r keeps selection r ---------------------------------------
     uint32_t taken = 0u, my_e = kUnboundSlot;
+    if (GROUPS) {
+        // a group's score is the sum of its two best; the experts of the groups outside the topk_group best count as taken
+        const uint32_t per = E / p.g.n_group, side = 32u / per;  // groups in a register slot of the warp
+        float my_group = kNegInf;
+#pragma unroll
+        for (int j = 0; j < EPL; j++) {
+            float first = lane + 32u * j < E && score[j] > kNegInf ? score[j] : kNegInf, second = kNegInf;
+            for (uint32_t o = 1u; o < per; o <<= 1) {
+                const float other_first = __shfl_xor_sync(kFull, first, o), other_second = __shfl_xor_sync(kFull, second, o);
+                second = fmaxf(fminf(first, other_first), fmaxf(second, other_second));
+                first = fmaxf(first, other_first);
+            }
+            const float group = __shfl_sync(kFull, per >= 2u ? __fadd_rn(first, second) : first, (lane % side) * per);
+            if (lane / side == (uint32_t)j) my_group = group;  // lane g keeps group g
+        }
+        uint32_t kept = 0u;
+        for (uint32_t round = 0; round < p.g.topk_group; round++) {
+            const bool open = lane < p.g.n_group && ((kept >> lane) & 1u) == 0u && my_group >= kNegInf;  // (not a NaN)
+            float s = open ? my_group : kNegInf;
+            uint32_t winner = open ? lane : kUnboundSlot;
+            warp_argmax(s, winner);
+            if (winner != kUnboundSlot) kept |= 1u << winner;
+        }
+#pragma unroll
+        for (int j = 0; j < EPL; j++) {
+            const uint32_t group = (uint32_t)j * side + lane / per;
+            if (group >= 32u || ((kept >> group) & 1u) == 0u) taken |= 1u << j;
+        }
+    }
     float my_v = 0.0f;
     bool missing = false;
     for (uint32_t r = 0; r < k; r++) {
@@ -453,7 +483,7 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
 
     // The sum order of a lane is fixed (its words in ascending order), the load order is not: the
     // loads of kDepth steps are issued together so that their latencies overlap.
-    constexpr int kDepth = TT * ET <= 16 ? 8 : 2;
+    constexpr int kDepth = TT * ET <= 16 ? 8 : TT * ET <= 32 ? 4 : 2;
     for (uint32_t cw0 = v; cw0 < words; cw0 += 64u * kDepth) {
         uint32_t xr[kDepth][TT], wr[kDepth][ET];
 #pragma unroll
@@ -627,14 +657,16 @@ void launch_router(const RouterLaunch& p, cudaStream_t stream) {
     const uint32_t total_k = p.g.routed_k + (p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u);
     // the routed form's softmax over all experts (neither normalised over the selection nor sigmoid) sums in expert order
     const bool sums_all = p.g.router_kind == NVMOE_ROUTER_TOPK_ROUTED && !p.g.normalize_selected && p.g.activation != NVMOE_ACT_SIGMOID;
-    if (E <= 256u && total_k <= 32u && p.g.n_group == 0u && !sums_all && p.g.router_kind <= NVMOE_ROUTER_TOPK_ROUTED) {
+    const uint32_t per = p.g.n_group ? E / p.g.n_group : 0u;
+    const bool lane_groups = p.g.n_group != 0u && per <= 32u && (per & (per - 1u)) == 0u;
+    if (E <= 256u && total_k <= 32u && (p.g.n_group == 0u || lane_groups) && !sums_all && p.g.router_kind <= NVMOE_ROUTER_TOPK_ROUTED) {
         const dim3 grid((p.tokens + 3u) / 4u), block(128);
-        if (E <= 32u) {
-            launch_chained(router_reg_kernel<1>, grid, block, 0, stream, p);
-        } else if (E <= 128u) {
-            launch_chained(router_reg_kernel<4>, grid, block, 0, stream, p);
+        if (lane_groups) {
+            launch_chained(E <= 32u ? router_reg_kernel<1, true> : E <= 128u ? router_reg_kernel<4, true> : router_reg_kernel<8, true>, grid,
+                           block, 0, stream, p);
         } else {
-            launch_chained(router_reg_kernel<8>, grid, block, 0, stream, p);
+            launch_chained(E <= 32u ? router_reg_kernel<1, false> : E <= 128u ? router_reg_kernel<4, false> : router_reg_kernel<8, false>, grid,
+                           block, 0, stream, p);
         }
         return;
     }
@@ -650,8 +682,15 @@ void launch_router(const RouterLaunch& p, cudaStream_t stream) {
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
                           uint32_t tokens, uint32_t hidden, uint32_t outputs, cudaStream_t stream) {
     if (tokens <= 256u) {
-        dim3 grid((outputs + 3u) / 4u, (tokens + 1u) / 2u);
-        launch_chained(router_linear_kernel<2, 4>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);
+        const dim3 grid((outputs + 3u) / 4u, (tokens + 1u) / 2u), wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
+        // small tiles for small calls, which need the blocks; a tile of 4 x 8 reads half the bytes from L2 per pair once
+        // its blocks still give every SM four (96 x 7168 x 256: 24 against 30 us with cold caches, 27 against 26 with
+        // warm ones; 256 x 2880 x 128 warm: 14.4 against 16.4)
+        if (wide.x * wide.y >= 4u * 148u) {
+            launch_chained(router_linear_kernel<4, 8>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);
+        } else {
+            launch_chained(router_linear_kernel<2, 4>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);
+        }
     } else if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u) {
         dim3 grid((outputs + kTileOutputs - 1u) / kTileOutputs, (tokens + kTileTokens - 1u) / kTileTokens);
         launch_chained(router_linear_tiled_kernel, grid, dim3(256), 0, stream, x, w, bias, logits, tokens, hidden, outputs);

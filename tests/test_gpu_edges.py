@@ -104,3 +104,43 @@ def test_layer_call_equals_its_nodes(device, name, shape, tokens, absent):
     np.testing.assert_array_equal(out.read(np.uint16), want.read(np.uint16))
     assert missed == plan.status() and (missed == 0) == (absent is None)
     plan.destroy()
+
+
+# the 4 x 8 tiles with ragged tokens, an odd expert count and rows that end inside a step; the call just below them;
+# the tiled form with a row of less than one chunk and last chunks that end in their first or second half
+@pytest.mark.parametrize("tokens,hidden,experts,bias", [(98, 288, 199, 1), (255, 1056, 74, 0), (94, 288, 192, 0), (257, 32, 17, 0),
+                                                        (289, 288, 8, 1), (300, 352, 33, 0)])
+def test_router_projection_tiles(device, tokens, hidden, experts, bias):
+    rng = np.random.default_rng(tokens + hidden)
+    plan = plan_of(device, tokens=tokens, hidden=hidden, experts=experts)
+    x, w = bf16(rng.standard_normal((tokens, hidden))), bf16(0.1 * rng.standard_normal((experts, hidden)))
+    b = bf16(rng.standard_normal(experts)) if bias else None
+    out = device.create_resident_buffer(tokens * ((experts + 1) // 2) * 4)
+    plan.linear(tokens, device.resident_buffer_from(x), out, device.resident_buffer_from(w),
+                device.resident_buffer_from(b) if bias else None)
+    np.testing.assert_array_equal(out.read(np.uint32).reshape(tokens, -1), mo.linear_bf16(x, w, b))
+    plan.destroy()
+
+
+# groups of one expert, of two (less than a warp of experts), of 16 and of 32, one beyond the lanes (the shared-memory
+# form), every group kept; logits with ties, infinities and NaN
+@pytest.mark.parametrize("experts,n_group,topk_group,k", [(24, 24, 5, 4), (16, 8, 3, 4), (128, 8, 4, 6), (256, 8, 4, 8), (256, 8, 8, 8),
+                                                          (64, 1, 1, 3), (256, 4, 2, 8)])
+@pytest.mark.parametrize("activation", [synthetic.ACT_SIGMOID, synthetic.ACT_SOFTMAX])
+def test_group_limited_routing(device, experts, n_group, topk_group, k, activation):
+    cfg = synthetic.MoeConfig("groups", 256, 256, experts, k, activation=activation, n_group=n_group, topk_group=topk_group,
+                              always_count=1, bias_dtype=synthetic.BIAS_F32, act_block=32)
+    rng = np.random.default_rng(experts + n_group)
+    tokens = 61
+    logits = np.round(2.0 * rng.standard_normal((tokens, experts))).astype(np.float32)
+    if activation == synthetic.ACT_SIGMOID:
+        logits[3, ::3], logits[4, 1::5], logits[5, :2] = np.inf, -np.inf, np.nan
+    bias = np.round(2.0 * rng.standard_normal(experts)).astype(np.float32) / 8
+    bias[:2] = 0.0
+    words = bf16(logits).view(np.uint32)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    routes = device.create_resident_buffer(tokens * cfg.total_k * 4)
+    plan.moe_route(tokens, device.resident_buffer_from(words), routes, device.resident_buffer_from(bias), None)
+    want, _ = mo.route(mo.router_params_from(cfg), words, bias)
+    np.testing.assert_array_equal(routes.read(np.uint32).reshape(want.shape), want)
+    plan.destroy()
