@@ -32,7 +32,10 @@ __global__ void __launch_bounds__(256) reduce_kernel(const uint32_t* __restrict_
 }
 
 // The same sum over 16-byte pieces (eight columns a thread) for rows that allow it: the order of the adds
-// of a column and every rounding are unchanged.
+// of a column and every rounding are unchanged. Bound by memory: DEPTH routes are fetched together, their marks first,
+// so that the usual layers (up to 4 or 9 routes a token) pay two memory round trips per piece and not two for every
+// four routes.
+template <uint32_t DEPTH>
 __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict__ expert_outputs, uint4* __restrict__ output,
                                                         uint32_t tokens, uint32_t K, uint32_t hidden_vecs, float routed_scale,
                                                         const uint32_t* __restrict__ computed) {
@@ -44,19 +47,18 @@ __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict
         float acc[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j] = 0.0f;
-        // four routes at a time: their marks and rows are fetched together (one memory round trip instead of one
-        // per route), the adds keep the route order
-        for (uint32_t r0 = 0; r0 < K; r0 += 4u) {
-            bool skipped[4];
-            uint4 c[4];
+        // (the adds keep the route order)
+        for (uint32_t r0 = 0; r0 < K; r0 += DEPTH) {
+            bool skipped[DEPTH];
+            uint4 c[DEPTH];
 #pragma unroll
-            for (uint32_t u = 0; u < 4u; u++)
+            for (uint32_t u = 0; u < DEPTH; u++)
                 // a route the down stage skipped (computed[route] says "nowhere") counts as a row of zeros
                 skipped[u] = r0 + u >= K || (computed && __ldg(computed + (size_t)t * K + r0 + u) == kUnboundSlot);
 #pragma unroll
-            for (uint32_t u = 0; u < 4u; u++) c[u] = skipped[u] ? make_uint4(0u, 0u, 0u, 0u) : in[(size_t)(r0 + u) * hidden_vecs];
+            for (uint32_t u = 0; u < DEPTH; u++) c[u] = skipped[u] ? make_uint4(0u, 0u, 0u, 0u) : in[(size_t)(r0 + u) * hidden_vecs];
 #pragma unroll
-            for (uint32_t u = 0; u < 4u; u++) {
+            for (uint32_t u = 0; u < DEPTH; u++) {
                 if (r0 + u >= K) break;
                 const uint32_t w[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
 #pragma unroll
@@ -176,7 +178,7 @@ void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t to
         const uint64_t vecs = (uint64_t)tokens * (hidden / 8u);
         uint64_t vec_blocks = (vecs + 255u) / 256u;
         if (vec_blocks > 148u * 16u) vec_blocks = 148u * 16u;
-        launch_chained(reduce_vec_kernel, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
+        launch_chained(K <= 4u ? reduce_vec_kernel<4u> : reduce_vec_kernel<9u>, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
                        reinterpret_cast<const uint4*>(expert_outputs), reinterpret_cast<uint4*>(output), tokens, K, hidden / 8u,
                        routed_scale, computed);
         return;
