@@ -632,9 +632,9 @@ int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, n
     return post_launch(p, "router projection");
 }
 
-int nvmoe_route(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* logits, nvmoe_buffer* routes,
-                const nvmoe_buffer* bias, nvmoe_buffer* telemetry) {
-    if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
+// checks the router's buffers and fills its launch block
+static int router_launch_for(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* logits, nvmoe_buffer* routes, const nvmoe_buffer* bias,
+                             nvmoe_buffer* telemetry, RouterLaunch* out) {
     NVMOE_TRY(check_tokens(p, T));
     const nvmoe_geometry& g = p->g;
     NVMOE_TRY(check_buffer(p, logits, (size_t)T * ((g.routed_experts + 1u) / 2u) * 4u, "logits"));
@@ -648,8 +648,8 @@ int nvmoe_route(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* logits, nvmoe_buf
         const size_t r = p->experts;
         NVMOE_TRY(check_buffer(p, telemetry, (r + r * (r - 1u) / 2u) * 4u, "telemetry"));
     }
-    NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
-    RouterLaunch rl{};
+    RouterLaunch& rl = *out;
+    rl = RouterLaunch{};
     rl.logits = (const uint32_t*)logits->ptr;
     rl.bias = uses_bias ? bias->ptr : nullptr;
     rl.routes = (uint32_t*)routes->ptr;
@@ -658,6 +658,15 @@ int nvmoe_route(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* logits, nvmoe_buf
     rl.tokens = T;
     rl.g = g;
     if (!uses_bias) rl.g.bias_dtype = NVMOE_BIAS_NONE;
+    return NVMOE_OK;
+}
+
+int nvmoe_route(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* logits, nvmoe_buffer* routes,
+                const nvmoe_buffer* bias, nvmoe_buffer* telemetry) {
+    if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
+    RouterLaunch rl;
+    NVMOE_TRY(router_launch_for(p, T, logits, routes, bias, telemetry, &rl));
+    NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     launch_router(rl, p->device->stream);
     p->launches++;
     return post_launch(p, "router");
@@ -1422,7 +1431,18 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     if (a->router_weights && !a->routes_in)
         NVMOE_TRY(nvmoe_router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias));
     mark(kStageRoute);
-    if (!a->routes_in) NVMOE_TRY(nvmoe_route(p, T, logits, routes, a->bias, a->telemetry));
+    // (with stage profiling on, the router keeps a launch and a time of its own)
+    RouterLaunch router{};
+    bool routes_in_schedule = false;
+    if (!a->routes_in) {
+        NVMOE_TRY(router_launch_for(p, T, logits, routes, a->bias, a->telemetry, &router));
+        routes_in_schedule = !prof && layer_routes_in_schedule(router, p->K, p->experts);
+        if (!routes_in_schedule) {
+            launch_router(router, st);
+            p->launches++;
+            NVMOE_TRY(post_launch(p, "router"));
+        }
+    }
     mark(kStageSchedule);
     const bool tensor = use_tensor_path(p);
     // with scale blocks of 32 or 128 (what a warp, or the four warps of an epilogue group, hold of a token) the tensor-path
@@ -1461,7 +1481,12 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         ls.num_experts = p->experts;
         ls.n_tile[0] = tc_token_tile_for(T, p->K, p->experts, g.intermediate_size, true);
         ls.n_tile[1] = tc_token_tile_for(T, p->K, p->experts, g.hidden_size, false);
-        p->launches += launch_layer_schedule(ls, sort_scratch(p), st);
+        if (routes_in_schedule) {
+            launch_route_schedule(router, ls, st);
+            p->launches++;
+        } else {
+            p->launches += launch_layer_schedule(ls, sort_scratch(p), st);
+        }
         NVMOE_TRY(post_launch(p, "layer schedule"));
     } else {
         write_control_kernel<<<1, 32, 0, st>>>((uint32_t*)gate_control.ptr, T, a->expert_start, a->expert_count);

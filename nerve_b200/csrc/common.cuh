@@ -104,6 +104,7 @@ struct RouterLaunch {  // router.cu
     nvmoe_geometry g;
 };
 void launch_router(const RouterLaunch& p, cudaStream_t stream);
+bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selections, no groups: route_token covers it
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
                           uint32_t tokens, uint32_t hidden, uint32_t outputs, cudaStream_t stream);
 
@@ -144,6 +145,9 @@ struct LayerSchedule {
     uint32_t tokens, expert_start, expert_count, K, I, tiles_per_route[2], num_experts, n_tile[2];
 };
 bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned);
+// the router and the schedule of a call of up to 32 tokens in one launch
+bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts);
+void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream);
 uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream);  // returns its launches
 // validates the address/slot tables of every expert once per call
 // (rows, cols: logical shape of one matrix; experts from native_start on hold native FP8; with

@@ -13,36 +13,10 @@
 // the softmax-over-all of the routed form); the one order the shaders leave to the hardware, the
 // subgroup sum of the score_topk softmax, is pinned to 64 lane-strided partials folded by an xor
 // butterfly (32,16,8,4,2,1) — the same definition the CPU checker uses.
-#include "common.cuh"
+#include "router_reg.cuh"
 
 namespace nvmoe {
 namespace {
-
-constexpr float kNegInf = -__builtin_huge_valf();
-
-__device__ __forceinline__ float unpack_logit(const uint32_t* row, uint32_t e) {
-    uint32_t packed = row[e >> 1];
-    return nvmoe_bf16_to_f32((e & 1u) ? (packed >> 16) : packed);
-}
-
-__device__ __forceinline__ bool better(float s, uint32_t e, float best, uint32_t best_e) {
-    return s > best || (s == best && e < best_e);
-}
-
-// warp-wide arg-max of (score, expert) pairs under `better`; all lanes return the winner
-__device__ __forceinline__ void warp_argmax(float& s, uint32_t& e) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float os = __shfl_xor_sync(0xffffffffu, s, o);
-        uint32_t oe = __shfl_xor_sync(0xffffffffu, e, o);
-        // an empty candidate carries e == kUnboundSlot and can only win over another empty one
-        bool take = (oe != kUnboundSlot) && (e == kUnboundSlot || better(os, oe, s, e));
-        if (take) {
-            s = os;
-            e = oe;
-        }
-    }
-}
 
 struct WarpSmem {
     float* values;      // activated value (score_topk) or soft-capped logit (routed) or raw logit
@@ -52,12 +26,6 @@ struct WarpSmem {
     float* top_w;       // [kMaxTopK]
     float* group_score; // [32]
 };
-
-__device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uint32_t e) {
-    if (dtype == NVMOE_BIAS_F32) return reinterpret_cast<const float*>(bias)[e];
-    if (dtype == NVMOE_BIAS_BF16) return nvmoe_bf16_to_f32(reinterpret_cast<const uint16_t*>(bias)[e]);
-    return 0.0f;
-}
 
 __global__ void __launch_bounds__(128) router_kernel(RouterLaunch p, uint32_t warps_per_block) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -270,189 +238,11 @@ __global__ void __launch_bounds__(128) router_kernel(RouterLaunch p, uint32_t wa
     }
 }
 
-// ---- the same router with a token's experts in registers ------------------------------------------
-// For up to 32 * EPL experts and at most 32 selections a token; GROUPS: with group-limited masking, for groups of a
-// power of two of experts up to 32, which are then a run of lanes: lane l keeps the
-// experts l, l + 32, .. in registers, lane r keeps selection r once it is made, and everything the kernel above
-// does through shared memory by one lane (the weights, the ascending order, packing, telemetry) is done by the
-// lanes side by side. Every sum that has an order keeps it (values travel by shuffle and are added in the same
-// sequence); the results are bit for bit those of router_kernel, which remains for the other cases.
 template <int EPL, bool GROUPS>
 __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
     grid_dependency_sync();
-    constexpr uint32_t kFull = 0xffffffffu;
-    const uint32_t E = p.g.routed_experts;
-    const uint32_t k = p.g.routed_k;
-    const uint32_t kind = p.g.router_kind;
-    const uint32_t always = kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
-    const uint32_t total_k = k + always;
-    const uint32_t total_resources = E + always;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t token = blockIdx.x * 4u + warp;
-    if (token >= p.tokens) return;
-    const uint32_t* row = p.logits + (size_t)token * ((E + 1u) / 2u);
-
-    float val[EPL], score[EPL];
-#pragma unroll
-    for (int j = 0; j < EPL; j++) {
-        const uint32_t e = lane + 32u * j;
-        val[j] = e < E ? unpack_logit(row, e) : 0.0f;
-        score[j] = 0.0f;
-    }
-    // ---- activation and selection score ---------------------------------------------------
-    if (kind == NVMOE_ROUTER_SCORE_TOPK) {
-        if (p.g.activation == NVMOE_ACT_SOFTMAX) {
-            float smax = kNegInf;
-#pragma unroll
-            for (int j = 0; j < EPL; j++)
-                if (lane + 32u * j < E) smax = fmaxf(smax, val[j]);
-            smax = warp_max(smax);
-            float lo = 0.0f, hi = 0.0f;  // virtual lanes `lane` and `lane + 32` of a 64-wide group
-#pragma unroll
-            for (int j = 0; j < EPL; j++) {
-                if (lane + 32u * j < E) {
-                    val[j] = nvmoe_expf(__fsub_rn(val[j], smax));
-                    if (j & 1) hi = __fadd_rn(hi, val[j]); else lo = __fadd_rn(lo, val[j]);
-                }
-            }
-            const float sden = warp_butterfly_sum(__fadd_rn(lo, hi));
-#pragma unroll
-            for (int j = 0; j < EPL; j++) val[j] = __fdiv_rn(val[j], sden);
-        } else {
-#pragma unroll
-            for (int j = 0; j < EPL; j++)
-                val[j] = p.g.activation == NVMOE_ACT_SIGMOID ? nvmoe_sigmoidf(val[j]) : __fsqrt_rn(nvmoe_softplusf(val[j]));
-        }
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            const uint32_t e = lane + 32u * j;
-            score[j] = e < E ? __fadd_rn(val[j], read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
-        }
-    } else if (kind == NVMOE_ROUTER_TOPK_SOFTMAX) {
-#pragma unroll
-        for (int j = 0; j < EPL; j++) score[j] = val[j];
-    } else {
-        const bool sigmoid = p.g.activation == NVMOE_ACT_SIGMOID;
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            const uint32_t e = lane + 32u * j;
-            float v = val[j];
-            if (p.g.logit_softcap > 0.0f) v = __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, p.g.logit_softcap)), p.g.logit_softcap);
-            val[j] = v;
-            score[j] = e < E ? __fadd_rn(sigmoid ? nvmoe_sigmoidf(v) : v, read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
-        }
-    }
-
-    // ---- k rounds of arg-max: lane r keeps selection r ---------------------------------------
-    uint32_t taken = 0u, my_e = kUnboundSlot;
-    if (GROUPS) {
-        // a group's score is the sum of its two best; the experts of the groups outside the topk_group best count as taken
-        const uint32_t per = E / p.g.n_group, side = 32u / per;  // groups in a register slot of the warp
-        float my_group = kNegInf;
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            float first = lane + 32u * j < E && score[j] > kNegInf ? score[j] : kNegInf, second = kNegInf;
-            for (uint32_t o = 1u; o < per; o <<= 1) {
-                const float other_first = __shfl_xor_sync(kFull, first, o), other_second = __shfl_xor_sync(kFull, second, o);
-                second = fmaxf(fminf(first, other_first), fmaxf(second, other_second));
-                first = fmaxf(first, other_first);
-            }
-            const float group = __shfl_sync(kFull, per >= 2u ? __fadd_rn(first, second) : first, (lane % side) * per);
-            if (lane / side == (uint32_t)j) my_group = group;  // lane g keeps group g
-        }
-        uint32_t kept = 0u;
-        for (uint32_t round = 0; round < p.g.topk_group; round++) {
-            const bool open = lane < p.g.n_group && ((kept >> lane) & 1u) == 0u && my_group >= kNegInf;  // (not a NaN)
-            float s = open ? my_group : kNegInf;
-            uint32_t winner = open ? lane : kUnboundSlot;
-            warp_argmax(s, winner);
-            if (winner != kUnboundSlot) kept |= 1u << winner;
-        }
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            const uint32_t group = (uint32_t)j * side + lane / per;
-            if (group >= 32u || ((kept >> group) & 1u) == 0u) taken |= 1u << j;
-        }
-    }
-    float my_v = 0.0f;
-    bool missing = false;
-    for (uint32_t r = 0; r < k; r++) {
-        float best = kNegInf, best_v = 0.0f;
-        uint32_t best_e = kUnboundSlot;
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            const uint32_t e = lane + 32u * j;
-            if (e < E && ((taken >> j) & 1u) == 0u && better(score[j], e, best, best_e)) {
-                best = score[j];
-                best_e = e;
-                best_v = val[j];
-            }
-        }
-        float s = best;
-        uint32_t winner = best_e;
-        warp_argmax(s, winner);
-        if (winner == kUnboundSlot) {
-            missing = true;
-            break;
-        }
-        // the winner is the best candidate of the lane that owns it
-        const float winner_v = __shfl_sync(kFull, best_v, winner & 31u);
-        if (lane == (winner & 31u)) taken |= 1u << (winner >> 5);
-        if (lane == r) {
-            my_e = winner;
-            my_v = winner_v;
-        }
-    }
-    uint32_t* out = p.routes + (size_t)token * total_k;
-    if (missing) {
-        // no selectable score (NaN logits): fail closed instead of indexing out of bounds
-        if (lane == 0u) {
-            for (uint32_t r = 0; r < total_k; r++) out[r] = 0u;
-            raise_status(p.status, NVMOE_STATUS_ROUTE_NONFINITE);
-        }
-        return;
-    }
-
-    // ---- weights, in the summation orders the shaders fix ----------------------------------
-    float w = 0.0f;
-    if (kind == NVMOE_ROUTER_SCORE_TOPK) {
-        float den = 0.0f;
-        if (p.g.normalize_selected)
-            for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, my_v, r));
-        w = p.g.normalize_selected ? __fmul_rn(__fdiv_rn(my_v, den), p.g.routed_scale) : __fmul_rn(my_v, p.g.routed_scale);
-        if (lane >= k && lane < total_k) {
-            my_e = E + (lane - k);
-            w = p.g.always_weight;
-        }
-    } else {
-        const bool sigmoid = kind == NVMOE_ROUTER_TOPK_ROUTED && p.g.activation == NVMOE_ACT_SIGMOID;
-        const bool divide = kind == NVMOE_ROUTER_TOPK_SOFTMAX || p.g.normalize_selected || !sigmoid;
-        const float maximum = __shfl_sync(kFull, my_v, 0);
-        const float t = sigmoid ? nvmoe_sigmoidf(my_v) : nvmoe_expf(__fsub_rn(my_v, maximum));
-        float den = 0.0f;
-        for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, t, r));
-        w = divide ? __fdiv_rn(t, den) : t;
-    }
-
-    // ---- ascending expert id, pack, telemetry ----------------------------------------------------
-    uint32_t rank = 0u;
-    for (uint32_t q = 0; q < total_k; q++) {
-        const uint32_t other = __shfl_sync(kFull, my_e, q);
-        if (other < my_e) rank++;
-    }
-    if (lane < total_k) {
-        out[rank] = (nvmoe_f32_to_bf16(w) << 16) | my_e;
-        if (p.telemetry) atomicAdd(p.telemetry + my_e, 1u);
-    }
-    if (p.telemetry) {
-        for (uint32_t q = 0; q < total_k; q++) {
-            const uint32_t right = __shfl_sync(kFull, my_e, q);
-            if (lane < total_k && my_e < right) {
-                const uint32_t preceding = my_e * (2u * total_resources - my_e - 1u) / 2u;
-                atomicAdd(p.telemetry + total_resources + preceding + right - my_e - 1u, 1u);
-            }
-        }
-    }
+    const uint32_t token = blockIdx.x * 4u + (threadIdx.x >> 5);
+    if (token < p.tokens) route_token<EPL, GROUPS>(p, token);
 }
 
 // ---- router projection ----------------------------------------------------------------------
@@ -652,9 +442,18 @@ __global__ void __launch_bounds__(256, 1) router_linear_tiled_kernel(const uint1
 
 }  // namespace
 
+static uint32_t router_total_k(const RouterLaunch& p) {
+    return p.g.routed_k + (p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u);
+}
+
+bool router_is_small(const RouterLaunch& p) {
+    return p.g.routed_experts <= 128u && router_total_k(p) <= 32u && p.g.n_group == 0u && p.g.router_kind <= NVMOE_ROUTER_TOPK_ROUTED &&
+           !(p.g.router_kind == NVMOE_ROUTER_TOPK_ROUTED && !p.g.normalize_selected && p.g.activation != NVMOE_ACT_SIGMOID);
+}
+
 void launch_router(const RouterLaunch& p, cudaStream_t stream) {
     const uint32_t E = p.g.routed_experts;
-    const uint32_t total_k = p.g.routed_k + (p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u);
+    const uint32_t total_k = router_total_k(p);
     // the routed form's softmax over all experts (neither normalised over the selection nor sigmoid) sums in expert order
     const bool sums_all = p.g.router_kind == NVMOE_ROUTER_TOPK_ROUTED && !p.g.normalize_selected && p.g.activation != NVMOE_ACT_SIGMOID;
     const uint32_t per = p.g.n_group ? E / p.g.n_group : 0u;

@@ -11,7 +11,7 @@
 // experts keep source order (warp match + popcount of lower lanes, warps taken in order).
 // Route ids at or above the expert count cannot be produced by the routers here; they are placed
 // after every valid id in source order (the reference would order them by id).
-#include "common.cuh"
+#include "router_reg.cuh"
 
 namespace nvmoe {
 namespace {
@@ -602,8 +602,9 @@ __host__ __device__ inline size_t layer_schedule_rank_smem_bytes(uint32_t count,
     return ((warps * columns + 1u) / 2u + 7u * (columns + 1u) + 2u) * sizeof(uint32_t) + 2u * columns;
 }
 
-template <uint32_t CHUNKS>
-__global__ void __launch_bounds__(1024) layer_schedule_rank_kernel(LayerSchedule s) {
+// `before` runs once the table has been cleared: the wait for the kernel before this one, or that and the routing.
+template <uint32_t CHUNKS, class BeforeFn>
+__device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s, BeforeFn before) {
     extern __shared__ uint32_t smem_words[];
     const uint32_t count = s.tokens * s.K;
     const uint32_t E = s.num_experts;
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(1024) layer_schedule_rank_kernel(LayerSchedule
 
     for (uint32_t w = threadIdx.x; w < table_words; w += blockDim.x) smem_words[w] = 0u;
     if (threadIdx.x < 2u) totals[threadIdx.x] = 0u;
-    grid_dependency_sync();
+    before();
     // residency of every expert for both stages (bucket E is never kept)
     for (uint32_t i = threadIdx.x; i < 2u * C; i += blockDim.x) {
         const uint32_t stage = i / C, b = i % C;
@@ -768,6 +769,22 @@ __global__ void __launch_bounds__(1024) layer_schedule_rank_kernel(LayerSchedule
         }
         if (s.tiles[stage] && b == E) *s.tile_count[stage] = tile_base[stage][E];
     }
+}
+
+template <uint32_t CHUNKS>
+__global__ void __launch_bounds__(1024) layer_schedule_rank_kernel(LayerSchedule s) {
+    layer_schedule_rank_body<CHUNKS>(s, [] { grid_dependency_sync(); });
+}
+
+// Router and schedule of a handful of tokens in one block: a warp routes a token, the block barrier inside the schedule
+// stands where the next launch would. Each of the two is a few microseconds of latency, so is the hand-over between them.
+template <int EPL>
+__global__ void __launch_bounds__(1024) route_schedule_kernel(RouterLaunch router, LayerSchedule s) {
+    layer_schedule_rank_body<1u>(s, [&] {
+        grid_dependency_sync();
+        const uint32_t token = threadIdx.x >> 5;
+        if (token < router.tokens) route_token<EPL, false>(router, token);
+    });
 }
 
 // The same schedule for more routes than one block ranks well: 256 routes a block, in three launches. As above, one
@@ -1119,6 +1136,18 @@ bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, 
     const uint64_t count = (uint64_t)tokens * K;
     return wide_schedule_fits(count, num_experts, partitioned) || rank_schedule_fits(count, num_experts) ||
            three_sort_schedule_fits(count, num_experts);
+}
+
+// a warp of the one block per token, all routes in one pass
+bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts) {
+    const uint64_t count = (uint64_t)router.tokens * K;
+    return router.tokens <= 32u && router_is_small(router) && count <= 1024u && rank_schedule_fits(count, num_experts);
+}
+
+void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream) {
+    const uint32_t count = s.tokens * s.K, warps = s.tokens > (count + 31u) / 32u ? s.tokens : (count + 31u) / 32u;
+    launch_chained(router.g.routed_experts <= 32u ? route_schedule_kernel<1> : route_schedule_kernel<4>, dim3(1),
+                   dim3(warps <= 8u ? 256u : warps <= 16u ? 512u : 1024u), layer_schedule_rank_smem_bytes(count, s.num_experts), stream, router, s);
 }
 
 uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream) {
