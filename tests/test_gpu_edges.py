@@ -5,7 +5,7 @@ import pytest
 from nerve_b200 import synthetic
 from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, geometry_from_config
 from oracle import moe_oracle as mo
-from tests.helpers import assert_close
+from tests.helpers import assert_close, oracle_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -143,4 +143,31 @@ def test_group_limited_routing(device, experts, n_group, topk_group, k, activati
     plan.moe_route(tokens, device.resident_buffer_from(words), routes, device.resident_buffer_from(bias), None)
     want, _ = mo.route(mo.router_params_from(cfg), words, bias)
     np.testing.assert_array_equal(routes.read(np.uint32).reshape(want.shape), want)
+    plan.destroy()
+
+
+# the last batch that is routed and scheduled in one launch and the first that is not; fewer warps of routes than of
+# tokens and the other way round; one and four experts a lane; an expert count beyond it
+@pytest.mark.parametrize("name,experts,tokens", [("gpt-oss-20b", 32, 1), ("gpt-oss-20b", 33, 9), ("gpt-oss-20b", 128, 17),
+                                                 ("gpt-oss-20b", 16, 32), ("gpt-oss-20b", 16, 33), ("tiny", 8, 32),
+                                                 ("gpt-oss-20b", 129, 8)])
+def test_layer_routes_equal_the_router_node(device, name, experts, tokens):
+    cfg = synthetic.small_variant(synthetic.CONFIGS[name], 256, 256, experts)
+    case = synthetic.make_case(cfg, tokens, seed=7)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    rb = device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None
+    make = device.create_resident_buffer
+    out, routes, want = make(tokens * cfg.hidden * 2), make(tokens * cfg.total_k * 4), make(tokens * cfg.total_k * 4)
+    logits, counts, want_counts = make(tokens * ((experts + 1) // 2) * 4), make(plan.telemetry_words() * 4), make(plan.telemetry_words() * 4)
+    counts.fill(0)
+    want_counts.fill(0)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw, router_bias=rb, routes_out=routes, telemetry=counts)
+    plan.linear(tokens, hidden, logits, rw, rb)
+    plan.moe_route(tokens, logits, want, None, want_counts)
+    np.testing.assert_array_equal(routes.read(np.uint32), want.read(np.uint32))
+    np.testing.assert_array_equal(counts.read(np.uint32), want_counts.read(np.uint32))
+    assert_close(out.read(np.uint16).reshape(tokens, -1), oracle_layer(case)["output"])
+    assert plan.status() == 0
     plan.destroy()
