@@ -822,17 +822,12 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
                           const uint32_t* intermediates, const uint32_t* control, bool tensor) {
     const int set = gate_up ? 0 : 1;
     cudaStream_t st = p->device->stream;
-    launch_group_slots(routes, intermediates, control, es->ptrs.as<ExpertPtrs>(), p->experts, T, p->K, p->g.intermediate_size,
-                       p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), p->position[set].as<uint32_t>(),
-                       p->status.as<uint32_t>(), sort_scratch(p), st);
-    p->launches += (size_t)T * p->K <= 4096u ? 1u : 3u;
-    if (tensor) {
-        uint32_t* region = p->tile_list.as<uint32_t>() + set * tile_region_words(p);
-        const uint32_t rows = gate_up ? p->g.intermediate_size : p->g.hidden_size;
-        launch_build_tiles(p->offsets[set].as<uint32_t>(), p->experts, tc_token_tile_for(T, p->K, p->experts, rows, gate_up), region + 64,
-                           region, st);
-        p->launches++;
-    }
+    uint32_t* region = p->tile_list.as<uint32_t>() + set * tile_region_words(p);
+    const uint32_t rows = gate_up ? p->g.intermediate_size : p->g.hidden_size;
+    const TileOut tiles{tensor ? region + 64 : nullptr, region, tc_token_tile_for(T, p->K, p->experts, rows, gate_up)};
+    p->launches += launch_group_slots(routes, intermediates, control, es->ptrs.as<ExpertPtrs>(), p->experts, T, p->K,
+                                      p->g.intermediate_size, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(),
+                                      p->position[set].as<uint32_t>(), tiles, p->status.as<uint32_t>(), sort_scratch(p), st);
     return post_launch(p, gate_up ? "gate/up schedule" : "down schedule");
 }
 

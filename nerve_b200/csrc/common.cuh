@@ -123,9 +123,13 @@ void launch_route_compact(const uint32_t* routes, uint32_t* intermediates, const
 void launch_route_count(const uint32_t* routes, const uint32_t* slots, uint32_t slot_words,
                         uint32_t params_per_resource, uint32_t* control, uint32_t max_tokens, uint32_t K,
                         uint32_t tiles_per_route, cudaStream_t stream);
-// (expert, token tile) list of the tensor-core expert kernels from the expert offsets
-void launch_build_tiles(const uint32_t* expert_offsets, uint32_t num_experts, uint32_t n_tile, uint32_t* tiles,
-                        uint32_t* count, cudaStream_t stream);
+// (expert, token tile) list of the tensor-core expert kernels; the list holds routes / 16 + experts + 1 entries: enough for
+// any token tile size. list null: none
+struct TileOut {
+    uint32_t* list;
+    uint32_t* count;
+    uint32_t n_tile;
+};
 // Schedule of a whole layer call in one launch, or three for large T*K (layer_schedule_is_fused): control words,
 // compact list, owned count, and per expert stage [gate/up, down] the grouped routes, expert offsets
 // and (when tiles[stage] is set) the tile list. experts[stage] must already be resolved.
@@ -159,11 +163,12 @@ void launch_resolve_experts(const uint32_t* addresses, uint32_t address_words, c
                             uint8_t* derived_scales, size_t derived_matrix_bytes, ExpertPtrs* out, cudaStream_t stream);
 // groups the compact slots the expert shaders would visit by expert (stable), skipping what the
 // shaders skip; writes grouped_routes and expert_offsets and, if `position` is given, the inverse
-// position[route] = place in grouped_routes (0xffffffff for routes that were skipped)
-void launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, const uint32_t* control,
+// position[route] = place in grouped_routes (0xffffffff for routes that were skipped) and the tile list; returns its launches
+uint32_t launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, const uint32_t* control,
                         const ExpertPtrs* experts, uint32_t num_experts, uint32_t max_tokens, uint32_t K,
                         uint32_t intermediate_size, uint32_t* grouped_routes, uint32_t* expert_offsets,
-                        uint32_t* position, uint32_t* status, const SortScratch& scratch, cudaStream_t stream);
+                        uint32_t* position, const TileOut& tiles, uint32_t* status, const SortScratch& scratch,
+                        cudaStream_t stream);
 
 // expert-parallel dispatch (schedule.cu): routes grouped by the rank owning their expert, stable
 // in source order; send_index[i] = position of source route i (kUnboundSlot if dropped),

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(1024) compact_small_kernel(const uint32_t* rou
                                                             uint32_t max_tokens, uint32_t K, uint32_t I,
                                                             uint32_t tiles_per_route, uint32_t num_experts) {
     extern __shared__ uint32_t hist[];
+    grid_dependency_sync();
     compact_small_body(routes, intermediates, slots, slot_words, params, control, max_tokens, K, I, tiles_per_route,
                        num_experts, hist);
 }
@@ -384,6 +385,7 @@ __device__ void route_count_body(const uint32_t* routes, const uint32_t* slots, 
 __global__ void __launch_bounds__(1024) route_count_kernel(const uint32_t* routes, const uint32_t* slots,
                                                           uint32_t slot_words, uint32_t params, uint32_t* control,
                                                           uint32_t max_tokens, uint32_t K, uint32_t tiles_per_route) {
+    grid_dependency_sync();
     route_count_body(routes, slots, slot_words, params, control, max_tokens, K, tiles_per_route);
 }
 
@@ -482,13 +484,6 @@ __device__ void group_small_body(SlotKey key, const uint32_t* control, uint32_t 
     });
 }
 
-__global__ void __launch_bounds__(1024) group_small_kernel(SlotKey key, const uint32_t* control,
-                                                          uint32_t max_tokens, uint32_t* grouped,
-                                                          uint32_t* expert_offsets, uint32_t* position) {
-    extern __shared__ uint32_t hist[];
-    group_small_body(key, control, max_tokens, grouped, expert_offsets, position, hist);
-}
-
 // (expert, token tile) pairs in expert order for the tensor-core expert kernels: entry =
 // (expert << 16) | token tile within the expert; every thread of one block calls it
 __device__ void build_tiles_body(const uint32_t* expert_offsets, uint32_t num_experts, uint32_t n_tile,
@@ -533,7 +528,21 @@ __device__ void build_tiles_body(const uint32_t* expert_offsets, uint32_t num_ex
 
 __global__ void __launch_bounds__(1024) build_tiles_kernel(const uint32_t* expert_offsets, uint32_t num_experts,
                                                           uint32_t n_tile, uint32_t* tiles, uint32_t* count) {
+    grid_dependency_sync();
     build_tiles_body(expert_offsets, num_experts, n_tile, tiles, count);
+}
+
+// one block groups the slots of a stage and, for the tensor path, lists its tiles
+__global__ void __launch_bounds__(1024) group_small_kernel(SlotKey key, const uint32_t* control,
+                                                          uint32_t max_tokens, uint32_t* grouped,
+                                                          uint32_t* expert_offsets, uint32_t* position, TileOut tiles) {
+    extern __shared__ uint32_t hist[];
+    grid_dependency_sync();
+    group_small_body(key, control, max_tokens, grouped, expert_offsets, position, hist);
+    if (tiles.list) {
+        __syncthreads();
+        build_tiles_body(expert_offsets, key.num_experts, tiles.n_tile, tiles.list, tiles.count);
+    }
 }
 
 // The whole schedule of one layer call in one block (T*K small): the control words the host of the
@@ -628,9 +637,10 @@ __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s,
     if (threadIdx.x < 2u) totals[threadIdx.x] = 0u;
     before();
     // residency of every expert for both stages (bucket E is never kept)
-    for (uint32_t i = threadIdx.x; i < 2u * C; i += blockDim.x) {
-        const uint32_t stage = i / C, b = i % C;
-        kept[i] = (b < E && s.experts[stage][b].w[0] != nullptr) ? 1u : 0u;
+    // (the two stages are unrolled throughout: pointers picked by a run-time stage would live in local memory)
+    for (uint32_t b = threadIdx.x; b < C; b += blockDim.x) {
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++) kept[stage * C + b] = (b < E && s.experts[stage][b].w[0] != nullptr) ? 1u : 0u;
     }
     // per route: bucket (16 bits) | routes of the same bucket before it in its warp (8) | owned routes before it (8)
     uint32_t state[CHUNKS];
@@ -697,39 +707,23 @@ __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s,
     if (warp < 5u) {
         const uint32_t stage = warp == 0u ? 0u : (warp - 1u) & 1u;
         const bool tiles = warp >= 3u;
-        uint32_t* out = warp == 0u ? base_all : tiles ? tile_base[stage] : gbase[stage];
         const uint32_t* counts = stage == 1u ? hist_down : hist;
-        uint32_t carry = 0u;
-        for (uint32_t b0 = 0; b0 < B; b0 += 32u) {
-            const uint32_t b = b0 + lane;
-            uint32_t v = b < B ? counts[b] : 0u;
-            if (warp != 0u && b < B) {
-                v = kept[stage * C + b] ? v : 0u;
-                if (tiles) v = (v + s.n_tile[stage] - 1u) / s.n_tile[stage];
-            }
-            uint32_t incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += n;
-            }
-            if (b < B) out[b] = carry + incl - v;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0u) out[B] = carry;
+        const uint32_t n_tile = stage == 0u ? s.n_tile[0] : s.n_tile[1];
+        warp_exclusive_scan(B, base_all + warp * (C + 1u), [&](uint32_t b) {  // (the arrays lie in the warps' order)
+            const uint32_t v = counts[b];
+            if (warp == 0u) return v;
+            if (!kept[stage * C + b]) return 0u;
+            return tiles ? (v + n_tile - 1u) / n_tile : v;
+        });
     }
     __syncthreads();
-    if (threadIdx.x < 14u) {
-        const uint32_t stage = threadIdx.x / 7u, j = threadIdx.x % 7u;
-        const uint32_t visited = stage == 0u ? listed_total : down_total;
-        uint32_t value = 1u;  // word 6; word 5 of a partitioned call
-        if (j == 0u) value = s.tokens;
-        if (j == 1u) value = s.expert_start;
-        if (j == 2u) value = s.expert_count;
-        if (j == 3u) value = visited;
-        if (j == 4u) value = (partitioned ? visited : s.K) * s.tiles_per_route[stage];
-        if (j == 5u && !partitioned) value = s.tokens;
-        s.control[stage][j] = value;
+#pragma unroll
+    for (uint32_t stage = 0; stage < 2u; stage++) {
+        const uint32_t j = threadIdx.x, visited = stage == 0u ? listed_total : down_total;
+        if (j < 7u)
+            s.control[stage][j] = j == 0u ? s.tokens : j == 1u ? s.expert_start : j == 2u ? s.expert_count : j == 3u ? visited
+                                  : j == 4u ? (partitioned ? visited : s.K) * s.tiles_per_route[stage]
+                                  : j == 5u && !partitioned ? s.tokens : 1u;
     }
     // a down count beyond the compact list makes the down stage read entries that were never written
     if (threadIdx.x == 0u && down_total > listed_total) raise_status(s.status, NVMOE_STATUS_ROUTE_OUT_OF_RANGE);
@@ -746,6 +740,7 @@ __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s,
             at = partitioned ? table[(size_t)(i >> 5) * C + B] + (state[c] >> 24) : base_all[b] + rank;
             s.intermediates[(size_t)(at / s.K) * frame_words + data_words + at % s.K] = i;
         }
+#pragma unroll
         for (uint32_t stage = 0; stage < 2u; stage++) {
             uint32_t place = kUnboundSlot;
             if (listed && (stage == 0u || at < down_total)) {
@@ -759,15 +754,17 @@ __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s,
             if (s.position[stage]) s.position[stage][i] = place;
         }
     }
-    for (uint32_t i = threadIdx.x; i < 2u * B; i += blockDim.x) {
-        const uint32_t stage = i / B, b = i % B;
-        // bucket E is never kept, so gbase[stage][E] is already the total the offsets end with
-        s.offsets[stage][b] = gbase[stage][b];
-        if (s.tiles[stage] && b < E) {
-            const uint32_t first = tile_base[stage][b], n = tile_base[stage][b + 1u] - first;
-            for (uint32_t j = 0; j < n; j++) s.tiles[stage][first + j] = (b << 16) | j;
+#pragma unroll
+    for (uint32_t stage = 0; stage < 2u; stage++) {
+        for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) {
+            // bucket E is never kept, so gbase[stage][E] is already the total the offsets end with
+            s.offsets[stage][b] = gbase[stage][b];
+            if (s.tiles[stage] && b < E) {
+                const uint32_t first = tile_base[stage][b], n = tile_base[stage][b + 1u] - first;
+                for (uint32_t j = 0; j < n; j++) s.tiles[stage][first + j] = (b << 16) | j;
+            }
+            if (s.tiles[stage] && b == E) *s.tile_count[stage] = tile_base[stage][E];
         }
-        if (s.tiles[stage] && b == E) *s.tile_count[stage] = tile_base[stage][E];
     }
 }
 
@@ -1101,9 +1098,8 @@ void launch_route_compact(const uint32_t* routes, uint32_t* intermediates, const
     const uint32_t buckets = num_experts + 1u;
     if (count <= kSmallSortLimit) {
         uint32_t threads = count <= 256u ? 256u : 1024u;
-        compact_small_kernel<<<1, threads, (buckets + 1u) * sizeof(uint32_t), stream>>>(
-            routes, intermediates, slots, slot_words, params_per_resource, control, max_tokens, K,
-            intermediate_size, tiles_per_route, num_experts);
+        launch_chained(compact_small_kernel, dim3(1), dim3(threads), (buckets + 1u) * sizeof(uint32_t), stream, routes, intermediates, slots,
+                       slot_words, params_per_resource, control, max_tokens, K, intermediate_size, tiles_per_route, num_experts);
         return;
     }
     const uint32_t blocks = (count + kSortChunk - 1u) / kSortChunk;
@@ -1174,17 +1170,11 @@ uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratc
     return 1u;
 }
 
-void launch_build_tiles(const uint32_t* expert_offsets, uint32_t num_experts, uint32_t n_tile, uint32_t* tiles,
-                        uint32_t* count, cudaStream_t stream) {
-    // tiles holds routes / 16 + experts + 1 entries: enough for any token tile size
-    build_tiles_kernel<<<1, 1024, 0, stream>>>(expert_offsets, num_experts, n_tile, tiles, count);
-}
-
 void launch_route_count(const uint32_t* routes, const uint32_t* slots, uint32_t slot_words,
                         uint32_t params_per_resource, uint32_t* control, uint32_t max_tokens, uint32_t K,
                         uint32_t tiles_per_route, cudaStream_t stream) {
-    route_count_kernel<<<1, 1024, 0, stream>>>(routes, slots, slot_words, params_per_resource, control,
-                                               max_tokens, K, tiles_per_route);
+    launch_chained(route_count_kernel, dim3(1), dim3(1024), 0, stream, routes, slots, slot_words, params_per_resource, control, max_tokens, K,
+                   tiles_per_route);
 }
 
 void launch_resolve_experts(const uint32_t* addresses, uint32_t address_words, const uint32_t* slots,
@@ -1196,18 +1186,19 @@ void launch_resolve_experts(const uint32_t* addresses, uint32_t address_words, c
         whole_blocks_only, derived_scales, derived_matrix_bytes, out);
 }
 
-void launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, const uint32_t* control,
+uint32_t launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, const uint32_t* control,
                         const ExpertPtrs* experts, uint32_t num_experts, uint32_t max_tokens, uint32_t K,
                         uint32_t intermediate_size, uint32_t* grouped_routes, uint32_t* expert_offsets,
-                        uint32_t* position, uint32_t* status, const SortScratch& scratch, cudaStream_t stream) {
+                        uint32_t* position, const TileOut& tiles, uint32_t* status, const SortScratch& scratch,
+                        cudaStream_t stream) {
     const uint32_t data_words = K * (intermediate_size / 2u);
     SlotKey key{routes, intermediates, experts, status, num_experts, K, data_words + K, data_words, 0u};
     const uint32_t count = max_tokens * K;
     if (count <= kSmallSortLimit) {
         uint32_t threads = count <= 256u ? 256u : 1024u;
-        group_small_kernel<<<1, threads, (num_experts + 1u) * sizeof(uint32_t), stream>>>(
-            key, control, max_tokens, grouped_routes, expert_offsets, position);
-        return;
+        launch_chained(group_small_kernel, dim3(1), dim3(threads), (num_experts + 1u) * sizeof(uint32_t), stream, key, control, max_tokens,
+                       grouped_routes, expert_offsets, position, tiles);
+        return 1u;
     }
     const uint32_t blocks = (count + kSortChunk - 1u) / kSortChunk;
     group_hist_kernel<<<blocks, 256, num_experts * sizeof(uint32_t), stream>>>(key, control, max_tokens,
@@ -1215,6 +1206,9 @@ void launch_group_slots(const uint32_t* routes, const uint32_t* intermediates, c
     launch_phase_scan(scratch, blocks, num_experts, stream);
     group_scatter_kernel<<<blocks, 256, (num_experts + 1u) * sizeof(uint32_t), stream>>>(
         key, control, max_tokens, grouped_routes, expert_offsets, scratch.block_hist, scratch.bucket_totals, position);
+    if (!tiles.list) return 3u;
+    launch_chained(build_tiles_kernel, dim3(1), dim3(1024), 0, stream, expert_offsets, num_experts, tiles.n_tile, tiles.list, tiles.count);
+    return 4u;
 }
 
 }  // namespace nvmoe
