@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, geometry_from_config
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, ResidentBuffer, geometry_from_config
 from oracle import moe_oracle as mo
 from tests.helpers import assert_close, oracle_layer
 
@@ -169,5 +169,27 @@ def test_layer_routes_equal_the_router_node(device, name, experts, tokens):
     np.testing.assert_array_equal(routes.read(np.uint32), want.read(np.uint32))
     np.testing.assert_array_equal(counts.read(np.uint32), want_counts.read(np.uint32))
     assert_close(out.read(np.uint16).reshape(tokens, -1), oracle_layer(case)["output"])
+    assert plan.status() == 0
+    plan.destroy()
+
+
+def test_layer_of_rows_off_the_16_byte_grid(device):
+    """Hidden rows that the token-wise quantisation cannot read take the general one: the same result."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 256, 320, 16)
+    tokens = 40
+    case = synthetic.make_case(cfg, tokens, seed=11)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    rw, rb = device.resident_buffer_from(case.router_w), device.resident_buffer_from(case.router_bias)
+    room = device.create_resident_buffer(case.hidden.nbytes + 16)
+    results = []
+    for shift in (0, 8):
+        room.write_bytes(case.hidden, shift)
+        hidden = ResidentBuffer.wrap(device, room.device_address() + shift, case.hidden.nbytes)
+        out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+        plan.layer(tokens, bank, hidden, out, router_weights=rw, router_bias=rb)
+        results.append(out.read(np.uint16))
+        hidden.destroy()
+    np.testing.assert_array_equal(results[0], results[1])
     assert plan.status() == 0
     plan.destroy()
