@@ -1210,6 +1210,9 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     NVMOE_TRY(check_buffer(p, output, (size_t)T * rows * 2u, "output"));
     NVMOE_TRY(check_buffer(p, weights, (size_t)rows * (cols / 2u), "weights"));
     NVMOE_TRY(check_buffer(p, scales, (size_t)rows * (cols / 32u), "weight scales"));
+    // what the expert kernels ask of a resident record: they read rows with 16-byte loads and TMA boxes
+    if (((reinterpret_cast<uintptr_t>(weights->ptr) | reinterpret_cast<uintptr_t>(scales->ptr)) & 31u) != 0u)
+        return fail(d, NVMOE_ERR_INVALID_ARGUMENT, "dense linear: weights and scales must start on 32-byte boundaries");
     NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
     nvmoe_plan::DenseLinear* dl = nullptr;
     for (auto& entry : p->dense)

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, ResidentBuffer, geometry_from_config
+from nerve_b200.backend import CudaComputeDevice, CudaError, ExpertBank, MoePlan, ResidentBuffer, geometry_from_config
 from oracle import moe_oracle as mo
 from tests.helpers import assert_close, oracle_layer
 
@@ -192,4 +192,27 @@ def test_layer_of_rows_off_the_16_byte_grid(device):
         hidden.destroy()
     np.testing.assert_array_equal(results[0], results[1])
     assert plan.status() == 0
+    plan.destroy()
+
+
+@pytest.mark.parametrize("path", [1, 2])
+def test_dense_linear_refuses_matrices_off_the_32_byte_grid(device, path):
+    rows, cols, tokens = 128, 256, 5
+    rng = np.random.default_rng(3)
+    plan = plan_of(device)
+    plan.set_expert_path(path)
+    x = bf16(rng.standard_normal((tokens, cols)))
+    w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(121, 128, (rows, cols // 32), dtype=np.uint8)
+    xb, ob = device.resident_buffer_from(x), device.create_resident_buffer(tokens * rows * 2)
+    wroom, sroom = device.create_resident_buffer(w.nbytes + 32), device.create_resident_buffer(s.nbytes + 32)
+    wroom.write_bytes(w), sroom.write_bytes(s)
+
+    def at(room, shift, array):
+        return ResidentBuffer.wrap(device, room.device_address() + shift, array.nbytes)
+
+    for weights, scales in ((at(wroom, 16, w), at(sroom, 0, s)), (at(wroom, 0, w), at(sroom, 4, s))):
+        with pytest.raises(CudaError):
+            plan.dense_linear(tokens, xb, ob, weights, scales, rows, cols)
+    plan.dense_linear(tokens, xb, ob, at(wroom, 0, w), at(sroom, 0, s), rows, cols)
+    assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
     plan.destroy()
