@@ -346,7 +346,8 @@ int nvmoe_residual_add(nvmoe_plan* plan, uint32_t rows, uint32_t element_count, 
  * bf16 or block-scaled FP8); this one computes what the MoE node computes for a resource every token selects
  * with weight one (independent_sparse_moe_down_batch1_mxfp4.comp.template:507-610): activations quantised
  * to E4M3 per geometry.act_block, f32 accumulation, one bf16 rounding, on the same kernels. Weights and scales
- * start on 32-byte boundaries, as a resident expert record does. */
+ * start on 32-byte boundaries, as a resident expert record does. Nothing of them is kept from one call to the next:
+ * a matrix may be rewritten in place between calls by any means and needs no mark. */
 int nvmoe_dense_linear(nvmoe_plan* plan, uint32_t batch_width, const nvmoe_buffer* input, nvmoe_buffer* output,
                        const nvmoe_buffer* weights, const nvmoe_buffer* scales, uint32_t rows, uint32_t cols);
 

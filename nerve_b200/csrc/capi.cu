@@ -149,21 +149,13 @@ struct nvmoe_plan {
     uint32_t launches = 0;
     long long wait_cycles = 4000000000ll;  // limit of the bounded in-kernel waits of the tensor path (about 2 s)
     uint32_t debug_flags = 0;
-    // dense linears run as one always-selected resource of a plan of their own shape (nvmoe_dense_linear); the
-    // matrices of one shape share that plan's scratch and have an address table each, so that a block whose gate and
-    // up projections have the same shape resolves each of them once and not on every call
-    struct DenseMatrix {
-        nvmoe_buffer* addresses = nullptr;
-        const void* weights = nullptr;
-        const void* scales = nullptr;
-        uint64_t weights_uid = 0, scales_uid = 0, weights_version = 0, scales_version = 0, last_use = 0;
-    };
+    // dense linears run as one always-selected resource of a plan of their own shape (nvmoe_dense_linear); whatever hangs
+    // on a matrix (`set`: pointers, re-tiled scales, tensor map) is made anew by every call, nothing of it is kept
     struct DenseLinear {
         uint32_t rows = 0, cols = 0;
         nvmoe_plan* plan = nullptr;
-        nvmoe_buffer* slots = nullptr;
         DeviceArray unit_routes;
-        std::vector<DenseMatrix> matrices;  // at most kMaxExpertSets, least recently used replaced
+        ExpertSet set;
     };
     std::vector<DenseLinear> dense;
 };
@@ -553,8 +545,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
     cudaStreamSynchronize(p->device->stream);
     for (auto& dl : p->dense) {
         nvmoe_plan_destroy(dl.plan);
-        for (auto& matrix : dl.matrices) nvmoe_buffer_destroy(matrix.addresses);
-        nvmoe_buffer_destroy(dl.slots);
+        dl.set.release();
         dl.unit_routes.release();
     }
     for (auto& stage_sets : p->sets)
@@ -1227,10 +1218,10 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         g.max_tokens = p->g.max_tokens;
         NVMOE_TRY(nvmoe_plan_create(d, &g, &fresh.plan));
         fresh.plan->expert_path = p->expert_path;
-        int rc = nvmoe_buffer_create(d, 8u, &fresh.slots);
-        const uint32_t slot_words[2] = {0u, 1u};
-        if (rc == NVMOE_OK) rc = nvmoe_buffer_write(fresh.slots, 0, slot_words, 8u);
-        if (rc == NVMOE_OK && fresh.unit_routes.ensure((size_t)g.max_tokens * 4u) != cudaSuccess)
+        int rc = NVMOE_OK;
+        const bool tensor_shape = tc_shape_supported(g);
+        if (fresh.unit_routes.ensure((size_t)g.max_tokens * 4u) != cudaSuccess || fresh.set.ptrs.ensure(sizeof(ExpertPtrs)) != cudaSuccess ||
+            (tensor_shape && (fresh.set.derived.ensure(tc_derived_scale_bytes(rows, cols)) != cudaSuccess || fresh.set.tmaps.ensure(128u) != cudaSuccess)))
             rc = fail(d, NVMOE_ERR_OUT_OF_MEMORY, "dense linear: out of device memory");
         if (rc == NVMOE_OK) {
             std::vector<uint32_t> ones(g.max_tokens, 0x3f80u << 16);  // weight 1.0, resource 0
@@ -1239,7 +1230,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         }
         if (rc != NVMOE_OK) {
             nvmoe_plan_destroy(fresh.plan);
-            nvmoe_buffer_destroy(fresh.slots);
+            fresh.set.release();
             fresh.unit_routes.release();
             return rc;
         }
@@ -1249,44 +1240,26 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     nvmoe_plan* sub = dl->plan;
     sub->expert_path = p->expert_path;
     sub->wait_cycles = p->wait_cycles;
-    nvmoe_plan::DenseMatrix* m = nullptr;
-    for (auto& entry : dl->matrices)
-        if (entry.weights == weights->ptr && entry.scales == scales->ptr) m = &entry;
-    if (!m) {
-        if (dl->matrices.size() < kMaxExpertSets) {
-            nvmoe_plan::DenseMatrix fresh;
-            NVMOE_TRY(nvmoe_buffer_create(d, 64u, &fresh.addresses));
-            dl->matrices.push_back(fresh);
-            m = &dl->matrices.back();
-        } else {
-            m = &dl->matrices[0];
-            for (auto& entry : dl->matrices)
-                if (entry.last_use < m->last_use) m = &entry;
-        }
-    }
-    m->last_use = ++sub->use_clock;
-    if (m->weights != weights->ptr || m->scales != scales->ptr || m->weights_uid != weights->uid || m->scales_uid != scales->uid ||
-        m->weights_version != weights->version || m->scales_version != scales->version) {
-        // the two address records of the one resource: {address, byte count, generation, resident, representation}; the
-        // generation keys the re-tiled scales, so no two contents of one scale address may share it
-        const uint64_t generation = ++sub->use_clock;
-        uint64_t records[8] = {(uint64_t)(uintptr_t)weights->ptr, (uint64_t)rows * (cols / 2u), generation, 1u,
-                               (uint64_t)(uintptr_t)scales->ptr,  (uint64_t)rows * (cols / 32u), generation, 1u};
-        NVMOE_TRY(nvmoe_buffer_write(m->addresses, 0, records, sizeof records));
-        m->weights = weights->ptr;
-        m->scales = scales->ptr;
-        m->weights_uid = weights->uid;
-        m->scales_uid = scales->uid;
-        m->weights_version = weights->version;
-        m->scales_version = scales->version;
-    }
     cudaStream_t st = d->stream;
     const bool tensor = use_tensor_path(sub);
-    ExpertSet* es = nullptr;
-    NVMOE_TRY(prepare_expert_set(sub, false, m->addresses, dl->slots, tensor, &es));
     uint32_t* region = sub->tile_list.as<uint32_t>() + tile_region_words(sub);
-    launch_dense_schedule(T, tc_token_tile_for(T, 1u, 1u, rows, false), sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(),
-                          sub->position[1].as<uint32_t>(), tensor ? region + 64 : nullptr, tensor ? region : nullptr, st);
+    DensePrepare dp{};
+    dp.weights = (const uint8_t*)weights->ptr;
+    dp.scales = (const uint8_t*)scales->ptr;
+    dp.out_rows = rows;
+    dp.cols = cols;
+    dp.tokens = T;
+    dp.grouped = sub->grouped[1].as<uint32_t>();
+    dp.offsets = sub->offsets[1].as<uint32_t>();
+    dp.position = sub->position[1].as<uint32_t>();
+    dp.ptrs = dl->set.ptrs.as<ExpertPtrs>();
+    if (tensor) {
+        dp.tiles = TileOut{region + 64, region, tc_token_tile_for(T, 1u, 1u, rows, false)};
+        dp.derived = dl->set.derived.as<uint8_t>();
+        dp.map_template = sub->tma[1] ? sub->tmap_templates.as<uint8_t>() + 256 : nullptr;
+        dp.map = dl->set.tmaps.as<uint8_t>();
+    }
+    launch_dense_prepare(dp, st);
     sub->launches++;
     NVMOE_TRY(post_launch(sub, "dense linear schedule"));
     if (tensor) {
@@ -1305,7 +1278,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     call.T = T;
     call.routes = dl->unit_routes.as<uint32_t>();
     call.outputs = (uint16_t*)output->ptr;
-    call.prepared = es;
+    call.prepared = &dl->set;
     call.scheduled = true;
     NVMOE_TRY(run_experts(sub, call));
     p->launches += sub->launches;

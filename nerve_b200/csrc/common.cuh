@@ -259,10 +259,6 @@ void launch_preselect_table(const uint32_t* token_ids, const uint32_t* table, ui
                             cudaStream_t stream);
 void launch_route_preselected(const uint32_t* logits, const uint32_t* selections, uint32_t tokens, uint32_t* routes, uint32_t* status,
                               const nvmoe_geometry& g, cudaStream_t stream);
-// every row a route of expert 0 in row order: grouped list, offsets [0, rows], inverse, (expert, token tile) list
-void launch_dense_schedule(uint32_t rows, uint32_t n_tile, uint32_t* grouped, uint32_t* offsets, uint32_t* position, uint32_t* tiles,
-                           uint32_t* tile_count, cudaStream_t stream);
-
 // reduce.cu: the same combine with route (t, r) read from row gather[t * K + r] of `rows` (all-ones = a row of
 // zeros); false when the shape needs the plain form (hidden not a multiple of 8, unaligned buffers)
 bool launch_reduce_gather(const uint16_t* rows, const uint32_t* gather, uint16_t* output, uint32_t tokens, uint32_t K,

@@ -870,6 +870,60 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
     tensormap_publish(maps + (size_t)blockIdx.x * 128u, sm);
 }
 
+// The same for the one matrix of a dense linear, whose addresses are the call's own: nothing about the matrix is kept
+// between calls, so that scales rewritten in place by any means are what the next call reads. A block re-tiles 128 rows
+// x 8 K blocks, a thread 4 rows of one K block: 32 neighbouring bytes of a scale row per 8 threads in, one 16-byte
+// store out. The last block writes the pointers and the tensor map. Bound by the latency of one load and one store:
+// the 458 KB of a 2048 x 7168 matrix are far below what the launch takes anyway.
+constexpr uint32_t kDenseKBlocks = 8u;
+__global__ void __launch_bounds__(256) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
+    __shared__ __align__(128) unsigned char sm[128];
+    grid_dependency_sync();
+    const uint32_t tile_total = p.tiles.list ? (p.tokens + p.tiles.n_tile - 1u) / p.tiles.n_tile : 0u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.tokens; i += gridDim.x * blockDim.x) {
+        p.grouped[i] = i;
+        p.position[i] = i;
+        if (i < tile_total) p.tiles.list[i] = i;  // (expert 0 << 16) | token tile
+    }
+    if (blockIdx.x < retile_blocks) {
+        const uint32_t k_groups = (k_blocks + kDenseKBlocks - 1u) / kDenseKBlocks;
+        const uint32_t m_tile = blockIdx.x / k_groups, row_bytes = p.cols / 32u;
+        const uint32_t kb = blockIdx.x % k_groups * kDenseKBlocks + threadIdx.x % kDenseKBlocks, q = threadIdx.x / kDenseKBlocks;
+        if (kb < k_blocks) {
+            uint32_t word[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) {
+                const uint32_t row = m_tile * kBlockM + q + 32u * j;
+                const uint8_t* in = p.scales + (size_t)row * row_bytes + kb * 4u;
+                word[j] = 0x7f7f7f7fu;
+                if (row < p.out_rows && row_bytes % 4u == 0u) {
+                    word[j] = __ldg(reinterpret_cast<const uint32_t*>(in));
+                } else if (row < p.out_rows) {
+                    word[j] = 0u;
+#pragma unroll
+                    for (uint32_t b = 0; b < 4u; b++) word[j] |= (uint32_t)(kb * 4u + b < row_bytes ? __ldg(in + b) : 127u) << (8u * b);
+                }
+            }
+            *reinterpret_cast<uint4*>(p.derived + ((size_t)m_tile * k_blocks + kb) * kScaleBlockBytes + q * 16u) =
+                make_uint4(word[0], word[1], word[2], word[3]);
+        }
+    }
+    if (blockIdx.x != gridDim.x - 1u) return;
+    if (threadIdx.x == 0u) {
+        p.offsets[0] = 0u;
+        p.offsets[1] = p.tokens;
+        if (p.tiles.count) *p.tiles.count = tile_total;
+        *p.ptrs = ExpertPtrs{{p.weights, nullptr}, {p.scales, nullptr}, {p.derived, nullptr}, {0u, 0u}, kFormatCompact, 0u};
+    }
+    if (p.map_template != nullptr && threadIdx.x < 32u) {
+        reinterpret_cast<uint32_t*>(sm)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t*>(p.map_template) + threadIdx.x);
+        __syncwarp();
+        if (threadIdx.x == 0u) tensormap_replace_address(sm, p.weights);
+        __syncwarp();
+        tensormap_publish(p.map, sm);
+    }
+}
+
 int g_sm_count[16] = {0};
 
 template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR>
@@ -1004,6 +1058,13 @@ void launch_derive_scales_tc(const ExpertLaunch& p, bool gate_up, cudaStream_t s
                                                                                       matrices, rows, cols);
     const uint32_t count = p.work.num_experts * matrices;
     commit_stamps_kernel<<<(count + 127u) / 128u, 128, 0, stream>>>(p.work.experts, p.scale_stamps, matrices, count);
+}
+
+void launch_dense_prepare(const DensePrepare& p, cudaStream_t stream) {
+    const uint32_t m_tiles = (p.out_rows + kBlockM - 1u) / kBlockM, k_blocks = (p.cols + kBlockK - 1u) / kBlockK;
+    const uint32_t retile = p.derived ? m_tiles * ((k_blocks + kDenseKBlocks - 1u) / kDenseKBlocks) : 0u;
+    const uint32_t schedule = (p.tokens + 255u) / 256u;
+    launch_chained(dense_prepare_kernel, dim3((retile > schedule ? retile : schedule) + 1u), dim3(256), 0, stream, p, k_blocks, retile);
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

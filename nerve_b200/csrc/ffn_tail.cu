@@ -263,25 +263,6 @@ __global__ void __launch_bounds__(128) route_preselected_kernel(const uint32_t* 
     }
 }
 
-// Identity schedule of a dense linear run as one always-selected resource: every row is a route of
-// expert 0 in row order, the (expert, token tile) list covers the rows.
-__global__ void dense_schedule_kernel(uint32_t rows, uint32_t n_tile, uint32_t* grouped, uint32_t* offsets, uint32_t* position,
-                                      uint32_t* tiles, uint32_t* tile_count) {
-    grid_dependency_sync();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < rows) {
-        grouped[i] = i;
-        position[i] = i;
-    }
-    const uint32_t tile_total = (rows + n_tile - 1u) / n_tile;
-    if (tiles && i < tile_total) tiles[i] = i;  // (expert 0 << 16) | token tile
-    if (i == 0u) {
-        offsets[0] = 0u;
-        offsets[1] = rows;
-        if (tile_count) *tile_count = tile_total;
-    }
-}
-
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
 
 }  // namespace
@@ -327,12 +308,6 @@ void launch_preselect_table(const uint32_t* token_ids, const uint32_t* table, ui
 void launch_route_preselected(const uint32_t* logits, const uint32_t* selections, uint32_t tokens, uint32_t* routes, uint32_t* status,
                               const nvmoe_geometry& g, cudaStream_t stream) {
     launch_chained(route_preselected_kernel, dim3((tokens + 3u) / 4u), dim3(128), 0, stream, logits, selections, tokens, routes, status, g);
-}
-
-void launch_dense_schedule(uint32_t rows, uint32_t n_tile, uint32_t* grouped, uint32_t* offsets, uint32_t* position, uint32_t* tiles,
-                           uint32_t* tile_count, cudaStream_t stream) {
-    launch_chained(dense_schedule_kernel, dim3((rows + 255u) / 256u), dim3(256), 0, stream, rows, n_tile, grouped, offsets, position,
-                   tiles, tile_count);
 }
 
 }  // namespace nvmoe

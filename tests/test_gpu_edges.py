@@ -216,3 +216,29 @@ def test_dense_linear_refuses_matrices_off_the_32_byte_grid(device, path):
     plan.dense_linear(tokens, xb, ob, at(wroom, 0, w), at(sroom, 0, s), rows, cols)
     assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
     plan.destroy()
+
+
+@pytest.mark.parametrize("path", [1, 2])
+@pytest.mark.parametrize("handles", ["kept", "fresh"])
+def test_dense_scales_rewritten_behind_wrapped_handles(device, path, handles):
+    """Two matrices of one shape in turn, their memory the caller's own: codes and scales are refilled in place, without
+    a word to the library, through the handles that were used before or through new ones. Every call reads what is there."""
+    rows, cols, tokens = 160, 352, 9
+    rng = np.random.default_rng(17)
+    plan = plan_of(device)
+    plan.set_expert_path(path)
+    x = bf16(rng.standard_normal((tokens, cols)))
+    xb, ob = device.resident_buffer_from(x), device.create_resident_buffer(tokens * rows * 2)
+    rooms = [[device.create_resident_buffer(rows * cols // 2), device.create_resident_buffer(rows * cols // 32)] for _ in range(2)]
+
+    def wrapped(i):
+        return [ResidentBuffer.wrap(device, room.device_address(), room.byte_capacity) for room in rooms[i]]
+
+    kept = [wrapped(0), wrapped(1)]
+    for which in (0, 1, 0, 1, 1, 0, 0):
+        w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(118, 128, (rows, cols // 32), dtype=np.uint8)
+        rooms[which][0].write_bytes(w), rooms[which][1].write_bytes(s)
+        plan.dense_linear(tokens, xb, ob, *(kept[which] if handles == "kept" else wrapped(which)), rows, cols)
+        assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
+    assert plan.status() == 0
+    plan.destroy()
