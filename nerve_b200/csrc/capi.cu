@@ -826,7 +826,9 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
 // with E8M0 scales for the tensor path (after the stage has been scheduled), token- or route-ordered
 // rows with f32 scales for the CUDA-core path. `source` is the bf16 hidden matrix (gate/up) or the
 // intermediates frames (down). `whole_call`: the stage's position table covers every route of the T tokens (it does
-// not when the caller's control words may name fewer tokens), so the hidden rows can be made token by token.
+// not when the caller's control words may name fewer tokens), so the hidden rows can be made token by token, and routes
+// that gate/up skipped are known when the frames are read: they count as rows of zeros there, whatever an earlier call
+// left in the plan's frames.
 // `fused`: gate/up will write the down stage's operands itself.
 static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void* source, bool tensor, bool whole_call, bool fused) {
     const nvmoe_geometry& g = p->g;
@@ -834,19 +836,20 @@ static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void
     cudaStream_t st = p->device->stream;
     const DownRows down{fused ? p->position[1].as<uint32_t>() : nullptr, p->grouped_q[1].as<uint8_t>(), p->grouped_e8m0[1].as<uint32_t>(),
                         g.intermediate_size};
+    const uint32_t* written = !gate_up && whole_call ? p->position[0].as<uint32_t>() : nullptr;
     if (tensor && gate_up && whole_call &&
         launch_quantize_tokens(source, p->position[0].as<uint32_t>(), T, p->K, g.hidden_size, g.act_block, p->grouped_q[0].as<uint8_t>(),
                                p->grouped_e8m0[0].as<uint32_t>(), down, st)) {
     } else if (tensor) {
         launch_quantize_grouped(source, !gate_up, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), p->experts,
                                 T * p->K, p->K, gate_up ? g.hidden_size : g.intermediate_size, g.intermediate_size,
-                                g.act_block, p->grouped_q[set].as<uint8_t>(), p->grouped_e8m0[set].as<uint32_t>(), st);
+                                g.act_block, p->grouped_q[set].as<uint8_t>(), p->grouped_e8m0[set].as<uint32_t>(), written, st);
     } else if (gate_up) {
         launch_quantize((const uint16_t*)source, T, g.hidden_size, g.act_block, g.hidden_size, p->xq.as<uint8_t>(),
                         p->x_scales.as<float>(), p->x_e8m0.as<uint32_t>(), st);
     } else {
         launch_quantize_frames((const uint32_t*)source, T, p->K, g.intermediate_size, g.act_block, p->iq.as<uint8_t>(),
-                               p->i_scales.as<float>(), p->i_e8m0.as<uint32_t>(), st);
+                               p->i_scales.as<float>(), p->i_e8m0.as<uint32_t>(), written, st);
     }
     p->launches++;
     return post_launch(p, gate_up ? "quantize hidden" : "quantize intermediates");
@@ -1266,7 +1269,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         if (!launch_quantize_tokens(input->ptr, sub->position[1].as<uint32_t>(), T, 1u, cols, sub->g.act_block,
                                     sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), DownRows{}, st))
             launch_quantize_grouped(input->ptr, false, sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(), 1u, T, 1u, cols, cols,
-                                    sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), st);
+                                    sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), nullptr, st);
     } else {
         launch_quantize((const uint16_t*)input->ptr, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(),
                         sub->i_e8m0.as<uint32_t>(), st);

@@ -191,11 +191,12 @@ void launch_quantize(const uint16_t* input, uint32_t rows, uint32_t cols, uint32
 // grouped_routes[pos] (the token's hidden row when frames is false: source row = route / K of
 // `input` with `cols` columns; the route's own row of the intermediates frames otherwise), for pos below
 // expert_offsets[num_experts]. Scales as E8M0 words only. Expert-grouped rows are what a tiled TMA
-// load can fetch as one box per (expert, token tile).
+// load can fetch as one box per (expert, token tile). `written` (optional, [route]): a route marked 0xffffffff there has
+// no frame of this call and gives a row of zeros.
 void launch_quantize_grouped(const void* input, bool frames, const uint32_t* grouped_routes,
                              const uint32_t* expert_offsets, uint32_t num_experts, uint32_t max_routes, uint32_t K,
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
-                             uint32_t* scales_e8m0, cudaStream_t stream);
+                             uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream);
 // The same gate/up operands from the inverse list: position[token * K + r] = row of that route (0xffffffff: skipped),
 // valid for every route of the call. `down` (position null: nothing) names the down stage's operand rows, of which those
 // of routes that only the down stage keeps are set to zero. False when the shape needs the form above (blocks other than
@@ -211,7 +212,7 @@ bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_
 // the same for the K rows of every intermediates frame (skips the schedule words)
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K,
                             uint32_t intermediate_size, uint32_t block, uint8_t* q, float* scales_f32,
-                            uint32_t* scales_e8m0, cudaStream_t stream);
+                            uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream);
 // f32 scales -> packed E8M0 words, for prequantised inputs; sets *not_pow2 if a scale is not a power of two
 void launch_scales_to_e8m0(const float* scales, uint32_t rows, uint32_t cols, uint32_t block,
                            uint32_t* scales_e8m0, uint32_t* status, cudaStream_t stream);

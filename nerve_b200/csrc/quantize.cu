@@ -24,7 +24,8 @@ __device__ __forceinline__ uint32_t to_e4m3x4(float a, float b, float c, float d
 
 // A lane owns 4 columns at a time, so a block of `block` columns keeps block/4 lanes busy: a warp takes
 // one block of 128 or more columns, or 32*4/block smaller ones side by side (four blocks of 32).
-// row_of(r) gives the bf16 row pointer, so the same body serves plain matrices and MoE frames.
+// row_of(r) gives the bf16 row pointer, so the same body serves plain matrices and MoE frames; null stands for a row
+// of zeros.
 template <class RowFn>
 __device__ void quantize_body(RowFn row_of, uint32_t rows, uint32_t cols, uint32_t block, uint8_t* q,
                               float* scales_f32, uint32_t* scales_e8m0) {
@@ -44,9 +45,10 @@ __device__ void quantize_body(RowFn row_of, uint32_t rows, uint32_t cols, uint32
         const bool active = item < total;
         const uint32_t r = active ? (uint32_t)(item / blocks_per_row) : 0u, b = active ? (uint32_t)(item % blocks_per_row) : 0u;
         // rows of a frame are only 4-byte aligned when the route count is odd: 4-byte loads
-        const uint32_t* in = reinterpret_cast<const uint32_t*>(row_of(r) + (size_t)b * block);
+        const uint16_t* row = row_of(r);
+        const uint32_t* in = reinterpret_cast<const uint32_t*>(row + (size_t)b * block);
         float m = 0.0f;
-        if (active) {
+        if (active && row != nullptr) {
             for (uint32_t c4 = gl; c4 < quarter; c4 += lanes) {
                 uint2 v = make_uint2(in[2u * c4], in[2u * c4 + 1u]);
                 m = fmaxf(m, fmaxf(fmaxf(fabsf(nvmoe_bf16_to_f32(v.x)), fabsf(nvmoe_bf16_to_f32(v.x >> 16))),
@@ -59,7 +61,7 @@ __device__ void quantize_body(RowFn row_of, uint32_t rows, uint32_t cols, uint32
         const float inv = __fdiv_rn(1.0f, scale);  // exact: the scale is a power of two
         uint32_t* out = reinterpret_cast<uint32_t*>(q + (size_t)r * cols + (size_t)b * block);
         for (uint32_t c4 = gl; c4 < quarter; c4 += lanes) {
-            uint2 v = make_uint2(in[2u * c4], in[2u * c4 + 1u]);
+            uint2 v = row != nullptr ? make_uint2(in[2u * c4], in[2u * c4 + 1u]) : make_uint2(0u, 0u);
             out[c4] = to_e4m3x4(nvmoe_bf16_to_f32(v.x) * inv, nvmoe_bf16_to_f32(v.x >> 16) * inv,
                                 nvmoe_bf16_to_f32(v.y) * inv, nvmoe_bf16_to_f32(v.y >> 16) * inv);
         }
@@ -83,11 +85,13 @@ __global__ void __launch_bounds__(256) quantize_kernel(const uint16_t* input, ui
 
 __global__ void __launch_bounds__(256) quantize_frames_kernel(const uint32_t* intermediates, uint32_t tokens,
                                                              uint32_t K, uint32_t I, uint32_t block, uint8_t* q,
-                                                             float* scales_f32, uint32_t* scales_e8m0) {
+                                                             float* scales_f32, uint32_t* scales_e8m0,
+                                                             const uint32_t* written) {
     grid_dependency_sync();
     const uint32_t frame_words = K * (I / 2u) + K;
     quantize_body(
-        [&](uint32_t r) {
+        [&](uint32_t r) -> const uint16_t* {
+            if (written && written[r] == kUnboundSlot) return nullptr;
             return reinterpret_cast<const uint16_t*>(intermediates + (size_t)(r / K) * frame_words) + (size_t)(r % K) * I;
         },
         tokens * K, I, block, q, scales_f32, scales_e8m0);
@@ -96,13 +100,15 @@ __global__ void __launch_bounds__(256) quantize_frames_kernel(const uint32_t* in
 __global__ void __launch_bounds__(256) quantize_grouped_kernel(const void* input, bool frames, const uint32_t* grouped,
                                                               const uint32_t* expert_offsets, uint32_t num_experts,
                                                               uint32_t max_routes, uint32_t K, uint32_t cols, uint32_t I,
-                                                              uint32_t block, uint8_t* q, uint32_t* scales_e8m0) {
+                                                              uint32_t block, uint8_t* q, uint32_t* scales_e8m0,
+                                                              const uint32_t* written) {
     grid_dependency_sync();
     const uint32_t total = min(expert_offsets[num_experts], max_routes);
     const uint32_t frame_words = K * (I / 2u) + K;
     quantize_body(
-        [&](uint32_t pos) {
+        [&](uint32_t pos) -> const uint16_t* {
             const uint32_t ri = grouped[pos];
+            if (written && written[ri] == kUnboundSlot) return nullptr;
             return frames ? reinterpret_cast<const uint16_t*>(static_cast<const uint32_t*>(input) + (size_t)(ri / K) * frame_words) +
                                 (size_t)(ri % K) * I
                           : static_cast<const uint16_t*>(input) + (size_t)(ri / K) * cols;
@@ -257,17 +263,17 @@ void launch_quantize(const uint16_t* input, uint32_t rows, uint32_t cols, uint32
 }
 
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K, uint32_t intermediate_size,
-                            uint32_t block, uint8_t* q, float* scales_f32, uint32_t* scales_e8m0,
+                            uint32_t block, uint8_t* q, float* scales_f32, uint32_t* scales_e8m0, const uint32_t* written,
                             cudaStream_t stream) {
     if (tokens == 0u) return;
     launch_chained(quantize_frames_kernel, dim3(grid_for((uint64_t)tokens * K * (intermediate_size / block))), dim3(256), 0,
-                   stream, intermediates, tokens, K, intermediate_size, block, q, scales_f32, scales_e8m0);
+                   stream, intermediates, tokens, K, intermediate_size, block, q, scales_f32, scales_e8m0, written);
 }
 
 void launch_quantize_grouped(const void* input, bool frames, const uint32_t* grouped_routes,
                              const uint32_t* expert_offsets, uint32_t num_experts, uint32_t max_routes, uint32_t K,
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
-                             uint32_t* scales_e8m0, cudaStream_t stream) {
+                             uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream) {
     if (max_routes == 0u) return;
     if (!frames && (block == 32u || block == 128u) && cols % 8u == 0u && (reinterpret_cast<uintptr_t>(input) & 15u) == 0u) {
         const uint32_t side = block == 32u ? 8u : 2u;  // blocks a warp takes at once
@@ -281,7 +287,7 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
     }
     launch_chained(quantize_grouped_kernel, dim3(grid_for((uint64_t)max_routes * (cols / block))), dim3(256), 0, stream, input,
                    frames, grouped_routes, expert_offsets, num_experts, max_routes, K, cols, intermediate_size, block, q,
-                   scales_e8m0);
+                   scales_e8m0, written);
 }
 
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,

@@ -242,3 +242,39 @@ def test_dense_scales_rewritten_behind_wrapped_handles(device, path, handles):
         assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
     assert plan.status() == 0
     plan.destroy()
+
+
+# the gate/up epilogue makes the down operands (scale blocks of 32 and 128 rows), or a pass over the frames does (blocks of
+# 64, hidden rows off the 16-byte grid, the CUDA-core path)
+@pytest.mark.parametrize("path,block,shift", [(2, 32, 0), (2, 32, 8), (2, 64, 0), (2, 128, 0), (2, 128, 8), (1, 32, 0)])
+@pytest.mark.parametrize("tokens", [37, 900])  # one-block and three-launch schedule
+def test_routes_without_gate_up_count_as_zeros(device, path, block, shift, tokens):
+    """An expert absent from the gate/up tables alone, after a call that had every expert: its routes give what they give
+    when it is absent from both tables, rows of zeros, and not what the earlier call left in the plan's frames."""
+    cfg = synthetic.MoeConfig("zeros", hidden=256, intermediate=384, experts=8, k=2, act_block=block)
+    case = synthetic.make_case(cfg, tokens, seed=23)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(path)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    room, rw = device.create_resident_buffer(case.hidden.nbytes + 16), device.resident_buffer_from(case.router_w)
+    room.write_bytes(case.hidden, shift)
+    hidden = ResidentBuffer.wrap(device, room.device_address() + shift, case.hidden.nbytes)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+
+    def call():
+        plan.layer(tokens, bank, hidden, out, router_weights=rw)
+        return out.read(np.uint16)
+
+    def drop(slots, params):
+        words = slots.read(np.uint32).copy()
+        words[3 * params:4 * params] = 0xffffffff
+        slots.write_bytes(words)
+
+    whole = call()
+    drop(bank.gate_up_slots, 4)
+    got = call()
+    drop(bank.down_slots, 2)
+    want = call()
+    assert not np.array_equal(whole, want)
+    np.testing.assert_array_equal(got, want)
+    plan.destroy()
