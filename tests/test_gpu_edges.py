@@ -27,8 +27,10 @@ def plan_of(device, **kw):
     return MoePlan(device, geometry_from_config(synthetic.MoeConfig("edges", **fields), tokens))
 
 
-# one vector, a partial pass of the block, the longest row a block keeps, the first that it does not
-@pytest.mark.parametrize("rows,hidden", [(3, 8), (2, 8200), (150, 1032), (2, 24544), (2, 24552)])
+# one vector, a partial pass of the block, the longest row a block keeps, the first that it does not; the last count of
+# short rows that goes to blocks and the first that goes to warps, the shortest row that always goes to blocks
+@pytest.mark.parametrize("rows,hidden", [(3, 8), (2, 8200), (150, 1032), (2, 24544), (2, 24552), (2368, 72), (2369, 72),
+                                         (2369, 2040), (2369, 2048)])
 def test_rms_norm_rows(device, rows, hidden):
     rng = np.random.default_rng(hidden)
     x, w = bf16(rng.standard_normal((rows, hidden))), bf16(1.0 + 0.1 * rng.standard_normal(hidden))
