@@ -281,3 +281,19 @@ def test_routes_without_gate_up_count_as_zeros(device, path, block, shift, token
     assert not np.array_equal(whole, want)
     np.testing.assert_array_equal(got, want)
     plan.destroy()
+
+
+# one step of four, a whole second one, the nine that are taken at once and the counts beside it, remainders beyond
+@pytest.mark.parametrize("k", [3, 8, 9, 10, 13, 18])
+@pytest.mark.parametrize("scale", [1.0, 2.5])
+def test_combine_of_any_route_count(device, k, scale):
+    tokens = 37
+    cfg = synthetic.MoeConfig("combine", hidden=288, intermediate=256, experts=32, k=k, act_block=32)
+    geometry = geometry_from_config(cfg, tokens)
+    geometry.reduce_scale = scale
+    plan = MoePlan(device, geometry)
+    rows = bf16(np.random.default_rng(k).standard_normal((tokens, k, cfg.hidden)))
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.moe_reduce(tokens, device.resident_buffer_from(rows), out)
+    np.testing.assert_array_equal(out.read(np.uint16).reshape(tokens, cfg.hidden), mo.reduce(rows, tokens, k, cfg.hidden, scale))
+    plan.destroy()
