@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(1024) layer_schedule_small_kernel(LayerSchedul
 // counts them per warp), and its down stage visits the first owned-by-the-down-table-count of them.
 // One round trip to global memory, five block barriers.
 constexpr uint32_t kRankChunks = 16u;  // routes per thread at most (count <= 16 * blockDim); the kernel is built for 1, 4 and 16
-constexpr uint32_t kWideScheduleRoutes = 1024u;
+constexpr uint32_t kWideScheduleRoutes = 1280u;
 constexpr uint32_t kNotListed = 0xffffu;  // bucket field of a route that is in no list
 
 __host__ __device__ inline uint32_t layer_schedule_rank_threads(uint32_t count) { return count <= 256u ? 256u : 1024u; }
@@ -1121,8 +1121,10 @@ static bool three_sort_schedule_fits(uint64_t count, uint32_t num_experts) {
     return count <= kSmallSortLimit && layer_schedule_smem_bytes((uint32_t)count, num_experts) <= 48u * 1024u;
 }
 
-// More routes than one pass of a 1024-thread block go to the three-launch form, unless it is a partitioned call or the
-// tables of that many experts do not fit.
+// Beyond 1280 routes the three launches are cheaper than the one block's longer loop, unless it is a partitioned call or
+// the tables of that many experts do not fit. Layer of 384 x 256, three launches / one, us: 1028 routes of 32 experts
+// 48.1 / 47.4, 1200 of 128 61.3 / 60.5, 1440 of 129 (512 x 256) 72.8 / 73.0, 1600 of 16 49.3 / 48.6, of 128 60.6 / 61.5,
+// 2048 of 32 50.4 / 51.6, 4096 of 128 72.6 / 80.5.
 static bool wide_schedule_fits(uint64_t count, uint32_t num_experts, bool partitioned) {
     return count > kWideScheduleRoutes && !partitioned && num_experts < kNotListed - 1u &&
            layer_schedule_wide_smem_bytes(num_experts) <= 48u * 1024u;

@@ -68,10 +68,11 @@ def test_dense_linears_of_one_shape_keep_their_own_tables(device):
     plan.destroy()
 
 
-# routes on either side of the one-block schedule's limit (1024), whole and ragged blocks of 256 routes, both scale
+# routes on either side of the one-block schedule's single pass (1024) and of its limit (1280), whole and ragged blocks of 256 routes, both scale
 # blocks, a K tail (352 = 2.75 x 128), an expert that is not resident
 @pytest.mark.parametrize("name,shape,tokens,absent", [
     ("gpt-oss-20b", (256, 384, 16), 256, None), ("gpt-oss-20b", (352, 160, 33), 257, 5), ("gpt-oss-20b", (1056, 320, 16), 1100, 0),
+    ("gpt-oss-20b", (256, 384, 16), 320, 3), ("gpt-oss-20b", (352, 160, 33), 321, 5), ("deepseek-v3", (256, 256, 24), 143, 24),
     ("deepseek-v3", (512, 256, 24), 113, None), ("deepseek-v3", (384, 640, 24), 114, 24), ("deepseek-v3", (1024, 256, 256), 512, 7)])
 def test_layer_call_equals_its_nodes(device, name, shape, tokens, absent):
     """The layer call schedules, quantises and fuses in its own way; the node operators are the plain one."""
