@@ -484,12 +484,12 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         const dim3 grid((outputs + 3u) / 4u, (tokens + 1u) / 2u), wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
         // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, but an
         // SM holds eight of its blocks and takes as long for one as for eight, where the time of 2 x 4 tiles grows with
-        // their number: the wide ones when they fill most of a first wave, and not just over it. Wide / small tiles at H
-        // 7168, us, by wide blocks per SM: 4.1 26.7 / 21.1, 5.2 26.8 / 27.4 (26.7 / 25.1 with warm caches), 6.05
-        // 27.0 / 29.5, 8.0 27.1 / 37.5, 8.2 39.3 / 37.9, 9.1 39.6 / 41.8, 10.4 39.7 / 47.2, 13.8 45.9 / 60.0; at H 512,
-        // 8.4 9.8 / 9.1, 9.95 10.4 / 10.1, 10.4 10.5 / 10.6, 13.8 11.2 / 13.2.
+        // their number: the wide ones when they fill most of a first wave, and not just over it. Wide / small tiles inside
+        // a layer call, us by wide blocks per SM: 4.1 195.3 / 191.4 (hidden 7168), 114.1 / 112.4 (2880); 4.5 197.2 /
+        // 197.7, 120.3 / 120.3; 5.2 197.5 / 203.1, 114.3 / 116.8; 6.5 209.5 / 213.2; 8.2 226.0 / 225.6; 9.1 228.4 /
+        // 231.5. By itself at 8.4 blocks 9.8 / 9.1 (hidden 512) and 20.1 / 18.4 (2880), at 9.1 39.6 / 41.8 (7168).
         const uint32_t blocks = wide.x * wide.y;
-        if (blocks >= 6u * 148u && (blocks <= 8u * 148u || blocks >= 10u * 148u)) {
+        if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
             launch_chained(router_linear_kernel<4, 8>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);
         } else {
             launch_chained(router_linear_kernel<2, 4>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);

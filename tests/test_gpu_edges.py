@@ -110,10 +110,10 @@ def test_layer_call_equals_its_nodes(device, name, shape, tokens, absent):
 
 
 # the 4 x 8 tiles with ragged tokens, an odd expert count and rows that end inside a step; the calls just below and above
-# each limit of their rule (6, 8 and 10 blocks of 148 SMs); the tiled form with a row of less than one chunk and last chunks that end in their first or second half
+# each limit of their rule (5, 8 and 9 blocks on each of 148 SMs); the tiled form with a row of less than one chunk and last chunks that end in their first or second half
 @pytest.mark.parametrize("tokens,hidden,experts,bias", [(98, 288, 199, 1), (255, 1056, 74, 0), (94, 288, 192, 0), (257, 32, 17, 0),
-                                                        (289, 288, 8, 1), (300, 352, 33, 0), (144, 96, 185, 1), (145, 96, 185, 0),
-                                                        (145, 96, 255, 1), (149, 96, 255, 0), (184, 96, 255, 0), (185, 96, 255, 1)])
+                                                        (289, 288, 8, 1), (300, 352, 33, 0), (144, 96, 159, 1), (145, 96, 159, 0),
+                                                        (145, 96, 255, 1), (149, 96, 255, 0), (164, 96, 255, 0), (165, 96, 255, 1)])
 def test_router_projection_tiles(device, tokens, hidden, experts, bias):
     rng = np.random.default_rng(tokens + hidden)
     plan = plan_of(device, tokens=tokens, hidden=hidden, experts=experts)
