@@ -1,10 +1,12 @@
-"""Sizes at which the launch rules change kernels, and the remainders inside them: every case against the CPU checker."""
+"""Sizes at which the launch rules change kernels, and the remainders inside them: against the CPU checker, or (the layer
+call and its nodes, rows off the 16-byte grid, routes without gate/up) against another form of the same work."""
 import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
 from nerve_b200.backend import CudaComputeDevice, CudaError, ExpertBank, MoePlan, ResidentBuffer, geometry_from_config
 from oracle import moe_oracle as mo
+from oracle import sampled
 from tests.helpers import assert_close, oracle_layer
 
 pytestmark = pytest.mark.gpu
@@ -299,3 +301,31 @@ def test_combine_of_any_route_count(device, k, scale):
     plan.moe_reduce(tokens, device.resident_buffer_from(rows), out)
     np.testing.assert_array_equal(out.read(np.uint16).reshape(tokens, cfg.hidden), mo.reduce(rows, tokens, k, cfg.hidden, scale))
     plan.destroy()
+
+
+# 16- and 32-token tiles in row pairs: enough experts for six rounds of the SMs (min(routes, experts) x 8 row pairs >= 888),
+# a last pair that is a lone 128-row half (1920 = 7.5 x 256), a K tail (352 = 2.75 x 128), a native FP8 resource
+@pytest.mark.parametrize("name,shape,tokens,native", [("gpt-oss-20b", (1920, 352, 128), 250, 0), ("gpt-oss-20b", (1920, 352, 128), 620, 0),
+                                                      ("deepseek-v3", (1920, 384, 128), 100, 1), ("deepseek-v3", (1920, 384, 128), 300, 1)])
+def test_narrow_row_pairs_match_the_checker(device, name, shape, tokens, native):
+    cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], *shape), native_fp8_resources=native)
+    assert min(tokens * cfg.total_k, cfg.total_experts) * -(-cfg.hidden // 256) >= 6 * 148
+    case = synthetic.make_case(cfg, tokens, seed=13)
+    tensors = [list(t) for t in (case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)]
+    for e in range(cfg.total_experts - native, cfg.total_experts):
+        for i, t in enumerate(synthetic.native_fp8_tensors(cfg, 13, e)):
+            tensors[i][e] = t
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(2)
+    bank = ExpertBank.upload(device, *tensors)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, device.resident_buffer_from(case.hidden), out, router_weights=device.resident_buffer_from(case.router_w),
+               router_bias=device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+               bias=device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None)
+    logits = mo.linear_bf16(case.hidden, case.router_w, case.router_bias)
+    sample = sampled.sample_tokens(tokens, 96, seed=tokens)
+    want = sampled.layer_on_sample(cfg, case.hidden, logits, case.select_bias, sample, lambda e: [t[e] for t in tensors])
+    assert_close(out.read(np.uint16).reshape(tokens, cfg.hidden)[sample], want["output"], f"{name} narrow row pairs T{tokens}")
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
