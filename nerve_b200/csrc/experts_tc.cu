@@ -48,8 +48,7 @@ constexpr uint32_t kTmaBoxBytes = kBlockM * 64u;   // global bytes of one 128 x 
 constexpr uint32_t kATileBytes = kBlockM * 128u;   // one byte slot per element
 constexpr uint32_t kScaleBlockBytes = 512u;        // 128 rows x 4 scale bytes
 constexpr uint32_t kMaxStages = 8u;
-constexpr uint32_t kTargetSms = 148u;
-constexpr uint32_t kRowPairRounds = 6u;  // tiles an SM goes through at least before narrow down tiles pair their rows
+constexpr uint32_t kRowPairRounds = 6u;  // rounds of the SMs, with every expert selected, from which narrow down tiles pair their rows
 constexpr uint32_t kWatchWarp = 2u;     // the epilogue warp that polls for a finished accumulator (not on the MMA or TMA warp's scheduler)
 
 struct TileList {
@@ -926,6 +925,13 @@ __global__ void __launch_bounds__(256) dense_prepare_kernel(DensePrepare p, uint
 
 int g_sm_count[16] = {0};
 
+int sm_count() {  // of the current device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (g_sm_count[dev & 15] == 0) cudaDeviceGetAttribute(&g_sm_count[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+    return g_sm_count[dev & 15];
+}
+
 template <bool GATE_UP, uint32_t N_TILE, bool USE_TMA, bool ROW_PAIR>
 void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
     using C = Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>;
@@ -940,9 +946,15 @@ void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
 }
 
 // Whether a down launch takes two row tiles at a time: always with wide token tiles, and with narrow ones (TMA form)
-// when that leaves every SM several tiles to go through. A stage of a row pair is one K block of two weight boxes, one
+// when that leaves an SM several tiles to go through, counted as if every expert were selected (what routing, a partition
+// or absent experts leave of them is not known here). A stage of a row pair is one K block of two weight boxes, one
 // token box and two scale copies, where a single row tile needs six copies for the same bytes (0.42 against 0.49 us per
-// stage); single row tiles spread over the SMs in finer steps, which is worth more when there are only a few rounds.
+// stage); single row tiles spread over the SMs in finer steps, which 32-token tiles gain from while there are few rounds.
+// Layer of intermediate 1536, single rows / row pairs, us, by rounds: 32-token tiles 0.65 54.9 / 57.6, 1.95 77.7 / 78.6,
+// 2.6 92.6 / 93.1, 3.5 108.1 / 108.2, 5.2 155.9 / 154.5, 6.05 158.5 / 151.9, 10.4 261.3 / 249.2; 16-token tiles 0.65 55.7 /
+// 51.6, 2.6 87.4 / 83.3, 6.05 150.6 / 142.2, 24 469.6 / 442.3. Partitioned calls of 128 experts with 16 and 32 of them
+// owned (1.3 and 2.6 rounds of their own): 115.3 / 115.6 and 136.4 / 132.4 with 32-token tiles, 87.3 / 87.7 and 105.1 /
+// 104.2 with 16.
 bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) {
     if (n_tile >= 64u) return true;
     if (!tma) return false;
@@ -953,10 +965,7 @@ bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) 
 
 template <bool GATE_UP>
 void launch(const ExpertLaunch& p, cudaStream_t stream) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (g_sm_count[dev & 15] == 0) cudaDeviceGetAttribute(&g_sm_count[dev & 15], cudaDevAttrMultiProcessorCount, dev);
-    const int sms = g_sm_count[dev & 15];
+    const int sms = sm_count();
     const uint32_t n = tc_token_tile_for(p.tokens, p.g.routed_k + p.g.always_count, p.work.num_experts,
                                          GATE_UP ? p.g.intermediate_size : p.g.hidden_size, GATE_UP);
     const bool tma = p.tmaps != nullptr;
@@ -1022,17 +1031,18 @@ uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t 
     if (per_expert <= 24u) return 32u;
     if (per_expert <= 48u) return 64u;
     if (per_expert <= 96u) return 96u;
-    // Beyond that an expert takes several tiles and the wide ones are the cheapest per token (a stage of 128 columns
-    // takes about 56/50 of the time of one of 96: 16384 tokens x 7168 x 2048 in 256 experts 9.98 against 10.48 ms), unless
-    // a wave of the SMs goes half empty with them (777 x 7168 x 2048 dense: 115 us with 128 columns, 109 with 96): the
-    // fewest rounds x stage time wins.
+    // Beyond that an expert takes several tiles and the wide ones are the cheapest per token, unless a wave of the SMs
+    // goes half empty with them (777 x 7168 x 2048 dense: 115 us with 128 columns, 109 with 96): the fewest rounds x
+    // stage time wins. A stage of 128 columns takes 8/7 of the time of one of 96 (0.527 and 0.461 us in the down kernel
+    // of 12288 x 2944 x 9472, whole rounds of either); 4096 tokens of 32 experts of 2880 x 2880 640 against 683 us.
     const uint32_t row_tiles = gate_up ? (out_rows + kBlockM - 1u) / kBlockM : (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM);
-    const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {56u, 50u};
+    const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {8u, 7u};
+    const uint64_t sms = (uint64_t)sm_count();
     uint32_t best = 0u;
     uint64_t best_cost = ~0ull;
     for (uint32_t i = 0; i < 2u; i++) {
         const uint64_t tiles = (uint64_t)num_experts * ((per_expert + widths[i] - 1u) / widths[i]) * row_tiles;
-        const uint64_t cost = (tiles + kTargetSms - 1u) / kTargetSms * stage_time[i];
+        const uint64_t cost = (tiles + sms - 1u) / sms * stage_time[i];
         if (cost < best_cost) {
             best_cost = cost;
             best = widths[i];
