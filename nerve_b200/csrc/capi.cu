@@ -1254,7 +1254,6 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     dp.tokens = T;
     dp.grouped = sub->grouped[1].as<uint32_t>();
     dp.offsets = sub->offsets[1].as<uint32_t>();
-    dp.position = sub->position[1].as<uint32_t>();
     dp.ptrs = dl->set.ptrs.as<ExpertPtrs>();
     if (tensor) {
         dp.tiles = TileOut{region + 64, region, tc_token_tile_for(T, 1u, 1u, rows, false)};
@@ -1262,20 +1261,23 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         dp.map_template = sub->tma[1] ? sub->tmap_templates.as<uint8_t>() + 256 : nullptr;
         dp.map = dl->set.tmaps.as<uint8_t>();
     }
-    launch_dense_prepare(dp, st);
+    dp.input = (const uint16_t*)input->ptr;
+    dp.q = sub->grouped_q[1].as<uint8_t>();
+    dp.q_e8m0 = sub->grouped_e8m0[1].as<uint32_t>();
+    const bool quantised = launch_dense_prepare(dp, sub->g.act_block, st);
     sub->launches++;
-    NVMOE_TRY(post_launch(sub, "dense linear schedule"));
-    if (tensor) {
-        if (!launch_quantize_tokens(input->ptr, sub->position[1].as<uint32_t>(), T, 1u, cols, sub->g.act_block,
-                                    sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), DownRows{}, st))
-            launch_quantize_grouped(input->ptr, false, sub->grouped[1].as<uint32_t>(), sub->offsets[1].as<uint32_t>(), 1u, T, 1u, cols, cols,
-                                    sub->g.act_block, sub->grouped_q[1].as<uint8_t>(), sub->grouped_e8m0[1].as<uint32_t>(), nullptr, st);
-    } else {
-        launch_quantize((const uint16_t*)input->ptr, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(),
-                        sub->i_e8m0.as<uint32_t>(), st);
+    NVMOE_TRY(post_launch(sub, "dense linear operands"));
+    if (!quantised) {
+        if (tensor) {
+            launch_quantize_grouped(input->ptr, false, dp.grouped, dp.offsets, 1u, T, 1u, cols, cols, sub->g.act_block, dp.q, dp.q_e8m0,
+                                    nullptr, st);
+        } else {
+            launch_quantize(dp.input, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(),
+                            sub->i_e8m0.as<uint32_t>(), st);
+        }
+        sub->launches++;
+        NVMOE_TRY(post_launch(sub, "dense linear quantise"));
     }
-    sub->launches++;
-    NVMOE_TRY(post_launch(sub, "dense linear quantise"));
     ExpertCall call;
     call.gate_up = false;
     call.T = T;

@@ -34,6 +34,7 @@
 #include <cstring>
 
 #include "experts_tc.cuh"
+#include "quantize.cuh"
 #include "tcgen05.cuh"
 
 namespace nvmoe {
@@ -871,43 +872,60 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 
 // The same for the one matrix of a dense linear, whose addresses are the call's own: nothing about the matrix is kept
 // between calls, so that scales rewritten in place by any means are what the next call reads. A block re-tiles 128 rows
-// x 8 K blocks, a thread 4 rows of one K block: 32 neighbouring bytes of a scale row per 8 threads in, one 16-byte
-// store out. The last block writes the pointers and the tensor map. Bound by the latency of one load and one store:
-// the 458 KB of a 2048 x 7168 matrix are far below what the launch takes anyway.
-constexpr uint32_t kDenseKBlocks = 8u;
-__global__ void __launch_bounds__(256) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
+// x 4 K blocks, a thread 4 rows of one K block and one 16-byte store. The last block writes the pointers and the tensor
+// map. With scale blocks of 32 or 128 columns (LANES = block / 16; 0: none) further blocks quantise the input, a warp 512
+// columns of one row, so that the launch takes little longer than that alone: bound by the latency of a load and a
+// store. Block of 777 x 7168 x 2048: 114.0 us with the quantisation in a launch of its own, 107 here.
+constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
     __shared__ __align__(128) unsigned char sm[128];
     grid_dependency_sync();
     const uint32_t tile_total = p.tiles.list ? (p.tokens + p.tiles.n_tile - 1u) / p.tiles.n_tile : 0u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.tokens; i += gridDim.x * blockDim.x) {
+    for (uint32_t i = blockIdx.x * kDenseThreads + threadIdx.x; i < p.tokens; i += gridDim.x * kDenseThreads) {
         p.grouped[i] = i;
-        p.position[i] = i;
         if (i < tile_total) p.tiles.list[i] = i;  // (expert 0 << 16) | token tile
     }
     if (blockIdx.x < retile_blocks) {
         const uint32_t k_groups = (k_blocks + kDenseKBlocks - 1u) / kDenseKBlocks;
         const uint32_t m_tile = blockIdx.x / k_groups, row_bytes = p.cols / 32u;
-        const uint32_t kb = blockIdx.x % k_groups * kDenseKBlocks + threadIdx.x % kDenseKBlocks, q = threadIdx.x / kDenseKBlocks;
-        if (kb < k_blocks) {
-            uint32_t word[4];
+        const uint32_t kb = blockIdx.x % k_groups * kDenseKBlocks + threadIdx.x % kDenseKBlocks, r = threadIdx.x / kDenseKBlocks;
+        if (kb >= k_blocks) return;
+        uint32_t word[4];
 #pragma unroll
-            for (uint32_t j = 0; j < 4u; j++) {
-                const uint32_t row = m_tile * kBlockM + q + 32u * j;
-                const uint8_t* in = p.scales + (size_t)row * row_bytes + kb * 4u;
-                word[j] = 0x7f7f7f7fu;
-                if (row < p.out_rows && row_bytes % 4u == 0u) {
-                    word[j] = __ldg(reinterpret_cast<const uint32_t*>(in));
-                } else if (row < p.out_rows) {
-                    word[j] = 0u;
+        for (uint32_t j = 0; j < 4u; j++) {
+            const uint32_t row = m_tile * kBlockM + r + 32u * j;
+            const uint8_t* in = p.scales + (size_t)row * row_bytes + kb * 4u;
+            word[j] = 0x7f7f7f7fu;
+            if (row < p.out_rows && row_bytes % 4u == 0u) {
+                word[j] = __ldg(reinterpret_cast<const uint32_t*>(in));
+            } else if (row < p.out_rows && row_bytes % 2u == 0u) {
+                word[j] = __ldg(reinterpret_cast<const uint16_t*>(in)) |
+                          (kb * 4u + 2u < row_bytes ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(in) + 1) : 0x7f7fu) << 16;
+            } else if (row < p.out_rows) {
+                word[j] = 0u;
 #pragma unroll
-                    for (uint32_t b = 0; b < 4u; b++) word[j] |= (uint32_t)(kb * 4u + b < row_bytes ? __ldg(in + b) : 127u) << (8u * b);
-                }
+                for (uint32_t b = 0; b < 4u; b++) word[j] |= (uint32_t)(kb * 4u + b < row_bytes ? __ldg(in + b) : 127u) << (8u * b);
             }
-            *reinterpret_cast<uint4*>(p.derived + ((size_t)m_tile * k_blocks + kb) * kScaleBlockBytes + q * 16u) =
-                make_uint4(word[0], word[1], word[2], word[3]);
         }
+        *reinterpret_cast<uint4*>(p.derived + ((size_t)m_tile * k_blocks + kb) * kScaleBlockBytes + r * 16u) =
+            make_uint4(word[0], word[1], word[2], word[3]);
+        return;
     }
-    if (blockIdx.x != gridDim.x - 1u) return;
+    if (blockIdx.x != gridDim.x - 1u) {
+        if (LANES == 0u) return;
+        const uint32_t lane = threadIdx.x & 31u, chunks = (p.cols + 511u) / 512u, words128 = (p.cols + 127u) / 128u;
+        const uint32_t item = (blockIdx.x - retile_blocks) * (kDenseThreads / 32u) + (threadIdx.x >> 5);
+        const uint32_t row = item / chunks, col = (item % chunks) * 512u + lane * 16u;
+        if (row >= p.tokens) return;
+        const bool active = col < p.cols;  // (columns come in whole blocks: the lanes of a block agree)
+        uint32_t out[4], word;
+        quantize_sixteen<(LANES == 0u ? 1u : LANES)>(p.input + (size_t)row * p.cols + col, active, lane, out, word);
+        if (!active) return;
+        *reinterpret_cast<uint4*>(p.q + (size_t)row * p.cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
+        if ((lane & 7u) == 0u) p.q_e8m0[(size_t)row * words128 + col / 128u] = word;
+        return;
+    }
     if (threadIdx.x == 0u) {
         p.offsets[0] = 0u;
         p.offsets[1] = p.tokens;
@@ -1070,11 +1088,17 @@ void launch_derive_scales_tc(const ExpertLaunch& p, bool gate_up, cudaStream_t s
     commit_stamps_kernel<<<(count + 127u) / 128u, 128, 0, stream>>>(p.work.experts, p.scale_stamps, matrices, count);
 }
 
-void launch_dense_prepare(const DensePrepare& p, cudaStream_t stream) {
+bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_t stream) {
     const uint32_t m_tiles = (p.out_rows + kBlockM - 1u) / kBlockM, k_blocks = (p.cols + kBlockK - 1u) / kBlockK;
     const uint32_t retile = p.derived ? m_tiles * ((k_blocks + kDenseKBlocks - 1u) / kDenseKBlocks) : 0u;
-    const uint32_t schedule = (p.tokens + 255u) / 256u;
-    launch_chained(dense_prepare_kernel, dim3((retile > schedule ? retile : schedule) + 1u), dim3(256), 0, stream, p, k_blocks, retile);
+    const uint64_t warps = (uint64_t)p.tokens * ((p.cols + 511u) / 512u);
+    const bool quantises = p.derived && (act_block == 32u || act_block == 128u) && (reinterpret_cast<uintptr_t>(p.input) & 15u) == 0u &&
+                           warps <= 0x3fffffffull;
+    // (without rows to quantise, as many blocks as the schedule's lists ask for)
+    const uint32_t others = quantises ? (uint32_t)((warps + 3u) / 4u) : (p.tokens + kDenseThreads - 1u) / kDenseThreads;
+    const auto kernel = !quantises ? dense_prepare_kernel<0u> : act_block == 32u ? dense_prepare_kernel<2u> : dense_prepare_kernel<8u>;
+    launch_chained(kernel, dim3(retile + others + 1u), dim3(kDenseThreads), 0, stream, p, k_blocks, retile);
+    return quantises;
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

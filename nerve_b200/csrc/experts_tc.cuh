@@ -20,23 +20,27 @@ bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t
 bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t n_tile);
 // per-expert tensor maps = template + the expert's weight address (p.tmaps must be set)
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream);
-// What a dense linear needs before its quantisation, in one launch: the schedule (every row a route of expert 0 in row
-// order) and what hangs on its matrix: the pointers and, for the tensor path (`derived` set), the re-tiled scales and the
-// tensor map (map_template null: none). weights and scales are 32-byte aligned.
+// What a dense linear needs before its expert kernel, in one launch: the schedule (every row a route of expert 0 in row
+// order), what hangs on its matrix (the pointers and, for the tensor path (`derived` set), the re-tiled scales and the
+// tensor map (map_template null: none); weights and scales are 32-byte aligned), and the quantised input rows. False when
+// the input needs one of the general quantisations, which then follows: CUDA-core path, scale blocks other than 32 or 128
+// columns, rows off the 16-byte grid.
 struct DensePrepare {
     const uint8_t* weights;
     const uint8_t* scales;
     uint32_t out_rows, cols, tokens;
     uint32_t* grouped;
     uint32_t* offsets;
-    uint32_t* position;
     TileOut tiles;
     ExpertPtrs* ptrs;
     uint8_t* derived;
     const uint8_t* map_template;
     uint8_t* map;
+    const uint16_t* input;
+    uint8_t* q;
+    uint32_t* q_e8m0;
 };
-void launch_dense_prepare(const DensePrepare& p, cudaStream_t stream);
+bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_t stream);
 // token tile size of a stage for this many tokens and rows of its weight matrix (the (expert, token tile) list must be
 // built with it)
 uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up);

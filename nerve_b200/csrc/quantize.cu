@@ -8,19 +8,10 @@
 // The reference block is 128 columns; any multiple of 32 that divides the row works here.  Besides
 // the f32 scales of the reference contract the kernel can emit the same scales as E8M0 bytes, one
 // per 32 columns, four to a word — the form a block-scaled MMA reads.
-#include <cuda_fp8.h>
-
-#include "common.cuh"
+#include "quantize.cuh"
 
 namespace nvmoe {
 namespace {
-
-__device__ __forceinline__ uint32_t to_e4m3x4(float a, float b, float c, float d) {
-    // cvt.rn.satfinite.e4m3x2.f32: round-to-nearest-even, saturating (|x/scale| <= 448 by construction)
-    uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-    uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
-    return lo | (hi << 16);
-}
 
 // A lane owns 4 columns at a time, so a block of `block` columns keeps block/4 lanes busy: a warp takes
 // one block of 128 or more columns, or 32*4/block smaller ones side by side (four blocks of 32).
@@ -184,29 +175,8 @@ __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __
     if (token >= tokens) return;
     const bool active = col < cols;  // (columns come in whole blocks: the lanes of a block agree)
     uint32_t mine = lane < K ? __ldg(position + (size_t)token * K + lane) : kUnboundSlot;
-    uint4 v[2] = {};
-    if (active) {
-        const uint4* src = reinterpret_cast<const uint4*>(input + (size_t)token * cols + col);
-        v[0] = __ldg(src);
-        v[1] = __ldg(src + 1);
-    }
-    const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
-    float m = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) m = fmaxf(m, fmaxf(fabsf(nvmoe_bf16_to_f32(w[i])), fabsf(nvmoe_bf16_to_f32(w[i] >> 16))));
-#pragma unroll
-    for (uint32_t o = 1u; o < LANES; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const float scale = nvmoe_rounded_fp8_scale(m);
-    const float inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
-    uint32_t out[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        out[i] = to_e4m3x4(nvmoe_bf16_to_f32(w[2 * i]) * inv, nvmoe_bf16_to_f32(w[2 * i] >> 16) * inv,
-                           nvmoe_bf16_to_f32(w[2 * i + 1]) * inv, nvmoe_bf16_to_f32(w[2 * i + 1] >> 16) * inv);
-    // two lanes hold 32 columns: byte (lane % 8) / 2 of the word of their 128
-    uint32_t word = active ? (nvmoe_f32_bits(scale) >> 23) << (8u * ((lane & 7u) >> 1)) : 0u;
-    word |= __shfl_xor_sync(0xffffffffu, word, 2);
-    word |= __shfl_xor_sync(0xffffffffu, word, 4);
+    uint32_t out[4], word;
+    quantize_sixteen<LANES>(input + (size_t)token * cols + col, active, lane, out, word);
     const uint32_t words128 = (cols + 127u) / 128u;
     for (uint32_t r0 = 0; r0 < K; r0 += 32u) {
         if (r0 != 0u) mine = r0 + lane < K ? __ldg(position + (size_t)token * K + r0 + lane) : kUnboundSlot;

@@ -225,12 +225,14 @@ def test_dense_linear_refuses_matrices_off_the_32_byte_grid(device, path):
     plan.destroy()
 
 
-@pytest.mark.parametrize("path", [1, 2])
+# rows of scale bytes of an odd count (352 / 32), an even one (320 / 32) and whole words (1152 / 32), K blocks in one, one and
+# three groups of four
+@pytest.mark.parametrize("path,cols", [(1, 352), (2, 352), (2, 320), (2, 1152)])
 @pytest.mark.parametrize("handles", ["kept", "fresh"])
-def test_dense_scales_rewritten_behind_wrapped_handles(device, path, handles):
+def test_dense_scales_rewritten_behind_wrapped_handles(device, path, cols, handles):
     """Two matrices of one shape in turn, their memory the caller's own: codes and scales are refilled in place, without
     a word to the library, through the handles that were used before or through new ones. Every call reads what is there."""
-    rows, cols, tokens = 160, 352, 9
+    rows, tokens = 160, 9
     rng = np.random.default_rng(17)
     plan = plan_of(device)
     plan.set_expert_path(path)
@@ -329,3 +331,22 @@ def test_narrow_row_pairs_match_the_checker(device, name, shape, tokens, native)
     assert plan.status() == 0
     plan.destroy()
     bank.destroy()
+
+
+# the input quantised beside the matrix (scale blocks of 32 and 128, a ragged last 512 columns) and in a launch of its own
+# (blocks of 64, rows off the 16-byte grid); several row tiles with a ragged last one, a row beyond one token tile
+@pytest.mark.parametrize("block,shift,rows,cols,tokens", [(32, 0, 288, 544, 5), (32, 0, 160, 1056, 131), (128, 0, 384, 640, 33),
+                                                         (64, 0, 320, 576, 17), (32, 8, 288, 544, 17), (128, 8, 256, 640, 200)])
+def test_dense_linear_operands(device, block, shift, rows, cols, tokens):
+    rng = np.random.default_rng(rows + cols)
+    plan = plan_of(device, act_block=block, tokens=256)
+    plan.set_expert_path(2)
+    x = bf16(rng.standard_normal((tokens, cols)))
+    w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(118, 128, (rows, cols // 32), dtype=np.uint8)
+    room, ob = device.create_resident_buffer(x.nbytes + 16), device.create_resident_buffer(tokens * rows * 2)
+    room.write_bytes(x, shift)
+    xb = ResidentBuffer.wrap(device, room.device_address() + shift, x.nbytes)
+    plan.dense_linear(tokens, xb, ob, device.resident_buffer_from(w), device.resident_buffer_from(s), rows, cols)
+    assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, block, tier=1))
+    assert plan.status() == 0
+    plan.destroy()
