@@ -149,7 +149,7 @@ struct LayerSchedule {
     uint32_t tokens, expert_start, expert_count, K, I, tiles_per_route[2], num_experts, n_tile[2];
 };
 bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned);
-// the router and the schedule of a call of up to 16 tokens in one launch
+// the router and the schedule of a call of up to 16 tokens (32 of up to 32 experts) in one launch
 bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts);
 void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream);
 uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream);  // returns its launches

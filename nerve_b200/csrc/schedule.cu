@@ -1138,11 +1138,12 @@ bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, 
 
 // A warp of the one block per token, all routes in one pass. The launch saved is about a microsecond; the router's own
 // chain grows with the experts a lane holds and the warps of the one SM get in each other's way, so it stops at sixteen
-// tokens. Layer of 384 x 256 in one launch / two, us: 8 tokens of 32 experts 33.0 / 34.0, 16 34.2 / 35.4, 24 36.4 /
-// 36.1; 16 of 128 41.9 / 41.8, 24 of 64 39.6 / 38.7, 32 of 128 46.0 / 44.8.
+// tokens where a lane holds several. Layer of 384 x 256 in one launch / two, us: 8 tokens of 32 experts 33.0 / 34.0, 16
+// 34.2 / 35.4, 24 36.4 / 36.1, 32 37.2 / 37.1 (32 from host buffers, 1024 x 512: 71.8 / 72.6); 16 of 128 41.9 / 41.8, 24
+// of 64 39.6 / 38.7, 32 of 128 46.0 / 44.8.
 bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts) {
     const uint64_t count = (uint64_t)router.tokens * K;
-    return router.tokens <= 16u && router_is_small(router) && count <= 1024u && rank_schedule_fits(count, num_experts);
+    return router.tokens <= (router.g.routed_experts <= 32u ? 32u : 16u) && router_is_small(router) && count <= 1024u && rank_schedule_fits(count, num_experts);
 }
 
 void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream) {

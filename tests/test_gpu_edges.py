@@ -155,7 +155,7 @@ def test_group_limited_routing(device, experts, n_group, topk_group, k, activati
 # the last batch that is routed and scheduled in one launch and the first that is not; fewer warps of routes than of
 # tokens and the other way round; one and four experts a lane; an expert count beyond it
 @pytest.mark.parametrize("name,experts,tokens", [("gpt-oss-20b", 32, 1), ("gpt-oss-20b", 33, 9), ("gpt-oss-20b", 128, 17),
-                                                 ("gpt-oss-20b", 128, 16), ("tiny", 8, 16),
+                                                 ("gpt-oss-20b", 128, 16), ("gpt-oss-20b", 33, 16), ("gpt-oss-20b", 33, 17),
                                                  ("gpt-oss-20b", 16, 32), ("gpt-oss-20b", 16, 33), ("tiny", 8, 32),
                                                  ("gpt-oss-20b", 129, 8)])
 def test_layer_routes_equal_the_router_node(device, name, experts, tokens):
