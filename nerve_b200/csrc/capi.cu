@@ -112,6 +112,7 @@ struct ExpertSet {
     }
 };
 constexpr size_t kMaxExpertSets = 64;
+constexpr size_t kMapTemplates = 5u * 128u;  // bytes of a stage's template tensor maps
 constexpr int kHostWaitSeconds = 60;  // how long the host-buffer layer call waits for its result
 
 enum Stage { kStageLinear, kStageRoute, kStageSchedule, kStageQuantX, kStageGateUp, kStageQuantI, kStageDown, kStageReduce, kStageCount };
@@ -129,9 +130,9 @@ struct nvmoe_plan {
     DeviceArray status, grouped[2], offsets[2], block_hist, bucket_totals;
     std::vector<std::unique_ptr<ExpertSet>> sets[2];  // [gate/up, down], least recently used replaced
     uint64_t use_clock = 0;
-    DeviceArray xq, x_scales, x_e8m0, iq, i_scales, i_e8m0, tile_list, ep_source;
+    DeviceArray xq, x_scales, iq, i_scales, tile_list, ep_source;
     // tensor path: expert-grouped quantised activations of the two stages (row = position in grouped[stage]),
-    // where each route landed, and the tensor maps of the two matrices for the four token tile sizes
+    // where each route landed, and the tensor maps of the operands for the token tile sizes
     DeviceArray grouped_q[2], grouped_e8m0[2], position[2], act_maps;
     DeviceArray cta_trace;       // per-CTA diagnostics of the tensor-path kernels, allocated on first request
     DeviceArray tmap_templates;  // tensor maps of the two weight matrix shapes; each expert's map is one with its address patched in
@@ -166,6 +167,22 @@ namespace {
 size_t tile_region_words(const nvmoe_plan* p) {
     const size_t list = (size_t)p->g.max_tokens * p->K / 16u + p->experts + 1u;
     return (64u + list + 63u) / 64u * 64u;
+}
+
+// Rows that the scale arrays of the expert-grouped operands hold per K block: whole 16-byte pieces.
+uint32_t scale_rows(const nvmoe_plan* p) { return (p->g.max_tokens * p->K + 3u) & ~3u; }
+
+// Token tile of a stage for T tokens.
+TokenTile token_tile(const nvmoe_plan* p, bool gate_up, uint32_t T) {
+    return tc_token_tile_for(T, p->K, p->experts, gate_up ? p->g.intermediate_size : p->g.hidden_size, gate_up, p->tma[gate_up ? 0 : 1]);
+}
+
+// The scales of a stage's operands in a call of T tokens.
+ScaleWords scale_words(const nvmoe_plan* p, bool gate_up, uint32_t T) {
+    const int set = gate_up ? 0 : 1;
+    const uint32_t blocks = ((gate_up ? p->g.hidden_size : p->g.intermediate_size) + 127u) / 128u;
+    uint32_t* words = p->grouped_e8m0[set].as<uint32_t>();
+    return token_tile(p, gate_up, T).pair ? ScaleWords{words, 1u, scale_rows(p)} : ScaleWords{words, blocks, 1u};
 }
 
 size_t scratch_blocks(const nvmoe_plan* p) { return ((size_t)p->g.max_tokens * p->K + kSortChunk - 1u) / kSortChunk; }
@@ -482,27 +499,30 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
     want(p->bucket_totals, sizeof(uint32_t) * (p->experts + 2u));
     want(p->xq, T * H);
     want(p->x_scales, sizeof(float) * T * (H / g.act_block));
-    want(p->x_e8m0, sizeof(uint32_t) * T * ((H + 127u) / 128u));
     want(p->iq, R * I);
     want(p->i_scales, sizeof(float) * R * (I / g.act_block));
-    want(p->i_e8m0, sizeof(uint32_t) * R * ((I + 127u) / 128u));
     want(p->tile_list, sizeof(uint32_t) * 2u * tile_region_words(p));
     want(p->position[0], sizeof(uint32_t) * R);
     want(p->position[1], sizeof(uint32_t) * R);
     if (tc_shape_supported(g)) {
         want(p->grouped_q[0], R * H);
         want(p->grouped_q[1], R * I);
-        want(p->grouped_e8m0[0], sizeof(uint32_t) * R * ((H + 127u) / 128u));
-        want(p->grouped_e8m0[1], sizeof(uint32_t) * R * ((I + 127u) / 128u));
-        want(p->act_maps, 10u * 128u);
+        want(p->grouped_e8m0[0], sizeof(uint32_t) * scale_rows(p) * ((H + 127u) / 128u));
+        want(p->grouped_e8m0[1], sizeof(uint32_t) * scale_rows(p) * ((I + 127u) / 128u));
+        want(p->act_maps, 2u * kActMaps * 128u);
         if (err == cudaSuccess) {
-            unsigned char maps[10 * 128];
-            const uint32_t token_tiles[5] = {16u, 32u, 64u, 96u, 128u};
+            unsigned char maps[2u * kActMaps * 128u] = {0};
             bool ok = true;
-            for (uint32_t set = 0; set < 2u && ok; set++)
-                for (uint32_t i = 0; i < 5u && ok; i++)
-                    ok = tc_encode_activation_map(maps + (set * 5u + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R,
-                                                  (uint32_t)(set == 0u ? H : I), token_tiles[i]);
+            for (uint32_t set = 0; set < 2u && ok; set++) {
+                const uint32_t cols = (uint32_t)(set == 0u ? H : I);
+                unsigned char* mine = maps + set * kActMaps * 128u;
+                for (uint32_t i = 0; i < kTokenMaps && ok; i++)
+                    ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
+                if (cols % 64u != 0u || cols < 128u) continue;  // (no map for its weights either)
+                for (uint32_t i = 0; i < 4u && ok; i++)
+                    ok = tc_encode_pair_token_map(mine + (kPairTokenMap + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[1u + i]);
+                ok = ok && tc_encode_token_scale_map(mine + kTokenScaleMap * 128u, p->grouped_e8m0[set].ptr, scale_rows(p), (cols + 127u) / 128u);
+            }
             if (ok) {
                 err = cudaMemcpyAsync(p->act_maps.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
                 if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
@@ -510,17 +530,23 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
                 p->act_maps.release();  // no tensor maps on this system: the tensor path copies with cp.async
             }
         }
-        want(p->tmap_templates, 512);
+        want(p->tmap_templates, 2u * kMapTemplates);
         if (err == cudaSuccess) {
-            // per stage: the map of the compact form, then the map of the one-byte-per-element forms (left zero
-            // when the shape has no whole 128-column blocks: such resources are then treated as not resident)
-            unsigned char maps[512] = {0};
-            p->tma[0] = tc_encode_weight_map(maps, p->tmap_templates.ptr, g.intermediate_size, g.hidden_size);
-            p->tma[1] = tc_encode_weight_map(maps + 256, p->tmap_templates.ptr, g.hidden_size, g.intermediate_size);
-            tc_encode_weight_map_bytes(maps + 128, p->tmap_templates.ptr, g.intermediate_size, g.hidden_size);
-            tc_encode_weight_map_bytes(maps + 384, p->tmap_templates.ptr, g.hidden_size, g.intermediate_size);
-            if (!p->act_maps.ptr) p->tma[0] = p->tma[1] = false;
-            err = cudaMemcpyAsync(p->tmap_templates.ptr, maps, 512, cudaMemcpyHostToDevice, d->stream);
+            // per stage: the maps of the compact form (boxes of one K block, of two), those of the one-byte-per-element forms (left
+            // zero when the shape has no whole 128-column blocks: such resources are then treated as not resident), the map
+            // of the derived scales
+            unsigned char maps[2u * kMapTemplates] = {0};
+            for (uint32_t set = 0; set < 2u; set++) {
+                const uint32_t rows = set == 0u ? g.intermediate_size : g.hidden_size, cols = set == 0u ? g.hidden_size : g.intermediate_size;
+                unsigned char* mine = maps + set * kMapTemplates;
+                const uint64_t blocks = tc_derived_scale_bytes(rows, cols) / 512u * p->experts;
+                p->tma[set] = p->act_maps.ptr && tc_encode_weight_map(mine, p->tmap_templates.ptr, rows, cols) &&
+                              tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false) && blocks <= 0x7fffffffull &&
+                              tc_encode_pair_scale_map(mine + 512, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks);
+                tc_encode_weight_map_bytes(mine + 256, p->tmap_templates.ptr, rows, cols);
+                tc_encode_pair_weight_map(mine + 384, p->tmap_templates.ptr, rows, cols, true);
+            }
+            err = cudaMemcpyAsync(p->tmap_templates.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
             if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
         }
     }
@@ -551,8 +577,8 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
     for (auto& stage_sets : p->sets)
         for (auto& es : stage_sets) es->release();
     DeviceArray* all[] = {&p->status, &p->grouped[0], &p->grouped[1], &p->offsets[0],
-                          &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->x_e8m0, &p->iq,
-                          &p->i_scales, &p->i_e8m0, &p->tile_list, &p->ep_source, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
+                          &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->iq,
+                          &p->i_scales, &p->tile_list, &p->ep_source, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
                           &p->controls, &p->hidden_dev, &p->output_dev};
     for (DeviceArray* a : all) a->release();
@@ -715,7 +741,7 @@ int nvmoe_quantize_fp8(nvmoe_plan* p, uint32_t rows, uint32_t columns, const nvm
     NVMOE_TRY(check_buffer(p, scales, (size_t)rows * (columns / block) * 4u, "scales"));
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     launch_quantize((const uint16_t*)input->ptr, rows, columns, block, columns, (uint8_t*)quantized->ptr,
-                    (float*)scales->ptr, nullptr, p->device->stream);
+                    (float*)scales->ptr, p->device->stream);
     p->launches++;
     return post_launch(p, "quantize");
 }
@@ -759,7 +785,7 @@ static int expert_set_for(nvmoe_plan* p, int set, const nvmoe_buffer* addresses,
                                            : tc_derived_scale_bytes(g.hidden_size, g.intermediate_size);
         NVMOE_CUDA(p->device, found->derived.ensure((size_t)p->experts * matrices * per_matrix));
         NVMOE_CUDA(p->device, found->stamps.ensure((size_t)p->experts * matrices * 16u));
-        NVMOE_CUDA(p->device, found->tmaps.ensure((size_t)p->experts * matrices * 128u));
+        NVMOE_CUDA(p->device, found->tmaps.ensure((size_t)p->experts * matrices * 256u + 128u));
         NVMOE_CUDA(p->device, cudaMemsetAsync(found->stamps.ptr, 0, found->stamps.bytes, p->device->stream));
         found->resolved = found->tensor_ready = false;  // the resolved pointers name the derived copies
     }
@@ -794,11 +820,12 @@ static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* a
         el.work = GroupedWork{nullptr, nullptr, es->ptrs.as<ExpertPtrs>(), p->experts};
         el.scale_stamps = es->stamps.as<uint64_t>();
         el.tmaps = p->tma[set] ? es->tmaps.as<uint8_t>() : nullptr;
+        el.scale_base = es->derived.as<uint8_t>();
         el.g = g;
         launch_derive_scales_tc(el, gate_up, st);
         p->launches += 2;
         if (el.tmaps) {
-            launch_build_tensormaps_tc(el, gate_up, p->tmap_templates.as<uint8_t>() + set * 256, st);
+            launch_build_tensormaps_tc(el, gate_up, p->tmap_templates.as<uint8_t>() + set * kMapTemplates, st);
             p->launches++;
         }
         es->tensor_ready = es->cacheable;
@@ -814,8 +841,7 @@ static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T
     const int set = gate_up ? 0 : 1;
     cudaStream_t st = p->device->stream;
     uint32_t* region = p->tile_list.as<uint32_t>() + set * tile_region_words(p);
-    const uint32_t rows = gate_up ? p->g.intermediate_size : p->g.hidden_size;
-    const TileOut tiles{tensor ? region + 64 : nullptr, region, tc_token_tile_for(T, p->K, p->experts, rows, gate_up)};
+    const TileOut tiles{tensor ? region + 64 : nullptr, region, token_tile(p, gate_up, T).rows};
     p->launches += launch_group_slots(routes, intermediates, control, es->ptrs.as<ExpertPtrs>(), p->experts, T, p->K,
                                       p->g.intermediate_size, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(),
                                       p->position[set].as<uint32_t>(), tiles, p->status.as<uint32_t>(), sort_scratch(p), st);
@@ -834,22 +860,22 @@ static int quantise_operands(nvmoe_plan* p, bool gate_up, uint32_t T, const void
     const nvmoe_geometry& g = p->g;
     const int set = gate_up ? 0 : 1;
     cudaStream_t st = p->device->stream;
-    const DownRows down{fused ? p->position[1].as<uint32_t>() : nullptr, p->grouped_q[1].as<uint8_t>(), p->grouped_e8m0[1].as<uint32_t>(),
+    const DownRows down{fused ? p->position[1].as<uint32_t>() : nullptr, p->grouped_q[1].as<uint8_t>(), scale_words(p, false, T),
                         g.intermediate_size};
     const uint32_t* written = !gate_up && whole_call ? p->position[0].as<uint32_t>() : nullptr;
     if (tensor && gate_up && whole_call &&
         launch_quantize_tokens(source, p->position[0].as<uint32_t>(), T, p->K, g.hidden_size, g.act_block, p->grouped_q[0].as<uint8_t>(),
-                               p->grouped_e8m0[0].as<uint32_t>(), down, st)) {
+                               scale_words(p, true, T), down, st)) {
     } else if (tensor) {
         launch_quantize_grouped(source, !gate_up, p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), p->experts,
                                 T * p->K, p->K, gate_up ? g.hidden_size : g.intermediate_size, g.intermediate_size,
-                                g.act_block, p->grouped_q[set].as<uint8_t>(), p->grouped_e8m0[set].as<uint32_t>(), written, st);
+                                g.act_block, p->grouped_q[set].as<uint8_t>(), scale_words(p, gate_up, T), written, st);
     } else if (gate_up) {
         launch_quantize((const uint16_t*)source, T, g.hidden_size, g.act_block, g.hidden_size, p->xq.as<uint8_t>(),
-                        p->x_scales.as<float>(), p->x_e8m0.as<uint32_t>(), st);
+                        p->x_scales.as<float>(), st);
     } else {
         launch_quantize_frames((const uint32_t*)source, T, p->K, g.intermediate_size, g.act_block, p->iq.as<uint8_t>(),
-                               p->i_scales.as<float>(), p->i_e8m0.as<uint32_t>(), written, st);
+                               p->i_scales.as<float>(), written, st);
     }
     p->launches++;
     return post_launch(p, gate_up ? "quantize hidden" : "quantize intermediates");
@@ -890,14 +916,13 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     el.work = GroupedWork{p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), es->ptrs.as<ExpertPtrs>(), p->experts};
     if (tensor) {
         el.act_q = p->grouped_q[set].as<uint8_t>();
-        el.act_e8m0 = p->grouped_e8m0[set].as<uint32_t>();
+        el.act_e8m0 = scale_words(p, gate_up, T);
     } else if (c.pre_q) {
         el.act_q = c.pre_q;
         el.act_scales = c.pre_scales;
     } else {
         el.act_q = (gate_up ? p->xq : p->iq).as<uint8_t>();
         el.act_scales = (gate_up ? p->x_scales : p->i_scales).as<float>();
-        el.act_e8m0 = (gate_up ? p->x_e8m0 : p->i_e8m0).as<uint32_t>();
     }
     el.routes = c.routes;
     el.intermediates = c.intermediates;
@@ -914,12 +939,13 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     el.wait_cycles = p->wait_cycles;
     el.debug_flags = p->debug_flags;
     if (tensor) {
-        const uint32_t size_index = tc_token_tile_index(
-            tc_token_tile_for(T, p->K, p->experts, gate_up ? g.intermediate_size : g.hidden_size, gate_up));
-        el.act_tmap = el.tmaps ? p->act_maps.as<uint8_t>() + (set * 5u + size_index) * 128u : nullptr;
+        const TokenTile tile = token_tile(p, gate_up, T);
+        el.token_rows = tile.rows;
+        el.pairs = tile.pair;
+        el.act_tmap = el.tmaps ? p->act_maps.as<uint8_t>() + (set * kActMaps + tc_token_map_for(tile)) * 128u : nullptr;
         if (c.fuse_quantise && gate_up) {
             el.q_out = p->grouped_q[1].as<uint8_t>();
-            el.q_e8m0 = p->grouped_e8m0[1].as<uint32_t>();
+            el.q_e8m0 = scale_words(p, false, T);
             el.down_position = p->position[1].as<uint32_t>();
             el.intermediates = nullptr;  // the down stage reads the codes only
         }
@@ -1224,12 +1250,20 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         int rc = NVMOE_OK;
         const bool tensor_shape = tc_shape_supported(g);
         if (fresh.unit_routes.ensure((size_t)g.max_tokens * 4u) != cudaSuccess || fresh.set.ptrs.ensure(sizeof(ExpertPtrs)) != cudaSuccess ||
-            (tensor_shape && (fresh.set.derived.ensure(tc_derived_scale_bytes(rows, cols)) != cudaSuccess || fresh.set.tmaps.ensure(128u) != cudaSuccess)))
+            (tensor_shape && (fresh.set.derived.ensure(tc_derived_scale_bytes(rows, cols)) != cudaSuccess || fresh.set.tmaps.ensure(384u) != cudaSuccess)))
             rc = fail(d, NVMOE_ERR_OUT_OF_MEMORY, "dense linear: out of device memory");
         if (rc == NVMOE_OK) {
             std::vector<uint32_t> ones(g.max_tokens, 0x3f80u << 16);  // weight 1.0, resource 0
             if (cudaMemcpy(fresh.unit_routes.ptr, ones.data(), ones.size() * 4u, cudaMemcpyHostToDevice) != cudaSuccess)
                 rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the unit routes");
+            // the map of the derived scales stays (the matrix's own maps, before it, are made by every call)
+            unsigned char map[128];
+            if (fresh.plan->tma[1]) {
+                if (!tc_encode_pair_scale_map(map, fresh.set.derived.ptr, 1u, (uint32_t)(tc_derived_scale_bytes(rows, cols) / 512u)))
+                    fresh.plan->tma[1] = false;
+                else if (cudaMemcpy(fresh.set.tmaps.as<uint8_t>() + 256, map, 128, cudaMemcpyHostToDevice) != cudaSuccess)
+                    rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the scale map");
+            }
         }
         if (rc != NVMOE_OK) {
             nvmoe_plan_destroy(fresh.plan);
@@ -1256,24 +1290,23 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     dp.offsets = sub->offsets[1].as<uint32_t>();
     dp.ptrs = dl->set.ptrs.as<ExpertPtrs>();
     if (tensor) {
-        dp.tiles = TileOut{region + 64, region, tc_token_tile_for(T, 1u, 1u, rows, false)};
+        dp.tiles = TileOut{region + 64, region, token_tile(sub, false, T).rows};
         dp.derived = dl->set.derived.as<uint8_t>();
-        dp.map_template = sub->tma[1] ? sub->tmap_templates.as<uint8_t>() + 256 : nullptr;
+        dp.map_template = sub->tma[1] ? sub->tmap_templates.as<uint8_t>() + kMapTemplates : nullptr;
         dp.map = dl->set.tmaps.as<uint8_t>();
     }
     dp.input = (const uint16_t*)input->ptr;
     dp.q = sub->grouped_q[1].as<uint8_t>();
-    dp.q_e8m0 = sub->grouped_e8m0[1].as<uint32_t>();
+    dp.q_e8m0 = scale_words(sub, false, T);
     const bool quantised = launch_dense_prepare(dp, sub->g.act_block, st);
     sub->launches++;
     NVMOE_TRY(post_launch(sub, "dense linear operands"));
     if (!quantised) {
         if (tensor) {
             launch_quantize_grouped(input->ptr, false, dp.grouped, dp.offsets, 1u, T, 1u, cols, cols, sub->g.act_block, dp.q, dp.q_e8m0,
-                                    nullptr, st);
+                                nullptr, st);
         } else {
-            launch_quantize(dp.input, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(),
-                            sub->i_e8m0.as<uint32_t>(), st);
+            launch_quantize(dp.input, T, cols, sub->g.act_block, cols, sub->iq.as<uint8_t>(), sub->i_scales.as<float>(), st);
         }
         sub->launches++;
         NVMOE_TRY(post_launch(sub, "dense linear quantise"));
@@ -1455,8 +1488,8 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         ls.tiles_per_route[0] = (g.intermediate_size + g.gate_tile_rows - 1u) / g.gate_tile_rows;
         ls.tiles_per_route[1] = (g.hidden_size + g.down_tile_rows - 1u) / g.down_tile_rows;
         ls.num_experts = p->experts;
-        ls.n_tile[0] = tc_token_tile_for(T, p->K, p->experts, g.intermediate_size, true);
-        ls.n_tile[1] = tc_token_tile_for(T, p->K, p->experts, g.hidden_size, false);
+        ls.n_tile[0] = token_tile(p, true, T).rows;
+        ls.n_tile[1] = token_tile(p, false, T).rows;
         if (routes_in_schedule) {
             launch_route_schedule(router, ls, st);
             p->launches++;

@@ -63,6 +63,20 @@ struct ExpertPtrs {
     uint32_t reserved;
 };
 
+// The E8M0 scales of an operand matrix: a word of four bytes per row and K block of 128 columns. The words of a row lie side
+// by side for the kernels of one CTA (a row's next word is then in the cache when its next K block is fetched) and those of a
+// K block for CTA pairs (the scales of a token tile are then one copy).
+struct ScaleWords {
+    uint32_t* words;
+    uint32_t row_stride, block_stride;
+    __device__ __forceinline__ uint32_t* at(uint32_t row, uint32_t block) const {
+        return words + (size_t)row * row_stride + (size_t)block * block_stride;
+    }
+    __device__ __forceinline__ uint8_t* byte_at(uint32_t row, uint32_t group) const {  // of columns 32 group ..
+        return reinterpret_cast<uint8_t*>(at(row, group / 4u)) + group % 4u;
+    }
+};
+
 // Everything a grouped expert kernel needs to find its work, produced by group_slots().
 struct GroupedWork {
     const uint32_t* grouped_routes;   // route indices (t*K + r) sorted by expert, stable
@@ -182,11 +196,9 @@ void launch_ep_unpack(const uint16_t* returned_rows, const uint32_t* send_index,
                       uint32_t hidden_size, uint16_t* expert_outputs, cudaStream_t stream);
 
 // quantize.cu: bf16 rows -> E4M3 bytes + per-block power-of-two scales.
-// scales_f32 ([rows][cols/block]) and scales_e8m0 ([rows][ceil(cols/128)] words, four E8M0 bytes of
-// consecutive 32-column blocks per word) are both optional.
+// scales_f32 is [rows][cols/block].
 void launch_quantize(const uint16_t* input, uint32_t rows, uint32_t cols, uint32_t block,
-                     size_t input_row_stride, uint8_t* q, float* scales_f32, uint32_t* scales_e8m0,
-                     cudaStream_t stream);
+                     size_t input_row_stride, uint8_t* q, float* scales_f32, cudaStream_t stream);
 // The tensor path's operand form: row `pos` of the output is the quantised source row of route
 // grouped_routes[pos] (the token's hidden row when frames is false: source row = route / K of
 // `input` with `cols` columns; the route's own row of the intermediates frames otherwise), for pos below
@@ -196,7 +208,7 @@ void launch_quantize(const uint16_t* input, uint32_t rows, uint32_t cols, uint32
 void launch_quantize_grouped(const void* input, bool frames, const uint32_t* grouped_routes,
                              const uint32_t* expert_offsets, uint32_t num_experts, uint32_t max_routes, uint32_t K,
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
-                             uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream);
+                             const ScaleWords& scales, const uint32_t* written, cudaStream_t stream);
 // The same gate/up operands from the inverse list: position[token * K + r] = row of that route (0xffffffff: skipped),
 // valid for every route of the call. `down` (position null: nothing) names the down stage's operand rows, of which those
 // of routes that only the down stage keeps are set to zero. False when the shape needs the form above (blocks other than
@@ -204,39 +216,40 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
 struct DownRows {
     const uint32_t* position;
     uint8_t* q;
-    uint32_t* scales_e8m0;
+    ScaleWords scales;
     uint32_t cols;
 };
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
-                            uint8_t* q, uint32_t* scales_e8m0, const DownRows& down, cudaStream_t stream);
+                            uint8_t* q, const ScaleWords& scales, const DownRows& down, cudaStream_t stream);
 // the same for the K rows of every intermediates frame (skips the schedule words)
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K,
                             uint32_t intermediate_size, uint32_t block, uint8_t* q, float* scales_f32,
-                            uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream);
-// f32 scales -> packed E8M0 words, for prequantised inputs; sets *not_pow2 if a scale is not a power of two
-void launch_scales_to_e8m0(const float* scales, uint32_t rows, uint32_t cols, uint32_t block,
-                           uint32_t* scales_e8m0, uint32_t* status, cudaStream_t stream);
-
+                            const uint32_t* written, cudaStream_t stream);
 struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     GroupedWork work;
     const uint8_t* act_q;        // [rows][K_dim] E4M3; row = token (gate/up) or route index (down)
     const float* act_scales;     // [rows][K_dim/act_block] f32
-    const uint32_t* act_e8m0;    // [rows][ceil(K_dim/128)] packed E8M0 (tensor path)
+    ScaleWords act_e8m0;         // packed E8M0 (tensor path)
     const uint32_t* routes;      // route words (down: weights)
     uint32_t* intermediates;     // gate/up output frames (tensor path with q_out: may be null)
     uint16_t* outputs;           // down output [T][K][H]
     float* partial_outputs;      // down, tensor-parallel form: raw f32 sums [T][K][H] instead of `outputs` (no route weight, no rounding)
     uint32_t* status;
-    const uint8_t* tmaps;        // tensor path: 128-byte tensor maps [expert][matrix], null = move weights with cp.async
+    const uint8_t* tmaps;        // tensor path: tensor maps [expert][matrix][boxes of one K block, of two][128 bytes], then that of
+                                 // the derived scales; null = move weights with cp.async
     // tensor path: act_q / act_e8m0 hold expert-grouped rows (row = position in grouped_routes);
-    // act_tmap is the tensor map of act_q with a box of [token tile][128 bytes] (null: fetch rows with cp.async)
+    // act_tmap is the tensor map of act_q with a box of [token tile][128 bytes] (null: fetch rows with cp.async); for CTA
+    // pairs the first of those of half tiles
     const uint8_t* act_tmap;
     // tensor path, gate/up only: where the down stage's grouping puts each route (its operand row)
     const uint32_t* down_position;
     // tensor path, gate/up only, optional: the down stage's activation quantisation done in the epilogue
-    // (E4M3 bytes [down_position][I], E8M0 bytes [down_position][ceil(I/128)] words); needs act_block 32 or 128
+    // (E4M3 bytes [down_position][I] and their scales); needs act_block 32 or 128
     uint8_t* q_out;
-    uint32_t* q_e8m0;
+    ScaleWords q_e8m0;
+    uint32_t token_rows;         // tensor path: rows of the operand matrix per token tile of the list
+    bool pairs;                  // tensor path: by CTA pairs
+    uint8_t* scale_base;         // tensor path: the derived scale copy of the whole expert set
     uint64_t* cta_trace;         // tensor path diagnostics: [2][grid][4] words per CTA, or null
     uint64_t* scale_stamps;      // tensor path: {scale pointer, generation} the derived tiles were built from
     uint32_t* tile_list;         // tensor path scratch: routes / 16 + experts + 1 words

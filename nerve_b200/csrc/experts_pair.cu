@@ -1,0 +1,581 @@
+// The grouped expert projections by CTA pairs (tcgen05 cta_group::2), for calls with many tokens per expert.
+//
+// Arithmetic, operands and results are those of experts_tc.cu. What differs is the tile: two CTAs of a cluster work on one
+// D[256 weight rows x up to 240 tokens], each with 128 of the rows and half of the tokens in its shared memory; the tensor
+// cores of both read the other's token rows through the pair. What bounds the one-CTA kernel with large batches is its
+// shared memory: for 256 rows x 128 tokens x 128 columns the MMAs read 64 KB and the copies write 48 KB (the 4-bit codes take
+// a byte each), 900 cycles at 128 bytes a clock beside 512 cycles of MMAs. A CTA of a pair does the same work with 32 KB
+// read and 32 KB written, and fetches 25 KB from L2 instead of 33.5.
+//
+// Gate/up: CTA 0 holds gate rows, CTA 1 the up rows of the same index; each takes half of the tokens through the activation
+// and sends the other half of its accumulators, rounded to bf16 as the activation reads them, to the other CTA's shared
+// memory. Down: the CTAs hold neighbouring 128-row tiles and have nothing to exchange.
+//
+// 240 columns: two accumulators of them and two sets of scales are 504 of the 512 columns of tensor memory. (256 columns,
+// with accumulators that share some, stop the MMAs at the end of every tile until the shared columns have been read.) A tile
+// with fewer tokens runs with 64, 128 or 192 columns.
+//
+// A stage is two K blocks, four copies: with one block a stage the lane that issues them and the one that issues the MMAs take
+// longer for a stage than the tensor cores. All operands come by TMA, a trailing half K block too (a stage of its own: a
+// whole block that ends with the row, of which only the second half is multiplied), credited to the barrier of CTA 0, whose
+// MMA thread feeds both. Only the token scales pass through
+// a warp: they lie as [K block][row], a tile's start at any row, and the 32 x 16-byte block that tcgen05.cp expands wants
+// four tokens, 32 apart, side by side; a warp of either CTA puts them there, in place, and arrives at CTA 0. All waits are
+// bounded (tcgen05.cuh); a CTA leaves only when both are done.
+#include <cuda_fp8.h>
+
+#include "experts_device.cuh"
+#include "experts_tc.cuh"
+#include "quantize.cuh"
+#include "tcgen05.cuh"
+
+namespace nvmoe {
+namespace {
+
+using namespace tc;
+
+constexpr uint32_t kPairEpilogueGroups = 4u;                            // of four warps, one per quadrant of tensor-memory lanes
+constexpr uint32_t kPairEpilogueWarps = 4u * kPairEpilogueGroups;
+constexpr uint32_t kPairMmaWarp = kPairEpilogueWarps, kPairTmaWarp = kPairMmaWarp + 1u, kPairInfoWarp = kPairTmaWarp + 1u;
+constexpr uint32_t kPairScaleWarp = kPairInfoWarp + 1u;
+constexpr uint32_t kPairThreads = 32u * (kPairScaleWarp + 1u);
+constexpr uint32_t kPairWatchWarp = 2u;                                 // polls for a finished accumulator (shares no scheduler with MMA and TMA)
+constexpr uint32_t kPairColumns = kPairTokens;
+constexpr uint32_t kPairStages = 3u;
+constexpr uint32_t kPairBlocks = 2u;                                     // K blocks a stage
+constexpr uint32_t kPairTokenBytes = kPairColumns / 2u * 128u;          // token rows of one K block in one CTA
+// a stage's weight scales, then its token scales: as they come, 244 words a K block, then as two blocks of 512 bytes each
+constexpr uint32_t kPairScaleBytes = kPairBlocks * 3u * kScaleBlockBytes;
+constexpr uint32_t kPairScaleWords = kPairTokens + 4u;
+static_assert(kPairTokenBytes % 1024u == 0u, "operand tiles keep their alignment");
+constexpr uint32_t kPairScaleColumn = 2u * kPairColumns, kPairScaleColumns = 12u;  // of either set: 4 for the weights, 8 for the tokens
+constexpr uint32_t kPairTmemColumns = 512u;
+static_assert(kPairScaleColumn + 2u * kPairScaleColumns <= kPairTmemColumns, "tensor memory");
+
+struct PairBarriers {
+    uint64_t full[kPairStages];    // CTA 0's count
+    uint64_t empty[kPairStages];
+    uint64_t staged[kPairStages];  // the token scales of a slot are there, as they lie in memory
+    uint64_t acc_full[2];
+    uint64_t acc_empty[2];         // CTA 0's
+    uint64_t info_full[2];         // what the epilogue has to know of a tile is there
+    uint64_t info_empty[2];
+    uint64_t drain;
+    uint64_t sent[kPairEpilogueWarps];    // the other CTA's warp has written its chunk
+    uint64_t taken[kPairEpilogueWarps];   // ... has read the chunk this warp sent
+    uint32_t tmem_base;
+    uint32_t abort;
+    uint32_t stage_info[kPairStages];     // of the tile whose operands a slot holds: format << 16 | first row % 4 << 12 | columns
+    uint32_t acc_ready[2];
+    // per tile, alternating: its tokens, its row tile, and per column the route (0xffffffff: no token) with its down row
+    // (gate/up) or its weight (down)
+    uint32_t tile_tokens[2], tile_rows[2];
+    __align__(16) uint32_t route[2][256];
+    __align__(16) uint32_t extra[2][256];
+    uint32_t maxima[kPairEpilogueGroups][2][4][8];  // [group][chunk, alternating][lane quadrant][tokens in pairs], bf16
+};
+constexpr uint32_t kPairExchangeBytes = kPairEpilogueWarps * 1024u;     // 16 columns x 32 rows of bf16 a warp
+constexpr uint32_t kPairTokenRegion = kPairStages * kPairBlocks * kATileBytes;
+constexpr uint32_t kPairScaleRegion = kPairTokenRegion + kPairStages * kPairBlocks * kPairTokenBytes;
+constexpr uint32_t kPairExchangeRegion = kPairScaleRegion + kPairStages * kPairScaleBytes;
+constexpr uint32_t kPairBarrierRegion = kPairExchangeRegion + kPairExchangeBytes;
+constexpr uint32_t kPairSmemBytes = kPairBarrierRegion + sizeof(PairBarriers) + 1024u;  // (the round-up to a 1024-byte boundary)
+static_assert(kPairSmemBytes <= 227u * 1024u && kPairBarrierRegion % 128u == 0u, "shared memory");
+
+__device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {  // (the number where the other is none)
+    const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float low_bf16(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float high_bf16(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+
+// columns an MMA takes for a tile of that many tokens, and which of the token rows' tensor maps fetches half of them
+__device__ __forceinline__ uint32_t columns_for(uint32_t tokens) { return tokens <= 64u ? 64u : tokens <= 128u ? 128u : tokens <= 192u ? 192u : kPairColumns; }
+
+template <bool GATE_UP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) experts_pair_kernel(ExpertLaunch p, TileList list) {
+    const long long wait_limit = p.wait_cycles;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
+    PairBarriers* bars = reinterpret_cast<PairBarriers*>(smem + kPairBarrierRegion);
+    volatile uint32_t* abort_flag = &bars->abort;
+
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t rank = cluster_rank();
+    const uint32_t pair_id = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const uint32_t H = p.g.hidden_size, I = p.g.intermediate_size;
+    const uint32_t K = p.g.routed_k + p.g.always_count;
+    const uint32_t k_dim = GATE_UP ? H : I;
+    const uint32_t out_rows = GATE_UP ? I : H;
+    const uint32_t k_blocks = (k_dim + kBlockK - 1u) / kBlockK;
+    const uint32_t row_tiles = (out_rows + kBlockM - 1u) / kBlockM;
+    // stages of a tile: two whole K blocks each, then a whole one and a trailing half one by themselves
+    const uint32_t doubles = k_dim / kBlockK / 2u, stages = doubles + (k_blocks - 2u * doubles);
+    const uint32_t m_tiles = GATE_UP ? row_tiles : (row_tiles + 1u) / 2u;
+    constexpr uint32_t kSources = GATE_UP ? 2u : 1u;
+
+    // ---- one-time setup ---------------------------------------------------------------------
+    if (threadIdx.x == 0u) {
+        for (uint32_t s = 0; s < kPairStages; s++) {
+            mbar_init(&bars->full[s], 3u);  // the announcement of the copies, the scale warps of both CTAs
+            mbar_init(&bars->empty[s], 1u);
+            mbar_init(&bars->staged[s], 1u);
+        }
+        for (uint32_t a = 0; a < 2u; a++) {
+            mbar_init(&bars->acc_full[a], 1u);
+            mbar_init(&bars->acc_empty[a], 2u * kPairEpilogueWarps);
+            mbar_init(&bars->info_full[a], 32u);
+            mbar_init(&bars->info_empty[a], kPairEpilogueWarps);
+        }
+        mbar_init(&bars->drain, 1u);
+        for (uint32_t w = 0; w < kPairEpilogueWarps; w++) {
+            mbar_init(&bars->sent[w], 1u);
+            mbar_init(&bars->taken[w], 1u);
+        }
+        bars->abort = 0u;
+        fence_mbar_init();
+    }
+    __syncwarp();
+    cluster_sync();  // the barriers of both CTAs are up before either arrives on the other's
+    if (warp == kPairMmaWarp) {
+        tmem_alloc_pair(&bars->tmem_base, kPairTmemColumns);
+        tmem_relinquish_pair();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = bars->tmem_base;
+    const uint32_t tmem_scales = tmem_base + kPairScaleColumn;
+    grid_dependency_sync();
+    const uint32_t tile_count = *list.count * m_tiles;
+    // (a tensor map written by an earlier kernel is acquired once per block before the TMA unit gets it)
+    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources + 1u; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u);
+    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u + 128u);
+    if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
+    __syncthreads();
+
+    // first row of a tile in the operand matrix, and how many rows it has
+    auto first_row_of = [&](uint32_t n_tile, uint32_t e_begin) { return e_begin + n_tile * p.token_rows; };
+
+    if (warp == kPairTmaWarp) {
+        // ===== TMA issue (one lane of each CTA) =====
+        if (lane == 0u) {
+            // the list entry of a tile is fetched two tiles ahead, what hangs on it one tile ahead (loads only: a thread
+            // stalls at the first instruction that needs a result)
+            struct Meta {
+                uint32_t pair, m_tile, e_begin, e_end, format;
+            };
+            auto entry_of = [&](uint32_t tile) { return tile < tile_count ? __ldg(list.tiles + tile / m_tiles) : 0u; };
+            auto meta_of = [&](uint32_t tile, uint32_t pair, Meta& m) {
+                m.pair = pair;
+                m.m_tile = tile % m_tiles;
+                m.e_begin = __ldg(p.work.expert_offsets + (pair >> 16));
+                m.e_end = __ldg(p.work.expert_offsets + (pair >> 16) + 1u);
+                m.format = p.work.experts[pair >> 16].format;
+            };
+            const uint64_t begin = p.cta_trace ? global_timer_ns() : 0u;
+            const uint32_t smem_base = smem_u32(smem), full0 = map_shared(smem_u32(&bars->full[0]), 0u);
+            const uint8_t* scale_map = p.tmaps + (size_t)p.work.num_experts * kSources * 256u;
+            const uint8_t* token_scale_map = p.act_tmap + (kTokenScaleMap - 1u) * 128u;
+            uint32_t slot = 0u, empty_parity = 1u, stage_it = 0u;
+            bool alive = true, withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
+            Meta cur{}, nxt{};
+            uint32_t pair_nxt = entry_of(pair_id + pairs);
+            if (pair_id < tile_count) meta_of(pair_id, entry_of(pair_id), cur);
+            for (uint32_t tile = pair_id; tile < tile_count && alive; tile += pairs) {
+                const uint32_t pair_nxt2 = entry_of(tile + 2u * pairs);
+                if (tile + pairs < tile_count) meta_of(tile + pairs, pair_nxt, nxt);
+                const uint32_t expert = cur.pair >> 16;
+                const uint32_t first = first_row_of(cur.pair & 0xffffu, cur.e_begin);
+                const uint32_t columns = columns_for(min(p.token_rows, cur.e_end - first));
+                const uint8_t* weight_map = p.tmaps + (size_t)(GATE_UP ? 2u * expert + rank : expert) * 256u;
+                const uint8_t* token_map = p.act_tmap + (columns - 1u) / 64u * 128u;
+                const int row0 = (int)(GATE_UP ? cur.m_tile * kBlockM : (2u * cur.m_tile + rank) * kBlockM);
+                // (a second tile past the last rows borrows the first's scale blocks: its weights arrive as zeros)
+                const uint32_t row_tile = GATE_UP ? cur.m_tile : min(2u * cur.m_tile + rank, row_tiles - 1u);
+                const int scale0 = (int)((expert * row_tiles + row_tile) * k_blocks), source = GATE_UP ? (int)rank : 0;
+                const int token_row = (int)(first + rank * columns / 2u);
+                const uint32_t box_bytes = cur.format == kFormatCompact ? kTmaBoxBytes : 2u * kTmaBoxBytes;
+                const uint32_t block_bytes = 2u * (box_bytes + columns / 2u * 128u);  // of both CTAs
+                const uint32_t info = (cur.format << 16) | (first & 3u) << 12 | columns;
+                for (uint32_t st = 0; st < stages; st++) {
+                    if (!mbar_wait(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
+                        alive = false;
+                        break;
+                    }
+                    const bool two = st < doubles;
+                    const uint32_t kb = two ? 2u * st : doubles + st;
+                    const uint32_t bar = full0 + slot * 8u;
+                    *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]) = info;
+                    if (!withhold) {
+                        const uint32_t a = smem_base + slot * kPairBlocks * kATileBytes;
+                        const uint32_t b = smem_base + kPairTokenRegion + slot * kPairBlocks * kPairTokenBytes;
+                        const uint32_t sf = smem_base + kPairScaleRegion + slot * kPairScaleBytes;
+                        mbar_arrive_expect_tx(&bars->staged[slot], kPairBlocks * kPairScaleWords * 4u);
+                        if (rank == 0u) mbar_arrive_expect_tx(&bars->full[slot], (two ? 2u * block_bytes : block_bytes) + 2u * kPairBlocks * kScaleBlockBytes);
+                        if (two) {
+                            tma_load_3d_pair(a, weight_map + 128u, 0, row0, (int)kb, bar);
+                            tma_load_3d_pair(b, token_map + (kPairTokenMap - 1u) * 128u, 0, token_row, (int)kb, bar);
+                        } else {
+                            // in units of 64 columns: a trailing half block ends with the row
+                            const uint32_t k64 = min(2u * kb, k_dim / 64u - 2u);
+                            tma_load_3d_pair(a, weight_map, 0, (int)k64, row0, bar);
+                            tma_load_2d_pair(b, token_map, (int)(k64 * 64u), token_row, bar);
+                        }
+                        // (of one block, too, the scales of two are fetched: zeros, or the next row tile's, that nothing uses)
+                        tma_load_3d_pair(sf, scale_map, 0, source, scale0 + (int)kb, bar);
+                        tma_load_2d(sf + kPairBlocks * kScaleBlockBytes, token_scale_map, (int)(first & ~3u), (int)kb, &bars->staged[slot]);
+                    }
+                    withhold = false;
+                    stage_it++;
+                    if (++slot == kPairStages) {
+                        slot = 0u;
+                        empty_parity ^= 1u;
+                    }
+                }
+                cur = nxt;
+                pair_nxt = pair_nxt2;
+            }
+            if (p.cta_trace) {  // per-CTA diagnostics: loop begin, loop end, stages, SM id
+                uint32_t smid;
+                asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+                uint64_t* mine = p.cta_trace + (size_t)((GATE_UP ? 0u : gridDim.x) + blockIdx.x) * 4u;
+                mine[0] = begin;
+                mine[1] = global_timer_ns();
+                mine[2] = stage_it;
+                mine[3] = smid;
+            }
+            if (!alive) {
+                // copies may still be on their way into either CTA's shared memory: wait, bounded, on the barriers of the last
+                // round (CTA 1 sees its scales land there, not its other copies, and waits out the time for those)
+                const uint32_t rounds = stage_it < kPairStages ? stage_it : kPairStages;
+                for (uint32_t back = 1u; back <= rounds; back++) {
+                    const uint32_t nth = stage_it - back;
+                    mbar_wait_winddown(&bars->full[nth % kPairStages], rank == 0u ? (nth / kPairStages) & 1u : 0u, kWinddownCycles / kPairStages);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kPairMmaWarp) {
+        // ===== MMA issue (one lane of CTA 0, for both) =====
+        if (rank == 0u && elect_one()) {
+            constexpr uint32_t kIdescCompact = idesc_mxf8f6f4(kFmtE2M1, kFmtE4M3, 2u * kBlockM, 0u);
+            constexpr uint32_t kIdescBytes = idesc_mxf8f6f4(kFmtE4M3, kFmtE4M3, 2u * kBlockM, 0u);
+            const uint32_t base = smem_u32(smem);
+            const uint64_t a_desc0 = desc_k_major_sw128(base);
+            const uint64_t b_desc0 = desc_k_major_sw128(base + kPairTokenRegion);
+            const uint64_t sf_desc0 = desc_scale_block(base + kPairScaleRegion);
+            const uint32_t tail_groups = (k_dim % kBlockK) / 32u;  // K steps of a trailing partial block, 0 = none
+            uint32_t acc_it = 0u, slot = 0u, full_parity = 0u;
+            bool alive = true;
+            for (uint32_t tile = pair_id; tile < tile_count && alive; tile += pairs, acc_it++) {
+                const uint32_t acc = acc_it & 1u;
+                if (!mbar_wait(&bars->acc_empty[acc], ((acc_it >> 1) & 1u) ^ 1u, abort_flag, wait_limit)) break;
+                const uint32_t d_tmem = tmem_base + acc * kPairColumns;
+                for (uint32_t st = 0; st < stages; st++) {
+                    if (!mbar_wait(&bars->full[slot], full_parity, abort_flag, wait_limit)) {
+                        alive = false;
+                        break;
+                    }
+                    const uint32_t info = *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]);
+                    const uint32_t columns = info & 0xfffu;
+                    tc_fence_after();
+                    const uint32_t idesc = ((info >> 16) == kFormatCompact ? kIdescCompact : kIdescBytes) | (columns >> 3) << 17;
+                    // (a trailing half block lies in the second half of its operand tiles; its scales come first in their words)
+                    const uint32_t groups = st + 1u == stages && tail_groups != 0u ? tail_groups : 4u;
+                    const uint32_t first = 2u * (4u - groups);  // a K step of 32 elements is two 16-byte units of the start address
+#pragma unroll
+                    for (uint32_t sub = 0; sub < kPairBlocks; sub++) {
+                        if (sub != 0u && st >= doubles) break;
+                        const uint32_t sfa = tmem_scales + sub * kPairScaleColumns, sfb = sfa + 4u;
+                        const uint64_t sf_desc = sf_desc0 + (uint64_t)(slot * (kPairScaleBytes >> 4));
+                        const uint64_t sfb_desc = sf_desc + (kPairBlocks + 2u * sub) * (kScaleBlockBytes >> 4);
+                        tc_copy_scales_pair(sfa, sf_desc + sub * (kScaleBlockBytes >> 4));
+                        tc_copy_scales_pair(sfb, sfb_desc);
+                        if (columns > 128u) tc_copy_scales_pair(sfb + 4u, sfb_desc + (kScaleBlockBytes >> 4));
+                        const uint64_t a_desc = a_desc0 + (uint64_t)((slot * kPairBlocks + sub) * (kATileBytes >> 4) + first);
+                        const uint64_t b_desc = b_desc0 + (uint64_t)(slot * kPairBlocks * (kPairTokenBytes >> 4) + sub * (columns << 2) + first);
+#pragma unroll
+                        for (uint32_t j = 0; j < 4u; j++) {
+                            if (j < groups)
+                                tc_mma_block_scaled_pair(d_tmem, a_desc + 2u * j, b_desc + 2u * j, idesc | (j << 4) | (j << 29), sfa, sfb,
+                                                         j == 0u && sub == 0u ? (st != 0u ? 1u : 0u) : 1u);
+                        }
+                    }
+                    tc_commit_pair_both(&bars->empty[slot]);
+                    if (++slot == kPairStages) {
+                        slot = 0u;
+                        full_parity ^= 1u;
+                    }
+                }
+                if (alive) tc_commit_pair_both(&bars->acc_full[acc]);
+            }
+            // (nothing may still be reading either CTA's shared memory or using tensor memory when they are released)
+            tc_commit_pair(&bars->drain);
+            mbar_wait_winddown(&bars->drain, 0u, kWinddownCycles);
+        }
+        __syncwarp();
+    } else if (warp == kPairScaleWarp) {
+        // ===== token scales: in place, from row order to the two 32 x 16-byte blocks =====
+        const uint32_t full0 = map_shared(smem_u32(&bars->full[0]), 0u);
+        uint32_t slot = 0u, parity = 0u;
+        bool alive = true;
+        for (uint32_t tile = pair_id; tile < tile_count && alive; tile += pairs) {
+            for (uint32_t st = 0; st < stages; st++) {
+                if (!mbar_wait_warp(&bars->staged[slot], parity, abort_flag, wait_limit)) {
+                    alive = false;
+                    break;
+                }
+                uint32_t* words = reinterpret_cast<uint32_t*>(smem + kPairScaleRegion + slot * kPairScaleBytes + kPairBlocks * kScaleBlockBytes);
+                const uint32_t info = *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]);
+                const volatile uint32_t* mine = words + ((info >> 12) & 3u) + lane;
+                uint32_t w[kPairBlocks][8];
+#pragma unroll
+                for (uint32_t sub = 0; sub < kPairBlocks; sub++) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; i++) w[sub][i] = mine[sub * kPairScaleWords + 32u * i];  // (past the columns: not multiplied with)
+                }
+                __syncwarp();
+#pragma unroll
+                for (uint32_t sub = 0; sub < kPairBlocks; sub++) {
+                    reinterpret_cast<uint4*>(words)[64u * sub + lane] = make_uint4(w[sub][0], w[sub][1], w[sub][2], w[sub][3]);
+                    reinterpret_cast<uint4*>(words)[64u * sub + 32u + lane] = make_uint4(w[sub][4], w[sub][5], w[sub][6], w[sub][7]);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0u) mbar_arrive_cluster(full0 + slot * 8u);
+                if (++slot == kPairStages) {
+                    slot = 0u;
+                    parity ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kPairInfoWarp) {
+        // ===== what the epilogue has to know of a tile: fetched a tile ahead, the chain of four dependent loads (list entry,
+        // expert offsets, route, its weight or row) would otherwise be the longest part of an epilogue =====
+        uint32_t acc_it = 0u;
+        for (uint32_t tile = pair_id; tile < tile_count; tile += pairs, acc_it++) {
+            const uint32_t buffer = acc_it & 1u;
+            const uint32_t pair = __ldg(list.tiles + tile / m_tiles), expert = pair >> 16;
+            const uint32_t first = first_row_of(pair & 0xffffu, __ldg(p.work.expert_offsets + expert));
+            const uint32_t tokens = min(p.token_rows, __ldg(p.work.expert_offsets + expert + 1u) - first);
+            uint32_t route[8], extra[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; i++) route[i] = 32u * i + lane < tokens ? __ldg(p.work.grouped_routes + first + 32u * i + lane) : kUnboundSlot;
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; i++) {
+                extra[i] = kUnboundSlot;
+                if (route[i] == kUnboundSlot) continue;
+                if (GATE_UP) {
+                    if (p.q_out != nullptr) extra[i] = __ldg(p.down_position + route[i]);
+                } else {
+                    extra[i] = __ldg(p.routes + route[i]) & 0xffff0000u;  // the bf16 weight as f32
+                }
+            }
+            if (!mbar_wait_warp(&bars->info_empty[buffer], ((acc_it >> 1) & 1u) ^ 1u, abort_flag, wait_limit)) break;
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; i++) {
+                bars->route[buffer][32u * i + lane] = route[i];
+                bars->extra[buffer][32u * i + lane] = extra[i];
+            }
+            if (lane == 0u) {
+                bars->tile_tokens[buffer] = tokens;
+                bars->tile_rows[buffer] = tile % m_tiles;
+            }
+            mbar_arrive(&bars->info_full[buffer]);
+        }
+        __syncwarp();
+    } else {
+        // ===== epilogue: TMEM -> registers -> global =============================================
+        // Sixteen tokens at a time go through each step together, without a branch, so that the latencies of their
+        // instructions overlap: columns without a token hold zeros or what is left of others and are only not stored.
+        const uint32_t quad = warp & 3u, group = warp >> 2;
+        const uint32_t frame_words = K * (I / 2u) + K;
+        const bool whole_block = GATE_UP && p.g.act_block == 128u;
+        const bool quantise = GATE_UP && p.q_out != nullptr;             // host: only with scale blocks of 32 or 128 rows
+        const bool store_rows = !GATE_UP || p.intermediates != nullptr;
+        uint32_t acc_it = 0u, sends = 0u, receipts = 0u, set_it = 0u;
+        // this warp's place in the exchange: its own (read) and the same place of the other CTA's warp (written)
+        const uint4* inbox = reinterpret_cast<const uint4*>(smem + kPairExchangeRegion + warp * 1024u) + lane;
+        const uint32_t outbox = map_shared(smem_u32(inbox), rank ^ 1u);
+        const uint32_t peer_sent = map_shared(smem_u32(&bars->sent[warp]), rank ^ 1u);
+        const uint32_t peer_taken = map_shared(smem_u32(&bars->taken[warp]), rank ^ 1u);
+        for (uint32_t tile = pair_id; tile < tile_count; tile += pairs, acc_it++) {
+            const uint32_t acc = acc_it & 1u;
+            // (one warp polls, the others sleep on a hardware barrier; every warp reaches it in every round)
+            if (warp == kPairWatchWarp) {
+                const bool ready = mbar_wait_warp(&bars->info_full[acc], (acc_it >> 1) & 1u, abort_flag, wait_limit) &&
+                                   mbar_wait_warp(&bars->acc_full[acc], (acc_it >> 1) & 1u, abort_flag, wait_limit);
+                if (lane == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) = ready ? 1u : 0u;
+                __threadfence_block();
+            }
+            named_barrier(1u, 32u * kPairEpilogueWarps);
+            if (*reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) == 0u) break;
+            tc_fence_after();
+            const uint32_t tokens = bars->tile_tokens[acc], m_tile = bars->tile_rows[acc];
+            const uint32_t first_row = (GATE_UP ? m_tile : 2u * m_tile + rank) * kBlockM + quad * 32u;
+            const uint32_t row = first_row + lane;
+            const bool row_ok = row < out_rows;
+            const uint32_t lane_addr = tmem_base + ((quad * 32u) << 16) + acc * kPairColumns;
+            const uint32_t chunks = (tokens + 15u) / 16u;                // of sixteen columns, with a token in them
+            const uint32_t half = GATE_UP ? (chunks + 1u) / 2u : chunks; // gate/up: CTA 0 takes these, CTA 1 the others
+            // the other CTA's i-th chunk, to its shared memory
+            auto send = [&](uint32_t i) {
+                const uint32_t c = rank == 0u ? half + i : i;
+                if (i >= half || c >= chunks) return;
+                uint32_t s[16];
+                tmem_ld16(lane_addr + 16u * c, s);
+                // (the place is free again once the other warp has taken what was sent last; a wait that gives up leaves
+                // rubbish behind: the call reports it, the next tile is not begun)
+                mbar_wait_warp(&bars->taken[warp], (sends & 1u) ^ 1u, abort_flag, wait_limit);
+                tmem_ld_wait();
+                uint32_t v[8];
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; j++) v[j] = bf16x2_bits(__uint_as_float(s[2u * j]), __uint_as_float(s[2u * j + 1u]));
+                store_async_cluster(outbox, v[0], v[1], v[2], v[3], peer_sent);
+                store_async_cluster(outbox + 512u, v[4], v[5], v[6], v[7], peer_sent);
+                sends++;
+            };
+            if (GATE_UP) send(group);
+            for (uint32_t i = group; i < half; i += kPairEpilogueGroups) {
+                const uint32_t c = GATE_UP && rank == 1u ? half + i : i;
+                const bool mine = c < chunks;
+                uint32_t d[16], other[8];
+                if (mine) tmem_ld16(lane_addr + 16u * c, d);
+                if (GATE_UP && mine) {
+                    if (lane == 0u) mbar_arrive_expect_tx(&bars->sent[warp], 1024u);
+                    mbar_wait_cluster_warp(&bars->sent[warp], receipts & 1u, abort_flag, wait_limit);
+                    const uint4 low = inbox[0], high = inbox[32];
+                    other[0] = low.x, other[1] = low.y, other[2] = low.z, other[3] = low.w;
+                    other[4] = high.x, other[5] = high.y, other[6] = high.z, other[7] = high.w;
+                    __syncwarp();
+                    if (lane == 0u) mbar_arrive_cluster(peer_taken);
+                    receipts++;
+                }
+                tmem_ld_wait();
+                if (GATE_UP) send(i + kPairEpilogueGroups);  // on its way while this chunk is worked on
+                if (!mine) continue;
+                const uint32_t* routes = &bars->route[acc][16u * c];
+                const uint32_t* extras = &bars->extra[acc][16u * c];
+                uint32_t v[8];  // the sixteen values as bf16, in pairs
+                if (GATE_UP) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++) {
+                        const uint32_t own = bf16x2_bits(__uint_as_float(d[2u * j]), __uint_as_float(d[2u * j + 1u]));
+                        const uint32_t g = rank == 0u ? own : other[j], u = rank == 0u ? other[j] : own;
+                        v[j] = bf16x2_bits(swiglu_approx(low_bf16(g), low_bf16(u), p.g.swiglu_limit, p.g.swiglu_alpha, p.g.swiglu_up_offset),
+                                           swiglu_approx(high_bf16(g), high_bf16(u), p.g.swiglu_limit, p.g.swiglu_alpha, p.g.swiglu_up_offset));
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++)
+                        v[j] = bf16x2_bits(__fmul_rn(__uint_as_float(d[2u * j]), __uint_as_float(extras[2u * j])),
+                                           __fmul_rn(__uint_as_float(d[2u * j + 1u]), __uint_as_float(extras[2u * j + 1u])));
+                }
+                if (store_rows) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; j++) {
+                        const uint32_t route = routes[j];
+                        if (route == kUnboundSlot || !row_ok) continue;
+                        const uint16_t bits = (uint16_t)((j & 1u) ? v[j / 2u] >> 16 : v[j / 2u]);
+                        if (GATE_UP) {
+                            reinterpret_cast<uint16_t*>(p.intermediates + (size_t)(route / K) * frame_words)[(size_t)(route % K) * I + row] = bits;
+                        } else if (p.partial_outputs != nullptr) {
+                            // tensor-parallel form: the raw f32 sums over this participant's columns
+                            p.partial_outputs[(size_t)route * H + row] = __uint_as_float(d[j]);
+                        } else {
+                            p.outputs[(size_t)route * H + row] = bits;
+                        }
+                    }
+                }
+                if (quantise) {
+                    // the down stage's activation quantisation, as in experts_tc.cu: a power-of-two scale per 32 rows (this warp's)
+                    // or per 128 (the four warps of the group, which hand their maxima round). The maxima of the sixteen tokens
+                    // are folded over the lanes by halves, so that four lanes end with those of one pair of tokens and each
+                    // token's scale is worked out once.
+                    uint32_t m[8];
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++) m[j] = row_ok ? v[j] & 0x7fff7fffu : 0u;
+#pragma unroll
+                    for (uint32_t o = 16u, n = 4u; n > 0u; o >>= 1, n >>= 1) {
+                        const bool upper = (lane & o) != 0u;
+#pragma unroll
+                        for (uint32_t j = 0; j < n; j++) {
+                            const uint32_t kept = upper ? m[j + n] : m[j], given = upper ? m[j] : m[j + n];
+                            m[j] = max_bf16x2(kept, __shfl_xor_sync(0xffffffffu, given, o));
+                        }
+                    }
+                    uint32_t top = max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
+                    top = max_bf16x2(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                    const uint32_t pair = lane >> 2;  // lane bits 4, 3, 2 chose the upper or lower four, two, one of the eight pairs
+                    if (whole_block) {
+                        // (a chunk's maxima are overwritten two chunks later, when every warp has passed the barrier between)
+                        uint32_t(&quad_max)[4][8] = bars->maxima[group][set_it++ & 1u];
+                        if ((lane & 3u) == 0u) quad_max[quad][pair] = top;
+                        named_barrier(2u + group, 128u);
+                        top = max_bf16x2(max_bf16x2(quad_max[0][pair], quad_max[1][pair]), max_bf16x2(quad_max[2][pair], quad_max[3][pair]));
+                    }
+                    // lanes 4 pair and 4 pair + 1: the two tokens of the pair
+                    const uint32_t token = 2u * pair + (lane & 1u), my_row = extras[token];
+                    const float scale = nvmoe_rounded_fp8_scale((lane & 1u) ? high_bf16(top) : low_bf16(top));
+                    const float my_inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
+                    if ((lane & 2u) == 0u && my_row != kUnboundSlot && first_row < out_rows)
+                        *p.q_e8m0.byte_at(my_row, first_row / 32u) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++) {
+                        const float inv0 = __shfl_sync(0xffffffffu, my_inv, 4u * j), inv1 = __shfl_sync(0xffffffffu, my_inv, 4u * j + 1u);
+                        const uint32_t q = __nv_cvt_float2_to_fp8x2(make_float2(low_bf16(v[j]) * inv0, high_bf16(v[j]) * inv1), __NV_SATFINITE, __NV_E4M3);
+                        const uint32_t row0 = extras[2u * j], row1 = extras[2u * j + 1u];
+                        // (0xffffffff: columns without a token and routes the down stage skips)
+                        if (row0 != kUnboundSlot && row_ok) p.q_out[(size_t)row0 * I + row] = (uint8_t)q;
+                        if (row1 != kUnboundSlot && row_ok) p.q_out[(size_t)row1 * I + row] = (uint8_t)(q >> 8);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0u) {
+                mbar_arrive(&bars->info_empty[acc]);
+                mbar_arrive_cluster(map_shared(smem_u32(&bars->acc_empty[acc]), 0u));
+            }
+        }
+    }
+
+    // ---- teardown: neither CTA leaves while the other may still reach into its shared memory -------------------
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0u) raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
+    __syncwarp();
+    cluster_sync();
+    if (warp == kPairMmaWarp) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, kPairTmemColumns);
+    }
+}
+
+template <bool GATE_UP>
+void launch(const ExpertLaunch& p, int sms, cudaStream_t stream) {
+    launch_chained(experts_pair_kernel<GATE_UP>, dim3((uint32_t)sms & ~1u), dim3(kPairThreads), kPairSmemBytes, stream, p,
+                   TileList{p.tile_list, p.tile_count});
+}
+
+}  // namespace
+
+void pair_configure_kernels() {
+    cudaFuncSetAttribute(experts_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
+    cudaFuncSetAttribute(experts_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
+}
+
+void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream) {
+    if (gate_up) {
+        launch<true>(p, sms, stream);
+    } else {
+        launch<false>(p, sms, stream);
+    }
+}
+
+}  // namespace nvmoe

@@ -33,6 +33,7 @@
 
 #include <cstring>
 
+#include "experts_device.cuh"
 #include "experts_tc.cuh"
 #include "quantize.cuh"
 #include "tcgen05.cuh"
@@ -42,20 +43,10 @@ namespace {
 
 using namespace tc;
 
-constexpr uint32_t kBlockM = 128u;   // weight rows per tile
-constexpr uint32_t kBlockK = 128u;   // K elements per pipeline stage = 4 MMAs of K = 32
 constexpr uint32_t kFirstProducerThread = 192u;    // warps 0-3 epilogue, 4 MMA, 5 TMA, 6.. cp.async, then more epilogue warps
-constexpr uint32_t kTmaBoxBytes = kBlockM * 64u;   // global bytes of one 128 x 128 box of 4-bit codes
-constexpr uint32_t kATileBytes = kBlockM * 128u;   // one byte slot per element
-constexpr uint32_t kScaleBlockBytes = 512u;        // 128 rows x 4 scale bytes
 constexpr uint32_t kMaxStages = 8u;
 constexpr uint32_t kRowPairRounds = 6u;  // rounds of the SMs, with every expert selected, from which narrow down tiles pair their rows
 constexpr uint32_t kWatchWarp = 2u;     // the epilogue warp that polls for a finished accumulator (not on the MMA or TMA warp's scheduler)
-
-struct TileList {
-    const uint32_t* tiles;   // (expert << 16) | token tile within the expert
-    const uint32_t* count;   // number of entries
-};
 
 // ROW_PAIR (down only): a tile covers two 128-row tiles of the one weight matrix, handled as the two
 // "matrices" of a stage exactly as gate and up are: two accumulators alternate (one MMA cannot follow
@@ -139,23 +130,6 @@ struct Config {
     static_assert(kBTileBytes % 1024u == 0u && kABytes % 1024u == 0u, "operand tiles keep their 1024-byte alignment");
     static_assert(kStages >= 3u, "pipeline too shallow");
 };
-
-// SwiGLU of the tensor path: the same expression and roundings as nvmoe_swiglu (accumulators rounded
-// to bf16, clamp, g / (1 + exp(-alpha g)) * (u + offset), result rounded to bf16) with the hardware's
-// approximate exponential and reciprocal (a few units in the last place of f32, far below the bf16
-// rounding that follows) instead of the pinned software forms: a wide token tile spends more issue
-// slots on its epilogue than on its MMAs, and the pinned forms cost several times as many.
-// Returns the bf16 bits. The CUDA-core path keeps the pinned forms.
-__device__ __forceinline__ uint32_t swiglu_bf16_bits(float gate_acc, float up_acc, float limit, float alpha, float up_offset) {
-    float g = __bfloat162float(__float2bfloat16_rn(gate_acc));
-    float u = __bfloat162float(__float2bfloat16_rn(up_acc));
-    if (limit > 0.0f) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-    }
-    const float act = __fdividef(g, 1.0f + __expf(-alpha * g)) * (u + up_offset);
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(act));
-}
 
 struct Barriers {
     uint64_t full[kMaxStages];
@@ -253,7 +227,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         // acquire such a map once before any of its threads hands it to the TMA unit; further uses by the
         // block need no fence. All threads share the maps out, so that the block pays one fence latency here
         // instead of one per map in the lane that issues the loads.
-        for (uint32_t m = threadIdx.x; m < p.work.num_experts * C::kSources; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 128u);
+        for (uint32_t m = threadIdx.x; m < p.work.num_experts * C::kSources; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u);
         if (threadIdx.x == 0u) tensormap_acquire(p.act_tmap);
         __syncthreads();
     }
@@ -298,7 +272,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 if (tile + gridDim.x < tile_count) meta_of(tile + gridDim.x, pair_nxt, nxt);
                 const uint32_t m_tile = cur.m_tile;
                 const int row0 = (int)(m_tile * C::kTileRows);
-                const uint8_t* maps = p.tmaps + (size_t)(cur.pair >> 16) * C::kSources * 128u;
+                const uint8_t* maps = p.tmaps + (size_t)(cur.pair >> 16) * C::kSources * 256u;
                 // first operand row of this token tile in the expert-grouped activation matrix
                 const int token0 = (int)(cur.expert_begin + (cur.pair & 0xffffu) * N_TILE);
                 const uint8_t* scale_blocks[C::kMatrices];
@@ -333,7 +307,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         if (sub < whole) {
 #pragma unroll
                             for (uint32_t mx = 0; mx < C::kMatrices; mx++)
-                                tma_load_3d(smem_base + block * C::kABytes + mx * kATileBytes, maps + C::source_of(mx) * 128u, 0, (int)kb,
+                                tma_load_3d(smem_base + block * C::kABytes + mx * kATileBytes, maps + C::source_of(mx) * 256u, 0, (int)(2u * kb),
                                             row0 + (int)C::row_shift(mx), &bars->full[slot]);  // rows past the matrix: zeros
                         }
                         tma_load_2d(smem_base + C::kBRegion + block * C::kBTileBytes, p.act_tmap, (int)(kb * kBlockK), token0,
@@ -490,14 +464,14 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 if (USE_TMA) {
                     for (uint32_t n = pt; n < N_TILE; n += kProducerThreads) {
                         const bool ok = n < cur.valid;
-                        const uint32_t* src = ok ? p.act_e8m0 + (size_t)(cur.first + n) * k_blocks + kb : p.act_e8m0;
+                        const uint32_t* src = ok ? p.act_e8m0.words + (size_t)(cur.first + n) * k_blocks + kb : p.act_e8m0.words;
                         cp_async_4(smem_u32(sf + C::kMatrices * kScaleBlockBytes + (n & 31u) * 16u + (n >> 5) * 4u), src,
                                    ok ? 4u : 0u);
                     }
                 } else if (st >= 64u && st < 64u + N_TILE) {
                     const uint32_t n = st - 64u;
                     const bool ok = n < cur.valid;
-                    const uint32_t* src = ok ? p.act_e8m0 + (size_t)cur.scale_row * k_blocks + kb : p.act_e8m0;
+                    const uint32_t* src = ok ? p.act_e8m0.words + (size_t)cur.scale_row * k_blocks + kb : p.act_e8m0.words;
                     cp_async_4(smem_u32(sf + C::kMatrices * kScaleBlockBytes + (n & 31u) * 16u + (n >> 5) * 4u), src,
                                ok ? 4u : 0u);
                 }
@@ -783,8 +757,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                             if (dp != kUnboundSlot) {  // (lanes past `valid` and routes the down stage skips)
                                 if (row_ok) p.q_out[(size_t)dp * I + row] = q;
                                 if (writes_scale)
-                                    reinterpret_cast<uint8_t*>(p.q_e8m0 + (size_t)dp * ((I + 127u) / 128u))[first_row / 32u] =
-                                        (uint8_t)(nvmoe_f32_bits(scale) >> 23);
+                                    *p.q_e8m0.byte_at(dp, first_row / 32u) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
                             }
                         }
                     }
@@ -854,20 +827,27 @@ __global__ void commit_stamps_kernel(const ExpertPtrs* experts, uint64_t* stamps
     stamps[(size_t)i * 2u + 1u] = ptrs.gen[mx];
 }
 
-// One warp per (expert, matrix): the template map with the expert's weight address patched in.
-__global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* experts, const uint8_t* templ,
+// (a whole warp) the template with an address patched in, as a map that the TMA unit may be given once it has been acquired
+__device__ __forceinline__ void publish_map(uint8_t* map, const uint8_t* templ, unsigned char* smem_map, const uint8_t* address) {
+    reinterpret_cast<uint32_t*>(smem_map)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t*>(templ) + threadIdx.x);
+    __syncwarp();
+    if (threadIdx.x == 0u) tensormap_replace_address(smem_map, address);
+    __syncwarp();
+    tensormap_publish(map, smem_map);
+}
+
+// One warp per (expert, matrix): the two template maps (a box of one K block, of two) with the expert's weight address
+// patched in; then one for the map of the set's derived scale copy.
+__global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* experts, const uint8_t* templ, const uint8_t* derived,
                                                              uint8_t* maps, uint32_t matrices) {
-    __shared__ __align__(128) unsigned char sm[128];
+    __shared__ __align__(128) unsigned char sm[256];
     const uint32_t e = blockIdx.x / matrices, mx = blockIdx.x % matrices;
-    const uint8_t* w = experts[e].w[mx];
-    if (experts[e].w[0] == nullptr || w == nullptr) return;
-    // `templ` holds the map of the compact form followed by the map of the one-byte-per-element forms
-    const uint8_t* mine = templ + (experts[e].format == kFormatCompact ? 0u : 128u);
-    reinterpret_cast<uint32_t*>(sm)[threadIdx.x] = reinterpret_cast<const uint32_t*>(mine)[threadIdx.x];
-    __syncwarp();
-    if (threadIdx.x == 0u) tensormap_replace_address(sm, w);
-    __syncwarp();
-    tensormap_publish(maps + (size_t)blockIdx.x * 128u, sm);
+    const bool scales = blockIdx.x == gridDim.x - 1u;
+    if (!scales && (experts[e].w[0] == nullptr || experts[e].w[mx] == nullptr)) return;
+    const uint8_t* w = scales ? derived : experts[e].w[mx];
+    // `templ` holds the maps of the compact form, those of the one-byte-per-element forms and that of the derived scales
+    const uint8_t* mine = templ + (scales ? 512u : experts[e].format == kFormatCompact ? 0u : 256u);
+    for (uint32_t i = 0; i < (scales ? 1u : 2u); i++) publish_map(maps + (size_t)blockIdx.x * 256u + i * 128u, mine + i * 128u, sm + i * 128u, w);
 }
 
 // The same for the one matrix of a dense linear, whose addresses are the call's own: nothing about the matrix is kept
@@ -879,7 +859,7 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
-    __shared__ __align__(128) unsigned char sm[128];
+    __shared__ __align__(128) unsigned char sm[256];
     grid_dependency_sync();
     const uint32_t tile_total = p.tiles.list ? (p.tokens + p.tiles.n_tile - 1u) / p.tiles.n_tile : 0u;
     for (uint32_t i = blockIdx.x * kDenseThreads + threadIdx.x; i < p.tokens; i += gridDim.x * kDenseThreads) {
@@ -914,7 +894,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
     }
     if (blockIdx.x != gridDim.x - 1u) {
         if (LANES == 0u) return;
-        const uint32_t lane = threadIdx.x & 31u, chunks = (p.cols + 511u) / 512u, words128 = (p.cols + 127u) / 128u;
+        const uint32_t lane = threadIdx.x & 31u, chunks = (p.cols + 511u) / 512u;
         const uint32_t item = (blockIdx.x - retile_blocks) * (kDenseThreads / 32u) + (threadIdx.x >> 5);
         const uint32_t row = item / chunks, col = (item % chunks) * 512u + lane * 16u;
         if (row >= p.tokens) return;
@@ -923,7 +903,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
         quantize_sixteen<(LANES == 0u ? 1u : LANES)>(p.input + (size_t)row * p.cols + col, active, lane, out, word);
         if (!active) return;
         *reinterpret_cast<uint4*>(p.q + (size_t)row * p.cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
-        if ((lane & 7u) == 0u) p.q_e8m0[(size_t)row * words128 + col / 128u] = word;
+        if ((lane & 7u) == 0u) *p.q_e8m0.at(row, col / 128u) = word;
         return;
     }
     if (threadIdx.x == 0u) {
@@ -933,11 +913,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
         *p.ptrs = ExpertPtrs{{p.weights, nullptr}, {p.scales, nullptr}, {p.derived, nullptr}, {0u, 0u}, kFormatCompact, 0u};
     }
     if (p.map_template != nullptr && threadIdx.x < 32u) {
-        reinterpret_cast<uint32_t*>(sm)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t*>(p.map_template) + threadIdx.x);
-        __syncwarp();
-        if (threadIdx.x == 0u) tensormap_replace_address(sm, p.weights);
-        __syncwarp();
-        tensormap_publish(p.map, sm);
+        for (uint32_t i = 0; i < 2u; i++) publish_map(p.map + i * 128u, p.map_template + i * 128u, sm + i * 128u, p.weights);
     }
 }
 
@@ -984,8 +960,11 @@ bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) 
 template <bool GATE_UP>
 void launch(const ExpertLaunch& p, cudaStream_t stream) {
     const int sms = sm_count();
-    const uint32_t n = tc_token_tile_for(p.tokens, p.g.routed_k + p.g.always_count, p.work.num_experts,
-                                         GATE_UP ? p.g.intermediate_size : p.g.hidden_size, GATE_UP);
+    const uint32_t n = p.token_rows;
+    if (p.pairs) {
+        launch_experts_pair(p, GATE_UP, sms, stream);
+        return;
+    }
     const bool tma = p.tmaps != nullptr;
     const bool pairs = !GATE_UP && takes_row_pairs(p, n, tma, sms);
     if (tma && pairs) {
@@ -993,16 +972,14 @@ void launch(const ExpertLaunch& p, cudaStream_t stream) {
             case 16u: launch_n<GATE_UP, 16u, true, !GATE_UP>(p, sms, stream); break;
             case 32u: launch_n<GATE_UP, 32u, true, !GATE_UP>(p, sms, stream); break;
             case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
-            case 96u: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
-            default: launch_n<GATE_UP, 128u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
         }
     } else if (tma) {
         switch (n) {
             case 16u: launch_n<GATE_UP, 16u, true, false>(p, sms, stream); break;
             case 32u: launch_n<GATE_UP, 32u, true, false>(p, sms, stream); break;
             case 64u: launch_n<GATE_UP, 64u, true, !GATE_UP>(p, sms, stream); break;
-            case 96u: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
-            default: launch_n<GATE_UP, 128u, true, !GATE_UP>(p, sms, stream); break;
+            default: launch_n<GATE_UP, 96u, true, !GATE_UP>(p, sms, stream); break;
         }
     } else {
         switch (n) {
@@ -1025,11 +1002,13 @@ void configure_one() {
 
 template <uint32_t N_TILE>
 void configure_tile() {
-    configure_one<true, N_TILE, true, false>();
     configure_one<true, N_TILE, false, false>();
-    configure_one<false, N_TILE, true, true>();
     configure_one<false, N_TILE, false, (N_TILE >= 64u)>();
-    if (N_TILE < 64u) configure_one<false, N_TILE, true, (N_TILE >= 64u)>();
+    if constexpr (N_TILE <= 96u) {
+        configure_one<true, N_TILE, true, false>();
+        configure_one<false, N_TILE, true, true>();
+    }
+    if constexpr (N_TILE < 64u) configure_one<false, N_TILE, true, false>();
 }
 
 }  // namespace
@@ -1040,22 +1019,38 @@ bool tc_shape_supported(const nvmoe_geometry& g) {
 
 bool tc_enabled_by_default() { return true; }
 
-uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up) {
+TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up, bool tma) {
     // tokens per expert if routing were uniform; skew only adds token tiles
     const uint32_t routes = tokens * routes_per_token;
     const uint32_t per_expert = (routes + num_experts - 1u) / num_experts;
     // the narrowest tile that holds an expert's tokens (with some room for skew: a second tile reads the weights again)
-    if (per_expert <= 12u) return 16u;
-    if (per_expert <= 24u) return 32u;
-    if (per_expert <= 48u) return 64u;
-    if (per_expert <= 96u) return 96u;
-    // Beyond that an expert takes several tiles and the wide ones are the cheapest per token, unless a wave of the SMs
-    // goes half empty with them (777 x 7168 x 2048 dense: 115 us with 128 columns, 109 with 96): the fewest rounds x
-    // stage time wins. A stage of 128 columns takes 8/7 of the time of one of 96 (0.527 and 0.461 us in the down kernel
-    // of 12288 x 2944 x 9472, whole rounds of either); 4096 tokens of 32 experts of 2880 x 2880 640 against 683 us.
+    if (per_expert <= 12u) return {16u, false};
+    if (per_expert <= 24u) return {32u, false};
+    if (per_expert <= 48u) return {64u, false};
+    if (per_expert <= 96u) return {96u, false};
     const uint32_t row_tiles = gate_up ? (out_rows + kBlockM - 1u) / kBlockM : (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM);
-    const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {8u, 7u};
     const uint64_t sms = (uint64_t)sm_count();
+    // Beyond that CTA pairs (one CTA of 128 columns / pairs: 4096 tokens of 32 experts of 2880 x 2880 672 / 589 us a layer,
+    // 8192 of 128 1640 / 1575, 16384 of 256 of 7168 x 2048 9960 / 9330). An expert takes several tiles, and the wide ones are
+    // the cheapest per token unless a wave of the pairs goes half empty with them: the fewest rounds x stage time wins, the
+    // time of a stage being that of its shared-memory traffic, 256 + columns.
+    if (tma) {
+        const uint32_t rows[4] = {kPairTokens, 192u, 128u, 64u};
+        TokenTile best{kPairTokens, true};
+        uint64_t best_cost = ~0ull;
+        for (uint32_t i = 0; i < 4u; i++) {
+            const uint64_t tiles = (uint64_t)num_experts * ((per_expert + rows[i] - 1u) / rows[i]) * row_tiles;
+            const uint64_t cost = (tiles + sms / 2u - 1u) / (sms / 2u) * (256u + rows[i]);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best.rows = rows[i];
+            }
+        }
+        return best;
+    }
+    // Shapes without tensor maps: the widest tile, by the same count of rounds. A stage of 128 columns takes 8/7 of the time
+    // of one of 96 (0.527 and 0.461 us with whole rounds of either).
+    const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {8u, 7u};
     uint32_t best = 0u;
     uint64_t best_cost = ~0ull;
     for (uint32_t i = 0; i < 2u; i++) {
@@ -1066,11 +1061,7 @@ uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t 
             best = widths[i];
         }
     }
-    return best;
-}
-
-uint32_t tc_token_tile_index(uint32_t n_tile) {
-    return n_tile == 16u ? 0u : n_tile == 32u ? 1u : n_tile == 64u ? 2u : n_tile == 96u ? 3u : 4u;
+    return {best, false};
 }
 
 size_t tc_derived_scale_bytes(uint32_t rows, uint32_t cols) {
@@ -1120,14 +1111,15 @@ static EncodeFn tensor_map_encoder() {
 }
 
 bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols) {
-    // The packaged [rows][cols/2] bytes seen as a 3-D tensor of 4-bit elements
-    // {128 elements, cols/128 K blocks, rows}: a box {128, 1, 128} is one operand tile. The padded 4-bit
-    // type wants 32-byte strides (cols % 64 == 0); a trailing partial K block is not part of the map.
+    // The packaged [rows][cols/2] bytes seen as a 3-D tensor of 4-bit elements {128 elements, blocks, rows} whose blocks of
+    // 128 columns start every 64: a box {128, 1, 128} is one operand tile, at block 2 kb that of K block kb, at the last
+    // block the 128 columns that end with the row. (The padded 4-bit type wants 32-byte strides, so cols % 64 == 0, and
+    // whole 128-element rows.)
     if (cols < kBlockK || cols % 64u != 0u) return false;
     EncodeFn encode = tensor_map_encoder();
     if (!encode) return false;
-    const cuuint64_t dims[3] = {kBlockK, cols / kBlockK, rows};
-    const cuuint64_t strides[2] = {kBlockK / 2u, cols / 2u};
+    const cuuint64_t dims[3] = {kBlockK, cols / 64u - 1u, rows};
+    const cuuint64_t strides[2] = {32u, cols / 2u};
     const cuuint32_t box[3] = {kBlockK, 1u, kBlockM};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUtensorMap map;
@@ -1140,19 +1132,67 @@ bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows,
 }
 
 bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols) {
-    // One E4M3 byte per element, seen like the compact form as {128 elements, cols/128 K blocks, rows}: the
+    // One E4M3 byte per element, seen like the compact form as {128 elements, blocks every 64 columns, rows}: the
     // same box coordinates fetch the same operand tile, now without padding.
     if (cols < kBlockK || cols % kBlockK != 0u) return false;
     EncodeFn encode = tensor_map_encoder();
     if (!encode) return false;
-    const cuuint64_t dims[3] = {kBlockK, cols / kBlockK, rows};
-    const cuuint64_t strides[2] = {kBlockK, cols};
+    const cuuint64_t dims[3] = {kBlockK, cols / 64u - 1u, rows};
+    const cuuint64_t strides[2] = {64u, cols};
     const cuuint32_t box[3] = {kBlockK, 1u, kBlockM};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUtensorMap map;
     if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, any_device_address, dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    std::memcpy(map128, &map, 128);
+    return true;
+}
+
+// a 3-D map of one- or four-byte elements, rows of `dims[0]` elements
+static bool encode_3d(void* map128, CUtensorMapDataType type, void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2],
+                      const cuuint32_t (&box)[3], CUtensorMapSwizzle swizzle) {
+    EncodeFn encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUtensorMap map;
+    if (encode(&map, type, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    std::memcpy(map128, &map, 128);
+    return true;
+}
+
+bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, bool bytes) {
+    if (cols < kBlockK || cols % (bytes ? kBlockK : 64u) != 0u) return false;
+    const uint32_t half = bytes ? 1u : 2u;  // elements to a byte
+    return encode_3d(map128, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, any_device_address,
+                     {kBlockK, rows, cols / kBlockK}, {cols / half, kBlockK / half}, {kBlockK, kBlockM, 2u}, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows) {
+    if (cols < kBlockK || cols % 16u != 0u || rows == 0u) return false;
+    return encode_3d(map128, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, {kBlockK, rows, cols / kBlockK}, {cols, kBlockK}, {kBlockK, box_rows, 2u},
+                     CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+bool tc_encode_pair_scale_map(void* map128, void* any_device_address, uint32_t sources, uint32_t blocks) {
+    return encode_3d(map128, CU_TENSOR_MAP_DATA_TYPE_UINT32, any_device_address, {kScaleBlockBytes / 4u, sources, blocks},
+                     {kScaleBlockBytes, sources * kScaleBlockBytes}, {kScaleBlockBytes / 4u, 1u, 2u}, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+bool tc_encode_token_scale_map(void* map128, void* base, uint32_t words, uint32_t rows) {
+    if (words % 4u != 0u || words == 0u || rows == 0u) return false;
+    EncodeFn encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {words, rows};
+    const cuuint64_t strides[1] = {4ull * words};
+    const cuuint32_t box[2] = {kPairTokens + 4u, 2u};
+    const cuuint32_t estr[2] = {1u, 1u};
+    CUtensorMap map;
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     std::memcpy(map128, &map, 128);
     return true;
@@ -1176,11 +1216,9 @@ bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t 
 
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream) {
     const uint32_t matrices = gate_up ? 2u : 1u;
-    build_tensormaps_kernel<<<p.work.num_experts * matrices, 32, 0, stream>>>(p.work.experts, templ,
-                                                                              const_cast<uint8_t*>(p.tmaps), matrices);
+    build_tensormaps_kernel<<<p.work.num_experts * matrices + 1u, 32, 0, stream>>>(p.work.experts, templ, p.scale_base,
+                                                                                   const_cast<uint8_t*>(p.tmaps), matrices);
 }
-
-
 
 void tc_configure_kernels() {
     configure_tile<16u>();
@@ -1188,6 +1226,7 @@ void tc_configure_kernels() {
     configure_tile<64u>();
     configure_tile<96u>();
     configure_tile<128u>();
+    pair_configure_kernels();
 }
 
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<true>(p, stream); }

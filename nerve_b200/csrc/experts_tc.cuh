@@ -18,7 +18,15 @@ bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t
 // Encodes the tensor map of an expert-grouped activation matrix [rows][cols] of E4M3 bytes with a box of
 // n_tile rows x 128 bytes (the operand tile of one K block). False when tensor maps are unavailable.
 bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t n_tile);
-// per-expert tensor maps = template + the expert's weight address (p.tmaps must be set)
+// The tensor maps of the CTA pair kernel, whose boxes bring two K blocks at a time: a weight matrix in the compact or a
+// one-byte form (128 rows), expert-grouped token rows, the derived scales of a set (blocks of 512 bytes, `sources` to a
+// (row tile, K block)), and the token scales [rows = K blocks][words].
+bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, bool bytes);
+bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows);
+bool tc_encode_pair_scale_map(void* map128, void* any_device_address, uint32_t sources, uint32_t blocks);
+bool tc_encode_token_scale_map(void* map128, void* base, uint32_t words, uint32_t rows);
+// per-expert tensor maps = template + the expert's weight address (p.tmaps must be set), and after them the map of the
+// derived scales (p.scale_base)
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream);
 // What a dense linear needs before its expert kernel, in one launch: the schedule (every row a route of expert 0 in row
 // order), what hangs on its matrix (the pointers and, for the tensor path (`derived` set), the re-tiled scales and the
@@ -38,14 +46,30 @@ struct DensePrepare {
     uint8_t* map;
     const uint16_t* input;
     uint8_t* q;
-    uint32_t* q_e8m0;
+    ScaleWords q_e8m0;
 };
 bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_t stream);
-// token tile size of a stage for this many tokens and rows of its weight matrix (the (expert, token tile) list must be
-// built with it)
-uint32_t tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up);
-// which of a stage's five tile sizes (and activation tensor maps) that is
-uint32_t tc_token_tile_index(uint32_t n_tile);
+// Token tile of a stage: rows of the operand matrix per entry of the (expert, token tile) list, by a CTA pair (experts_pair.cu)
+// or by one CTA (then one of the kernel's tile widths).
+struct TokenTile {
+    uint32_t rows;
+    bool pair;
+};
+// token tile of a stage for this many tokens and rows of its weight matrix (the (expert, token tile) list must be
+// built with it); tma: the stage's shapes have tensor maps
+TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up, bool tma);
+constexpr uint32_t kPairTokens = 240u;  // the most tokens of a pair's tile
+void pair_configure_kernels();
+void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream);
+// Tensor maps of a stage's operands: token rows in boxes of one K block, for one CTA's token tiles and, from the second on,
+// for four of a pair's (half a tile); the same four in boxes of two; the token scales.
+constexpr uint32_t kTokenMaps = 6u, kPairTokenMap = kTokenMaps, kTokenScaleMap = kPairTokenMap + 4u, kActMaps = kTokenScaleMap + 1u;
+constexpr uint32_t kTokenMapRows[kTokenMaps] = {16u, 32u, 64u, 96u, kPairTokens / 2u, 128u};
+inline uint32_t tc_token_map_for(const TokenTile& t) {
+    uint32_t i = 0u;
+    while (i + 1u < kTokenMaps && kTokenMapRows[i] != t.rows) i++;
+    return t.pair ? 1u : i;
+}
 // bytes of the derived (tiled) scale copy of one expert matrix with `rows` x `cols` elements
 size_t tc_derived_scale_bytes(uint32_t rows, uint32_t cols);
 // re-tiles the scales of every expert whose scale record changed since the last call

@@ -5,8 +5,8 @@
 //   independent_sparse_moe_down_batch1_mxfp4.comp.template:307-353 (quantize_intermediate)
 //
 // scale = 2^ceil(log2(max(|x|, 1e-4) / 448)), q = E4M3(x / scale) with round-to-nearest-even.
-// The reference block is 128 columns; any multiple of 32 that divides the row works here.  Besides
-// the f32 scales of the reference contract the kernel can emit the same scales as E8M0 bytes, one
+// The reference block is 128 columns; any multiple of 32 that divides the row works here.  In the place of
+// the f32 scales of the reference contract the tensor path takes the same scales as E8M0 bytes, one
 // per 32 columns, four to a word — the form a block-scaled MMA reads.
 #include "quantize.cuh"
 
@@ -19,11 +19,10 @@ namespace {
 // of zeros.
 template <class RowFn>
 __device__ void quantize_body(RowFn row_of, uint32_t rows, uint32_t cols, uint32_t block, uint8_t* q,
-                              float* scales_f32, uint32_t* scales_e8m0) {
+                              float* scales_f32, const ScaleWords& scales) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps_per_grid = (gridDim.x * blockDim.x) >> 5;
     const uint32_t blocks_per_row = cols / block;
-    const uint32_t words128 = (cols + 127u) / 128u;
     const uint64_t total = (uint64_t)rows * blocks_per_row;
     // lanes per block: a power of two that divides 32 (blocks of 32, 64 or 128+ columns), else the whole warp
     const uint32_t quarter = block / 4u;
@@ -57,27 +56,26 @@ __device__ void quantize_body(RowFn row_of, uint32_t rows, uint32_t cols, uint32
                                 nvmoe_bf16_to_f32(v.y) * inv, nvmoe_bf16_to_f32(v.y >> 16) * inv);
         }
         if (scales_f32 && gl == 0u) scales_f32[(size_t)r * blocks_per_row + b] = scale;
-        if (scales_e8m0) {
+        if (scales.words) {
             // one byte per 32 columns; this block covers block/32 of them
-            uint8_t* bytes = reinterpret_cast<uint8_t*>(scales_e8m0 + (size_t)r * words128);
             const uint32_t e8 = nvmoe_f32_bits(scale) >> 23;
-            for (uint32_t j = gl; j < block / 32u; j += lanes) bytes[b * (block / 32u) + j] = (uint8_t)e8;
+            for (uint32_t j = gl; j < block / 32u; j += lanes) {
+                *scales.byte_at(r, b * (block / 32u) + j) = (uint8_t)e8;
+            }
         }
     }
 }
 
 __global__ void __launch_bounds__(256) quantize_kernel(const uint16_t* input, uint32_t rows, uint32_t cols,
                                                       uint32_t block, size_t row_stride, uint8_t* q,
-                                                      float* scales_f32, uint32_t* scales_e8m0) {
+                                                      float* scales_f32) {
     grid_dependency_sync();
-    quantize_body([&](uint32_t r) { return input + (size_t)r * row_stride; }, rows, cols, block, q, scales_f32,
-                  scales_e8m0);
+    quantize_body([&](uint32_t r) { return input + (size_t)r * row_stride; }, rows, cols, block, q, scales_f32, ScaleWords{});
 }
 
 __global__ void __launch_bounds__(256) quantize_frames_kernel(const uint32_t* intermediates, uint32_t tokens,
                                                              uint32_t K, uint32_t I, uint32_t block, uint8_t* q,
-                                                             float* scales_f32, uint32_t* scales_e8m0,
-                                                             const uint32_t* written) {
+                                                             float* scales_f32, const uint32_t* written) {
     grid_dependency_sync();
     const uint32_t frame_words = K * (I / 2u) + K;
     quantize_body(
@@ -85,13 +83,13 @@ __global__ void __launch_bounds__(256) quantize_frames_kernel(const uint32_t* in
             if (written && written[r] == kUnboundSlot) return nullptr;
             return reinterpret_cast<const uint16_t*>(intermediates + (size_t)(r / K) * frame_words) + (size_t)(r % K) * I;
         },
-        tokens * K, I, block, q, scales_f32, scales_e8m0);
+        tokens * K, I, block, q, scales_f32, ScaleWords{});
 }
 
 __global__ void __launch_bounds__(256) quantize_grouped_kernel(const void* input, bool frames, const uint32_t* grouped,
                                                               const uint32_t* expert_offsets, uint32_t num_experts,
                                                               uint32_t max_routes, uint32_t K, uint32_t cols, uint32_t I,
-                                                              uint32_t block, uint8_t* q, uint32_t* scales_e8m0,
+                                                              uint32_t block, uint8_t* q, ScaleWords scales,
                                                               const uint32_t* written) {
     grid_dependency_sync();
     const uint32_t total = min(expert_offsets[num_experts], max_routes);
@@ -104,7 +102,7 @@ __global__ void __launch_bounds__(256) quantize_grouped_kernel(const void* input
                                 (size_t)(ri % K) * I
                           : static_cast<const uint16_t*>(input) + (size_t)(ri / K) * cols;
         },
-        total, cols, block, q, nullptr, scales_e8m0);
+        total, cols, block, q, nullptr, scales);
 }
 
 // The common cases of the tensor path's gate/up operands (32- or 128-column blocks, hidden rows 16-byte
@@ -116,11 +114,11 @@ __global__ void __launch_bounds__(256) quantize_grouped_rows_kernel(const uint16
                                                                    const uint32_t* __restrict__ expert_offsets,
                                                                    uint32_t num_experts, uint32_t max_routes, uint32_t K,
                                                                    uint32_t cols, uint8_t* __restrict__ q,
-                                                                   uint32_t* __restrict__ scales_e8m0) {
+                                                                   ScaleWords scales) {
     grid_dependency_sync();
     constexpr uint32_t kBlock = LANES * 8u, kSide = 32u / LANES;
     const uint32_t total_rows = min(expert_offsets[num_experts], max_routes);
-    const uint32_t blocks_per_row = cols / kBlock, words128 = (cols + 127u) / 128u;
+    const uint32_t blocks_per_row = cols / kBlock;
     const uint64_t total = (uint64_t)total_rows * blocks_per_row;
     const uint32_t lane = threadIdx.x & 31u, sub = lane / LANES, part = lane % LANES;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -150,9 +148,7 @@ __global__ void __launch_bounds__(256) quantize_grouped_rows_kernel(const uint16
                           nvmoe_bf16_to_f32(w[3] >> 16) * inv);
         reinterpret_cast<uint2*>(q + (size_t)pos * cols + (size_t)b * kBlock)[part] = out;
         // one scale byte per 32 columns: a block of 128 fills four
-        if (part < kBlock / 32u)
-            reinterpret_cast<uint8_t*>(scales_e8m0 + (size_t)pos * words128)[b * (kBlock / 32u) + part] =
-                (uint8_t)(nvmoe_f32_bits(scale) >> 23);
+        if (part < kBlock / 32u) *scales.byte_at(pos, b * (kBlock / 32u) + part) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
     }
 }
 
@@ -168,8 +164,7 @@ __global__ void __launch_bounds__(256) quantize_grouped_rows_kernel(const uint16
 template <uint32_t LANES>
 __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __restrict__ input, const uint32_t* __restrict__ position,
                                                              uint32_t tokens, uint32_t K, uint32_t cols, uint32_t chunks,
-                                                             uint8_t* __restrict__ q, uint32_t* __restrict__ scales_e8m0,
-                                                             DownRows down) {
+                                                             uint8_t* __restrict__ q, ScaleWords scales, DownRows down) {
     grid_dependency_sync();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t item = blockIdx.x * 4u + (threadIdx.x >> 5);
@@ -181,7 +176,6 @@ __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __
     uint32_t mine_down = zeroes && lane < K ? __ldg(down.position + (size_t)token * K + lane) : kUnboundSlot;
     uint32_t out[4], word;
     quantize_sixteen<LANES>(input + (size_t)token * cols + col, active, lane, out, word);
-    const uint32_t words128 = (cols + 127u) / 128u;
     for (uint32_t r0 = 0; r0 < K; r0 += 32u) {
         if (r0 != 0u) {
             mine = r0 + lane < K ? __ldg(position + (size_t)token * K + r0 + lane) : kUnboundSlot;
@@ -196,29 +190,14 @@ __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __
                     for (uint32_t c = lane * 16u; c < down.cols; c += 512u)
                         *reinterpret_cast<uint4*>(down.q + (size_t)down_row * down.cols + c) = make_uint4(0u, 0u, 0u, 0u);
                     const uint32_t down_words = (down.cols + 127u) / 128u;
-                    for (uint32_t c = lane; c < down_words; c += 32u) down.scales_e8m0[(size_t)down_row * down_words + c] = 0x7f7f7f7fu;
+                    for (uint32_t c = lane; c < down_words; c += 32u) *down.scales.at(down_row, c) = 0x7f7f7f7fu;
                 }
                 continue;
             }
             if (!active) continue;
             *reinterpret_cast<uint4*>(q + (size_t)row * cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
-            if ((lane & 7u) == 0u) scales_e8m0[(size_t)row * words128 + col / 128u] = word;
+            if ((lane & 7u) == 0u) *scales.at(row, col / 128u) = word;
         }
-    }
-}
-
-__global__ void __launch_bounds__(256) scales_to_e8m0_kernel(const float* scales, uint32_t rows, uint32_t cols,
-                                                            uint32_t block, uint32_t* scales_e8m0, uint32_t* status) {
-    const uint32_t blocks_per_row = cols / block;
-    const uint32_t words128 = (cols + 127u) / 128u;
-    const uint64_t total = (uint64_t)rows * blocks_per_row;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = (uint32_t)(i / blocks_per_row), b = (uint32_t)(i % blocks_per_row);
-        const uint32_t bits = nvmoe_f32_bits(scales[i]);
-        // a block-scaled MMA can only take power-of-two scales with a biased exponent in 1..254
-        if ((bits & 0x807fffffu) != 0u || (bits >> 23) == 0u || (bits >> 23) == 255u) raise_status(status, 1u);
-        uint8_t* bytes = reinterpret_cast<uint8_t*>(scales_e8m0 + (size_t)r * words128);
-        for (uint32_t j = 0; j < block / 32u; j++) bytes[b * (block / 32u) + j] = (uint8_t)(bits >> 23);
     }
 }
 
@@ -233,24 +212,24 @@ uint32_t grid_for(uint64_t warps) {
 }  // namespace
 
 void launch_quantize(const uint16_t* input, uint32_t rows, uint32_t cols, uint32_t block, size_t input_row_stride,
-                     uint8_t* q, float* scales_f32, uint32_t* scales_e8m0, cudaStream_t stream) {
+                     uint8_t* q, float* scales_f32, cudaStream_t stream) {
     if (rows == 0u) return;
     launch_chained(quantize_kernel, dim3(grid_for((uint64_t)rows * (cols / block))), dim3(256), 0, stream, input, rows, cols,
-                   block, input_row_stride, q, scales_f32, scales_e8m0);
+                   block, input_row_stride, q, scales_f32);
 }
 
 void launch_quantize_frames(const uint32_t* intermediates, uint32_t tokens, uint32_t K, uint32_t intermediate_size,
-                            uint32_t block, uint8_t* q, float* scales_f32, uint32_t* scales_e8m0, const uint32_t* written,
+                            uint32_t block, uint8_t* q, float* scales_f32, const uint32_t* written,
                             cudaStream_t stream) {
     if (tokens == 0u) return;
     launch_chained(quantize_frames_kernel, dim3(grid_for((uint64_t)tokens * K * (intermediate_size / block))), dim3(256), 0,
-                   stream, intermediates, tokens, K, intermediate_size, block, q, scales_f32, scales_e8m0, written);
+                   stream, intermediates, tokens, K, intermediate_size, block, q, scales_f32, written);
 }
 
 void launch_quantize_grouped(const void* input, bool frames, const uint32_t* grouped_routes,
                              const uint32_t* expert_offsets, uint32_t num_experts, uint32_t max_routes, uint32_t K,
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
-                             uint32_t* scales_e8m0, const uint32_t* written, cudaStream_t stream) {
+                             const ScaleWords& scales, const uint32_t* written, cudaStream_t stream) {
     if (max_routes == 0u) return;
     if (!frames && (block == 32u || block == 128u) && cols % 8u == 0u && (reinterpret_cast<uintptr_t>(input) & 15u) == 0u) {
         const uint32_t side = block == 32u ? 8u : 2u;  // blocks a warp takes at once
@@ -259,16 +238,16 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
         if (blocks > 148u * 64u) blocks = 148u * 64u;
         const auto kernel = block == 32u ? quantize_grouped_rows_kernel<4u> : quantize_grouped_rows_kernel<16u>;
         launch_chained(kernel, dim3((uint32_t)blocks), dim3(256), 0, stream, static_cast<const uint16_t*>(input), grouped_routes,
-                       expert_offsets, num_experts, max_routes, K, cols, q, scales_e8m0);
+                       expert_offsets, num_experts, max_routes, K, cols, q, scales);
         return;
     }
     launch_chained(quantize_grouped_kernel, dim3(grid_for((uint64_t)max_routes * (cols / block))), dim3(256), 0, stream, input,
                    frames, grouped_routes, expert_offsets, num_experts, max_routes, K, cols, intermediate_size, block, q,
-                   scales_e8m0, written);
+                   scales, written);
 }
 
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
-                            uint8_t* q, uint32_t* scales_e8m0, const DownRows& down, cudaStream_t stream) {
+                            uint8_t* q, const ScaleWords& scales, const DownRows& down, cudaStream_t stream) {
     if ((block != 32u && block != 128u) || cols % block != 0u || (reinterpret_cast<uintptr_t>(input) & 15u) != 0u) return false;
     const uint32_t chunks = (cols + 511u) / 512u;
     const uint64_t warps = (uint64_t)tokens * chunks;
@@ -276,17 +255,8 @@ bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_
     if (warps > 0x7fffffffull) return false;
     const auto kernel = block == 32u ? quantize_tokens_kernel<2u> : quantize_tokens_kernel<8u>;
     launch_chained(kernel, dim3((uint32_t)((warps + 3u) / 4u)), dim3(128), 0, stream, static_cast<const uint16_t*>(input), position, tokens,
-                   K, cols, chunks, q, scales_e8m0, down);
+                   K, cols, chunks, q, scales, down);
     return true;
-}
-
-void launch_scales_to_e8m0(const float* scales, uint32_t rows, uint32_t cols, uint32_t block,
-                           uint32_t* scales_e8m0, uint32_t* status, cudaStream_t stream) {
-    if (rows == 0u) return;
-    uint64_t total = (uint64_t)rows * (cols / block);
-    uint32_t blocks = (uint32_t)((total + 255u) / 256u);
-    scales_to_e8m0_kernel<<<blocks > 2368u ? 2368u : blocks, 256, 0, stream>>>(scales, rows, cols, block,
-                                                                               scales_e8m0, status);
 }
 
 }  // namespace nvmoe

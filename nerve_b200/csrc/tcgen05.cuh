@@ -93,6 +93,64 @@ __device__ __forceinline__ bool mbar_wait_winddown(uint64_t* bar, uint32_t parit
 }
 constexpr long long kWinddownCycles = 4000000ll;  // about two milliseconds
 
+// ---- CTA pairs ------------------------------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// address, in the cluster's shared memory window, of the same variable in CTA `rank`
+__device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// all threads of both CTAs: orders what either wrote before it
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// arrival on a barrier of either CTA (`addr` from map_shared)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// mbar_wait, by a whole warp, for what store_async_cluster of the other CTA brings
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, long long limit) {
+    uint32_t ok = 0u;
+    if ((threadIdx.x & 31u) == 0u) {
+        ok = mbar_try_wait_cluster(bar, parity) ? 1u : 0u;
+        const long long start = clock64();
+        while (ok == 0u) {
+            for (int i = 0; i < 64 && ok == 0u; i++) ok = mbar_try_wait_cluster(bar, parity) ? 1u : 0u;
+            if (ok != 0u || *abort_flag) break;
+            if (clock64() - start > limit) {
+                *abort_flag = 1u;
+                break;
+            }
+        }
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0u;
+}
+// sixteen bytes to the other CTA's shared memory, credited to its barrier (both addresses from map_shared)
+__device__ __forceinline__ void store_async_cluster(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(a), "r"(b),
+                 "r"(c), "r"(d), "r"(bar)
+                 : "memory");
+}
+
 // ---- generic-proxy staging into shared memory ---------------------------------------------------
 
 // src_bytes < size zero-fills the rest (src_bytes == 0 reads nothing)
@@ -141,6 +199,20 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void* tenso
         ::"r"(dst_smem), "l"(tensor_map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
         : "memory");
 }
+// The same loads by one CTA of a pair: the box lands in this CTA's shared memory, the barrier (`bar` from map_shared) may
+// be the other CTA's.
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void* tensor_map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst_smem), "l"(tensor_map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* tensor_map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst_smem), "l"(tensor_map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
 // linear copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) credited to the barrier
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -184,6 +256,27 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // arrive on `bar` once every tcgen05 operation this thread issued so far has completed
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+// The same by a CTA pair. Allocation, its permit and release: one warp of each CTA. The others: one thread of the CTA of
+// even rank, for both.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t columns) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(columns)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t columns) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {  // arrives on this CTA's barrier
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair_both(uint64_t* bar) {  // ... and on the other CTA's barrier at the same offset
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3u)
                  : "memory");
 }
 
@@ -236,6 +329,23 @@ __device__ __forceinline__ void tc_mma_block_scaled(uint32_t d_tmem, uint64_t a_
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
+        : "memory");
+}
+
+// Both for a pair: each CTA's block goes from its shared memory to its tensor memory; D and the rows of A are split over
+// the two CTAs (256 rows), each of which holds half the rows of B in shared memory and the scales of all of them in tensor
+// memory. Addresses and descriptors name the same place in both.
+__device__ __forceinline__ void tc_copy_scales_pair(uint32_t taddr, uint64_t desc) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void tc_mma_block_scaled_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                         uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         :
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
         : "memory");

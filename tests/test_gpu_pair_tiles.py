@@ -1,0 +1,101 @@
+"""Expert kernels of CTA pairs (many tokens per expert): the edges of their token tiles, K remainders and row remainders,
+against the CPU checker."""
+import numpy as np
+import pytest
+
+from nerve_b200 import synthetic
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan
+from oracle import moe_oracle as mo
+from oracle import sampled
+from tests.helpers import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    dev = CudaComputeDevice(0)
+    yield dev
+    dev.close()
+
+
+def with_native(case, cfg, seed):
+    tensors = [list(t) for t in (case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)]
+    for e in range(cfg.total_experts - cfg.native_fp8_resources, cfg.total_experts):
+        for i, t in enumerate(synthetic.native_fp8_tensors(cfg, seed, e)):
+            tensors[i][e] = t
+    return tensors
+
+
+# K remainders of either stage (128 columns: one block; 384: a lone whole block after a pair; 576 = 4.5, 320 = 2.5, 704 = 5.5,
+# 448 = 3.5 blocks: a half block after whole pairs, and after a lone block), weight rows that end inside a row tile and after
+# the first of two (384, 576, 704), scale blocks of 32 and 128, a native FP8 resource; token counts per expert that end just
+# before and after a tile's widths (the always-selected resource of the second configuration has every token)
+@pytest.mark.parametrize("name,shape,tokens,native", [
+    ("gpt-oss-20b", (576, 320, 8), 400, 0), ("gpt-oss-20b", (704, 448, 4), 241, 0), ("gpt-oss-20b", (384, 128, 16), 499, 0),
+    ("gpt-oss-20b", (128, 192, 4), 97, 0), ("deepseek-v3", (512, 384, 16), 240, 0), ("deepseek-v3", (640, 256, 16), 481, 1),
+    ("deepseek-v3", (384, 640, 16), 193, 1)])
+def test_layer_matches_the_checker(device, name, shape, tokens, native):
+    cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], *shape), native_fp8_resources=native)
+    assert tokens * cfg.total_k > 96 * cfg.total_experts  # what takes a call to these kernels
+    case = synthetic.make_case(cfg, tokens, seed=17)
+    tensors = with_native(case, cfg, 17)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(2)
+    bank = ExpertBank.upload(device, *tensors)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, device.resident_buffer_from(case.hidden), out, router_weights=device.resident_buffer_from(case.router_w),
+               router_bias=device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+               bias=device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None)
+    logits = mo.linear_bf16(case.hidden, case.router_w, case.router_bias)
+    everyone = np.arange(tokens)
+    want = sampled.layer_on_sample(cfg, case.hidden, logits, case.select_bias, everyone, lambda e: [t[e] for t in tensors])
+    assert_close(out.read(np.uint16).reshape(tokens, cfg.hidden), want["output"], f"{name} {shape} CTA pairs T{tokens}")
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+
+
+# one matrix, every row count of interest: one row over each tile width, the widths, a row over the widest
+@pytest.mark.parametrize("rows,cols,tokens", [(256, 256, 97), (288, 448, 128), (160, 576, 129), (384, 704, 192), (256, 128, 193),
+                                              (320, 192, 240), (544, 320, 241), (1152, 640, 300)])
+def test_dense_linear_matches_the_checker(device, rows, cols, tokens):
+    rng = np.random.default_rng(rows + cols + tokens)
+    cfg = synthetic.MoeConfig("pairs", 256, 256, 8, 2, act_block=32)
+    plan = MoePlan.for_config(device, cfg, 320)
+    plan.set_expert_path(2)
+    x = synthetic.f32_to_bf16(rng.standard_normal((tokens, cols)).astype(np.float32))
+    w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(118, 128, (rows, cols // 32), dtype=np.uint8)
+    out = device.create_resident_buffer(tokens * rows * 2)
+    plan.dense_linear(tokens, device.resident_buffer_from(x), out, device.resident_buffer_from(w), device.resident_buffer_from(s), rows, cols)
+    assert_close(out.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
+    assert plan.status() == 0
+    plan.destroy()
+
+
+def test_a_wait_that_expires_is_reported(device):
+    """An announcement that one CTA of a pair leaves out: both wind down, the call reports it, the next call is whole."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 576, 320, 8)
+    tokens = 400
+    case = synthetic.make_case(cfg, tokens, seed=18)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(2)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw)
+    assert plan.status() == 0
+    before = out.read(np.uint16).copy()
+    plan.set_wait_limit(2_000_000)  # about a millisecond
+    plan.debug_withhold_arrival(True)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw)
+    device.synchronize(timeout_ns=20_000_000_000)
+    assert plan.status() & 8
+    plan.debug_withhold_arrival(False)
+    plan.set_wait_limit(0)
+    for _ in range(2):
+        plan.layer(tokens, bank, hidden, out, router_weights=rw)
+        assert plan.status() == 0
+        np.testing.assert_array_equal(out.read(np.uint16), before)
+    plan.destroy()
+    bank.destroy()
