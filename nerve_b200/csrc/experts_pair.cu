@@ -215,7 +215,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                         const uint32_t a = smem_base + slot * kPairBlocks * kATileBytes;
                         const uint32_t b = smem_base + kPairTokenRegion + slot * kPairBlocks * kPairTokenBytes;
                         const uint32_t sf = smem_base + kPairScaleRegion + slot * kPairScaleBytes;
+                        // the token scales first, which have the longest way to go (of one block, too, the scales of two are
+                        // fetched: zeros, or the next row tile's, that nothing uses)
                         mbar_arrive_expect_tx(&bars->staged[slot], kPairBlocks * kPairScaleWords * 4u);
+                        tma_load_2d(sf + kPairBlocks * kScaleBlockBytes, token_scale_map, (int)(first & ~3u), (int)kb, &bars->staged[slot]);
                         if (rank == 0u) mbar_arrive_expect_tx(&bars->full[slot], (two ? 2u * block_bytes : block_bytes) + 2u * kPairBlocks * kScaleBlockBytes);
                         if (two) {
                             tma_load_3d_pair(a, weight_map + 128u, 0, row0, (int)kb, bar);
@@ -226,9 +229,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                             tma_load_3d_pair(a, weight_map, 0, (int)k64, row0, bar);
                             tma_load_2d_pair(b, token_map, (int)(k64 * 64u), token_row, bar);
                         }
-                        // (of one block, too, the scales of two are fetched: zeros, or the next row tile's, that nothing uses)
                         tma_load_3d_pair(sf, scale_map, 0, source, scale0 + (int)kb, bar);
-                        tma_load_2d(sf + kPairBlocks * kScaleBlockBytes, token_scale_map, (int)(first & ~3u), (int)kb, &bars->staged[slot]);
                     }
                     withhold = false;
                     stage_it++;
