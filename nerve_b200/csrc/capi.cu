@@ -559,6 +559,7 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         nvmoe_plan_destroy(p);
         return code;
     }
+    configure_router_kernels();
     configure_simt_kernels();
     tc_configure_kernels();
     *out = p;

@@ -117,6 +117,7 @@ struct RouterLaunch {  // router.cu
     uint32_t tokens;
     nvmoe_geometry g;
 };
+void configure_router_kernels();
 void launch_router(const RouterLaunch& p, cudaStream_t stream);
 bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selections, no groups: route_token covers it
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,

@@ -335,94 +335,135 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
     }
 }
 
-// The same projection for large batches. What bounds the kernel above there is not the arithmetic but the
-// operands: a block of 4 x 16 pairs reads its 20 rows from L2 for 128 multiply-adds a step, and every weight row is
-// fetched again by every block of four tokens. Here a block of 256 threads owns 32 tokens x 16 outputs: the rows of
-// a 128-column chunk are staged in shared memory by 16-byte asynchronous copies (two buffers, the next chunk lands
-// while this one is used) and shared by the block's eight warps, each of which owns 8 tokens x 8 outputs. A thread
-// plays two of the shader's 64 lanes, l and l + 32, for every pair of its warp's tile: the first butterfly step
-// (lane v with lane v ^ 32) is then an add inside the thread and the other five are the usual shuffles. Sums, their
-// order and the roundings are those of router_linear_kernel, bit for bit.
-constexpr int kTileTokens = 32, kTileOutputs = 16, kSubTokens = 8, kSubOutputs = 8;
+// One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the
+// instruction itself.
+__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
+    float d;
+    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
+    return d;
+}
+
+// The same projection for large batches, bound by the multiply-adds: an SM does 128 a clock, and every other instruction of
+// the loop takes its turn among theirs. A block of 256 threads owns 32 tokens x 16 outputs: the rows of a 512-column chunk are
+// staged in shared memory by 16-byte asynchronous copies, three chunks ahead, one barrier a chunk. A warp owns 16 tokens x 8
+// outputs and half of the shader's 64 lanes, so that 24 words from shared memory serve 256 multiply-adds, which take their
+// operands as bf16: 16384 x 7168 x 256 in 1.46 ms, 70 a clock (with chunks of 256 columns 1.52). With both conversions as
+// instructions of their own, tiles of 8 x 8 for both halves of the lanes, two chunks and two barriers a chunk it was 2.04 ms, 50
+// a clock; with twelve warps 1.40, but 36 us instead of 27 for 4096 x 2880 x 32. (Packed pairs, fma.rn.f32x2, run at 68
+// to 75 whatever surrounds them.) Sums, their order and the roundings are those of router_linear_kernel, bit for bit.
+constexpr int kTileTokens = 32, kTileOutputs = 16, kSubTokens = 16, kSubOutputs = 8;
+constexpr uint32_t kTileRows = kTileTokens + kTileOutputs, kChunkWords = 256, kChunks = 4;
+constexpr uint32_t kRouterTileBytes = kChunks * kTileRows * kChunkWords * 4;
 __global__ void __launch_bounds__(256, 1) router_linear_tiled_kernel(const uint16_t* __restrict__ x,
                                                                     const uint16_t* __restrict__ w,
                                                                     const uint16_t* __restrict__ bias,
                                                                     uint32_t* __restrict__ logits, uint32_t tokens,
                                                                     uint32_t hidden, uint32_t outputs) {
-    constexpr int kRows = kTileTokens + kTileOutputs;
-    __shared__ __align__(16) uint32_t stage[2][kRows][64];   // [buffer][token rows, then output rows][word of the chunk]
+    extern __shared__ __align__(16) uint32_t stage[];  // [buffer][token rows, then output rows][word of the chunk]
     __shared__ float result[kTileTokens][kTileOutputs];
     grid_dependency_sync();
     const uint32_t warp = threadIdx.x >> 5, l = threadIdx.x & 31u;
     const uint32_t t0 = blockIdx.y * kTileTokens, e0 = blockIdx.x * kTileOutputs;
-    const uint32_t ta = (warp >> 1) * kSubTokens, eb = (warp & 1u) * kSubOutputs;  // this warp's corner of the block's tile
+    const uint32_t h = warp & 1u;  // lanes l + 32 h of the shader
+    const uint32_t ta = ((warp >> 1) & 1u) * kSubTokens, eb = (warp >> 2) * kSubOutputs;  // this warp's corner of the block's tile
     const uint32_t words = hidden / 2u;
-    const uint32_t chunks = (words + 63u) / 64u;
+    const uint32_t chunks = (words + kChunkWords - 1u) / kChunkWords;
     const uint32_t* xw = reinterpret_cast<const uint32_t*>(x);
     const uint32_t* ww = reinterpret_cast<const uint32_t*>(w);
-    // the 16-byte pieces of a chunk this thread copies: row = piece / 16, four words from word 4 (piece % 16)
-    auto fetch = [&](uint32_t chunk, uint32_t buffer) {
+    // the 16-byte pieces of a chunk this thread copies: rows threadIdx / 32 + 8 i, four words from word 4 l of each 128
+    const uint32_t* src[kTileRows / 8];
 #pragma unroll
-        for (uint32_t i = 0; i < (kRows * 16u) / 256u; i++) {
-            const uint32_t piece = threadIdx.x + 256u * i;
-            const uint32_t row = piece >> 4, col = (piece & 15u) * 4u;
-            const uint32_t cw = chunk * 64u + col;
-            const bool token_row = row < (uint32_t)kTileTokens;
-            const uint32_t index = token_row ? t0 + row : e0 + row - kTileTokens;
-            const bool ok = cw < words && index < (token_row ? tokens : outputs);
-            const uint32_t* src = ok ? (token_row ? xw : ww) + (size_t)index * words + cw : xw;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&stage[buffer][row][col]);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    float acc[2][kSubTokens][kSubOutputs];
+    for (uint32_t i = 0; i < kTileRows / 8; i++) {
+        const uint32_t row = warp + 8u * i;
+        const bool token_row = row < (uint32_t)kTileTokens;
+        const uint32_t index = token_row ? t0 + row : e0 + row - kTileTokens;
+        src[i] = index < (token_row ? tokens : outputs) ? (token_row ? xw : ww) + (size_t)index * words + 4u * l : nullptr;
+    }
+    auto fetch = [&](uint32_t chunk) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + (chunk % kChunks) * (kTileRows * kChunkWords) + warp * kChunkWords + 4u * l);
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+        for (uint32_t i = 0; i < kTileRows / 8; i++) {
 #pragma unroll
-        for (int a = 0; a < kSubTokens; a++)
-#pragma unroll
-            for (int b = 0; b < kSubOutputs; b++) acc[h][a][b] = 0.0f;
-    fetch(0u, 0u);
-    for (uint32_t chunk = 0; chunk < chunks; chunk++) {
-        const uint32_t buffer = chunk & 1u;
-        if (chunk + 1u < chunks) {
-            fetch(chunk + 1u, buffer ^ 1u);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            // lane l + 32 h of the shader; a lane whose word lies past the row adds nothing (not even zeros: -0 + 0 = +0)
-            if (chunk * 64u + l + 32u * h < words) {
-                uint32_t xr[kSubTokens], wr[kSubOutputs];
-#pragma unroll
-                for (int a = 0; a < kSubTokens; a++) xr[a] = stage[buffer][ta + a][l + 32u * h];
-#pragma unroll
-                for (int b = 0; b < kSubOutputs; b++) wr[b] = stage[buffer][kTileTokens + eb + b][l + 32u * h];
-#pragma unroll
-                for (int a = 0; a < kSubTokens; a++) {
-                    const float xl = nvmoe_bf16_to_f32(xr[a]), xh = nvmoe_bf16_to_f32(xr[a] >> 16);
-#pragma unroll
-                    for (int b = 0; b < kSubOutputs; b++) {
-                        acc[h][a][b] = __fmaf_rn(xl, nvmoe_bf16_to_f32(wr[b]), acc[h][a][b]);
-                        acc[h][a][b] = __fmaf_rn(xh, nvmoe_bf16_to_f32(wr[b] >> 16), acc[h][a][b]);
-                    }
-                }
+            for (uint32_t q = 0; q < kChunkWords; q += 128u) {
+                const bool ok = chunk * kChunkWords + q + 4u * l < words && src[i] != nullptr;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (i * 8u * kChunkWords + q) * 4u),
+                             "l"(ok ? src[i] + chunk * kChunkWords + q : xw), "r"(ok ? 16u : 0u)
+                             : "memory");
             }
         }
-        __syncthreads();  // the buffer is refilled by the fetch of the next round
-    }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    float acc[kSubTokens][kSubOutputs];
 #pragma unroll
     for (int a = 0; a < kSubTokens; a++)
 #pragma unroll
-        for (int b = 0; b < kSubOutputs; b++) {
-            // butterfly step 32 (lane l with lane l + 32) inside the thread, then 16 .. 1 across the warp
-            const float sum = warp_butterfly_sum(__fadd_rn(acc[0][a][b], acc[1][a][b]));
-            if (l == 0u) result[ta + a][eb + b] = sum;
+        for (int b = 0; b < kSubOutputs; b++) acc[a][b] = 0.0f;
+    for (uint32_t c = 0; c + 1u < kChunks; c++) {
+        if (c < chunks) fetch(c);
+        commit();
+    }
+    for (uint32_t chunk = 0; chunk < chunks; chunk++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kChunks - 2) : "memory");
+        __syncthreads();  // this chunk has landed; everyone is through with the one before, whose buffer is filled next
+        if (chunk + kChunks - 1u < chunks) fetch(chunk + kChunks - 1u);
+        commit();
+        const uint32_t* tile = stage + (chunk % kChunks) * (kTileRows * kChunkWords) + 32u * h + l;
+        auto step = [&](uint32_t s) {
+            uint32_t xr[kSubTokens], wr[kSubOutputs];
+#pragma unroll
+            for (int b = 0; b < kSubOutputs; b++) wr[b] = tile[(kTileTokens + eb + b) * kChunkWords + 64u * s];
+#pragma unroll
+            for (int a = 0; a < kSubTokens; a++) xr[a] = tile[(ta + a) * kChunkWords + 64u * s];
+#pragma unroll
+            for (int a = 0; a < kSubTokens; a++) {
+#pragma unroll
+                for (int b = 0; b < kSubOutputs; b++) acc[a][b] = fma_bf16((uint16_t)xr[a], (uint16_t)wr[b], acc[a][b]);
+#pragma unroll
+                for (int b = 0; b < kSubOutputs; b++) acc[a][b] = fma_bf16((uint16_t)(xr[a] >> 16), (uint16_t)(wr[b] >> 16), acc[a][b]);
+            }
+        };
+        if ((chunk + 1u) * kChunkWords <= words) {  // (without a branch between them the second step's words are read under the first's sums)
+#pragma unroll
+            for (uint32_t s = 0; s < kChunkWords / 64; s++) step(s);
+        } else {
+            // a lane whose word lies past the row adds nothing (not even zeros: -0 + 0 = +0)
+#pragma unroll 1
+            for (uint32_t s = 0; s < kChunkWords / 64; s++)
+                if (chunk * kChunkWords + 64u * s + 32u * h + l < words) step(s);
         }
+    }
+    // Butterfly step 32, lane l with lane l + 32: the two warps of a corner hand each other half of their sums (of 8 of the 16
+    // tokens) through the chunk buffers and add. Steps 16 .. 1 fold the remaining 64 sums over the lanes by halves: a sum goes on
+    // in the half of the lanes that its step chooses, with the operands and the order of the full butterfly.
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    constexpr int kHalf = kSubTokens * kSubOutputs / 2;
+    float* exchange = reinterpret_cast<float*>(stage);
+    float v[kHalf];
+#pragma unroll
+    for (int i = 0; i < kHalf; i++) {
+        const float low = acc[i / kSubOutputs][i % kSubOutputs], high = acc[kSubTokens / 2 + i / kSubOutputs][i % kSubOutputs];
+        exchange[(warp * kHalf + i) * 32u + l] = h == 0u ? high : low;
+        v[i] = h == 0u ? low : high;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kHalf; i++) v[i] = __fadd_rn(v[i], exchange[((warp ^ 1u) * kHalf + i) * 32u + l]);
+#pragma unroll
+    for (int o = 16, n = kHalf / 2; o > 0; o >>= 1, n >>= 1) {
+        const bool upper = (l & o) != 0u;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const float kept = upper ? v[i + n] : v[i], given = upper ? v[i] : v[i + n];
+            v[i] = __fadd_rn(kept, __shfl_xor_sync(0xffffffffu, given, o));
+        }
+    }
+    // (lane bits 16 .. 1 chose bits 32 .. 2 of the sum's number; two sums are left to a lane)
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; i++) {
+        const uint32_t n = 2u * l + i;
+        result[ta + h * (kSubTokens / 2) + n / kSubOutputs][eb + n % kSubOutputs] = v[i];
+    }
     __syncthreads();
     const uint32_t out_words = (outputs + 1u) / 2u;
     for (uint32_t i = threadIdx.x; i < kTileTokens * (kTileOutputs / 2); i += 256u) {
@@ -449,6 +490,10 @@ static uint32_t router_total_k(const RouterLaunch& p) {
 bool router_is_small(const RouterLaunch& p) {
     return p.g.routed_experts <= 128u && router_total_k(p) <= 32u && p.g.n_group == 0u && p.g.router_kind <= NVMOE_ROUTER_TOPK_ROUTED &&
            !(p.g.router_kind == NVMOE_ROUTER_TOPK_ROUTED && !p.g.normalize_selected && p.g.activation != NVMOE_ACT_SIGMOID);
+}
+
+void configure_router_kernels() {
+    cudaFuncSetAttribute(router_linear_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouterTileBytes);
 }
 
 void launch_router(const RouterLaunch& p, cudaStream_t stream) {
@@ -496,7 +541,7 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         }
     } else if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u) {
         dim3 grid((outputs + kTileOutputs - 1u) / kTileOutputs, (tokens + kTileTokens - 1u) / kTileTokens);
-        launch_chained(router_linear_tiled_kernel, grid, dim3(256), 0, stream, x, w, bias, logits, tokens, hidden, outputs);
+        launch_chained(router_linear_tiled_kernel, grid, dim3(256), kRouterTileBytes, stream, x, w, bias, logits, tokens, hidden, outputs);
     } else {
         dim3 grid((outputs + 15u) / 16u, (tokens + 3u) / 4u);
         launch_chained(router_linear_kernel<4, 16>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs);

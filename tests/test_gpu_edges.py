@@ -128,6 +128,20 @@ def test_router_projection_tiles(device, tokens, hidden, experts, bias):
     plan.destroy()
 
 
+# the tiled form beyond its ring of four chunks of 512 columns: rows of whole chunks, rows that end in each quarter of one and
+# inside a step, ragged token and output tiles; subnormal inputs count in full
+@pytest.mark.parametrize("tokens,hidden,experts", [(257, 2560, 16), (261, 2592, 18), (257, 2880, 32), (290, 4992, 5), (257, 2432, 17)])
+def test_router_projection_long_rows(device, tokens, hidden, experts):
+    rng = np.random.default_rng(tokens + hidden)
+    plan = plan_of(device, tokens=tokens, hidden=hidden, experts=experts)
+    x, w = bf16(rng.standard_normal((tokens, hidden))), bf16(0.1 * rng.standard_normal((experts, hidden)))
+    x[:, ::7], w[0] = x[:, ::7] & 0x807F, w[0] & 0x807F
+    out = device.create_resident_buffer(tokens * ((experts + 1) // 2) * 4)
+    plan.linear(tokens, device.resident_buffer_from(x), out, device.resident_buffer_from(w), None)
+    np.testing.assert_array_equal(out.read(np.uint32).reshape(tokens, -1), mo.linear_bf16(x, w, None))
+    plan.destroy()
+
+
 # groups of one expert, of two (less than a warp of experts), of 16 and of 32, one beyond the lanes (the shared-memory
 # form), every group kept; logits with ties, infinities and NaN
 @pytest.mark.parametrize("experts,n_group,topk_group,k", [(24, 24, 5, 4), (16, 8, 3, 4), (128, 8, 4, 6), (256, 8, 4, 8), (256, 8, 8, 8),
