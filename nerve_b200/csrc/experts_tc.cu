@@ -605,6 +605,31 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             const uint32_t first = e_begin + n_tile * N_TILE;
             const uint32_t valid = min(N_TILE, e_end - first);
             const uint32_t acc = acc_it % C::kAccStages;
+            // where token j of the tile goes, and its route weight: a chain of two loads. With narrow tiles it is over before the
+            // accumulator is ready, a lane per token; at the end of the kernel nothing else would hide it.
+            uint64_t my_row = 0u;
+            float my_weight = 0.0f;
+            uint32_t my_route = kUnboundSlot;
+            auto find = [&](uint32_t j, bool active) {
+                my_row = 0u;
+                my_weight = 0.0f;
+                my_route = kUnboundSlot;
+                if (!active || j >= valid) return;
+                const uint32_t ri = __ldg(p.work.grouped_routes + first + j);
+                // the row of the down stage's operand matrix that this route's activations go to
+                my_route = (GATE_UP && p.q_out != nullptr) ? __ldg(p.down_position + ri) : kUnboundSlot;
+                if (GATE_UP) {
+                    if (p.intermediates != nullptr) my_row = reinterpret_cast<uint64_t>(reinterpret_cast<uint16_t*>(p.intermediates + (size_t)(ri / K) * frame_words) +
+                                                        (size_t)(ri % K) * I);
+                } else if (p.partial_outputs != nullptr) {
+                    my_row = reinterpret_cast<uint64_t>(p.partial_outputs + (size_t)ri * H);
+                } else {
+                    my_row = reinterpret_cast<uint64_t>(p.outputs + (size_t)ri * H);
+                    my_weight = nvmoe_bf16_to_f32(__ldg(p.routes + ri) >> 16);
+                }
+            };
+            constexpr bool kNarrow = N_TILE <= 32u;
+            if (kNarrow) find(lane, true);
             const long long e0 = TRACE ? clock64() : 0;
             // One warp watches the accumulator's barrier; the others sleep on a hardware barrier until it has a
             // verdict. A warp that polls takes issue slots from whatever shares its scheduler, and the epilogue warps
@@ -650,25 +675,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 uint32_t d0[16], d1[16];
                 tmem_ld16(lane_addr + c0, d0);
                 if (C::kMatrices == 2u) tmem_ld16(lane_addr + N_TILE + c0, d1);  // up, or the second 128 rows
-                // lane j < 16 works out where token c0 + j of the tile goes (and its route weight)
-                // while the accumulators arrive; the sixteen results are then handed round by shuffles
-                uint64_t my_row = 0u;
-                float my_weight = 0.0f;
-                uint32_t my_route = kUnboundSlot;
-                if (lane < 16u && c0 + lane < valid) {
-                    const uint32_t ri = __ldg(p.work.grouped_routes + first + c0 + lane);
-                    // the row of the down stage's operand matrix that this route's activations go to
-                    my_route = (GATE_UP && p.q_out != nullptr) ? __ldg(p.down_position + ri) : kUnboundSlot;
-                    if (GATE_UP) {
-                        if (p.intermediates != nullptr) my_row = reinterpret_cast<uint64_t>(reinterpret_cast<uint16_t*>(p.intermediates + (size_t)(ri / K) * frame_words) +
-                                                            (size_t)(ri % K) * I);
-                    } else if (p.partial_outputs != nullptr) {
-                        my_row = reinterpret_cast<uint64_t>(p.partial_outputs + (size_t)ri * H);
-                    } else {
-                        my_row = reinterpret_cast<uint64_t>(p.outputs + (size_t)ri * H);
-                        my_weight = nvmoe_bf16_to_f32(__ldg(p.routes + ri) >> 16);
-                    }
-                }
+                // lane j < 16 works out where token c0 + j of the tile goes (and its route weight) while the accumulators arrive; the
+                // sixteen results are then handed round by shuffles. (A narrow tile has done so for all its tokens by now.)
+                if (!kNarrow) find(c0 + lane, lane < 16u);
+                const uint32_t t0 = kNarrow ? c0 : 0u;  // the lane that knows token c0
                 tmem_ld_wait();
                 if (head) {
                     tc_fence_before();
@@ -691,7 +701,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                             bits[t] = swiglu_bf16_bits(__uint_as_float(d0[j]), __uint_as_float(d1[j]), p.g.swiglu_limit,
                                                        p.g.swiglu_alpha, p.g.swiglu_up_offset);
                         } else {
-                            const float weight = __shfl_sync(0xffffffffu, my_weight, j);
+                            const float weight = __shfl_sync(0xffffffffu, my_weight, t0 + j);
                             bits[t] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(d0[j]), weight)));
                         }
                     }
@@ -700,7 +710,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         // only after the participants' planes have been added
 #pragma unroll
                         for (uint32_t t = 0; t < 4u; t++) {
-                            float* out = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, my_row, g0 + t));
+                            float* out = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, my_row, t0 + g0 + t));
                             if (c0 + g0 + t < valid && row_ok) out[row] = __uint_as_float(d0[g0 + t]);
                             if (ROW_PAIR && c0 + g0 + t < valid && row + kBlockM < out_rows) out[row + kBlockM] = __uint_as_float(d1[g0 + t]);
                         }
@@ -709,10 +719,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                     if (store_rows) {
 #pragma unroll
                     for (uint32_t t = 0; t < 4u; t++) {
-                        uint16_t* out = reinterpret_cast<uint16_t*>(__shfl_sync(0xffffffffu, my_row, g0 + t));
+                        uint16_t* out = reinterpret_cast<uint16_t*>(__shfl_sync(0xffffffffu, my_row, t0 + g0 + t));
                         if (c0 + g0 + t < valid && row_ok) out[row] = (uint16_t)bits[t];
                         if (ROW_PAIR) {  // the second accumulator holds the next 128 output rows of the same tokens
-                            const float weight = __shfl_sync(0xffffffffu, my_weight, g0 + t);
+                            const float weight = __shfl_sync(0xffffffffu, my_weight, t0 + g0 + t);
                             const uint32_t second = (uint32_t)__bfloat16_as_ushort(
                                 __float2bfloat16_rn(__fmul_rn(__uint_as_float(d1[g0 + t]), weight)));
                             if (c0 + g0 + t < valid && row + kBlockM < out_rows) out[row + kBlockM] = (uint16_t)second;
@@ -748,7 +758,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         const bool writes_scale = lane == 0u && first_row < out_rows;
 #pragma unroll
                         for (uint32_t t = 0; t < 4u; t++) {
-                            const uint32_t dp = __shfl_sync(0xffffffffu, my_route, g0 + t);
+                            const uint32_t dp = __shfl_sync(0xffffffffu, my_route, t0 + g0 + t);
                             const float scale = nvmoe_rounded_fp8_scale(m[t]);
                             // 1 / scale, exact: the scale is a power of two with a biased exponent in [107, 247]
                             const float inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));
