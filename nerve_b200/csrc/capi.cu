@@ -112,7 +112,7 @@ struct ExpertSet {
     }
 };
 constexpr size_t kMaxExpertSets = 64;
-constexpr size_t kMapTemplates = 5u * 128u;  // bytes of a stage's template tensor maps
+constexpr size_t kMapTemplates = (2u * kWeightMaps + 1u) * 128u;  // bytes of a stage's template tensor maps
 constexpr int kHostWaitSeconds = 60;  // how long the host-buffer layer call waits for its result
 
 enum Stage { kStageLinear, kStageRoute, kStageSchedule, kStageQuantX, kStageGateUp, kStageQuantI, kStageDown, kStageReduce, kStageCount };
@@ -519,8 +519,8 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
                 for (uint32_t i = 0; i < kTokenMaps && ok; i++)
                     ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
                 if (cols % 64u != 0u || cols < 128u) continue;  // (no map for its weights either)
-                for (uint32_t i = 0; i < 4u && ok; i++)
-                    ok = tc_encode_pair_token_map(mine + (kPairTokenMap + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[1u + i]);
+                for (uint32_t i = 0; i < kTokenMaps && ok; i++)
+                    ok = tc_encode_pair_token_map(mine + (kTokenMaps + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
                 ok = ok && tc_encode_token_scale_map(mine + kTokenScaleMap * 128u, p->grouped_e8m0[set].ptr, scale_rows(p), (cols + 127u) / 128u);
             }
             if (ok) {
@@ -532,19 +532,20 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         }
         want(p->tmap_templates, 2u * kMapTemplates);
         if (err == cudaSuccess) {
-            // per stage: the maps of the compact form (boxes of one K block, of two), those of the one-byte-per-element forms (left
-            // zero when the shape has no whole 128-column blocks: such resources are then treated as not resident), the map
-            // of the derived scales
+            // per stage: the maps of the compact form, those of the one-byte-per-element forms (left zero when the shape has no
+            // whole 128-column blocks: such resources are then treated as not resident), the map of the derived scales
             unsigned char maps[2u * kMapTemplates] = {0};
             for (uint32_t set = 0; set < 2u; set++) {
                 const uint32_t rows = set == 0u ? g.intermediate_size : g.hidden_size, cols = set == 0u ? g.hidden_size : g.intermediate_size;
                 unsigned char* mine = maps + set * kMapTemplates;
                 const uint64_t blocks = tc_derived_scale_bytes(rows, cols) / 512u * p->experts;
-                p->tma[set] = p->act_maps.ptr && tc_encode_weight_map(mine, p->tmap_templates.ptr, rows, cols) &&
-                              tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false) && blocks <= 0x7fffffffull &&
-                              tc_encode_pair_scale_map(mine + 512, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks);
-                tc_encode_weight_map_bytes(mine + 256, p->tmap_templates.ptr, rows, cols);
-                tc_encode_pair_weight_map(mine + 384, p->tmap_templates.ptr, rows, cols, true);
+                p->tma[set] = p->act_maps.ptr && tc_encode_weight_map(mine, p->tmap_templates.ptr, rows, cols, 128u) &&
+                              tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false) &&
+                              tc_encode_weight_map(mine + 256, p->tmap_templates.ptr, rows, cols, 256u) && blocks <= 0x7fffffffull &&
+                              tc_encode_pair_scale_map(mine + 768, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks);
+                tc_encode_weight_map_bytes(mine + 384, p->tmap_templates.ptr, rows, cols, 128u);
+                tc_encode_pair_weight_map(mine + 512, p->tmap_templates.ptr, rows, cols, true);
+                tc_encode_weight_map_bytes(mine + 640, p->tmap_templates.ptr, rows, cols, 256u);
             }
             err = cudaMemcpyAsync(p->tmap_templates.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
             if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
@@ -786,7 +787,7 @@ static int expert_set_for(nvmoe_plan* p, int set, const nvmoe_buffer* addresses,
                                            : tc_derived_scale_bytes(g.hidden_size, g.intermediate_size);
         NVMOE_CUDA(p->device, found->derived.ensure((size_t)p->experts * matrices * per_matrix));
         NVMOE_CUDA(p->device, found->stamps.ensure((size_t)p->experts * matrices * 16u));
-        NVMOE_CUDA(p->device, found->tmaps.ensure((size_t)p->experts * matrices * 256u + 128u));
+        NVMOE_CUDA(p->device, found->tmaps.ensure(((size_t)p->experts * matrices * kWeightMaps + 1u) * 128u));
         NVMOE_CUDA(p->device, cudaMemsetAsync(found->stamps.ptr, 0, found->stamps.bytes, p->device->stream));
         found->resolved = found->tensor_ready = false;  // the resolved pointers name the derived copies
     }
@@ -1251,7 +1252,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         int rc = NVMOE_OK;
         const bool tensor_shape = tc_shape_supported(g);
         if (fresh.unit_routes.ensure((size_t)g.max_tokens * 4u) != cudaSuccess || fresh.set.ptrs.ensure(sizeof(ExpertPtrs)) != cudaSuccess ||
-            (tensor_shape && (fresh.set.derived.ensure(tc_derived_scale_bytes(rows, cols)) != cudaSuccess || fresh.set.tmaps.ensure(384u) != cudaSuccess)))
+            (tensor_shape && (fresh.set.derived.ensure(tc_derived_scale_bytes(rows, cols)) != cudaSuccess || fresh.set.tmaps.ensure((kWeightMaps + 1u) * 128u) != cudaSuccess)))
             rc = fail(d, NVMOE_ERR_OUT_OF_MEMORY, "dense linear: out of device memory");
         if (rc == NVMOE_OK) {
             std::vector<uint32_t> ones(g.max_tokens, 0x3f80u << 16);  // weight 1.0, resource 0
@@ -1262,7 +1263,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
             if (fresh.plan->tma[1]) {
                 if (!tc_encode_pair_scale_map(map, fresh.set.derived.ptr, 1u, (uint32_t)(tc_derived_scale_bytes(rows, cols) / 512u)))
                     fresh.plan->tma[1] = false;
-                else if (cudaMemcpy(fresh.set.tmaps.as<uint8_t>() + 256, map, 128, cudaMemcpyHostToDevice) != cudaSuccess)
+                else if (cudaMemcpy(fresh.set.tmaps.as<uint8_t>() + kWeightMaps * 128u, map, 128, cudaMemcpyHostToDevice) != cudaSuccess)
                     rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the scale map");
             }
         }

@@ -236,8 +236,8 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     uint16_t* outputs;           // down output [T][K][H]
     float* partial_outputs;      // down, tensor-parallel form: raw f32 sums [T][K][H] instead of `outputs` (no route weight, no rounding)
     uint32_t* status;
-    const uint8_t* tmaps;        // tensor path: tensor maps [expert][matrix][boxes of one K block, of two][128 bytes], then that of
-                                 // the derived scales; null = move weights with cp.async
+    const uint8_t* tmaps;        // tensor path: tensor maps [expert][matrix][kWeightMaps][128 bytes], then that of the derived scales;
+                                 // null = move weights with cp.async
     // tensor path: act_q / act_e8m0 hold expert-grouped rows (row = position in grouped_routes);
     // act_tmap is the tensor map of act_q with a box of [token tile][128 bytes] (null: fetch rows with cp.async); for CTA
     // pairs the first of those of half tiles

@@ -153,8 +153,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     grid_dependency_sync();
     const uint32_t tile_count = *list.count * m_tiles;
     // (a tensor map written by an earlier kernel is acquired once per block before the TMA unit gets it)
-    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources + 1u; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u);
-    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u + 128u);
+    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources + 1u; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * kWeightMaps * 128u);
+    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources; m += blockDim.x) tensormap_acquire(p.tmaps + ((size_t)m * kWeightMaps + 1u) * 128u);
     if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
     __syncthreads();
 
@@ -179,7 +179,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             };
             const uint64_t begin = p.cta_trace ? global_timer_ns() : 0u;
             const uint32_t smem_base = smem_u32(smem), full0 = map_shared(smem_u32(&bars->full[0]), 0u);
-            const uint8_t* scale_map = p.tmaps + (size_t)p.work.num_experts * kSources * 256u;
+            const uint8_t* scale_map = p.tmaps + (size_t)p.work.num_experts * kSources * kWeightMaps * 128u;
             const uint8_t* token_scale_map = p.act_tmap + (kTokenScaleMap - 1u) * 128u;
             uint32_t slot = 0u, empty_parity = 1u, stage_it = 0u;
             bool alive = true, withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
@@ -192,7 +192,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                 const uint32_t expert = cur.pair >> 16;
                 const uint32_t first = first_row_of(cur.pair & 0xffffu, cur.e_begin);
                 const uint32_t columns = columns_for(min(p.token_rows, cur.e_end - first));
-                const uint8_t* weight_map = p.tmaps + (size_t)(GATE_UP ? 2u * expert + rank : expert) * 256u;
+                const uint8_t* weight_map = p.tmaps + (size_t)(GATE_UP ? 2u * expert + rank : expert) * kWeightMaps * 128u;
                 const uint8_t* token_map = p.act_tmap + (columns - 1u) / 64u * 128u;
                 const int row0 = (int)(GATE_UP ? cur.m_tile * kBlockM : (2u * cur.m_tile + rank) * kBlockM);
                 // (a second tile past the last rows borrows the first's scale blocks: its weights arrive as zeros)
@@ -222,7 +222,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                         if (rank == 0u) mbar_arrive_expect_tx(&bars->full[slot], (two ? 2u * block_bytes : block_bytes) + 2u * kPairBlocks * kScaleBlockBytes);
                         if (two) {
                             tma_load_3d_pair(a, weight_map + 128u, 0, row0, (int)kb, bar);
-                            tma_load_3d_pair(b, token_map + (kPairTokenMap - 1u) * 128u, 0, token_row, (int)kb, bar);
+                            tma_load_3d_pair(b, token_map + kTokenMaps * 128u, 0, token_row, (int)kb, bar);
                         } else {
                             // in units of 64 columns: a trailing half block ends with the row
                             const uint32_t k64 = min(2u * kb, k_dim / 64u - 2u);

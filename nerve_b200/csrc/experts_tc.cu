@@ -19,10 +19,10 @@
 // issues the scale copies and MMAs; one lane of warp 5 issues TMA loads of whole 128 x 128 boxes of
 // weight codes through a per-expert tensor map (the template map with the expert's address patched in
 // on the device; the padded 4-bit tensor-map type spreads the codes into the 16-byte slots the f8f6f4
-// kinds read and applies the 128-byte swizzle); warps 6.. stage the token rows, the scales and any
-// trailing partial K block with cp.async whose completion arrives on the stage's mbarrier without
-// stalling the issuer.  Shapes the tensor map cannot describe (K % 64 != 0) move the weights with
-// cp.async too: 8-byte pieces into the low half of the 16-byte slots.  Token rows are gathered
+// kinds read and applies the 128-byte swizzle) and of the token rows; warp 6 stores the token scales.
+// Shapes the tensor map cannot describe (K % 64 != 0) stage everything with cp.async by warps 6..,
+// whose completion arrives on the stage's mbarrier without stalling the issuer: the codes in 8-byte
+// pieces into the low half of the 16-byte slots.  Token rows are gathered
 // through the expert-grouped route list (the permutation costs no pass of its own), and E8M0 scales
 // come as ready 32x16-byte blocks (the layout tcgen05.cp expands into TMEM) from a derived copy of
 // the packaged scale tensors that is rebuilt whenever a scale record's address or generation
@@ -65,11 +65,11 @@ struct Config {
     // cp.async producers: one warp sustains only about one copy instruction every 60-130 cycles, so the
     // copies of a stage are spread over eight warps (with TMA for the weights: token rows on the first
     // four, scales on the other four)
-    // With TMA two cp.async warps are left with the token scales and a trailing partial K block, and the
-    // warps they free become epilogue warps: the epilogue (activation, rounding, re-quantisation: a
-    // couple of hundred instructions per value) is what large token tiles wait for, and a warp only
-    // issues one instruction at a time. Epilogue warps come in groups of four, one per quadrant of
-    // tensor-memory lanes (a warp reads the quadrant warp_id % 4); the groups share out a tile's columns.
+    // With TMA one warp is left with the token scales (a second idles, so that the ones after it keep warp % 4), and the warps
+    // this frees become epilogue warps: the epilogue (activation, rounding, re-quantisation: a couple of hundred instructions
+    // per value) is what large token tiles wait for, and a warp only issues one instruction at a time. Epilogue warps come in
+    // groups of four, one per quadrant of tensor-memory lanes (a warp reads the quadrant warp_id % 4); the groups share out a
+    // tile's columns.
     static constexpr uint32_t kProducerWarps = USE_TMA ? 2u : 8u;
     static constexpr uint32_t kProducerThreads = 32u * kProducerWarps;
     static constexpr uint32_t kRowsPerPass = kProducerThreads / 8u;  // eight threads cover the 128 bytes of one row
@@ -90,11 +90,18 @@ struct Config {
     // slots and six.
     static constexpr uint32_t kScaleStride = kSources * kScaleBlockBytes;      // between K blocks of the derived weight scales
     static constexpr uint32_t kABytes = kMatrices * kATileBytes;               // weight tiles of one K block
-    // weight scale blocks, then the token scale block: 32 entries of 16 bytes, entry n % 32 holding token n's scales.
+    // weight scale blocks and the token scale block: 32 entries of 16 bytes, entry n % 32 holding token n's scales.
     // A tile of 16 tokens fills half of it; the copy into tensor memory still reads 512 bytes, the second half
     // being whatever follows in shared memory (the next block's scales, or the barriers): scales of token columns
     // that do not exist.
     static constexpr uint32_t kSfBytes = kMatrices * kScaleBlockBytes + (N_TILE <= 16u ? kScaleBlockBytes / 2u : kScaleBlockBytes);
+    // offsets in the scale region: a slot's weight scale blocks (neighbouring K blocks come in one copy), then its token scales
+    static constexpr uint32_t weight_scales(uint32_t slot, uint32_t sub, uint32_t mx) {
+        return slot * kSub * kSfBytes + (sub * kMatrices + mx) * kScaleBlockBytes;
+    }
+    static constexpr uint32_t token_scales(uint32_t slot, uint32_t sub) {
+        return slot * kSub * kSfBytes + kSub * kMatrices * kScaleBlockBytes + sub * (kSfBytes - kMatrices * kScaleBlockBytes);
+    }
     static constexpr uint32_t kStageBytes = kSub * (kABytes + kBTileBytes + kSfBytes);
     static constexpr uint32_t kBarrierBytes = 256u + (GATE_UP ? 64u * kEpilogueGroups : 0u);  // barriers, then the block maxima
     // The arrays start at the first 1024-byte boundary of the dynamic shared memory. Room for that round-up is set
@@ -175,7 +182,11 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     const uint32_t k_dim = GATE_UP ? H : I;
     const uint32_t out_rows = GATE_UP ? I : H;
     const uint32_t k_blocks = (k_dim + kBlockK - 1u) / kBlockK;
-    const uint32_t k_stages = (k_blocks + C::kSub - 1u) / C::kSub;
+    // K blocks of a stage. By TMA a stage of two brings whole blocks only, both in one copy; a lone whole block and a trailing
+    // half one are stages of their own.
+    const uint32_t doubles = C::kSub == 2u ? (USE_TMA ? k_dim / kBlockK / 2u : k_blocks / 2u) : 0u;
+    const uint32_t k_stages = k_blocks - doubles;
+    auto first_block = [&](uint32_t ks) { return ks < doubles ? 2u * ks : doubles + ks; };
     const uint32_t m_tiles = (out_rows + C::kTileRows - 1u) / C::kTileRows;   // tiles along the weight rows
     const uint32_t row_tiles = (out_rows + kBlockM - 1u) / kBlockM;           // 128-row tiles (scale blocks are kept per these)
     // the derived scale blocks of matrix mx of tile m_tile (a second half past the last rows borrows the first's:
@@ -191,7 +202,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     // ---- one-time setup ---------------------------------------------------------------------
     if (threadIdx.x == 0u) {
         for (uint32_t s = 0; s < C::kStages; s++) {
-            mbar_init(&bars->full[s], kProducerThreads + (USE_TMA ? 1u : 0u));
+            mbar_init(&bars->full[s], USE_TMA ? 2u : kProducerThreads);  // TMA: the announcement of the copies, the scale warp
             mbar_init(&bars->empty[s], 1u);
         }
         for (uint32_t a = 0; a < 2u; a++) {
@@ -227,8 +238,12 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         // acquire such a map once before any of its threads hands it to the TMA unit; further uses by the
         // block need no fence. All threads share the maps out, so that the block pays one fence latency here
         // instead of one per map in the lane that issues the loads.
-        for (uint32_t m = threadIdx.x; m < p.work.num_experts * C::kSources; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * 256u);
-        if (threadIdx.x == 0u) tensormap_acquire(p.act_tmap);
+        for (uint32_t m = threadIdx.x; m < p.work.num_experts * C::kSources; m += blockDim.x) {
+            const uint8_t* maps = p.tmaps + (size_t)m * kWeightMaps * 128u;
+            tensormap_acquire(maps + (ROW_PAIR ? 256u : 0u));
+            if (C::kSub == 2u) tensormap_acquire(maps + 128u);
+        }
+        if (threadIdx.x < C::kSub) tensormap_acquire(p.act_tmap + threadIdx.x * kTokenMaps * 128u);
         __syncthreads();
     }
 
@@ -272,7 +287,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 if (tile + gridDim.x < tile_count) meta_of(tile + gridDim.x, pair_nxt, nxt);
                 const uint32_t m_tile = cur.m_tile;
                 const int row0 = (int)(m_tile * C::kTileRows);
-                const uint8_t* maps = p.tmaps + (size_t)(cur.pair >> 16) * C::kSources * 256u;
+                const uint8_t* maps = p.tmaps + (size_t)(cur.pair >> 16) * C::kSources * kWeightMaps * 128u;
                 // first operand row of this token tile in the expert-grouped activation matrix
                 const int token0 = (int)(cur.expert_begin + (cur.pair & 0xffffu) * N_TILE);
                 const uint8_t* scale_blocks[C::kMatrices];
@@ -284,44 +299,43 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         alive = false;
                         break;
                     }
-                    // whole K blocks of this stage come by TMA; a trailing partial one is staged by the cp.async warps
-                    uint32_t whole = 0u, present = 0u;
-#pragma unroll
-                    for (uint32_t sub = 0; sub < C::kSub; sub++) {
-                        whole += ((ks * C::kSub + sub + 1u) * kBlockK <= k_dim) ? 1u : 0u;
-                        present += (ks * C::kSub + sub < k_blocks) ? 1u : 0u;
-                    }
+                    const bool two = ks < doubles;
+                    const uint32_t kb = first_block(ks), present = two ? 2u : 1u;
                     if (withhold) {
                         withhold = false;
                     } else {
-                    // token rows (zeros past the edge of K) and weight scale blocks of every K block present
+                    // the K blocks' weight codes, token rows and weight scales: one copy each (gate and up: one each for the codes)
+                    const uint32_t block = slot * C::kSub;  // index into the shared-memory arrays
                     const uint32_t smem_base = smem_u32(smem);
+                    const uint32_t a = smem_base + block * C::kABytes, b = smem_base + C::kBRegion + block * C::kBTileBytes;
+                    const uint32_t sf = smem_base + C::kSfRegion + C::weight_scales(slot, 0u, 0u);
                     // a box of one-byte elements brings twice the bytes of a box of packed 4-bit codes
                     const uint32_t box_bytes = cur.format == kFormatCompact ? kTmaBoxBytes : 2u * kTmaBoxBytes;
                     *reinterpret_cast<volatile uint32_t*>(&bars->format[slot]) = cur.format;
-                    mbar_arrive_expect_tx(&bars->full[slot], whole * C::kMatrices * box_bytes +
-                                                                 present * (C::kBTileBytes + C::kMatrices * kScaleBlockBytes));
-                    for (uint32_t sub = 0; sub < present; sub++) {
-                        const uint32_t kb = ks * C::kSub + sub;
-                        const uint32_t block = slot * C::kSub + sub;  // index into the three shared-memory arrays
-                        if (sub < whole) {
-#pragma unroll
-                            for (uint32_t mx = 0; mx < C::kMatrices; mx++)
-                                tma_load_3d(smem_base + block * C::kABytes + mx * kATileBytes, maps + C::source_of(mx) * 256u, 0, (int)(2u * kb),
-                                            row0 + (int)C::row_shift(mx), &bars->full[slot]);  // rows past the matrix: zeros
-                        }
-                        tma_load_2d(smem_base + C::kBRegion + block * C::kBTileBytes, p.act_tmap, (int)(kb * kBlockK), token0,
-                                    &bars->full[slot]);
-                        if (C::kSources == 2u) {
-                            // the gate and the up block of this (row tile, K block) are neighbours in the derived copy
-                            bulk_copy_g2s(smem_base + C::kSfRegion + block * C::kSfBytes, scale_blocks[0] + (size_t)kb * C::kScaleStride,
-                                          2u * kScaleBlockBytes, &bars->full[slot]);
+                    mbar_arrive_expect_tx(&bars->full[slot], present * (C::kMatrices * box_bytes + C::kBTileBytes + C::kMatrices * kScaleBlockBytes));
+                    // (rows past the matrix arrive as zeros)
+                    if (two) {
+                        tma_load_3d(a, maps + 128u, 0, row0, (int)kb, &bars->full[slot]);
+                        tma_load_3d(b, p.act_tmap + kTokenMaps * 128u, 0, token0, (int)kb, &bars->full[slot]);
+                    } else {
+                        // in units of 64 columns: a trailing half block comes as a whole one that ends with the row
+                        const uint32_t k64 = min(2u * kb, k_dim / 64u - 2u);
+                        if (ROW_PAIR) {
+                            tma_load_3d(a, maps + 256u, 0, (int)k64, row0, &bars->full[slot]);
                         } else {
 #pragma unroll
-                            for (uint32_t mx = 0; mx < C::kMatrices; mx++)
-                                bulk_copy_g2s(smem_base + C::kSfRegion + block * C::kSfBytes + mx * kScaleBlockBytes,
-                                              scale_blocks[mx] + (size_t)kb * C::kScaleStride, kScaleBlockBytes, &bars->full[slot]);
+                            for (uint32_t src = 0; src < C::kSources; src++)
+                                tma_load_3d(a + src * kATileBytes, maps + src * (kWeightMaps * 128u), 0, (int)k64, row0, &bars->full[slot]);
                         }
+                        tma_load_2d(b, p.act_tmap, (int)(k64 * 64u), token0, &bars->full[slot]);
+                    }
+                    if (ROW_PAIR) {
+#pragma unroll
+                        for (uint32_t mx = 0; mx < C::kMatrices; mx++)
+                            bulk_copy_g2s(sf + mx * kScaleBlockBytes, scale_blocks[mx] + (size_t)kb * C::kScaleStride, kScaleBlockBytes, &bars->full[slot]);
+                    } else {
+                        // the gate and the up block of this (row tile, K block) are neighbours in the derived copy, and so are two K blocks
+                        bulk_copy_g2s(sf, scale_blocks[0] + (size_t)kb * C::kScaleStride, present * C::kMatrices * kScaleBlockBytes, &bars->full[slot]);
                     }
                     }
                     stage_it++;
@@ -345,7 +359,70 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 }
             }
         }
-    } else if (warp >= 6u && warp < 6u + C::kProducerWarps) {
+    } else if (USE_TMA && warp >= 6u && warp < 6u + C::kProducerWarps) {
+        // ===== token scales (one warp): a lane per token, words fetched four stages ahead and stored to the stage's block =====
+        // (As 4-byte asynchronous copies that arrived on the barrier by themselves, by 64 threads, with the trailing half block of
+        // the weights, they were the last operands of many stages: layer of 64 tokens of 32 experts of 2880 x 2880 122.5 us, 114.7 this way.)
+        if (warp == 6u) {
+            constexpr uint32_t kAhead = 4u, kPer = (N_TILE + 31u) / 32u;
+            struct Meta {
+                uint32_t first, valid;
+            };
+            auto load_meta = [&](uint32_t tile, Meta& m) {
+                const uint32_t pair = __ldg(list.tiles + tile / m_tiles), expert = pair >> 16;
+                m.first = __ldg(p.work.expert_offsets + expert) + (pair & 0xffffu) * N_TILE;
+                m.valid = min(N_TILE, __ldg(p.work.expert_offsets + expert + 1u) - m.first);
+            };
+            uint32_t slot = 0u, empty_parity = 1u;
+            bool alive = true;
+            Meta cur{}, nxt{};
+            if (blockIdx.x < tile_count) load_meta(blockIdx.x, cur);
+            for (uint32_t tile = blockIdx.x; tile < tile_count && alive; tile += gridDim.x) {
+                const uint32_t* row = p.act_e8m0.words + (size_t)(cur.first + lane) * k_blocks;
+                const uint32_t valid = cur.valid;
+                uint32_t w[kAhead][C::kSub][kPer];
+                auto fetch = [&](uint32_t ks, uint32_t (&into)[C::kSub][kPer]) {
+#pragma unroll
+                    for (uint32_t sub = 0; sub < C::kSub; sub++) {
+#pragma unroll
+                        for (uint32_t i = 0; i < kPer; i++) {
+                            const bool ok = ks < k_stages && (sub == 0u || ks < doubles) && lane + 32u * i < valid;
+                            into[sub][i] = ok ? __ldg(row + (size_t)(32u * i) * k_blocks + first_block(ks) + sub) : 0u;
+                        }
+                    }
+                };
+#pragma unroll
+                for (uint32_t u = 0; u < kAhead; u++) fetch(u, w[u]);
+                if (tile + gridDim.x < tile_count) load_meta(tile + gridDim.x, nxt);
+                for (uint32_t ks0 = 0; ks0 < k_stages && alive; ks0 += kAhead) {
+#pragma unroll
+                    for (uint32_t u = 0; u < kAhead; u++) {
+                        if (ks0 + u >= k_stages) break;
+                        if (!mbar_wait_warp(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
+                            alive = false;
+                            break;
+                        }
+#pragma unroll
+                        for (uint32_t sub = 0; sub < C::kSub; sub++) {
+                            uint32_t* block = reinterpret_cast<uint32_t*>(smem + C::kSfRegion + C::token_scales(slot, sub));
+#pragma unroll
+                            for (uint32_t i = 0; i < kPer; i++)
+                                if (lane + 32u * i < N_TILE) block[lane * 4u + i] = w[u][sub][i];
+                        }
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0u) mbar_arrive(&bars->full[slot]);
+                        fetch(ks0 + u + kAhead, w[u]);
+                        if (++slot == C::kStages) {
+                            slot = 0u;
+                            empty_parity ^= 1u;
+                        }
+                    }
+                }
+                cur = nxt;
+            }
+        }
+    } else if (!USE_TMA && warp >= 6u && warp < 6u + C::kProducerWarps) {
         // ===== operand producers: cp.async into the swizzled tiles, completion arrives on `full` =====
         const uint32_t pt = threadIdx.x - kFirstProducerThread;  // 0..kProducerThreads-1
         const uint32_t my_r = pt >> 3, my_c = pt & 7u;  // this thread's row (plus kRowsPerPass i) and 16-element chunk
@@ -381,7 +458,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             // (the thread that copies token n's scales is kProducerThreads - 65 - n: see the copy below)
             m.scale_row = first + (kProducerThreads - 65u - pt);
         };
-        uint32_t it = 0u, slot = 0u, empty_parity = 1u;  // a fresh barrier passes a wait on parity 1
+        uint32_t slot = 0u, empty_parity = 1u;  // a fresh barrier passes a wait on parity 1
         long long trace_wait = 0;
         const long long trace_begin = TRACE ? clock64() : 0;
         const uint32_t my_dst = swizzle128_offset(my_r, my_c);
@@ -403,7 +480,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 wcol[mx] = cur.w[mx] + (size_t)(row0 + my_r) * form_row_bytes + my_c * (bytes_form ? 16u : 8u);
             }
             const size_t row_step = (size_t)kRowsPerPass * form_row_bytes;
-            for (uint32_t ks = 0; ks < k_stages; ks++, it++) {
+            for (uint32_t ks = 0; ks < k_stages; ks++) {
                 const long long w0 = TRACE ? clock64() : 0;
                 if (!mbar_wait_warp(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
                     alive = false;
@@ -412,15 +489,13 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 if (TRACE) trace_wait += clock64() - w0;
 #pragma unroll
                 for (uint32_t sub = 0; sub < C::kSub; sub++) {
-                const uint32_t kb = ks * C::kSub + sub;
-                if (kb >= k_blocks) break;  // the last stage of an odd count holds one block
-                const uint32_t block = slot * C::kSub + sub;  // index into the three shared-memory arrays
+                if (sub != 0u && ks >= doubles) break;  // the last stage of an odd count holds one block
+                const uint32_t kb = first_block(ks) + sub;
+                const uint32_t block = slot * C::kSub + sub;  // index into the shared-memory arrays
                 unsigned char* a_tiles = smem + block * C::kABytes;
                 const uint32_t k_left = k_dim - kb * kBlockK;  // elements of K from this block on
                 const bool chunk_ok = my_c * 16u < k_left;
                 // weights: 8-byte pieces of 16 codes into the low half of 16-byte slots
-                // (with TMA only the trailing partial K block comes this way)
-                if (!USE_TMA || k_left < kBlockK) {
 #pragma unroll
                 for (uint32_t mx = 0; mx < C::kMatrices; mx++) {
                     const uint32_t a_dst = smem_u32(a_tiles + mx * kATileBytes) + my_dst;
@@ -436,10 +511,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         }
                     }
                 }
-                }
-                // activations: 16-byte pieces of 16 E4M3 codes (with TMA the whole tile is one box)
+                // activations: 16-byte pieces of 16 E4M3 codes
                 const uint32_t b_dst = smem_u32(smem + C::kBRegion + block * C::kBTileBytes) + my_dst;
-                if (!USE_TMA) {
 #pragma unroll
                 for (uint32_t i = 0; i < kTokenPasses; i++) {
                     const uint32_t n = my_r + kRowsPerPass * i;
@@ -449,34 +522,25 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         cp_async_16(b_dst + i * (kRowsPerPass * 128u), src, ok ? 16u : 0u);
                     }
                 }
-                }
                 // scales: the derived copy already has the 32x16-byte layout tcgen05.cp reads, one 512-byte
                 // block per (row tile, K block); token scales are gathered four bytes (one K block) a row
-                unsigned char* sf = smem + C::kSfRegion + block * C::kSfBytes;
                 // (threads from the far end of the producer group, so that with few tokens a tile these are not
                 // the threads that carry the token rows)
                 const uint32_t st = kProducerThreads - 1u - pt;
-                if (!USE_TMA && st < 32u * C::kMatrices) {
+                if (st < 32u * C::kMatrices) {
                     const uint32_t mx = st >> 5, l = st & 31u;
                     const uint8_t* src = cur.ts[mx] + ((size_t)scale_tile(cur.m_tile, mx) * k_blocks + kb) * C::kScaleStride + l * 16u;
-                    cp_async_16(smem_u32(sf + mx * kScaleBlockBytes + l * 16u), src, 16u);
+                    cp_async_16(smem_u32(smem + C::kSfRegion + C::weight_scales(slot, sub, mx) + l * 16u), src, 16u);
                 }
-                if (USE_TMA) {
-                    for (uint32_t n = pt; n < N_TILE; n += kProducerThreads) {
-                        const bool ok = n < cur.valid;
-                        const uint32_t* src = ok ? p.act_e8m0.words + (size_t)(cur.first + n) * k_blocks + kb : p.act_e8m0.words;
-                        cp_async_4(smem_u32(sf + C::kMatrices * kScaleBlockBytes + (n & 31u) * 16u + (n >> 5) * 4u), src,
-                                   ok ? 4u : 0u);
-                    }
-                } else if (st >= 64u && st < 64u + N_TILE) {
+                if (st >= 64u && st < 64u + N_TILE) {
                     const uint32_t n = st - 64u;
                     const bool ok = n < cur.valid;
                     const uint32_t* src = ok ? p.act_e8m0.words + (size_t)cur.scale_row * k_blocks + kb : p.act_e8m0.words;
-                    cp_async_4(smem_u32(sf + C::kMatrices * kScaleBlockBytes + (n & 31u) * 16u + (n >> 5) * 4u), src,
+                    cp_async_4(smem_u32(smem + C::kSfRegion + C::token_scales(slot, sub) + (n & 31u) * 16u + (n >> 5) * 4u), src,
                                ok ? 4u : 0u);
                 }
                 }
-                if (!USE_TMA && pt == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->format[slot]) = cur.format;
+                if (pt == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->format[slot]) = cur.format;
                 // the arrival fires when this thread's copies have landed; the thread moves on at once
                 cp_async_arrive_noinc(&bars->full[slot]);
                 if (++slot == C::kStages) {
@@ -534,22 +598,23 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                                                                                                                  : kIdescBytes;
 #pragma unroll
                     for (uint32_t sub = 0; sub < C::kSub; sub++) {
-                    const uint32_t kb = ks * C::kSub + sub;
-                    if (kb >= k_blocks) break;
-                    const uint32_t block = slot * C::kSub + sub;  // index into the three shared-memory arrays
-                    const uint64_t a_desc = a_desc0 + (uint64_t)(block * (C::kABytes >> 4));
-                    const uint64_t b_desc = b_desc0 + (uint64_t)(block * (C::kBTileBytes >> 4));
-                    const uint64_t sf_desc = sf_desc0 + (uint64_t)(block * (C::kSfBytes >> 4));
-#pragma unroll
-                    for (uint32_t mx = 0; mx <= C::kMatrices; mx++)
-                        tc_copy_scales(tmem_scales + 4u * mx, sf_desc + mx * (kScaleBlockBytes >> 4));
+                    if (sub != 0u && ks >= doubles) break;
+                    const uint32_t kb = first_block(ks) + sub;
+                    const uint32_t block = slot * C::kSub + sub;  // index into the shared-memory arrays
                     const uint32_t groups = (kb + 1u == k_blocks && tail_groups != 0u) ? tail_groups : 4u;
+                    // (by TMA a trailing half block lies in the second half of its operand tiles; a K step of 32 elements is 32 bytes:
+                    // two 16-byte units of the start address)
+                    const uint32_t first = USE_TMA ? 2u * (4u - groups) : 0u;
+                    const uint64_t a_desc = a_desc0 + (uint64_t)(block * (C::kABytes >> 4) + first);
+                    const uint64_t b_desc = b_desc0 + (uint64_t)(block * (C::kBTileBytes >> 4) + first);
+#pragma unroll
+                    for (uint32_t mx = 0; mx < C::kMatrices; mx++) tc_copy_scales(tmem_scales + 4u * mx, sf_desc0 + (C::weight_scales(slot, sub, mx) >> 4));
+                    tc_copy_scales(sfb_tmem, sf_desc0 + (C::token_scales(slot, sub) >> 4));
 #pragma unroll
                     for (uint32_t j = 0; j < 4u; j++) {
                         if (j < groups) {
 #pragma unroll
                             for (uint32_t mx = 0; mx < C::kMatrices; mx++) {
-                                // a K step of 32 elements is 32 bytes: two 16-byte units of the start address
                                 tc_mma_block_scaled(d_tmem + mx * N_TILE, a_desc + (mx * (kATileBytes >> 4) + 2u * j),
                                                     b_desc + 2u * j, kIdesc | (j << 4) | (j << 29), tmem_scales + 4u * mx,
                                                     sfb_tmem, j == 0u ? (kb != 0u ? 1u : 0u) : 1u);
@@ -846,18 +911,18 @@ __device__ __forceinline__ void publish_map(uint8_t* map, const uint8_t* templ, 
     tensormap_publish(map, smem_map);
 }
 
-// One warp per (expert, matrix): the two template maps (a box of one K block, of two) with the expert's weight address
-// patched in; then one for the map of the set's derived scale copy.
+// One warp per (expert, matrix): the template maps (kWeightMaps) with the expert's weight address patched in; then one for the map of the set's derived scale copy.
 __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* experts, const uint8_t* templ, const uint8_t* derived,
                                                              uint8_t* maps, uint32_t matrices) {
-    __shared__ __align__(128) unsigned char sm[256];
+    __shared__ __align__(128) unsigned char sm[kWeightMaps * 128u];
     const uint32_t e = blockIdx.x / matrices, mx = blockIdx.x % matrices;
     const bool scales = blockIdx.x == gridDim.x - 1u;
     if (!scales && (experts[e].w[0] == nullptr || experts[e].w[mx] == nullptr)) return;
     const uint8_t* w = scales ? derived : experts[e].w[mx];
     // `templ` holds the maps of the compact form, those of the one-byte-per-element forms and that of the derived scales
-    const uint8_t* mine = templ + (scales ? 512u : experts[e].format == kFormatCompact ? 0u : 256u);
-    for (uint32_t i = 0; i < (scales ? 1u : 2u); i++) publish_map(maps + (size_t)blockIdx.x * 256u + i * 128u, mine + i * 128u, sm + i * 128u, w);
+    const uint8_t* mine = templ + (scales ? 2u : experts[e].format == kFormatCompact ? 0u : 1u) * kWeightMaps * 128u;
+    for (uint32_t i = 0; i < (scales ? 1u : kWeightMaps); i++)
+        publish_map(maps + ((size_t)blockIdx.x * kWeightMaps + i) * 128u, mine + i * 128u, sm + i * 128u, w);
 }
 
 // The same for the one matrix of a dense linear, whose addresses are the call's own: nothing about the matrix is kept
@@ -869,7 +934,7 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
-    __shared__ __align__(128) unsigned char sm[256];
+    __shared__ __align__(128) unsigned char sm[kWeightMaps * 128u];
     grid_dependency_sync();
     const uint32_t tile_total = p.tiles.list ? (p.tokens + p.tiles.n_tile - 1u) / p.tiles.n_tile : 0u;
     for (uint32_t i = blockIdx.x * kDenseThreads + threadIdx.x; i < p.tokens; i += gridDim.x * kDenseThreads) {
@@ -923,7 +988,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
         *p.ptrs = ExpertPtrs{{p.weights, nullptr}, {p.scales, nullptr}, {p.derived, nullptr}, {0u, 0u}, kFormatCompact, 0u};
     }
     if (p.map_template != nullptr && threadIdx.x < 32u) {
-        for (uint32_t i = 0; i < 2u; i++) publish_map(p.map + i * 128u, p.map_template + i * 128u, sm + i * 128u, p.weights);
+        for (uint32_t i = 0; i < kWeightMaps; i++) publish_map(p.map + i * 128u, p.map_template + i * 128u, sm + i * 128u, p.weights);
     }
 }
 
@@ -1120,7 +1185,7 @@ static EncodeFn tensor_map_encoder() {
     return encode;
 }
 
-bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols) {
+bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows) {
     // The packaged [rows][cols/2] bytes seen as a 3-D tensor of 4-bit elements {128 elements, blocks, rows} whose blocks of
     // 128 columns start every 64: a box {128, 1, 128} is one operand tile, at block 2 kb that of K block kb, at the last
     // block the 128 columns that end with the row. (The padded 4-bit type wants 32-byte strides, so cols % 64 == 0, and
@@ -1130,7 +1195,7 @@ bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows,
     if (!encode) return false;
     const cuuint64_t dims[3] = {kBlockK, cols / 64u - 1u, rows};
     const cuuint64_t strides[2] = {32u, cols / 2u};
-    const cuuint32_t box[3] = {kBlockK, 1u, kBlockM};
+    const cuuint32_t box[3] = {kBlockK, 1u, box_rows};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUtensorMap map;
     if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, any_device_address, dims, strides, box, estr,
@@ -1141,7 +1206,7 @@ bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows,
     return true;
 }
 
-bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols) {
+bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows) {
     // One E4M3 byte per element, seen like the compact form as {128 elements, blocks every 64 columns, rows}: the
     // same box coordinates fetch the same operand tile, now without padding.
     if (cols < kBlockK || cols % kBlockK != 0u) return false;
@@ -1149,7 +1214,7 @@ bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t
     if (!encode) return false;
     const cuuint64_t dims[3] = {kBlockK, cols / 64u - 1u, rows};
     const cuuint64_t strides[2] = {64u, cols};
-    const cuuint32_t box[3] = {kBlockK, 1u, kBlockM};
+    const cuuint32_t box[3] = {kBlockK, 1u, box_rows};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUtensorMap map;
     if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, any_device_address, dims, strides, box, estr,

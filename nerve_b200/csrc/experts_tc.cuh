@@ -12,15 +12,17 @@ bool tc_enabled_by_default();
 void tc_configure_kernels();
 // Encodes the template tensor map of a [rows][cols] weight matrix (any 32-byte aligned device address
 // will do: it is replaced per expert). False when the shape cannot use TMA.
-bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols);
+bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows);
 // The same for a matrix held as one E4M3 byte per element (pre-expanded or native FP8 resources).
-bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols);
+bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows);
+// Tensor maps of a weight matrix: boxes of 128 rows x one K block, 128 rows x two, 256 rows x one.
+constexpr uint32_t kWeightMaps = 3u;
 // Encodes the tensor map of an expert-grouped activation matrix [rows][cols] of E4M3 bytes with a box of
 // n_tile rows x 128 bytes (the operand tile of one K block). False when tensor maps are unavailable.
 bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t n_tile);
-// The tensor maps of the CTA pair kernel, whose boxes bring two K blocks at a time: a weight matrix in the compact or a
-// one-byte form (128 rows), expert-grouped token rows, the derived scales of a set (blocks of 512 bytes, `sources` to a
-// (row tile, K block)), and the token scales [rows = K blocks][words].
+// The tensor maps whose boxes bring two K blocks at a time: a weight matrix in the compact or a one-byte form (128 rows),
+// expert-grouped token rows, and for CTA pairs the derived scales of a set (blocks of 512 bytes, `sources` to a (row tile,
+// K block)) and the token scales [rows = K blocks][words].
 bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, bool bytes);
 bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows);
 bool tc_encode_pair_scale_map(void* map128, void* any_device_address, uint32_t sources, uint32_t blocks);
@@ -62,8 +64,8 @@ constexpr uint32_t kPairTokens = 240u;  // the most tokens of a pair's tile
 void pair_configure_kernels();
 void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream);
 // Tensor maps of a stage's operands: token rows in boxes of one K block, for one CTA's token tiles and, from the second on,
-// for four of a pair's (half a tile); the same four in boxes of two; the token scales.
-constexpr uint32_t kTokenMaps = 6u, kPairTokenMap = kTokenMaps, kTokenScaleMap = kPairTokenMap + 4u, kActMaps = kTokenScaleMap + 1u;
+// for four of a pair's (half a tile); the same in boxes of two K blocks, kTokenMaps further on; the token scales.
+constexpr uint32_t kTokenMaps = 6u, kTokenScaleMap = 2u * kTokenMaps, kActMaps = kTokenScaleMap + 1u;
 constexpr uint32_t kTokenMapRows[kTokenMaps] = {16u, 32u, 64u, 96u, kPairTokens / 2u, 128u};
 inline uint32_t tc_token_map_for(const TokenTile& t) {
     uint32_t i = 0u;

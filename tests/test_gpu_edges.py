@@ -347,6 +347,38 @@ def test_narrow_row_pairs_match_the_checker(device, name, shape, tokens, native)
     bank.destroy()
 
 
+# one CTA's tiles with tensor maps, by width (16, 32, 64, 96 tokens): K of whole pairs of blocks, of a lone block after them, of
+# a trailing half block after either, of a single block; rows that end inside a tile; a native FP8 resource; and 16- and
+# 32-token tiles in row pairs (tall boxes) with a last pair that is a lone half
+@pytest.mark.parametrize("name,shape,tokens,native", [
+    ("gpt-oss-20b", (576, 320, 16), 9, 0), ("gpt-oss-20b", (704, 448, 16), 60, 0), ("gpt-oss-20b", (384, 128, 16), 150, 0),
+    ("gpt-oss-20b", (128, 192, 16), 340, 0), ("gpt-oss-20b", (448, 576, 16), 48, 0), ("deepseek-v3", (512, 384, 16), 5, 0),
+    ("deepseek-v3", (384, 640, 16), 33, 1), ("deepseek-v3", (640, 256, 16), 150, 1), ("gpt-oss-20b", (1920, 448, 128), 250, 0),
+    ("deepseek-v3", (1920, 384, 128), 300, 1)])
+def test_tiles_by_tensor_map_match_the_checker(device, name, shape, tokens, native):
+    cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], *shape), native_fp8_resources=native)
+    assert tokens * cfg.total_k <= 96 * cfg.total_experts
+    case = synthetic.make_case(cfg, tokens, seed=19)
+    tensors = [list(t) for t in (case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)]
+    for e in range(cfg.total_experts - native, cfg.total_experts):
+        for i, t in enumerate(synthetic.native_fp8_tensors(cfg, 19, e)):
+            tensors[i][e] = t
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(2)
+    bank = ExpertBank.upload(device, *tensors)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, device.resident_buffer_from(case.hidden), out, router_weights=device.resident_buffer_from(case.router_w),
+               router_bias=device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+               bias=device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None)
+    logits = mo.linear_bf16(case.hidden, case.router_w, case.router_bias)
+    sample = sampled.sample_tokens(tokens, 64, seed=tokens)
+    want = sampled.layer_on_sample(cfg, case.hidden, logits, case.select_bias, sample, lambda e: [t[e] for t in tensors])
+    assert_close(out.read(np.uint16).reshape(tokens, cfg.hidden)[sample], want["output"], f"{name} {shape} one CTA T{tokens}")
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+
+
 # the input quantised beside the matrix (scale blocks of 32 and 128, a ragged last 512 columns) and in a launch of its own
 # (blocks of 64, rows off the 16-byte grid); several row tiles with a ragged last one, a row beyond one token tile
 @pytest.mark.parametrize("block,shift,rows,cols,tokens", [(32, 0, 288, 544, 5), (32, 0, 160, 1056, 131), (128, 0, 384, 640, 33),
