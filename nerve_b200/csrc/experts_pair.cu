@@ -41,7 +41,10 @@ constexpr uint32_t kPairScaleWarp = kPairInfoWarp + 1u;
 constexpr uint32_t kPairThreads = 32u * (kPairScaleWarp + 1u);
 constexpr uint32_t kPairWatchWarp = 2u;                                 // polls for a finished accumulator (shares no scheduler with MMA and TMA)
 constexpr uint32_t kPairColumns = kPairTokens;
-constexpr uint32_t kPairStages = 3u;
+// Slots of the ring: three of 240 columns; four of 128 where nothing is exchanged, for calls whose list has no wider tiles (a
+// slot is held for about two microseconds, most of it latency, so that the narrower stages wait for the ring: dense block of
+// 777 rows of 7168 x 2048 98.7 us with three, 94.7 with four, of 100 rows 68.8 / 63.4; 2000 rows, wider tiles, 155.9 / 156.4).
+constexpr uint32_t kPairStages = 3u, kPairNarrowStages = 4u, kPairNarrowTokens = 128u;
 constexpr uint32_t kPairBlocks = 2u;                                     // K blocks a stage
 constexpr uint32_t kPairTokenBytes = kPairColumns / 2u * 128u;          // token rows of one K block in one CTA
 // a stage's weight scales, then its token scales: as they come, 244 words a K block, then as two blocks of 512 bytes each
@@ -53,9 +56,9 @@ constexpr uint32_t kPairTmemColumns = 512u;
 static_assert(kPairScaleColumn + 2u * kPairScaleColumns <= kPairTmemColumns, "tensor memory");
 
 struct PairBarriers {
-    uint64_t full[kPairStages];    // CTA 0's count
-    uint64_t empty[kPairStages];
-    uint64_t staged[kPairStages];  // the token scales of a slot are there, as they lie in memory
+    uint64_t full[kPairNarrowStages];    // CTA 0's count
+    uint64_t empty[kPairNarrowStages];
+    uint64_t staged[kPairNarrowStages];  // the token scales of a slot are there, as they lie in memory
     uint64_t acc_full[2];
     uint64_t acc_empty[2];         // CTA 0's
     uint64_t info_full[2];         // what the epilogue has to know of a tile is there
@@ -65,7 +68,7 @@ struct PairBarriers {
     uint64_t taken[kPairEpilogueWarps];   // ... has read the chunk this warp sent
     uint32_t tmem_base;
     uint32_t abort;
-    uint32_t stage_info[kPairStages];     // of the tile whose operands a slot holds: format << 16 | first row % 4 << 12 | columns
+    uint32_t stage_info[kPairNarrowStages];     // of the tile whose operands a slot holds: format << 16 | first row % 4 << 12 | columns
     uint32_t acc_ready[2];
     // per tile, alternating: its tokens, its row tile, and per column the route (0xffffffff: no token) with its down row
     // (gate/up) or its weight (down)
@@ -75,12 +78,11 @@ struct PairBarriers {
     uint32_t maxima[kPairEpilogueGroups][2][4][8];  // [group][chunk, alternating][lane quadrant][tokens in pairs], bf16
 };
 constexpr uint32_t kPairExchangeBytes = kPairEpilogueWarps * 1024u;     // 16 columns x 32 rows of bf16 a warp
-constexpr uint32_t kPairTokenRegion = kPairStages * kPairBlocks * kATileBytes;
-constexpr uint32_t kPairScaleRegion = kPairTokenRegion + kPairStages * kPairBlocks * kPairTokenBytes;
-constexpr uint32_t kPairExchangeRegion = kPairScaleRegion + kPairStages * kPairScaleBytes;
+constexpr uint32_t kPairExchangeRegion = kPairStages * (kPairBlocks * (kATileBytes + kPairTokenBytes) + kPairScaleBytes);
 constexpr uint32_t kPairBarrierRegion = kPairExchangeRegion + kPairExchangeBytes;
 constexpr uint32_t kPairSmemBytes = kPairBarrierRegion + sizeof(PairBarriers) + 1024u;  // (the round-up to a 1024-byte boundary)
 static_assert(kPairSmemBytes <= 227u * 1024u && kPairBarrierRegion % 128u == 0u, "shared memory");
+static_assert(kPairNarrowStages * (kPairBlocks * (kATileBytes + kPairNarrowTokens / 2u * 128u) + kPairScaleBytes) <= kPairBarrierRegion, "narrow slots");
 
 __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -118,9 +120,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     const uint32_t m_tiles = GATE_UP ? row_tiles : (row_tiles + 1u) / 2u;
     constexpr uint32_t kSources = GATE_UP ? 2u : 1u;
 
+    // the ring: weight tiles, token tiles, scales, each an array over (slot, K block)
+    const bool narrow = !GATE_UP && p.token_rows <= kPairNarrowTokens;
+    const uint32_t slots = narrow ? kPairNarrowStages : kPairStages;
+    const uint32_t token_bytes = narrow ? kPairNarrowTokens / 2u * 128u : kPairTokenBytes;
+    const uint32_t token_region = slots * kPairBlocks * kATileBytes, scale_region = token_region + slots * kPairBlocks * token_bytes;
+
     // ---- one-time setup ---------------------------------------------------------------------
     if (threadIdx.x == 0u) {
-        for (uint32_t s = 0; s < kPairStages; s++) {
+        for (uint32_t s = 0; s < slots; s++) {
             mbar_init(&bars->full[s], 3u);  // the announcement of the copies, the scale warps of both CTAs
             mbar_init(&bars->empty[s], 1u);
             mbar_init(&bars->staged[s], 1u);
@@ -213,8 +221,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]) = info;
                     if (!withhold) {
                         const uint32_t a = smem_base + slot * kPairBlocks * kATileBytes;
-                        const uint32_t b = smem_base + kPairTokenRegion + slot * kPairBlocks * kPairTokenBytes;
-                        const uint32_t sf = smem_base + kPairScaleRegion + slot * kPairScaleBytes;
+                        const uint32_t b = smem_base + token_region + slot * kPairBlocks * token_bytes;
+                        const uint32_t sf = smem_base + scale_region + slot * kPairScaleBytes;
                         // the token scales first, which have the longest way to go (of one block, too, the scales of two are
                         // fetched: zeros, or the next row tile's, that nothing uses)
                         mbar_arrive_expect_tx(&bars->staged[slot], kPairBlocks * kPairScaleWords * 4u);
@@ -233,7 +241,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     }
                     withhold = false;
                     stage_it++;
-                    if (++slot == kPairStages) {
+                    if (++slot == slots) {
                         slot = 0u;
                         empty_parity ^= 1u;
                     }
@@ -253,10 +261,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             if (!alive) {
                 // copies may still be on their way into either CTA's shared memory: wait, bounded, on the barriers of the last
                 // round (CTA 1 sees its scales land there, not its other copies, and waits out the time for those)
-                const uint32_t rounds = stage_it < kPairStages ? stage_it : kPairStages;
+                const uint32_t rounds = stage_it < slots ? stage_it : slots;
                 for (uint32_t back = 1u; back <= rounds; back++) {
                     const uint32_t nth = stage_it - back;
-                    mbar_wait_winddown(&bars->full[nth % kPairStages], rank == 0u ? (nth / kPairStages) & 1u : 0u, kWinddownCycles / kPairStages);
+                    mbar_wait_winddown(&bars->full[nth % slots], rank == 0u ? (nth / slots) & 1u : 0u, kWinddownCycles / slots);
                 }
             }
         }
@@ -268,8 +276,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             constexpr uint32_t kIdescBytes = idesc_mxf8f6f4(kFmtE4M3, kFmtE4M3, 2u * kBlockM, 0u);
             const uint32_t base = smem_u32(smem);
             const uint64_t a_desc0 = desc_k_major_sw128(base);
-            const uint64_t b_desc0 = desc_k_major_sw128(base + kPairTokenRegion);
-            const uint64_t sf_desc0 = desc_scale_block(base + kPairScaleRegion);
+            const uint64_t b_desc0 = desc_k_major_sw128(base + token_region);
+            const uint64_t sf_desc0 = desc_scale_block(base + scale_region);
             const uint32_t tail_groups = (k_dim % kBlockK) / 32u;  // K steps of a trailing partial block, 0 = none
             uint32_t acc_it = 0u, slot = 0u, full_parity = 0u;
             bool alive = true;
@@ -299,7 +307,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                         tc_copy_scales_pair(sfb, sfb_desc);
                         if (columns > 128u) tc_copy_scales_pair(sfb + 4u, sfb_desc + (kScaleBlockBytes >> 4));
                         const uint64_t a_desc = a_desc0 + (uint64_t)((slot * kPairBlocks + sub) * (kATileBytes >> 4) + first);
-                        const uint64_t b_desc = b_desc0 + (uint64_t)(slot * kPairBlocks * (kPairTokenBytes >> 4) + sub * (columns << 2) + first);
+                        const uint64_t b_desc = b_desc0 + (uint64_t)(slot * kPairBlocks * (token_bytes >> 4) + sub * (columns << 2) + first);
 #pragma unroll
                         for (uint32_t j = 0; j < 4u; j++) {
                             if (j < groups)
@@ -308,7 +316,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                         }
                     }
                     tc_commit_pair_both(&bars->empty[slot]);
-                    if (++slot == kPairStages) {
+                    if (++slot == slots) {
                         slot = 0u;
                         full_parity ^= 1u;
                     }
@@ -331,7 +339,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     alive = false;
                     break;
                 }
-                uint32_t* words = reinterpret_cast<uint32_t*>(smem + kPairScaleRegion + slot * kPairScaleBytes + kPairBlocks * kScaleBlockBytes);
+                uint32_t* words = reinterpret_cast<uint32_t*>(smem + scale_region + slot * kPairScaleBytes + kPairBlocks * kScaleBlockBytes);
                 const uint32_t info = *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]);
                 const volatile uint32_t* mine = words + ((info >> 12) & 3u) + lane;
                 uint32_t w[kPairBlocks][8];
@@ -349,7 +357,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0u) mbar_arrive_cluster(full0 + slot * 8u);
-                if (++slot == kPairStages) {
+                if (++slot == slots) {
                     slot = 0u;
                     parity ^= 1u;
                 }
