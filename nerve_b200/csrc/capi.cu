@@ -900,6 +900,7 @@ struct ExpertCall {
     ExpertSet* prepared = nullptr;
     bool scheduled = false;         // grouping (and tile list) already built for this call
     bool fuse_quantise = false;     // gate/up on the tensor path: the epilogue also writes the down stage's operands
+    bool fresh_maps = false;        // the last launch before this one writes the tensor maps
 };
 
 // shared tail of the two gate/up entry points and of down
@@ -936,6 +937,8 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     el.tmaps = tensor && p->tma[set] ? es->tmaps.as<uint8_t>() : nullptr;
     el.tile_count = p->tile_list.as<uint32_t>() + set * tile_region_words(p);  // first word of the stage's region
     el.tile_list = el.tile_count + 64;
+    el.tile_capacity = (uint32_t)(tile_region_words(p) - 64u);
+    el.fresh_maps = c.fresh_maps;
     el.tokens = T;
     el.g = g;
     el.wait_cycles = p->wait_cycles;
@@ -1319,6 +1322,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     call.routes = dl->unit_routes.as<uint32_t>();
     call.outputs = (uint16_t*)output->ptr;
     call.prepared = &dl->set;
+    call.fresh_maps = true;
     call.scheduled = true;
     NVMOE_TRY(run_experts(sub, call));
     p->launches += sub->launches;

@@ -254,6 +254,8 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     uint64_t* cta_trace;         // tensor path diagnostics: [2][grid][4] words per CTA, or null
     uint64_t* scale_stamps;      // tensor path: {scale pointer, generation} the derived tiles were built from
     uint32_t* tile_list;         // tensor path scratch: routes / 16 + experts + 1 words
+    uint32_t tile_capacity;      // ... of which so many may be read
+    bool fresh_maps;             // tensor path: the launch right before this one wrote the tensor maps
     uint32_t* tile_count;        // tensor path scratch: one word
     uint32_t tokens;             // upper bound (max over what control may hold)
     long long wait_cycles;       // tensor path: clock cycles after which a bounded in-kernel wait gives up

@@ -158,13 +158,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
     const uint32_t tmem_scales = tmem_base + kPairScaleColumn;
+    auto acquire_maps = [&] {  // (a tensor map written by an earlier kernel is acquired once per block before the TMA unit gets it)
+        for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources + 1u; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * kWeightMaps * 128u);
+        for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources; m += blockDim.x) tensormap_acquire(p.tmaps + ((size_t)m * kWeightMaps + 1u) * 128u);
+        if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
+        __syncthreads();
+    };
+    if (!p.fresh_maps) acquire_maps();  // as in experts_tc.cu: while the kernel ahead still runs
     grid_dependency_sync();
+    const uint32_t first_entry = warp == kPairTmaWarp ? __ldg(list.tiles + min(pair_id / m_tiles, p.tile_capacity - 1u)) : 0u;
     const uint32_t tile_count = *list.count * m_tiles;
-    // (a tensor map written by an earlier kernel is acquired once per block before the TMA unit gets it)
-    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources + 1u; m += blockDim.x) tensormap_acquire(p.tmaps + (size_t)m * kWeightMaps * 128u);
-    for (uint32_t m = threadIdx.x; m < p.work.num_experts * kSources; m += blockDim.x) tensormap_acquire(p.tmaps + ((size_t)m * kWeightMaps + 1u) * 128u);
-    if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
-    __syncthreads();
+    if (p.fresh_maps) acquire_maps();
 
     // first row of a tile in the operand matrix, and how many rows it has
     auto first_row_of = [&](uint32_t n_tile, uint32_t e_begin) { return e_begin + n_tile * p.token_rows; };
@@ -192,8 +196,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             uint32_t slot = 0u, empty_parity = 1u, stage_it = 0u;
             bool alive = true, withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
             Meta cur{}, nxt{};
+            if (pair_id < tile_count) meta_of(pair_id, first_entry, cur);
             uint32_t pair_nxt = entry_of(pair_id + pairs);
-            if (pair_id < tile_count) meta_of(pair_id, entry_of(pair_id), cur);
             for (uint32_t tile = pair_id; tile < tile_count && alive; tile += pairs) {
                 const uint32_t pair_nxt2 = entry_of(tile + 2u * pairs);
                 if (tile + pairs < tile_count) meta_of(tile + pairs, pair_nxt, nxt);

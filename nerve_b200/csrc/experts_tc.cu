@@ -228,12 +228,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
     const uint32_t tmem_scales = tmem_base + C::kScaleColumn0;
-    // everything above touched only this CTA's shared and tensor memory; what follows reads what the
-    // kernels before this one wrote
-    grid_dependency_sync();
-    const uint32_t pair_count = *list.count;
-    const uint32_t tile_count = pair_count * m_tiles;
-    if (USE_TMA) {
+    auto acquire_maps = [&] {
         // The per-expert tensor maps were written to global memory by an earlier kernel. A thread block must
         // acquire such a map once before any of its threads hands it to the TMA unit; further uses by the
         // block need no fence. All threads share the maps out, so that the block pays one fence latency here
@@ -245,7 +240,18 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         }
         if (threadIdx.x < C::kSub) tensormap_acquire(p.act_tmap + threadIdx.x * kTokenMaps * 128u);
         __syncthreads();
-    }
+    };
+    // Maps of earlier calls, or of this one with a launch between (which has completed by the time this kernel may start), are
+    // acquired while the kernel ahead still runs.
+    if (USE_TMA && !p.fresh_maps) acquire_maps();
+    // everything above touched only this CTA's shared and tensor memory and maps that stand; what follows reads what the
+    // kernels before this one wrote
+    grid_dependency_sync();
+    // (the first list entry is fetched with the count it may turn out to lie beyond, not after it)
+    const uint32_t first_entry = USE_TMA && warp == 5u ? __ldg(list.tiles + min(blockIdx.x / m_tiles, p.tile_capacity - 1u)) : 0u;
+    const uint32_t pair_count = *list.count;
+    const uint32_t tile_count = pair_count * m_tiles;
+    if (USE_TMA && p.fresh_maps) acquire_maps();
 
     if (warp == 5u) {
         // ===== TMA issue (one lane): whole 128 x 128 boxes of weight codes, padded and swizzled by the unit =====
@@ -277,8 +283,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 for (uint32_t src = 0; src < C::kSources; src++) m.ts[src] = p.work.experts[expert].ts[src];
             };
             Meta cur{}, nxt{};
+            if (blockIdx.x < tile_count) meta_of(blockIdx.x, first_entry, cur);
             uint32_t pair_nxt = entry_of(blockIdx.x + gridDim.x);
-            if (blockIdx.x < tile_count) meta_of(blockIdx.x, entry_of(blockIdx.x), cur);
             // (debug) leave out the very first arrival of CTA 0: its consumer's bounded wait must then give up
             bool withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
             uint32_t stage_it = 0u;  // stages this lane has gone through (stage n used slot n % kStages, phase n / kStages)
