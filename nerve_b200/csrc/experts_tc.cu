@@ -248,7 +248,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
     // kernels before this one wrote
     grid_dependency_sync();
     // (the first list entry is fetched with the count it may turn out to lie beyond, not after it)
-    const uint32_t first_entry = USE_TMA && warp == 5u ? __ldg(list.tiles + min(blockIdx.x / m_tiles, p.tile_capacity - 1u)) : 0u;
+    const uint32_t first_entry = USE_TMA && (warp == 5u || warp == 6u) ? __ldg(list.tiles + min(blockIdx.x / m_tiles, p.tile_capacity - 1u)) : 0u;
     const uint32_t pair_count = *list.count;
     const uint32_t tile_count = pair_count * m_tiles;
     if (USE_TMA && p.fresh_maps) acquire_maps();
@@ -374,15 +374,15 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             struct Meta {
                 uint32_t first, valid;
             };
-            auto load_meta = [&](uint32_t tile, Meta& m) {
-                const uint32_t pair = __ldg(list.tiles + tile / m_tiles), expert = pair >> 16;
+            auto load_meta = [&](uint32_t pair, Meta& m) {
+                const uint32_t expert = pair >> 16;
                 m.first = __ldg(p.work.expert_offsets + expert) + (pair & 0xffffu) * N_TILE;
                 m.valid = min(N_TILE, __ldg(p.work.expert_offsets + expert + 1u) - m.first);
             };
             uint32_t slot = 0u, empty_parity = 1u;
             bool alive = true;
             Meta cur{}, nxt{};
-            if (blockIdx.x < tile_count) load_meta(blockIdx.x, cur);
+            if (blockIdx.x < tile_count) load_meta(first_entry, cur);
             for (uint32_t tile = blockIdx.x; tile < tile_count && alive; tile += gridDim.x) {
                 const uint32_t* row = p.act_e8m0.words + (size_t)(cur.first + lane) * k_blocks;
                 const uint32_t valid = cur.valid;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 };
 #pragma unroll
                 for (uint32_t u = 0; u < kAhead; u++) fetch(u, w[u]);
-                if (tile + gridDim.x < tile_count) load_meta(tile + gridDim.x, nxt);
+                if (tile + gridDim.x < tile_count) load_meta(__ldg(list.tiles + (tile + gridDim.x) / m_tiles), nxt);
                 for (uint32_t ks0 = 0; ks0 < k_stages && alive; ks0 += kAhead) {
 #pragma unroll
                     for (uint32_t u = 0; u < kAhead; u++) {
