@@ -172,6 +172,9 @@ size_t tile_region_words(const nvmoe_plan* p) {
 // Rows that the scale arrays of the expert-grouped operands hold per K block: whole 16-byte pieces.
 uint32_t scale_rows(const nvmoe_plan* p) { return (p->g.max_tokens * p->K + 3u) & ~3u; }
 
+// Tokens per expert in the largest call, as the choice of a token tile counts them.
+size_t most_tokens_per_expert(const nvmoe_plan* p) { return ((size_t)p->g.max_tokens * p->K + p->experts - 1u) / p->experts; }
+
 // Token tile of a stage for T tokens.
 TokenTile token_tile(const nvmoe_plan* p, bool gate_up, uint32_t T) {
     return tc_token_tile_for(T, p->K, p->experts, gate_up ? p->g.intermediate_size : p->g.hidden_size, gate_up, p->tma[gate_up ? 0 : 1]);
@@ -510,18 +513,21 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         want(p->grouped_e8m0[0], sizeof(uint32_t) * scale_rows(p) * ((H + 127u) / 128u));
         want(p->grouped_e8m0[1], sizeof(uint32_t) * scale_rows(p) * ((I + 127u) / 128u));
         want(p->act_maps, 2u * kActMaps * 128u);
+        const size_t most = most_tokens_per_expert(p);
+        const bool with_pairs = most > kPairsFrom;
         if (err == cudaSuccess) {
-            unsigned char maps[2u * kActMaps * 128u] = {0};
+            unsigned char maps[2u * kActMaps * 128u] = {0};  // (maps of tiles that no call of the plan uses stay zero)
             bool ok = true;
             for (uint32_t set = 0; set < 2u && ok; set++) {
                 const uint32_t cols = (uint32_t)(set == 0u ? H : I);
                 unsigned char* mine = maps + set * kActMaps * 128u;
-                for (uint32_t i = 0; i < kTokenMaps && ok; i++)
-                    ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
                 if (cols % 64u != 0u || cols < 128u) continue;  // (no map for its weights either)
-                for (uint32_t i = 0; i < kTokenMaps && ok; i++)
-                    ok = tc_encode_pair_token_map(mine + (kTokenMaps + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
-                ok = ok && tc_encode_token_scale_map(mine + kTokenScaleMap * 128u, p->grouped_e8m0[set].ptr, scale_rows(p), (cols + 127u) / 128u);
+                for (uint32_t i = 0; i < kTokenMaps && ok; i++) {
+                    if (most <= kTokenMapFrom[i]) continue;
+                    ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]) &&
+                         tc_encode_pair_token_map(mine + (kTokenMaps + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
+                }
+                if (with_pairs) ok = ok && tc_encode_token_scale_map(mine + kTokenScaleMap * 128u, p->grouped_e8m0[set].ptr, scale_rows(p), (cols + 127u) / 128u);
             }
             if (ok) {
                 err = cudaMemcpyAsync(p->act_maps.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
@@ -541,8 +547,9 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
                 const uint64_t blocks = tc_derived_scale_bytes(rows, cols) / 512u * p->experts;
                 p->tma[set] = p->act_maps.ptr && tc_encode_weight_map(mine, p->tmap_templates.ptr, rows, cols, 128u) &&
                               tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false) &&
-                              tc_encode_weight_map(mine + 256, p->tmap_templates.ptr, rows, cols, 256u) && blocks <= 0x7fffffffull &&
-                              tc_encode_pair_scale_map(mine + 768, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks);
+                              tc_encode_weight_map(mine + 256, p->tmap_templates.ptr, rows, cols, 256u) &&
+                              (!with_pairs || (blocks <= 0x7fffffffull &&
+                                               tc_encode_pair_scale_map(mine + 768, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks)));
                 tc_encode_weight_map_bytes(mine + 384, p->tmap_templates.ptr, rows, cols, 128u);
                 tc_encode_pair_weight_map(mine + 512, p->tmap_templates.ptr, rows, cols, true);
                 tc_encode_weight_map_bytes(mine + 640, p->tmap_templates.ptr, rows, cols, 256u);
@@ -822,7 +829,7 @@ static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* a
         el.work = GroupedWork{nullptr, nullptr, es->ptrs.as<ExpertPtrs>(), p->experts};
         el.scale_stamps = es->stamps.as<uint64_t>();
         el.tmaps = p->tma[set] ? es->tmaps.as<uint8_t>() : nullptr;
-        el.scale_base = es->derived.as<uint8_t>();
+        el.scale_base = most_tokens_per_expert(p) > kPairsFrom ? es->derived.as<uint8_t>() : nullptr;
         el.g = g;
         launch_derive_scales_tc(el, gate_up, st);
         p->launches += 2;
@@ -1263,7 +1270,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
                 rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the unit routes");
             // the map of the derived scales stays (the matrix's own maps, before it, are made by every call)
             unsigned char map[128];
-            if (fresh.plan->tma[1]) {
+            if (fresh.plan->tma[1] && most_tokens_per_expert(fresh.plan) > kPairsFrom) {
                 if (!tc_encode_pair_scale_map(map, fresh.set.derived.ptr, 1u, (uint32_t)(tc_derived_scale_bytes(rows, cols) / 512u)))
                     fresh.plan->tma[1] = false;
                 else if (cudaMemcpy(fresh.set.tmaps.as<uint8_t>() + kWeightMaps * 128u, map, 128, cudaMemcpyHostToDevice) != cudaSuccess)

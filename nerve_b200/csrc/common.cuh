@@ -250,7 +250,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     ScaleWords q_e8m0;
     uint32_t token_rows;         // tensor path: rows of the operand matrix per token tile of the list
     bool pairs;                  // tensor path: by CTA pairs
-    uint8_t* scale_base;         // tensor path: the derived scale copy of the whole expert set
+    uint8_t* scale_base;         // tensor path: the derived scale copy of the whole expert set (null: no map of it is needed)
     uint64_t* cta_trace;         // tensor path diagnostics: [2][grid][4] words per CTA, or null
     uint64_t* scale_stamps;      // tensor path: {scale pointer, generation} the derived tiles were built from
     uint32_t* tile_list;         // tensor path scratch: routes / 16 + experts + 1 words

@@ -922,7 +922,7 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
                                                              uint8_t* maps, uint32_t matrices) {
     __shared__ __align__(128) unsigned char sm[kWeightMaps * 128u];
     const uint32_t e = blockIdx.x / matrices, mx = blockIdx.x % matrices;
-    const bool scales = blockIdx.x == gridDim.x - 1u;
+    const bool scales = derived != nullptr && blockIdx.x == gridDim.x - 1u;
     if (!scales && (experts[e].w[0] == nullptr || experts[e].w[mx] == nullptr)) return;
     const uint8_t* w = scales ? derived : experts[e].w[mx];
     // `templ` holds the maps of the compact form, those of the one-byte-per-element forms and that of the derived scales
@@ -1105,10 +1105,10 @@ TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t
     const uint32_t routes = tokens * routes_per_token;
     const uint32_t per_expert = (routes + num_experts - 1u) / num_experts;
     // the narrowest tile that holds an expert's tokens (with some room for skew: a second tile reads the weights again)
-    if (per_expert <= 12u) return {16u, false};
-    if (per_expert <= 24u) return {32u, false};
-    if (per_expert <= 48u) return {64u, false};
-    if (per_expert <= 96u) return {96u, false};
+    if (per_expert <= kTokenMapFrom[1]) return {16u, false};
+    if (per_expert <= kTokenMapFrom[2]) return {32u, false};
+    if (per_expert <= kTokenMapFrom[3]) return {64u, false};
+    if (per_expert <= kPairsFrom) return {96u, false};
     const uint32_t row_tiles = gate_up ? (out_rows + kBlockM - 1u) / kBlockM : (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM);
     const uint64_t sms = (uint64_t)sm_count();
     // Beyond that CTA pairs (one CTA of 128 columns / pairs: 4096 tokens of 32 experts of 2880 x 2880 672 / 589 us a layer,
@@ -1297,7 +1297,7 @@ bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t 
 
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream) {
     const uint32_t matrices = gate_up ? 2u : 1u;
-    build_tensormaps_kernel<<<p.work.num_experts * matrices + 1u, 32, 0, stream>>>(p.work.experts, templ, p.scale_base,
+    build_tensormaps_kernel<<<p.work.num_experts * matrices + (p.scale_base ? 1u : 0u), 32, 0, stream>>>(p.work.experts, templ, p.scale_base,
                                                                                    const_cast<uint8_t*>(p.tmaps), matrices);
 }
 

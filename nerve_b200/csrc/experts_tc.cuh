@@ -65,8 +65,10 @@ void pair_configure_kernels();
 void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream);
 // Tensor maps of a stage's operands: token rows in boxes of one K block, for one CTA's token tiles and, from the second on,
 // for four of a pair's (half a tile); the same in boxes of two K blocks, kTokenMaps further on; the token scales.
-constexpr uint32_t kTokenMaps = 6u, kTokenScaleMap = 2u * kTokenMaps, kActMaps = kTokenScaleMap + 1u;
-constexpr uint32_t kTokenMapRows[kTokenMaps] = {16u, 32u, 64u, 96u, kPairTokens / 2u, 128u};
+constexpr uint32_t kTokenMaps = 5u, kTokenScaleMap = 2u * kTokenMaps, kActMaps = kTokenScaleMap + 1u;
+constexpr uint32_t kTokenMapRows[kTokenMaps] = {16u, 32u, 64u, 96u, kPairTokens / 2u};
+// tokens per expert above which a tile of those rows, or half a pair's tile, may be used (pairs above the last)
+constexpr uint32_t kTokenMapFrom[kTokenMaps] = {0u, 12u, 24u, 48u, 96u}, kPairsFrom = kTokenMapFrom[kTokenMaps - 1u];
 inline uint32_t tc_token_map_for(const TokenTile& t) {
     uint32_t i = 0u;
     while (i + 1u < kTokenMaps && kTokenMapRows[i] != t.rows) i++;
