@@ -56,9 +56,9 @@ def measured_peaks() -> tuple[dict, str]:
 
 
 def kernel_source_hash() -> str:
-    """Identifies the expert kernels a DRAM-traffic capture was taken on."""
+    """Identifies the tensor-path expert kernels (of one CTA and of CTA pairs) a DRAM-traffic capture was taken on."""
     h = hashlib.sha256()
-    for name in ("experts_tc.cu", "tcgen05.cuh"):
+    for name in ("experts_device.cuh", "experts_pair.cu", "experts_tc.cu", "experts_tc.cuh", "tcgen05.cuh"):
         h.update((ROOT / "nerve_b200" / "csrc" / name).read_bytes())
     return h.hexdigest()[:12]
 

@@ -89,3 +89,22 @@ def test_public_headers_compile_as_plain_c(tmp_path):
                     str(source), "-o", str(binary), "-lm"], check=True)
     subprocess.run([str(binary)], check=True)
 
+
+
+def test_traffic_captures_are_keyed_by_every_tensor_path_source(tmp_path, monkeypatch):
+    """A capture counts for the benchmark only while the kernels it was taken on stand, those of CTA pairs among them."""
+    import bench
+
+    csrc = tmp_path / "nerve_b200" / "csrc"
+    csrc.mkdir(parents=True)
+    for source in (ROOT / "nerve_b200" / "csrc").glob("*.cu*"):
+        (csrc / source.name).write_bytes(source.read_bytes())
+    monkeypatch.setattr(bench, "ROOT", tmp_path)
+    keys = {bench.kernel_source_hash()}
+    names = [n.name for n in csrc.iterdir() if n.name == "tcgen05.cuh" or (n.name.startswith("experts_") and "simt" not in n.name)]
+    assert {"experts_tc.cu", "experts_pair.cu", "experts_device.cuh"} <= set(names)
+    for name in names:
+        with open(csrc / name, "ab") as f:
+            f.write(b"\n")
+        keys.add(bench.kernel_source_hash())
+    assert len(keys) == 1 + len(names)
