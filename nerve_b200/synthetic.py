@@ -71,20 +71,20 @@ class MoeConfig:
 
 
 CONFIGS = {
-    # BASELINE.json configs[0]
+    # the smallest layer: softmax over all scores
     "tiny": MoeConfig("tiny", 256, 512, 8, 2, ROUTER_SCORE_TOPK, ACT_SOFTMAX, 1, 1.0),
-    # configs[1] and [2]: gpt-oss-20b shape, softmax over the selected k, logit bias, clamped SwiGLU
+    # gpt-oss-20b shape, decode and prefill, softmax over the selected k, logit bias, clamped SwiGLU
     "gpt-oss-20b": MoeConfig("gpt-oss-20b", 2880, 2880, 32, 4, ROUTER_TOPK_SOFTMAX, ACT_SOFTMAX, 1, 1.0,
                              logit_bias=True, swiglu_limit=7.0, swiglu_alpha=1.702,
                              swiglu_up_offset=1.0, act_block=32),
     "gpt-oss-20b-prefill": MoeConfig("gpt-oss-20b-prefill", 2880, 2880, 32, 4, ROUTER_TOPK_SOFTMAX,
                                      ACT_SOFTMAX, 1, 1.0, logit_bias=True, swiglu_limit=7.0,
                                      swiglu_alpha=1.702, swiglu_up_offset=1.0, act_block=32, zipf_s=1.1),
-    # configs[3]
+    # gpt-oss-120b shape
     "gpt-oss-120b": MoeConfig("gpt-oss-120b", 2880, 2880, 128, 4, ROUTER_TOPK_SOFTMAX, ACT_SOFTMAX, 1, 1.0,
                               logit_bias=True, swiglu_limit=7.0, swiglu_alpha=1.702,
                               swiglu_up_offset=1.0, act_block=32),
-    # configs[4]
+    # DeepSeek-V3 shape: grouped sigmoid routing, a shared expert
     "deepseek-v3": MoeConfig("deepseek-v3", 7168, 2048, 256, 8, ROUTER_SCORE_TOPK, ACT_SIGMOID, 1, 2.5,
                              bias_dtype=BIAS_F32, always_count=1, always_weight=1.0, n_group=8,
                              topk_group=4, act_block=128),

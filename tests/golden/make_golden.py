@@ -1,6 +1,6 @@
 """Regenerates the golden fixtures in this folder from the importable Python half of the reference.
 
-Run once, in a container that has the reference checkout (it cannot travel to a GPU box):
+Run once, in a container that has the reference checkout (the committed vectors need none):
 
     PYTHONPATH=<reference checkout> python tests/golden/make_golden.py
 

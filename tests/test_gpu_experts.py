@@ -263,10 +263,10 @@ def test_reduce_is_bit_exact(device):
 
 
 LAYER_CASES = [
-    pytest.param("tiny", None, 64, id="tiny-T64"),                                  # BASELINE configs[0]
+    pytest.param("tiny", None, 64, id="tiny-T64"),
     pytest.param("gpt-oss-20b", (256, 384, 16), 1, id="gptoss-small-T1"),
     pytest.param("gpt-oss-20b", (256, 384, 16), 33, id="gptoss-small-T33"),
-    pytest.param("gpt-oss-20b", (2880, 2880, 32), 8, id="gptoss-20b-T8"),            # configs[1] shape
+    pytest.param("gpt-oss-20b", (2880, 2880, 32), 8, id="gptoss-20b-T8"),
     pytest.param("gpt-oss-20b-prefill", (352, 160, 32), 600, id="gptoss-zipf-small-T600"),
     # wide token tiles on the TMA path: ragged row tiles (320 = 2.5 x 128), a K tail in down, row pairs with a lone half
     pytest.param("gpt-oss-20b-prefill", (384, 320, 8), 300, id="gptoss-zipf-tma-T300"),

@@ -19,10 +19,10 @@ pytestmark = pytest.mark.gpu
 
 # config name, batch sizes sharing one upload of the weights, sampled tokens per batch, expert paths
 FULL_CASES = [
-    pytest.param("gpt-oss-20b", (1, 8, 32, 64), 64, (1, 2), id="gpt-oss-20b-decode"),       # BASELINE configs[1]
-    pytest.param("gpt-oss-20b-prefill", (4096,), 48, (1, 2), id="gpt-oss-20b-prefill-zipf"),  # configs[2]
-    pytest.param("gpt-oss-120b", (8192,), 32, (2,), id="gpt-oss-120b"),                      # configs[3]
-    pytest.param("deepseek-v3", (16384,), 16, (2,), id="deepseek-v3"),                       # configs[4]
+    pytest.param("gpt-oss-20b", (1, 8, 32, 64), 64, (1, 2), id="gpt-oss-20b-decode"),
+    pytest.param("gpt-oss-20b-prefill", (4096,), 48, (1, 2), id="gpt-oss-20b-prefill-zipf"),
+    pytest.param("gpt-oss-120b", (8192,), 32, (2,), id="gpt-oss-120b"),
+    pytest.param("deepseek-v3", (16384,), 16, (2,), id="deepseek-v3"),
 ]
 
 

@@ -1,6 +1,7 @@
 """CPU-side checks of the product: the library loads, exports every declared symbol, and the
 host logic that needs no GPU behaves (no compute calls are made here)."""
 import ctypes
+import json
 import re
 from pathlib import Path
 
@@ -108,3 +109,16 @@ def test_traffic_captures_are_keyed_by_every_tensor_path_source(tmp_path, monkey
             f.write(b"\n")
         keys.add(bench.kernel_source_hash())
     assert len(keys) == 1 + len(names)
+
+
+def test_parity_metrics_are_written_only_where_the_caller_says(tmp_path, monkeypatch):
+    from tests import helpers
+
+    monkeypatch.delenv("NVMOE_PARITY_METRICS", raising=False)
+    before = sorted(p.name for p in ROOT.iterdir())
+    helpers.record_metrics("a", {"rel_l2": 0.0})
+    assert sorted(p.name for p in ROOT.iterdir()) == before
+    monkeypatch.setenv("NVMOE_PARITY_METRICS", str(tmp_path / "m.jsonl"))
+    helpers.record_metrics("a", {"rel_l2": 0.0})
+    helpers.record_metrics("b", {"rel_l2": 1.0})
+    assert [json.loads(line)["case"] for line in (tmp_path / "m.jsonl").read_text().splitlines()] == ["a", "b"]
