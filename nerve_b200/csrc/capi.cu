@@ -1266,16 +1266,19 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
             rc = fail(d, NVMOE_ERR_OUT_OF_MEMORY, "dense linear: out of device memory");
         if (rc == NVMOE_OK) {
             std::vector<uint32_t> ones(g.max_tokens, 0x3f80u << 16);  // weight 1.0, resource 0
-            if (cudaMemcpy(fresh.unit_routes.ptr, ones.data(), ones.size() * 4u, cudaMemcpyHostToDevice) != cudaSuccess)
-                rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the unit routes");
+            // (on the device's stream, which does not wait for copies of the legacy one: the first call's kernels read both)
+            cudaError_t err = cudaMemcpyAsync(fresh.unit_routes.ptr, ones.data(), ones.size() * 4u, cudaMemcpyHostToDevice, d->stream);
             // the map of the derived scales stays (the matrix's own maps, before it, are made by every call)
             unsigned char map[128];
             if (fresh.plan->tma[1] && most_tokens_per_expert(fresh.plan) > kPairsFrom) {
                 if (!tc_encode_pair_scale_map(map, fresh.set.derived.ptr, 1u, (uint32_t)(tc_derived_scale_bytes(rows, cols) / 512u)))
                     fresh.plan->tma[1] = false;
-                else if (cudaMemcpy(fresh.set.tmaps.as<uint8_t>() + kWeightMaps * 128u, map, 128, cudaMemcpyHostToDevice) != cudaSuccess)
-                    rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the scale map");
+                else if (err == cudaSuccess)
+                    err = cudaMemcpyAsync(fresh.set.tmaps.as<uint8_t>() + kWeightMaps * 128u, map, 128, cudaMemcpyHostToDevice, d->stream);
             }
+            const cudaError_t done = cudaStreamSynchronize(d->stream);  // `ones` and `map` go with this block
+            if (err == cudaSuccess) err = done;
+            if (err != cudaSuccess) rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the unit routes and the scale map: %s", cudaGetErrorString(err));
         }
         if (rc != NVMOE_OK) {
             nvmoe_plan_destroy(fresh.plan);
@@ -1699,7 +1702,7 @@ int nvmoe_plan_debug_cta_trace(nvmoe_plan* p, uint64_t* out, uint32_t max_ctas, 
     NVMOE_CUDA(d, cudaStreamSynchronize(d->stream));
     if (!p->cta_trace.ptr) {  // first request: arm the trace, the next calls fill it
         NVMOE_CUDA(d, p->cta_trace.ensure(bytes));
-        NVMOE_CUDA(d, cudaMemset(p->cta_trace.ptr, 0, bytes));
+        NVMOE_CUDA(d, cudaMemsetAsync(p->cta_trace.ptr, 0, bytes, d->stream));  // (in order with the kernels that fill it)
         return NVMOE_OK;
     }
     if (out && max_ctas >= (uint32_t)sms) NVMOE_CUDA(d, cudaMemcpy(out, p->cta_trace.ptr, bytes, cudaMemcpyDeviceToHost));

@@ -129,6 +129,28 @@ def test_dense_linear_matches_checker(device, path, tokens, rows, cols, block):
     plan.destroy()
 
 
+@pytest.mark.parametrize("cols", [128, 320])
+def test_first_dense_linear_of_a_plan_equals_the_next(device, cols):
+    """What the first call of a shape writes from the host (a weight per row, the map of the scales) is there when its
+    kernels read it: more rows than one staged copy holds."""
+    rng = np.random.default_rng(cols)
+    tokens, rows = 40000, 128
+    xb = device.resident_buffer_from(bf16(rng.standard_normal((tokens, cols))))
+    wb = device.resident_buffer_from(rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8))
+    sb = device.resident_buffer_from(rng.integers(121, 128, (rows, cols // 32), dtype=np.uint8))
+    ob = device.create_resident_buffer(tokens * rows * 2)
+    for _ in range(3):
+        _, plan = small_plan(device, tokens=tokens, act_block=32, path=2, hidden=256, intermediate=384)
+        got = []
+        for _call in range(2):
+            ob.fill(0)
+            plan.dense_linear(tokens, xb, ob, wb, sb, rows, cols)
+            got.append(ob.read(np.uint16))
+        assert plan.status() == 0
+        np.testing.assert_array_equal(got[0], got[1])
+        plan.destroy()
+
+
 def _ffn_block_nodes(hidden, intermediate, experts, k, limit):
     """The compiler's node list for one feed-forward block, resized from the committed one (4 experts of
     128 x 128) by editing exactly the attributes the compiler derives from the sizes."""
