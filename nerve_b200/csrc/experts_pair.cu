@@ -262,15 +262,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                 mine[2] = stage_it;
                 mine[3] = smid;
             }
-            if (!alive) {
-                // copies may still be on their way into either CTA's shared memory: wait, bounded, on the barriers of the last
-                // round (CTA 1 sees its scales land there, not its other copies, and waits out the time for those)
-                const uint32_t rounds = stage_it < slots ? stage_it : slots;
-                for (uint32_t back = 1u; back <= rounds; back++) {
-                    const uint32_t nth = stage_it - back;
-                    mbar_wait_winddown(&bars->full[nth % slots], rank == 0u ? (nth / slots) & 1u : 0u, kWinddownCycles / slots);
-                }
-            }
         }
         __syncwarp();
     } else if (warp == kPairMmaWarp) {
@@ -564,6 +555,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     if (*abort_flag && threadIdx.x == 0u) raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
     __syncwarp();
     cluster_sync();
+    // A CTA that did not give up has seen every copy, store and commit that reaches its shared memory (each of its tiles was
+    // finished); one that did may have some on their way that no role waited for, its own or, until the barrier above, the
+    // other CTA's.
+    if (*abort_flag && threadIdx.x == 0u) winddown_pause();
     if (warp == kPairMmaWarp) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, kPairTmemColumns);

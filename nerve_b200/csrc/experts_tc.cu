@@ -287,7 +287,6 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             uint32_t pair_nxt = entry_of(blockIdx.x + gridDim.x);
             // (debug) leave out the very first arrival of CTA 0: its consumer's bounded wait must then give up
             bool withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
-            uint32_t stage_it = 0u;  // stages this lane has gone through (stage n used slot n % kStages, phase n / kStages)
             for (uint32_t tile = blockIdx.x; tile < tile_count && alive; tile += gridDim.x) {
                 const uint32_t pair_nxt2 = entry_of(tile + 2u * gridDim.x);
                 if (tile + gridDim.x < tile_count) meta_of(tile + gridDim.x, pair_nxt, nxt);
@@ -344,7 +343,6 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                         bulk_copy_g2s(sf, scale_blocks[0] + (size_t)kb * C::kScaleStride, present * C::kMatrices * kScaleBlockBytes, &bars->full[slot]);
                     }
                     }
-                    stage_it++;
                     if (++slot == C::kStages) {
                         slot = 0u;
                         empty_parity ^= 1u;
@@ -352,17 +350,6 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 }
                 cur = nxt;
                 pair_nxt = pair_nxt2;
-            }
-            if (!alive) {
-                // The pipeline was aborted with copies of this lane possibly still on their way into shared
-                // memory: the CTA must not retire under them. Wait, bounded, on the stage barriers of the last
-                // round this lane armed; a barrier that also lacks an aborted role's arrivals never completes,
-                // and the time spent on it is the grace period instead.
-                const uint32_t rounds = stage_it < C::kStages ? stage_it : C::kStages;
-                for (uint32_t back = 1u; back <= rounds; back++) {
-                    const uint32_t nth = stage_it - back;
-                    mbar_wait_winddown(&bars->full[nth % C::kStages], (nth / C::kStages) & 1u, kWinddownCycles / C::kStages);
-                }
             }
         }
     } else if (USE_TMA && warp >= 6u && warp < 6u + C::kProducerWarps) {
@@ -855,7 +842,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
 
     // ---- teardown -------------------------------------------------------------------------------
     __syncthreads();
-    if (*abort_flag && threadIdx.x == 0u) raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
+    if (*abort_flag && threadIdx.x == 0u) {
+        raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
+        winddown_pause();  // copies that no role waited for any more may still be landing
+    }
     if (warp == 4u) {
         tc_fence_after();
         tmem_dealloc(tmem_base, C::kTmemColumns);

@@ -78,11 +78,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     return ok != 0u;
 }
 
-// Wind-down wait: for a role that is leaving after the pipeline was aborted and must first see what it
-// has in flight (bulk copies, tensor-core operations) finish.  It ignores the abort flag, which is set
-// by then, and gives up after `limit` cycles on its own; what it waits for completes within
-// microseconds unless the barrier also counts arrivals that an aborted role will never make, in which
-// case the time spent here is itself the grace period for the copies.
+// Wind-down wait: for the MMA thread, which must see the tensor-core operations it has in flight finish before tensor memory
+// is released, also when the pipeline was aborted. It ignores the abort flag, which is set by then, and gives up after `limit`
+// cycles on its own; what it waits for completes within microseconds.
 __device__ __forceinline__ bool mbar_wait_winddown(uint64_t* bar, uint32_t parity, long long limit) {
     const long long start = clock64();
     for (;;) {
@@ -92,6 +90,14 @@ __device__ __forceinline__ bool mbar_wait_winddown(uint64_t* bar, uint32_t parit
     }
 }
 constexpr long long kWinddownCycles = 4000000ll;  // about two milliseconds
+// One thread of a CTA whose pipeline was aborted, before the CTA retires: asynchronous copies into its shared memory may be on
+// their way, issued by a role that gave up, or by one that had gone through its loop to the end (a short K fits the ring, so that
+// the issuing lane never waits) when another gave up. Their barriers may lack an aborted role's arrivals and tell nothing, so
+// the CTA stays for a time that any copy is through in.
+__device__ __forceinline__ void winddown_pause() {
+    const long long start = clock64();
+    while (clock64() - start < kWinddownCycles) __nanosleep(1000);
+}
 
 // ---- CTA pairs ------------------------------------------------------------------------------------------
 

@@ -454,3 +454,33 @@ def test_bounded_wait_gives_up_and_the_plan_recovers(device):
         assert plan.status() == 0
         np.testing.assert_array_equal(out.read(np.uint16), before)
     plan.destroy()
+
+
+# K that fits the ring of stages, so that the issuing lane is through before any wait runs out, and K beyond it; operands by
+# TMA and (columns off the 64 grid) by cp.async; narrow tiles and wide ones
+@pytest.mark.parametrize("shape,tokens", [((256, 512, 8), 64), ((128, 128, 8), 5), ((1152, 1216, 8), 100), ((288, 352, 8), 40), ((288, 96, 8), 300)])
+def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, shape, tokens):
+    """Limits from a cycle up end waits of every role in the middle of the pipeline: each call returns, and with the ordinary
+    limit the next one is bit-identical to the one before."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], *shape)
+    case = synthetic.make_case(cfg, tokens, seed=31)
+    plan = make_plan(device, cfg, tokens, 2)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw)
+    assert plan.status() == 0
+    before, seen = out.read(np.uint16).copy(), 0
+    for limit in (1, 400, 1500, 4000, 20000):
+        plan.set_wait_limit(limit)
+        for _ in range(4):
+            plan.layer(tokens, bank, hidden, out, router_weights=rw)
+        device.synchronize(timeout_ns=20_000_000_000)
+        seen |= plan.status()
+    assert seen & ~8 == 0
+    plan.set_wait_limit(0)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw)
+    assert plan.status() == 0
+    np.testing.assert_array_equal(out.read(np.uint16), before)
+    plan.destroy()
+    bank.destroy()
