@@ -99,3 +99,33 @@ def test_a_wait_that_expires_is_reported(device):
         np.testing.assert_array_equal(out.read(np.uint16), before)
     plan.destroy()
     bank.destroy()
+
+
+# K of one stage and of several, weight rows of one tile and of more, scale blocks of 32 and of 128 (the warps of a group hand
+# maxima round in the middle of the exchange)
+@pytest.mark.parametrize("name,shape,tokens", [("gpt-oss-20b", (128, 192, 4), 97), ("gpt-oss-20b", (704, 448, 4), 241), ("deepseek-v3", (512, 384, 16), 240)])
+def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, name, shape, tokens):
+    cfg = synthetic.small_variant(synthetic.CONFIGS[name], *shape)
+    case = synthetic.make_case(cfg, tokens, seed=33)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_expert_path(2)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    bias = device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw, bias=bias)
+    assert plan.status() == 0
+    before, seen = out.read(np.uint16).copy(), 0
+    for limit in (1, 400, 1500, 4000, 20000):
+        plan.set_wait_limit(limit)
+        for _ in range(4):
+            plan.layer(tokens, bank, hidden, out, router_weights=rw, bias=bias)
+        device.synchronize(timeout_ns=20_000_000_000)
+        seen |= plan.status()
+    assert seen & ~8 == 0
+    plan.set_wait_limit(0)
+    plan.layer(tokens, bank, hidden, out, router_weights=rw, bias=bias)
+    assert plan.status() == 0
+    np.testing.assert_array_equal(out.read(np.uint16), before)
+    plan.destroy()
+    bank.destroy()
