@@ -438,7 +438,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                 uint32_t s[16];
                 tmem_ld16(lane_addr + 16u * c, s);
                 // (the place is free again once the other warp has taken what was sent last)
-                lost = !mbar_wait_warp(&bars->taken[warp], (sends & 1u) ^ 1u, abort_flag, wait_limit);
+                lost = !mbar_wait_cluster_warp(&bars->taken[warp], (sends & 1u) ^ 1u, abort_flag, wait_limit);
                 tmem_ld_wait();
                 if (lost) return;
                 uint32_t v[8];

@@ -116,7 +116,12 @@ __device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// arrival on a barrier of either CTA (`addr` from map_shared)
+// Arrival on a barrier of either CTA (`addr` from map_shared). It releases at CTA scope, the default: release.cluster also waits
+// for the thread's global stores, which nothing here hands over, and cost more than 1000 cycles an arrival. What the arrivals of
+// a pair do hand over is complete before them without it: scale words written in place are put before the tensor core's proxy by
+// fence.proxy.async and stay in the CTA that wrote them; accumulator columns and exchanged chunks are reads, performed in the
+// warp's order ahead of its arrival (tcgen05.wait::ld and fence::before_thread_sync; loads from its own shared memory, which
+// a release at CTA scope orders), and whoever sees the arrival overwrites them only after that.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
@@ -131,7 +136,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
         : "memory");
     return ok != 0;
 }
-// mbar_wait, by a whole warp, for what store_async_cluster of the other CTA brings
+// mbar_wait, by a whole warp, for what the other CTA does to or with shared memory that store_async_cluster fills
 __device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, long long limit) {
     uint32_t ok = 0u;
     if ((threadIdx.x & 31u) == 0u) {
