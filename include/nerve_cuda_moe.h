@@ -425,7 +425,7 @@ int nvmoe_plan_debug_counters(nvmoe_plan* plan, uint64_t* out24);
  * consumed, SM id} of the most recent kernels into `out` (room for max_ctas CTAs per stage).
  * Synchronises the stream. No reference counterpart. */
 int nvmoe_plan_debug_cta_trace(nvmoe_plan* plan, uint64_t* out, uint32_t max_ctas, uint32_t* ctas);
-/* Makes CTA 0 of the gate/up tensor-core kernel leave out its first pipeline-stage arrival, so that its
+/* Makes CTA 0 of the tensor-core expert kernels leave out its first pipeline-stage arrival, so that its
  * consumer's bounded wait runs out: the way the give-up path (nvmoe_plan_set_wait_limit) is tested
  * without faulting or hanging anything. The call's output is incomplete and NVMOE_STATUS_WAIT_EXPIRED is
  * raised; switch it off again for the next call. */

@@ -318,7 +318,7 @@ class MoePlan:
         self._call("nvmoe_plan_set_wait_limit", clock_cycles)
 
     def debug_withhold_arrival(self, enabled: bool) -> None:
-        """Test aid: CTA 0 of the gate/up kernel leaves out one stage arrival, so that a bounded wait runs out."""
+        """Test aid: CTA 0 of the expert kernels leaves out one stage arrival, so that a bounded wait runs out."""
         self._call("nvmoe_plan_debug_withhold_arrival", int(enabled))
 
     def set_profiling(self, enabled: bool) -> None:

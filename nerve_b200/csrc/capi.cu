@@ -908,6 +908,7 @@ struct ExpertCall {
     bool scheduled = false;         // grouping (and tile list) already built for this call
     bool fuse_quantise = false;     // gate/up on the tensor path: the epilogue also writes the down stage's operands
     bool fresh_maps = false;        // the last launch before this one writes the tensor maps
+    uint32_t* status = nullptr;     // the word that the caller's plan reads (null: this plan's own)
 };
 
 // shared tail of the two gate/up entry points and of down
@@ -938,7 +939,7 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
     el.intermediates = c.intermediates;
     el.outputs = c.outputs;
     el.partial_outputs = c.partial_outputs;
-    el.status = p->status.as<uint32_t>();
+    el.status = c.status ? c.status : p->status.as<uint32_t>();
     el.scale_stamps = es->stamps.as<uint64_t>();
     el.cta_trace = p->cta_trace.as<uint64_t>();
     el.tmaps = tensor && p->tma[set] ? es->tmaps.as<uint8_t>() : nullptr;
@@ -1292,6 +1293,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     nvmoe_plan* sub = dl->plan;
     sub->expert_path = p->expert_path;
     sub->wait_cycles = p->wait_cycles;
+    sub->debug_flags = p->debug_flags;
     cudaStream_t st = d->stream;
     const bool tensor = use_tensor_path(sub);
     uint32_t* region = sub->tile_list.as<uint32_t>() + tile_region_words(sub);
@@ -1333,6 +1335,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     call.outputs = (uint16_t*)output->ptr;
     call.prepared = &dl->set;
     call.fresh_maps = true;
+    call.status = p->status.as<uint32_t>();
     call.scheduled = true;
     NVMOE_TRY(run_experts(sub, call));
     p->launches += sub->launches;

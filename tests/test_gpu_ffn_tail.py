@@ -151,6 +151,29 @@ def test_first_dense_linear_of_a_plan_equals_the_next(device, cols):
         plan.destroy()
 
 
+# one CTA a tile, CTA pairs
+@pytest.mark.parametrize("tokens", [40, 130])
+def test_dense_linear_reports_a_wait_that_expires(device, tokens):
+    rng = np.random.default_rng(tokens)
+    rows, cols = 384, 256
+    x = bf16(rng.standard_normal((tokens, cols)))
+    w, sc = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(121, 128, (rows, cols // 32), dtype=np.uint8)
+    _, plan = small_plan(device, tokens=tokens, path=2)
+    xb, wb, sb = device.resident_buffer_from(x), device.resident_buffer_from(w), device.resident_buffer_from(sc)
+    ob = device.create_resident_buffer(tokens * rows * 2)
+    plan.set_wait_limit(2_000_000)  # about a millisecond
+    plan.debug_withhold_arrival(True)
+    plan.dense_linear(tokens, xb, ob, wb, sb, rows, cols)
+    device.synchronize(timeout_ns=20_000_000_000)
+    assert plan.status() & 8
+    plan.debug_withhold_arrival(False)
+    plan.set_wait_limit(0)
+    plan.dense_linear(tokens, xb, ob, wb, sb, rows, cols)
+    assert plan.status() == 0
+    assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, sc, 32, tier=1))
+    plan.destroy()
+
+
 def _ffn_block_nodes(hidden, intermediate, experts, k, limit):
     """The compiler's node list for one feed-forward block, resized from the committed one (4 experts of
     128 x 128) by editing exactly the attributes the compiler derives from the sizes."""
