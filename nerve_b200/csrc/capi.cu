@@ -474,7 +474,8 @@ int nvmoe_sync(nvmoe_device* d, uint64_t timeout_ns) {
 
 // ---- plan ------------------------------------------------------------------------------------
 
-int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_plan** out) {
+// dense: a plan of which only the down stage runs, on a compact matrix (nvmoe_dense_linear).
+static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool dense, nvmoe_plan** out) {
     if (!d || !geometry || !out) return fail(d, NVMOE_ERR_INVALID_ARGUMENT, "null argument");
     *out = nullptr;
     int rc = validate_geometry(*geometry);
@@ -515,17 +516,22 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
         want(p->act_maps, 2u * kActMaps * 128u);
         const size_t most = most_tokens_per_expert(p);
         const bool with_pairs = most > kPairsFrom;
+        // Only the maps that the plan's calls can use are encoded, at about 2.8 us each; the others stay zero and are not looked at.
         if (err == cudaSuccess) {
-            unsigned char maps[2u * kActMaps * 128u] = {0};  // (maps of tiles that no call of the plan uses stay zero)
+            unsigned char maps[2u * kActMaps * 128u] = {0};
             bool ok = true;
-            for (uint32_t set = 0; set < 2u && ok; set++) {
+            for (uint32_t set = dense ? 1u : 0u; set < 2u && ok; set++) {
                 const uint32_t cols = (uint32_t)(set == 0u ? H : I);
                 unsigned char* mine = maps + set * kActMaps * 128u;
                 if (cols % 64u != 0u || cols < 128u) continue;  // (no map for its weights either)
                 for (uint32_t i = 0; i < kTokenMaps && ok; i++) {
                     if (most <= kTokenMapFrom[i]) continue;
-                    ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]) &&
-                         tc_encode_pair_token_map(mine + (kTokenMaps + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
+                    // one K block: tiles of one CTA (of every width but the last), a pair's lone or trailing half block; two: pairs,
+                    // and the narrow down tiles of a single row tile
+                    if (i + 1u < kTokenMaps || cols % 256u != 0u)
+                        ok = tc_encode_activation_map(mine + i * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
+                    if ((with_pairs && i > 0u) || (set == 1u && kTokenMapRows[i] < kRowPairTokens))
+                        ok = ok && tc_encode_pair_token_map(mine + (kTokenMaps + i) * 128u, p->grouped_q[set].ptr, (uint32_t)R, cols, kTokenMapRows[i]);
                 }
                 if (with_pairs) ok = ok && tc_encode_token_scale_map(mine + kTokenScaleMap * 128u, p->grouped_e8m0[set].ptr, scale_rows(p), (cols + 127u) / 128u);
             }
@@ -541,18 +547,21 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
             // per stage: the maps of the compact form, those of the one-byte-per-element forms (left zero when the shape has no
             // whole 128-column blocks: such resources are then treated as not resident), the map of the derived scales
             unsigned char maps[2u * kMapTemplates] = {0};
-            for (uint32_t set = 0; set < 2u; set++) {
+            for (uint32_t set = dense ? 1u : 0u; set < 2u; set++) {
                 const uint32_t rows = set == 0u ? g.intermediate_size : g.hidden_size, cols = set == 0u ? g.hidden_size : g.intermediate_size;
                 unsigned char* mine = maps + set * kMapTemplates;
                 const uint64_t blocks = tc_derived_scale_bytes(rows, cols) / 512u * p->experts;
+                // (the maps of launch_build_tensormaps_tc)
+                const uint32_t count = tc_weight_maps(set == 0u, with_pairs);
                 p->tma[set] = p->act_maps.ptr && tc_encode_weight_map(mine, p->tmap_templates.ptr, rows, cols, 128u) &&
-                              tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false) &&
-                              tc_encode_weight_map(mine + 256, p->tmap_templates.ptr, rows, cols, 256u) &&
+                              (count < 2u || tc_encode_pair_weight_map(mine + 128, p->tmap_templates.ptr, rows, cols, false)) &&
+                              (count < 3u || tc_encode_weight_map(mine + 256, p->tmap_templates.ptr, rows, cols, 256u)) &&
                               (!with_pairs || (blocks <= 0x7fffffffull &&
                                                tc_encode_pair_scale_map(mine + 768, p->tmap_templates.ptr, set == 0u ? 2u : 1u, (uint32_t)blocks)));
+                if (dense) continue;
                 tc_encode_weight_map_bytes(mine + 384, p->tmap_templates.ptr, rows, cols, 128u);
-                tc_encode_pair_weight_map(mine + 512, p->tmap_templates.ptr, rows, cols, true);
-                tc_encode_weight_map_bytes(mine + 640, p->tmap_templates.ptr, rows, cols, 256u);
+                if (count > 1u) tc_encode_pair_weight_map(mine + 512, p->tmap_templates.ptr, rows, cols, true);
+                if (count > 2u) tc_encode_weight_map_bytes(mine + 640, p->tmap_templates.ptr, rows, cols, 256u);
             }
             err = cudaMemcpyAsync(p->tmap_templates.ptr, maps, sizeof maps, cudaMemcpyHostToDevice, d->stream);
             if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
@@ -573,6 +582,8 @@ int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_pla
     *out = p;
     return NVMOE_OK;
 }
+
+int nvmoe_plan_create(nvmoe_device* d, const nvmoe_geometry* geometry, nvmoe_plan** out) { return create_plan(d, geometry, false, out); }
 
 void nvmoe_plan_destroy(nvmoe_plan* p) {
     if (!p) return;
@@ -1258,7 +1269,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         nvmoe_geometry_default(&g, rows, cols, 1u, 1u);
         g.act_block = p->g.act_block;
         g.max_tokens = p->g.max_tokens;
-        NVMOE_TRY(nvmoe_plan_create(d, &g, &fresh.plan));
+        NVMOE_TRY(create_plan(d, &g, true, &fresh.plan));
         fresh.plan->expert_path = p->expert_path;
         int rc = NVMOE_OK;
         const bool tensor_shape = tc_shape_supported(g);

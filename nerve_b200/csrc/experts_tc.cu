@@ -900,31 +900,33 @@ __global__ void commit_stamps_kernel(const ExpertPtrs* experts, uint64_t* stamps
 
 // (a whole warp) the template with an address patched in, as a map that the TMA unit may be given once it has been acquired
 __device__ __forceinline__ void publish_map(uint8_t* map, const uint8_t* templ, unsigned char* smem_map, const uint8_t* address) {
-    reinterpret_cast<uint32_t*>(smem_map)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t*>(templ) + threadIdx.x);
+    const uint32_t lane = threadIdx.x & 31u;
+    reinterpret_cast<uint32_t*>(smem_map)[lane] = __ldg(reinterpret_cast<const uint32_t*>(templ) + lane);
     __syncwarp();
-    if (threadIdx.x == 0u) tensormap_replace_address(smem_map, address);
+    if (lane == 0u) tensormap_replace_address(smem_map, address);
     __syncwarp();
     tensormap_publish(map, smem_map);
 }
 
-// One warp per (expert, matrix): the template maps (kWeightMaps) with the expert's weight address patched in; then one for the map of the set's derived scale copy.
+// One warp per map (an expert matrix's `per_matrix` of kWeightMaps): the template with the expert's weight address patched in;
+// then one for the map of the set's derived scale copy. Bound by the latency of the copy's fence, once this way: tables that are
+// resolved in every call add 35 us with 32 experts and 65 with 257 (38 and 69 with a warp that wrote three maps in turn).
 __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* experts, const uint8_t* templ, const uint8_t* derived,
-                                                             uint8_t* maps, uint32_t matrices) {
-    __shared__ __align__(128) unsigned char sm[kWeightMaps * 128u];
-    const uint32_t e = blockIdx.x / matrices, mx = blockIdx.x % matrices;
+                                                             uint8_t* maps, uint32_t matrices, uint32_t per_matrix) {
+    __shared__ __align__(128) unsigned char sm[128];
+    const uint32_t matrix = blockIdx.x / per_matrix, i = blockIdx.x % per_matrix;
+    const uint32_t e = matrix / matrices, mx = matrix % matrices;
     const bool scales = derived != nullptr && blockIdx.x == gridDim.x - 1u;
     if (!scales && (experts[e].w[0] == nullptr || experts[e].w[mx] == nullptr)) return;
-    const uint8_t* w = scales ? derived : experts[e].w[mx];
     // `templ` holds the maps of the compact form, those of the one-byte-per-element forms and that of the derived scales
-    const uint8_t* mine = templ + (scales ? 2u : experts[e].format == kFormatCompact ? 0u : 1u) * kWeightMaps * 128u;
-    for (uint32_t i = 0; i < (scales ? 1u : kWeightMaps); i++)
-        publish_map(maps + ((size_t)blockIdx.x * kWeightMaps + i) * 128u, mine + i * 128u, sm + i * 128u, w);
+    const uint8_t* mine = templ + ((scales ? 2u : experts[e].format == kFormatCompact ? 0u : 1u) * kWeightMaps + i) * 128u;
+    publish_map(maps + ((size_t)matrix * kWeightMaps + i) * 128u, mine, sm, scales ? derived : experts[e].w[mx]);
 }
 
 // The same for the one matrix of a dense linear, whose addresses are the call's own: nothing about the matrix is kept
 // between calls, so that scales rewritten in place by any means are what the next call reads. A block re-tiles 128 rows
 // x 4 K blocks, a thread 4 rows of one K block and one 16-byte store. The last block writes the pointers and the tensor
-// map. With scale blocks of 32 or 128 columns (LANES = block / 16; 0: none) further blocks quantise the input, a warp 512
+// maps, a warp each. With scale blocks of 32 or 128 columns (LANES = block / 16; 0: none) further blocks quantise the input, a warp 512
 // columns of one row, so that the launch takes little longer than that alone: bound by the latency of a load and a
 // store. Block of 777 x 7168 x 2048: 114.0 us with the quantisation in a launch of its own, 107 here.
 constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
@@ -983,9 +985,8 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
         if (p.tiles.count) *p.tiles.count = tile_total;
         *p.ptrs = ExpertPtrs{{p.weights, nullptr}, {p.scales, nullptr}, {p.derived, nullptr}, {0u, 0u}, kFormatCompact, 0u};
     }
-    if (p.map_template != nullptr && threadIdx.x < 32u) {
-        for (uint32_t i = 0; i < kWeightMaps; i++) publish_map(p.map + i * 128u, p.map_template + i * 128u, sm + i * 128u, p.weights);
-    }
+    const uint32_t i = threadIdx.x / 32u;
+    if (p.map_template != nullptr && i < kWeightMaps) publish_map(p.map + i * 128u, p.map_template + i * 128u, sm + i * 128u, p.weights);
 }
 
 int g_sm_count[16] = {0};
@@ -1021,7 +1022,7 @@ void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
 // owned (1.3 and 2.6 rounds of their own): 115.3 / 115.6 and 136.4 / 132.4 with 32-token tiles, 87.3 / 87.7 and 105.1 /
 // 104.2 with 16.
 bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) {
-    if (n_tile >= 64u) return true;
+    if (n_tile >= kRowPairTokens) return true;
     if (!tma) return false;
     const uint64_t routes = (uint64_t)p.tokens * (p.g.routed_k + p.g.always_count);
     const uint64_t lists = routes < p.work.num_experts ? routes : p.work.num_experts;
@@ -1286,9 +1287,9 @@ bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t 
 }
 
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream) {
-    const uint32_t matrices = gate_up ? 2u : 1u;
-    build_tensormaps_kernel<<<p.work.num_experts * matrices + (p.scale_base ? 1u : 0u), 32, 0, stream>>>(p.work.experts, templ, p.scale_base,
-                                                                                   const_cast<uint8_t*>(p.tmaps), matrices);
+    const uint32_t matrices = gate_up ? 2u : 1u, per_matrix = tc_weight_maps(gate_up, p.scale_base != nullptr);
+    build_tensormaps_kernel<<<p.work.num_experts * matrices * per_matrix + (p.scale_base ? 1u : 0u), 32, 0, stream>>>(
+        p.work.experts, templ, p.scale_base, const_cast<uint8_t*>(p.tmaps), matrices, per_matrix);
 }
 
 void tc_configure_kernels() {

@@ -15,8 +15,10 @@ void tc_configure_kernels();
 bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows);
 // The same for a matrix held as one E4M3 byte per element (pre-expanded or native FP8 resources).
 bool tc_encode_weight_map_bytes(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows);
-// Tensor maps of a weight matrix: boxes of 128 rows x one K block, 128 rows x two, 256 rows x one.
+// Tensor maps of a weight matrix: boxes of 128 rows x one K block, 128 rows x two, 256 rows x one; and how many of them a
+// stage's kernels use (gate/up has tiles of 128 rows of either matrix, and two K blocks a copy in CTA pairs only).
 constexpr uint32_t kWeightMaps = 3u;
+constexpr uint32_t tc_weight_maps(bool gate_up, bool with_pairs) { return !gate_up ? 3u : with_pairs ? 2u : 1u; }
 // Encodes the tensor map of an expert-grouped activation matrix [rows][cols] of E4M3 bytes with a box of
 // n_tile rows x 128 bytes (the operand tile of one K block). False when tensor maps are unavailable.
 bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t n_tile);
@@ -27,8 +29,8 @@ bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t 
 bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows);
 bool tc_encode_pair_scale_map(void* map128, void* any_device_address, uint32_t sources, uint32_t blocks);
 bool tc_encode_token_scale_map(void* map128, void* base, uint32_t words, uint32_t rows);
-// per-expert tensor maps = template + the expert's weight address (p.tmaps must be set), and after them the map of the
-// derived scales (p.scale_base)
+// per-expert tensor maps = template + the expert's weight address (p.tmaps must be set; tc_weight_maps of each matrix), and
+// after them the map of the derived scales (p.scale_base: the plan's calls may run by CTA pairs)
 void launch_build_tensormaps_tc(const ExpertLaunch& p, bool gate_up, const uint8_t* templ, cudaStream_t stream);
 // What a dense linear needs before its expert kernel, in one launch: the schedule (every row a route of expert 0 in row
 // order), what hangs on its matrix (the pointers and, for the tensor path (`derived` set), the re-tiled scales and the
@@ -60,7 +62,8 @@ struct TokenTile {
 // token tile of a stage for this many tokens and rows of its weight matrix (the (expert, token tile) list must be
 // built with it); tma: the stage's shapes have tensor maps
 TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up, bool tma);
-constexpr uint32_t kPairTokens = 240u;  // the most tokens of a pair's tile
+constexpr uint32_t kPairTokens = 240u;    // the most tokens of a pair's tile
+constexpr uint32_t kRowPairTokens = 64u;  // one CTA's down tiles of that many tokens and more always take two row tiles
 void pair_configure_kernels();
 void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream);
 // Tensor maps of a stage's operands: token rows in boxes of one K block, for one CTA's token tiles and, from the second on,

@@ -396,3 +396,34 @@ def test_dense_linear_operands(device, block, shift, rows, cols, tokens):
     assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, block, tier=1))
     assert plan.status() == 0
     plan.destroy()
+
+
+# every token tile from one plan: a call has the tensor maps of its tile whatever the plan's largest call is (boxes of one K
+# block and of two, whole pairs of blocks and a trailing half; one-byte weights)
+@pytest.mark.parametrize("name,shape,native", [("gpt-oss-20b", (576, 512, 8), 0), ("deepseek-v3", (512, 384, 16), 1)])
+def test_calls_of_every_tile_from_one_plan(device, name, shape, native):
+    cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], *shape), native_fp8_resources=native)
+    case = synthetic.make_case(cfg, 500, seed=23)
+    tensors = [list(t) for t in (case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)]
+    for e in range(cfg.total_experts - native, cfg.total_experts):
+        for i, t in enumerate(synthetic.native_fp8_tensors(cfg, 23, e)):
+            tensors[i][e] = t
+    bank = ExpertBank.upload(device, *tensors)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    args = {"router_weights": rw, "router_bias": device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+            "bias": device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None}
+    out = device.create_resident_buffer(500 * cfg.hidden * 2)
+    large = MoePlan.for_config(device, cfg, 500)
+    for tokens in (1, 9, 10, 20, 40, 80, 96, 200, 500):
+        own = MoePlan.for_config(device, cfg, tokens)
+        got = []
+        for plan in (large, own):
+            plan.set_expert_path(2)
+            out.fill(0)
+            plan.layer(tokens, bank, hidden, out, **args)
+            assert plan.status() == 0
+            got.append(out.read(np.uint16))
+        np.testing.assert_array_equal(got[0], got[1], err_msg=f"{tokens} tokens")
+        own.destroy()
+    large.destroy()
+    bank.destroy()
