@@ -415,14 +415,16 @@ int nvmoe_plan_last_report(nvmoe_plan* plan, nvmoe_work_report* report);
  * switches the plan to instantiations that carry them.
  *
  * Diagnostics of the last tensor-core expert kernels (valid once the trace is armed): counters of CTA 0, twelve words for
- * gate/up then twelve for down: cycles {producer wait, producer total, MMA wait-operands, MMA
- * wait-accumulator, MMA total}, stages, cycles {epilogue wait, epilogue total}, then global-timer
- * nanoseconds {kernel entry, MMA loop begin, MMA loop end, latest exit of any CTA}. Synchronises
- * the stream. No reference counterpart. */
+ * gate/up then twelve for down: cycles of the lane that issues the copies {wait for a free stage, total}, of the MMA thread
+ * {wait for operands, for an accumulator, total}, stages, cycles of the epilogue {wait, total}, then global-timer
+ * nanoseconds {kernel entry, MMA loop begin, MMA loop end, latest exit of any CTA}. Zeros after a call that ran by CTA pairs
+ * or without tensor maps (columns that 64 does not divide), whose kernels count nothing. Synchronises the stream. No
+ * reference counterpart. */
 int nvmoe_plan_debug_counters(nvmoe_plan* plan, uint64_t* out24);
 /* Per-CTA diagnostics of the tensor-core expert kernels. The first call arms the trace (and writes
  * the CTA count); later calls copy [2 stages][ctas][4] words {loop begin ns, loop end ns, stages
- * consumed, SM id} of the most recent kernels into `out` (room for max_ctas CTAs per stage).
+ * consumed, SM id} of the most recent kernels into `out` (room for max_ctas CTAs per stage): of the MMA thread's loop, of
+ * the copy-issuing lane's in CTA pairs, zeros without tensor maps.
  * Synchronises the stream. No reference counterpart. */
 int nvmoe_plan_debug_cta_trace(nvmoe_plan* plan, uint64_t* out, uint32_t max_ctas, uint32_t* ctas);
 /* Makes CTA 0 of the tensor-core expert kernels leave out its first pipeline-stage arrival, so that its

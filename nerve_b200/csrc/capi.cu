@@ -967,6 +967,12 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
         el.token_rows = tile.rows;
         el.pairs = tile.pair;
         el.act_tmap = el.tmaps ? p->act_maps.as<uint8_t>() + (set * kActMaps + tc_token_map_for(tile)) * 128u : nullptr;
+        if (el.cta_trace && (tile.pair || !el.tmaps)) {
+            // kernels that write no counters (CTA pairs), nor a trace (operands by cp.async): an earlier call's must not pass for theirs
+            NVMOE_CUDA(p->device, cudaMemsetAsync(el.tile_count + (gate_up ? 16 : 40), 0, 96, st));
+            const size_t half = p->cta_trace.bytes / 2u;
+            if (!el.tmaps) NVMOE_CUDA(p->device, cudaMemsetAsync(p->cta_trace.as<uint8_t>() + (gate_up ? 0u : half), 0, half, st));
+        }
         if (c.fuse_quantise && gate_up) {
             el.q_out = p->grouped_q[1].as<uint8_t>();
             el.q_e8m0 = scale_words(p, false, T);

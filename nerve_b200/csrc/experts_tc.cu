@@ -258,6 +258,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
         if (USE_TMA && lane == 0u) {
             uint32_t slot = 0u, empty_parity = 1u;
             bool alive = true;
+            long long trace_wait = 0;
+            const long long trace_begin = TRACE ? clock64() : 0;
             // What the lane needs to know about a tile. The list entry of a tile is fetched two tiles ahead and
             // what hangs on it (the expert's offset, scale and tensor-map addresses) one tile ahead, so that the
             // chain of dependent loads is over by the time the tile starts: a lane that stalled on it at every
@@ -300,10 +302,12 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 for (uint32_t mx = 0; mx < C::kMatrices; mx++)
                     scale_blocks[mx] = cur.ts[C::source_of(mx)] + (size_t)scale_tile(m_tile, mx) * k_blocks * C::kScaleStride;
                 for (uint32_t ks = 0; ks < k_stages; ks++) {
+                    const long long w0 = TRACE ? clock64() : 0;
                     if (!mbar_wait(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
                         alive = false;
                         break;
                     }
+                    if (TRACE) trace_wait += clock64() - w0;
                     const bool two = ks < doubles;
                     const uint32_t kb = first_block(ks), present = two ? 2u : 1u;
                     if (withhold) {
@@ -350,6 +354,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
                 }
                 cur = nxt;
                 pair_nxt = pair_nxt2;
+            }
+            if (TRACE && blockIdx.x == 0u) {
+                trace[0] = (uint64_t)trace_wait;                    // copy-issuing lane: cycles waiting for a free stage
+                trace[1] = (uint64_t)(clock64() - trace_begin);     // copy-issuing lane: cycles in its loop
             }
         }
     } else if (USE_TMA && warp >= 6u && warp < 6u + C::kProducerWarps) {
@@ -452,8 +460,6 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             m.scale_row = first + (kProducerThreads - 65u - pt);
         };
         uint32_t slot = 0u, empty_parity = 1u;  // a fresh barrier passes a wait on parity 1
-        long long trace_wait = 0;
-        const long long trace_begin = TRACE ? clock64() : 0;
         const uint32_t my_dst = swizzle128_offset(my_r, my_c);
         bool alive = true;
         Meta cur, nxt;
@@ -474,12 +480,10 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             }
             const size_t row_step = (size_t)kRowsPerPass * form_row_bytes;
             for (uint32_t ks = 0; ks < k_stages; ks++) {
-                const long long w0 = TRACE ? clock64() : 0;
                 if (!mbar_wait_warp(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
                     alive = false;
                     break;
                 }
-                if (TRACE) trace_wait += clock64() - w0;
 #pragma unroll
                 for (uint32_t sub = 0; sub < C::kSub; sub++) {
                 if (sub != 0u && ks >= doubles) break;  // the last stage of an odd count holds one block
@@ -544,10 +548,6 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             cur = nxt;
         }
         cp_async_wait_all();  // nothing of this thread may still be landing when the CTA retires
-        if (TRACE && blockIdx.x == 0u && pt == 0u) {
-            trace[0] = (uint64_t)trace_wait;                    // producer: cycles waiting for a free stage
-            trace[1] = (uint64_t)(clock64() - trace_begin);     // producer: cycles in its loop
-        }
     } else if (warp == 4u) {
         // ===== MMA issue (one elected lane) ======================================================
         if (elect_one()) {

@@ -5,6 +5,7 @@ layers against the CPU checker: indices bit-exact, bf16 outputs within the state
 f64-accumulated reference on the same quantised operands.  Every case runs on both expert paths
 (1 = CUDA-core dequant-GEMV, 2 = tcgen05 grouped MMA).
 """
+import ctypes
 import json
 from pathlib import Path
 
@@ -484,3 +485,44 @@ def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, shape, tokens)
     np.testing.assert_array_equal(out.read(np.uint16), before)
     plan.destroy()
     bank.destroy()
+
+
+def test_debug_counters_are_those_of_the_last_kernels(device):
+    """One CTA a tile fills its counters and trace; CTA pairs fill the trace and leave zeros for the counters, kernels without
+    tensor maps zeros for both, whatever ran before."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 320, 448, 8)
+    odd = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 352, 416, 8)
+    runs = []
+    for c in (cfg, odd):
+        case = synthetic.make_case(c, 300, seed=35)
+        plan = make_plan(device, c, 300, 2)
+        bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+        runs.append((plan, bank, device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w),
+                     device.create_resident_buffer(300 * c.hidden * 2)))
+
+    def call(run, tokens):
+        plan, bank, hidden, rw, out = run
+        ctas = ctypes.c_uint32()
+        plan._call("nvmoe_plan_debug_cta_trace", None, 0, ctypes.byref(ctas))
+        plan.layer(tokens, bank, hidden, out, router_weights=rw)
+        counters, trace = (ctypes.c_uint64 * 24)(), np.zeros((2, ctas.value, 4), dtype=np.uint64)
+        plan._call("nvmoe_plan_debug_counters", counters)
+        plan._call("nvmoe_plan_debug_cta_trace", trace.ctypes.data, ctas.value, ctypes.byref(ctas))
+        assert plan.status() == 0
+        return np.array(counters, dtype=np.uint64).reshape(2, 12), trace
+
+    call(runs[0], 8)  # (arms the trace; the next calls fill it)
+    for _ in range(2):
+        counters, trace = call(runs[0], 40)   # a tile of one CTA: 20 tokens an expert
+        assert (counters[:, [1, 4, 5, 7, 8, 9, 10, 11]] > 0).all() and (counters[:, 0] <= counters[:, 1]).all()
+        # gate/up: 2.5 K blocks, a stage each; down: 3.5, two to a stage but for the lone and the half one
+        assert counters[0, 5] % 3 == 0 and counters[1, 5] % 3 == 0
+        assert (trace[:, 0, 2] == counters[:, 5]).all()
+        counters, trace = call(runs[0], 300)  # CTA pairs: 150 tokens an expert
+        assert not counters.any() and (trace[:, :2, 2] > 0).all()
+    call(runs[1], 8)
+    counters, trace = call(runs[1], 300)
+    assert not counters.any() and not trace.any()
+    for plan, bank, *_ in runs:
+        plan.destroy()
+        bank.destroy()
