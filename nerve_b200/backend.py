@@ -317,9 +317,17 @@ class MoePlan:
         """SM clock cycles after which a bounded wait inside the tensor-core kernels gives up (0 = default)."""
         self._call("nvmoe_plan_set_wait_limit", clock_cycles)
 
-    def debug_withhold_arrival(self, enabled: bool) -> None:
-        """Test aid: CTA 0 of the expert kernels leaves out one stage arrival, so that a bounded wait runs out."""
+    def debug_withhold_arrival(self, enabled: int) -> None:
+        """Test aid: CTA 0 (1 or True) or CTA 1 (2) of the expert kernels leaves out one stage arrival, so that a bounded wait
+        runs out."""
         self._call("nvmoe_plan_debug_withhold_arrival", int(enabled))
+
+    def debug_token_tile(self, stage: int, batch_width: int) -> tuple[int, bool]:
+        """Test aid: operand rows of the token tile that a call takes in stage 0 (gate/up) or 1 (down), and whether a CTA
+        pair works on it."""
+        rows, pair = ctypes.c_uint32(), ctypes.c_uint32()
+        self._call("nvmoe_plan_debug_token_tile", stage, batch_width, ctypes.byref(rows), ctypes.byref(pair))
+        return rows.value, bool(pair.value)
 
     def set_profiling(self, enabled: bool) -> None:
         self._call("nvmoe_plan_set_profiling", int(enabled))

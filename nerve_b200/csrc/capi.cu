@@ -640,7 +640,7 @@ int nvmoe_plan_set_wait_limit(nvmoe_plan* p, uint64_t clock_cycles) {
 
 int nvmoe_plan_debug_withhold_arrival(nvmoe_plan* p, int enabled) {
     if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
-    p->debug_flags = enabled ? (p->debug_flags | 1u) : (p->debug_flags & ~1u);
+    p->debug_flags = enabled == 2 ? 2u : enabled ? 1u : 0u;
     return NVMOE_OK;
 }
 
@@ -1708,6 +1708,15 @@ int nvmoe_plan_debug_counters(nvmoe_plan* p, uint64_t* out24) {
     NVMOE_CUDA(d, cudaStreamSynchronize(d->stream));
     NVMOE_CUDA(d, cudaMemcpy(out8, p->tile_list.as<uint32_t>() + 16, 96, cudaMemcpyDeviceToHost));
     NVMOE_CUDA(d, cudaMemcpy(out8 + 12, p->tile_list.as<uint32_t>() + tile_region_words(p) + 16 + 24, 96, cudaMemcpyDeviceToHost));
+    return NVMOE_OK;
+}
+
+int nvmoe_plan_debug_token_tile(const nvmoe_plan* p, uint32_t stage, uint32_t T, uint32_t* rows, uint32_t* pair) {
+    if (!p || !rows || !pair || stage > 1u || T == 0u) return NVMOE_ERR_INVALID_ARGUMENT;
+    NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
+    const TokenTile tile = token_tile(p, stage == 0u, T);
+    *rows = tile.rows;
+    *pair = tile.pair ? 1u : 0u;
     return NVMOE_OK;
 }
 

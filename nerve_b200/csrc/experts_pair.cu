@@ -194,7 +194,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             const uint8_t* scale_map = p.tmaps + (size_t)p.work.num_experts * kSources * kWeightMaps * 128u;
             const uint8_t* token_scale_map = p.act_tmap + (kTokenScaleMap - 1u) * 128u;
             uint32_t slot = 0u, empty_parity = 1u, stage_it = 0u;
-            bool alive = true, withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
+            bool alive = true, withhold = blockIdx.x < 2u && ((p.debug_flags >> blockIdx.x) & 1u) != 0u;
             Meta cur{}, nxt{};
             if (pair_id < tile_count) meta_of(pair_id, first_entry, cur);
             uint32_t pair_nxt = entry_of(pair_id + pairs);

@@ -287,8 +287,8 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
             Meta cur{}, nxt{};
             if (blockIdx.x < tile_count) meta_of(blockIdx.x, first_entry, cur);
             uint32_t pair_nxt = entry_of(blockIdx.x + gridDim.x);
-            // (debug) leave out the very first arrival of CTA 0: its consumer's bounded wait must then give up
-            bool withhold = (p.debug_flags & 1u) != 0u && blockIdx.x == 0u;
+            // (debug) leave out the very first arrival of CTA 0 or 1: its consumer's bounded wait must then give up
+            bool withhold = blockIdx.x < 2u && ((p.debug_flags >> blockIdx.x) & 1u) != 0u;
             for (uint32_t tile = blockIdx.x; tile < tile_count && alive; tile += gridDim.x) {
                 const uint32_t pair_nxt2 = entry_of(tile + 2u * gridDim.x);
                 if (tile + gridDim.x < tile_count) meta_of(tile + gridDim.x, pair_nxt, nxt);

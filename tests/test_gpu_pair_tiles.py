@@ -29,18 +29,25 @@ def with_native(case, cfg, seed):
 
 # K remainders of either stage (128 columns: one block; 384: a lone whole block after a pair; 576 = 4.5, 320 = 2.5, 704 = 5.5,
 # 448 = 3.5 blocks: a half block after whole pairs, and after a lone block), weight rows that end inside a row tile and after
-# the first of two (384, 576, 704), scale blocks of 32 and 128, a native FP8 resource; token counts per expert that end just
-# before and after a tile's widths (the always-selected resource of the second configuration has every token)
-@pytest.mark.parametrize("name,shape,tokens,native", [
-    ("gpt-oss-20b", (576, 320, 8), 400, 0), ("gpt-oss-20b", (704, 448, 4), 241, 0), ("gpt-oss-20b", (384, 128, 16), 499, 0),
-    ("gpt-oss-20b", (128, 192, 4), 97, 0), ("deepseek-v3", (512, 384, 16), 240, 0), ("deepseek-v3", (640, 256, 16), 481, 1),
-    ("deepseek-v3", (384, 640, 16), 193, 1)])
-def test_layer_matches_the_checker(device, name, shape, tokens, native):
+# the first of two (384, 576, 704), scale blocks of 32 and 128, a native FP8 resource; the rows a tile may have in either stage
+# (`widths`), whose experts start at any row and end at any row of a tile, so that the last tiles run with fewer columns (the
+# always-selected resource of the second configuration has every token)
+@pytest.mark.parametrize("name,shape,tokens,native,widths", [
+    ("gpt-oss-20b", (576, 320, 8), 400, 0, (128, 128)), ("gpt-oss-20b", (704, 448, 4), 241, 0, (64, 64)),
+    ("gpt-oss-20b", (384, 128, 16), 499, 0, (64, 64)), ("gpt-oss-20b", (128, 192, 4), 97, 0, (64, 64)),
+    ("deepseek-v3", (512, 384, 16), 240, 0, (128, 64)), ("deepseek-v3", (640, 256, 16), 481, 1, (128, 128)),
+    ("deepseek-v3", (384, 640, 16), 193, 1, (128, 64)),
+    ("gpt-oss-20b", (704, 448, 16), 940, 0, (240, 240)), ("gpt-oss-20b", (576, 320, 16), 700, 0, (192, 192)),
+    ("gpt-oss-20b", (1152, 704, 8), 470, 0, (240, 240)), ("gpt-oss-20b", (640, 512, 16), 770, 0, (240, 240)),
+    ("deepseek-v3", (640, 384, 16), 420, 1, (240, 240)), ("deepseek-v3", (768, 512, 16), 330, 0, (192, 192)),
+    ("deepseek-v3", (640, 384, 16), 330, 1, (192, 192))])
+def test_layer_matches_the_checker(device, name, shape, tokens, native, widths):
     cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], *shape), native_fp8_resources=native)
     assert tokens * cfg.total_k > 96 * cfg.total_experts  # what takes a call to these kernels
     case = synthetic.make_case(cfg, tokens, seed=17)
     tensors = with_native(case, cfg, 17)
     plan = MoePlan.for_config(device, cfg, tokens)
+    assert (plan.debug_token_tile(0, tokens), plan.debug_token_tile(1, tokens)) == ((widths[0], True), (widths[1], True))
     plan.set_expert_path(2)
     bank = ExpertBank.upload(device, *tensors)
     out = device.create_resident_buffer(tokens * cfg.hidden * 2)
@@ -56,13 +63,19 @@ def test_layer_matches_the_checker(device, name, shape, tokens, native):
     bank.destroy()
 
 
-# one matrix, every row count of interest: one row over each tile width, the widths, a row over the widest
-@pytest.mark.parametrize("rows,cols,tokens", [(256, 256, 97), (288, 448, 128), (160, 576, 129), (384, 704, 192), (256, 128, 193),
-                                              (320, 192, 240), (544, 320, 241), (1152, 640, 300)])
-def test_dense_linear_matches_the_checker(device, rows, cols, tokens):
+# one matrix: of few rows (64 tokens a tile, whole and ragged last tiles), and of rows that fill the pairs once or twice, where
+# tiles of 192 and 240 tokens are taken: the widths, a token less, a token more, two whole tiles
+@pytest.mark.parametrize("rows,cols,tokens,width", [
+    (256, 256, 97, 64), (288, 448, 128, 64), (160, 576, 129, 64), (384, 704, 192, 64), (256, 128, 193, 64), (320, 192, 240, 64),
+    (544, 320, 241, 64), (1152, 640, 300, 64),
+    (9888, 128, 191, 192), (9888, 192, 192, 192), (9888, 128, 193, 240), (9856, 192, 239, 240), (9888, 320, 240, 240),
+    (18912, 128, 300, 192), (18912, 128, 385, 240), (18912, 192, 433, 240), (18912, 192, 480, 240)])
+def test_dense_linear_matches_the_checker(device, rows, cols, tokens, width):
     rng = np.random.default_rng(rows + cols + tokens)
-    cfg = synthetic.MoeConfig("pairs", 256, 256, 8, 2, act_block=32)
-    plan = MoePlan.for_config(device, cfg, 320)
+    plan = MoePlan.for_config(device, synthetic.MoeConfig("pairs", 256, 256, 8, 2, act_block=32), 480)
+    shape = MoePlan.for_config(device, synthetic.MoeConfig("linear", rows, cols, 1, 1, act_block=32), tokens)  # its down stage
+    assert shape.debug_token_tile(1, tokens) == (width, True)
+    shape.destroy()
     plan.set_expert_path(2)
     x = synthetic.f32_to_bf16(rng.standard_normal((tokens, cols)).astype(np.float32))
     w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(118, 128, (rows, cols // 32), dtype=np.uint8)
@@ -73,8 +86,10 @@ def test_dense_linear_matches_the_checker(device, rows, cols, tokens):
     plan.destroy()
 
 
-def test_a_wait_that_expires_is_reported(device):
-    """An announcement that one CTA of a pair leaves out: both wind down, the call reports it, the next call is whole."""
+@pytest.mark.parametrize("cta", [0, 1])
+def test_a_wait_that_expires_is_reported(device, cta):
+    """Copies that one CTA of a pair leaves out, the announcement of both CTAs' (0) or only its own (1): both wind down, the call
+    reports it, the next call is whole."""
     cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 576, 320, 8)
     tokens = 400
     case = synthetic.make_case(cfg, tokens, seed=18)
@@ -87,7 +102,7 @@ def test_a_wait_that_expires_is_reported(device):
     assert plan.status() == 0
     before = out.read(np.uint16).copy()
     plan.set_wait_limit(2_000_000)  # about a millisecond
-    plan.debug_withhold_arrival(True)
+    plan.debug_withhold_arrival(1 + cta)
     plan.layer(tokens, bank, hidden, out, router_weights=rw)
     device.synchronize(timeout_ns=20_000_000_000)
     assert plan.status() & 8

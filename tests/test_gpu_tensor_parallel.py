@@ -25,9 +25,11 @@ def device():
 
 @pytest.mark.parametrize("path", PATHS)
 @pytest.mark.parametrize("participants", [1, 2, 4])
-def test_partitioned_intermediate_reproduces_the_layer(device, path, participants):
-    cfg = synthetic.MoeConfig("tp", 256, 512, 8, 2, router_kind=synthetic.ROUTER_TOPK_SOFTMAX, act_block=128, swiglu_limit=7.0)
-    tokens, K, H = 70, cfg.total_k, cfg.hidden
+# 18 tokens an expert (one CTA a tile), 125 (CTA pairs, the last of the 128-row tiles without a partner)
+@pytest.mark.parametrize("hidden_size,tokens,pairs", [(256, 70, False), (640, 500, True)])
+def test_partitioned_intermediate_reproduces_the_layer(device, path, participants, hidden_size, tokens, pairs):
+    cfg = synthetic.MoeConfig("tp", hidden_size, 512, 8, 2, router_kind=synthetic.ROUTER_TOPK_SOFTMAX, act_block=128, swiglu_limit=7.0)
+    K, H = cfg.total_k, cfg.hidden
     case = synthetic.make_case(cfg, tokens, seed=13)
     want = oracle_layer(case, tier=1)
     # one device, the whole layer: routes for everyone and the result to compare with
@@ -48,6 +50,7 @@ def test_partitioned_intermediate_reproduces_the_layer(device, path, participant
         part = TensorParallelParticipant(device, cfg, tokens, p, participants,
                                          lambda e: (case.w1[e], case.s1[e], case.w3[e], case.s3[e], case.w2[e], case.s2[e]), path)
         plane = ResidentBuffer.wrap(device, planes.device_address() + p * plane_bytes, plane_bytes)
+        assert part.plan.debug_token_tile(1, tokens)[1] == pairs
         part.partial_outputs(tokens, hidden, routes, plane)
         assert part.plan.status() == 0
         part.plan.destroy()
