@@ -557,17 +557,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
 
     // ---- teardown: neither CTA leaves while the other may still reach into its shared memory -------------------
     __syncthreads();
-    if (*abort_flag && threadIdx.x == 0u) raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
+    const bool gave_up = threadIdx.x == 0u && *abort_flag != 0u;
+    if (gave_up) raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
     __syncwarp();
     cluster_sync();
-    // A CTA that did not give up has seen every copy, store and commit that reaches its shared memory (each of its tiles was
-    // finished); one that did may have some on their way that no role waited for, its own or, until the barrier above, the
-    // other CTA's.
-    if (*abort_flag && threadIdx.x == 0u) winddown_pause();
     if (warp == kPairMmaWarp) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, kPairTmemColumns);
     }
+    // A CTA that did not give up has seen every copy, store and commit that reaches its shared memory (each of its tiles was
+    // finished); one that did may have some on their way that no role waited for, its own or, until the barrier above, the
+    // other CTA's.
+    if (gave_up) winddown_pause();
 }
 
 template <bool GATE_UP>

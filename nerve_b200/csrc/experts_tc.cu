@@ -842,13 +842,13 @@ __global__ void __launch_bounds__((Config<GATE_UP, N_TILE, USE_TMA, ROW_PAIR>::k
 
     // ---- teardown -------------------------------------------------------------------------------
     __syncthreads();
-    if (*abort_flag && threadIdx.x == 0u) {
-        raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
-        winddown_pause();  // copies that no role waited for any more may still be landing
-    }
     if (warp == 4u) {
         tc_fence_after();
         tmem_dealloc(tmem_base, C::kTmemColumns);
+    }
+    if (threadIdx.x == 0u && *abort_flag) {
+        raise_status(p.status, NVMOE_STATUS_WAIT_EXPIRED);
+        winddown_pause();  // copies that no role waited for any more may still be landing
     }
     // latest exit over all CTAs (the timer only grows, so the last launch wins)
     if (TRACE && threadIdx.x == 0u) atomicMax(reinterpret_cast<unsigned long long*>(trace + 11), (unsigned long long)global_timer_ns());
