@@ -62,9 +62,8 @@ struct Config {
     // matrix mx of a stage = weight tensor source_of(mx), rows shifted by row_shift(mx)
     static constexpr uint32_t source_of(uint32_t mx) { return GATE_UP ? mx : 0u; }
     static constexpr uint32_t row_shift(uint32_t mx) { return ROW_PAIR ? mx * kBlockM : 0u; }
-    // cp.async producers: one warp sustains only about one copy instruction every 60-130 cycles, so the
-    // copies of a stage are spread over eight warps (with TMA for the weights: token rows on the first
-    // four, scales on the other four)
+    // Without tensor maps everything comes by cp.async: one warp sustains only about one copy instruction every 60-130
+    // cycles, so the copies of a stage are spread over eight warps.
     // With TMA one warp is left with the token scales (a second idles, so that the ones after it keep warp % 4), and the warps
     // this frees become epilogue warps: the epilogue (activation, rounding, re-quantisation: a couple of hundred instructions
     // per value) is what large token tiles wait for, and a warp only issues one instruction at a time. Epilogue warps come in
@@ -120,8 +119,8 @@ struct Config {
     static constexpr uint32_t kAccColumns = kMatrices * N_TILE;
     static constexpr uint32_t kAccStages = 2u;
     static constexpr uint32_t kScaleColumns = 4u * (kMatrices + 1u);
-    // Two accumulators of 128 tokens and two matrices would be all of tensor memory, with no columns left for the
-    // scales. They share 16 columns instead: the last tokens' second matrix of the first accumulator lies where the
+    // Two accumulators of 128 tokens and two matrices (the widest tile of shapes without tensor maps; with them so many tokens
+    // run by CTA pairs) would be all of tensor memory, with no columns left for the scales. They share 16 columns instead: the last tokens' second matrix of the first accumulator lies where the
     // second accumulator keeps the first tokens' first matrix. The epilogue reads that chunk before all others and
     // says so (acc_head), and the MMAs of the next tile wait for it: about a microsecond per tile, during which the
     // ring fills. Wider tiles fetch fewer weight bytes per token, and the MMA itself is bound by its operand reads
@@ -1013,14 +1012,14 @@ void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
 
 // Whether a down launch takes two row tiles at a time: always with wide token tiles, and with narrow ones (TMA form)
 // when that leaves an SM several tiles to go through, counted as if every expert were selected (what routing, a partition
-// or absent experts leave of them is not known here). A stage of a row pair is one K block of two weight boxes, one
-// token box and two scale copies, where a single row tile needs six copies for the same bytes (0.42 against 0.49 us per
-// stage); single row tiles spread over the SMs in finer steps, which 32-token tiles gain from while there are few rounds.
-// Layer of intermediate 1536, single rows / row pairs, us, by rounds: 32-token tiles 0.65 54.9 / 57.6, 1.95 77.7 / 78.6,
-// 2.6 92.6 / 93.1, 3.5 108.1 / 108.2, 5.2 155.9 / 154.5, 6.05 158.5 / 151.9, 10.4 261.3 / 249.2; 16-token tiles 0.65 55.7 /
-// 51.6, 2.6 87.4 / 83.3, 6.05 150.6 / 142.2, 24 469.6 / 442.3. Partitioned calls of 128 experts with 16 and 32 of them
-// owned (1.3 and 2.6 rounds of their own): 115.3 / 115.6 and 136.4 / 132.4 with 32-token tiles, 87.3 / 87.7 and 105.1 /
-// 104.2 with 16.
+// or absent experts leave of them is not known here). A stage of a row pair is one K block: one box of 256 weight rows, one token
+// box, two scale copies. One of a single row tile is two K blocks: a weight box, a token box and a scale copy, for the
+// same weight bytes and twice the token rows. Single row tiles spread over the SMs in finer steps, which 32-token tiles gain
+// from while there are few rounds. Layer of intermediate 1536, single rows / row pairs, us, by rounds: 32-token tiles 0.65 51.3 /
+// 52.2, 1.3 62.9 / 67.4, 1.95 81.2 / 85.0, 2.6 100.4 / 101.4, 3.5 113.4 / 113.6, 3.9 124.6 / 126.0, 5.2 143.4 / 142.6, 6.05 167.8 / 165.9,
+// 7.8 191.9 / 188.8, 10.4 234.1 / 228.7, 24 519 / 506; 16-token tiles 0.65 51.8 / 48.9, 1.3 60.7 / 58.3, 2.6 84.3 / 80.1, 5.2 129.9 / 126.5,
+// 6.05 147.5 / 142.7, 10.4 212.2 / 207.1, 24 436 / 425: the line lies where 32-token tiles have it; 16-token tiles would gain
+// below it too.
 bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) {
     if (n_tile >= kRowPairTokens) return true;
     if (!tma) return false;
@@ -1102,10 +1101,17 @@ TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t
     if (per_expert <= kPairsFrom) return {96u, false};
     const uint32_t row_tiles = gate_up ? (out_rows + kBlockM - 1u) / kBlockM : (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM);
     const uint64_t sms = (uint64_t)sm_count();
-    // Beyond that CTA pairs (one CTA of 128 columns / pairs: 4096 tokens of 32 experts of 2880 x 2880 672 / 589 us a layer,
-    // 8192 of 128 1640 / 1575, 16384 of 256 of 7168 x 2048 9960 / 9330). An expert takes several tiles, and the wide ones are
-    // the cheapest per token unless a wave of the pairs goes half empty with them: the fewest rounds x stage time wins, the
-    // time of a stage being that of its shared-memory traffic, 256 + columns.
+    // Beyond that CTA pairs. One CTA with tiles of 96 / pairs, us a layer, by tokens an expert: 32 experts of 2880 x 2880, 104
+    // 205.7 / 183.8, 128 223.4 / 219.7, 192 290.4 / 264.7, 240 323.4 / 283.1; 128 of them, 104 731 / 711, 128 867 / 835, 192 1128 /
+    // 1031; a dense block of 7168 x 2048, 100 78.3 / 58.6, 240 84.9 / 66.5. In layers that take one round of the SMs either way
+    // the two are within a few percent: 16 experts of 768 x 512, 104 55.5 / 55.6, 128 54.0 / 55.3, 192 60.8 / 60.3, 240 61.9 / 66.0;
+    // 8 of 1024 x 1024, 128 47.2 / 47.3, 192 60.3 / 61.2. Dense blocks would gain below the line too (96 rows 77.7 by one CTA).
+    // An expert takes several tiles, and the fewest rounds of the pairs x stage time wins, the time of a stage being that of its
+    // shared-memory traffic, 256 + columns (gate/up of 4096 tokens of 32 experts, all tiles of one width, ns a stage: 64 467, 128
+    // 581, 192 672, 240 761). The count takes every expert at the mean load and its last tile at full width. Loads differ, so that
+    // it misses tiles of a width that the mean just fills. Gate/up as chosen / with 240 throughout, us: 4096 tokens of 32 experts (192)
+    // 267 / 247, 8192 of 128 (128) 748 / 567, 16384 of 256 of 7168 x 2048 (192) 3580 / 3230. Where the tiles fit one round the choice is
+    // right: dense block of 777 rows as chosen 95.7, with 192 throughout 110, with 240 139.
     if (tma) {
         const uint32_t rows[4] = {kPairTokens, 192u, 128u, 64u};
         TokenTile best{kPairTokens, true};
