@@ -404,14 +404,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
         const bool quantise = GATE_UP && p.q_out != nullptr;             // host: only with scale blocks of 32 or 128 rows
         const bool store_rows = !GATE_UP || p.intermediates != nullptr;
         uint32_t acc_it = 0u, sends = 0u, receipts = 0u, set_it = 0u;
-        // A wait of the exchange gave up (the call reports it): this warp exchanges nothing more. Another arrival on a barrier whose
-        // bytes are outstanding would be one more than it counts.
-        bool lost = false;
         // this warp's place in the exchange: its own (read) and the same place of the other CTA's warp (written)
         const uint4* inbox = reinterpret_cast<const uint4*>(smem + kPairExchangeRegion + warp * 1024u) + lane;
         const uint32_t outbox = map_shared(smem_u32(inbox), rank ^ 1u);
         const uint32_t peer_sent = map_shared(smem_u32(&bars->sent[warp]), rank ^ 1u);
         const uint32_t peer_taken = map_shared(smem_u32(&bars->taken[warp]), rank ^ 1u);
+        if (GATE_UP && lane == 0u) mbar_arrive_expect_tx(&bars->sent[warp], 1024u);  // the first chunk's
         for (uint32_t tile = pair_id; tile < tile_count; tile += pairs, acc_it++) {
             const uint32_t acc = acc_it & 1u;
             // (one warp polls, the others sleep on a hardware barrier; every warp reaches it in every round)
@@ -434,13 +432,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             // the other CTA's i-th chunk, to its shared memory
             auto send = [&](uint32_t i) {
                 const uint32_t c = rank == 0u ? half + i : i;
-                if (i >= half || c >= chunks || lost) return;
+                if (i >= half || c >= chunks) return;
                 uint32_t s[16];
                 tmem_ld16(lane_addr + 16u * c, s);
-                // (the place is free again once the other warp has taken what was sent last)
-                lost = !mbar_wait_cluster_warp(&bars->taken[warp], (sends & 1u) ^ 1u, abort_flag, wait_limit);
+                // (the place is free again once the other warp has taken what was sent last; a wait that gives up leaves rubbish
+                // there, which the call reports: bytes that nobody announced keep the other warp's next wait from passing, no more)
+                mbar_wait_cluster_warp(&bars->taken[warp], (sends & 1u) ^ 1u, abort_flag, wait_limit);
                 tmem_ld_wait();
-                if (lost) return;
                 uint32_t v[8];
 #pragma unroll
                 for (uint32_t j = 0; j < 8u; j++) v[j] = bf16x2_bits(__uint_as_float(s[2u * j]), __uint_as_float(s[2u * j + 1u]));
@@ -455,16 +453,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                 uint32_t d[16], other[8];
                 if (mine) tmem_ld16(lane_addr + 16u * c, d);
                 if (GATE_UP && mine) {
-                    if (!lost) {
-                        if (lane == 0u) mbar_arrive_expect_tx(&bars->sent[warp], 1024u);
-                        lost = !mbar_wait_cluster_warp(&bars->sent[warp], receipts & 1u, abort_flag, wait_limit);
-                    }
+                    const bool here = mbar_wait_cluster_warp(&bars->sent[warp], receipts & 1u, abort_flag, wait_limit);
                     const uint4 low = inbox[0], high = inbox[32];
                     other[0] = low.x, other[1] = low.y, other[2] = low.z, other[3] = low.w;
                     other[4] = high.x, other[5] = high.y, other[6] = high.z, other[7] = high.w;
                     __syncwarp();
-                    if (lane == 0u && !lost) mbar_arrive_cluster(peer_taken);
-                    receipts++;
+                    // (the announcement of a chunk only follows the arrival of the last: one more, on a barrier whose bytes are
+                    // outstanding, would be one more than it counts)
+                    if (here) {
+                        if (lane == 0u) {
+                            mbar_arrive_expect_tx(&bars->sent[warp], 1024u);
+                            mbar_arrive_cluster(peer_taken);
+                        }
+                        receipts++;
+                    }
                 }
                 tmem_ld_wait();
                 if (GATE_UP) send(i + kPairEpilogueGroups);  // on its way while this chunk is worked on
