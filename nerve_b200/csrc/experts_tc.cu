@@ -1106,15 +1106,19 @@ TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t
     // 1031; a dense block of 7168 x 2048, 100 78.3 / 58.6, 240 84.9 / 66.5. In layers that take one round of the SMs either way
     // the two are within a few percent: 16 experts of 768 x 512, 104 55.5 / 55.6, 128 54.0 / 55.3, 192 60.8 / 60.3, 240 61.9 / 66.0;
     // 8 of 1024 x 1024, 128 47.2 / 47.3, 192 60.3 / 61.2. Dense blocks would gain below the line too (96 rows 77.7 by one CTA).
-    // An expert takes several tiles, and the fewest rounds of the pairs x stage time wins, the time of a stage being that of its
-    // shared-memory traffic, 256 + columns (gate/up of 4096 tokens of 32 experts, all tiles of one width, ns a stage: 64 467, 128
-    // 581, 192 672, 240 761). The count takes every expert at the mean load and its last tile at full width. Loads differ, so that
-    // it misses tiles of a width that the mean just fills. Gate/up as chosen / with 240 throughout, us: 4096 tokens of 32 experts (192)
-    // 267 / 247, 8192 of 128 (128) 748 / 567, 16384 of 256 of 7168 x 2048 (192) 3580 / 3230. Where the tiles fit one round the choice is
-    // right: dense block of 777 rows as chosen 95.7, with 192 throughout 110, with 240 139.
+    // An expert takes several tiles. Where they are more than two rounds of the pairs, the widest: a stage takes 350 ns and 1.7 a
+    // column (gate/up of 4096 tokens of 32 experts, all tiles of one width, ns a stage: 64 467, 128 581, 192 672, 240 761), a tile
+    // with fewer tokens runs with fewer columns, and the loads of several experts differ, so that narrower tiles fit none of them
+    // better: layers with the width that the count below chose / 240, 4096 tokens of 32 experts (192) 557.6 / 534.0 us, 8192 of 128
+    // (128) 1439 / 1274, 16384 of 256 of 7168 x 2048 (192) 8606 / 8352. (An expert's last tile counts as half full.)
+    // In fewer rounds, or with one expert, whose load is the call's, the fewest rounds x stage time wins, as 256 + columns, with
+    // every expert at the mean load and its last tile at full width: dense block of 777 rows (128) 95.7 us, with 192 throughout
+    // 110, with 240 139.
     if (tma) {
         const uint32_t rows[4] = {kPairTokens, 192u, 128u, 64u};
         TokenTile best{kPairTokens, true};
+        const uint64_t half_tiles = (uint64_t)num_experts * (2ull * per_expert + kPairTokens) / kPairTokens;
+        if (num_experts > 1u && (half_tiles + 1u) / 2u * row_tiles > sms) return best;
         uint64_t best_cost = ~0ull;
         for (uint32_t i = 0; i < 4u; i++) {
             const uint64_t tiles = (uint64_t)num_experts * ((per_expert + rows[i] - 1u) / rows[i]) * row_tiles;
