@@ -145,6 +145,8 @@ struct nvmoe_plan {
     cudaEvent_t ev[kStageCount + 1] = {};
     cudaEvent_t kernel_ev[2][2] = {};  // [gate_up, down][begin, end] around the expert kernel alone
     bool events_valid = false;
+    bool clocked = false;        // the last layer call's time is in `clock`, else between the first and the last event
+    DeviceArray clock;
     bool profile_stages = false;
     nvmoe_work_report report{};
     uint32_t launches = 0;
@@ -567,6 +569,7 @@ static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool den
             if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);  // `maps` is a stack buffer
         }
     }
+    want(p->clock, sizeof(CallClock));
     if (err == cudaSuccess) err = cudaMemsetAsync(p->status.ptr, 0, 256, d->stream);
     for (int i = 0; i <= kStageCount && err == cudaSuccess; i++) err = cudaEventCreate(&p->ev[i]);
     for (int i = 0; i < 4 && err == cudaSuccess; i++) err = cudaEventCreate(&p->kernel_ev[i / 2][i % 2]);
@@ -598,7 +601,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
         for (auto& es : stage_sets) es->release();
     DeviceArray* all[] = {&p->status, &p->grouped[0], &p->grouped[1], &p->offsets[0],
                           &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->iq,
-                          &p->i_scales, &p->tile_list, &p->ep_source, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
+                          &p->i_scales, &p->tile_list, &p->ep_source, &p->clock, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
                           &p->controls, &p->hidden_dev, &p->output_dev};
     for (DeviceArray* a : all) a->release();
@@ -652,8 +655,8 @@ int nvmoe_plan_set_profiling(nvmoe_plan* p, int enabled) {
 
 // ---- node-granular operators -----------------------------------------------------------------
 
-int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits,
-                        const nvmoe_buffer* router_weights, const nvmoe_buffer* router_bias) {
+static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
+                         const nvmoe_buffer* router_bias, CallClock* clock) {
     if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
     NVMOE_TRY(check_tokens(p, T));
     const nvmoe_geometry& g = p->g;
@@ -664,9 +667,14 @@ int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, n
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     launch_router_linear((const uint16_t*)hidden->ptr, (const uint16_t*)router_weights->ptr,
                          router_bias ? (const uint16_t*)router_bias->ptr : nullptr, (uint32_t*)logits->ptr, T,
-                         g.hidden_size, g.routed_experts, p->device->stream);
+                         g.hidden_size, g.routed_experts, clock, p->device->stream);
     p->launches++;
     return post_launch(p, "router projection");
+}
+
+int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits,
+                        const nvmoe_buffer* router_weights, const nvmoe_buffer* router_bias) {
+    return router_linear(p, T, hidden, logits, router_weights, router_bias, nullptr);
 }
 
 // checks the router's buffers and fills its launch block
@@ -1143,7 +1151,7 @@ int nvmoe_reduce(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* expert_outputs, 
     NVMOE_TRY(check_buffer(p, output, (size_t)T * g.hidden_size * 2u, "output"));
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     launch_reduce((const uint16_t*)expert_outputs->ptr, (uint16_t*)output->ptr, T, p->K, g.hidden_size, g.reduce_scale,
-                  nullptr, p->device->stream);
+                  nullptr, nullptr, p->device->stream);
     p->launches++;
     return post_launch(p, "reduce");
 }
@@ -1458,8 +1466,12 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     cudaStream_t st = d->stream;
     const uint32_t launches_before = p->launches;
     const bool prof = p->profile_stages;
+    // the time of a call that begins with the projection and ends with the combine is noted by these kernels, of another or
+    // of stages by events
+    p->clocked = !prof && a->router_weights && !a->routes_in && !a->expert_outputs;
+    CallClock* clock = p->clocked ? p->clock.as<CallClock>() : nullptr;
     auto mark = [&](int i) {
-        if (prof || i == 0 || i == kStageCount) cudaEventRecord(p->ev[i], st);
+        if (prof || (clock == nullptr && (i == 0 || i == kStageCount))) cudaEventRecord(p->ev[i], st);
     };
 
     nvmoe_buffer logits_view{d, p->logits.ptr, p->logits.bytes};
@@ -1474,7 +1486,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
 
     mark(kStageLinear);
     if (a->router_weights && !a->routes_in)
-        NVMOE_TRY(nvmoe_router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias));
+        NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, clock));
     mark(kStageRoute);
     // (with stage profiling on, the router keeps a launch and a time of its own)
     RouterLaunch router{};
@@ -1579,7 +1591,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     mark(kStageReduce);
     if (!a->expert_outputs) {
         launch_reduce((const uint16_t*)outs.ptr, (uint16_t*)a->output->ptr, T, p->K, g.hidden_size, g.reduce_scale,
-                      p->position[1].as<uint32_t>(), st);
+                      p->position[1].as<uint32_t>(), clock, st);
         p->launches++;
         NVMOE_TRY(post_launch(p, "reduce"));
     }
@@ -1744,7 +1756,13 @@ int nvmoe_plan_last_report(nvmoe_plan* p, nvmoe_work_report* report) {
     if (!p->events_valid) return fail(d, NVMOE_ERR_INVALID_ARGUMENT, "no layer call has run on this plan");
     NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
     NVMOE_CUDA(d, cudaStreamSynchronize(d->stream));
-    NVMOE_CUDA(d, cudaEventElapsedTime(&p->report.total_ms, p->ev[0], p->ev[kStageCount]));
+    if (p->clocked) {
+        CallClock clock;
+        NVMOE_CUDA(d, cudaMemcpy(&clock, p->clock.ptr, sizeof clock, cudaMemcpyDeviceToHost));
+        p->report.total_ms = (float)((double)(clock.end - clock.begin) * 1e-6);
+    } else {
+        NVMOE_CUDA(d, cudaEventElapsedTime(&p->report.total_ms, p->ev[0], p->ev[kStageCount]));
+    }
     for (int i = 0; i < kStageCount; i++) {
         p->report.stage_ms[i] = 0.0f;
         if (p->profile_stages) cudaEventElapsedTime(&p->report.stage_ms[i], p->ev[i], p->ev[i + 1]);

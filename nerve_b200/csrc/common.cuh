@@ -85,6 +85,26 @@ struct GroupedWork {
     uint32_t num_experts;
 };
 
+// When a layer call ran, by the device's clock in ns: its first kernel notes when it starts, every block of its last one when it
+// ends. Events around the call would do, but stand between its kernels and those of the calls before and after it, which then
+// do not start while the kernel ahead still runs: tiny layer of 64 tokens 32.8 us, 25.2 without them. Null: not noted.
+struct CallClock {
+    unsigned long long begin, end;
+};
+__device__ __forceinline__ unsigned long long device_clock_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void note_begin(CallClock* clock) {
+    if (clock == nullptr || (blockIdx.x | blockIdx.y | threadIdx.x) != 0u) return;
+    clock->begin = device_clock_ns();
+    clock->end = 0u;
+}
+__device__ __forceinline__ void note_end(CallClock* clock) {
+    if (clock != nullptr && threadIdx.x == 0u) atomicMax(&clock->end, device_clock_ns());
+}
+
 __device__ __forceinline__ void raise_status(uint32_t* status, uint32_t bit) {
     if (status) atomicOr(status, bit);
 }
@@ -121,7 +141,7 @@ void configure_router_kernels();
 void launch_router(const RouterLaunch& p, cudaStream_t stream);
 bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selections, no groups: route_token covers it
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
-                          uint32_t tokens, uint32_t hidden, uint32_t outputs, cudaStream_t stream);
+                          uint32_t tokens, uint32_t hidden, uint32_t outputs, CallClock* clock, cudaStream_t stream);
 
 struct SortScratch {  // schedule.cu: scratch of the counting sort, sized for max_tokens
     uint32_t* block_hist;      // [blocks][buckets]
@@ -294,6 +314,6 @@ cudaError_t launch_mma_rate_probe(uint32_t n_tile, uint32_t groups, uint32_t cta
 // reduce.cu: moe_reduce_batch1_bf16. `computed` (optional, [tokens * K]) marks with 0xffffffff the routes
 // whose rows were never written: they count as zeros, so the rows need no clearing beforehand.
 void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t tokens, uint32_t K,
-                   uint32_t hidden, float routed_scale, const uint32_t* computed, cudaStream_t stream);
+                   uint32_t hidden, float routed_scale, const uint32_t* computed, CallClock* clock, cudaStream_t stream);
 
 }  // namespace nvmoe

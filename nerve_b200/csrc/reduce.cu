@@ -14,7 +14,7 @@ namespace {
 __global__ void __launch_bounds__(256) reduce_kernel(const uint32_t* __restrict__ expert_outputs,
                                                     uint32_t* __restrict__ output, uint32_t tokens, uint32_t K,
                                                     uint32_t hidden_words, float routed_scale,
-                                                    const uint32_t* __restrict__ computed) {
+                                                    const uint32_t* __restrict__ computed, CallClock* clock) {
     grid_dependency_sync();
     const uint64_t total = (uint64_t)tokens * hidden_words;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const uint32_t* __restrict_
         }
         output[i] = pack_bf16x2(__fmul_rn(lo, routed_scale), __fmul_rn(hi, routed_scale));
     }
+    note_end(clock);
 }
 
 // The same sum over 16-byte pieces (eight columns a thread) for rows that allow it: the order of the adds
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const uint32_t* __restrict_
 template <uint32_t DEPTH>
 __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict__ expert_outputs, uint4* __restrict__ output,
                                                         uint32_t tokens, uint32_t K, uint32_t hidden_vecs, float routed_scale,
-                                                        const uint32_t* __restrict__ computed) {
+                                                        const uint32_t* __restrict__ computed, CallClock* clock) {
     grid_dependency_sync();
     const uint64_t total = (uint64_t)tokens * hidden_vecs;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict
         out.w = pack_bf16x2(__fmul_rn(acc[6], routed_scale), __fmul_rn(acc[7], routed_scale));
         output[i] = out;
     }
+    note_end(clock);
 }
 
 // The combine of an expert-parallel step read straight from the rows that came back from the owners:
@@ -174,7 +176,7 @@ bool launch_reduce_gather(const uint16_t* rows, const uint32_t* gather, uint16_t
 }
 
 void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t tokens, uint32_t K, uint32_t hidden,
-                   float routed_scale, const uint32_t* computed, cudaStream_t stream) {
+                   float routed_scale, const uint32_t* computed, CallClock* clock, cudaStream_t stream) {
     if (tokens == 0u) return;
     if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(expert_outputs) | reinterpret_cast<uintptr_t>(output)) & 15u) == 0u) {
         const uint64_t vecs = (uint64_t)tokens * (hidden / 8u);
@@ -182,7 +184,7 @@ void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t to
         if (vec_blocks > 148u * 16u) vec_blocks = 148u * 16u;
         launch_chained(K == 9u ? reduce_vec_kernel<9u> : reduce_vec_kernel<4u>, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
                        reinterpret_cast<const uint4*>(expert_outputs), reinterpret_cast<uint4*>(output), tokens, K, hidden / 8u,
-                       routed_scale, computed);
+                       routed_scale, computed, clock);
         return;
     }
     const uint64_t total = (uint64_t)tokens * (hidden / 2u);
@@ -190,7 +192,7 @@ void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t to
     if (blocks > 148u * 8u) blocks = 148u * 8u;
     launch_chained(reduce_kernel, dim3((uint32_t)blocks), dim3(256), 0, stream,
                    reinterpret_cast<const uint32_t*>(expert_outputs), reinterpret_cast<uint32_t*>(output), tokens, K,
-                   hidden / 2u, routed_scale, computed);
+                   hidden / 2u, routed_scale, computed, clock);
 }
 
 }  // namespace nvmoe
