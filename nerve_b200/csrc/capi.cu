@@ -130,7 +130,7 @@ struct nvmoe_plan {
     DeviceArray status, grouped[2], offsets[2], block_hist, bucket_totals;
     std::vector<std::unique_ptr<ExpertSet>> sets[2];  // [gate/up, down], least recently used replaced
     uint64_t use_clock = 0;
-    DeviceArray xq, x_scales, iq, i_scales, tile_list, ep_source;
+    DeviceArray xq, x_scales, iq, i_scales, tile_list, ep_source, layer_sync;
     // tensor path: expert-grouped quantised activations of the two stages (row = position in grouped[stage]),
     // where each route landed, and the tensor maps of the operands for the token tile sizes
     DeviceArray grouped_q[2], grouped_e8m0[2], position[2], act_maps;
@@ -570,6 +570,7 @@ static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool den
         }
     }
     want(p->clock, sizeof(CallClock));
+    want(p->layer_sync, sizeof(uint32_t) * (p->experts + 1u));
     if (err == cudaSuccess) err = cudaMemsetAsync(p->status.ptr, 0, 256, d->stream);
     for (int i = 0; i <= kStageCount && err == cudaSuccess; i++) err = cudaEventCreate(&p->ev[i]);
     for (int i = 0; i < 4 && err == cudaSuccess; i++) err = cudaEventCreate(&p->kernel_ev[i / 2][i % 2]);
@@ -601,7 +602,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
         for (auto& es : stage_sets) es->release();
     DeviceArray* all[] = {&p->status, &p->grouped[0], &p->grouped[1], &p->offsets[0],
                           &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->iq,
-                          &p->i_scales, &p->tile_list, &p->ep_source, &p->clock, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
+                          &p->i_scales, &p->tile_list, &p->ep_source, &p->layer_sync, &p->clock, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
                           &p->controls, &p->hidden_dev, &p->output_dev};
     for (DeviceArray* a : all) a->release();
@@ -862,6 +863,13 @@ static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* a
     return post_launch(p, gate_up ? "gate/up expert tables" : "down expert tables");
 }
 
+// Whether the expert stages of a layer call of T tokens may run in one launch: one CTA a tile, the same tile and tensor maps in both.
+static bool layer_in_one_launch(const nvmoe_plan* p, uint32_t T) {
+    const TokenTile gate = token_tile(p, true, T), down = token_tile(p, false, T);
+    return p->tma[0] && p->tma[1] && !gate.pair && !down.pair && gate.rows == down.rows && p->experts <= kLayerExperts &&
+           tc_layer_in_one_launch(T, p->K, p->experts, p->g.intermediate_size);
+}
+
 // Groups the routes of one expert stage by expert (and, for the tensor path, records where each route
 // landed and lists the (expert, token tile) pairs).
 static int schedule_stage(nvmoe_plan* p, bool gate_up, ExpertSet* es, uint32_t T, const uint32_t* routes,
@@ -930,18 +938,13 @@ struct ExpertCall {
     uint32_t* status = nullptr;     // the word that the caller's plan reads (null: this plan's own)
 };
 
-// shared tail of the two gate/up entry points and of down
-static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
+// The launch parameters of one expert stage.
+static int expert_launch(nvmoe_plan* p, const ExpertCall& c, ExpertSet* es, bool tensor, ExpertLaunch* out) {
     const nvmoe_geometry& g = p->g;
     cudaStream_t st = p->device->stream;
     const bool gate_up = c.gate_up;
     const int set = gate_up ? 0 : 1;
     const uint32_t T = c.T;
-    const bool tensor = c.allow_tensor_path && use_tensor_path(p);
-    ExpertSet* es = c.prepared;
-    if (!es) NVMOE_TRY(prepare_expert_set(p, gate_up, c.addresses, c.slots, tensor, &es));
-    if (!c.scheduled) NVMOE_TRY(schedule_stage(p, gate_up, es, T, c.routes, c.intermediates, c.control, tensor));
-    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor, false, false));
     ExpertLaunch el{};
     el.work = GroupedWork{p->grouped[set].as<uint32_t>(), p->offsets[set].as<uint32_t>(), es->ptrs.as<ExpertPtrs>(), p->experts};
     if (tensor) {
@@ -988,6 +991,24 @@ static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
             el.intermediates = nullptr;  // the down stage reads the codes only
         }
     }
+    *out = el;
+    return NVMOE_OK;
+}
+
+// shared tail of the two gate/up entry points and of down
+static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
+    const nvmoe_geometry& g = p->g;
+    cudaStream_t st = p->device->stream;
+    const bool gate_up = c.gate_up;
+    const int set = gate_up ? 0 : 1;
+    const uint32_t T = c.T;
+    const bool tensor = c.allow_tensor_path && use_tensor_path(p);
+    ExpertSet* es = c.prepared;
+    if (!es) NVMOE_TRY(prepare_expert_set(p, gate_up, c.addresses, c.slots, tensor, &es));
+    if (!c.scheduled) NVMOE_TRY(schedule_stage(p, gate_up, es, T, c.routes, c.intermediates, c.control, tensor));
+    if (c.source) NVMOE_TRY(quantise_operands(p, gate_up, T, c.source, tensor, false, false));
+    ExpertLaunch el{};
+    NVMOE_TRY(expert_launch(p, c, es, tensor, &el));
     if (p->profile_stages) cudaEventRecord(p->kernel_ev[set][0], st);
     if (tensor) {
         if (gate_up) {
@@ -1506,11 +1527,18 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     // gate/up epilogue quantises its own output for the down stage
     const bool fused_quantise = tensor && (g.act_block == 32u || g.act_block == 128u) &&
                                 (reinterpret_cast<uintptr_t>(a->hidden->ptr) & 15u) == 0u;  // (as launch_quantize_tokens wants it)
+    // Narrow tiles: both expert stages in one launch. (A stage that is timed, traced or given out by itself keeps its own.)
+    const bool fused_schedule = layer_schedule_is_fused(T, p->K, p->experts, a->expert_count != 0u);
+    const bool one_launch = fused_quantise && fused_schedule && !prof && !p->cta_trace.ptr && !a->expert_outputs && layer_in_one_launch(p, T);
     ExpertSet* sets[2] = {nullptr, nullptr};
     NVMOE_TRY(prepare_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
     NVMOE_TRY(prepare_expert_set(p, false, a->down_addresses, a->down_slots, tensor, &sets[1]));
-    if (layer_schedule_is_fused(T, p->K, p->experts, a->expert_count != 0u)) {
+    if (fused_schedule) {
         LayerSchedule ls{};
+        if (one_launch) {
+            ls.clear = p->layer_sync.as<uint32_t>();
+            ls.clear_words = p->experts + 1u;
+        }
         ls.routes = (const uint32_t*)routes->ptr;
         ls.intermediates = (uint32_t*)frames.ptr;
         ls.slots[0] = (const uint32_t*)a->gate_up_slots->ptr;
@@ -1572,6 +1600,21 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     call.control = (const uint32_t*)gate_control.ptr;
     call.prepared = sets[0];
     call.fuse_quantise = fused_quantise;
+    if (one_launch) {
+        LayerLaunch ll{};
+        for (int i = 0; i < 2; i++) {
+            call.gate_up = i == 0;
+            call.fuse_quantise = i == 0;
+            call.outputs = i == 0 ? nullptr : (uint16_t*)outs.ptr;
+            NVMOE_TRY(expert_launch(p, call, sets[i], true, &ll.stage[i]));
+            ll.stage[i].scale_base = sets[i]->derived.as<uint8_t>();
+        }
+        ll.sync = p->layer_sync.as<uint32_t>();
+        launch_layer_tc(ll, st);
+        p->report.tensor_path = 1u;
+        p->launches++;
+        NVMOE_TRY(post_launch(p, "experts"));
+    } else {
     NVMOE_TRY(run_experts(p, call));
     mark(kStageQuantI);
     if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true, false));
@@ -1588,6 +1631,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     call.prepared = sets[1];
     call.fuse_quantise = false;
     NVMOE_TRY(run_experts(p, call));
+    }
     mark(kStageReduce);
     if (!a->expert_outputs) {
         launch_reduce((const uint16_t*)outs.ptr, (uint16_t*)a->output->ptr, T, p->K, g.hidden_size, g.reduce_scale,

@@ -182,6 +182,8 @@ struct LayerSchedule {
     uint32_t* tile_count[2];
     uint32_t* status;
     uint32_t tokens, expert_start, expert_count, K, I, tiles_per_route[2], num_experts, n_tile[2];
+    uint32_t* clear;       // words that a later kernel of the call counts in, to be zeroed
+    uint32_t clear_words;
 };
 bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned);
 // the router and the schedule of a call of up to 16 tokens (32 of up to 32 experts) in one launch

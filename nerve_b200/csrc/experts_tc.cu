@@ -1309,8 +1309,20 @@ void tc_configure_kernels() {
     configure_tile<96u>();
     configure_tile<128u>();
     pair_configure_kernels();
+    layer_configure_kernels();
 }
 
+// Both expert stages of a layer call in one launch: where gate/up is more than a round of the SMs, counted as if every expert were
+// selected. In less, the one kernel's longer set-up and the down tiles of 256 rows (of 128 in launches of their own) cost more
+// than the second launch. Layers, two launches / one, us, by gate/up tiles: 16 (tiny, 8 tokens) 22.0 / 23.3, 32 (64 tokens) 25.2 / 28.0,
+// 92 (one token of 32 experts of 2880 x 2880) 38.9 / 40.7, 184 (two) 51.4 / 48.3, 276 55.0 / 53.1, 644 (seven) 73.4 / 67.6, 736 (64) 102.5
+// / 93.8; 128 experts, 2944 tiles, 64 tokens 280.7 / 268.5, 501 362.6 / 348.8, 1200 445.2 / 439.6, 2000 (96-token tiles) 537 / 537; 256 of 7168 x
+// 2048, 4112 tiles, 24 tokens 462 / 442, 300 1058 / 1062, 1000 1454 / 1398.
+bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t gate_rows) {
+    const uint64_t routes = (uint64_t)tokens * routes_per_token, lists = routes < num_experts ? routes : num_experts;
+    return lists * ((gate_rows + kBlockM - 1u) / kBlockM) > (uint64_t)sm_count();
+}
+void launch_layer_tc(const LayerLaunch& p, cudaStream_t stream) { launch_experts_layer(p, sm_count(), stream); }
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<true>(p, stream); }
 void launch_down_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<false>(p, stream); }
 

@@ -81,6 +81,18 @@ inline uint32_t tc_token_map_for(const TokenTile& t) {
 size_t tc_derived_scale_bytes(uint32_t rows, uint32_t cols);
 // re-tiles the scales of every expert whose scale record changed since the last call
 void launch_derive_scales_tc(const ExpertLaunch& p, bool gate_up, cudaStream_t stream);
+// Both expert stages of a layer call in one launch (experts_layer.cu): one CTA a tile, the same token tile in both, tensor maps,
+// the down operands made by gate/up.
+struct LayerLaunch {
+    ExpertLaunch stage[2];
+    uint32_t* sync;    // experts + 1 words, cleared by the schedule: chunks claimed, per expert the warps done with its gate/up tiles
+};
+constexpr uint32_t kLayerExperts = 1024u;  // at most
+void layer_configure_kernels();
+// whether a call is large enough for it
+bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t gate_rows);
+void launch_layer_tc(const LayerLaunch& p, cudaStream_t stream);
+void launch_experts_layer(const LayerLaunch& p, int sms, cudaStream_t stream);
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream);
 void launch_down_tc(const ExpertLaunch& p, cudaStream_t stream);
 

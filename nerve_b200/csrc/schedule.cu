@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(1024) layer_schedule_small_kernel(LayerSchedul
     uint32_t* compact_list = route_words + count;
     uint8_t* resident = reinterpret_cast<uint8_t*>(compact_list + count);
     grid_dependency_sync();
+    for (uint32_t w = threadIdx.x; w < s.clear_words; w += blockDim.x) s.clear[w] = 0u;
     if (threadIdx.x < 14u) {
         const uint32_t j = threadIdx.x % 7u;
         s.control[threadIdx.x / 7u][j] = j == 0u ? s.tokens : j == 1u ? s.expert_start : j == 2u ? s.expert_count : 0u;
@@ -636,6 +637,7 @@ __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s,
     for (uint32_t w = threadIdx.x; w < table_words; w += blockDim.x) smem_words[w] = 0u;
     if (threadIdx.x < 2u) totals[threadIdx.x] = 0u;
     before();
+    for (uint32_t w = threadIdx.x; w < s.clear_words; w += blockDim.x) s.clear[w] = 0u;
     // residency of every expert for both stages (bucket E is never kept)
     // (the two stages are unrolled throughout: pointers picked by a run-time stage would live in local memory)
     for (uint32_t b = threadIdx.x; b < C; b += blockDim.x) {
@@ -817,6 +819,8 @@ __global__ void __launch_bounds__(256) layer_schedule_scatter_kernel(LayerSchedu
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     for (uint32_t w = threadIdx.x; w < (8u * B + 1u) / 2u; w += blockDim.x) table_words[w] = 0u;
     grid_dependency_sync();
+    if (blockIdx.x == 0u)
+        for (uint32_t w = threadIdx.x; w < s.clear_words; w += blockDim.x) s.clear[w] = 0u;
     const uint32_t i = blockIdx.x * kSortChunk + threadIdx.x;
     uint32_t bucket = kNotListed;
     if (i < count) bucket = min_u32(__ldg(s.routes + i) & 0xffffu, E);
