@@ -32,6 +32,20 @@ __device__ __forceinline__ void warp_argmax(float& s, uint32_t& e) {
     }
 }
 
+// A score as a number whose order is the score's: equal for equal scores (-0 and 0 are), above 0 for every score but a NaN, which is 0.
+__device__ __forceinline__ uint32_t score_key(float s) {
+    const uint32_t bits = __float_as_uint(__fadd_rn(s, 0.0f));
+    return s != s ? 0u : bits ^ ((uint32_t)((int32_t)bits >> 31) | 0x80000000u);
+}
+// warp_argmax by the warp's integer maximum: of the lanes' (score, expert) pairs the one with the higher score, of equal ones with
+// the lower expert; kUnboundSlot stands for no pair. All lanes return the winner. Ten shuffles and five compares in a chain a
+// round otherwise: layers, us, one token of 32 experts 38.4 / 37.3 with four rounds of this, tiny layer of 64 25.8 / 25.4.
+__device__ __forceinline__ uint32_t warp_best(float s, uint32_t e) {
+    const uint32_t key = e == kUnboundSlot ? 0u : score_key(s);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    return __reduce_min_sync(0xffffffffu, top != 0u && key == top ? e : kUnboundSlot);
+}
+
 __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uint32_t e) {
     if (dtype == NVMOE_BIAS_F32) return reinterpret_cast<const float*>(bias)[e];
     if (dtype == NVMOE_BIAS_BF16) return nvmoe_bf16_to_f32(reinterpret_cast<const uint16_t*>(bias)[e]);
@@ -128,9 +142,7 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
         uint32_t kept = 0u;
         for (uint32_t round = 0; round < p.g.topk_group; round++) {
             const bool open = lane < p.g.n_group && ((kept >> lane) & 1u) == 0u && my_group >= kNegInf;  // (not a NaN)
-            float s = open ? my_group : kNegInf;
-            uint32_t winner = open ? lane : kUnboundSlot;
-            warp_argmax(s, winner);
+            const uint32_t winner = warp_best(my_group, open ? lane : kUnboundSlot);
             if (winner != kUnboundSlot) kept |= 1u << winner;
         }
 #pragma unroll
@@ -153,9 +165,7 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
                 best_v = val[j];
             }
         }
-        float s = best;
-        uint32_t winner = best_e;
-        warp_argmax(s, winner);
+        const uint32_t winner = warp_best(best, best_e);
         if (winner == kUnboundSlot) {
             missing = true;
             break;
