@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
 // (token, output) pairs: thread v plays lane v of every pair in the tile, so each x and w word is
 // loaded once per thread and reused across the tile, and the 64 lane sums of a pair are folded
 // with the pinned butterfly (step 32 through shared memory, 16..1 by shuffles).
-template <int TT, int ET>
+template <int TT, int ET, int DEPTH>
 __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __restrict__ x,
                                                            const uint16_t* __restrict__ w,
                                                            const uint16_t* __restrict__ bias,
@@ -273,12 +273,11 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
         for (int b = 0; b < ET; b++) acc[a][b] = 0.0f;
 
     // The sum order of a lane is fixed (its words in ascending order), the load order is not: the
-    // loads of kDepth steps are issued together so that their latencies overlap.
-    constexpr int kDepth = TT * ET <= 16 ? 8 : TT * ET <= 32 ? 4 : 2;
-    for (uint32_t cw0 = v; cw0 < words; cw0 += 64u * kDepth) {
-        uint32_t xr[kDepth][TT], wr[kDepth][ET];
+    // loads of DEPTH steps are issued together so that their latencies overlap.
+    for (uint32_t cw0 = v; cw0 < words; cw0 += 64u * DEPTH) {
+        uint32_t xr[DEPTH][TT], wr[DEPTH][ET];
 #pragma unroll
-        for (int u = 0; u < kDepth; u++) {
+        for (int u = 0; u < DEPTH; u++) {
             const uint32_t cw = cw0 + 64u * u;
             const bool in = cw < words;
 #pragma unroll
@@ -287,7 +286,7 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
             for (int b = 0; b < ET; b++) wr[u][b] = (in && e0 + b < outputs) ? __ldg(ww + (size_t)(e0 + b) * words + cw) : 0u;
         }
 #pragma unroll
-        for (int u = 0; u < kDepth; u++) {
+        for (int u = 0; u < DEPTH; u++) {
             if (cw0 + 64u * u >= words) break;  // a step past the end must not even add zeros (-0 + 0 = +0)
 #pragma unroll
             for (int a = 0; a < TT; a++) {
@@ -537,16 +536,20 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         // 231.5. By itself at 8.4 blocks 9.8 / 9.1 (hidden 512) and 20.1 / 18.4 (2880), at 9.1 39.6 / 41.8 (7168).
         const uint32_t blocks = wide.x * wide.y;
         if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
-            launch_chained(router_linear_kernel<4, 8>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+            launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+        } else if (grid.x * grid.y <= 4u * 148u && hidden > 1024u) {
+            // Few blocks of long rows: a call waits for the latency of their loads, so that 24 steps are under way instead of 8. Layers, us,
+            // 8 / 24: one token of 32 experts of 2880 39.0 / 38.4, 64 tokens 95.2 / 94.8; rows of 512, which are four steps, 25.1 / 25.5.
+            launch_chained(router_linear_kernel<2, 4, 24>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
         } else {
-            launch_chained(router_linear_kernel<2, 4>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+            launch_chained(router_linear_kernel<2, 4, 8>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
         }
     } else if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u) {
         dim3 grid((outputs + kTileOutputs - 1u) / kTileOutputs, (tokens + kTileTokens - 1u) / kTileTokens);
         launch_chained(router_linear_tiled_kernel, grid, dim3(256), kRouterTileBytes, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
     } else {
         dim3 grid((outputs + 15u) / 16u, (tokens + 3u) / 4u);
-        launch_chained(router_linear_kernel<4, 16>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+        launch_chained(router_linear_kernel<4, 16, 2>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
     }
 }
 
