@@ -15,6 +15,7 @@
 #include <type_traits>
 #include <vector>
 
+#include <cuda.h>
 #include <dlfcn.h>
 #include <nccl.h>
 
@@ -113,6 +114,10 @@ struct ExpertSet {
 };
 constexpr size_t kMaxExpertSets = 64;
 constexpr size_t kMapTemplates = (2u * kWeightMaps + 1u) * 128u;  // bytes of a stage's template tensor maps
+// Rows of a host-buffer layer call that kernels fetch and store, at most. Copy engine / kernels, us: tiny, 64 tokens (64 KB) 51.3 / 46.4, 1024
+// (1 MB) 94.9 / 83.4; hidden 2880, 1 token 60.8 / 58.5, 32 121.9 / 120.7, 128 159 / 149, 512 (2.9 MB) 282 / 268, 1024 (5.9 MB) 425 / 426;
+// 7168, 64 709 / 660, 400 (5.7 MB) 1246 / 1172.
+constexpr size_t kHostKernelBytes = 4u << 20;
 constexpr int kHostWaitSeconds = 60;  // how long the host-buffer layer call waits for its result
 
 enum Stage { kStageLinear, kStageRoute, kStageSchedule, kStageQuantX, kStageGateUp, kStageQuantI, kStageDown, kStageReduce, kStageCount };
@@ -1647,6 +1652,41 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     return NVMOE_OK;
 }
 
+static bool page_locked(const void* ptr) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return attr.type == cudaMemoryTypeHost;
+}
+
+// The device's address of a range of page-locked host memory; null when the range is not wholly inside one allocation, has another address there
+// or does not lie on the 16-byte grid.
+static void* host_range_address(const void* ptr, size_t bytes) {
+    typedef CUresult (*AttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+    static const AttributeFn attribute = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<AttributeFn>(ok ? fn : nullptr);
+    }();
+    if (!attribute) return nullptr;
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)ptr;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (attr.type != cudaMemoryTypeHost || attr.devicePointer != ptr || ((uintptr_t)ptr & 15u) != 0u ||
+        attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS || start > at || at - start > size || bytes > size - (at - start))
+        return nullptr;
+    return attr.devicePointer;
+}
+
 int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hidden_host, void* output_host) {
     if (!p || !args || !hidden_host || !output_host) return NVMOE_ERR_INVALID_ARGUMENT;
     const uint32_t T = args->batch_width;
@@ -1663,28 +1703,28 @@ int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hi
     cudaError_t err = p->hidden_dev.ensure(cap);
     if (err == cudaSuccess) err = p->output_dev.ensure(cap);
     if (err != cudaSuccess) return fail(d, NVMOE_ERR_OUT_OF_MEMORY, "staging allocation failed: %s", cudaGetErrorString(err));
-    // page-locked caller memory is read and written by the copy engine directly; anything else goes
-    // through the plan's own page-locked staging buffers
-    auto page_locked = [](const void* ptr) {
-        cudaPointerAttributes attr{};
-        if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return attr.type == cudaMemoryTypeHost;
-    };
+    // Page-locked caller memory is read and written directly, by the copy engine or, few rows, by kernels: one fetches the input, the
+    // combine writes the result. Anything else goes through the plan's own page-locked staging buffers.
     const bool direct_in = page_locked(hidden_host), direct_out = page_locked(output_host);
     if (!direct_in) std::memcpy(p->pinned_in, hidden_host, bytes);
-    NVMOE_CUDA(d, cudaMemcpyAsync(p->hidden_dev.ptr, direct_in ? hidden_host : p->pinned_in, bytes, cudaMemcpyHostToDevice,
-                                  d->stream));
+    const bool few = bytes <= kHostKernelBytes && bytes % 16u == 0u;
+    void* in_address = few ? host_range_address(direct_in ? hidden_host : p->pinned_in, bytes) : nullptr;
+    void* out_address = few && !args->expert_outputs ? host_range_address(direct_out ? output_host : p->pinned_out, bytes) : nullptr;
+    if (in_address) {
+        launch_fetch_host(in_address, p->hidden_dev.ptr, bytes, d->stream);
+        p->launches++;
+        NVMOE_TRY(post_launch(p, "fetch hidden"));
+    } else {
+        NVMOE_CUDA(d, cudaMemcpyAsync(p->hidden_dev.ptr, direct_in ? hidden_host : p->pinned_in, bytes, cudaMemcpyHostToDevice, d->stream));
+    }
     nvmoe_buffer hidden{d, p->hidden_dev.ptr, cap};
-    nvmoe_buffer output{d, p->output_dev.ptr, cap};
+    nvmoe_buffer output{d, out_address ? out_address : p->output_dev.ptr, out_address ? bytes : cap};
     nvmoe_layer_args local = *args;
     local.hidden = &hidden;
     local.output = &output;
     NVMOE_TRY(nvmoe_layer(p, &local));
-    NVMOE_CUDA(d, cudaMemcpyAsync(direct_out ? output_host : p->pinned_out, p->output_dev.ptr, bytes, cudaMemcpyDeviceToHost,
-                                  d->stream));
+    if (!out_address)
+        NVMOE_CUDA(d, cudaMemcpyAsync(direct_out ? output_host : p->pinned_out, p->output_dev.ptr, bytes, cudaMemcpyDeviceToHost, d->stream));
     // The caller waits for this result. A decode step is over in well under a millisecond, so poll for it
     // first (a blocking wait would add the wake-up of a sleeping thread to every step); after two
     // milliseconds yield the core between polls; and give up after kHostWaitSeconds, like nvmoe_sync.
