@@ -45,7 +45,7 @@ using namespace tc;
 
 constexpr uint32_t kFirstProducerThread = 192u;    // warps 0-3 epilogue, 4 MMA, 5 TMA, 6.. cp.async, then more epilogue warps
 constexpr uint32_t kMaxStages = 8u;
-constexpr uint32_t kRowPairRounds = 6u;  // rounds of the SMs, with every expert selected, from which narrow down tiles pair their rows
+constexpr uint32_t kRowPairRounds = 6u;  // rounds of the SMs, with every expert selected, from which down tiles of 32 tokens pair their rows
 constexpr uint32_t kWatchWarp = 2u;     // the epilogue warp that polls for a finished accumulator (not on the MMA or TMA warp's scheduler)
 
 // ROW_PAIR (down only): a tile covers two 128-row tiles of the one weight matrix, handled as the two
@@ -1011,21 +1011,22 @@ void launch_n(const ExpertLaunch& p, int sms, cudaStream_t stream) {
 }
 
 // Whether a down launch takes two row tiles at a time: always with wide token tiles, and with narrow ones (TMA form)
-// when that leaves an SM several tiles to go through, counted as if every expert were selected (what routing, a partition
+// when that leaves the SMs enough tiles, counted as if every expert were selected (what routing, a partition
 // or absent experts leave of them is not known here). A stage of a row pair is one K block: one box of 256 weight rows, one token
 // box, two scale copies. One of a single row tile is two K blocks: a weight box, a token box and a scale copy, for the
 // same weight bytes and twice the token rows. Single row tiles spread over the SMs in finer steps, which 32-token tiles gain
-// from while there are few rounds. Layer of intermediate 1536, single rows / row pairs, us, by rounds: 32-token tiles 0.65 51.3 /
-// 52.2, 1.3 62.9 / 67.4, 1.95 81.2 / 85.0, 2.6 100.4 / 101.4, 3.5 113.4 / 113.6, 3.9 124.6 / 126.0, 5.2 143.4 / 142.6, 6.05 167.8 / 165.9,
-// 7.8 191.9 / 188.8, 10.4 234.1 / 228.7, 24 519 / 506; 16-token tiles 0.65 51.8 / 48.9, 1.3 60.7 / 58.3, 2.6 84.3 / 80.1, 5.2 129.9 / 126.5,
-// 6.05 147.5 / 142.7, 10.4 212.2 / 207.1, 24 436 / 425: the line lies where 32-token tiles have it; 16-token tiles would gain
-// below it too.
+// from while there are few rounds, 16-token tiles only where pairs leave SMs without a tile. Layer of intermediate 1536, single rows /
+// row pairs, us, by rounds: 32-token tiles 0.65 51.3 / 52.2, 1.3 62.9 / 67.4, 1.95 81.2 / 85.0, 2.6 100.4 / 101.4, 3.5 113.4 / 113.6, 3.9
+// 124.6 / 126.0, 5.2 143.4 / 142.6, 6.05 167.8 / 165.9, 7.8 191.9 / 188.8, 10.4 234.1 / 228.7, 24 519 / 506; 16-token tiles 0.65 51.8 /
+// 48.9, 1.3 60.7 / 58.3, 2.6 84.3 / 80.1, 5.2 129.9 / 126.5, 6.05 147.5 / 142.7, 10.4 212.2 / 207.1, 24 436 / 425; 16 experts of 2048 x 256 and x 512, 0.86
+// 29.6 / 27.0, 32.3 / 29.3; 24 of 4096 x 256, 2.6 42.1 / 38.2.
 bool takes_row_pairs(const ExpertLaunch& p, uint32_t n_tile, bool tma, int sms) {
     if (n_tile >= kRowPairTokens) return true;
     if (!tma) return false;
     const uint64_t routes = (uint64_t)p.tokens * (p.g.routed_k + p.g.always_count);
     const uint64_t lists = routes < p.work.num_experts ? routes : p.work.num_experts;
-    return lists * ((p.g.hidden_size + 2u * kBlockM - 1u) / (2u * kBlockM)) >= (uint64_t)kRowPairRounds * (uint64_t)sms;
+    const uint64_t tiles = lists * ((p.g.hidden_size + 2u * kBlockM - 1u) / (2u * kBlockM));
+    return n_tile <= 16u ? 2u * tiles >= (uint64_t)sms : tiles >= (uint64_t)kRowPairRounds * (uint64_t)sms;
 }
 
 template <bool GATE_UP>
