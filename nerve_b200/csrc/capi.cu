@@ -1494,8 +1494,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     const bool prof = p->profile_stages;
     // the time of a call that begins with the projection and ends with the combine is noted by these kernels, of another or
     // of stages by events
-    p->clocked = !prof && a->router_weights && !a->routes_in && !a->expert_outputs;
-    CallClock* clock = p->clocked ? p->clock.as<CallClock>() : nullptr;
+    CallClock* clock = !prof && a->router_weights && !a->routes_in && !a->expert_outputs ? p->clock.as<CallClock>() : nullptr;
     auto mark = [&](int i) {
         if (prof || (clock == nullptr && (i == 0 || i == kStageCount))) cudaEventRecord(p->ev[i], st);
     };
@@ -1645,6 +1644,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         NVMOE_TRY(post_launch(p, "reduce"));
     }
     mark(kStageCount);
+    p->clocked = clock != nullptr;
     p->events_valid = true;
     p->report.batch_width = T;
     p->report.routes = T * p->K;
@@ -1843,7 +1843,8 @@ int nvmoe_plan_last_report(nvmoe_plan* p, nvmoe_work_report* report) {
     if (p->clocked) {
         CallClock clock;
         NVMOE_CUDA(d, cudaMemcpy(&clock, p->clock.ptr, sizeof clock, cudaMemcpyDeviceToHost));
-        p->report.total_ms = (float)((double)(clock.end - clock.begin) * 1e-6);
+        // (a later call that was refused half-way has noted its begin alone)
+        p->report.total_ms = clock.end > clock.begin ? (float)((double)(clock.end - clock.begin) * 1e-6) : 0.0f;
     } else {
         NVMOE_CUDA(d, cudaEventElapsedTime(&p->report.total_ms, p->ev[0], p->ev[kStageCount]));
     }

@@ -76,6 +76,26 @@ def test_experts_that_one_stage_lacks(device):
     bank.destroy()
 
 
+@pytest.mark.parametrize("tokens", [20, 200, 500])
+def test_expert_ranges(device, tokens):
+    """Calls of a range of the experts: the same output as from launches of their own, and routes of other experts count as zeros."""
+    cfg, case, tensors, plan, bank, out, call = prepared(device, "gpt-oss-20b", (320, 704, 32), tokens)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    rbias = device.resident_buffer_from(case.router_bias)
+    for start, count in ((0, 32), (0, 9), (9, 23), (31, 1)):
+        got = []
+        for profiled in (False, True, False):
+            plan.set_profiling(profiled)
+            plan.layer(tokens, bank, hidden, out, router_weights=rw, router_bias=rbias, expert_start=start, expert_count=count)
+            assert plan.status() == 0
+            got.append(out.read(np.uint16).copy())
+        np.testing.assert_array_equal(got[0], got[1])
+        np.testing.assert_array_equal(got[0], got[2])
+        assert 0.0 < plan.last_report()["total_ms"] < 1000.0
+    plan.destroy()
+    bank.destroy()
+
+
 @pytest.mark.parametrize("name,shape,tokens", [("gpt-oss-20b", (320, 704, 32), 40), ("gpt-oss-20b", (1152, 640, 32), 700), ("deepseek-v3", (384, 640, 32), 35)])
 def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, name, shape, tokens):
     cfg, case, tensors, plan, bank, out, call = prepared(device, name, shape, tokens)
