@@ -32,24 +32,45 @@ __global__ void __launch_bounds__(256) reduce_kernel(const uint32_t* __restrict_
     note_end(clock);
 }
 
+// Two columns of a sum, rounded to bf16: as the f32 sum rounded, since 24 bits are more than twice 8 and two.
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ bool either_is_nan(uint32_t pair) { return (pair & 0x7fffu) > 0x7f80u || (pair & 0x7fff0000u) > 0x7f800000u; }
+
+// One word of a token's sum as reduce_kernel takes it, for words in which a NaN turns up (its bits are those of the f32 sums rounded).
+__device__ __noinline__ uint32_t combine_word(const uint32_t* in, const uint32_t* marks, uint32_t K, uint32_t hidden_words, float routed_scale) {
+    float lo = 0.0f, hi = 0.0f;
+    for (uint32_t r = 0; r < K; r++) {
+        const uint32_t c = (marks && marks[r] == kUnboundSlot) ? 0u : in[(size_t)r * hidden_words];
+        lo = nvmoe_round_bf16(__fadd_rn(lo, nvmoe_bf16_to_f32(c)));
+        hi = nvmoe_round_bf16(__fadd_rn(hi, nvmoe_bf16_to_f32(c >> 16)));
+    }
+    return pack_bf16x2(__fmul_rn(lo, routed_scale), __fmul_rn(hi, routed_scale));
+}
+
 // The same sum over 16-byte pieces (eight columns a thread) for rows that allow it: the order of the adds
-// of a column and every rounding are unchanged. Bound by memory: DEPTH routes are fetched together, their marks first.
-// Four at a time, except for nine routes, which then take one step where fours would take three (4096 tokens of 4096
-// columns 67.8 against 72.4 us). A deeper step that fours need only two for, or that ends in a second one, costs more in
-// registers than it saves: nine against four at a time 62.1 / 61.4 us for 8 routes, 84.0 / 77.4 for 10, 58.1 / 54.6 for
-// 16 of 2048 columns.
-template <uint32_t DEPTH>
+// of a column and every rounding are unchanged. Bound by memory: DEPTH routes are fetched together, in a call of all experts (WHOLE) with
+// their marks, which then only choose what is added, in a call of a range of them after their marks, since most rows are skipped.
+// Four at a time, except for nine routes, which then take one step where fours would take three (with adds in f32, 4096 tokens of
+// 4096 columns 67.8 against 72.4 us). A deeper step that fours need only two for, or that ends in a second one, costs more in
+// registers than it saves (with adds in f32, nine against four at a time 62.1 / 61.4 us for 8 routes, 84.0 / 77.4 for 10, 58.1 /
+// 54.6 for 16 of 2048 columns).
+// Adds in pairs of columns, whole-number arithmetic in 32 bits and marks that rows do not wait for, before / after: 4096 tokens of four
+// routes of 2880 columns 25.8 / 21.0 us, 16384 93.1 / 76.2, 96 of nine of 7168 6.3 / 4.1, 16384 434 / 341 (6.9 TB/s). A grid of the
+// resident blocks, 4 or 6 per SM, 74.8 and 344; a thread a piece 76.2 and 337, but 11.5 against 10.5 at 2048 tokens.
+template <uint32_t DEPTH, bool WHOLE>
 __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict__ expert_outputs, uint4* __restrict__ output,
-                                                        uint32_t tokens, uint32_t K, uint32_t hidden_vecs, float routed_scale,
+                                                        uint32_t total, uint32_t K, uint32_t hidden_vecs, float routed_scale,
                                                         const uint32_t* __restrict__ computed, CallClock* clock) {
     grid_dependency_sync();
-    const uint64_t total = (uint64_t)tokens * hidden_vecs;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = (uint32_t)(i / hidden_vecs), vec = (uint32_t)(i % hidden_vecs);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const uint32_t t = i / hidden_vecs, vec = i - t * hidden_vecs;
         const uint4* in = expert_outputs + (size_t)t * K * hidden_vecs + vec;
-        float acc[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] = 0.0f;
+        const uint32_t* marks = computed ? computed + (size_t)t * K : nullptr;
+        uint32_t acc[4] = {0u, 0u, 0u, 0u};
         // (the adds keep the route order)
         for (uint32_t r0 = 0; r0 < K; r0 += DEPTH) {
             bool skipped[DEPTH];
@@ -57,26 +78,25 @@ __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict
 #pragma unroll
             for (uint32_t u = 0; u < DEPTH; u++)
                 // a route the down stage skipped (computed[route] says "nowhere") counts as a row of zeros
-                skipped[u] = r0 + u >= K || (computed && __ldg(computed + (size_t)t * K + r0 + u) == kUnboundSlot);
+                skipped[u] = r0 + u >= K || (marks && __ldg(marks + r0 + u) == kUnboundSlot);
 #pragma unroll
-            for (uint32_t u = 0; u < DEPTH; u++) c[u] = skipped[u] ? make_uint4(0u, 0u, 0u, 0u) : in[(size_t)(r0 + u) * hidden_vecs];
+            for (uint32_t u = 0; u < DEPTH; u++)
+                c[u] = (WHOLE ? r0 + u >= K : skipped[u]) ? make_uint4(0u, 0u, 0u, 0u) : __ldg(in + (size_t)(r0 + u) * hidden_vecs);
 #pragma unroll
             for (uint32_t u = 0; u < DEPTH; u++) {
                 if (r0 + u >= K) break;
                 const uint32_t w[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    acc[2 * j] = nvmoe_round_bf16(__fadd_rn(acc[2 * j], nvmoe_bf16_to_f32(w[j])));
-                    acc[2 * j + 1] = nvmoe_round_bf16(__fadd_rn(acc[2 * j + 1], nvmoe_bf16_to_f32(w[j] >> 16)));
-                }
+                for (int j = 0; j < 4; j++) acc[j] = add_bf16x2(acc[j], WHOLE && skipped[u] ? 0u : w[j]);
             }
         }
-        uint4 out;
-        out.x = pack_bf16x2(__fmul_rn(acc[0], routed_scale), __fmul_rn(acc[1], routed_scale));
-        out.y = pack_bf16x2(__fmul_rn(acc[2], routed_scale), __fmul_rn(acc[3], routed_scale));
-        out.z = pack_bf16x2(__fmul_rn(acc[4], routed_scale), __fmul_rn(acc[5], routed_scale));
-        out.w = pack_bf16x2(__fmul_rn(acc[6], routed_scale), __fmul_rn(acc[7], routed_scale));
-        output[i] = out;
+        uint32_t out[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            out[j] = pack_bf16x2(__fmul_rn(nvmoe_bf16_to_f32(acc[j]), routed_scale), __fmul_rn(nvmoe_bf16_to_f32(acc[j] >> 16), routed_scale));
+            if (either_is_nan(acc[j])) out[j] = combine_word(reinterpret_cast<const uint32_t*>(in) + j, marks, K, 4u * hidden_vecs, routed_scale);
+        }
+        output[i] = make_uint4(out[0], out[1], out[2], out[3]);
     }
     note_end(clock);
 }
@@ -190,14 +210,16 @@ bool launch_reduce_gather(const uint16_t* rows, const uint32_t* gather, uint16_t
 }
 
 void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t tokens, uint32_t K, uint32_t hidden,
-                   float routed_scale, const uint32_t* computed, CallClock* clock, cudaStream_t stream) {
+                   float routed_scale, const uint32_t* computed, bool partitioned, CallClock* clock, cudaStream_t stream) {
     if (tokens == 0u) return;
-    if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(expert_outputs) | reinterpret_cast<uintptr_t>(output)) & 15u) == 0u) {
-        const uint64_t vecs = (uint64_t)tokens * (hidden / 8u);
+    const uint64_t vecs = (uint64_t)tokens * (hidden / 8u);
+    if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(expert_outputs) | reinterpret_cast<uintptr_t>(output)) & 15u) == 0u && vecs < (1ull << 31)) {
         uint64_t vec_blocks = (vecs + 255u) / 256u;
         if (vec_blocks > 148u * 16u) vec_blocks = 148u * 16u;
-        launch_chained(K == 9u ? reduce_vec_kernel<9u> : reduce_vec_kernel<4u>, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
-                       reinterpret_cast<const uint4*>(expert_outputs), reinterpret_cast<uint4*>(output), tokens, K, hidden / 8u,
+        const auto kernel = K == 9u ? (partitioned ? reduce_vec_kernel<9u, false> : reduce_vec_kernel<9u, true>)
+                                    : (partitioned ? reduce_vec_kernel<4u, false> : reduce_vec_kernel<4u, true>);
+        launch_chained(kernel, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
+                       reinterpret_cast<const uint4*>(expert_outputs), reinterpret_cast<uint4*>(output), (uint32_t)vecs, K, hidden / 8u,
                        routed_scale, computed, clock);
         return;
     }
