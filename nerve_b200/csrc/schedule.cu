@@ -114,7 +114,9 @@ __device__ __forceinline__ void warp_exclusive_scan(uint32_t buckets, uint32_t* 
 __host__ __device__ inline size_t rank_block_words(uint32_t threads, uint32_t buckets) {
     return (size_t)buckets + 2u * (buckets + 1u) + ((size_t)threads / 32u * buckets + 1u) / 2u;
 }
-__host__ __device__ inline bool rank_block_fits(uint32_t threads, uint32_t buckets) { return rank_block_words(threads, buckets) * 4u <= 48u * 1024u; }
+// Shared memory that a launch may ask for beside the static arrays of the one-block kernels (144 bytes, the tile list's): together 48 KB.
+constexpr size_t kOneBlockBytes = 48u * 1024u - 256u;
+__host__ __device__ inline bool rank_block_fits(uint32_t threads, uint32_t buckets) { return rank_block_words(threads, buckets) * 4u <= kOneBlockBytes; }
 template <class KeyFn, class EmitFn, class DoneFn>
 __device__ void rank_single_block(uint32_t count, uint32_t buckets, uint32_t* words, uint32_t n_tile, KeyFn key, EmitFn emit, DoneFn done) {
     uint32_t* total = words;
@@ -1208,7 +1210,7 @@ static bool rank_schedule_fits(uint64_t count, uint32_t num_experts) {
 }
 
 static bool three_sort_schedule_fits(uint64_t count, uint32_t num_experts) {
-    return count <= kSmallSortLimit && layer_schedule_smem_bytes((uint32_t)count, num_experts) <= 48u * 1024u;
+    return count <= kSmallSortLimit && layer_schedule_smem_bytes((uint32_t)count, num_experts) <= kOneBlockBytes;
 }
 
 // Beyond 1280 routes the three launches are cheaper than the one block's longer loop, unless it is a partitioned call or
