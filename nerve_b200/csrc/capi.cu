@@ -661,16 +661,20 @@ int nvmoe_plan_set_profiling(nvmoe_plan* p, int enabled) {
 
 // ---- node-granular operators -----------------------------------------------------------------
 
-static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
-                         const nvmoe_buffer* router_bias, CallClock* clock) {
-    if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
+static int check_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, const nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
+                               const nvmoe_buffer* router_bias) {
     NVMOE_TRY(check_tokens(p, T));
     const nvmoe_geometry& g = p->g;
     NVMOE_TRY(check_buffer(p, hidden, (size_t)T * g.hidden_size * 2u, "hidden"));
     NVMOE_TRY(check_buffer(p, logits, (size_t)T * ((g.routed_experts + 1u) / 2u) * 4u, "logits"));
     NVMOE_TRY(check_buffer(p, router_weights, (size_t)g.routed_experts * g.hidden_size * 2u, "router weights"));
     if (router_bias) NVMOE_TRY(check_buffer(p, router_bias, (size_t)g.routed_experts * 2u, "router bias"));
-    NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
+    return NVMOE_OK;
+}
+
+static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
+                         const nvmoe_buffer* router_bias, CallClock* clock) {
+    const nvmoe_geometry& g = p->g;
     launch_router_linear((const uint16_t*)hidden->ptr, (const uint16_t*)router_weights->ptr,
                          router_bias ? (const uint16_t*)router_bias->ptr : nullptr, (uint32_t*)logits->ptr, T,
                          g.hidden_size, g.routed_experts, clock, p->device->stream);
@@ -680,6 +684,9 @@ static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, 
 
 int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits,
                         const nvmoe_buffer* router_weights, const nvmoe_buffer* router_bias) {
+    if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
+    NVMOE_TRY(check_router_linear(p, T, hidden, logits, router_weights, router_bias));
+    NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     return router_linear(p, T, hidden, logits, router_weights, router_bias, nullptr);
 }
 
@@ -827,17 +834,12 @@ static int expert_set_for(nvmoe_plan* p, int set, const nvmoe_buffer* addresses,
     return NVMOE_OK;
 }
 
-// shared tail of the two gate/up entry points and of down
-// The resolved expert set of a table pair, with everything the kernels of this call need from it on
-// the device: validated pointers and, for the tensor path, re-tiled scales and tensor maps. Launches
-// only what the cached state lacks.
-static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* addresses, const nvmoe_buffer* slots,
-                              bool tensor, ExpertSet** out) {
+// Everything the kernels of this call need of an expert set (expert_set_for) on the device: validated pointers and, for the
+// tensor path, re-tiled scales and tensor maps. Launches only what the cached state lacks.
+static int fill_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* addresses, const nvmoe_buffer* slots, bool tensor, ExpertSet* es) {
     const nvmoe_geometry& g = p->g;
     cudaStream_t st = p->device->stream;
     const int set = gate_up ? 0 : 1;
-    ExpertSet* es = nullptr;
-    NVMOE_TRY(expert_set_for(p, set, addresses, slots, tensor, &es));
     const uint64_t rows = gate_up ? g.intermediate_size : g.hidden_size;
     const uint64_t cols = gate_up ? g.hidden_size : g.intermediate_size;
     if (!es->resolved || es->resolved_for_tensor != tensor) {
@@ -864,8 +866,14 @@ static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* a
         }
         es->tensor_ready = es->cacheable;
     }
-    *out = es;
     return post_launch(p, gate_up ? "gate/up expert tables" : "down expert tables");
+}
+
+// The resolved expert set of a table pair, filled.
+static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* addresses, const nvmoe_buffer* slots,
+                              bool tensor, ExpertSet** out) {
+    NVMOE_TRY(expert_set_for(p, gate_up ? 0 : 1, addresses, slots, tensor, out));
+    return fill_expert_set(p, gate_up, addresses, slots, tensor, *out);
 }
 
 // Whether the expert stages of a layer call of T tokens may run in one launch: one CTA a tile, the same tile and tensor maps in both.
@@ -1466,8 +1474,17 @@ static int ensure_layer_scratch(nvmoe_plan* p) {
     return NVMOE_OK;
 }
 
-int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
-    if (!p || !a) return NVMOE_ERR_INVALID_ARGUMENT;
+// Where the input rows of a host-buffer call come from: fetched by a kernel from their address on the device, else copied.
+struct HostRows {
+    const void* rows;
+    const void* address;  // null: copied
+    void* device;
+    size_t bytes;
+};
+
+// The layer call, after the input rows have been brought to the device (`host`, if given). Whatever can refuse it stands before the
+// first launch: a refused call does nothing, and the report keeps the time of the last whole one.
+static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* host) {
     const uint32_t T = a->batch_width;
     NVMOE_TRY(check_tokens(p, T));
     const nvmoe_geometry& g = p->g;
@@ -1490,7 +1507,6 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
     NVMOE_TRY(ensure_layer_scratch(p));
     cudaStream_t st = d->stream;
-    const uint32_t launches_before = p->launches;
     const bool prof = p->profile_stages;
     // the time of a call that begins with the projection and ends with the combine is noted by these kernels, of another or
     // of stages by events
@@ -1498,6 +1514,7 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     auto mark = [&](int i) {
         if (prof || (clock == nullptr && (i == 0 || i == kStageCount))) cudaEventRecord(p->ev[i], st);
     };
+    const bool tensor = use_tensor_path(p);
 
     nvmoe_buffer logits_view{d, p->logits.ptr, p->logits.bytes};
     nvmoe_buffer* logits = a->logits ? a->logits : &logits_view;
@@ -1509,15 +1526,28 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     nvmoe_buffer gate_control{d, p->controls.ptr, 28u};
     nvmoe_buffer down_control{d, (char*)p->controls.ptr + 32u, 28u};
 
+    const bool projects = a->router_weights && !a->routes_in;
+    RouterLaunch router{};
+    ExpertSet* sets[2] = {nullptr, nullptr};
+    if (projects) NVMOE_TRY(check_router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias));
+    if (!a->routes_in) NVMOE_TRY(router_launch_for(p, T, logits, routes, a->bias, a->telemetry, &router));
+    NVMOE_TRY(expert_set_for(p, 0, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
+    NVMOE_TRY(expert_set_for(p, 1, a->down_addresses, a->down_slots, tensor, &sets[1]));
+
+    if (host && host->address) {
+        launch_fetch_host(host->address, host->device, host->bytes, st);
+        p->launches++;
+        NVMOE_TRY(post_launch(p, "fetch hidden"));
+    } else if (host) {
+        NVMOE_CUDA(d, cudaMemcpyAsync(host->device, host->rows, host->bytes, cudaMemcpyHostToDevice, st));
+    }
+    const uint32_t launches_before = p->launches;
     mark(kStageLinear);
-    if (a->router_weights && !a->routes_in)
-        NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, clock));
+    if (projects) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, clock));
     mark(kStageRoute);
     // (with stage profiling on, the router keeps a launch and a time of its own)
-    RouterLaunch router{};
     bool routes_in_schedule = false;
     if (!a->routes_in) {
-        NVMOE_TRY(router_launch_for(p, T, logits, routes, a->bias, a->telemetry, &router));
         routes_in_schedule = !prof && layer_routes_in_schedule(router, p->K, p->experts);
         if (!routes_in_schedule) {
             launch_router(router, st);
@@ -1526,7 +1556,6 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
         }
     }
     mark(kStageSchedule);
-    const bool tensor = use_tensor_path(p);
     // with scale blocks of 32 or 128 (what a warp, or the four warps of an epilogue group, hold of a token) the tensor-path
     // gate/up epilogue quantises its own output for the down stage
     const bool fused_quantise = tensor && (g.act_block == 32u || g.act_block == 128u) &&
@@ -1534,9 +1563,8 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     // Narrow tiles: both expert stages in one launch. (A stage that is timed, traced or given out by itself keeps its own.)
     const bool fused_schedule = layer_schedule_is_fused(T, p->K, p->experts, a->expert_count != 0u);
     const bool one_launch = fused_quantise && fused_schedule && !prof && !p->cta_trace.ptr && !a->expert_outputs && layer_in_one_launch(p, T);
-    ExpertSet* sets[2] = {nullptr, nullptr};
-    NVMOE_TRY(prepare_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
-    NVMOE_TRY(prepare_expert_set(p, false, a->down_addresses, a->down_slots, tensor, &sets[1]));
+    NVMOE_TRY(fill_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, sets[0]));
+    NVMOE_TRY(fill_expert_set(p, false, a->down_addresses, a->down_slots, tensor, sets[1]));
     if (fused_schedule) {
         LayerSchedule ls{};
         if (one_launch) {
@@ -1652,6 +1680,11 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     return NVMOE_OK;
 }
 
+int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
+    if (!p || !a) return NVMOE_ERR_INVALID_ARGUMENT;
+    return layer_call(p, a, nullptr);
+}
+
 static bool page_locked(const void* ptr) {
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
@@ -1710,19 +1743,13 @@ int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hi
     const bool few = bytes <= kHostKernelBytes && bytes % 16u == 0u;
     void* in_address = few ? host_range_address(direct_in ? hidden_host : p->pinned_in, bytes) : nullptr;
     void* out_address = few && !args->expert_outputs ? host_range_address(direct_out ? output_host : p->pinned_out, bytes) : nullptr;
-    if (in_address) {
-        launch_fetch_host(in_address, p->hidden_dev.ptr, bytes, d->stream);
-        p->launches++;
-        NVMOE_TRY(post_launch(p, "fetch hidden"));
-    } else {
-        NVMOE_CUDA(d, cudaMemcpyAsync(p->hidden_dev.ptr, direct_in ? hidden_host : p->pinned_in, bytes, cudaMemcpyHostToDevice, d->stream));
-    }
+    const HostRows rows{direct_in ? hidden_host : p->pinned_in, in_address, p->hidden_dev.ptr, bytes};
     nvmoe_buffer hidden{d, p->hidden_dev.ptr, cap};
     nvmoe_buffer output{d, out_address ? out_address : p->output_dev.ptr, out_address ? bytes : cap};
     nvmoe_layer_args local = *args;
     local.hidden = &hidden;
     local.output = &output;
-    NVMOE_TRY(nvmoe_layer(p, &local));
+    NVMOE_TRY(layer_call(p, &local, &rows));
     if (!out_address)
         NVMOE_CUDA(d, cudaMemcpyAsync(direct_out ? output_host : p->pinned_out, p->output_dev.ptr, bytes, cudaMemcpyDeviceToHost, d->stream));
     // The caller waits for this result. A decode step is over in well under a millisecond, so poll for it
@@ -1839,11 +1866,11 @@ int nvmoe_plan_last_report(nvmoe_plan* p, nvmoe_work_report* report) {
     nvmoe_device* d = p->device;
     if (!p->events_valid) return fail(d, NVMOE_ERR_INVALID_ARGUMENT, "no layer call has run on this plan");
     NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
+    CallClock clock{};
+    if (p->clocked) NVMOE_CUDA(d, cudaMemcpyAsync(&clock, p->clock.ptr, sizeof clock, cudaMemcpyDeviceToHost, d->stream));
     NVMOE_CUDA(d, cudaStreamSynchronize(d->stream));
     if (p->clocked) {
-        CallClock clock;
-        NVMOE_CUDA(d, cudaMemcpy(&clock, p->clock.ptr, sizeof clock, cudaMemcpyDeviceToHost));
-        // (a later call that was refused half-way has noted its begin alone)
+        // (a later call whose launches failed may have noted its begin alone)
         p->report.total_ms = clock.end > clock.begin ? (float)((double)(clock.end - clock.begin) * 1e-6) : 0.0f;
     } else {
         NVMOE_CUDA(d, cudaEventElapsedTime(&p->report.total_ms, p->ev[0], p->ev[kStageCount]));

@@ -1,0 +1,41 @@
+"""A layer call that is refused launches nothing and leaves what the plan reports of the last whole call."""
+import numpy as np
+import pytest
+
+from nerve_b200 import synthetic
+from nerve_b200.backend import CudaComputeDevice, CudaError, ExpertBank, MoePlan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("profiled", [False, True])
+def test_refused_layer_calls(profiled):
+    device = CudaComputeDevice(0)
+    tokens = 9
+    cfg = synthetic.small_variant(synthetic.CONFIGS["deepseek-v3"], 256, 128, 16)
+    case = synthetic.make_case(cfg, tokens, seed=53)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    plan.set_profiling(profiled)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, out = device.resident_buffer_from(case.hidden), device.create_resident_buffer(tokens * cfg.hidden * 2)
+    good = {"router_weights": device.resident_buffer_from(case.router_w), "bias": device.resident_buffer_from(case.select_bias)}
+    plan.layer(tokens, bank, hidden, out, **good)
+    small = device.create_resident_buffer(4)
+    before, launches = plan.last_report(), plan.launches()
+    assert before["total_ms"] > 0.0
+    x, y = case.hidden.copy(), np.zeros_like(case.hidden)
+    for bad in ({"telemetry": small}, {"bias": small}, {"bias": None}, {"logits": small}, {"router_weights": small}, {"router_bias": small},
+                {"routes_out": small}):
+        with pytest.raises(CudaError):
+            plan.layer(tokens, bank, hidden, out, **(good | bad))
+        with pytest.raises(CudaError):
+            plan.layer_host(tokens, bank, x, y, **(good | bad))
+        assert plan.launches() == launches, bad
+        assert plan.last_report() == before, bad
+    assert not y.any()
+    plan.layer_host(tokens, bank, x, y, **good)
+    np.testing.assert_array_equal(y, out.read(np.uint16).reshape(y.shape))
+    assert plan.launches() > launches and plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+    device.close()
