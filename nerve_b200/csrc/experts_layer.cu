@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
                     }
                     if (rows) fence_proxy_async_all();
                 }
+                __syncwarp();  // what lane 0 has acquired is every lane's from here on (a shuffle orders no memory)
                 if (__shfl_sync(0xffffffffu, ok, 0) == 0u) break;
             }
             nxt = cur;

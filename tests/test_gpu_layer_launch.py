@@ -55,6 +55,34 @@ def test_layer_matches_the_checker(device, name, shape, tokens, native):
     bank.destroy()
 
 
+@pytest.mark.parametrize("name,shape,tokens,native", [
+    ("gpt-oss-20b", (1920, 1152, 32), 40, 0), ("gpt-oss-20b", (2624, 1216, 32), 160, 0), ("gpt-oss-20b", (2752, 1088, 32), 290, 0),
+    ("gpt-oss-20b", (3008, 1152, 32), 700, 0), ("deepseek-v3", (2048, 1280, 32), 35, 1), ("deepseek-v3", (3072, 1280, 32), 340, 0)])
+def test_successive_calls_hand_over_their_own_rows(device, name, shape, tokens, native):
+    """Calls of the same plan on tokens of very different size: a down tile that read codes or scales from before its gate/up tiles
+    were done would find those of the call ahead. The outputs are those of launches of their own (a profiled call)."""
+    cfg, case, tensors, plan, bank, out, call = prepared(device, name, shape, tokens, native)
+    rng = np.random.default_rng(3)
+    rw = device.resident_buffer_from(case.router_w)
+    kw = dict(router_weights=rw, router_bias=device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+              bias=device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None)
+    sources = [device.resident_buffer_from(synthetic.f32_to_bf16(rng.standard_normal((tokens, cfg.hidden), dtype=np.float32) * np.float32(size)))
+               for size in (1.0, 1e-3, 60.0)]
+    want = []
+    plan.set_profiling(True)
+    for source in sources:
+        plan.layer(tokens, bank, source, out, **kw)
+        want.append(out.read(np.uint16).copy())
+    plan.set_profiling(False)
+    for i in (0, 1, 2, 1, 0, 2, 0, 1, 1, 2):
+        plan.layer(tokens, bank, sources[i], out, **kw)
+        np.testing.assert_array_equal(out.read(np.uint16), want[i])
+    assert plan.last_report()["kernel_launches"] == (6 if tokens * cfg.total_k < 1280 else 8)  # (one launch for both stages)
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+
+
 def test_experts_that_one_stage_lacks(device):
     """An expert without down weights, one without gate/up weights (whose down rows are zeros) and one without either: the same
     output as from the launches of their own that a profiled call makes."""
