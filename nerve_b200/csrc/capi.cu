@@ -880,7 +880,7 @@ static int prepare_expert_set(nvmoe_plan* p, bool gate_up, const nvmoe_buffer* a
 static bool layer_in_one_launch(const nvmoe_plan* p, uint32_t T) {
     const TokenTile gate = token_tile(p, true, T), down = token_tile(p, false, T);
     return p->tma[0] && p->tma[1] && !gate.pair && !down.pair && gate.rows == down.rows && p->experts <= kLayerExperts &&
-           tc_layer_in_one_launch(T, p->K, p->experts, p->g.intermediate_size);
+           tc_layer_in_one_launch(T, p->K, p->experts, p->g.hidden_size, p->g.intermediate_size, gate.rows);
 }
 
 // Groups the routes of one expert stage by expert (and, for the tensor path, records where each route

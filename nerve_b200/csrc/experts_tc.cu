@@ -1313,15 +1313,30 @@ void tc_configure_kernels() {
     layer_configure_kernels();
 }
 
-// Both expert stages of a layer call in one launch: where gate/up is more than a round of the SMs, counted as if every expert were
-// selected. In less, the one kernel's longer set-up and the down tiles of 256 rows (of 128 in launches of their own) cost more
-// than the second launch. Layers, two launches / one, us, by gate/up tiles: 16 (tiny, 8 tokens) 22.0 / 23.3, 32 (64 tokens) 25.2 / 28.0,
-// 92 (one token of 32 experts of 2880 x 2880) 38.9 / 40.7, 184 (two) 51.4 / 48.3, 276 55.0 / 53.1, 644 (seven) 73.4 / 67.6, 736 (64) 102.5
-// / 93.8; 128 experts, 2944 tiles, 64 tokens 280.7 / 268.5, 501 362.6 / 348.8, 1200 445.2 / 439.6, 2000 (96-token tiles) 537 / 537; 256 of 7168 x
-// 2048, 4112 tiles, 24 tokens 462 / 442, 300 1058 / 1062, 1000 1454 / 1398.
-bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t gate_rows) {
-    const uint64_t routes = (uint64_t)tokens * routes_per_token, lists = routes < num_experts ? routes : num_experts;
-    return lists * ((gate_rows + kBlockM - 1u) / kBlockM) > (uint64_t)sm_count();
+// Both expert stages of a layer call in one launch, counted as if every expert were selected and had the mean load:
+// - Gate/up is more than a round of the SMs. In less, the one kernel's longer set-up and its down tiles of 256 rows cost more than the second
+//   launch: 16 gate/up tiles (tiny, 8 tokens) 22.0 us by two launches / 23.3, 32 (64 tokens) 25.2 / 28.0, 92 (one token of 32 experts of
+//   2880 x 2880) 38.9 / 40.7.
+// - Beyond 1.6 rounds, K of gate/up is long enough: 12 stages for tiles of 16 tokens, for wider ones 18 and one for every twenty tokens of an
+//   expert. The one kernel's epilogue takes longer than that of the two (a further polling warp beside it; a warp of its own for the
+//   announcements made it no better), and only the stages of the next tile hide that. Layers, two / one, us: 16-token tiles, 4 stages (512 x
+//   4096, 32 experts) 49.7 / 63.7, 6 (768 x 3072, 64) 75.1 / 83.0, 12 (1536 x 768, 128, one token each) 58.9 / 57.1, 16 (2048 x 1536, 64)
+//   86.3 / 78.8; 32 tokens, 12 stages (1536 x 2304, 32) 64.8 / 70.8, 23 (2880 x 2880, 32) 114.6 / 101.4; 64, 12 stages (1536 x 768, 128) 112.6 /
+//   121.3, 23 128.3 / 120.9; 96, 12 stages 182.7 / 203.8, 16 (2048 x 1536, 64) 157.3 / 172.5, 23 180.2 / 172.5.
+// - K of down is at least eight stages, or that of gate/up 32 with tiles of 64 tokens or more, and the down tiles of 256 rows fill the SMs:
+//   4608 x 256, 128 experts, 32 tokens 65.2 / 70.7, 2048 x 2560, 16, eight tokens 44.0 / 46.6.
+// Over 2000 layers drawn from 384 to 7168 columns, 256 to 4096 intermediate ones and 16 to 128 experts, two / one: the 932 beyond 1.6 rounds that
+// these lines send here, medians 1.04 to 1.05 by width of the tile, 0.94 to 1.17; the 795 others there, medians 0.93 to 0.96, 0.70 to 1.10. In fewer
+// rounds the two are level on the whole, whatever K is: medians 1.00 to 1.02, 0.84 to 1.37.
+bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t hidden, uint32_t intermediate, uint32_t token_rows) {
+    const uint64_t routes = (uint64_t)tokens * routes_per_token, lists = routes < num_experts ? routes : num_experts, sms = (uint64_t)sm_count();
+    const uint64_t tiles = lists * ((intermediate + kBlockM - 1u) / kBlockM), down_tiles = lists * ((hidden + 2u * kBlockM - 1u) / (2u * kBlockM));
+    if (tiles <= sms) return false;
+    if (5u * tiles <= 8u * sms) return true;
+    const uint64_t stages = (hidden + kBlockK - 1u) / kBlockK, per_expert = (routes + num_experts - 1u) / num_experts;
+    const bool long_gate = token_rows <= 16u ? stages >= 12u : 20u * stages >= 360u + per_expert;
+    const bool long_down = intermediate > 7u * kBlockK || (token_rows >= 64u && stages >= 32u);
+    return long_gate && long_down && down_tiles >= sms;
 }
 void launch_layer_tc(const LayerLaunch& p, cudaStream_t stream) { launch_experts_layer(p, sm_count(), stream); }
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream) { launch<true>(p, stream); }

@@ -89,8 +89,8 @@ struct LayerLaunch {
 };
 constexpr uint32_t kLayerExperts = 1024u;  // at most
 void layer_configure_kernels();
-// whether a call is large enough for it
-bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t gate_rows);
+// whether a call gains by it
+bool tc_layer_in_one_launch(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t hidden, uint32_t intermediate, uint32_t token_rows);
 void launch_layer_tc(const LayerLaunch& p, cudaStream_t stream);
 void launch_experts_layer(const LayerLaunch& p, int sms, cudaStream_t stream);
 void launch_gate_up_tc(const ExpertLaunch& p, cudaStream_t stream);

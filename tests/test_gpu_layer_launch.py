@@ -83,6 +83,29 @@ def test_successive_calls_hand_over_their_own_rows(device, name, shape, tokens, 
     bank.destroy()
 
 
+# Either side of the lines of the rule: K of gate/up by token tile (16, 32, 64, 96), K of down, rounds of gate/up, tiles of down
+@pytest.mark.parametrize("shape,tokens,one", [
+    ((1408, 1152, 32), 64, False), ((1536, 1152, 32), 64, True), ((2304, 1152, 32), 160, False), ((2432, 1152, 32), 160, True),
+    ((2432, 1152, 32), 290, False), ((2560, 1152, 32), 290, True), ((2816, 1152, 32), 700, False), ((2944, 1152, 32), 700, True),
+    ((2048, 896, 40), 40, False), ((2048, 960, 40), 40, True), ((3968, 384, 80), 720, False), ((4096, 384, 80), 720, True),
+    ((512, 896, 32), 40, True), ((512, 960, 32), 40, False), ((1792, 1536, 32), 5, False), ((1792, 1536, 32), 6, True)])
+def test_which_calls_take_one_launch(device, shape, tokens, one):
+    cfg, case, tensors, plan, bank, out, call = prepared(device, "gpt-oss-20b", shape, tokens)
+    got = []
+    call()  # (builds the tables of the experts)
+    for profiled in (False, True):
+        plan.set_profiling(profiled)
+        call()
+        got.append(out.read(np.uint16).copy())
+        if not profiled:  # projection, router, schedule, quantisation, one or two, combine; up to 32 tokens route in the schedule
+            separate = 8 if tokens * cfg.total_k >= 1280 else 6 if tokens > 32 else 5
+            assert plan.last_report()["kernel_launches"] == separate + (0 if one else 1)
+    np.testing.assert_array_equal(got[0], got[1])
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+
+
 def test_experts_that_one_stage_lacks(device):
     """An expert without down weights, one without gate/up weights (whose down rows are zeros) and one without either: the same
     output as from the launches of their own that a profiled call makes."""
