@@ -145,6 +145,7 @@ struct nvmoe_plan {
     // scratch of the fused layer call
     DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev;
     void* pinned_in = nullptr;
+    bool pinned_mapped = false;  // both have the same address on the device
     void* pinned_out = nullptr;
     size_t pinned_bytes = 0;
     cudaEvent_t ev[kStageCount + 1] = {};
@@ -1685,39 +1686,33 @@ int nvmoe_layer(nvmoe_plan* p, const nvmoe_layer_args* a) {
     return layer_call(p, a, nullptr);
 }
 
-static bool page_locked(const void* ptr) {
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return attr.type == cudaMemoryTypeHost;
-}
-
-// The device's address of a range of page-locked host memory; null when the range is not wholly inside one allocation, has another address there
-// or does not lie on the 16-byte grid.
-static void* host_range_address(const void* ptr, size_t bytes) {
-    typedef CUresult (*AttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
-    static const AttributeFn attribute = [] {
+// What the host-buffer call needs to know of a caller's buffer: whether it is page-locked, and the device's address of it, null when
+// the range is not wholly inside one allocation, has another address there or does not lie on the 16-byte grid. One query of the driver
+// a buffer: with four for the two kinds of attributes, tiny layer of 31 tokens 44.2 us, 43.5 this way, one token of 2880 columns 57.9 / 57.3.
+struct HostRange {
+    bool page_locked;
+    void* address;
+};
+static HostRange host_range(const void* ptr, size_t bytes) {
+    typedef CUresult (*AttributesFn)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const AttributesFn attributes = [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult found;
-        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
-        return reinterpret_cast<AttributeFn>(ok ? fn : nullptr);
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<AttributesFn>(ok ? fn : nullptr);
     }();
-    if (!attribute) return nullptr;
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)ptr;
-    CUdeviceptr start = 0;
+    // (a pointer that the driver does not know leaves all of them zero)
+    CUmemorytype type{};
+    unsigned int managed = 0u;
+    CUdeviceptr device = 0, start = 0;
     size_t size = 0;
-    if (attr.type != cudaMemoryTypeHost || attr.devicePointer != ptr || ((uintptr_t)ptr & 15u) != 0u ||
-        attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
-        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS || start > at || at - start > size || bytes > size - (at - start))
-        return nullptr;
-    return attr.devicePointer;
+    CUpointer_attribute which[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                    CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* into[5] = {&type, &managed, &device, &start, &size};
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)ptr;
+    if (!attributes || attributes(5u, which, into, at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed != 0u) return HostRange{false, nullptr};
+    const bool whole = device == at && (at & 15u) == 0u && start <= at && at - start <= size && bytes <= size - (at - start);
+    return HostRange{true, whole ? const_cast<void*>(ptr) : nullptr};
 }
 
 int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hidden_host, void* output_host) {
@@ -1728,22 +1723,23 @@ int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hi
     NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
     const size_t bytes = (size_t)T * p->g.hidden_size * 2u;
     const size_t cap = (size_t)p->g.max_tokens * p->g.hidden_size * 2u;
-    if (!p->pinned_in) {
-        NVMOE_CUDA(d, cudaMallocHost(&p->pinned_in, cap));
+    if (!p->pinned_out) {
+        if (!p->pinned_in) NVMOE_CUDA(d, cudaMallocHost(&p->pinned_in, cap));
         NVMOE_CUDA(d, cudaMallocHost(&p->pinned_out, cap));
         p->pinned_bytes = cap;
+        p->pinned_mapped = host_range(p->pinned_in, cap).address != nullptr && host_range(p->pinned_out, cap).address != nullptr;
     }
     cudaError_t err = p->hidden_dev.ensure(cap);
     if (err == cudaSuccess) err = p->output_dev.ensure(cap);
     if (err != cudaSuccess) return fail(d, NVMOE_ERR_OUT_OF_MEMORY, "staging allocation failed: %s", cudaGetErrorString(err));
     // Page-locked caller memory is read and written directly, by the copy engine or, few rows, by kernels: one fetches the input, the
     // combine writes the result. Anything else goes through the plan's own page-locked staging buffers.
-    const bool direct_in = page_locked(hidden_host), direct_out = page_locked(output_host);
-    if (!direct_in) std::memcpy(p->pinned_in, hidden_host, bytes);
+    const HostRange in = host_range(hidden_host, bytes), out = host_range(output_host, bytes);
     const bool few = bytes <= kHostKernelBytes && bytes % 16u == 0u;
-    void* in_address = few ? host_range_address(direct_in ? hidden_host : p->pinned_in, bytes) : nullptr;
-    void* out_address = few && !args->expert_outputs ? host_range_address(direct_out ? output_host : p->pinned_out, bytes) : nullptr;
-    const HostRows rows{direct_in ? hidden_host : p->pinned_in, in_address, p->hidden_dev.ptr, bytes};
+    if (!in.page_locked) std::memcpy(p->pinned_in, hidden_host, bytes);
+    void* in_address = !few ? nullptr : in.page_locked ? in.address : p->pinned_mapped ? p->pinned_in : nullptr;
+    void* out_address = !few || args->expert_outputs ? nullptr : out.page_locked ? out.address : p->pinned_mapped ? p->pinned_out : nullptr;
+    const HostRows rows{in.page_locked ? hidden_host : p->pinned_in, in_address, p->hidden_dev.ptr, bytes};
     nvmoe_buffer hidden{d, p->hidden_dev.ptr, cap};
     nvmoe_buffer output{d, out_address ? out_address : p->output_dev.ptr, out_address ? bytes : cap};
     nvmoe_layer_args local = *args;
@@ -1751,7 +1747,7 @@ int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hi
     local.output = &output;
     NVMOE_TRY(layer_call(p, &local, &rows));
     if (!out_address)
-        NVMOE_CUDA(d, cudaMemcpyAsync(direct_out ? output_host : p->pinned_out, p->output_dev.ptr, bytes, cudaMemcpyDeviceToHost, d->stream));
+        NVMOE_CUDA(d, cudaMemcpyAsync(out.page_locked ? output_host : p->pinned_out, p->output_dev.ptr, bytes, cudaMemcpyDeviceToHost, d->stream));
     // The caller waits for this result. A decode step is over in well under a millisecond, so poll for it
     // first (a blocking wait would add the wake-up of a sleeping thread to every step); after two
     // milliseconds yield the core between polls; and give up after kHostWaitSeconds, like nvmoe_sync.
@@ -1770,7 +1766,7 @@ int nvmoe_layer_host(nvmoe_plan* p, const nvmoe_layer_args* args, const void* hi
             if (now >= spin_until) std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
     }
-    if (!direct_out) std::memcpy(output_host, p->pinned_out, bytes);
+    if (!out.page_locked) std::memcpy(output_host, p->pinned_out, bytes);
     return NVMOE_OK;
 }
 

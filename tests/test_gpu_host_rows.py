@@ -42,3 +42,35 @@ def test_host_rows(tokens):
     plan.destroy()
     bank.destroy()
     device.close()
+
+
+@pytest.mark.parametrize("words", [0, 8, 5])  # of an offset on the 16-byte grid and off it
+def test_registered_host_rows(words):
+    """Pageable memory that the caller has registered counts as page-locked."""
+    torch = pytest.importorskip("torch")
+    device = CudaComputeDevice(0)
+    tokens = 21
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 512, 128, 8)
+    case = synthetic.make_case(cfg, tokens, seed=47)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    rw = device.resident_buffer_from(case.router_w)
+    out = device.create_resident_buffer(tokens * cfg.hidden * 2)
+    plan.layer(tokens, bank, device.resident_buffer_from(case.hidden), out, router_weights=rw)
+    whole = np.zeros(2 * 4096 + 2 * tokens * cfg.hidden, dtype=np.uint16)  # (whole pages inside it are registered)
+    start = -(-whole.ctypes.data // 4096) * 4096
+    size = (whole.ctypes.data + whole.nbytes - start) // 4096 * 4096
+    assert int(torch.cuda.cudart().cudaHostRegister(start, size, 0)) == 0
+    first = (start - whole.ctypes.data) // 2 + words
+    count = tokens * cfg.hidden
+    x, y = (whole[first + i * count:first + (i + 1) * count].reshape(tokens, cfg.hidden) for i in (0, 1))
+    assert y.ctypes.data + y.nbytes <= start + size
+    x[...] = case.hidden
+    for _ in range(2):
+        y[...] = 0
+        plan.layer_host(tokens, bank, x, y, router_weights=rw)
+        np.testing.assert_array_equal(y, out.read(np.uint16).reshape(tokens, cfg.hidden))
+    assert int(torch.cuda.cudart().cudaHostUnregister(start)) == 0
+    plan.destroy()
+    bank.destroy()
+    device.close()
