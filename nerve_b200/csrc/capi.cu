@@ -1186,7 +1186,7 @@ int nvmoe_reduce(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* expert_outputs, 
     NVMOE_TRY(check_buffer(p, output, (size_t)T * g.hidden_size * 2u, "output"));
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
     launch_reduce((const uint16_t*)expert_outputs->ptr, (uint16_t*)output->ptr, T, p->K, g.hidden_size, g.reduce_scale,
-                  nullptr, false, nullptr, p->device->stream);
+                  nullptr, nullptr, p->device->stream);
     p->launches++;
     return post_launch(p, "reduce");
 }
@@ -1668,7 +1668,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     mark(kStageReduce);
     if (!a->expert_outputs) {
         launch_reduce((const uint16_t*)outs.ptr, (uint16_t*)a->output->ptr, T, p->K, g.hidden_size, g.reduce_scale,
-                      p->position[1].as<uint32_t>(), a->expert_count != 0u, clock, st);
+                      p->position[1].as<uint32_t>(), clock, st);
         p->launches++;
         NVMOE_TRY(post_launch(p, "reduce"));
     }

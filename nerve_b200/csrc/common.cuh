@@ -316,9 +316,8 @@ cudaError_t launch_mma_rate_probe(uint32_t n_tile, uint32_t groups, uint32_t cta
 // reduce.cu: `bytes` (a multiple of 16, both addresses 16-byte aligned) from page-locked host memory, at its device address
 void launch_fetch_host(const void* host, void* device, size_t bytes, cudaStream_t stream);
 // reduce.cu: moe_reduce_batch1_bf16. `computed` (optional, [tokens * K]) marks with 0xffffffff the routes
-// whose rows were never written: they count as zeros, so the rows need no clearing beforehand. In a `partitioned` call
-// these are most, and are not fetched.
+// whose rows were never written: they count as zeros, so the rows need no clearing beforehand.
 void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t tokens, uint32_t K,
-                   uint32_t hidden, float routed_scale, const uint32_t* computed, bool partitioned, CallClock* clock, cudaStream_t stream);
+                   uint32_t hidden, float routed_scale, const uint32_t* computed, CallClock* clock, cudaStream_t stream);
 
 }  // namespace nvmoe

@@ -52,16 +52,16 @@ __device__ __noinline__ uint32_t combine_word(const uint32_t* in, const uint32_t
 }
 
 // The same sum over 16-byte pieces (eight columns a thread) for rows that allow it: the order of the adds
-// of a column and every rounding are unchanged. Bound by memory: DEPTH routes are fetched together, in a call of all experts (WHOLE) with
-// their marks, which then only choose what is added, in a call of a range of them after their marks, since most rows are skipped.
+// of a column and every rounding are unchanged. Bound by memory: DEPTH routes are fetched together, in small calls with their marks
+// (EARLY), which then only choose what is added, else after their marks, so that rows of skipped routes are not read.
 // Four at a time, except for nine routes, which then take one step where fours would take three (with adds in f32, 4096 tokens of
 // 4096 columns 67.8 against 72.4 us). A deeper step that fours need only two for, or that ends in a second one, costs more in
 // registers than it saves (with adds in f32, nine against four at a time 62.1 / 61.4 us for 8 routes, 84.0 / 77.4 for 10, 58.1 /
 // 54.6 for 16 of 2048 columns).
-// Adds in pairs of columns, whole-number arithmetic in 32 bits and marks that rows do not wait for, before / after: 4096 tokens of four
+// Adds in pairs of columns and whole-number arithmetic in 32 bits, before / after: 4096 tokens of four
 // routes of 2880 columns 25.8 / 21.0 us, 16384 93.1 / 76.2, 96 of nine of 7168 6.3 / 4.1, 16384 434 / 341 (6.9 TB/s). A grid of the
 // resident blocks, 4 or 6 per SM, 74.8 and 344; a thread a piece 76.2 and 337, but 11.5 against 10.5 at 2048 tokens.
-template <uint32_t DEPTH, bool WHOLE>
+template <uint32_t DEPTH, bool EARLY>
 __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict__ expert_outputs, uint4* __restrict__ output,
                                                         uint32_t total, uint32_t K, uint32_t hidden_vecs, float routed_scale,
                                                         const uint32_t* __restrict__ computed, CallClock* clock) {
@@ -81,13 +81,13 @@ __global__ void __launch_bounds__(256) reduce_vec_kernel(const uint4* __restrict
                 skipped[u] = r0 + u >= K || (marks && __ldg(marks + r0 + u) == kUnboundSlot);
 #pragma unroll
             for (uint32_t u = 0; u < DEPTH; u++)
-                c[u] = (WHOLE ? r0 + u >= K : skipped[u]) ? make_uint4(0u, 0u, 0u, 0u) : __ldg(in + (size_t)(r0 + u) * hidden_vecs);
+                c[u] = (EARLY ? r0 + u >= K : skipped[u]) ? make_uint4(0u, 0u, 0u, 0u) : __ldg(in + (size_t)(r0 + u) * hidden_vecs);
 #pragma unroll
             for (uint32_t u = 0; u < DEPTH; u++) {
                 if (r0 + u >= K) break;
                 const uint32_t w[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[j] = add_bf16x2(acc[j], WHOLE && skipped[u] ? 0u : w[j]);
+                for (int j = 0; j < 4; j++) acc[j] = add_bf16x2(acc[j], EARLY && skipped[u] ? 0u : w[j]);
             }
         }
         uint32_t out[4];
@@ -210,14 +210,19 @@ bool launch_reduce_gather(const uint16_t* rows, const uint32_t* gather, uint16_t
 }
 
 void launch_reduce(const uint16_t* expert_outputs, uint16_t* output, uint32_t tokens, uint32_t K, uint32_t hidden,
-                   float routed_scale, const uint32_t* computed, bool partitioned, CallClock* clock, cudaStream_t stream) {
+                   float routed_scale, const uint32_t* computed, CallClock* clock, cudaStream_t stream) {
     if (tokens == 0u) return;
     const uint64_t vecs = (uint64_t)tokens * (hidden / 8u);
     if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(expert_outputs) | reinterpret_cast<uintptr_t>(output)) & 15u) == 0u && vecs < (1ull << 31)) {
+        // Up to two blocks per SM (one with nine routes) the latency of the marks counts, beyond it what is read. Layers of 2880 x 256, 32 experts, rows with their marks /
+        // after them, us, all experts resident and an eighth of them: 1 token 28.5 / 28.7, 19.9 / 19.8, 64 (90 blocks) 35.5 / 35.7, 31.5 / 31.7,
+        // 200 (282) 45.4 / 45.7, 39.7 / 39.3, 1024 87.5 / 87.6, 58.9 / 55.9, 8192 353.5 / 353.5, 189.8 / 166.6; nine routes of 4096 columns,
+        // 64 experts, 96 tokens (192) 69.2 / 68.7, 49.2 / 48.2, 4096 494 / 491, 235 / 192.
         uint64_t vec_blocks = (vecs + 255u) / 256u;
+        const bool early = vec_blocks <= (K == 9u ? 148u : 2u * 148u);
         if (vec_blocks > 148u * 16u) vec_blocks = 148u * 16u;
-        const auto kernel = K == 9u ? (partitioned ? reduce_vec_kernel<9u, false> : reduce_vec_kernel<9u, true>)
-                                    : (partitioned ? reduce_vec_kernel<4u, false> : reduce_vec_kernel<4u, true>);
+        const auto kernel = K == 9u ? (early ? reduce_vec_kernel<9u, true> : reduce_vec_kernel<9u, false>)
+                                    : (early ? reduce_vec_kernel<4u, true> : reduce_vec_kernel<4u, false>);
         launch_chained(kernel, dim3((uint32_t)vec_blocks), dim3(256), 0, stream,
                        reinterpret_cast<const uint4*>(expert_outputs), reinterpret_cast<uint4*>(output), (uint32_t)vecs, K, hidden / 8u,
                        routed_scale, computed, clock);

@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, MoePlan, ResidentBuffer, geometry_from_config
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, ResidentBuffer, geometry_from_config
+from oracle import moe_oracle as mo
 
 pytestmark = pytest.mark.gpu
 
@@ -54,4 +55,32 @@ def test_combine_matches_its_definition(k, values):
     np.testing.assert_array_equal(out.read(np.uint16)[2:2 + want.size].reshape(want.shape), want)
     shifted.destroy()
     plan.destroy()
+    device.close()
+
+
+# as many blocks of 16-byte pieces as rows are fetched with their marks in (296, 148 of nine routes), and one more (after them)
+@pytest.mark.parametrize("name,tokens", [("gpt-oss-20b", 1894), ("gpt-oss-20b", 1895), ("deepseek-v3", 947), ("deepseek-v3", 948)])
+def test_combine_leaves_skipped_routes_out(name, tokens):
+    """Routes of an expert that is not resident and of experts out of a call's range count as zeros, whatever an earlier call left in
+    their rows."""
+    device = CudaComputeDevice(0)
+    cfg = synthetic.replace(synthetic.small_variant(synthetic.CONFIGS[name], 320, 128, 16), act_block=32)
+    case = synthetic.make_case(cfg, tokens, seed=61)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, rw = device.resident_buffer_from(case.hidden), device.resident_buffer_from(case.router_w)
+    kw = dict(router_weights=rw, router_bias=device.resident_buffer_from(case.router_bias) if case.router_bias is not None else None,
+              bias=device.resident_buffer_from(case.select_bias) if case.select_bias is not None else None)
+    out, rows = device.create_resident_buffer(tokens * cfg.hidden * 2), device.create_resident_buffer(tokens * cfg.total_k * cfg.hidden * 2)
+    scale = geometry_from_config(cfg, tokens).reduce_scale
+    loud = device.resident_buffer_from(np.full_like(case.hidden, 0x7f00))  # (finite, sums of which are not)
+    bank.down_slots.write_bytes(np.full(2, 0xffffffff, dtype=np.uint32), offset=8 * 3)
+    for start, count in ((0, 0), (0, 7), (5, cfg.total_experts - 5)):
+        plan.layer(tokens, bank, loud, out, **kw)
+        plan.layer(tokens, bank, hidden, out, expert_start=start, expert_count=count, **kw)
+        got = out.read(np.uint16).reshape(tokens, cfg.hidden)
+        plan.layer(tokens, bank, hidden, None, expert_start=start, expert_count=count, expert_outputs=rows, **kw)
+        np.testing.assert_array_equal(got, mo.reduce(rows.read(np.uint16).reshape(tokens, cfg.total_k, cfg.hidden), tokens, cfg.total_k, cfg.hidden, scale))
+    plan.destroy()
+    bank.destroy()
     device.close()
