@@ -537,9 +537,12 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         const uint32_t blocks = wide.x * wide.y;
         if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
             launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
-        } else if (grid.x * grid.y <= 4u * 148u && hidden > 1024u) {
-            // Few blocks of long rows: a call waits for the latency of their loads, so that 24 steps are under way instead of 8. Layers, us,
-            // 8 / 24: one token of 32 experts of 2880 39.0 / 38.4, 64 tokens 95.2 / 94.8; rows of 512, which are four steps, 25.1 / 25.5.
+        } else if (grid.x * grid.y <= 4u * 148u && (hidden > 2048u || (hidden > 1024u && grid.x * grid.y <= 148u))) {
+            // Few blocks of long rows: a call waits for the latency of their loads, so that 24 steps (of 128 columns) are under way instead of 8,
+            // which shorter rows gain from only where an SM has one block. Layers, us, 8 / 24: one token of 32 experts of 2880 columns 29.4 / 28.6,
+            // 64 tokens (256 blocks) 38.2 / 37.8, 100 45.6 / 44.9; of 2304 27.9 / 27.1, 34.5 / 34.0, 40.9 / 40.3; of 2048 27.0 / 26.8, 32.4 / 32.5, 37.6 /
+            // 37.6; of 1536 25.6 / 25.1, 30.2 / 30.5, 33.2 / 33.8; of 1088 24.6 / 24.1, 28.8 / 28.9, 31.8 / 32.3; 16 tokens (64 blocks) 26.7 / 26.5; rows
+            // of 512, which are four steps, 25.1 / 25.5. Beyond four blocks an SM 24 steps lose: 64 tokens of 128 experts of 2880 columns 64.1 / 65.9.
             launch_chained(router_linear_kernel<2, 4, 24>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
         } else {
             launch_chained(router_linear_kernel<2, 4, 8>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);

@@ -427,3 +427,19 @@ def test_calls_of_every_tile_from_one_plan(device, name, shape, native):
         own.destroy()
     large.destroy()
     bank.destroy()
+
+
+# few blocks of long rows, whose loads run 24 steps of 128 columns ahead: either side of the lines of the rule (148 and 592 blocks of 2 tokens x
+# 4 outputs, 1024 and 2048 columns), rows that end inside a step, with and beyond the first 24
+@pytest.mark.parametrize("tokens,hidden,experts", [(73, 1056, 16), (75, 1056, 16), (1, 1024, 30), (75, 2048, 16), (75, 2080, 16), (255, 3072, 16),
+                                                   (255, 3104, 15), (2, 6176, 5), (236, 2080, 19), (238, 2080, 19)])
+def test_router_projection_of_few_blocks(device, tokens, hidden, experts):
+    rng = np.random.default_rng(tokens + hidden)
+    plan = plan_of(device, tokens=tokens, hidden=hidden, experts=experts)
+    x, w = bf16(rng.standard_normal((tokens, hidden))), bf16(0.1 * rng.standard_normal((experts, hidden)))
+    x[0] = 0x8000  # (sums of minus zero, which a step past the end would turn into zero)
+    w[1] &= 0x7FFF
+    out = device.create_resident_buffer(tokens * ((experts + 1) // 2) * 4)
+    plan.linear(tokens, device.resident_buffer_from(x), out, device.resident_buffer_from(w), None)
+    np.testing.assert_array_equal(out.read(np.uint32).reshape(tokens, -1), mo.linear_bf16(x, w, None))
+    plan.destroy()
