@@ -46,15 +46,10 @@ struct LayerConfig {
     static constexpr uint32_t kStageBytes = kABytes + kBBytes + kSfBytes;
     static constexpr uint32_t kBarrierBytes = 512u + 64u * kLayerGroups;  // barriers, then the block maxima
     static constexpr uint32_t kSmemMax = 227u * 1024u;
-    // (room for the round-up to a 1024-byte boundary is left out where that buys a slot; the kernel then insists on an aligned base)
-    static constexpr uint32_t slots_for(uint32_t slack) {
-        const uint32_t n = (kSmemMax - kBarrierBytes - slack) / kStageBytes;
-        return n > kLayerMaxSlots ? kLayerMaxSlots : n;
-    }
-    static constexpr bool kNeedsAlignedBase = slots_for(0u) > slots_for(1024u);
-    static constexpr uint32_t kSlots = slots_for(kNeedsAlignedBase ? 0u : 1024u);
+    // (1024 bytes for the round-up to a boundary of as many: 6, 6, 5 and 4 slots, and leaving it out would buy none)
+    static constexpr uint32_t kFit = (kSmemMax - kBarrierBytes - 1024u) / kStageBytes, kSlots = kFit > kLayerMaxSlots ? kLayerMaxSlots : kFit;
     static constexpr uint32_t kBRegion = kSlots * kABytes, kSfRegion = kBRegion + kSlots * kBBytes;
-    static constexpr uint32_t kSmemBytes = kSlots * kStageBytes + (kNeedsAlignedBase ? 0u : 1024u) + kBarrierBytes;
+    static constexpr uint32_t kSmemBytes = kSlots * kStageBytes + 1024u + kBarrierBytes;
     static constexpr uint32_t kAccColumns = 2u * N_TILE, kScaleColumn0 = 2u * kAccColumns, kColumnsUsed = kScaleColumn0 + 12u;
     static constexpr uint32_t kTmemColumns = kColumnsUsed <= 128u ? 128u : kColumnsUsed <= 256u ? 256u : 512u;
     static_assert(kSlots >= 4u && kColumnsUsed <= 512u && kBBytes % 1024u == 0u, "layout");
@@ -106,11 +101,6 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     static_assert(sizeof(LayerBarriers) <= 512u && sizeof(BlockMaxima) == 64u, "barrier block");
     BlockMaxima* maxima = reinterpret_cast<BlockMaxima*>(reinterpret_cast<unsigned char*>(bars) + 512u);
     volatile uint32_t* abort_flag = &bars->abort;
-    if (C::kNeedsAlignedBase && smem != smem_raw) {  // (uniform) no room was set aside for the round-up
-        grid_dependency_sync();
-        if (threadIdx.x == 0u) raise_status(p.stage[0].status, NVMOE_STATUS_INTERNAL);
-        return;
-    }
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const nvmoe_geometry& g = p.stage[0].g;
     const uint32_t H = g.hidden_size, I = g.intermediate_size, K = g.routed_k + g.always_count;
