@@ -391,14 +391,18 @@ int nvmoe_layer(nvmoe_plan* plan, const nvmoe_layer_args* args);
 int nvmoe_layer_host(nvmoe_plan* plan, const nvmoe_layer_args* args, const void* hidden_host,
                      void* output_host);
 
-/* Device time of the last nvmoe_layer call in milliseconds (CUDA events on the device stream);
- * the per-stage report mirrors RuntimeSparseMoeWorkReport
- * (runtime-rs/src/vulkan_stream_circuit/sparse_moe_execution.rs:176-208). */
+/* Device time of the last whole nvmoe_layer call in milliseconds; the per-stage report mirrors RuntimeSparseMoeWorkReport
+ * (runtime-rs/src/vulkan_stream_circuit/sparse_moe_execution.rs:176-208). A call that begins with the projection and ends with
+ * the combine, with profiling off, is timed by the device's nanosecond timer, from when its projection may start (what ran
+ * before it has completed) to the end of its last block; any other by CUDA events on the device stream, which stand before and
+ * after its launches. A call that is refused launches nothing and leaves the report of the last whole one; one whose launches
+ * failed may leave total_ms at 0. With profiling on, a call launches its router, gate/up and down each by itself, where one
+ * without may combine them: stage_ms and the two kernel times are those of such a call. */
 enum { NVMOE_STAGE_LINEAR, NVMOE_STAGE_ROUTE, NVMOE_STAGE_SCHEDULE, NVMOE_STAGE_QUANTIZE_HIDDEN,
        NVMOE_STAGE_GATE_UP, NVMOE_STAGE_QUANTIZE_INTERMEDIATE, NVMOE_STAGE_DOWN, NVMOE_STAGE_REDUCE,
        NVMOE_STAGE_COUNT };
 typedef struct nvmoe_work_report {
-    float total_ms;
+    float total_ms;                    /* see above */
     float stage_ms[NVMOE_STAGE_COUNT]; /* zeros unless profiling is on */
     float gate_up_kernel_ms;           /* the gate/up expert kernel alone (profiling on) */
     float down_kernel_ms;              /* the down expert kernel alone (profiling on) */
@@ -412,7 +416,8 @@ typedef struct nvmoe_work_report {
 int nvmoe_plan_last_report(nvmoe_plan* plan, nvmoe_work_report* report);
 /* ---- diagnostics (unstable: not part of the drop-in surface, may change between builds) --------------
  * The expert kernels that run by default are compiled without any of these; arming the per-CTA trace
- * switches the plan to instantiations that carry them.
+ * switches the plan to instantiations that carry them, and keeps its layer calls from running both expert
+ * stages in one launch, whose kernel has none.
  *
  * Diagnostics of the last tensor-core expert kernels (valid once the trace is armed): counters of CTA 0, twelve words for
  * gate/up then twelve for down: cycles of the lane that issues the copies {wait for a free stage, total}, of the MMA thread

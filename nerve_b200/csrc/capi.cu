@@ -1011,7 +1011,6 @@ static int expert_launch(nvmoe_plan* p, const ExpertCall& c, ExpertSet* es, bool
 
 // shared tail of the two gate/up entry points and of down
 static int run_experts(nvmoe_plan* p, const ExpertCall& c) {
-    const nvmoe_geometry& g = p->g;
     cudaStream_t st = p->device->stream;
     const bool gate_up = c.gate_up;
     const int set = gate_up ? 0 : 1;
@@ -1620,6 +1619,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
                                  (const uint32_t*)down_control.ptr, tensor));
     }
     mark(kStageQuantX);
+    // (this launch also keeps the one for both expert stages, which counts before it waits, apart from the schedule, which clears the counters)
     NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true, fused_quantise));
     mark(kStageGateUp);
     ExpertCall call;
@@ -1648,22 +1648,22 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         p->launches++;
         NVMOE_TRY(post_launch(p, "experts"));
     } else {
-    NVMOE_TRY(run_experts(p, call));
-    mark(kStageQuantI);
-    if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true, false));
-    mark(kStageDown);
-    // routes that are skipped (owned by another device, expert not resident) leave their rows untouched:
-    // the combine below reads the down stage's position table and counts them as zeros; rows handed to
-    // the caller instead start at zero
-    if (a->expert_outputs) cudaMemsetAsync(outs.ptr, 0, (size_t)T * p->K * g.hidden_size * 2u, st);
-    call.gate_up = false;
-    call.outputs = (uint16_t*)outs.ptr;
-    call.addresses = a->down_addresses;
-    call.slots = a->down_slots;
-    call.control = (const uint32_t*)down_control.ptr;
-    call.prepared = sets[1];
-    call.fuse_quantise = false;
-    NVMOE_TRY(run_experts(p, call));
+        NVMOE_TRY(run_experts(p, call));
+        mark(kStageQuantI);
+        if (!fused_quantise) NVMOE_TRY(quantise_operands(p, false, T, frames.ptr, tensor, true, false));
+        mark(kStageDown);
+        // routes that are skipped (owned by another device, expert not resident) leave their rows untouched:
+        // the combine below reads the down stage's position table and counts them as zeros; rows handed to
+        // the caller instead start at zero
+        if (a->expert_outputs) cudaMemsetAsync(outs.ptr, 0, (size_t)T * p->K * g.hidden_size * 2u, st);
+        call.gate_up = false;
+        call.outputs = (uint16_t*)outs.ptr;
+        call.addresses = a->down_addresses;
+        call.slots = a->down_slots;
+        call.control = (const uint32_t*)down_control.ptr;
+        call.prepared = sets[1];
+        call.fuse_quantise = false;
+        NVMOE_TRY(run_experts(p, call));
     }
     mark(kStageReduce);
     if (!a->expert_outputs) {

@@ -18,8 +18,12 @@ constexpr uint32_t kMaxExperts = 4096u;  // ids travel in the low 16 bits of a r
 // precedes its grid_dependency_sync) while the kernel before it in the stream is still running;
 // grid_dependency_sync returns once that kernel has completed and its writes are visible, and lets
 // the next kernel in the stream start in the same way. Every thread of a chained kernel calls it
-// before touching global memory and before any return, so completion still implies that all earlier
-// kernels have completed. Launched the ordinary way, the same kernels run unchanged.
+// before any return, so completion still implies that all earlier kernels have completed, and before
+// touching global memory that the launch ahead of it may write or read. What stands before the call may
+// rely on the launches before that one: the kernel ahead let this one start after its own wait, when they
+// had completed. (Tensor maps and expert tables are read there, and experts_layer.cu claims its first work
+// from a counter that the launch before the one ahead cleared: no kernel may let the next start before its wait, and a
+// launch has to stay between those two.) Launched the ordinary way, the same kernels run unchanged.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_dependency_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

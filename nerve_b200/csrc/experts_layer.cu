@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     volatile uint32_t* abort_flag = &bars->abort;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const nvmoe_geometry& g = p.stage[0].g;
-    const uint32_t H = g.hidden_size, I = g.intermediate_size, K = g.routed_k + g.always_count;
+    const uint32_t H = g.hidden_size, I = g.intermediate_size;
     const uint32_t G = gridDim.x;
 
     // ---- one-time setup ---------------------------------------------------------------------
@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         if (threadIdx.x < 2u) tensormap_acquire(p.stage[threadIdx.x].act_tmap);
         __syncthreads();
     };
-    // What is read before the wait: what stands since earlier calls, or since a launch of this one that had completed when the
-    // kernel ahead could start: that one waited for all before it, the schedule (which cleared the counters) among them.
+    // What is read, and counted, before the wait: what stands since earlier calls, or since a launch of this one that had completed
+    // when the kernel ahead let this one start. That one waited for all before it, the schedule (which cleared the counters) among
+    // them: a launch has to stay between the schedule and this one (the quantisation is), or the claim has to follow the wait.
     uint32_t claimed = 0u;
     if (warp == 7u && lane == 0u) claimed = atomicAdd(p.sync, 1u);
     for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) {
@@ -476,125 +477,126 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
             const uint32_t id = *reinterpret_cast<volatile uint32_t*>(&bars->epilogue_chunk[k & 1u]);
             if (id >= 2u * G) break;
             auto run = [&](auto tag) {
-            constexpr uint32_t phase = decltype(tag)::value;
-            const LayerPhase s = phase_of(phase);
-            const ExpertLaunch& e = p.stage[phase];
-            constexpr bool gate_up = phase == 0u;
-            for (uint32_t tile = id - phase * G; tile < s.tile_count; tile += G, acc_it++) {
-                const uint32_t entry = __ldg(e.tile_list + tile / s.m_tiles), m_tile = tile % s.m_tiles, expert = entry >> 16;
-                const uint32_t first = __ldg(e.work.expert_offsets + expert) + (entry & 0xffffu) * N_TILE;
-                const uint32_t valid = min(N_TILE, __ldg(e.work.expert_offsets + expert + 1u) - first);
-                const uint32_t acc = acc_it & 1u;
-                // where token j of the tile goes (its row among the down operands, or its output row and weight): a chain of two
-                // loads, over before the accumulator is ready for narrow tiles, a lane per token
-                uint32_t my_row = kUnboundSlot;
-                float my_weight = 0.0f;
-                auto find = [&](uint32_t j, bool active) {
-                    my_row = kUnboundSlot;
-                    my_weight = 0.0f;
-                    if (!active || j >= valid) return;
-                    const uint32_t ri = __ldg(e.work.grouped_routes + first + j);
-                    if (gate_up) {
-                        my_row = __ldg(e.down_position + ri);
-                    } else {
-                        my_row = ri;
-                        my_weight = nvmoe_bf16_to_f32(__ldg(e.routes + ri) >> 16);
+                constexpr uint32_t phase = decltype(tag)::value;
+                const LayerPhase s = phase_of(phase);
+                const ExpertLaunch& e = p.stage[phase];
+                constexpr bool gate_up = phase == 0u;
+                for (uint32_t tile = id - phase * G; tile < s.tile_count; tile += G, acc_it++) {
+                    const uint32_t entry = __ldg(e.tile_list + tile / s.m_tiles), m_tile = tile % s.m_tiles, expert = entry >> 16;
+                    const uint32_t first = __ldg(e.work.expert_offsets + expert) + (entry & 0xffffu) * N_TILE;
+                    const uint32_t valid = min(N_TILE, __ldg(e.work.expert_offsets + expert + 1u) - first);
+                    const uint32_t acc = acc_it & 1u;
+                    // where token j of the tile goes (its row among the down operands, or its output row and weight): a chain of two
+                    // loads, over before the accumulator is ready for narrow tiles, a lane per token
+                    uint32_t my_row = kUnboundSlot;
+                    float my_weight = 0.0f;
+                    auto find = [&](uint32_t j, bool active) {
+                        my_row = kUnboundSlot;
+                        my_weight = 0.0f;
+                        if (!active || j >= valid) return;
+                        const uint32_t ri = __ldg(e.work.grouped_routes + first + j);
+                        if (gate_up) {
+                            my_row = __ldg(e.down_position + ri);
+                        } else {
+                            my_row = ri;
+                            my_weight = nvmoe_bf16_to_f32(__ldg(e.routes + ri) >> 16);
+                        }
+                    };
+                    constexpr bool kNarrow = N_TILE <= 32u;
+                    if (kNarrow) find(lane, true);
+                    // (one warp polls, the others sleep on a hardware barrier; every warp reaches it in every round)
+                    if (warp == kLayerWatchWarp) {
+                        const bool ready = mbar_wait_warp(&bars->acc_full[acc], (acc_it >> 1) & 1u, abort_flag, wait_limit);
+                        if (lane == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) = ready ? 1u : 0u;
+                        __threadfence_block();
                     }
-                };
-                constexpr bool kNarrow = N_TILE <= 32u;
-                if (kNarrow) find(lane, true);
-                // (one warp polls, the others sleep on a hardware barrier; every warp reaches it in every round)
-                if (warp == kLayerWatchWarp) {
-                    const bool ready = mbar_wait_warp(&bars->acc_full[acc], (acc_it >> 1) & 1u, abort_flag, wait_limit);
-                    if (lane == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) = ready ? 1u : 0u;
-                    __threadfence_block();
-                }
-                named_barrier(1u, 32u * kLayerEpilogueWarps);
-                if (*reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) == 0u) {
-                    alive = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t row = m_tile * (gate_up ? kBlockM : 2u * kBlockM) + quad * 32u + lane;
-                const bool row_ok = row < s.out_rows;
-                const uint32_t lane_addr = tmem_base + ((quad * 32u) << 16) + acc * C::kAccColumns;
-                // a narrow tile is shared out by sets of four tokens, a wide one by chunks of sixteen
-                for (uint32_t c0 = kNarrow ? 0u : 16u * group; c0 < valid; c0 += kNarrow ? 16u : 16u * kLayerGroups) {
-                    if (kNarrow) {
-                        bool mine = false;  // (uniform)
-#pragma unroll
-                        for (uint32_t g0 = 0; g0 < 16u; g0 += 4u) mine = mine || (c0 + g0 < valid && ((c0 + g0) / 4u) % kLayerGroups == group);
-                        if (!mine) continue;
+                    named_barrier(1u, 32u * kLayerEpilogueWarps);
+                    if (*reinterpret_cast<volatile uint32_t*>(&bars->acc_ready[acc]) == 0u) {
+                        alive = false;
+                        break;
                     }
-                    uint32_t d0[16], d1[16];
-                    tmem_ld16(lane_addr + c0, d0);
-                    tmem_ld16(lane_addr + N_TILE + c0, d1);  // up, or the second 128 rows
-                    if (!kNarrow) find(c0 + lane, lane < 16u);
-                    const uint32_t t0 = kNarrow ? c0 : 0u;  // the lane that knows token c0
-                    tmem_ld_wait();
+                    tc_fence_after();
+                    const uint32_t row = m_tile * (gate_up ? kBlockM : 2u * kBlockM) + quad * 32u + lane;
+                    const bool row_ok = row < s.out_rows;
+                    const uint32_t lane_addr = tmem_base + ((quad * 32u) << 16) + acc * C::kAccColumns;
+                    // a narrow tile is shared out by sets of four tokens, a wide one by chunks of sixteen
+                    for (uint32_t c0 = kNarrow ? 0u : 16u * group; c0 < valid; c0 += kNarrow ? 16u : 16u * kLayerGroups) {
+                        if (kNarrow) {
+                            bool mine = false;  // (uniform)
 #pragma unroll
-                    for (uint32_t g0 = 0; g0 < 16u; g0 += 4u) {
-                        if (c0 + g0 >= valid) break;  // uniform
-                        if (kNarrow && ((c0 + g0) / 4u) % kLayerGroups != group) continue;  // another group's
-                        if (!gate_up) {
+                            for (uint32_t g0 = 0; g0 < 16u; g0 += 4u) mine = mine || (c0 + g0 < valid && ((c0 + g0) / 4u) % kLayerGroups == group);
+                            if (!mine) continue;
+                        }
+                        uint32_t d0[16], d1[16];
+                        tmem_ld16(lane_addr + c0, d0);
+                        tmem_ld16(lane_addr + N_TILE + c0, d1);  // up, or the second 128 rows
+                        if (!kNarrow) find(c0 + lane, lane < 16u);
+                        const uint32_t t0 = kNarrow ? c0 : 0u;  // the lane that knows token c0
+                        tmem_ld_wait();
 #pragma unroll
-                            for (uint32_t t = 0; t < 4u; t++) {
-                                const float weight = __shfl_sync(0xffffffffu, my_weight, t0 + g0 + t);
-                                uint16_t* out = e.outputs + (size_t)__shfl_sync(0xffffffffu, my_row, t0 + g0 + t) * H;
-                                if (c0 + g0 + t < valid && row_ok)
-                                    out[row] = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(d0[g0 + t]), weight)));
-                                if (c0 + g0 + t < valid && row + kBlockM < s.out_rows)
-                                    out[row + kBlockM] = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(d1[g0 + t]), weight)));
+                        for (uint32_t g0 = 0; g0 < 16u; g0 += 4u) {
+                            if (c0 + g0 >= valid) break;  // uniform
+                            if (kNarrow && ((c0 + g0) / 4u) % kLayerGroups != group) continue;  // another group's
+                            if constexpr (gate_up) {
+                                // SwiGLU, then the activation quantisation of the down stage, as in experts_tc.cu (by one function for both,
+                                // layers with scale blocks of 128 took up to 1.3 % longer)
+                                uint32_t bits[4];
+#pragma unroll
+                                for (uint32_t t = 0; t < 4u; t++)
+                                    bits[t] = swiglu_bf16_bits(__uint_as_float(d0[g0 + t]), __uint_as_float(d1[g0 + t]), g.swiglu_limit, g.swiglu_alpha, g.swiglu_up_offset);
+                                float m[4];
+#pragma unroll
+                                for (uint32_t t = 0; t < 4u; t++) m[t] = row_ok ? fabsf(nvmoe_bf16_to_f32(bits[t])) : 0.0f;
+#pragma unroll
+                                for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                                    for (uint32_t t = 0; t < 4u; t++) m[t] = fmaxf(m[t], __shfl_xor_sync(0xffffffffu, m[t], o));
+                                }
+                                if (whole_block) {
+                                    // (a set's maxima are overwritten two sets later, when every warp has passed the barrier of the set between)
+                                    uint16_t(&quad_max)[4][4] = maxima[group][set_it++ & 1u];
+                                    if (lane < 4u)
+                                        quad_max[quad][lane] = (uint16_t)(__float_as_uint(lane == 0u ? m[0] : lane == 1u ? m[1] : lane == 2u ? m[2] : m[3]) >> 16);
+                                    named_barrier(2u + group, 128u);
+#pragma unroll
+                                    for (uint32_t t = 0; t < 4u; t++)
+                                        m[t] = fmaxf(fmaxf(fmaxf(0.0f, nvmoe_bf16_to_f32(quad_max[0][t])), nvmoe_bf16_to_f32(quad_max[1][t])),
+                                                     fmaxf(nvmoe_bf16_to_f32(quad_max[2][t]), nvmoe_bf16_to_f32(quad_max[3][t])));
+                                }
+                                const uint32_t first_row = m_tile * kBlockM + quad * 32u;
+                                const bool writes_scale = lane == 0u && first_row < s.out_rows;
+#pragma unroll
+                                for (uint32_t t = 0; t < 4u; t++) {
+                                    const uint32_t dp = __shfl_sync(0xffffffffu, my_row, t0 + g0 + t);
+                                    const float scale = nvmoe_rounded_fp8_scale(m[t]);
+                                    const float inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
+                                    const uint8_t q = (uint8_t)__nv_cvt_float_to_fp8(nvmoe_bf16_to_f32(bits[t]) * inv, __NV_SATFINITE, __NV_E4M3);
+                                    if (dp != kUnboundSlot) {  // (lanes past `valid` and routes the down stage skips)
+                                        if (row_ok) e.q_out[(size_t)dp * I + row] = q;
+                                        if (writes_scale) *e.q_e8m0.byte_at(dp, first_row / 32u) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
+                                    }
+                                }
+                            } else {
+#pragma unroll
+                                for (uint32_t t = 0; t < 4u; t++) {
+                                    const float weight = __shfl_sync(0xffffffffu, my_weight, t0 + g0 + t);
+                                    uint16_t* out = e.outputs + (size_t)__shfl_sync(0xffffffffu, my_row, t0 + g0 + t) * H;
+                                    if (c0 + g0 + t < valid && row_ok)
+                                        out[row] = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(d0[g0 + t]), weight)));
+                                    if (c0 + g0 + t < valid && row + kBlockM < s.out_rows)
+                                        out[row + kBlockM] = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(d1[g0 + t]), weight)));
+                                }
                             }
-                            continue;
-                        }
-                        // SwiGLU, then the activation quantisation of the down stage, as in experts_tc.cu
-                        uint32_t bits[4];
-                        float m[4];
-#pragma unroll
-                        for (uint32_t t = 0; t < 4u; t++)
-                            bits[t] = swiglu_bf16_bits(__uint_as_float(d0[g0 + t]), __uint_as_float(d1[g0 + t]), g.swiglu_limit, g.swiglu_alpha, g.swiglu_up_offset);
-#pragma unroll
-                        for (uint32_t t = 0; t < 4u; t++) m[t] = row_ok ? fabsf(nvmoe_bf16_to_f32(bits[t])) : 0.0f;
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                            for (uint32_t t = 0; t < 4u; t++) m[t] = fmaxf(m[t], __shfl_xor_sync(0xffffffffu, m[t], o));
-                        }
-                        if (whole_block) {
-                            // (a set's maxima are overwritten two sets later, when every warp has passed the barrier of the set between)
-                            uint16_t(&quad_max)[4][4] = maxima[group][set_it++ & 1u];
-                            if (lane < 4u)
-                                quad_max[quad][lane] = (uint16_t)(__float_as_uint(lane == 0u ? m[0] : lane == 1u ? m[1] : lane == 2u ? m[2] : m[3]) >> 16);
-                            named_barrier(2u + group, 128u);
-#pragma unroll
-                            for (uint32_t t = 0; t < 4u; t++)
-                                m[t] = fmaxf(fmaxf(fmaxf(0.0f, nvmoe_bf16_to_f32(quad_max[0][t])), nvmoe_bf16_to_f32(quad_max[1][t])),
-                                             fmaxf(nvmoe_bf16_to_f32(quad_max[2][t]), nvmoe_bf16_to_f32(quad_max[3][t])));
-                        }
-                        const uint32_t first_row = m_tile * kBlockM + quad * 32u;
-                        const bool writes_scale = lane == 0u && first_row < s.out_rows;
-#pragma unroll
-                        for (uint32_t t = 0; t < 4u; t++) {
-                            const uint32_t dp = __shfl_sync(0xffffffffu, my_row, t0 + g0 + t);
-                            const float scale = nvmoe_rounded_fp8_scale(m[t]);
-                            const float inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
-                            const uint8_t q = (uint8_t)__nv_cvt_float_to_fp8(nvmoe_bf16_to_f32(bits[t]) * inv, __NV_SATFINITE, __NV_E4M3);
-                            if (dp != kUnboundSlot) {  // (lanes past `valid` and routes the down stage skips)
-                                if (row_ok) e.q_out[(size_t)dp * I + row] = q;
-                                if (writes_scale) *e.q_e8m0.byte_at(dp, first_row / 32u) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
-                            }
                         }
                     }
+                    tc_fence_before();
+                    mbar_arrive(&bars->acc_empty[acc]);
+                    if (gate_up) {  // this warp's part of the tile is stored
+                        fence_proxy_async_all();
+                        __syncwarp();
+                        if (lane == 0u) add_release(p.sync + 1u + expert, 1u);
+                    }
                 }
-                tc_fence_before();
-                mbar_arrive(&bars->acc_empty[acc]);
-                if (gate_up) {  // this warp's part of the tile is stored
-                    fence_proxy_async_all();
-                    __syncwarp();
-                    if (lane == 0u) add_release(p.sync + 1u + expert, 1u);
-                }
-            }
             };
             if (id < G) {
                 run(PhaseTag<0u>{});
