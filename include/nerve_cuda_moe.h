@@ -403,9 +403,9 @@ enum { NVMOE_STAGE_LINEAR, NVMOE_STAGE_ROUTE, NVMOE_STAGE_SCHEDULE, NVMOE_STAGE_
        NVMOE_STAGE_COUNT };
 typedef struct nvmoe_work_report {
     float total_ms;                    /* see above */
-    float stage_ms[NVMOE_STAGE_COUNT]; /* zeros unless profiling is on */
-    float gate_up_kernel_ms;           /* the gate/up expert kernel alone (profiling on) */
-    float down_kernel_ms;              /* the down expert kernel alone (profiling on) */
+    float stage_ms[NVMOE_STAGE_COUNT]; /* zeros unless profiling is on, and was in that call */
+    float gate_up_kernel_ms;           /* the gate/up expert kernel alone (likewise) */
+    float down_kernel_ms;              /* the down expert kernel alone (likewise) */
     uint32_t tensor_path;              /* 1 when the expert kernels ran on tcgen05 */
     uint32_t batch_width;
     uint32_t routes;

@@ -152,6 +152,7 @@ struct nvmoe_plan {
     cudaEvent_t kernel_ev[2][2] = {};  // [gate_up, down][begin, end] around the expert kernel alone
     bool events_valid = false;
     bool clocked = false;        // the last layer call's time is in `clock`, else between the first and the last event
+    bool profiled = false;       // it has recorded the events of its stages
     DeviceArray clock;
     bool profile_stages = false;
     nvmoe_work_report report{};
@@ -1674,6 +1675,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     }
     mark(kStageCount);
     p->clocked = clock != nullptr;
+    p->profiled = prof;
     p->events_valid = true;
     p->report.batch_width = T;
     p->report.routes = T * p->K;
@@ -1871,12 +1873,13 @@ int nvmoe_plan_last_report(nvmoe_plan* p, nvmoe_work_report* report) {
     } else {
         NVMOE_CUDA(d, cudaEventElapsedTime(&p->report.total_ms, p->ev[0], p->ev[kStageCount]));
     }
+    const bool stages = p->profile_stages && p->profiled;  // (events that no call has recorded would leave an error for the next launch)
     for (int i = 0; i < kStageCount; i++) {
         p->report.stage_ms[i] = 0.0f;
-        if (p->profile_stages) cudaEventElapsedTime(&p->report.stage_ms[i], p->ev[i], p->ev[i + 1]);
+        if (stages) cudaEventElapsedTime(&p->report.stage_ms[i], p->ev[i], p->ev[i + 1]);
     }
     p->report.gate_up_kernel_ms = p->report.down_kernel_ms = 0.0f;
-    if (p->profile_stages) {
+    if (stages) {
         cudaEventElapsedTime(&p->report.gate_up_kernel_ms, p->kernel_ev[0][0], p->kernel_ev[0][1]);
         cudaEventElapsedTime(&p->report.down_kernel_ms, p->kernel_ev[1][0], p->kernel_ev[1][1]);
     }

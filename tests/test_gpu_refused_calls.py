@@ -39,3 +39,26 @@ def test_refused_layer_calls(profiled):
     plan.destroy()
     bank.destroy()
     device.close()
+
+
+def test_profiling_turned_on_after_the_call():
+    """A report asked for with profiling on, after a call without it, has no stage times and leaves no error behind."""
+    device = CudaComputeDevice(0)
+    tokens = 9
+    cfg = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 256, 128, 16)
+    case = synthetic.make_case(cfg, tokens, seed=59)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, out = device.resident_buffer_from(case.hidden), device.create_resident_buffer(tokens * cfg.hidden * 2)
+    rw = device.resident_buffer_from(case.router_w)
+    for profiled, asked in ((False, True), (True, True), (True, False), (False, True), (False, False)):
+        plan.set_profiling(profiled)
+        plan.layer(tokens, bank, hidden, out, router_weights=rw)
+        plan.set_profiling(asked)
+        report = plan.last_report()
+        times = [*report["stage_ms"].values(), report["gate_up_kernel_ms"], report["down_kernel_ms"]]
+        assert any(times) == (profiled and asked) and report["total_ms"] > 0.0
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
+    device.close()
