@@ -398,6 +398,21 @@ def test_dense_linear_operands(device, block, shift, rows, cols, tokens):
     plan.destroy()
 
 
+# matrices of so many rows that their 16-token tiles take two row tiles at a time: the last that do not (73 pairs of 128 rows), the first, with
+# a lone last half, and whole pairs; a K tail
+@pytest.mark.parametrize("rows,cols,tokens", [(18688, 352, 12), (18720, 352, 12), (18944, 256, 3), (18944, 128, 1)])
+def test_dense_linear_of_many_rows(device, rows, cols, tokens):
+    rng = np.random.default_rng(rows + cols)
+    plan = plan_of(device, act_block=32, tokens=16)
+    x = bf16(rng.standard_normal((tokens, cols)))
+    w, s = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8), rng.integers(118, 128, (rows, cols // 32), dtype=np.uint8)
+    ob = device.create_resident_buffer(tokens * rows * 2)
+    plan.dense_linear(tokens, device.resident_buffer_from(x), ob, device.resident_buffer_from(w), device.resident_buffer_from(s), rows, cols)
+    assert_close(ob.read(np.uint16).reshape(tokens, rows), mo.dense_linear_mxfp4(x, w, s, 32, tier=1))
+    assert plan.status() == 0
+    plan.destroy()
+
+
 # every token tile from one plan: a call has the tensor maps of its tile whatever the plan's largest call is (boxes of one K
 # block and of two, whole pairs of blocks and a trailing half; one-byte weights)
 @pytest.mark.parametrize("name,shape,native", [("gpt-oss-20b", (576, 512, 8), 0), ("deepseek-v3", (512, 384, 16), 1)])
