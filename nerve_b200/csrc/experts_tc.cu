@@ -1318,9 +1318,9 @@ void tc_configure_kernels() {
 //   launch: 16 gate/up tiles (tiny, 8 tokens) 22.0 us by two launches / 23.3, 32 (64 tokens) 25.2 / 28.0, 92 (one token of 32 experts of
 //   2880 x 2880) 38.9 / 40.7.
 // - Beyond 1.6 rounds, K of gate/up is long enough: 12 stages for tiles of 16 tokens, for wider ones 18 and one for every twenty tokens of an
-//   expert. The one kernel's epilogue takes longer than that of the two (a further polling warp beside it; a warp of its own for the
-//   announcements made it no better), and only the stages of the next tile hide that. Layers, two / one, us: 16-token tiles, 4 stages (512 x
-//   4096, 32 experts) 49.7 / 63.7, 6 (768 x 3072, 64) 75.1 / 83.0, 12 (1536 x 768, 128, one token each) 58.9 / 57.1, 16 (2048 x 1536, 64)
+//   expert. Short K loses by the one kernel, the more the more tokens a tile has, as if its epilogue took longer than that of the two and
+//   the stages of the next tile alone hid it (announcements by a warp of their own made it no better). Layers, two / one, us: 16-token
+//   tiles, 4 stages (512 x 4096, 32 experts) 49.7 / 63.7, 6 (768 x 3072, 64) 75.1 / 83.0, 12 (1536 x 2048, 128, 64 tokens) 120.6 / 114.3, 16 (2048 x 1536, 64)
 //   86.3 / 78.8; 32 tokens, 12 stages (1536 x 2304, 32) 64.8 / 70.8, 23 (2880 x 2880, 32) 114.6 / 101.4; 64, 12 stages (1536 x 768, 128) 112.6 /
 //   121.3, 23 128.3 / 120.9; 96, 12 stages 182.7 / 203.8, 16 (2048 x 1536, 64) 157.3 / 172.5, 23 180.2 / 172.5.
 // - K of down is at least eight stages, or that of gate/up 32 with tiles of 64 tokens or more, and the down tiles of 256 rows fill the SMs:
