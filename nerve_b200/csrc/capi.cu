@@ -675,11 +675,11 @@ static int check_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hi
 }
 
 static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
-                         const nvmoe_buffer* router_bias, CallClock* clock) {
+                         const nvmoe_buffer* router_bias, const CallStart& start) {
     const nvmoe_geometry& g = p->g;
     launch_router_linear((const uint16_t*)hidden->ptr, (const uint16_t*)router_weights->ptr,
                          router_bias ? (const uint16_t*)router_bias->ptr : nullptr, (uint32_t*)logits->ptr, T,
-                         g.hidden_size, g.routed_experts, clock, p->device->stream);
+                         g.hidden_size, g.routed_experts, start, p->device->stream);
     p->launches++;
     return post_launch(p, "router projection");
 }
@@ -689,7 +689,7 @@ int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, n
     if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
     NVMOE_TRY(check_router_linear(p, T, hidden, logits, router_weights, router_bias));
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
-    return router_linear(p, T, hidden, logits, router_weights, router_bias, nullptr);
+    return router_linear(p, T, hidden, logits, router_weights, router_bias, CallStart{});
 }
 
 // checks the router's buffers and fills its launch block
@@ -1535,28 +1535,6 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     NVMOE_TRY(expert_set_for(p, 0, a->gate_up_addresses, a->gate_up_slots, tensor, &sets[0]));
     NVMOE_TRY(expert_set_for(p, 1, a->down_addresses, a->down_slots, tensor, &sets[1]));
 
-    if (host && host->address) {
-        launch_fetch_host(host->address, host->device, host->bytes, st);
-        p->launches++;
-        NVMOE_TRY(post_launch(p, "fetch hidden"));
-    } else if (host) {
-        NVMOE_CUDA(d, cudaMemcpyAsync(host->device, host->rows, host->bytes, cudaMemcpyHostToDevice, st));
-    }
-    const uint32_t launches_before = p->launches;
-    mark(kStageLinear);
-    if (projects) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, clock));
-    mark(kStageRoute);
-    // (with stage profiling on, the router keeps a launch and a time of its own)
-    bool routes_in_schedule = false;
-    if (!a->routes_in) {
-        routes_in_schedule = !prof && layer_routes_in_schedule(router, p->K, p->experts);
-        if (!routes_in_schedule) {
-            launch_router(router, st);
-            p->launches++;
-            NVMOE_TRY(post_launch(p, "router"));
-        }
-    }
-    mark(kStageSchedule);
     // with scale blocks of 32 or 128 (what a warp, or the four warps of an epilogue group, hold of a token) the tensor-path
     // gate/up epilogue quantises its own output for the down stage
     const bool fused_quantise = tensor && (g.act_block == 32u || g.act_block == 128u) &&
@@ -1564,14 +1542,8 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     // Narrow tiles: both expert stages in one launch. (A stage that is timed, traced or given out by itself keeps its own.)
     const bool fused_schedule = layer_schedule_is_fused(T, p->K, p->experts, a->expert_count != 0u);
     const bool one_launch = fused_quantise && fused_schedule && !prof && !p->cta_trace.ptr && !a->expert_outputs && layer_in_one_launch(p, T);
-    NVMOE_TRY(fill_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, sets[0]));
-    NVMOE_TRY(fill_expert_set(p, false, a->down_addresses, a->down_slots, tensor, sets[1]));
+    LayerSchedule ls{};
     if (fused_schedule) {
-        LayerSchedule ls{};
-        if (one_launch) {
-            ls.clear = p->layer_sync.as<uint32_t>();
-            ls.clear_words = p->experts + 1u;
-        }
         ls.routes = (const uint32_t*)routes->ptr;
         ls.intermediates = (uint32_t*)frames.ptr;
         ls.slots[0] = (const uint32_t*)a->gate_up_slots->ptr;
@@ -1599,7 +1571,56 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         ls.num_experts = p->experts;
         ls.n_tile[0] = token_tile(p, true, T).rows;
         ls.n_tile[1] = token_tile(p, false, T).rows;
-        if (routes_in_schedule) {
+    }
+    const bool routes_in_schedule = !a->routes_in && !prof && layer_routes_in_schedule(router, p->K, p->experts);
+    // Small calls: the gate/up operands beside the schedule. (`early`: the projection, or a router with a launch of its own, is then ahead)
+    OperandRows rows{};
+    rows.input = (const uint16_t*)a->hidden->ptr;
+    rows.cols = g.hidden_size;
+    rows.chunks = (g.hidden_size + 511u) / 512u;
+    rows.q = p->grouped_q[0].as<uint8_t>();
+    rows.scales = scale_words(p, true, T);
+    rows.down.q = p->grouped_q[1].as<uint8_t>();
+    rows.down.scales = scale_words(p, false, T);
+    rows.down.cols = g.intermediate_size;
+    rows.early = projects || (!a->routes_in && !routes_in_schedule);
+    const bool beside = fused_quantise && fused_schedule && !prof && places_operands(ls, routes_in_schedule, rows, g.act_block);
+    // The counters of the one launch for both expert stages are cleared two launches before it, or else it counts after its wait.
+    CallStart start{clock, nullptr, 0u};
+    if (one_launch && beside && projects) {
+        start.clear = p->layer_sync.as<uint32_t>();
+        start.clear_words = p->experts + 1u;
+    } else if (one_launch) {
+        ls.clear = p->layer_sync.as<uint32_t>();
+        ls.clear_words = p->experts + 1u;
+    }
+
+    if (host && host->address) {
+        launch_fetch_host(host->address, host->device, host->bytes, st);
+        p->launches++;
+        NVMOE_TRY(post_launch(p, "fetch hidden"));
+    } else if (host) {
+        NVMOE_CUDA(d, cudaMemcpyAsync(host->device, host->rows, host->bytes, cudaMemcpyHostToDevice, st));
+    }
+    const uint32_t launches_before = p->launches;
+    mark(kStageLinear);
+    if (projects) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, start));
+    mark(kStageRoute);
+    // (with stage profiling on, the router keeps a launch and a time of its own)
+    if (!a->routes_in && !routes_in_schedule) {
+        launch_router(router, st);
+        p->launches++;
+        NVMOE_TRY(post_launch(p, "router"));
+    }
+    mark(kStageSchedule);
+    NVMOE_TRY(fill_expert_set(p, true, a->gate_up_addresses, a->gate_up_slots, tensor, sets[0]));
+    NVMOE_TRY(fill_expert_set(p, false, a->down_addresses, a->down_slots, tensor, sets[1]));
+    if (fused_schedule) {
+        if (beside) {
+            launch_place_operands(routes_in_schedule ? &router : nullptr, ls, rows, g.act_block, st);
+            launch_small_schedule(routes_in_schedule ? &router : nullptr, ls, st);
+            p->launches += 2;
+        } else if (routes_in_schedule) {
             launch_route_schedule(router, ls, st);
             p->launches++;
         } else {
@@ -1621,7 +1642,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     }
     mark(kStageQuantX);
     // (this launch also keeps the one for both expert stages, which counts before it waits, apart from the schedule, which clears the counters)
-    NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true, fused_quantise));
+    if (!beside) NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true, fused_quantise));
     mark(kStageGateUp);
     ExpertCall call;
     call.T = T;
@@ -1644,6 +1665,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
             ll.stage[i].scale_base = sets[i]->derived.as<uint8_t>();
         }
         ll.sync = p->layer_sync.as<uint32_t>();
+        ll.claim_late = beside && !projects;
         launch_layer_tc(ll, st);
         p->report.tensor_path = 1u;
         p->launches++;

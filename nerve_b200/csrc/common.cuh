@@ -21,9 +21,9 @@ constexpr uint32_t kMaxExperts = 4096u;  // ids travel in the low 16 bits of a r
 // before any return, so completion still implies that all earlier kernels have completed, and before
 // touching global memory that the launch ahead of it may write or read. What stands before the call may
 // rely on the launches before that one: the kernel ahead let this one start after its own wait, when they
-// had completed. (Tensor maps and expert tables are read there, and experts_layer.cu claims its first work
-// from a counter that the launch before the one ahead cleared: no kernel may let the next start before its wait, and a
-// launch has to stay between those two.) Launched the ordinary way, the same kernels run unchanged.
+// had completed. (Tensor maps and expert tables are read there, place_operands_kernel reads the tokens, the schedule behind that one does
+// all of its work, and experts_layer.cu claims its first work from a counter that a launch before the one ahead cleared: no other kernel
+// may let the next start before its wait, and a launch has to stay between those two.) Launched the ordinary way, the same kernels run unchanged.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_dependency_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -100,10 +100,19 @@ __device__ __forceinline__ unsigned long long device_clock_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ void note_begin(CallClock* clock) {
-    if (clock == nullptr || (blockIdx.x | blockIdx.y | threadIdx.x) != 0u) return;
-    clock->begin = device_clock_ns();
-    clock->end = 0u;
+// What a layer call's first kernel does beside its own work: it notes the time (clock null: not), and zeroes words that a later kernel of the
+// call counts in, where that one counts before the launch ahead of it is through.
+struct CallStart {
+    CallClock* clock;
+    uint32_t* clear;
+    uint32_t clear_words;
+};
+__device__ __forceinline__ void begin_call(const CallStart& start) {
+    if ((blockIdx.x | blockIdx.y) != 0u) return;
+    for (uint32_t w = threadIdx.x; w < start.clear_words; w += blockDim.x) start.clear[w] = 0u;
+    if (start.clock == nullptr || threadIdx.x != 0u) return;
+    start.clock->begin = device_clock_ns();
+    start.clock->end = 0u;
 }
 __device__ __forceinline__ void note_end(CallClock* clock) {
     if (clock != nullptr && threadIdx.x == 0u) atomicMax(&clock->end, device_clock_ns());
@@ -145,7 +154,7 @@ void configure_router_kernels();
 void launch_router(const RouterLaunch& p, cudaStream_t stream);
 bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selections, no groups: route_token covers it
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
-                          uint32_t tokens, uint32_t hidden, uint32_t outputs, CallClock* clock, cudaStream_t stream);
+                          uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream);
 
 struct SortScratch {  // schedule.cu: scratch of the counting sort, sized for max_tokens
     uint32_t* block_hist;      // [blocks][buckets]
@@ -189,6 +198,28 @@ struct LayerSchedule {
     uint32_t* clear;       // words that a later kernel of the call counts in, to be zeroed
     uint32_t clear_words;
 };
+// The down stage's operand rows, of which those of routes that only the down stage keeps are set to zero (q null: none).
+struct DownRows {
+    const uint32_t* position;  // [route] (null where the places come from elsewhere)
+    uint8_t* q;
+    ScaleWords scales;
+    uint32_t cols;
+};
+// The gate/up operands of a small call, made ahead of its schedule: a launch that counts the places of its rows itself.
+struct OperandRows {
+    const uint16_t* input;  // [tokens][cols]
+    uint32_t cols, chunks;  // (chunks of 512 columns a row)
+    uint8_t* q;
+    ScaleWords scales;
+    DownRows down;
+    bool early;             // the launch ahead has waited for whatever writes the input
+};
+bool places_operands(const LayerSchedule& s, bool routed, const OperandRows& o, uint32_t block);  // whether a call's are
+// (router: the tokens are routed here too, else by a launch ahead)
+void launch_place_operands(const RouterLaunch* router, const LayerSchedule& s, const OperandRows& o, uint32_t block, cudaStream_t stream);
+// ... and, right behind it, what the later kernels of the call read of its schedule: offsets, grouped routes, positions and tiles of both
+// stages, but neither the compact list nor the control words. (tiles, position and so on are all set)
+void launch_small_schedule(const RouterLaunch* router, const LayerSchedule& s, cudaStream_t stream);
 bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, bool partitioned);
 // the router and the schedule of a call of up to 16 tokens (32 of up to 32 experts) in one launch
 bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts);
@@ -237,15 +268,8 @@ void launch_quantize_grouped(const void* input, bool frames, const uint32_t* gro
                              uint32_t cols, uint32_t intermediate_size, uint32_t block, uint8_t* q,
                              const ScaleWords& scales, const uint32_t* written, cudaStream_t stream);
 // The same gate/up operands from the inverse list: position[token * K + r] = row of that route (0xffffffff: skipped),
-// valid for every route of the call. `down` (position null: nothing) names the down stage's operand rows, of which those
-// of routes that only the down stage keeps are set to zero. False when the shape needs the form above (blocks other than
+// valid for every route of the call; `down` (position null: nothing). False when the shape needs the form above (blocks other than
 // 32 or 128 columns, input not 16-byte aligned).
-struct DownRows {
-    const uint32_t* position;
-    uint8_t* q;
-    ScaleWords scales;
-    uint32_t cols;
-};
 bool launch_quantize_tokens(const void* input, const uint32_t* position, uint32_t tokens, uint32_t K, uint32_t cols, uint32_t block,
                             uint8_t* q, const ScaleWords& scales, const DownRows& down, cudaStream_t stream);
 // the same for the K rows of every intermediates frame (skips the schedule words)

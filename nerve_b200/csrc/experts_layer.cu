@@ -16,7 +16,7 @@
 //
 // Hand-over.  A gate/up epilogue warp counts itself into its expert's counter (release) when its part of the tile is stored; the
 // warp that fetches a down tile's token rows and scales waits until the counter holds all of the expert's tiles (acquire, and a
-// proxy fence: the rows are written by threads and read by the TMA unit). The call's schedule clears the counters.
+// proxy fence: the rows are written by threads and read by the TMA unit). The call's projection or schedule clears the counters.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -142,16 +142,17 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         __syncthreads();
     };
     // What is read, and counted, before the wait: what stands since earlier calls, or since a launch of this one that had completed
-    // when the kernel ahead let this one start. That one waited for all before it, the schedule (which cleared the counters) among
-    // them: a launch has to stay between the schedule and this one (the quantisation is), or the claim has to follow the wait.
+    // when the kernel ahead let this one start. That one waited for all before it, the one that cleared the counters among them (the
+    // projection, or the schedule where the quantisation is a launch of its own); where it clears them itself, the claim follows the wait.
     uint32_t claimed = 0u;
-    if (warp == 7u && lane == 0u) claimed = atomicAdd(p.sync, 1u);
+    if (warp == 7u && lane == 0u && !p.claim_late) claimed = atomicAdd(p.sync, 1u);
     for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) {
         const bool bytes = (m < experts ? p.stage[0].work.experts[m].format : p.stage[1].work.experts[m - experts].format) != kFormatCompact;
         if (bytes) atomicOr(&bars->bytes_form[m / 32u], 1u << (m % 32u));
     }
     acquire_maps();
     grid_dependency_sync();
+    if (warp == 7u && lane == 0u && p.claim_late) claimed = atomicAdd(p.sync, 1u);
     const uint32_t entries[2] = {*p.stage[0].tile_count, *p.stage[1].tile_count};
     auto phase_of = [&](uint32_t phase) {
         LayerPhase s;

@@ -85,7 +85,8 @@ void launch_derive_scales_tc(const ExpertLaunch& p, bool gate_up, cudaStream_t s
 // the down operands made by gate/up.
 struct LayerLaunch {
     ExpertLaunch stage[2];
-    uint32_t* sync;    // experts + 1 words, cleared by the schedule: chunks claimed, per expert the warps done with its gate/up tiles
+    uint32_t* sync;    // experts + 1 words, cleared earlier in the call: chunks claimed, per expert the warps done with its gate/up tiles
+    bool claim_late;   // the launch right before this one clears them
 };
 constexpr uint32_t kLayerExperts = 1024u;  // at most
 void layer_configure_kernels();

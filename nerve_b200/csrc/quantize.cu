@@ -186,12 +186,7 @@ __global__ void __launch_bounds__(128) quantize_tokens_kernel(const uint16_t* __
             const uint32_t row = __shfl_sync(0xffffffffu, mine, r);
             if (row == kUnboundSlot) {  // a route that the stage skips
                 const uint32_t down_row = __shfl_sync(0xffffffffu, mine_down, r);
-                if (down_row != kUnboundSlot) {
-                    for (uint32_t c = lane * 16u; c < down.cols; c += 512u)
-                        *reinterpret_cast<uint4*>(down.q + (size_t)down_row * down.cols + c) = make_uint4(0u, 0u, 0u, 0u);
-                    const uint32_t down_words = (down.cols + 127u) / 128u;
-                    for (uint32_t c = lane; c < down_words; c += 32u) *down.scales.at(down_row, c) = 0x7f7f7f7fu;
-                }
+                if (down_row != kUnboundSlot) zero_down_row(down, down_row, lane);
                 continue;
             }
             if (!active) continue;

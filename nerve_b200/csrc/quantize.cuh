@@ -43,5 +43,13 @@ __device__ __forceinline__ void quantize_sixteen(const uint16_t* src, bool activ
     word |= __shfl_xor_sync(0xffffffffu, word, 4);
 }
 
+// By a warp: the down operands of a route that only the down stage keeps, as if its gate/up frame had never been written.
+__device__ __forceinline__ void zero_down_row(const DownRows& down, uint32_t row, uint32_t lane) {
+    for (uint32_t c = lane * 16u; c < down.cols; c += 512u)
+        *reinterpret_cast<uint4*>(down.q + (size_t)row * down.cols + c) = make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t words = (down.cols + 127u) / 128u;
+    for (uint32_t c = lane; c < words; c += 32u) *down.scales.at(row, c) = 0x7f7f7f7fu;
+}
+
 }  // namespace
 }  // namespace nvmoe

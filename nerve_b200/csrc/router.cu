@@ -256,11 +256,11 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
                                                            const uint16_t* __restrict__ w,
                                                            const uint16_t* __restrict__ bias,
                                                            uint32_t* __restrict__ logits, uint32_t tokens,
-                                                           uint32_t hidden, uint32_t outputs, CallClock* clock) {
+                                                           uint32_t hidden, uint32_t outputs, CallStart start) {
     __shared__ float fold[TT * ET][32];
     __shared__ float result[TT * ET];
     grid_dependency_sync();
-    note_begin(clock);
+    begin_call(start);
     const uint32_t v = threadIdx.x;
     const uint32_t t0 = blockIdx.y * TT, e0 = blockIdx.x * ET;
     const uint32_t words = hidden / 2u;
@@ -358,11 +358,11 @@ __global__ void __launch_bounds__(256, 1) router_linear_tiled_kernel(const uint1
                                                                     const uint16_t* __restrict__ w,
                                                                     const uint16_t* __restrict__ bias,
                                                                     uint32_t* __restrict__ logits, uint32_t tokens,
-                                                                    uint32_t hidden, uint32_t outputs, CallClock* clock) {
+                                                                    uint32_t hidden, uint32_t outputs, CallStart start) {
     extern __shared__ __align__(16) uint32_t stage[];  // [buffer][token rows, then output rows][word of the chunk]
     __shared__ float result[kTileTokens][kTileOutputs];
     grid_dependency_sync();
-    note_begin(clock);
+    begin_call(start);
     const uint32_t warp = threadIdx.x >> 5, l = threadIdx.x & 31u;
     const uint32_t t0 = blockIdx.y * kTileTokens, e0 = blockIdx.x * kTileOutputs;
     const uint32_t h = warp & 1u;  // lanes l + 32 h of the shader
@@ -525,7 +525,7 @@ void launch_router(const RouterLaunch& p, cudaStream_t stream) {
 }
 
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
-                          uint32_t tokens, uint32_t hidden, uint32_t outputs, CallClock* clock, cudaStream_t stream) {
+                          uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream) {
     if (tokens <= 256u) {
         const dim3 grid((outputs + 3u) / 4u, (tokens + 1u) / 2u), wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
         // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, but an
@@ -536,23 +536,23 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         // 231.5. By itself at 8.4 blocks 9.8 / 9.1 (hidden 512) and 20.1 / 18.4 (2880), at 9.1 39.6 / 41.8 (7168).
         const uint32_t blocks = wide.x * wide.y;
         if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
-            launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+            launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else if (grid.x * grid.y <= 4u * 148u && (hidden > 2048u || (hidden > 1024u && grid.x * grid.y <= 148u))) {
             // Few blocks of long rows: a call waits for the latency of their loads, so that 24 steps (of 128 columns) are under way instead of 8,
             // which shorter rows gain from only where an SM has one block. Layers, us, 8 / 24: one token of 32 experts of 2880 columns 29.4 / 28.6,
             // 64 tokens (256 blocks) 38.2 / 37.8, 100 45.6 / 44.9; of 2304 27.9 / 27.1, 34.5 / 34.0, 40.9 / 40.3; of 2048 27.0 / 26.8, 32.4 / 32.5, 37.6 /
             // 37.6; of 1536 25.6 / 25.1, 30.2 / 30.5, 33.2 / 33.8; of 1088 24.6 / 24.1, 28.8 / 28.9, 31.8 / 32.3; 16 tokens (64 blocks) 26.7 / 26.5; rows
             // of 512, which are four steps, 25.1 / 25.5. Beyond four blocks an SM 24 steps lose: 64 tokens of 128 experts of 2880 columns 64.1 / 65.9.
-            launch_chained(router_linear_kernel<2, 4, 24>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+            launch_chained(router_linear_kernel<2, 4, 24>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else {
-            launch_chained(router_linear_kernel<2, 4, 8>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+            launch_chained(router_linear_kernel<2, 4, 8>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         }
     } else if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u) {
         dim3 grid((outputs + kTileOutputs - 1u) / kTileOutputs, (tokens + kTileTokens - 1u) / kTileTokens);
-        launch_chained(router_linear_tiled_kernel, grid, dim3(256), kRouterTileBytes, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+        launch_chained(router_linear_tiled_kernel, grid, dim3(256), kRouterTileBytes, stream, x, w, bias, logits, tokens, hidden, outputs, start);
     } else {
         dim3 grid((outputs + 15u) / 16u, (tokens + 3u) / 4u);
-        launch_chained(router_linear_kernel<4, 16, 2>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, clock);
+        launch_chained(router_linear_kernel<4, 16, 2>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
     }
 }
 

@@ -59,15 +59,14 @@ __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uin
 // does through shared memory by one lane (the weights, the ascending order, packing, telemetry) is done by the
 // lanes side by side. Every sum that has an order keeps it (values travel by shuffle and are added in the same
 // sequence); the results are bit for bit those of router_kernel, which remains for the other cases. Called by a whole warp.
+//
+// The selection: lane r receives selection r (expert and activated value). False if there are fewer than k selectable scores.
 template <int EPL, bool GROUPS>
-__device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token) {
+__device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t token, uint32_t& my_e, float& my_v) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t E = p.g.routed_experts;
     const uint32_t k = p.g.routed_k;
     const uint32_t kind = p.g.router_kind;
-    const uint32_t always = kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
-    const uint32_t total_k = k + always;
-    const uint32_t total_resources = E + always;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t* row = p.logits + (size_t)token * ((E + 1u) / 2u);
 
@@ -123,7 +122,9 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
     }
 
     // ---- k rounds of arg-max: lane r keeps selection r ---------------------------------------
-    uint32_t taken = 0u, my_e = kUnboundSlot;
+    uint32_t taken = 0u;
+    my_e = kUnboundSlot;
+    my_v = 0.0f;
     if (GROUPS) {
         // a group's score is the sum of its two best; the experts of the groups outside the topk_group best count as taken
         const uint32_t per = E / p.g.n_group, side = 32u / per;  // groups in a register slot of the warp
@@ -151,8 +152,6 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
             if (group >= 32u || ((kept >> group) & 1u) == 0u) taken |= 1u << j;
         }
     }
-    float my_v = 0.0f;
-    bool missing = false;
     for (uint32_t r = 0; r < k; r++) {
         float best = kNegInf, best_v = 0.0f;
         uint32_t best_e = kUnboundSlot;
@@ -166,10 +165,7 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
             }
         }
         const uint32_t winner = warp_best(best, best_e);
-        if (winner == kUnboundSlot) {
-            missing = true;
-            break;
-        }
+        if (winner == kUnboundSlot) return false;
         // the winner is the best candidate of the lane that owns it
         const float winner_v = __shfl_sync(kFull, best_v, winner & 31u);
         if (lane == (winner & 31u)) taken |= 1u << (winner >> 5);
@@ -178,13 +174,55 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
             my_v = winner_v;
         }
     }
+    return true;
+}
+
+// The places of a token's selections in ascending order of the experts: lane r < total_k holds selection r.
+__device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total_k) {
+    uint32_t rank = 0u;
+    for (uint32_t q = 0; q < total_k; q++) {
+        const uint32_t other = __shfl_sync(0xffffffffu, my_e, q);
+        if (other < my_e) rank++;
+    }
+    return rank;
+}
+
+// Lane r < total_k receives the expert and the place of one of the token's route words, as route_token writes them.
+template <int EPL>
+__device__ __forceinline__ void select_ascending(const RouterLaunch& p, uint32_t token, uint32_t& my_e, uint32_t& rank) {
+    const uint32_t lane = threadIdx.x & 31u, k = p.g.routed_k, always = p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
+    float v;
+    if (!select_experts<EPL, false>(p, token, my_e, v)) {  // words of zeros
+        my_e = 0u;
+        rank = lane;
+        return;
+    }
+    if (lane >= k) my_e = p.g.routed_experts + (lane - k);
+    rank = ascending_rank(my_e, k + always);
+}
+
+// Selection, weights, route words and telemetry of a token; my_e and rank as above.
+template <int EPL, bool GROUPS>
+__device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token, uint32_t& my_e, uint32_t& rank) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t E = p.g.routed_experts;
+    const uint32_t k = p.g.routed_k;
+    const uint32_t kind = p.g.router_kind;
+    const uint32_t always = kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
+    const uint32_t total_k = k + always;
+    const uint32_t total_resources = E + always;
+    const uint32_t lane = threadIdx.x & 31u;
+    float my_v;
+    const bool found = select_experts<EPL, GROUPS>(p, token, my_e, my_v);
     uint32_t* out = p.routes + (size_t)token * total_k;
-    if (missing) {
+    if (!found) {
         // no selectable score (NaN logits): fail closed instead of indexing out of bounds
         if (lane == 0u) {
             for (uint32_t r = 0; r < total_k; r++) out[r] = 0u;
             raise_status(p.status, NVMOE_STATUS_ROUTE_NONFINITE);
         }
+        my_e = 0u;
+        rank = lane;
         return;
     }
 
@@ -210,11 +248,7 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
     }
 
     // ---- ascending expert id, pack, telemetry ----------------------------------------------------
-    uint32_t rank = 0u;
-    for (uint32_t q = 0; q < total_k; q++) {
-        const uint32_t other = __shfl_sync(kFull, my_e, q);
-        if (other < my_e) rank++;
-    }
+    rank = ascending_rank(my_e, total_k);
     if (lane < total_k) {
         out[rank] = (nvmoe_f32_to_bf16(w) << 16) | my_e;
         if (p.telemetry) atomicAdd(p.telemetry + my_e, 1u);
@@ -228,6 +262,12 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
             }
         }
     }
+}
+
+template <int EPL, bool GROUPS>
+__device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token) {
+    uint32_t e, rank;
+    route_token<EPL, GROUPS>(p, token, e, rank);
 }
 
 }  // namespace

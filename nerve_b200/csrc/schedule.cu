@@ -11,6 +11,7 @@
 // experts keep source order (warp match + popcount of lower lanes, warps taken in order).
 // Route ids at or above the expert count cannot be produced by the routers here; they are placed
 // after every valid id in source order (the reference would order them by id).
+#include "quantize.cuh"
 #include "router_reg.cuh"
 
 namespace nvmoe {
@@ -699,6 +700,9 @@ __host__ __device__ inline size_t layer_schedule_rank_smem_bytes(uint32_t count,
     return ((warps * columns + 1u) / 2u + 7u * (columns + 1u) + 2u) * sizeof(uint32_t) + 2u * columns;
 }
 
+// words for the places of the routes of the tokens that a block of so many warps, each with one of a token's `chunks` of columns, can meet
+__host__ __device__ inline uint32_t place_words(uint32_t warps, uint32_t chunks, uint32_t K) { return ((warps + chunks - 2u) / chunks + 1u) * K; }
+
 // `before` runs once the table has been cleared: the wait for the kernel before this one, or that and the routing.
 template <uint32_t CHUNKS, class BeforeFn>
 __device__ __forceinline__ void layer_schedule_rank_body(const LayerSchedule& s, BeforeFn before) {
@@ -871,6 +875,179 @@ __global__ void __launch_bounds__(1024) route_schedule_kernel(RouterLaunch route
         const uint32_t token = threadIdx.x >> 5;
         if (token < router.tokens) route_token<EPL, false>(router, token);
     });
+}
+
+// ---- small calls: operands and schedule side by side -------------------------------------------------------
+// A layer call of at most 1024 routes of all experts, a route a thread: the gate/up operands (place_operands_kernel) are made ahead of the
+// schedule (small_schedule_kernel) instead of behind it, and the two run at the same time.
+//
+// What a block of operands has to know of the schedule are the places of its own tokens' routes, which it counts itself: a place is the number
+// of kept routes that come before by (expert, route index). The rows are read and quantised before the wait where the launches ahead allow it
+// (`early`); after it a block loads the route words, counts and stores. Where the call's tokens are routed here too (EPL != 0), every block
+// selects the experts of all of them from the logits, and the first one also writes the route words.
+//
+// Both are bound by latency. In turn, the quantisation added a hand-over, two dependent loads and the rows' fetch to the schedule. Layers, us,
+// in turn / side by side: 64 tokens of the tiny layer 24.4 / 23.1; 32 experts of 2880 x 2880, one token 37.0 / 35.0, seven 67.1 / 63.7, 64 94.8 / 92.1, 32 from
+// host buffers 121.0 / 118.0; 96 of 257 of 7168 x 2048 749 / 737.
+template <int EPL, uint32_t LANES>
+__global__ void __launch_bounds__(1024) place_operands_kernel(RouterLaunch router, LayerSchedule s, OperandRows o) {
+    extern __shared__ uint32_t smem_words[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t count = s.tokens * s.K, first = blockIdx.x * warps, item = first + warp;
+    const uint32_t token = item / o.chunks, col = (item % o.chunks) * 512u + lane * 16u;
+    const bool active = token < s.tokens && col < o.cols;  // (columns come in whole blocks: the lanes of a block agree)
+    uint32_t out[4], word;
+    if (o.early) quantize_sixteen<LANES>(o.input + (size_t)token * o.cols + col, active, lane, out, word);
+    // per stage (expert << 16 | route) of every route that the stage keeps, all ones above the route of the others: their order is the grouping's
+    uint32_t* keys[2] = {smem_words, smem_words + count};
+    uint32_t* places[2] = {smem_words + 2u * count, smem_words + 2u * count + place_words(warps, o.chunks, s.K)};
+    auto list_route = [&](uint32_t i, uint32_t e) {
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++)
+            keys[stage][i] = (e < s.num_experts && s.experts[stage][e].w[0] != nullptr ? e << 16 : 0xffff0000u) | i;
+    };
+    grid_dependency_sync();
+    if (EPL != 0) {
+        if (warp < router.tokens) {
+            uint32_t e, rank;
+            if (blockIdx.x == 0u) {
+                route_token<EPL == 0 ? 1 : EPL, false>(router, warp, e, rank);
+            } else {
+                select_ascending<EPL == 0 ? 1 : EPL>(router, warp, e, rank);
+            }
+            if (lane < s.K) list_route(warp * s.K + rank, e);
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) list_route(i, __ldg(s.routes + i) & 0xffffu);
+    }
+    if (!o.early) quantize_sixteen<LANES>(o.input + (size_t)token * o.cols + col, active, lane, out, word);
+    __syncthreads();
+    const uint32_t token0 = first / o.chunks, token1 = min_u32((first + warps - 1u) / o.chunks + 1u, s.tokens);
+    for (uint32_t n = warp; n < (token1 - token0) * s.K; n += warps) {
+        const uint32_t i = token0 * s.K + n;
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++) {
+            if (stage == 1u && keys[0][i] < 0xffff0000u) continue;  // (uniform) the down place is asked for only where gate/up skips the route
+            const uint32_t mine = keys[stage][i];
+            uint32_t before = 0u;
+            for (uint32_t j = lane; j < count; j += 32u) before += keys[stage][j] < mine ? 1u : 0u;
+            before = __reduce_add_sync(0xffffffffu, before);
+            if (lane == 0u) places[stage][n] = mine < 0xffff0000u ? before : kUnboundSlot;
+        }
+    }
+    __syncthreads();
+    if (token >= s.tokens) return;
+    for (uint32_t r = 0; r < s.K; r++) {
+        const uint32_t n = (token - token0) * s.K + r, row = places[0][n];
+        if (row == kUnboundSlot) {  // a route that gate/up skips: zeros for the down stage, if that keeps it
+            if (o.down.q == nullptr || item % o.chunks != 0u || places[1][n] == kUnboundSlot) continue;
+            zero_down_row(o.down, places[1][n], lane);
+            continue;
+        }
+        if (!active) continue;
+        *reinterpret_cast<uint4*>(o.q + (size_t)row * o.cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
+        if ((lane & 7u) == 0u) *o.scales.at(row, col / 128u) = word;
+    }
+}
+
+// What the expert kernels and the combine read of a schedule (layer_schedule_rank_body makes the reference's lists too), by one block.
+// place_operands_kernel, the launch ahead, writes nothing that this one touches but at most the route words, which it then selects itself (EPL !=
+// 0), reads nothing that this one writes, and let it start once all launches before it had completed: the work stands before the wait,
+// which is there so that who waits for this launch has waited for both. The next one may start at once: what it does before its wait relies on
+// launches before place_operands_kernel. (That the code is short counts: a block of this kind runs it once, and waits for each line of
+// it. The end of the general form, with the lists, took 1.6 to 2.6 us of its 3.4 to 7.8.)
+__host__ __device__ inline size_t small_schedule_words(uint32_t count, uint32_t num_experts) {
+    // per route its expert; per stage and expert the routes before it << 16 | tiles before it within its 32 experts, and its own; the sums of
+    // the 32s; [warp][expert] counts (u16)
+    return (size_t)count + 4u * (size_t)num_experts + 2u * ((num_experts + 31u) / 32u) + ((size_t)(count + 31u) / 32u * num_experts + 1u) / 2u;
+}
+template <int EPL>
+__global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch router, LayerSchedule s) {
+    extern __shared__ uint32_t smem_words[];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t E = s.num_experts, count = s.tokens * s.K, groups = (E + 31u) / 32u, rows = (count + 31u) / 32u;
+    uint32_t* ids = smem_words;
+    uint32_t* before_expert = ids + count;           // [stage][expert]
+    uint32_t* of_expert = before_expert + 2u * E;    // [stage][expert]
+    uint32_t* of_group = of_expert + 2u * E;         // [stage][32 experts]
+    uint16_t* table = reinterpret_cast<uint16_t*>(of_group + 2u * groups);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i = threadIdx.x;
+    for (uint32_t w = threadIdx.x; w < (rows * E + 1u) / 2u; w += blockDim.x) reinterpret_cast<uint32_t*>(table)[w] = 0u;
+    for (uint32_t w = threadIdx.x; w < s.clear_words; w += blockDim.x) s.clear[w] = 0u;
+    for (uint32_t b = threadIdx.x; b < 2u * E; b += blockDim.x)  // (for now whether the stage has the expert)
+        of_expert[b] = (b < E ? s.experts[0][b] : s.experts[1][b - E]).w[0] != nullptr ? 1u : 0u;
+    uint32_t e = kUnboundSlot;
+    if (EPL != 0) {
+        if (warp < router.tokens) {
+            uint32_t mine, rank;
+            select_ascending<EPL == 0 ? 1 : EPL>(router, warp, mine, rank);
+            if (lane < s.K) ids[warp * s.K + rank] = mine;
+        }
+        __syncthreads();
+        if (i < count) e = ids[i];
+    } else {
+        if (i < count) e = __ldg(s.routes + i) & 0xffffu;
+        __syncthreads();
+    }
+    const uint32_t peers = __match_any_sync(0xffffffffu, e), before = __popc(peers & ((1u << lane) - 1u));
+    if (e < E && before == 0u) table[warp * E + e] = (uint16_t)__popc(peers);
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; (b & ~31u) < E; b += blockDim.x) {
+        uint32_t total = 0u;
+        if (b < E) {
+            for (uint32_t r = 0; r < rows; r++) {
+                const uint32_t here = table[r * E + b];
+                table[r * E + b] = (uint16_t)total;
+                total += here;
+            }
+        }
+#pragma unroll
+        for (uint32_t stage = 0; stage < 2u; stage++) {
+            const uint32_t n_tile = s.n_tile[stage];
+            const uint32_t own = b < E && of_expert[stage * E + b] != 0u ? total << 16 | (total + n_tile - 1u) / n_tile : 0u;
+            uint32_t sum = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t n = __shfl_up_sync(0xffffffffu, sum, o);
+                if ((int)lane >= o) sum += n;
+            }
+            if (b < E) {
+                before_expert[stage * E + b] = sum - own;
+                of_expert[stage * E + b] = own;
+            }
+            if (lane == 31u) of_group[stage * groups + b / 32u] = sum;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t stage = 0; stage < 2u; stage++) {
+        auto base_of = [&](uint32_t b) {
+            uint32_t sum = before_expert[stage * E + b];
+            for (uint32_t w = 0; w < b / 32u; w++) sum += of_group[stage * groups + w];
+            return sum;
+        };
+        if (i < count) {
+            uint32_t place = kUnboundSlot;
+            if (e < E && of_expert[stage * E + e] != 0u) {
+                place = (base_of(e) >> 16) + table[warp * E + e] + before;
+                s.grouped[stage][place] = i;
+            } else {
+                raise_status(s.status, e >= E ? NVMOE_STATUS_ROUTE_OUT_OF_RANGE : NVMOE_STATUS_EXPERT_NOT_RESIDENT);
+            }
+            s.position[stage][i] = place;
+        }
+        for (uint32_t b = threadIdx.x; b < E; b += blockDim.x) {
+            const uint32_t base = base_of(b), own = of_expert[stage * E + b], first = base & 0xffffu;
+            const uint32_t tiles = own & 0xffffu;
+            s.offsets[stage][b] = base >> 16;
+            for (uint32_t t = 0; t < tiles; t++) s.tiles[stage][first + t] = b << 16 | t;
+            if (b + 1u == E) {
+                s.offsets[stage][E] = (base + own) >> 16;
+                *s.tile_count[stage] = first + tiles;
+            }
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // The same schedule for more routes than one block ranks well: 256 routes a block, in three launches. As above, one
@@ -1238,10 +1415,46 @@ bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t n
     return router.tokens <= (router.g.routed_experts <= 32u ? 32u : 16u) && router_is_small(router) && count <= 1024u && rank_schedule_fits(count, num_experts);
 }
 
-void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream) {
+static uint32_t route_schedule_threads(const LayerSchedule& s) {
     const uint32_t count = s.tokens * s.K, warps = s.tokens > (count + 31u) / 32u ? s.tokens : (count + 31u) / 32u;
+    return warps <= 8u ? 256u : warps <= 16u ? 512u : 1024u;
+}
+
+// A block of the operands' kernel has a warp for every token where it routes them, and as many threads as the schedule's otherwise.
+static uint32_t place_operands_threads(const LayerSchedule& s, bool routed) {
+    return routed ? route_schedule_threads(s) : layer_schedule_rank_threads(s.tokens * s.K);
+}
+static size_t place_operands_smem_bytes(const LayerSchedule& s, const OperandRows& o, bool routed) {
+    return (2u * (size_t)s.tokens * s.K + 2u * place_words(place_operands_threads(s, routed) / 32u, o.chunks, s.K)) * sizeof(uint32_t);
+}
+
+bool places_operands(const LayerSchedule& s, bool routed, const OperandRows& o, uint32_t block) {
+    const uint64_t count = (uint64_t)s.tokens * s.K;
+    return s.expert_count == 0u && count <= 1024u && small_schedule_words((uint32_t)count, s.num_experts) <= 12u * 1024u &&
+           (block == 32u || block == 128u) && o.cols % block == 0u && (reinterpret_cast<uintptr_t>(o.input) & 15u) == 0u &&
+           place_operands_smem_bytes(s, o, routed) <= 48u * 1024u;
+}
+
+void launch_place_operands(const RouterLaunch* router, const LayerSchedule& s, const OperandRows& o, uint32_t block, cudaStream_t stream) {
+    const uint32_t threads = place_operands_threads(s, router != nullptr), warps = threads / 32u;
+    const int epl = !router ? 0 : router->g.routed_experts <= 32u ? 1 : 4;
+    const auto kernel = block == 32u ? (epl == 0 ? place_operands_kernel<0, 2u> : epl == 1 ? place_operands_kernel<1, 2u> : place_operands_kernel<4, 2u>)
+                                     : (epl == 0 ? place_operands_kernel<0, 8u> : epl == 1 ? place_operands_kernel<1, 8u> : place_operands_kernel<4, 8u>);
+    launch_chained(kernel, dim3((s.tokens * o.chunks + warps - 1u) / warps), dim3(threads), place_operands_smem_bytes(s, o, router != nullptr), stream,
+                   router ? *router : RouterLaunch{}, s, o);
+}
+
+void launch_small_schedule(const RouterLaunch* router, const LayerSchedule& s, cudaStream_t stream) {
+    const int epl = !router ? 0 : router->g.routed_experts <= 32u ? 1 : 4;
+    launch_chained(epl == 0 ? small_schedule_kernel<0> : epl == 1 ? small_schedule_kernel<1> : small_schedule_kernel<4>, dim3(1),
+                   dim3(place_operands_threads(s, router != nullptr)), small_schedule_words(s.tokens * s.K, s.num_experts) * sizeof(uint32_t), stream,
+                   router ? *router : RouterLaunch{}, s);
+}
+
+void launch_route_schedule(const RouterLaunch& router, const LayerSchedule& s, cudaStream_t stream) {
+    const uint32_t count = s.tokens * s.K;
     launch_chained(router.g.routed_experts <= 32u ? route_schedule_kernel<1> : route_schedule_kernel<4>, dim3(1),
-                   dim3(warps <= 8u ? 256u : warps <= 16u ? 512u : 1024u), layer_schedule_rank_smem_bytes(count, s.num_experts), stream, router, s);
+                   dim3(route_schedule_threads(s)), layer_schedule_rank_smem_bytes(count, s.num_experts), stream, router, s);
 }
 
 uint32_t launch_layer_schedule(const LayerSchedule& s, const SortScratch& scratch, cudaStream_t stream) {
