@@ -52,6 +52,16 @@ __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uin
     return 0.0f;
 }
 
+// The functions of the scores as calls: a token is routed by code that runs once, and waits for every line of it, so that one copy for all places
+// counts more than what a call costs; for the same reason loops over selections are not unrolled. Layers, times as fast as with the schedule and the
+// quantisation in turn, inlined and unrolled / this way: one token of 32 experts 1.057 / 1.076, seven 1.054 / 1.070, 32 from host buffers 1.025 /
+// 1.036, 64 1.029 / 1.030, tiny 1.060 / 1.055, 96 of 257 1.017 / 1.012 (small_schedule_kernel<1> 34.7 KB / 21.1 KB, router_reg_kernel<8, true> 73 / 32).
+__device__ __noinline__ float route_exp(float v) { return nvmoe_expf(v); }
+__device__ __noinline__ float route_divide(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __noinline__ float route_sigmoid(float v) { return nvmoe_sigmoidf(v); }
+__device__ __noinline__ float route_softplus_root(float v) { return __fsqrt_rn(nvmoe_softplusf(v)); }
+__device__ __noinline__ float route_softcap(float v, float cap) { return __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, cap)), cap); }
+
 // ---- the same router with a token's experts in registers ------------------------------------------
 // For up to 32 * EPL experts and at most 32 selections a token; GROUPS: with group-limited masking, for groups of a
 // power of two of experts up to 32, which are then a run of lanes: lane l keeps the
@@ -59,7 +69,41 @@ __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uin
 // does through shared memory by one lane (the weights, the ascending order, packing, telemetry) is done by the
 // lanes side by side. Every sum that has an order keeps it (values travel by shuffle and are added in the same
 // sequence); the results are bit for bit those of router_kernel, which remains for the other cases. Called by a whole warp.
-//
+
+// k rounds of arg-max over the experts that `taken` does not name: lane r keeps selection r (expert and value). False if there are fewer than k
+// selectable scores.
+template <int EPL>
+__device__ __forceinline__ bool pick_experts(uint32_t E, uint32_t k, const float (&val)[EPL], const float (&score)[EPL], uint32_t taken, uint32_t& my_e, float& my_v) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    my_e = kUnboundSlot;
+    my_v = 0.0f;
+#pragma unroll 1
+    for (uint32_t r = 0; r < k; r++) {
+        float best = kNegInf, best_v = 0.0f;
+        uint32_t best_e = kUnboundSlot;
+#pragma unroll
+        for (int j = 0; j < EPL; j++) {
+            const uint32_t e = lane + 32u * j;
+            if (e < E && ((taken >> j) & 1u) == 0u && better(score[j], e, best, best_e)) {
+                best = score[j];
+                best_e = e;
+                best_v = val[j];
+            }
+        }
+        const uint32_t winner = warp_best(best, best_e);
+        if (winner == kUnboundSlot) return false;
+        // the winner is the best candidate of the lane that owns it
+        const float winner_v = __shfl_sync(kFull, best_v, winner & 31u);
+        if (lane == (winner & 31u)) taken |= 1u << (winner >> 5);
+        if (lane == r) {
+            my_e = winner;
+            my_v = winner_v;
+        }
+    }
+    return true;
+}
+
 // The selection: lane r receives selection r (expert and activated value). False if there are fewer than k selectable scores.
 template <int EPL, bool GROUPS>
 __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t token, uint32_t& my_e, float& my_v) {
@@ -89,17 +133,17 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
 #pragma unroll
             for (int j = 0; j < EPL; j++) {
                 if (lane + 32u * j < E) {
-                    val[j] = nvmoe_expf(__fsub_rn(val[j], smax));
+                    val[j] = route_exp(__fsub_rn(val[j], smax));
                     if (j & 1) hi = __fadd_rn(hi, val[j]); else lo = __fadd_rn(lo, val[j]);
                 }
             }
             const float sden = warp_butterfly_sum(__fadd_rn(lo, hi));
 #pragma unroll
-            for (int j = 0; j < EPL; j++) val[j] = __fdiv_rn(val[j], sden);
+            for (int j = 0; j < EPL; j++) val[j] = route_divide(val[j], sden);
         } else {
 #pragma unroll
             for (int j = 0; j < EPL; j++)
-                val[j] = p.g.activation == NVMOE_ACT_SIGMOID ? nvmoe_sigmoidf(val[j]) : __fsqrt_rn(nvmoe_softplusf(val[j]));
+                val[j] = p.g.activation == NVMOE_ACT_SIGMOID ? route_sigmoid(val[j]) : route_softplus_root(val[j]);
         }
 #pragma unroll
         for (int j = 0; j < EPL; j++) {
@@ -115,16 +159,13 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
         for (int j = 0; j < EPL; j++) {
             const uint32_t e = lane + 32u * j;
             float v = val[j];
-            if (p.g.logit_softcap > 0.0f) v = __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, p.g.logit_softcap)), p.g.logit_softcap);
+            if (p.g.logit_softcap > 0.0f) v = route_softcap(v, p.g.logit_softcap);
             val[j] = v;
-            score[j] = e < E ? __fadd_rn(sigmoid ? nvmoe_sigmoidf(v) : v, read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
+            score[j] = e < E ? __fadd_rn(sigmoid ? route_sigmoid(v) : v, read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
         }
     }
 
-    // ---- k rounds of arg-max: lane r keeps selection r ---------------------------------------
     uint32_t taken = 0u;
-    my_e = kUnboundSlot;
-    my_v = 0.0f;
     if (GROUPS) {
         // a group's score is the sum of its two best; the experts of the groups outside the topk_group best count as taken
         const uint32_t per = E / p.g.n_group, side = 32u / per;  // groups in a register slot of the warp
@@ -132,6 +173,7 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
 #pragma unroll
         for (int j = 0; j < EPL; j++) {
             float first = lane + 32u * j < E && score[j] > kNegInf ? score[j] : kNegInf, second = kNegInf;
+#pragma unroll 1
             for (uint32_t o = 1u; o < per; o <<= 1) {
                 const float other_first = __shfl_xor_sync(kFull, first, o), other_second = __shfl_xor_sync(kFull, second, o);
                 second = fmaxf(fminf(first, other_first), fmaxf(second, other_second));
@@ -141,6 +183,7 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
             if (lane / side == (uint32_t)j) my_group = group;  // lane g keeps group g
         }
         uint32_t kept = 0u;
+#pragma unroll 1
         for (uint32_t round = 0; round < p.g.topk_group; round++) {
             const bool open = lane < p.g.n_group && ((kept >> lane) & 1u) == 0u && my_group >= kNegInf;  // (not a NaN)
             const uint32_t winner = warp_best(my_group, open ? lane : kUnboundSlot);
@@ -152,34 +195,13 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
             if (group >= 32u || ((kept >> group) & 1u) == 0u) taken |= 1u << j;
         }
     }
-    for (uint32_t r = 0; r < k; r++) {
-        float best = kNegInf, best_v = 0.0f;
-        uint32_t best_e = kUnboundSlot;
-#pragma unroll
-        for (int j = 0; j < EPL; j++) {
-            const uint32_t e = lane + 32u * j;
-            if (e < E && ((taken >> j) & 1u) == 0u && better(score[j], e, best, best_e)) {
-                best = score[j];
-                best_e = e;
-                best_v = val[j];
-            }
-        }
-        const uint32_t winner = warp_best(best, best_e);
-        if (winner == kUnboundSlot) return false;
-        // the winner is the best candidate of the lane that owns it
-        const float winner_v = __shfl_sync(kFull, best_v, winner & 31u);
-        if (lane == (winner & 31u)) taken |= 1u << (winner >> 5);
-        if (lane == r) {
-            my_e = winner;
-            my_v = winner_v;
-        }
-    }
-    return true;
+    return pick_experts<EPL>(E, k, val, score, taken, my_e, my_v);
 }
 
 // The places of a token's selections in ascending order of the experts: lane r < total_k holds selection r.
 __device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total_k) {
     uint32_t rank = 0u;
+#pragma unroll 1
     for (uint32_t q = 0; q < total_k; q++) {
         const uint32_t other = __shfl_sync(0xffffffffu, my_e, q);
         if (other < my_e) rank++;
@@ -187,23 +209,17 @@ __device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total
     return rank;
 }
 
-// Lane r < total_k receives the expert and the place of one of the token's route words, as route_token writes them.
-template <int EPL>
-__device__ __forceinline__ void select_ascending(const RouterLaunch& p, uint32_t token, uint32_t& my_e, uint32_t& rank) {
+// Of a token whose selections the lanes hold (`found`: there are k): lane r < total_k receives the expert and the place of one of its route words, as
+// finish_token writes them.
+__device__ __forceinline__ void order_token(const RouterLaunch& p, bool found, uint32_t& my_e, uint32_t& rank) {
     const uint32_t lane = threadIdx.x & 31u, k = p.g.routed_k, always = p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
-    float v;
-    if (!select_experts<EPL, false>(p, token, my_e, v)) {  // words of zeros
-        my_e = 0u;
-        rank = lane;
-        return;
-    }
-    if (lane >= k) my_e = p.g.routed_experts + (lane - k);
-    rank = ascending_rank(my_e, k + always);
+    if (!found) my_e = 0u;  // words of zeros
+    if (found && lane >= k) my_e = p.g.routed_experts + (lane - k);
+    rank = found ? ascending_rank(my_e, k + always) : lane;
 }
 
-// Selection, weights, route words and telemetry of a token; my_e and rank as above.
-template <int EPL, bool GROUPS>
-__device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token, uint32_t& my_e, uint32_t& rank) {
+// Weights, route words and telemetry of such a token; my_e and rank as above.
+__device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t token, bool found, uint32_t& my_e, float my_v, uint32_t& rank) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t E = p.g.routed_experts;
     const uint32_t k = p.g.routed_k;
@@ -212,8 +228,6 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
     const uint32_t total_k = k + always;
     const uint32_t total_resources = E + always;
     const uint32_t lane = threadIdx.x & 31u;
-    float my_v;
-    const bool found = select_experts<EPL, GROUPS>(p, token, my_e, my_v);
     uint32_t* out = p.routes + (size_t)token * total_k;
     if (!found) {
         // no selectable score (NaN logits): fail closed instead of indexing out of bounds
@@ -230,9 +244,9 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
     float w = 0.0f;
     if (kind == NVMOE_ROUTER_SCORE_TOPK) {
         float den = 0.0f;
-        if (p.g.normalize_selected)
-            for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, my_v, r));
-        w = p.g.normalize_selected ? __fmul_rn(__fdiv_rn(my_v, den), p.g.routed_scale) : __fmul_rn(my_v, p.g.routed_scale);
+#pragma unroll 1
+        for (uint32_t r = 0; p.g.normalize_selected && r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, my_v, r));
+        w = p.g.normalize_selected ? __fmul_rn(route_divide(my_v, den), p.g.routed_scale) : __fmul_rn(my_v, p.g.routed_scale);
         if (lane >= k && lane < total_k) {
             my_e = E + (lane - k);
             w = p.g.always_weight;
@@ -241,10 +255,11 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
         const bool sigmoid = kind == NVMOE_ROUTER_TOPK_ROUTED && p.g.activation == NVMOE_ACT_SIGMOID;
         const bool divide = kind == NVMOE_ROUTER_TOPK_SOFTMAX || p.g.normalize_selected || !sigmoid;
         const float maximum = __shfl_sync(kFull, my_v, 0);
-        const float t = sigmoid ? nvmoe_sigmoidf(my_v) : nvmoe_expf(__fsub_rn(my_v, maximum));
+        const float t = sigmoid ? route_sigmoid(my_v) : route_exp(__fsub_rn(my_v, maximum));
         float den = 0.0f;
+#pragma unroll 1
         for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, t, r));
-        w = divide ? __fdiv_rn(t, den) : t;
+        w = divide ? route_divide(t, den) : t;
     }
 
     // ---- ascending expert id, pack, telemetry ----------------------------------------------------
@@ -254,6 +269,7 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
         if (p.telemetry) atomicAdd(p.telemetry + my_e, 1u);
     }
     if (p.telemetry) {
+#pragma unroll 1
         for (uint32_t q = 0; q < total_k; q++) {
             const uint32_t right = __shfl_sync(kFull, my_e, q);
             if (lane < total_k && my_e < right) {
@@ -266,8 +282,10 @@ __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t toke
 
 template <int EPL, bool GROUPS>
 __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token) {
-    uint32_t e, rank;
-    route_token<EPL, GROUPS>(p, token, e, rank);
+    uint32_t my_e, rank;
+    float my_v;
+    const bool found = select_experts<EPL, GROUPS>(p, token, my_e, my_v);
+    finish_token(p, token, found, my_e, my_v, rank);
 }
 
 }  // namespace

@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(1024) route_schedule_kernel(RouterLaunch route
 // in turn / side by side: 64 tokens of the tiny layer 24.4 / 23.1; 32 experts of 2880 x 2880, one token 37.0 / 35.0, seven 67.1 / 63.7, 64 94.8 / 92.1, 32 from
 // host buffers 121.0 / 118.0; 96 of 257 of 7168 x 2048 749 / 737.
 template <int EPL, uint32_t LANES>
-__global__ void __launch_bounds__(1024) place_operands_kernel(RouterLaunch router, LayerSchedule s, OperandRows o) {
+__global__ void __launch_bounds__(1024) place_operands_kernel(const __grid_constant__ RouterLaunch router, const __grid_constant__ LayerSchedule s, const __grid_constant__ OperandRows o) {
     extern __shared__ uint32_t smem_words[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t count = s.tokens * s.K, first = blockIdx.x * warps, item = first + warp;
@@ -910,19 +910,23 @@ __global__ void __launch_bounds__(1024) place_operands_kernel(RouterLaunch route
     if (EPL != 0) {
         if (warp < router.tokens) {
             uint32_t e, rank;
+            float v;
+            const bool found = select_experts<EPL == 0 ? 1 : EPL, false>(router, warp, e, v);
             if (blockIdx.x == 0u) {
-                route_token<EPL == 0 ? 1 : EPL, false>(router, warp, e, rank);
+                finish_token(router, warp, found, e, v, rank);
             } else {
-                select_ascending<EPL == 0 ? 1 : EPL>(router, warp, e, rank);
+                order_token(router, found, e, rank);
             }
             if (lane < s.K) list_route(warp * s.K + rank, e);
         }
     } else {
+#pragma unroll 1
         for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) list_route(i, __ldg(s.routes + i) & 0xffffu);
     }
     if (!o.early) quantize_sixteen<LANES>(o.input + (size_t)token * o.cols + col, active, lane, out, word);
     __syncthreads();
     const uint32_t token0 = first / o.chunks, token1 = min_u32((first + warps - 1u) / o.chunks + 1u, s.tokens);
+#pragma unroll 1
     for (uint32_t n = warp; n < (token1 - token0) * s.K; n += warps) {
         const uint32_t i = token0 * s.K + n;
 #pragma unroll
@@ -937,6 +941,7 @@ __global__ void __launch_bounds__(1024) place_operands_kernel(RouterLaunch route
     }
     __syncthreads();
     if (token >= s.tokens) return;
+#pragma unroll 1
     for (uint32_t r = 0; r < s.K; r++) {
         const uint32_t n = (token - token0) * s.K + r, row = places[0][n];
         if (row == kUnboundSlot) {  // a route that gate/up skips: zeros for the down stage, if that keeps it
@@ -962,7 +967,7 @@ __host__ __device__ inline size_t small_schedule_words(uint32_t count, uint32_t 
     return (size_t)count + 4u * (size_t)num_experts + 2u * ((num_experts + 31u) / 32u) + ((size_t)(count + 31u) / 32u * num_experts + 1u) / 2u;
 }
 template <int EPL>
-__global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch router, LayerSchedule s) {
+__global__ void __launch_bounds__(1024) small_schedule_kernel(const __grid_constant__ RouterLaunch router, const __grid_constant__ LayerSchedule s) {
     extern __shared__ uint32_t smem_words[];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t E = s.num_experts, count = s.tokens * s.K, groups = (E + 31u) / 32u, rows = (count + 31u) / 32u;
@@ -972,15 +977,19 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch route
     uint32_t* of_group = of_expert + 2u * E;         // [stage][32 experts]
     uint16_t* table = reinterpret_cast<uint16_t*>(of_group + 2u * groups);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i = threadIdx.x;
+#pragma unroll 1
     for (uint32_t w = threadIdx.x; w < (rows * E + 1u) / 2u; w += blockDim.x) reinterpret_cast<uint32_t*>(table)[w] = 0u;
+#pragma unroll 1
     for (uint32_t w = threadIdx.x; w < s.clear_words; w += blockDim.x) s.clear[w] = 0u;
+#pragma unroll 1
     for (uint32_t b = threadIdx.x; b < 2u * E; b += blockDim.x)  // (for now whether the stage has the expert)
         of_expert[b] = (b < E ? s.experts[0][b] : s.experts[1][b - E]).w[0] != nullptr ? 1u : 0u;
     uint32_t e = kUnboundSlot;
     if (EPL != 0) {
         if (warp < router.tokens) {
             uint32_t mine, rank;
-            select_ascending<EPL == 0 ? 1 : EPL>(router, warp, mine, rank);
+            float v;
+            order_token(router, select_experts<EPL == 0 ? 1 : EPL, false>(router, warp, mine, v), mine, rank);
             if (lane < s.K) ids[warp * s.K + rank] = mine;
         }
         __syncthreads();
@@ -992,6 +1001,7 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch route
     const uint32_t peers = __match_any_sync(0xffffffffu, e), before = __popc(peers & ((1u << lane) - 1u));
     if (e < E && before == 0u) table[warp * E + e] = (uint16_t)__popc(peers);
     __syncthreads();
+#pragma unroll 1
     for (uint32_t b = threadIdx.x; (b & ~31u) < E; b += blockDim.x) {
         uint32_t total = 0u;
         if (b < E) {
@@ -1001,7 +1011,7 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch route
                 total += here;
             }
         }
-#pragma unroll
+#pragma unroll 1
         for (uint32_t stage = 0; stage < 2u; stage++) {
             const uint32_t n_tile = s.n_tile[stage];
             const uint32_t own = b < E && of_expert[stage * E + b] != 0u ? total << 16 | (total + n_tile - 1u) / n_tile : 0u;
@@ -1019,10 +1029,11 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch route
         }
     }
     __syncthreads();
-#pragma unroll
+#pragma unroll 1
     for (uint32_t stage = 0; stage < 2u; stage++) {
         auto base_of = [&](uint32_t b) {
             uint32_t sum = before_expert[stage * E + b];
+#pragma unroll 1
             for (uint32_t w = 0; w < b / 32u; w++) sum += of_group[stage * groups + w];
             return sum;
         };
@@ -1036,10 +1047,12 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(RouterLaunch route
             }
             s.position[stage][i] = place;
         }
+#pragma unroll 1
         for (uint32_t b = threadIdx.x; b < E; b += blockDim.x) {
             const uint32_t base = base_of(b), own = of_expert[stage * E + b], first = base & 0xffffu;
             const uint32_t tiles = own & 0xffffu;
             s.offsets[stage][b] = base >> 16;
+#pragma unroll 1
             for (uint32_t t = 0; t < tiles; t++) s.tiles[stage][first + t] = b << 16 | t;
             if (b + 1u == E) {
                 s.offsets[stage][E] = (base + own) >> 16;
