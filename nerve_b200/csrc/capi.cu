@@ -143,7 +143,7 @@ struct nvmoe_plan {
     DeviceArray tmap_templates;  // tensor maps of the two weight matrix shapes; each expert's map is one with its address patched in
     bool tma[2] = {false, false};
     // scratch of the fused layer call
-    DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev;
+    DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev, filter;
     void* pinned_in = nullptr;
     bool pinned_mapped = false;  // both have the same address on the device
     void* pinned_out = nullptr;
@@ -588,6 +588,7 @@ static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool den
         return code;
     }
     configure_router_kernels();
+    configure_router_filter();
     configure_simt_kernels();
     tc_configure_kernels();
     *out = p;
@@ -611,7 +612,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
                           &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->iq,
                           &p->i_scales, &p->tile_list, &p->ep_source, &p->layer_sync, &p->clock, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
-                          &p->controls, &p->hidden_dev, &p->output_dev};
+                          &p->controls, &p->hidden_dev, &p->output_dev, &p->filter};
     for (DeviceArray* a : all) a->release();
     if (p->pinned_in) cudaFreeHost(p->pinned_in);
     if (p->pinned_out) cudaFreeHost(p->pinned_out);
@@ -1468,6 +1469,7 @@ static int ensure_layer_scratch(nvmoe_plan* p) {
     want(p->frames, T * (size_t)p->frame_words * 4u);
     want(p->expert_outputs, T * p->K * (size_t)g.hidden_size * 2u);
     want(p->controls, 64u);
+    if (router_filter_takes(g, g.max_tokens)) want(p->filter, router_filter_floats(g.max_tokens, g.routed_experts) * 4u);
     if (err == cudaSuccess && fresh_frames) err = cudaMemsetAsync(p->frames.ptr, 0, p->frames.bytes, p->device->stream);
     if (err != cudaSuccess)
         return fail(p->device, err == cudaErrorMemoryAllocation ? NVMOE_ERR_OUT_OF_MEMORY : NVMOE_ERR_CUDA,
@@ -1604,11 +1606,30 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     }
     const uint32_t launches_before = p->launches;
     mark(kStageLinear);
-    if (projects) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, start));
+    RouterFilter filter{};
+    bool filters = projects && !a->logits && !routes_in_schedule && router_filter_takes(g, T) &&
+                   ((reinterpret_cast<uintptr_t>(a->hidden->ptr) | reinterpret_cast<uintptr_t>(a->router_weights->ptr)) & 15u) == 0u;
+    if (filters) {
+        filter.x = (const uint16_t*)a->hidden->ptr;
+        filter.w = (const uint16_t*)a->router_weights->ptr;
+        filter.logit_bias = a->router_bias ? (const uint16_t*)a->router_bias->ptr : nullptr;
+        filter.scratch = p->filter.as<float>();
+        filter.hidden = g.hidden_size;
+        filter.wait_cycles = p->wait_cycles;
+        filter.start = start;
+        filters = launch_router_filter(router, filter, st);
+        if (filters) p->launches++;
+        NVMOE_TRY(post_launch(p, "router projection"));
+    }
+    if (projects && !filters) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, start));
     mark(kStageRoute);
     // (with stage profiling on, the router keeps a launch and a time of its own)
     if (!a->routes_in && !routes_in_schedule) {
-        launch_router(router, st);
+        if (filters) {
+            launch_router_refine(router, filter, st);
+        } else {
+            launch_router(router, st);
+        }
         p->launches++;
         NVMOE_TRY(post_launch(p, "router"));
     }

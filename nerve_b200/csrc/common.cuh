@@ -156,6 +156,22 @@ bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selecti
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
                           uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream);
 
+// router_filter.cu: projection and routing of a large call, of which only the logits that matter are made exactly.
+struct RouterFilter {
+    const uint16_t* x;
+    const uint16_t* w;
+    const uint16_t* logit_bias;  // or null
+    float* scratch;              // router_filter_floats of them
+    uint32_t hidden;
+    long long wait_cycles;
+    CallStart start;
+};
+void configure_router_filter();
+bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens);  // the call, if its buffers lie on the 16-byte grid
+size_t router_filter_floats(uint32_t max_tokens, uint32_t experts);  // scratch of calls of up to so many tokens
+bool launch_router_filter(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream);  // false: no tensor maps here
+void launch_router_refine(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream);
+
 struct SortScratch {  // schedule.cu: scratch of the counting sort, sized for max_tokens
     uint32_t* block_hist;      // [blocks][buckets]
     uint32_t* bucket_totals;   // [buckets]
