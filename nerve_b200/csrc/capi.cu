@@ -142,6 +142,7 @@ struct nvmoe_plan {
     DeviceArray cta_trace;       // per-CTA diagnostics of the tensor-path kernels, allocated on first request
     DeviceArray tmap_templates;  // tensor maps of the two weight matrix shapes; each expert's map is one with its address patched in
     bool tma[2] = {false, false};
+    bool one_matrix = false;     // the plan of a dense linear's shape
     // scratch of the fused layer call
     DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev, filter;
     void* pinned_in = nullptr;
@@ -186,6 +187,7 @@ size_t most_tokens_per_expert(const nvmoe_plan* p) { return ((size_t)p->g.max_to
 
 // Token tile of a stage for T tokens.
 TokenTile token_tile(const nvmoe_plan* p, bool gate_up, uint32_t T) {
+    if (p->one_matrix) return tc_dense_tile_for(T, p->g.hidden_size, p->g.intermediate_size, p->tma[1]);
     return tc_token_tile_for(T, p->K, p->experts, gate_up ? p->g.intermediate_size : p->g.hidden_size, gate_up, p->tma[gate_up ? 0 : 1]);
 }
 
@@ -494,6 +496,7 @@ static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool den
     if (!p) return fail(d, NVMOE_ERR_OUT_OF_MEMORY, "out of host memory");
     p->device = d;
     p->g = *geometry;
+    p->one_matrix = dense;
     const nvmoe_geometry& g = p->g;
     p->K = g.routed_k + g.always_count;
     p->experts = g.routed_experts + g.always_count;
@@ -524,7 +527,7 @@ static int create_plan(nvmoe_device* d, const nvmoe_geometry* geometry, bool den
         want(p->grouped_e8m0[1], sizeof(uint32_t) * scale_rows(p) * ((I + 127u) / 128u));
         want(p->act_maps, 2u * kActMaps * 128u);
         const size_t most = most_tokens_per_expert(p);
-        const bool with_pairs = most > kPairsFrom;
+        const bool with_pairs = most > (dense ? kTokenMapFrom[2] : kPairsFrom);  // (tc_dense_tile_for)
         // Only the maps that the plan's calls can use are encoded, at about 2.8 us each; the others stay zero and are not looked at.
         if (err == cudaSuccess) {
             unsigned char maps[2u * kActMaps * 128u] = {0};
@@ -1332,7 +1335,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
             cudaError_t err = cudaMemcpyAsync(fresh.unit_routes.ptr, ones.data(), ones.size() * 4u, cudaMemcpyHostToDevice, d->stream);
             // the map of the derived scales stays (the matrix's own maps, before it, are made by every call)
             unsigned char map[128];
-            if (fresh.plan->tma[1] && most_tokens_per_expert(fresh.plan) > kPairsFrom) {
+            if (fresh.plan->tma[1] && most_tokens_per_expert(fresh.plan) > kTokenMapFrom[2]) {
                 if (!tc_encode_pair_scale_map(map, fresh.set.derived.ptr, 1u, (uint32_t)(tc_derived_scale_bytes(rows, cols) / 512u)))
                     fresh.plan->tma[1] = false;
                 else if (err == cudaSuccess)

@@ -1091,6 +1091,37 @@ bool tc_shape_supported(const nvmoe_geometry& g) {
 
 bool tc_enabled_by_default() { return true; }
 
+// The token tile of CTA pairs (the reasons stand with tc_token_tile_for).
+static TokenTile pair_tile_for(uint32_t num_experts, uint32_t per_expert, uint32_t row_tiles) {
+    const uint64_t sms = (uint64_t)sm_count();
+    const uint32_t rows[4] = {kPairTokens, 192u, 128u, 64u};
+    TokenTile best{kPairTokens, true};
+    const uint64_t half_tiles = (uint64_t)num_experts * (2ull * per_expert + kPairTokens) / kPairTokens;
+    if (num_experts > 1u && (half_tiles + 1u) / 2u * row_tiles > sms) return best;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t i = 0; i < 4u; i++) {
+        const uint64_t tiles = (uint64_t)num_experts * ((per_expert + rows[i] - 1u) / rows[i]) * row_tiles;
+        const uint64_t cost = (tiles + sms / 2u - 1u) / (sms / 2u) * (256u + rows[i]);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best.rows = rows[i];
+        }
+    }
+    return best;
+}
+
+// A dense linear has one matrix, whose row tiles leave most SMs idle, so that what a stage takes by itself counts: pairs from fewer tokens on than
+// for a layer's experts, where K is long. One CTA a tile / pairs, us a call (quantisation included), 7168 columns to 2048 rows: 24 tokens 15.8 / 17.7,
+// 32 23.9 / 17.6, 48 24.2 / 17.8, 64 26.3 / 17.9, 96 26.8 / 18.1; 2880 to 2880: 24 10.7 / 12.5, 32 14.6 / 12.7, 64 16.1 / 13.0; 2048 to 7168: 24 9.5 / 11.1, 32 12.2 /
+// 11.3, 64 13.7 / 11.5; 1024 to 4096: 32 9.3 / 9.8, 48 9.6 / 9.9, 64 10.7 / 9.9; 512 to 1024: 24 7.0 / 8.8, 64 9.3 / 9.0. (Runs of a tile's stages by several
+// pairs, whose sums the last one adds up: 2 us less for 7168 columns and up to 64 tokens, level or slower elsewhere. Token rows by linear copies from
+// operands that lie as shared memory holds them, past the scale warp: 2 us more at 7168 columns.)
+TokenTile tc_dense_tile_for(uint32_t tokens, uint32_t out_rows, uint32_t cols, bool tma) {
+    const bool pairs = tma && tokens > (cols >= 2048u ? kTokenMapFrom[2] : kTokenMapFrom[3]) && tokens <= kPairsFrom;
+    if (pairs) return pair_tile_for(1u, tokens, (out_rows + 2u * kBlockM - 1u) / (2u * kBlockM));
+    return tc_token_tile_for(tokens, 1u, 1u, out_rows, false, tma);
+}
+
 TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up, bool tma) {
     // tokens per expert if routing were uniform; skew only adds token tiles
     const uint32_t routes = tokens * routes_per_token;
@@ -1104,9 +1135,9 @@ TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t
     const uint64_t sms = (uint64_t)sm_count();
     // Beyond that CTA pairs. One CTA with tiles of 96 / pairs, us a layer, by tokens an expert: 32 experts of 2880 x 2880, 104
     // 205.7 / 183.8, 128 223.4 / 219.7, 192 290.4 / 264.7, 240 323.4 / 283.1; 128 of them, 104 731 / 711, 128 867 / 835, 192 1128 /
-    // 1031; a dense block of 7168 x 2048, 100 78.3 / 58.6, 240 84.9 / 66.5. In layers that take one round of the SMs either way
+    // 1031. In layers that take one round of the SMs either way
     // the two are within a few percent: 16 experts of 768 x 512, 104 55.5 / 55.6, 128 54.0 / 55.3, 192 60.8 / 60.3, 240 61.9 / 66.0;
-    // 8 of 1024 x 1024, 128 47.2 / 47.3, 192 60.3 / 61.2. Dense blocks would gain below the line too (96 rows 77.7 by one CTA).
+    // 8 of 1024 x 1024, 128 47.2 / 47.3, 192 60.3 / 61.2. (Dense linears have a lower line: tc_dense_tile_for.)
     // An expert takes several tiles. Where they are more than two rounds of the pairs, the widest: a stage takes 350 ns and 1.7 a
     // column (gate/up of 4096 tokens of 32 experts, all tiles of one width, ns a stage: 64 467, 128 581, 192 672, 240 761), a tile
     // with fewer tokens runs with fewer columns, and the loads of several experts differ, so that narrower tiles fit none of them
@@ -1115,22 +1146,7 @@ TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t
     // In fewer rounds, or with one expert, whose load is the call's, the fewest rounds x stage time wins, as 256 + columns, with
     // every expert at the mean load and its last tile at full width: dense block of 777 rows (128) 95.7 us, with 192 throughout
     // 110, with 240 139.
-    if (tma) {
-        const uint32_t rows[4] = {kPairTokens, 192u, 128u, 64u};
-        TokenTile best{kPairTokens, true};
-        const uint64_t half_tiles = (uint64_t)num_experts * (2ull * per_expert + kPairTokens) / kPairTokens;
-        if (num_experts > 1u && (half_tiles + 1u) / 2u * row_tiles > sms) return best;
-        uint64_t best_cost = ~0ull;
-        for (uint32_t i = 0; i < 4u; i++) {
-            const uint64_t tiles = (uint64_t)num_experts * ((per_expert + rows[i] - 1u) / rows[i]) * row_tiles;
-            const uint64_t cost = (tiles + sms / 2u - 1u) / (sms / 2u) * (256u + rows[i]);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best.rows = rows[i];
-            }
-        }
-        return best;
-    }
+    if (tma) return pair_tile_for(num_experts, per_expert, row_tiles);
     // Shapes without tensor maps: the widest tile, by the same count of rounds. A stage of 128 columns takes 8/7 of the time
     // of one of 96 (0.527 and 0.461 us with whole rounds of either).
     const uint32_t widths[2] = {128u, 96u}, stage_time[2] = {8u, 7u};

@@ -62,6 +62,7 @@ struct TokenTile {
 // token tile of a stage for this many tokens and rows of its weight matrix (the (expert, token tile) list must be
 // built with it); tma: the stage's shapes have tensor maps
 TokenTile tc_token_tile_for(uint32_t tokens, uint32_t routes_per_token, uint32_t num_experts, uint32_t out_rows, bool gate_up, bool tma);
+TokenTile tc_dense_tile_for(uint32_t tokens, uint32_t out_rows, uint32_t cols, bool tma);  // of a dense linear of a [out_rows][cols] matrix
 constexpr uint32_t kPairTokens = 240u;    // the most tokens of a pair's tile
 constexpr uint32_t kRowPairTokens = 64u;  // one CTA's down tiles of that many tokens and more always take two row tiles
 void pair_configure_kernels();
