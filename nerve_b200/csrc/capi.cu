@@ -167,6 +167,8 @@ struct nvmoe_plan {
         nvmoe_plan* plan = nullptr;
         DeviceArray unit_routes;
         ExpertSet set;
+        bool host_maps = false;  // CTA pairs: the matrix's maps are made on the host, from these, and go with the launch
+        unsigned char maps[2][128];
     };
     std::vector<DenseLinear> dense;
 };
@@ -954,6 +956,7 @@ struct ExpertCall {
     bool scheduled = false;         // grouping (and tile list) already built for this call
     bool fuse_quantise = false;     // gate/up on the tensor path: the epilogue also writes the down stage's operands
     bool fresh_maps = false;        // the last launch before this one writes the tensor maps
+    const void* dense_maps = nullptr;  // ExpertLaunch.dense_maps
     uint32_t* status = nullptr;     // the word that the caller's plan reads (null: this plan's own)
 };
 
@@ -988,6 +991,7 @@ static int expert_launch(nvmoe_plan* p, const ExpertCall& c, ExpertSet* es, bool
     el.tile_list = el.tile_count + 64;
     el.tile_capacity = (uint32_t)(tile_region_words(p) - 64u);
     el.fresh_maps = c.fresh_maps;
+    el.dense_maps = c.dense_maps;
     el.tokens = T;
     el.g = g;
     el.wait_cycles = p->wait_cycles;
@@ -1345,6 +1349,8 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
             if (err == cudaSuccess) err = done;
             if (err != cudaSuccess) rc = fail(d, NVMOE_ERR_CUDA, "dense linear: could not write the unit routes and the scale map: %s", cudaGetErrorString(err));
         }
+        fresh.host_maps = rc == NVMOE_OK && fresh.plan->tma[1] && tc_encode_weight_map(fresh.maps[0], fresh.set.ptrs.ptr, rows, cols, 128u) &&
+                          tc_encode_pair_weight_map(fresh.maps[1], fresh.set.ptrs.ptr, rows, cols, false);
         if (rc != NVMOE_OK) {
             nvmoe_plan_destroy(fresh.plan);
             fresh.set.release();
@@ -1376,7 +1382,12 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
         dp.map_template = sub->tma[1] ? sub->tmap_templates.as<uint8_t>() + kMapTemplates : nullptr;
         dp.map = dl->set.tmaps.as<uint8_t>();
     }
+    unsigned char maps[2][128];
+    std::memcpy(maps, dl->maps, sizeof maps);
     dp.input = (const uint16_t*)input->ptr;
+    const bool host_maps = tensor && dl->host_maps && token_tile(sub, false, T).pair && dense_prepare_quantises(dp, sub->g.act_block) &&
+                           tc_replace_map_address(maps[0], weights->ptr) && tc_replace_map_address(maps[1], weights->ptr);
+    dp.lists = !host_maps;
     dp.q = sub->grouped_q[1].as<uint8_t>();
     dp.q_e8m0 = scale_words(sub, false, T);
     const bool quantised = launch_dense_prepare(dp, sub->g.act_block, st);
@@ -1399,6 +1410,7 @@ int nvmoe_dense_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* input, nvm
     call.outputs = (uint16_t*)output->ptr;
     call.prepared = &dl->set;
     call.fresh_maps = true;
+    call.dense_maps = host_maps ? maps : nullptr;
     call.status = p->status.as<uint32_t>();
     call.scheduled = true;
     NVMOE_TRY(run_experts(sub, call));

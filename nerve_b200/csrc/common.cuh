@@ -322,6 +322,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     uint32_t* tile_list;         // tensor path scratch: routes / 16 + experts + 1 words
     uint32_t tile_capacity;      // ... of which so many may be read
     bool fresh_maps;             // tensor path: the launch right before this one wrote the tensor maps
+    const void* dense_maps;      // CTA pairs, down, one matrix: its tensor maps on the host (boxes of one K block and of two), rows in order
     uint32_t* tile_count;        // tensor path scratch: one word
     uint32_t tokens;             // upper bound (max over what control may hold)
     long long wait_cycles;       // tensor path: clock cycles after which a bounded in-kernel wait gives up

@@ -22,7 +22,11 @@
 // a warp: they lie as [K block][row], a tile's start at any row, and the 32 x 16-byte block that tcgen05.cp expands wants
 // four tokens, 32 apart, side by side; a warp of either CTA puts them there, in place, and arrives at CTA 0. All waits are
 // bounded (tcgen05.cuh); a CTA leaves only when both are done.
+#include <cuda.h>
 #include <cuda_fp8.h>
+
+#include <cstddef>
+#include <cstring>
 
 #include "experts_device.cuh"
 #include "experts_tc.cuh"
@@ -101,8 +105,20 @@ __device__ __forceinline__ float high_bf16(uint32_t pair) { return __uint_as_flo
 __device__ __forceinline__ uint32_t columns_for(uint32_t tokens) { return tokens <= 32u ? 32u : (tokens + 15u) & ~15u; }
 __device__ __forceinline__ uint32_t fetched_for(uint32_t columns) { return columns <= 64u ? 64u : columns <= 128u ? 128u : columns <= 192u ? 192u : kPairColumns; }
 
-template <bool GATE_UP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) experts_pair_kernel(ExpertLaunch p, TileList list) {
+// DENSE: one matrix, whose tensor maps come with the launch and whose tiles follow from its sizes, so that nothing has to be acquired or looked up
+// when the launch ahead (which quantises the tokens and re-tiles the scales) is through: its SMs are taken over by CTAs that have all of their set-up still
+// to do, and the first stage came 4.2 us after their start, of which the maps 1.0 and the list 0.7. The weights of the first stages are asked for before the
+// wait, while tensor memory is allocated. With that, barriers that the lanes of a warp set up and sums stored two rows at a time (below), us a call before / after: 100
+// rows of 7168 columns to 2048 18.0 / 17.1, 777 24.1 / 22.9, 4096 68.6 / 64.3; of 2048 to 7168 11.7 / 10.6, 23.1 / 19.1, 70.7 / 55.2.
+template <bool DENSE>
+struct PairMaps {};
+template <>
+struct PairMaps<true> {
+    CUtensorMap weights[2];  // boxes of one K block, of two
+};
+template <bool GATE_UP, bool DENSE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) experts_pair_kernel(ExpertLaunch p, TileList list, const __grid_constant__ PairMaps<DENSE> maps) {
+    const uint8_t* const dense_maps = DENSE ? reinterpret_cast<const uint8_t*>(&maps) : nullptr;
     const long long wait_limit = p.wait_cycles;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
@@ -129,29 +145,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     const uint32_t token_bytes = narrow ? kPairNarrowTokens / 2u * 128u : kPairTokenBytes;
     const uint32_t token_region = slots * kPairBlocks * kATileBytes, scale_region = token_region + slots * kPairBlocks * token_bytes;
 
-    // ---- one-time setup ---------------------------------------------------------------------
-    if (threadIdx.x == 0u) {
-        for (uint32_t s = 0; s < slots; s++) {
-            mbar_init(&bars->full[s], 3u);  // the announcement of the copies, the scale warps of both CTAs
-            mbar_init(&bars->empty[s], 1u);
-            mbar_init(&bars->staged[s], 1u);
+    // ---- one-time setup (the barriers by the lanes of a warp: one after the other they took half a microsecond) -----------------
+    if (warp == 0u) {
+        uint64_t* all = bars->full;
+        constexpr uint32_t kSlots = kPairNarrowStages, kAcc = 3u * kSlots, kDrain = kAcc + 8u, kCount = kDrain + 1u + 2u * kPairEpilogueWarps;
+        static_assert(offsetof(PairBarriers, tmem_base) == kCount * 8u, "the barriers come first and in this order");
+        for (uint32_t i = lane; i < kCount; i += 32u) {
+            uint32_t arrivals = 1u;
+            if (i < kSlots) arrivals = 3u;                                               // full: the announcement of the copies, the scale warps of both CTAs
+            if (i >= kAcc + 2u && i < kAcc + 4u) arrivals = 2u * kPairEpilogueWarps;     // acc_empty
+            if (i >= kAcc + 4u && i < kAcc + 6u) arrivals = 32u;                         // info_full
+            if (i >= kAcc + 6u && i < kDrain) arrivals = kPairEpilogueWarps;             // info_empty
+            mbar_init(all + i, arrivals);
         }
-        for (uint32_t a = 0; a < 2u; a++) {
-            mbar_init(&bars->acc_full[a], 1u);
-            mbar_init(&bars->acc_empty[a], 2u * kPairEpilogueWarps);
-            mbar_init(&bars->info_full[a], 32u);
-            mbar_init(&bars->info_empty[a], kPairEpilogueWarps);
-        }
-        mbar_init(&bars->drain, 1u);
-        for (uint32_t w = 0; w < kPairEpilogueWarps; w++) {
-            mbar_init(&bars->sent[w], 1u);
-            mbar_init(&bars->taken[w], 1u);
-        }
-        bars->abort = 0u;
+        if (lane == 0u) bars->abort = 0u;
         fence_mbar_init();
     }
     __syncwarp();
     cluster_sync();  // the barriers of both CTAs are up before either arrives on the other's
+    // a stage's weights; CTA 0 announces with them what both CTAs fetch for it
+    auto load_weights = [&](uint32_t st, uint32_t into, const uint8_t* weight_map, int row0, uint32_t bytes) {
+        const bool two = st < doubles;
+        const uint32_t kb = two ? 2u * st : doubles + st, at = smem_u32(smem) + into * kPairBlocks * kATileBytes, bar = map_shared(smem_u32(&bars->full[into]), 0u);
+        if (rank == 0u) mbar_arrive_expect_tx(&bars->full[into], (two ? 2u * bytes : bytes) + 2u * kPairBlocks * kScaleBlockBytes);
+        if (two) {
+            tma_load_3d_pair(at, weight_map + 128u, 0, row0, (int)kb, bar);
+        } else {
+            tma_load_3d_pair(at, weight_map, 0, (int)min(2u * kb, k_dim / 64u - 2u), row0, bar);  // in units of 64 columns: a trailing half block ends with the row
+        }
+    };
+    // DENSE: stages of the first tile whose weights are on their way before the wait
+    const uint32_t dense_tiles = DENSE ? (p.tokens + p.token_rows - 1u) / p.token_rows * m_tiles : 0u;
+    const uint32_t ahead = pair_id < dense_tiles ? min(slots, stages) : 0u;
+    const bool withheld = blockIdx.x < 2u && ((p.debug_flags >> blockIdx.x) & 1u) != 0u;  // (debug) the first stage is left out
+    if (DENSE && warp == kPairTmaWarp && lane == 0u && ahead != 0u) {
+        const uint32_t first = pair_id / m_tiles * p.token_rows, columns = columns_for(min(p.token_rows, p.tokens - first));
+        for (uint32_t st = withheld ? 1u : 0u; st < ahead; st++)
+            load_weights(st, st, dense_maps, (int)((2u * (pair_id % m_tiles) + rank) * kBlockM), 2u * (kTmaBoxBytes + fetched_for(columns) / 2u * 128u));
+    }
+    __syncwarp();
     if (warp == kPairMmaWarp) {
         tmem_alloc_pair(&bars->tmem_base, kPairTmemColumns);
         tmem_relinquish_pair();
@@ -167,11 +199,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
         if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
         __syncthreads();
     };
-    if (!p.fresh_maps) acquire_maps();  // as in experts_tc.cu: while the kernel ahead still runs
+    if (DENSE) {  // (those that stand)
+        if (threadIdx.x < kActMaps - 1u) tensormap_acquire(p.act_tmap + threadIdx.x * 128u);
+        if (threadIdx.x == kActMaps) tensormap_acquire(p.tmaps + (size_t)kWeightMaps * 128u);
+        __syncthreads();
+    } else if (!p.fresh_maps) {
+        acquire_maps();  // as in experts_tc.cu: while the kernel ahead still runs
+    }
     grid_dependency_sync();
-    const uint32_t first_entry = warp == kPairTmaWarp ? __ldg(list.tiles + min(pair_id / m_tiles, p.tile_capacity - 1u)) : 0u;
-    const uint32_t tile_count = *list.count * m_tiles;
-    if (p.fresh_maps) acquire_maps();
+    const uint32_t first_entry = !DENSE && warp == kPairTmaWarp ? __ldg(list.tiles + min(pair_id / m_tiles, p.tile_capacity - 1u)) : 0u;
+    const uint32_t tile_count = DENSE ? dense_tiles : *list.count * m_tiles;
+    if (!DENSE && p.fresh_maps) acquire_maps();
 
     // first row of a tile in the operand matrix, and how many rows it has
     auto first_row_of = [&](uint32_t n_tile, uint32_t e_begin) { return e_begin + n_tile * p.token_rows; };
@@ -184,10 +222,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             struct Meta {
                 uint32_t pair, m_tile, e_begin, e_end, format;
             };
-            auto entry_of = [&](uint32_t tile) { return tile < tile_count ? __ldg(list.tiles + tile / m_tiles) : 0u; };
+            auto entry_of = [&](uint32_t tile) { return !DENSE && tile < tile_count ? __ldg(list.tiles + tile / m_tiles) : 0u; };
             auto meta_of = [&](uint32_t tile, uint32_t pair, Meta& m) {
-                m.pair = pair;
+                m.pair = DENSE ? tile / m_tiles : pair;
                 m.m_tile = tile % m_tiles;
+                if (DENSE) {
+                    m.e_begin = 0u;
+                    m.e_end = p.tokens;
+                    m.format = kFormatCompact;
+                    return;
+                }
                 m.e_begin = __ldg(p.work.expert_offsets + (pair >> 16));
                 m.e_end = __ldg(p.work.expert_offsets + (pair >> 16) + 1u);
                 m.format = p.work.experts[pair >> 16].format;
@@ -197,17 +241,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
             const uint8_t* scale_map = p.tmaps + (size_t)p.work.num_experts * kSources * kWeightMaps * 128u;
             const uint8_t* token_scale_map = p.act_tmap + (kTokenScaleMap - 1u) * 128u;
             uint32_t slot = 0u, empty_parity = 1u, stage_it = 0u;
-            bool alive = true, withhold = blockIdx.x < 2u && ((p.debug_flags >> blockIdx.x) & 1u) != 0u;
+            bool alive = true, withhold = withheld;
             Meta cur{}, nxt{};
             if (pair_id < tile_count) meta_of(pair_id, first_entry, cur);
             uint32_t pair_nxt = entry_of(pair_id + pairs);
             for (uint32_t tile = pair_id; tile < tile_count && alive; tile += pairs) {
                 const uint32_t pair_nxt2 = entry_of(tile + 2u * pairs);
                 if (tile + pairs < tile_count) meta_of(tile + pairs, pair_nxt, nxt);
-                const uint32_t expert = cur.pair >> 16;
-                const uint32_t first = first_row_of(cur.pair & 0xffffu, cur.e_begin);
+                const uint32_t expert = DENSE ? 0u : cur.pair >> 16;
+                const uint32_t first = first_row_of(DENSE ? cur.pair : cur.pair & 0xffffu, cur.e_begin);
                 const uint32_t columns = columns_for(min(p.token_rows, cur.e_end - first));
-                const uint8_t* weight_map = p.tmaps + (size_t)(GATE_UP ? 2u * expert + rank : expert) * kWeightMaps * 128u;
+                const uint8_t* weight_map = DENSE ? dense_maps : p.tmaps + (size_t)(GATE_UP ? 2u * expert + rank : expert) * kWeightMaps * 128u;
                 const uint8_t* token_map = p.act_tmap + (columns - 1u) / 64u * 128u;
                 const int row0 = (int)(GATE_UP ? cur.m_tile * kBlockM : (2u * cur.m_tile + rank) * kBlockM);
                 // (a second tile past the last rows borrows the first's scale blocks: its weights arrive as zeros)
@@ -227,22 +271,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     const uint32_t bar = full0 + slot * 8u;
                     *reinterpret_cast<volatile uint32_t*>(&bars->stage_info[slot]) = info;
                     if (!withhold) {
-                        const uint32_t a = smem_base + slot * kPairBlocks * kATileBytes;
                         const uint32_t b = smem_base + token_region + slot * kPairBlocks * token_bytes;
                         const uint32_t sf = smem_base + scale_region + slot * kPairScaleBytes;
                         // the token scales first, which have the longest way to go (of one block, too, the scales of two are
                         // fetched: zeros, or the next row tile's, that nothing uses)
                         mbar_arrive_expect_tx(&bars->staged[slot], kPairBlocks * kPairScaleWords * 4u);
                         tma_load_2d(sf + kPairBlocks * kScaleBlockBytes, token_scale_map, (int)(first & ~3u), (int)kb, &bars->staged[slot]);
-                        if (rank == 0u) mbar_arrive_expect_tx(&bars->full[slot], (two ? 2u * block_bytes : block_bytes) + 2u * kPairBlocks * kScaleBlockBytes);
+                        if (tile != pair_id || st >= ahead) load_weights(st, slot, weight_map, row0, block_bytes);
                         if (two) {
-                            tma_load_3d_pair(a, weight_map + 128u, 0, row0, (int)kb, bar);
                             tma_load_3d_pair(b, token_map + kTokenMaps * 128u, 0, token_row, (int)kb, bar);
                         } else {
                             // in units of 64 columns: a trailing half block ends with the row
-                            const uint32_t k64 = min(2u * kb, k_dim / 64u - 2u);
-                            tma_load_3d_pair(a, weight_map, 0, (int)k64, row0, bar);
-                            tma_load_2d_pair(b, token_map, (int)(k64 * 64u), token_row, bar);
+                            tma_load_2d_pair(b, token_map, (int)(min(2u * kb, k_dim / 64u - 2u) * 64u), token_row, bar);
                         }
                         tma_load_3d_pair(sf, scale_map, 0, source, scale0 + (int)kb, bar);
                     }
@@ -368,16 +408,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
         uint32_t acc_it = 0u;
         for (uint32_t tile = pair_id; tile < tile_count; tile += pairs, acc_it++) {
             const uint32_t buffer = acc_it & 1u;
-            const uint32_t pair = __ldg(list.tiles + tile / m_tiles), expert = pair >> 16;
-            const uint32_t first = first_row_of(pair & 0xffffu, __ldg(p.work.expert_offsets + expert));
-            const uint32_t tokens = min(p.token_rows, __ldg(p.work.expert_offsets + expert + 1u) - first);
+            const uint32_t pair = DENSE ? tile / m_tiles : __ldg(list.tiles + tile / m_tiles), expert = pair >> 16;
+            const uint32_t first = DENSE ? first_row_of(pair, 0u) : first_row_of(pair & 0xffffu, __ldg(p.work.expert_offsets + expert));
+            const uint32_t tokens = min(p.token_rows, (DENSE ? p.tokens : __ldg(p.work.expert_offsets + expert + 1u)) - first);
             uint32_t route[8], extra[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 8u; i++) route[i] = 32u * i + lane < tokens ? __ldg(p.work.grouped_routes + first + 32u * i + lane) : kUnboundSlot;
+            for (uint32_t i = 0; i < 8u; i++)
+                route[i] = 32u * i + lane < tokens ? (DENSE ? first + 32u * i + lane : __ldg(p.work.grouped_routes + first + 32u * i + lane)) : kUnboundSlot;
 #pragma unroll
             for (uint32_t i = 0; i < 8u; i++) {
-                extra[i] = kUnboundSlot;
-                if (route[i] == kUnboundSlot) continue;
+                extra[i] = DENSE ? 0x3f800000u : kUnboundSlot;
+                if (DENSE || route[i] == kUnboundSlot) continue;
                 if (GATE_UP) {
                     if (p.q_out != nullptr) extra[i] = __ldg(p.down_position + route[i]);
                 } else {
@@ -406,6 +447,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
         const bool whole_block = GATE_UP && p.g.act_block == 128u;
         const bool quantise = GATE_UP && p.q_out != nullptr;             // host: only with scale blocks of 32 or 128 rows
         const bool store_rows = !GATE_UP || p.intermediates != nullptr;
+        const bool words_of_rows = !GATE_UP && p.partial_outputs == nullptr && ((reinterpret_cast<uintptr_t>(p.outputs) | (2u * H)) & 3u) == 0u;  // (uniform)
         uint32_t acc_it = 0u, sends = 0u, receipts = 0u, set_it = 0u;
         // this warp's place in the exchange: its own (read) and the same place of the other CTA's warp (written)
         const uint4* inbox = reinterpret_cast<const uint4*>(smem + kPairExchangeRegion + warp * 1024u) + lane;
@@ -491,7 +533,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                         v[j] = bf16x2_bits(__fmul_rn(__uint_as_float(d[2u * j]), __uint_as_float(extras[2u * j])),
                                            __fmul_rn(__uint_as_float(d[2u * j + 1u]), __uint_as_float(extras[2u * j + 1u])));
                 }
-                if (store_rows) {
+                if (!GATE_UP && words_of_rows) {
+                    // Neighbouring lanes (rows) hand each other one of two tokens, so that a lane stores two rows of a token at once: two bytes a lane
+                    // a store took up the end of every tile (16384 tokens of 256 experts 7339 / 7142 us a layer, 4096 of 32 511.7 / 509.7).
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++) {
+                        const uint32_t theirs = __shfl_xor_sync(0xffffffffu, v[j], 1), route = routes[2u * j + (lane & 1u)];
+                        const uint32_t word = (lane & 1u) ? __byte_perm(theirs, v[j], 0x7632) : __byte_perm(v[j], theirs, 0x5410);
+                        if (route != kUnboundSlot && row_ok) *reinterpret_cast<uint32_t*>(p.outputs + (size_t)route * H + (row & ~1u)) = word;
+                    }
+                } else if (store_rows) {
 #pragma unroll
                     for (uint32_t j = 0; j < 16u; j++) {
                         const uint32_t route = routes[j];
@@ -576,24 +627,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
     if (gave_up) winddown_pause();
 }
 
-template <bool GATE_UP>
-void launch(const ExpertLaunch& p, int sms, cudaStream_t stream) {
-    launch_chained(experts_pair_kernel<GATE_UP>, dim3((uint32_t)sms & ~1u), dim3(kPairThreads), kPairSmemBytes, stream, p,
-                   TileList{p.tile_list, p.tile_count});
+template <bool GATE_UP, bool DENSE>
+void launch(const ExpertLaunch& p, int sms, const PairMaps<DENSE>& maps, cudaStream_t stream) {
+    launch_chained(experts_pair_kernel<GATE_UP, DENSE>, dim3((uint32_t)sms & ~1u), dim3(kPairThreads), kPairSmemBytes, stream, p,
+                   TileList{p.tile_list, p.tile_count}, maps);
 }
 
 }  // namespace
 
 void pair_configure_kernels() {
-    cudaFuncSetAttribute(experts_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
-    cudaFuncSetAttribute(experts_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
+    cudaFuncSetAttribute(experts_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
+    cudaFuncSetAttribute(experts_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
+    cudaFuncSetAttribute(experts_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes);
 }
 
 void launch_experts_pair(const ExpertLaunch& p, bool gate_up, int sms, cudaStream_t stream) {
     if (gate_up) {
-        launch<true>(p, sms, stream);
+        launch<true, false>(p, sms, PairMaps<false>{}, stream);
+    } else if (p.dense_maps != nullptr) {
+        PairMaps<true> maps;
+        std::memcpy(maps.weights, p.dense_maps, sizeof maps.weights);
+        launch<false, true>(p, sms, maps, stream);
     } else {
-        launch<false>(p, sms, stream);
+        launch<false, false>(p, sms, PairMaps<false>{}, stream);
     }
 }
 

@@ -927,14 +927,15 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 // x 4 K blocks, a thread 4 rows of one K block and one 16-byte store. The last block writes the pointers and the tensor
 // maps, a warp each. With scale blocks of 32 or 128 columns (LANES = block / 16; 0: none) further blocks quantise the input, a warp 512
 // columns of one row, so that the launch takes little longer than that alone: bound by the latency of a load and a
-// store. Block of 777 x 7168 x 2048: 114.0 us with the quantisation in a launch of its own, 107 here.
+// store; a warp takes a second piece, whose load is under way with the first's, where the pieces are more than a wave of blocks (777 rows of 7168 columns 4.1 us, two
+// waves, before). Block of 777 x 7168 x 2048: 114.0 us with the quantisation in a launch of its own, 107 here.
 constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
     __shared__ __align__(128) unsigned char sm[kWeightMaps * 128u];
     grid_dependency_sync();
     const uint32_t tile_total = p.tiles.list ? (p.tokens + p.tiles.n_tile - 1u) / p.tiles.n_tile : 0u;
-    for (uint32_t i = blockIdx.x * kDenseThreads + threadIdx.x; i < p.tokens; i += gridDim.x * kDenseThreads) {
+    for (uint32_t i = blockIdx.x * kDenseThreads + threadIdx.x; p.lists && i < p.tokens; i += gridDim.x * kDenseThreads) {
         p.grouped[i] = i;
         if (i < tile_total) p.tiles.list[i] = i;  // (expert 0 << 16) | token tile
     }
@@ -966,18 +967,28 @@ __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepa
     }
     if (blockIdx.x != gridDim.x - 1u) {
         if (LANES == 0u) return;
-        const uint32_t lane = threadIdx.x & 31u, chunks = (p.cols + 511u) / 512u;
-        const uint32_t item = (blockIdx.x - retile_blocks) * (kDenseThreads / 32u) + (threadIdx.x >> 5);
-        const uint32_t row = item / chunks, col = (item % chunks) * 512u + lane * 16u;
-        if (row >= p.tokens) return;
-        const bool active = col < p.cols;  // (columns come in whole blocks: the lanes of a block agree)
-        uint32_t out[4], word;
-        quantize_sixteen<(LANES == 0u ? 1u : LANES)>(p.input + (size_t)row * p.cols + col, active, lane, out, word);
-        if (!active) return;
-        *reinterpret_cast<uint4*>(p.q + (size_t)row * p.cols + col) = make_uint4(out[0], out[1], out[2], out[3]);
-        if ((lane & 7u) == 0u) *p.q_e8m0.at(row, col / 128u) = word;
+        const uint32_t lane = threadIdx.x & 31u, chunks = (p.cols + 511u) / 512u, items = p.tokens * chunks;
+        const uint32_t warps = (gridDim.x - 1u - retile_blocks) * (kDenseThreads / 32u);
+        // two pieces at a time, whose loads are under way together
+        for (uint32_t item = (blockIdx.x - retile_blocks) * (kDenseThreads / 32u) + (threadIdx.x >> 5); item < items; item += 2u * warps) {
+            uint32_t out[2][4], word[2];
+#pragma unroll
+            for (uint32_t u = 0; u < 2u; u++) {
+                const uint32_t at = item + u * warps, row = at / chunks, col = (at % chunks) * 512u + lane * 16u;
+                // (columns come in whole blocks: the lanes of a block agree)
+                quantize_sixteen<(LANES == 0u ? 1u : LANES)>(p.input + (size_t)row * p.cols + col, at < items && col < p.cols, lane, out[u], word[u]);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 2u; u++) {
+                const uint32_t at = item + u * warps, row = at / chunks, col = (at % chunks) * 512u + lane * 16u;
+                if (at >= items || col >= p.cols) continue;
+                *reinterpret_cast<uint4*>(p.q + (size_t)row * p.cols + col) = make_uint4(out[u][0], out[u][1], out[u][2], out[u][3]);
+                if ((lane & 7u) == 0u) *p.q_e8m0.at(row, col / 128u) = word[u];
+            }
+        }
         return;
     }
+    if (!p.lists) return;
     if (threadIdx.x == 0u) {
         p.offsets[0] = 0u;
         p.offsets[1] = p.tokens;
@@ -1178,14 +1189,21 @@ void launch_derive_scales_tc(const ExpertLaunch& p, bool gate_up, cudaStream_t s
     commit_stamps_kernel<<<(count + 127u) / 128u, 128, 0, stream>>>(p.work.experts, p.scale_stamps, matrices, count);
 }
 
+bool dense_prepare_quantises(const DensePrepare& p, uint32_t act_block) {
+    return p.derived && (act_block == 32u || act_block == 128u) && (reinterpret_cast<uintptr_t>(p.input) & 15u) == 0u &&
+           (uint64_t)p.tokens * ((p.cols + 511u) / 512u) <= 0x3fffffffull;
+}
+
 bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_t stream) {
     const uint32_t m_tiles = (p.out_rows + kBlockM - 1u) / kBlockM, k_blocks = (p.cols + kBlockK - 1u) / kBlockK;
     const uint32_t retile = p.derived ? m_tiles * ((k_blocks + kDenseKBlocks - 1u) / kDenseKBlocks) : 0u;
     const uint64_t warps = (uint64_t)p.tokens * ((p.cols + 511u) / 512u);
-    const bool quantises = p.derived && (act_block == 32u || act_block == 128u) && (reinterpret_cast<uintptr_t>(p.input) & 15u) == 0u &&
-                           warps <= 0x3fffffffull;
+    const bool quantises = dense_prepare_quantises(p, act_block);
     // (without rows to quantise, as many blocks as the schedule's lists ask for)
-    const uint32_t others = quantises ? (uint32_t)((warps + 3u) / 4u) : (p.tokens + kDenseThreads - 1u) / kDenseThreads;
+    uint32_t others = quantises ? (uint32_t)((warps + 3u) / 4u) : (p.tokens + kDenseThreads - 1u) / kDenseThreads;
+    // A warp takes a second piece of a row, and more, rather than that a second wave of blocks is needed
+    const uint32_t room = 148u * (2048u / kDenseThreads) > retile + 1u + 148u ? 148u * (2048u / kDenseThreads) - retile - 1u : 148u;
+    if (quantises && others > room) others = room;
     const auto kernel = !quantises ? dense_prepare_kernel<0u> : act_block == 32u ? dense_prepare_kernel<2u> : dense_prepare_kernel<8u>;
     launch_chained(kernel, dim3(retile + others + 1u), dim3(kDenseThreads), 0, stream, p, k_blocks, retile);
     return quantises;
@@ -1207,6 +1225,21 @@ static EncodeFn tensor_map_encoder() {
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     return encode;
+}
+
+bool tc_replace_map_address(void* map128, const void* device_address) {
+    typedef CUresult (*ReplaceFn)(CUtensorMap*, void*);
+    static const ReplaceFn replace = [] {
+        cudaDriverEntryPointQueryResult q;
+        void* fn = nullptr;
+        const bool ok = cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<ReplaceFn>(ok ? fn : nullptr);
+    }();
+    CUtensorMap map;
+    std::memcpy(&map, map128, 128);
+    if (!replace || replace(&map, const_cast<void*>(device_address)) != CUDA_SUCCESS) return false;
+    std::memcpy(map128, &map, 128);
+    return true;
 }
 
 bool tc_encode_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, uint32_t box_rows) {

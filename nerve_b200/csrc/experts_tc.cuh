@@ -26,6 +26,8 @@ bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t 
 // expert-grouped token rows, and for CTA pairs the derived scales of a set (blocks of 512 bytes, `sources` to a (row tile,
 // K block)) and the token scales [rows = K blocks][words].
 bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, bool bytes);
+// A map encoded above, for another address. False where the driver cannot.
+bool tc_replace_map_address(void* map128, const void* device_address);
 bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows);
 bool tc_encode_pair_scale_map(void* map128, void* any_device_address, uint32_t sources, uint32_t blocks);
 bool tc_encode_token_scale_map(void* map128, void* base, uint32_t words, uint32_t rows);
@@ -48,10 +50,12 @@ struct DensePrepare {
     uint8_t* derived;
     const uint8_t* map_template;
     uint8_t* map;
+    bool lists;              // whether the lists, the pointers and the maps are asked for (CTA pairs need none of them)
     const uint16_t* input;
     uint8_t* q;
     ScaleWords q_e8m0;
 };
+bool dense_prepare_quantises(const DensePrepare& p, uint32_t act_block);  // whether it quantises the input too
 bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_t stream);
 // Token tile of a stage: rows of the operand matrix per entry of the (expert, token tile) list, by a CTA pair (experts_pair.cu)
 // or by one CTA (then one of the kernel's tile widths).
