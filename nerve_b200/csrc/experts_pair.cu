@@ -591,14 +591,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     const float my_inv = __uint_as_float(0x7f000000u - __float_as_uint(scale));  // 1 / scale, exact (a power of two)
                     if ((lane & 2u) == 0u && my_row != kUnboundSlot && first_row < out_rows)
                         *p.q_e8m0.byte_at(my_row, first_row / 32u) = (uint8_t)(nvmoe_f32_bits(scale) >> 23);
+                    // Four tokens' codes of a row are a word; four lanes (rows) turn their words round, so that each stores four rows of a token
+                    // at once (a byte a lane a store: 0.2 to 1.2 % of the layers below more).
+                    const uint32_t turn1 = (lane & 1u) ? 0x3715u : 0x6240u, turn2 = (lane & 2u) ? 0x3276u : 0x5410u;
 #pragma unroll
-                    for (uint32_t j = 0; j < 8u; j++) {
-                        const float inv0 = __shfl_sync(0xffffffffu, my_inv, 4u * j), inv1 = __shfl_sync(0xffffffffu, my_inv, 4u * j + 1u);
-                        const uint32_t q = __nv_cvt_float2_to_fp8x2(make_float2(low_bf16(v[j]) * inv0, high_bf16(v[j]) * inv1), __NV_SATFINITE, __NV_E4M3);
-                        const uint32_t row0 = extras[2u * j], row1 = extras[2u * j + 1u];
+                    for (uint32_t i = 0; i < 4u; i++) {
+                        uint32_t word = 0u;
+#pragma unroll
+                        for (uint32_t h = 0; h < 2u; h++) {
+                            const uint32_t j = 2u * i + h;
+                            const float inv0 = __shfl_sync(0xffffffffu, my_inv, 4u * j), inv1 = __shfl_sync(0xffffffffu, my_inv, 4u * j + 1u);
+                            word |= (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(low_bf16(v[j]) * inv0, high_bf16(v[j]) * inv1), __NV_SATFINITE, __NV_E4M3) << (16u * h);
+                        }
+                        word = __byte_perm(word, __shfl_xor_sync(0xffffffffu, word, 1), turn1);  // two rows of two tokens
+                        word = __byte_perm(word, __shfl_xor_sync(0xffffffffu, word, 2), turn2);  // four rows of token 4 i + lane % 4
+                        const uint32_t to = extras[4u * i + (lane & 3u)];
                         // (0xffffffff: columns without a token and routes the down stage skips)
-                        if (row0 != kUnboundSlot && row_ok) p.q_out[(size_t)row0 * I + row] = (uint8_t)q;
-                        if (row1 != kUnboundSlot && row_ok) p.q_out[(size_t)row1 * I + row] = (uint8_t)(q >> 8);
+                        if (to != kUnboundSlot && row_ok) *reinterpret_cast<uint32_t*>(p.q_out + (size_t)to * I + (row & ~3u)) = word;
                     }
                 }
             }
