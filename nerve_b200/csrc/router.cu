@@ -245,12 +245,62 @@ __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
     if (token < p.tokens) route_token<EPL, GROUPS>(p, token);
 }
 
+// One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the
+// instruction itself.
+__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
+    float d;
+    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
+    return d;
+}
+
 // ---- router projection ----------------------------------------------------------------------
 // The shader gives every output row 64 lanes that stride over the packed input words with two
 // f32 fma per word and then sums the lanes.  Here a block of 64 threads owns a TT x ET tile of
 // (token, output) pairs: thread v plays lane v of every pair in the tile, so each x and w word is
 // loaded once per thread and reused across the tile, and the 64 lane sums of a pair are folded
 // with the pinned butterfly (step 32 through shared memory, 16..1 by shuffles).
+
+// The 64 lanes' sums of a block's tile, folded in the pinned order (lane v by thread v), rounded and stored.
+template <int TT, int ET>
+__device__ __forceinline__ void fold_and_store(const float (&acc)[TT][ET], float (&fold)[TT * ET][32], float (&result)[TT * ET], const uint16_t* __restrict__ bias,
+                                               uint32_t* __restrict__ logits, uint32_t t0, uint32_t e0, uint32_t tokens, uint32_t outputs) {
+    const uint32_t v = threadIdx.x;
+    // butterfly step 32: lanes v and v^32 live in different warps
+    if (v >= 32u) {
+#pragma unroll
+        for (int a = 0; a < TT; a++)
+#pragma unroll
+            for (int b = 0; b < ET; b++) fold[a * ET + b][v - 32u] = acc[a][b];
+    }
+    __syncthreads();
+    if (v < 32u) {
+#pragma unroll
+        for (int a = 0; a < TT; a++)
+#pragma unroll
+            for (int b = 0; b < ET; b++) {
+                float sum = warp_butterfly_sum(__fadd_rn(acc[a][b], fold[a * ET + b][v]));
+                if (v == 0u) result[a * ET + b] = sum;
+            }
+    }
+    __syncthreads();
+    // pack pairs of outputs into words; ET is even so a word never straddles two blocks
+    const uint32_t out_words = (outputs + 1u) / 2u;
+    for (uint32_t i = v; i < TT * (ET / 2); i += 64u) {
+        uint32_t a = i / (ET / 2), bw = i % (ET / 2);
+        uint32_t t = t0 + a, e = e0 + 2u * bw;
+        if (t >= tokens || e >= outputs) continue;
+        float lo = result[a * ET + 2u * bw];
+        float hi = result[a * ET + 2u * bw + 1u];
+        if (bias) {
+            lo = __fadd_rn(lo, nvmoe_bf16_to_f32(bias[e]));
+            if (e + 1u < outputs) hi = __fadd_rn(hi, nvmoe_bf16_to_f32(bias[e + 1u]));
+        }
+        uint32_t word = nvmoe_f32_to_bf16(lo);
+        if (e + 1u < outputs) word |= nvmoe_f32_to_bf16(hi) << 16;
+        logits[(size_t)t * out_words + e / 2u] = word;
+    }
+}
+
 template <int TT, int ET, int DEPTH>
 __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __restrict__ x,
                                                            const uint16_t* __restrict__ w,
@@ -299,48 +349,55 @@ __global__ void __launch_bounds__(64) router_linear_kernel(const uint16_t* __res
             }
         }
     }
-    // butterfly step 32: lanes v and v^32 live in different warps
-    if (v >= 32u) {
-#pragma unroll
-        for (int a = 0; a < TT; a++)
-#pragma unroll
-            for (int b = 0; b < ET; b++) fold[a * ET + b][v - 32u] = acc[a][b];
-    }
-    __syncthreads();
-    if (v < 32u) {
-#pragma unroll
-        for (int a = 0; a < TT; a++)
-#pragma unroll
-            for (int b = 0; b < ET; b++) {
-                float sum = warp_butterfly_sum(__fadd_rn(acc[a][b], fold[a * ET + b][v]));
-                if (v == 0u) result[a * ET + b] = sum;
-            }
-    }
-    __syncthreads();
-    // pack pairs of outputs into words; ET is even so a word never straddles two blocks
-    const uint32_t out_words = (outputs + 1u) / 2u;
-    for (uint32_t i = v; i < TT * (ET / 2); i += 64u) {
-        uint32_t a = i / (ET / 2), bw = i % (ET / 2);
-        uint32_t t = t0 + a, e = e0 + 2u * bw;
-        if (t >= tokens || e >= outputs) continue;
-        float lo = result[a * ET + 2u * bw];
-        float hi = result[a * ET + 2u * bw + 1u];
-        if (bias) {
-            lo = __fadd_rn(lo, nvmoe_bf16_to_f32(bias[e]));
-            if (e + 1u < outputs) hi = __fadd_rn(hi, nvmoe_bf16_to_f32(bias[e + 1u]));
-        }
-        uint32_t word = nvmoe_f32_to_bf16(lo);
-        if (e + 1u < outputs) word |= nvmoe_f32_to_bf16(hi) << 16;
-        logits[(size_t)t * out_words + e / 2u] = word;
-    }
+    fold_and_store<TT, ET>(acc, fold, result, bias, logits, t0, e0, tokens, outputs);
 }
 
-// One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the
-// instruction itself.
-__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
-    float d;
-    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
-    return d;
+// The same sums for small calls of aligned rows, which wait for the latency of the rows' loads and for the lines of code: the rows are staged whole in shared
+// memory by 16-byte asynchronous copies, all under way at once without a register, and a short loop adds them up (4 to 12 KB of code where the loads through
+// registers take 16 to 27).
+constexpr uint32_t kStagedHidden = 8192u;  // (two blocks of six rows an SM)
+
+template <int TT, int ET>
+__global__ void __launch_bounds__(64) router_linear_staged_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const uint16_t* __restrict__ bias,
+                                                                  uint32_t* __restrict__ logits, uint32_t tokens, uint32_t hidden, uint32_t outputs, CallStart start) {
+    extern __shared__ __align__(16) uint32_t stage[];  // [token rows, then output rows][words]
+    __shared__ float fold[TT * ET][32];
+    __shared__ float result[TT * ET];
+    const uint32_t v = threadIdx.x, t0 = blockIdx.y * TT, e0 = blockIdx.x * ET, words = hidden / 2u;
+    grid_dependency_sync();
+    begin_call(start);
+#pragma unroll 1
+    for (uint32_t r = 0; r < TT + ET; r++) {  // (rows past the last ones repeat them: their sums are not stored)
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(r < TT ? x : w) + (size_t)(r < TT ? min(t0 + r, tokens - 1u) : min(e0 + r - TT, outputs - 1u)) * words;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + r * words);
+#pragma unroll 4
+        for (uint32_t c = 4u * v; c < words; c += 256u)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4u * c), "l"(row + c) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    float acc[TT][ET];
+#pragma unroll
+    for (int a = 0; a < TT; a++)
+#pragma unroll
+        for (int b = 0; b < ET; b++) acc[a][b] = 0.0f;
+#pragma unroll 4
+    for (uint32_t c = v; c < words; c += 64u) {  // (the order of the loads through registers: the same sums bit for bit)
+        uint32_t xv[TT], wv[ET];
+#pragma unroll
+        for (int a = 0; a < TT; a++) xv[a] = stage[a * words + c];
+#pragma unroll
+        for (int b = 0; b < ET; b++) wv[b] = stage[(TT + b) * words + c];
+#pragma unroll
+        for (int a = 0; a < TT; a++)
+#pragma unroll
+            for (int b = 0; b < ET; b++) acc[a][b] = fma_bf16((uint16_t)xv[a], (uint16_t)wv[b], acc[a][b]);
+#pragma unroll
+        for (int a = 0; a < TT; a++)
+#pragma unroll
+            for (int b = 0; b < ET; b++) acc[a][b] = fma_bf16((uint16_t)(xv[a] >> 16), (uint16_t)(wv[b] >> 16), acc[a][b]);
+    }
+    fold_and_store<TT, ET>(acc, fold, result, bias, logits, t0, e0, tokens, outputs);
 }
 
 // The same projection for large batches, bound by the multiply-adds: an SM does 128 a clock, and every other instruction of
@@ -495,6 +552,8 @@ bool router_is_small(const RouterLaunch& p) {
 
 void configure_router_kernels() {
     cudaFuncSetAttribute(router_linear_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouterTileBytes);
+    cudaFuncSetAttribute(router_linear_staged_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * kStagedHidden * 2);
+    cudaFuncSetAttribute(router_linear_staged_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kStagedHidden * 2);
 }
 
 void launch_router(const RouterLaunch& p, cudaStream_t stream) {
@@ -526,8 +585,23 @@ void launch_router(const RouterLaunch& p, cudaStream_t stream) {
 
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
                           uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream) {
-    if (tokens <= 256u) {
-        const dim3 grid((outputs + 3u) / 4u, (tokens + 1u) / 2u), wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
+    const bool aligned = hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u;
+    const dim3 narrow((outputs + 1u) / 2u, tokens), grid((outputs + 3u) / 4u, (tokens + 1u) / 2u);
+    if (tokens <= 256u && aligned && hidden <= kStagedHidden && narrow.x * narrow.y <= 256u) {
+        // Staged rows, one token by two outputs a block, while that makes few blocks: each has half a row less to wait for and a quarter of the sums. Layers,
+        // us, rows through registers / staged 2 x 4 / 1 x 2: 1 token of 32 experts of 2880 columns 26.8 / 26.5 / 25.3, 7 tokens 32.9 / 32.6 / 31.2, 16 (256
+        // blocks) 35.9 / 35.4 / 34.5; 128 experts, 1 token 30.7 / 28.8 / 27.5, 4 28.2 / 27.8 / 27.5, but 5 (320 blocks) 29.0 / 28.8 / 29.8; 64 experts, 9
+        // tokens (288) 29.3 / 28.9 / 29.3; 256 experts of 7168 columns, 1 token 59.3 / 57.6 / 56.4; of 1024 columns 30.2 / 30.3 / 29.6; 8 experts of 256
+        // columns, 64 tokens 23.1 / 23.5 / 22.7.
+        launch_chained(router_linear_staged_kernel<1, 2>, narrow, dim3(64), 3u * hidden * 2u, stream, x, w, bias, logits, tokens, hidden, outputs, start);
+    } else if (tokens <= 256u && aligned && hidden >= 1536u && hidden <= kStagedHidden && grid.x * grid.y <= 2u * 148u) {
+        // Staged rows, 2 x 4, of long rows while every block finds room at once (at 7168 columns an SM holds two). Layers, us, through registers / staged: 64
+        // tokens of 32 experts of 2880 columns 39.5 / 39.1, 8 of 256 experts of 7168 77.8 / 75.2, 10 of 64 of 4096 45.9 / 44.1, 40 of 64 of 1536 (160
+        // blocks) 38.2 / 37.6; on the other side of the line 16 tokens of 32 of 1024 columns 23.9 / 24.2, 128 of 32 of 2880 (512 blocks) 45.4 / 45.4,
+        // 18 of 256 of 7168 (576) 87.9 / 90.0, 64 of 128 of 2880 (1024) 75.7 / 78.0.
+        launch_chained(router_linear_staged_kernel<2, 4>, grid, dim3(64), 6u * hidden * 2u, stream, x, w, bias, logits, tokens, hidden, outputs, start);
+    } else if (tokens <= 256u) {
+        const dim3 wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
         // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, but an
         // SM holds eight of its blocks and takes as long for one as for eight, where the time of 2 x 4 tiles grows with
         // their number: the wide ones when they fill most of a first wave, and not just over it. Wide / small tiles inside
@@ -538,16 +612,14 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
             launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else if (grid.x * grid.y <= 4u * 148u && (hidden > 2048u || (hidden > 1024u && grid.x * grid.y <= 148u))) {
-            // Few blocks of long rows: a call waits for the latency of their loads, so that 24 steps (of 128 columns) are under way instead of 8,
-            // which shorter rows gain from only where an SM has one block. Layers, us, 8 / 24: one token of 32 experts of 2880 columns 29.4 / 28.6,
-            // 64 tokens (256 blocks) 38.2 / 37.8, 100 45.6 / 44.9; of 2304 27.9 / 27.1, 34.5 / 34.0, 40.9 / 40.3; of 2048 27.0 / 26.8, 32.4 / 32.5, 37.6 /
-            // 37.6; of 1536 25.6 / 25.1, 30.2 / 30.5, 33.2 / 33.8; of 1088 24.6 / 24.1, 28.8 / 28.9, 31.8 / 32.3; 16 tokens (64 blocks) 26.7 / 26.5; rows
-            // of 512, which are four steps, 25.1 / 25.5. Beyond four blocks an SM 24 steps lose: 64 tokens of 128 experts of 2880 columns 64.1 / 65.9.
+            // Few blocks of long rows, but too many to be staged, or unaligned: a call waits for the latency of their loads, so that 24 steps (of 128
+            // columns) are under way instead of 8. Layers, us, 8 / 24: 100 tokens of 32 experts of 2880 columns 45.6 / 44.9, of 2304 40.9 / 40.3, of 2048
+            // 37.6 / 37.6, of 1536 33.2 / 33.8. Beyond four blocks an SM 24 steps lose: 64 tokens of 128 experts of 2880 columns 64.1 / 65.9.
             launch_chained(router_linear_kernel<2, 4, 24>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else {
             launch_chained(router_linear_kernel<2, 4, 8>, grid, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         }
-    } else if (hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u) {
+    } else if (aligned) {
         dim3 grid((outputs + kTileOutputs - 1u) / kTileOutputs, (tokens + kTileTokens - 1u) / kTileTokens);
         launch_chained(router_linear_tiled_kernel, grid, dim3(256), kRouterTileBytes, stream, x, w, bias, logits, tokens, hidden, outputs, start);
     } else {
