@@ -602,14 +602,17 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         launch_chained(router_linear_staged_kernel<2, 4>, grid, dim3(64), 6u * hidden * 2u, stream, x, w, bias, logits, tokens, hidden, outputs, start);
     } else if (tokens <= 256u) {
         const dim3 wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
-        // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, but an
-        // SM holds eight of its blocks and takes as long for one as for eight, where the time of 2 x 4 tiles grows with
-        // their number: the wide ones when they fill most of a first wave, and not just over it. Wide / small tiles inside
-        // a layer call, us by wide blocks per SM: 4.1 195.3 / 191.4 (hidden 7168), 114.1 / 112.4 (2880); 4.5 197.2 /
-        // 197.7, 120.3 / 120.3; 5.2 197.5 / 203.1, 114.3 / 116.8; 6.5 209.5 / 213.2; 8.2 226.0 / 225.6; 9.1 228.4 /
-        // 231.5. By itself at 8.4 blocks 9.8 / 9.1 (hidden 512) and 20.1 / 18.4 (2880), at 9.1 39.6 / 41.8 (7168).
+        // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, and an SM takes as long for one of its
+        // blocks as for all that it holds, where the time of 2 x 4 tiles grows with their number. With eight steps under way an SM holds six wide blocks,
+        // with four eight: the most steps that let one wave take the call, from three blocks an SM on, and four steps again once a second wave is full.
+        // Layers, us, small tiles / wide of four / of eight steps, by wide blocks an SM: 2.6 135.8 / 137.4 / 137.2 (hidden 7168) and 62.7 / 62.9 / 62.4
+        // (2880); 3.0 150.2 / 149.8 / 149.2 and 64.0 / 64.3 / 63.3; 4.3 164.8 / 169.2 / 164.3 and 67.1 / 66.5 / 66.4; 4.8 169.3 / 171.0 / 166.6 and 67.9 /
+        // 68.5 / 66.7; 5.2 - / 170.5 / 167.2 and - / 69.9 / 67.9; 5.8 - / 175.8 / 173.9 and - / 73.6 / 72.4; 6.1 - / 74.1 / 76.7; 6.9 - / 194.1 / 201.1.
+        // Four steps against small tiles further on: 8.2 225.6 / 226.0 (small / wide), 9.1 231.5 / 228.4.
         const uint32_t blocks = wide.x * wide.y;
-        if (blocks >= 5u * 148u && (blocks <= 8u * 148u || blocks >= 9u * 148u)) {
+        if (blocks >= 3u * 148u && blocks <= 6u * 148u) {
+            launch_chained(router_linear_kernel<4, 8, 8>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
+        } else if ((blocks > 6u * 148u && blocks <= 8u * 148u) || blocks >= 9u * 148u) {
             launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else if (grid.x * grid.y <= 4u * 148u && (hidden > 2048u || (hidden > 1024u && grid.x * grid.y <= 148u))) {
             // Few blocks of long rows, but too many to be staged, or unaligned: a call waits for the latency of their loads, so that 24 steps (of 128

@@ -1,5 +1,5 @@
 """The router projection of small calls with its rows staged in shared memory, against the CPU checker: the same bits on both sides of each line of its rule (blocks of one token by
-two outputs, of two by four, the loads through registers), with odd tokens and outputs, rows that fill no whole step and the longest staged rows."""
+two outputs, of two by four, the loads through registers in small and wide tiles), with odd tokens and outputs, rows that fill no whole step and the longest staged rows."""
 import numpy as np
 import pytest
 
@@ -12,9 +12,10 @@ pytestmark = pytest.mark.gpu
 ONE_BY_TWO = [(1, 256, 2), (1, 2880, 33), (3, 544, 31), (128, 288, 4), (1, 8192, 31), (2, 96, 255)]
 TWO_BY_FOUR = [(5, 1536, 131), (8, 1536, 295), (3, 8192, 255), (65, 2880, 33)]
 THROUGH_REGISTERS = [(129, 288, 4), (9, 1504, 131), (9, 1536, 259), (2, 8224, 9)]
+WIDE = [(221, 320, 63), (147, 1088, 192), (223, 288, 127), (245, 320, 113)]  # tiles of 4 x 8: 448 and 888 blocks with eight steps, 896 and 930 with four
 
 
-@pytest.mark.parametrize("tokens,hidden,outputs", ONE_BY_TWO + TWO_BY_FOUR + THROUGH_REGISTERS)
+@pytest.mark.parametrize("tokens,hidden,outputs", ONE_BY_TWO + TWO_BY_FOUR + THROUGH_REGISTERS + WIDE)
 def test_staged_projection_is_bit_exact(tokens, hidden, outputs):
     rng = np.random.default_rng(tokens * 1000 + outputs)
     x = synthetic.f32_to_bf16(rng.standard_normal((tokens, hidden), dtype=np.float32))
