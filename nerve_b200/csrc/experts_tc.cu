@@ -927,8 +927,8 @@ __global__ void __launch_bounds__(32) build_tensormaps_kernel(const ExpertPtrs* 
 // x 4 K blocks, a thread 4 rows of one K block and one 16-byte store. The last block writes the pointers and the tensor
 // maps, a warp each. With scale blocks of 32 or 128 columns (LANES = block / 16; 0: none) further blocks quantise the input, a warp 512
 // columns of one row, so that the launch takes little longer than that alone: bound by the latency of a load and a
-// store; a warp takes a second piece, whose load is under way with the first's, where the pieces are more than a wave of blocks (777 rows of 7168 columns 4.1 us, two
-// waves, before). Block of 777 x 7168 x 2048: 114.0 us with the quantisation in a launch of its own, 107 here.
+// store; a warp takes a second piece, whose load is under way with the first's, where the pieces are more than a wave of blocks. Block of 777 x 7168 x 2048: 114.0 us
+// with the quantisation in a launch of its own, 107 here; later 84.4 with one piece or two by blocks of 1.6 waves, 82.9 by one wave.
 constexpr uint32_t kDenseKBlocks = 4u, kDenseThreads = 128u;
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kDenseThreads) dense_prepare_kernel(DensePrepare p, uint32_t k_blocks, uint32_t retile_blocks) {
@@ -1201,8 +1201,11 @@ bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_
     const bool quantises = dense_prepare_quantises(p, act_block);
     // (without rows to quantise, as many blocks as the schedule's lists ask for)
     uint32_t others = quantises ? (uint32_t)((warps + 3u) / 4u) : (p.tokens + kDenseThreads - 1u) / kDenseThreads;
-    // A warp takes a second piece of a row, and more, rather than that a second wave of blocks is needed
-    const uint32_t room = 148u * (2048u / kDenseThreads) > retile + 1u + 148u ? 148u * (2048u / kDenseThreads) - retile - 1u : 148u;
+    // A warp takes further pieces of rows, two at a time, rather than that a second wave of blocks is needed (an SM holds 10): while that asks for two rounds
+    // at most. Beyond, 16 blocks an SM, which even out the rounds. Block of 2048 rows of 7168 columns, us, 16 / 10 an SM: 501 tokens 75.6 / 73.8, 777 84.4 /
+    // 82.9, 1200 (1.7 rounds) 99.8 / 99.4, 2048 (2.9) 139.4 / 140.9.
+    const uint32_t wave = 148u * 10u > retile + 1u + 148u ? 148u * 10u - retile - 1u : 148u;
+    const uint32_t room = warps <= 16ull * wave ? wave : 148u * 16u > retile + 1u + 148u ? 148u * 16u - retile - 1u : 148u;
     if (quantises && others > room) others = room;
     const auto kernel = !quantises ? dense_prepare_kernel<0u> : act_block == 32u ? dense_prepare_kernel<2u> : dense_prepare_kernel<8u>;
     launch_chained(kernel, dim3(retile + others + 1u), dim3(kDenseThreads), 0, stream, p, k_blocks, retile);
