@@ -1,5 +1,5 @@
 """Dense linears of few tokens: either side of the lines from which on they run by CTA pairs (25 tokens with 2048 columns and more, 49 with
-fewer), with whole and ragged last tiles of 64 tokens, K and row remainders, and calls of fewer tokens on a plan of more, against the CPU checker."""
+fewer), with whole and ragged last tiles of 64 tokens, K and row remainders, and calls of fewer tokens on a plan of more, against the oracle."""
 import numpy as np
 import pytest
 

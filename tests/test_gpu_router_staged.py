@@ -1,4 +1,4 @@
-"""The router projection of small calls with its rows staged in shared memory, against the CPU checker: the same bits on both sides of each line of its rule (blocks of one token by
+"""The router projection of small calls with its rows staged in shared memory, against the oracle: the same bits on both sides of each line of its rule (blocks of one token by
 two outputs, of two by four, the loads through registers in small and wide tiles), with odd tokens and outputs, rows that fill no whole step and the longest staged rows."""
 import numpy as np
 import pytest
