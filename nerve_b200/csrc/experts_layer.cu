@@ -32,6 +32,8 @@ using namespace tc;
 
 // Roles, as in experts_tc.cu: warps 0-3 and 8-15 epilogue, 4 MMA, 5 weights, 6 token scales, 7 token rows and the claims.
 constexpr uint32_t kLayerThreads = 512u, kLayerGroups = 3u, kLayerEpilogueWarps = 4u * kLayerGroups;
+constexpr uint32_t kLayerMapsAhead = 64u;  // up to so many experts a block acquires the gate/up maps before its wait
+constexpr uint32_t kLayerMapWarp = 10u;    // beyond, the epilogue warp that acquires them beside the first copies
 constexpr uint32_t kLayerWatchWarp = 2u;  // the epilogue warp that polls (not on the MMA or TMA warp's scheduler)
 constexpr uint32_t kLayerMaxSlots = 6u;
 constexpr uint32_t kLayerMaxExperts = 2u * kLayerExperts;  // of both stages together
@@ -63,7 +65,8 @@ struct LayerBarriers {
     uint64_t chunk_full[2];   // a claimed chunk is there
     uint64_t chunk_empty[2];  // ... has been read by the four that work by it
     uint64_t drain;
-    uint64_t down_maps;       // the tensor maps of the down weights have been acquired
+    uint64_t gate_maps;       // the tensor maps of the gate/up weights have been acquired
+    uint64_t down_maps;       // those of the down weights
     uint32_t tmem_base;
     uint32_t abort;
     uint32_t format[kLayerMaxSlots];  // of the weights in a slot: 0 packed E2M1, 1 one byte an element
@@ -106,6 +109,9 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     const uint32_t H = g.hidden_size, I = g.intermediate_size;
     const uint32_t G = gridDim.x;
 
+    const uint32_t experts = p.stage[0].work.num_experts;
+    const bool maps_beside = experts > kLayerMapsAhead;
+
     // ---- one-time setup ---------------------------------------------------------------------
     if (threadIdx.x >= 32u && threadIdx.x < 32u + kLayerMaxExperts / 32u) bars->bytes_form[threadIdx.x - 32u] = 0u;
     if (threadIdx.x == 0u) {
@@ -120,7 +126,8 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
             mbar_init(&bars->chunk_empty[a], 4u);
         }
         mbar_init(&bars->drain, 1u);
-        mbar_init(&bars->down_maps, 32u * kLayerEpilogueWarps);
+        mbar_init(&bars->gate_maps, 32u);
+        mbar_init(&bars->down_maps, maps_beside ? 32u : 32u * kLayerEpilogueWarps);
         bars->abort = 0u;
         fence_mbar_init();
     }
@@ -133,14 +140,6 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
-    // (as in experts_tc.cu: a block acquires the tensor maps once, while the kernel ahead still runs; 25 ns a map, so that those of
-    // the down weights are left to epilogue warps that have nothing to do yet)
-    const uint32_t experts = p.stage[0].work.num_experts;
-    auto acquire_maps = [&] {
-        for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) tensormap_acquire(p.stage[0].tmaps + (size_t)m * kWeightMaps * 128u);
-        if (threadIdx.x < 2u) tensormap_acquire(p.stage[threadIdx.x].act_tmap);
-        __syncthreads();
-    };
     // What is read, and counted, before the wait: what stands since earlier calls, or since a launch of this one that had completed
     // when the kernel ahead let this one start. That one waited for all before it, the one that cleared the counters among them (the
     // projection, or the schedule where the quantisation is a launch of its own); where it clears them itself, the claim follows the wait.
@@ -150,7 +149,20 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         const bool bytes = (m < experts ? p.stage[0].work.experts[m].format : p.stage[1].work.experts[m - experts].format) != kFormatCompact;
         if (bytes) atomicOr(&bars->bytes_form[m / 32u], 1u << (m % 32u));
     }
-    acquire_maps();
+    // (as in experts_tc.cu: a block acquires a tensor map once, while the kernel ahead still runs; 13 to 29 ns a map, one after the other, so that those of
+    // the down weights are left to epilogue warps that have nothing to do yet. With many experts one epilogue warp acquires all, a few at a time, and the lane that
+    // issues the copies goes ahead with maps that it acquires itself where that warp is not through: a block that starts late, on an SM that
+    // the kernel ahead still used, had 15 us of maps before its first copy with 257 experts. Layers, us, all ahead / beside: 256 experts of 4096 x 1024, 30
+    // tokens 142.8 / 137.4, 96 260.3 / 256.0; 128 of 2880 x 2880, 64 239.0 / 239.3, 300 315.5 / 313.6; 64 of 4096 x 2048, 50 151.8 / 152.3.)
+    if (!maps_beside)
+        for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) tensormap_acquire(p.stage[0].tmaps + (size_t)m * kWeightMaps * 128u);
+    if (threadIdx.x < 2u) tensormap_acquire(p.stage[threadIdx.x].act_tmap);
+    __syncthreads();
+    if (maps_beside && warp == kLayerMapWarp) {
+#pragma unroll 1
+        for (uint32_t m = lane; m < 2u * experts; m += 32u) tensormap_acquire(p.stage[0].tmaps + (size_t)m * kWeightMaps * 128u);
+        mbar_arrive(&bars->gate_maps);
+    }
     grid_dependency_sync();
     if (warp == 7u && lane == 0u && p.claim_late) claimed = atomicAdd(p.sync, 1u);
     const uint32_t entries[2] = {*p.stage[0].tile_count, *p.stage[1].tile_count};
@@ -176,7 +188,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         // ===== weights and their scales (one lane) =====
         if (lane == 0u) {
             uint32_t slot = 0u, empty_parity = 1u;
-            bool alive = true;
+            bool alive = true, maps_stand = !maps_beside;
             auto run = [&](auto tag, uint32_t id) {
                 constexpr uint32_t phase = decltype(tag)::value;
                 // (debug) leave out the very first arrival of chunk 0 or 1: its consumer's bounded wait must then give up
@@ -205,6 +217,10 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
                     const uint8_t* scales2 = row_tile + 1u < s.row_tiles ? scales + (size_t)s.stages * scale_stride : scales;
                     const uint8_t* maps = e.tmaps + (size_t)expert * (phase == 0u ? 2u : 1u) * kWeightMaps * 128u;
                     const uint32_t box_bytes = format == 0u ? kTmaBoxBytes : 2u * kTmaBoxBytes;
+                    if (phase == 0u && !maps_stand && !(maps_stand = mbar_test(&bars->gate_maps, 0u))) {
+                        tensormap_acquire(maps);
+                        tensormap_acquire(maps + kWeightMaps * 128u);
+                    }
                     for (uint32_t ks = 0; ks < s.stages; ks++) {
                         if (!mbar_wait(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
                             alive = false;
@@ -466,9 +482,12 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         const bool whole_block = g.act_block == 128u;  // the scale block of the down operands is the tile's 128 rows
         uint32_t acc_it = 0u, set_it = 0u;
         bool alive = true;
-        for (uint32_t m = group * 128u + quad * 32u + lane; m < experts; m += 32u * kLayerEpilogueWarps)
-            tensormap_acquire(p.stage[1].tmaps + (size_t)m * kWeightMaps * 128u + 256u);
-        mbar_arrive(&bars->down_maps);
+        if (!maps_beside || warp == kLayerMapWarp) {
+            const uint32_t first = maps_beside ? lane : group * 128u + quad * 32u + lane, step = maps_beside ? 32u : 32u * kLayerEpilogueWarps;
+#pragma unroll 1
+            for (uint32_t m = first; m < experts; m += step) tensormap_acquire(p.stage[1].tmaps + (size_t)m * kWeightMaps * 128u + 256u);
+            mbar_arrive(&bars->down_maps);
+        }
         for (uint32_t k = 0; alive; k++) {
             if (warp == kLayerWatchWarp) {
                 if (lane == 0u) *reinterpret_cast<volatile uint32_t*>(&bars->epilogue_chunk[k & 1u]) = chunk_at(k);
