@@ -435,8 +435,8 @@ int nvmoe_plan_debug_cta_trace(nvmoe_plan* plan, uint64_t* out, uint32_t max_cta
 /* The token tile that a call of batch_width tokens takes in the tensor-core kernels of a stage (0 gate/up, 1 down): operand rows
  * per tile, and whether a CTA pair works on it. No reference counterpart. */
 int nvmoe_plan_debug_token_tile(const nvmoe_plan* plan, uint32_t stage, uint32_t batch_width, uint32_t* rows, uint32_t* pair);
-/* Makes CTA 0 (enabled = 1) or CTA 1 (2) of the tensor-core expert kernels leave out its first pipeline-stage arrival, so that its
- * consumer's bounded wait runs out: the way the give-up path (nvmoe_plan_set_wait_limit) is tested
+/* Makes CTA 0 (enabled = 1) or CTA 1 (2) of the tensor-core expert kernels, or CTA 0 of the matrix product that a large layer
+ * call's projection starts with (3), leave out its first pipeline-stage arrival, so that its consumer's bounded wait runs out: the way the give-up path (nvmoe_plan_set_wait_limit) is tested
  * without faulting or hanging anything. The call's output is incomplete and NVMOE_STATUS_WAIT_EXPIRED is
  * raised; switch it off again for the next call. */
 int nvmoe_plan_debug_withhold_arrival(nvmoe_plan* plan, int enabled);

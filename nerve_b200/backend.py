@@ -318,8 +318,8 @@ class MoePlan:
         self._call("nvmoe_plan_set_wait_limit", clock_cycles)
 
     def debug_withhold_arrival(self, enabled: int) -> None:
-        """Test aid: CTA 0 (1 or True) or CTA 1 (2) of the expert kernels leaves out one stage arrival, so that a bounded wait
-        runs out."""
+        """Test aid: CTA 0 (1 or True) or CTA 1 (2) of the expert kernels, or CTA 0 of a large call's router product (3), leaves
+        out one stage arrival, so that a bounded wait runs out."""
         self._call("nvmoe_plan_debug_withhold_arrival", int(enabled))
 
     def debug_token_tile(self, stage: int, batch_width: int) -> tuple[int, bool]:

@@ -657,7 +657,7 @@ int nvmoe_plan_set_wait_limit(nvmoe_plan* p, uint64_t clock_cycles) {
 
 int nvmoe_plan_debug_withhold_arrival(nvmoe_plan* p, int enabled) {
     if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
-    p->debug_flags = enabled == 2 ? 2u : enabled ? 1u : 0u;
+    p->debug_flags = enabled == 2 ? 2u : enabled == 3 ? 4u : enabled ? 1u : 0u;
     return NVMOE_OK;
 }
 
@@ -1631,6 +1631,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         filter.scratch = p->filter.as<float>();
         filter.hidden = g.hidden_size;
         filter.wait_cycles = p->wait_cycles;
+        filter.withhold = (p->debug_flags & 4u) != 0u;
         filter.start = start;
         filters = launch_router_filter(router, filter, st);
         if (filters) p->launches++;

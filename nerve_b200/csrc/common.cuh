@@ -164,6 +164,7 @@ struct RouterFilter {
     float* scratch;              // router_filter_floats of them
     uint32_t hidden;
     long long wait_cycles;
+    bool withhold;  // (debug) one stage is left out
     CallStart start;
 };
 void configure_router_filter();
@@ -326,7 +327,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     uint32_t* tile_count;        // tensor path scratch: one word
     uint32_t tokens;             // upper bound (max over what control may hold)
     long long wait_cycles;       // tensor path: clock cycles after which a bounded in-kernel wait gives up
-    uint32_t debug_flags;        // tensor path: bit n = CTA n (0 or 1) leaves out its first stage arrival (exercises the give-up path)
+    uint32_t debug_flags;        // tensor path: bit n = CTA n (0 or 1) leaves out its first stage arrival (exercises the give-up path); bit 2: RouterFilter.withhold
     nvmoe_geometry g;
 };
 void configure_simt_kernels();

@@ -48,6 +48,7 @@ struct FilterKernel {
     uint32_t* status;
     uint32_t tokens, hidden, outputs, n, slots, tmem_columns;
     long long wait_cycles;
+    bool withhold;  // (debug) the first CTA leaves out its first stage, whose waits must then give up
     CallStart start;
 };
 
@@ -115,16 +116,17 @@ __global__ void __launch_bounds__(kFilterThreads, 1) router_filter_kernel(const 
     const uint32_t tmem = bars.tmem_base, token0 = blockIdx.x * kFilterTokens;
     grid_dependency_sync();
     begin_call(p.start);
-    bool in_flight = false;
     if (warp == 0u) {
         if (lane == 0u) {
             uint32_t slot = 0u, parity = 1u;
             for (uint32_t b = block0; b < block1; b++) {
                 if (!mbar_wait(&bars.empty[slot], parity, abort_flag, p.wait_cycles)) break;
                 const uint32_t at = smem_u32(smem) + slot * stage_bytes;
-                mbar_arrive_expect_tx(&bars.full[slot], stage_bytes);
-                tma_load_2d(at, &x_map, (int)(b * kFilterColumns), (int)token0, &bars.full[slot]);
-                tma_load_2d(at + x_bytes, &w_map, (int)(b * kFilterColumns), 0, &bars.full[slot]);
+                if (!p.withhold || b != 0u || blockIdx.x != 0u) {
+                    mbar_arrive_expect_tx(&bars.full[slot], stage_bytes);
+                    tma_load_2d(at, &x_map, (int)(b * kFilterColumns), (int)token0, &bars.full[slot]);
+                    tma_load_2d(at + x_bytes, &w_map, (int)(b * kFilterColumns), 0, &bars.full[slot]);
+                }
                 if (++slot == p.slots) {
                     slot = 0u;
                     parity ^= 1u;
@@ -148,16 +150,15 @@ __global__ void __launch_bounds__(kFilterThreads, 1) router_filter_kernel(const 
                     tc_mma_bf16(tmem + acc * p.n, a + 2u * k, w + 2u * k, idesc, at_chunk != 0u || k != 0u ? 1u : 0u);
                 tc_commit(&bars.empty[slot]);
                 if (at_chunk + 1u == kFlushBlocks || b + 1u == block1) tc_commit(&bars.acc_full[acc]);
-                in_flight = true;
                 if (++slot == p.slots) {
                     slot = 0u;
                     parity ^= 1u;
                 }
             }
-            if (in_flight && *abort_flag) {
-                tc_commit(&bars.drain);
-                mbar_wait_winddown(&bars.drain, 0u, kWinddownCycles);
-            }
+            // (nothing of this CTA may still be reading shared memory or using tensor memory when they are released, and another role may give
+            // up when this one is through with its loop)
+            tc_commit(&bars.drain);
+            mbar_wait_winddown(&bars.drain, 0u, kWinddownCycles);
         }
     } else if (warp < 4u) {
         const uint32_t ctas = gridDim.x * gridDim.y;
@@ -635,6 +636,7 @@ bool launch_router_filter(const RouterLaunch& router, const RouterFilter& f, cud
     k.tmem_columns = 32u;
     while (k.tmem_columns < 2u * n) k.tmem_columns *= 2u;
     k.wait_cycles = f.wait_cycles;
+    k.withhold = f.withhold;
     k.start = f.start;
     launch_chained(router_filter_kernel, dim3(filter_tiles(router.tokens), filter_splits(router.tokens, f.hidden)), dim3(kFilterThreads),
                    (size_t)k.slots * (kFilterTokens * 128u + n * 128u) + 1024u, stream, x_map, w_map, k);

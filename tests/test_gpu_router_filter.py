@@ -129,11 +129,13 @@ def test_inputs_that_the_product_says_little_of(device, name, shape, changes, ki
     layer.close()
 
 
-def test_a_wait_that_runs_out(device):
-    """The status says so, routes stay in range, and the next call is whole."""
+# (a clock, some, about as many as the product takes, so that the roles give up at different places; every one that does holds its CTA two milliseconds)
+@pytest.mark.parametrize("limit", [1, 300, 1500, 5000])
+def test_waits_that_may_run_out(device, limit):
+    """Whichever of the waits run out: no status but theirs, routes in range, and the next call is whole."""
     layer = Layer(device, "gpt-oss-20b", (2880, 64, 32), 1024)
     want = layer.both_ways()
-    layer.plan.set_wait_limit(1)
+    layer.plan.set_wait_limit(limit)
     buffer = layer.device.resident_buffer_from
     args = dict(router_weights=buffer(layer.w), router_bias=buffer(layer.logit_bias))
     routes, out = buffer(np.zeros((1024, 4), dtype=np.uint32)), buffer(np.zeros((1024, 2880), dtype=np.uint16))
@@ -145,5 +147,30 @@ def test_a_wait_that_runs_out(device):
     layer.plan.set_wait_limit(0)
     got = layer.both_ways()
     for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    layer.close()
+
+
+@pytest.mark.parametrize("name,shape,tokens", [("gpt-oss-20b", (2880, 64, 32), 1024), ("gpt-oss-20b", (2880, 64, 128), 2051), ("deepseek-v3", (2560, 128, 64), 1300)])
+def test_a_copy_that_does_not_come(device, name, shape, tokens):
+    """The first CTA of the product waits for a stage that is left out: the status says so, routes are in range, the other CTAs' tokens are whole, and so is
+    the next call."""
+    layer = Layer(device, name, shape, tokens)
+    want = layer.both_ways()
+    layer.plan.set_wait_limit(2_000_000)  # about a millisecond
+    layer.plan.debug_withhold_arrival(3)
+    buffer = lambda a: None if a is None else device.resident_buffer_from(a)
+    cfg = layer.cfg
+    routes, out = buffer(np.zeros((tokens, cfg.total_k), dtype=np.uint32)), buffer(np.zeros((tokens, cfg.hidden), dtype=np.uint16))
+    layer.plan.layer(tokens, layer.bank, buffer(layer.x), out, routes_out=routes, router_weights=buffer(layer.w), router_bias=buffer(layer.logit_bias),
+                     bias=buffer(layer.select_bias))
+    device.synchronize(timeout_ns=20_000_000_000)
+    assert layer.plan.status() == 8
+    got = routes.read(np.uint32)
+    assert (got & 0xffff).max() < cfg.total_experts
+    np.testing.assert_array_equal(got.reshape(tokens, -1)[128:], want[0].reshape(tokens, -1)[128:])
+    layer.plan.debug_withhold_arrival(0)
+    layer.plan.set_wait_limit(0)
+    for a, b in zip(layer.both_ways(), want):
         np.testing.assert_array_equal(a, b)
     layer.close()
