@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(1024) route_schedule_kernel(RouterLaunch route
 }
 
 // ---- small calls: operands and schedule side by side -------------------------------------------------------
-// A layer call of at most 1024 routes of all experts, a route a thread: the gate/up operands (place_operands_kernel) are made ahead of the
+// A layer call of at most 1024 routes of all experts, a route a thread, of not too many a token (places_operands): the gate/up operands (place_operands_kernel) are made ahead of the
 // schedule (small_schedule_kernel) instead of behind it, and the two run at the same time.
 //
 // What a block of operands has to know of the schedule are the places of its own tokens' routes, which it counts itself: a place is the number
@@ -934,6 +934,7 @@ __global__ void __launch_bounds__(1024) place_operands_kernel(const __grid_const
             if (stage == 1u && keys[0][i] < 0xffff0000u) continue;  // (uniform) the down place is asked for only where gate/up skips the route
             const uint32_t mine = keys[stage][i];
             uint32_t before = 0u;
+#pragma unroll 4
             for (uint32_t j = lane; j < count; j += 32u) before += keys[stage][j] < mine ? 1u : 0u;
             before = __reduce_add_sync(0xffffffffu, before);
             if (lane == 0u) places[stage][n] = mine < 0xffff0000u ? before : kUnboundSlot;
@@ -1441,11 +1442,28 @@ static size_t place_operands_smem_bytes(const LayerSchedule& s, const OperandRow
     return (2u * (size_t)s.tokens * s.K + 2u * place_words(place_operands_threads(s, routed) / 32u, o.chunks, s.K)) * sizeof(uint32_t);
 }
 
+// Which calls. A block ranks the routes of its own tokens, each by a pass over all routes, and a warp stores a piece of a row as often as its token has routes:
+// with many routes a token and few pieces a row these take longer than what stands beside them. `steps` are a warp's passes, in 32 routes. Layers of 64
+// experts, us, in turn / beside: 16 routes a token 64 tokens of 512 columns (steps 512) 38.1 / 50.8, of 1024 (288) 42.0 / 47.3, of 2048 (160) 50.6 / 52.6, of
+// 2880 (128) 59.6 / 59.7; 25 tokens of 2048 (65) 39.1 / 40.9; 12 routes 66 tokens of 2048 (100) 47.1 / 47.4, of 2880 (75) 55.9 / 54.7; 8 routes 128 tokens
+// of 512 (256) 35.6 / 38.6, of 1024 (160) 40.1 / 38.7, 50 of 512 (104) 29.5 / 30.7, of 1024 (65) 32.0 / 31.2; 6 routes 170 of 512 (192) 35.6 / 36.9, 133 (150) 34.0 /
+// 34.5, 66 (78) 29.2 / 28.9; 4 routes 256 (128) 37.2 / 35.7, 150 (76) 30.0 / 27.9; 2 routes 512 (64) 36.1 / 32.1. By blocks of eight warps 12 routes 21 tokens of 512
+// (96) 30.6 / 30.7, of 1024 (64) 32.1 / 30.5; 9 routes 28 of 256 (72) 29.9 / 29.8. Routed in the same blocks, 32 routes 8 of 512 (256) 38.8 / 44.7, 4 of 512 (64)
+// 36.6 / 38.2, of 2048 (48) 44.2 / 43.4; 16 routes 16 of 1024 (72) 35.0 / 34.4, of 512 (128) 33.0 / 34.8, 8 of 512 (64) 30.2 / 30.8, of 1024 (40) 32.5 / 30.8; 12
+// routes 10 of 512 (32) 28.9 / 28.3.
+static bool operands_gain(const LayerSchedule& s, const OperandRows& o, bool routed) {
+    const uint32_t count = s.tokens * s.K, warps = place_operands_threads(s, routed) / 32u;
+    const uint32_t most = place_words(warps, o.chunks, s.K), routes = most < count ? most : count;
+    const uint32_t steps = (routes + warps - 1u) / warps * ((count + 31u) / 32u);
+    if (routed) return steps <= 48u;
+    return steps + 8u * s.K <= (warps <= 8u ? 180u : 100u + count / 8u);
+}
+
 bool places_operands(const LayerSchedule& s, bool routed, const OperandRows& o, uint32_t block) {
     const uint64_t count = (uint64_t)s.tokens * s.K;
     return s.expert_count == 0u && count <= 1024u && small_schedule_words((uint32_t)count, s.num_experts) <= 12u * 1024u &&
            (block == 32u || block == 128u) && o.cols % block == 0u && (reinterpret_cast<uintptr_t>(o.input) & 15u) == 0u &&
-           place_operands_smem_bytes(s, o, routed) <= 48u * 1024u;
+           place_operands_smem_bytes(s, o, routed) <= 48u * 1024u && operands_gain(s, o, routed);
 }
 
 void launch_place_operands(const RouterLaunch* router, const LayerSchedule& s, const OperandRows& o, uint32_t block, cudaStream_t stream) {

@@ -69,6 +69,16 @@ def test_operands_beside_the_schedule(device, name, shape, tokens):
     layer.close()
 
 
+# many routes a token: either side of the lines from which on the schedule comes first (routed in the same blocks, by eight warps, by 32)
+@pytest.mark.parametrize("k,hidden,tokens", [
+    (16, 1088, 8), (16, 512, 8), (32, 2048, 4), (32, 1024, 4), (32, 512, 16), (12, 1024, 21), (12, 512, 21), (6, 1088, 170), (6, 512, 170), (16, 2880, 30), (16, 2880, 64),
+    (32, 512, 32)])
+def test_many_routes_a_token(device, k, hidden, tokens):
+    layer = Layer(device, "gpt-oss-20b", (hidden, 128, 64), tokens, k=k)
+    assert layer.same_both_ways() == 0
+    layer.close()
+
+
 @pytest.mark.parametrize("tokens", [5, 20, 200])
 def test_experts_that_a_stage_lacks(device, tokens):
     layer = Layer(device, "gpt-oss-20b", (1088, 192, 32), tokens)
