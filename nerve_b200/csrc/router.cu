@@ -242,7 +242,7 @@ template <int EPL, bool GROUPS>
 __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
     grid_dependency_sync();
     const uint32_t token = blockIdx.x * 4u + (threadIdx.x >> 5);
-    if (token < p.tokens) route_token<EPL, GROUPS>(p, token);
+    if (token < p.tokens) route_token<false, EPL, GROUPS>(p, token);
 }
 
 // One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the

@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(32 * kRefineWarps, EPL > 4 ? 3 : 4) router_ref
     float my_v;
     if (!valid) return;
     const bool found = pick_experts<EPL>(E, k, val, score, taken, my_e, my_v);
-    finish_token(p.router, token, found, my_e, my_v, rank);
+    finish_token<true>(p.router, token, found, my_e, my_v, rank);
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,

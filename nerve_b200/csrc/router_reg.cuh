@@ -52,15 +52,24 @@ __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uin
     return 0.0f;
 }
 
-// The functions of the scores as calls: a token is routed by code that runs once, and waits for every line of it, so that one copy for all places
-// counts more than what a call costs; for the same reason loops over selections are not unrolled. Layers, times as fast as with the schedule and the
-// quantisation in turn, inlined and unrolled / this way: one token of 32 experts 1.057 / 1.076, seven 1.054 / 1.070, 32 from host buffers 1.025 /
-// 1.036, 64 1.029 / 1.030, tiny 1.060 / 1.055, 96 of 257 1.017 / 1.012 (small_schedule_kernel<1> 34.7 KB / 21.1 KB, router_reg_kernel<8, true> 73 / 32).
-__device__ __noinline__ float route_exp(float v) { return nvmoe_expf(v); }
-__device__ __noinline__ float route_divide(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __noinline__ float route_sigmoid(float v) { return nvmoe_sigmoidf(v); }
-__device__ __noinline__ float route_softplus_root(float v) { return __fsqrt_rn(nvmoe_softplusf(v)); }
-__device__ __noinline__ float route_softcap(float v, float cap) { return __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, cap)), cap); }
+// SHORT, for the blocks of a small call that route beside its operands and schedule, which run their code once and wait for every line of it: the functions
+// of the scores are calls, one copy for all places. Kernels that only route have them inlined. Layers, us, calls everywhere and no loop unrolled / calls in those
+// blocks only: 256 experts of 2048 x 512 in groups, 16 tokens 72.8 / 71.6, 250 151.2 / 149.1; 250 of 64 of 1024 x 512 63.7 / 63.3; 4 of 64 of 256 x 128, 32 routes a
+// token, 42.2 / 36.7; 64 of 8 of 256 x 512 23.2 / 23.1; 33 to 200 of 32 of 2880 x 2880 level. router_reg_kernel by itself, 256 experts in groups: 64 tokens
+// 8.1 / 6.7, 2048 11.5 / 10.4, 16384 50.1 / 51.6; without groups 5.9 / 4.9, 7.9 / 7.8, 35.8 / 38.5; 32 experts, 16384 9.0 / 8.5. (Loops over selections unrolled by four
+// as well: layers of 256 experts 1 to 3 us more.)
+__device__ __noinline__ float call_exp(float v) { return nvmoe_expf(v); }
+__device__ __noinline__ float call_divide(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __noinline__ float call_sigmoid(float v) { return nvmoe_sigmoidf(v); }
+__device__ __noinline__ float call_softplus_root(float v) { return __fsqrt_rn(nvmoe_softplusf(v)); }
+__device__ __noinline__ float call_softcap(float v, float cap) { return __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, cap)), cap); }
+template <bool SHORT> __device__ __forceinline__ float route_exp(float v) { return SHORT ? call_exp(v) : nvmoe_expf(v); }
+template <bool SHORT> __device__ __forceinline__ float route_divide(float a, float b) { return SHORT ? call_divide(a, b) : __fdiv_rn(a, b); }
+template <bool SHORT> __device__ __forceinline__ float route_sigmoid(float v) { return SHORT ? call_sigmoid(v) : nvmoe_sigmoidf(v); }
+template <bool SHORT> __device__ __forceinline__ float route_softplus_root(float v) { return SHORT ? call_softplus_root(v) : __fsqrt_rn(nvmoe_softplusf(v)); }
+template <bool SHORT> __device__ __forceinline__ float route_softcap(float v, float cap) {
+    return SHORT ? call_softcap(v, cap) : __fmul_rn(nvmoe_tanhf(__fdiv_rn(v, cap)), cap);
+}
 
 // ---- the same router with a token's experts in registers ------------------------------------------
 // For up to 32 * EPL experts and at most 32 selections a token; GROUPS: with group-limited masking, for groups of a
@@ -78,7 +87,6 @@ __device__ __forceinline__ bool pick_experts(uint32_t E, uint32_t k, const float
     const uint32_t lane = threadIdx.x & 31u;
     my_e = kUnboundSlot;
     my_v = 0.0f;
-#pragma unroll 1
     for (uint32_t r = 0; r < k; r++) {
         float best = kNegInf, best_v = 0.0f;
         uint32_t best_e = kUnboundSlot;
@@ -105,7 +113,7 @@ __device__ __forceinline__ bool pick_experts(uint32_t E, uint32_t k, const float
 }
 
 // The selection: lane r receives selection r (expert and activated value). False if there are fewer than k selectable scores.
-template <int EPL, bool GROUPS>
+template <bool SHORT, int EPL, bool GROUPS>
 __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t token, uint32_t& my_e, float& my_v) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t E = p.g.routed_experts;
@@ -133,17 +141,17 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
 #pragma unroll
             for (int j = 0; j < EPL; j++) {
                 if (lane + 32u * j < E) {
-                    val[j] = route_exp(__fsub_rn(val[j], smax));
+                    val[j] = route_exp<SHORT>(__fsub_rn(val[j], smax));
                     if (j & 1) hi = __fadd_rn(hi, val[j]); else lo = __fadd_rn(lo, val[j]);
                 }
             }
             const float sden = warp_butterfly_sum(__fadd_rn(lo, hi));
 #pragma unroll
-            for (int j = 0; j < EPL; j++) val[j] = route_divide(val[j], sden);
+            for (int j = 0; j < EPL; j++) val[j] = route_divide<SHORT>(val[j], sden);
         } else {
 #pragma unroll
             for (int j = 0; j < EPL; j++)
-                val[j] = p.g.activation == NVMOE_ACT_SIGMOID ? route_sigmoid(val[j]) : route_softplus_root(val[j]);
+                val[j] = p.g.activation == NVMOE_ACT_SIGMOID ? route_sigmoid<SHORT>(val[j]) : route_softplus_root<SHORT>(val[j]);
         }
 #pragma unroll
         for (int j = 0; j < EPL; j++) {
@@ -159,9 +167,9 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
         for (int j = 0; j < EPL; j++) {
             const uint32_t e = lane + 32u * j;
             float v = val[j];
-            if (p.g.logit_softcap > 0.0f) v = route_softcap(v, p.g.logit_softcap);
+            if (p.g.logit_softcap > 0.0f) v = route_softcap<SHORT>(v, p.g.logit_softcap);
             val[j] = v;
-            score[j] = e < E ? __fadd_rn(sigmoid ? route_sigmoid(v) : v, read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
+            score[j] = e < E ? __fadd_rn(sigmoid ? route_sigmoid<SHORT>(v) : v, read_bias(p.bias, p.g.bias_dtype, e)) : 0.0f;
         }
     }
 
@@ -173,7 +181,6 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
 #pragma unroll
         for (int j = 0; j < EPL; j++) {
             float first = lane + 32u * j < E && score[j] > kNegInf ? score[j] : kNegInf, second = kNegInf;
-#pragma unroll 1
             for (uint32_t o = 1u; o < per; o <<= 1) {
                 const float other_first = __shfl_xor_sync(kFull, first, o), other_second = __shfl_xor_sync(kFull, second, o);
                 second = fmaxf(fminf(first, other_first), fmaxf(second, other_second));
@@ -183,7 +190,6 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
             if (lane / side == (uint32_t)j) my_group = group;  // lane g keeps group g
         }
         uint32_t kept = 0u;
-#pragma unroll 1
         for (uint32_t round = 0; round < p.g.topk_group; round++) {
             const bool open = lane < p.g.n_group && ((kept >> lane) & 1u) == 0u && my_group >= kNegInf;  // (not a NaN)
             const uint32_t winner = warp_best(my_group, open ? lane : kUnboundSlot);
@@ -201,7 +207,6 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
 // The places of a token's selections in ascending order of the experts: lane r < total_k holds selection r.
 __device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total_k) {
     uint32_t rank = 0u;
-#pragma unroll 1
     for (uint32_t q = 0; q < total_k; q++) {
         const uint32_t other = __shfl_sync(0xffffffffu, my_e, q);
         if (other < my_e) rank++;
@@ -219,6 +224,7 @@ __device__ __forceinline__ void order_token(const RouterLaunch& p, bool found, u
 }
 
 // Weights, route words and telemetry of such a token; my_e and rank as above.
+template <bool SHORT>
 __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t token, bool found, uint32_t& my_e, float my_v, uint32_t& rank) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t E = p.g.routed_experts;
@@ -244,9 +250,9 @@ __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t tok
     float w = 0.0f;
     if (kind == NVMOE_ROUTER_SCORE_TOPK) {
         float den = 0.0f;
-#pragma unroll 1
-        for (uint32_t r = 0; p.g.normalize_selected && r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, my_v, r));
-        w = p.g.normalize_selected ? __fmul_rn(route_divide(my_v, den), p.g.routed_scale) : __fmul_rn(my_v, p.g.routed_scale);
+        if (p.g.normalize_selected)
+            for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, my_v, r));
+        w = p.g.normalize_selected ? __fmul_rn(route_divide<SHORT>(my_v, den), p.g.routed_scale) : __fmul_rn(my_v, p.g.routed_scale);
         if (lane >= k && lane < total_k) {
             my_e = E + (lane - k);
             w = p.g.always_weight;
@@ -255,11 +261,10 @@ __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t tok
         const bool sigmoid = kind == NVMOE_ROUTER_TOPK_ROUTED && p.g.activation == NVMOE_ACT_SIGMOID;
         const bool divide = kind == NVMOE_ROUTER_TOPK_SOFTMAX || p.g.normalize_selected || !sigmoid;
         const float maximum = __shfl_sync(kFull, my_v, 0);
-        const float t = sigmoid ? route_sigmoid(my_v) : route_exp(__fsub_rn(my_v, maximum));
+        const float t = sigmoid ? route_sigmoid<SHORT>(my_v) : route_exp<SHORT>(__fsub_rn(my_v, maximum));
         float den = 0.0f;
-#pragma unroll 1
         for (uint32_t r = 0; r < k; r++) den = __fadd_rn(den, __shfl_sync(kFull, t, r));
-        w = divide ? route_divide(t, den) : t;
+        w = divide ? route_divide<SHORT>(t, den) : t;
     }
 
     // ---- ascending expert id, pack, telemetry ----------------------------------------------------
@@ -269,7 +274,6 @@ __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t tok
         if (p.telemetry) atomicAdd(p.telemetry + my_e, 1u);
     }
     if (p.telemetry) {
-#pragma unroll 1
         for (uint32_t q = 0; q < total_k; q++) {
             const uint32_t right = __shfl_sync(kFull, my_e, q);
             if (lane < total_k && my_e < right) {
@@ -280,12 +284,12 @@ __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t tok
     }
 }
 
-template <int EPL, bool GROUPS>
+template <bool SHORT, int EPL, bool GROUPS>
 __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token) {
     uint32_t my_e, rank;
     float my_v;
-    const bool found = select_experts<EPL, GROUPS>(p, token, my_e, my_v);
-    finish_token(p, token, found, my_e, my_v, rank);
+    const bool found = select_experts<SHORT, EPL, GROUPS>(p, token, my_e, my_v);
+    finish_token<SHORT>(p, token, found, my_e, my_v, rank);
 }
 
 }  // namespace

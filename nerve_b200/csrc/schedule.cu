@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(1024) route_schedule_kernel(RouterLaunch route
     layer_schedule_rank_body<1u>(s, [&] {
         grid_dependency_sync();
         const uint32_t token = threadIdx.x >> 5;
-        if (token < router.tokens) route_token<EPL, false>(router, token);
+        if (token < router.tokens) route_token<false, EPL, false>(router, token);
     });
 }
 
@@ -911,9 +911,9 @@ __global__ void __launch_bounds__(1024) place_operands_kernel(const __grid_const
         if (warp < router.tokens) {
             uint32_t e, rank;
             float v;
-            const bool found = select_experts<EPL == 0 ? 1 : EPL, false>(router, warp, e, v);
+            const bool found = select_experts<true, EPL == 0 ? 1 : EPL, false>(router, warp, e, v);
             if (blockIdx.x == 0u) {
-                finish_token(router, warp, found, e, v, rank);
+                finish_token<true>(router, warp, found, e, v, rank);
             } else {
                 order_token(router, found, e, rank);
             }
@@ -990,7 +990,7 @@ __global__ void __launch_bounds__(1024) small_schedule_kernel(const __grid_const
         if (warp < router.tokens) {
             uint32_t mine, rank;
             float v;
-            order_token(router, select_experts<EPL == 0 ? 1 : EPL, false>(router, warp, mine, v), mine, rank);
+            order_token(router, select_experts<true, EPL == 0 ? 1 : EPL, false>(router, warp, mine, v), mine, rank);
             if (lane < s.K) ids[warp * s.K + rank] = mine;
         }
         __syncthreads();
