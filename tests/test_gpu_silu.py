@@ -9,7 +9,8 @@ from oracle import moe_oracle as mo
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("limit", [0.0, 7.0, 100.0, 3e38])
+# (limits that are no bf16 number among them: the bounded gate is then any f32 number)
+@pytest.mark.parametrize("limit", [0.0, 7.0, 100.0, 3e38, 6.9999, 7.1, 0.3, 88.7])
 def test_all_gates(limit):
     device = CudaComputeDevice(0)
     rng = np.random.default_rng(int(limit))
@@ -31,5 +32,20 @@ def test_all_gates(limit):
         number = numbers & ~np.isnan(g / (1 + np.exp(-g)) * up) & ~(np.isinf(up) & (np.abs(g / (1 + np.exp(-g))) < 1e-30))
     got, want = out.read(np.uint16).reshape(gates.shape), mo.silu_multiply(gates, u, limit)
     np.testing.assert_array_equal(got[number], want[number])
+    plan.destroy()
+    device.close()
+
+
+@pytest.mark.parametrize("limit", [0.0, 7.0])
+def test_zeros(limit):
+    """Zeros of either sign by gates and ups of either, small, large and below the exponential's range: the zero that the pinned form makes."""
+    device = CudaComputeDevice(0)
+    zeros, others = np.array([0x0000, 0x8000]), np.array([0x0000, 0x8000, 0x3f80, 0xbf80, 0x0080, 0x8001, 0x4120, 0xc120, 0xc2ae, 0xc2b0, 0xc2b2, 0xc2b4, 0xc2c8, 0x7f7f, 0xff7f, 0x7f00])
+    pairs = [(z, o) for z in zeros for o in others] + [(o, z) for z in zeros for o in others]
+    gates, ups = (np.tile(np.array([p[i] for p in pairs], dtype=np.uint16), (3, 8)) for i in (0, 1))
+    plan = MoePlan.for_config(device, synthetic.MoeConfig("silu", 256, 256, 8, 2, act_block=32), 3)
+    out = device.create_resident_buffer(gates.nbytes)
+    plan.silu_multiply(3, gates.shape[1], device.resident_buffer_from(gates), device.resident_buffer_from(ups), out, limit)
+    np.testing.assert_array_equal(out.read(np.uint16).reshape(gates.shape), mo.silu_multiply(gates, ups, limit))
     plan.destroy()
     device.close()
