@@ -681,11 +681,11 @@ static int check_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hi
 }
 
 static int router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, nvmoe_buffer* logits, const nvmoe_buffer* router_weights,
-                         const nvmoe_buffer* router_bias, const CallStart& start) {
+                         const nvmoe_buffer* router_bias, bool beside, const CallStart& start) {
     const nvmoe_geometry& g = p->g;
     launch_router_linear((const uint16_t*)hidden->ptr, (const uint16_t*)router_weights->ptr,
                          router_bias ? (const uint16_t*)router_bias->ptr : nullptr, (uint32_t*)logits->ptr, T,
-                         g.hidden_size, g.routed_experts, start, p->device->stream);
+                         g.hidden_size, g.routed_experts, beside, start, p->device->stream);
     p->launches++;
     return post_launch(p, "router projection");
 }
@@ -695,7 +695,7 @@ int nvmoe_router_linear(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, n
     if (!p) return NVMOE_ERR_INVALID_ARGUMENT;
     NVMOE_TRY(check_router_linear(p, T, hidden, logits, router_weights, router_bias));
     NVMOE_CUDA(p->device, cudaSetDevice(p->device->ordinal));
-    return router_linear(p, T, hidden, logits, router_weights, router_bias, CallStart{});
+    return router_linear(p, T, hidden, logits, router_weights, router_bias, false, CallStart{});
 }
 
 // checks the router's buffers and fills its launch block
@@ -1637,7 +1637,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         if (filters) p->launches++;
         NVMOE_TRY(post_launch(p, "router projection"));
     }
-    if (projects && !filters) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, start));
+    if (projects && !filters) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, beside, start));
     mark(kStageRoute);
     // (with stage profiling on, the router keeps a launch and a time of its own)
     if (!a->routes_in && !routes_in_schedule) {

@@ -154,7 +154,7 @@ void configure_router_kernels();
 void launch_router(const RouterLaunch& p, cudaStream_t stream);
 bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selections, no groups: route_token covers it
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
-                          uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream);
+                          uint32_t tokens, uint32_t hidden, uint32_t outputs, bool beside, const CallStart& start, cudaStream_t stream);  // (beside: see there)
 
 // router_filter.cu: projection and routing of a large call, of which only the logits that matter are made exactly.
 struct RouterFilter {

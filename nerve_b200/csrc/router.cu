@@ -584,7 +584,7 @@ void launch_router(const RouterLaunch& p, cudaStream_t stream) {
 }
 
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
-                          uint32_t tokens, uint32_t hidden, uint32_t outputs, const CallStart& start, cudaStream_t stream) {
+                          uint32_t tokens, uint32_t hidden, uint32_t outputs, bool beside, const CallStart& start, cudaStream_t stream) {
     const bool aligned = hidden % 8u == 0u && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0u;
     const dim3 narrow((outputs + 1u) / 2u, tokens), grid((outputs + 3u) / 4u, (tokens + 1u) / 2u);
     if (tokens <= 256u && aligned && hidden <= kStagedHidden && narrow.x * narrow.y <= 256u) {
@@ -604,13 +604,16 @@ void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* 
         const dim3 wide((outputs + 7u) / 8u, (tokens + 3u) / 4u);
         // Small tiles for small calls, which need the blocks. A tile of 4 x 8 reads half the bytes from L2 per pair, and an SM takes as long for one of its
         // blocks as for all that it holds, where the time of 2 x 4 tiles grows with their number. With eight steps under way an SM holds six wide blocks,
-        // with four eight: the most steps that let one wave take the call, from three blocks an SM on, and four steps again once a second wave is full.
-        // Layers, us, small tiles / wide of four / of eight steps, by wide blocks an SM: 2.6 135.8 / 137.4 / 137.2 (hidden 7168) and 62.7 / 62.9 / 62.4
-        // (2880); 3.0 150.2 / 149.8 / 149.2 and 64.0 / 64.3 / 63.3; 4.3 164.8 / 169.2 / 164.3 and 67.1 / 66.5 / 66.4; 4.8 169.3 / 171.0 / 166.6 and 67.9 /
-        // 68.5 / 66.7; 5.2 - / 170.5 / 167.2 and - / 69.9 / 67.9; 5.8 - / 175.8 / 173.9 and - / 73.6 / 72.4; 6.1 - / 74.1 / 76.7; 6.9 - / 194.1 / 201.1.
+        // with four eight: the most steps that let one wave take the call, and four steps again once a second wave is full. From three blocks an SM on where
+        // the operands are made beside the schedule (`beside`), else from five: by itself, with the rows in L2, the wide kernel takes longer below that (7168
+        // columns 2.6 17.1 / 20.3 small / wide, 2880 3.5 9.0 / 11.1). Layers, us, small tiles / wide of eight steps, by wide blocks an SM: operands
+        // beside, 7168 columns 3.2 209.1 / 206.2, 3.9 218.0 / 215.5, 4.3 226.0 / 225.2, 5.2 252.7 / 247.6; 2880 columns 3.2 64.3 / 63.1, 4.1 66.2 / 65.5, 4.9 68.6 / 67.5;
+        // 4096 columns 3.1 64.5 / 65.3, 4.1 78.5 / 78.1, 5.1 83.8 / 80.9; else, 2048 columns 3.2 85.4 / 84.5, 4.1 91.9 / 94.1, 4.5 94.2 / 97.8; 4096 columns 3.1
+        // 89.6 / 91.6, 3.5 90.9 / 91.7, 4.1 112.9 / 110.8; 5120 columns 3.7 115.6 / 113.8, 4.1 123.6 / 124.1, 4.3 129.3 / 130.7.
+        // Wide of four / eight steps: 5.2 170.5 / 167.2 and 69.9 / 67.9; 5.8 175.8 / 173.9 and 73.6 / 72.4; 6.1 74.1 / 76.7; 6.9 194.1 / 201.1.
         // Four steps against small tiles further on: 8.2 225.6 / 226.0 (small / wide), 9.1 231.5 / 228.4.
         const uint32_t blocks = wide.x * wide.y;
-        if (blocks >= 3u * 148u && blocks <= 6u * 148u) {
+        if (blocks >= (beside ? 3u : 5u) * 148u && blocks <= 6u * 148u) {
             launch_chained(router_linear_kernel<4, 8, 8>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
         } else if ((blocks > 6u * 148u && blocks <= 8u * 148u) || blocks >= 9u * 148u) {
             launch_chained(router_linear_kernel<4, 8, 4>, wide, dim3(64), 0, stream, x, w, bias, logits, tokens, hidden, outputs, start);
