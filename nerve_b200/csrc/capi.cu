@@ -144,7 +144,7 @@ struct nvmoe_plan {
     bool tma[2] = {false, false};
     bool one_matrix = false;     // the plan of a dense linear's shape
     // scratch of the fused layer call
-    DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev, filter;
+    DeviceArray logits, routes, frames, expert_outputs, controls, hidden_dev, output_dev;
     void* pinned_in = nullptr;
     bool pinned_mapped = false;  // both have the same address on the device
     void* pinned_out = nullptr;
@@ -617,7 +617,7 @@ void nvmoe_plan_destroy(nvmoe_plan* p) {
                           &p->offsets[1], &p->block_hist, &p->bucket_totals, &p->xq, &p->x_scales, &p->iq,
                           &p->i_scales, &p->tile_list, &p->ep_source, &p->layer_sync, &p->clock, &p->tmap_templates, &p->cta_trace, &p->grouped_q[0], &p->grouped_q[1],
                           &p->grouped_e8m0[0], &p->grouped_e8m0[1], &p->position[0], &p->position[1], &p->act_maps, &p->logits, &p->routes, &p->frames, &p->expert_outputs,
-                          &p->controls, &p->hidden_dev, &p->output_dev, &p->filter};
+                          &p->controls, &p->hidden_dev, &p->output_dev};
     for (DeviceArray* a : all) a->release();
     if (p->pinned_in) cudaFreeHost(p->pinned_in);
     if (p->pinned_out) cudaFreeHost(p->pinned_out);
@@ -1482,9 +1482,11 @@ static int ensure_layer_scratch(nvmoe_plan* p) {
     want(p->logits, T * ((g.routed_experts + 1u) / 2u) * 4u);
     want(p->routes, T * p->K * 4u);
     want(p->frames, T * (size_t)p->frame_words * 4u);
-    want(p->expert_outputs, T * p->K * (size_t)g.hidden_size * 2u);
+    // (until the down stage writes them, the projection of a large call has its product where the expert rows go)
+    const size_t outputs = T * p->K * (size_t)g.hidden_size * 2u;
+    const size_t product = router_filter_takes(g, g.max_tokens) ? router_filter_floats(g.max_tokens, g.routed_experts) * 4u : 0u;
+    want(p->expert_outputs, outputs > product ? outputs : product);
     want(p->controls, 64u);
-    if (router_filter_takes(g, g.max_tokens)) want(p->filter, router_filter_floats(g.max_tokens, g.routed_experts) * 4u);
     if (err == cudaSuccess && fresh_frames) err = cudaMemsetAsync(p->frames.ptr, 0, p->frames.bytes, p->device->stream);
     if (err != cudaSuccess)
         return fail(p->device, err == cudaErrorMemoryAllocation ? NVMOE_ERR_OUT_OF_MEMORY : NVMOE_ERR_CUDA,
@@ -1628,7 +1630,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         filter.x = (const uint16_t*)a->hidden->ptr;
         filter.w = (const uint16_t*)a->router_weights->ptr;
         filter.logit_bias = a->router_bias ? (const uint16_t*)a->router_bias->ptr : nullptr;
-        filter.scratch = p->filter.as<float>();
+        filter.scratch = p->expert_outputs.as<float>();
         filter.hidden = g.hidden_size;
         filter.wait_cycles = p->wait_cycles;
         filter.withhold = (p->debug_flags & 4u) != 0u;

@@ -174,3 +174,26 @@ def test_a_copy_that_does_not_come(device, name, shape, tokens):
     for a, b in zip(layer.both_ways(), want):
         np.testing.assert_array_equal(a, b)
     layer.close()
+
+
+@pytest.mark.parametrize("shape,tokens,k,fits", [((1024, 128, 256), 2304, 8, True), ((3584, 64, 256), 2304, 2, True), ((1536, 64, 256), 1400, 1, False)])
+def test_scratch_is_shared_with_the_expert_rows(device, shape, tokens, k, fits):
+    """A plan's first layer call takes what its logits, routes, frames and expert rows need, and nothing for the product where that is no more than the rows."""
+    import torch
+
+    layer = Layer(device, "gpt-oss-20b", shape, tokens, k=k)
+    buffer = device.resident_buffer_from
+    args = dict(router_weights=buffer(layer.w), router_bias=buffer(layer.logit_bias))
+    hidden, out = buffer(layer.x), buffer(np.zeros((tokens, shape[0]), dtype=np.uint16))
+    device.synchronize()
+    before = torch.cuda.mem_get_info(0)[0]
+    layer.plan.layer(tokens, layer.bank, hidden, out, **args)
+    device.synchronize()
+    taken = before - torch.cuda.mem_get_info(0)[0]
+    rows, product = tokens * k * shape[0] * 2, min(8 * tokens, 148 * 128) * (shape[2] + 1) * 4
+    assert (product <= rows) == fits
+    others = tokens * (shape[2] // 2 * 4 + k * 4 + layer.plan.frame_words * 4)
+    scales = shape[2] * 3 * -(-shape[0] // 128) * -(-shape[1] // 128) * 512  # of the experts, in the kernels' order
+    # (each allocation is rounded up to 2 MiB)
+    assert taken <= max(rows, product) + others + scales + (8 << 20), (taken, rows, product, others, scales)
+    layer.close()
