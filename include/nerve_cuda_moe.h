@@ -435,6 +435,15 @@ int nvmoe_plan_debug_cta_trace(nvmoe_plan* plan, uint64_t* out, uint32_t max_cta
 /* The token tile that a call of batch_width tokens takes in the tensor-core kernels of a stage (0 gate/up, 1 down): operand rows
  * per tile, and whether a CTA pair works on it. No reference counterpart. */
 int nvmoe_plan_debug_token_tile(const nvmoe_plan* plan, uint32_t stage, uint32_t batch_width, uint32_t* rows, uint32_t* pair);
+/* 1 if the plan's last layer call made its logits by the tensor-core product and exact sums of those that matter, 0 if every logit was
+ * summed (or the call had no projection). No reference counterpart. */
+int nvmoe_plan_debug_projection(const nvmoe_plan* plan, uint32_t* product);
+/* That product alone, of as many tokens as the plan's calls may have, whatever the rule for calls: [batch_width][experts] sums, the norms of
+ * the token rows (0 for rows of zeros) and of the router's rows, as the refinement uses them, all in host memory; `relative`: the part of the
+ * norms' product within which it takes the sums of the projection to lie; into how many parts the columns are split. Synchronises the
+ * stream. No reference counterpart. */
+int nvmoe_plan_debug_router_product(nvmoe_plan* plan, uint32_t batch_width, const nvmoe_buffer* hidden, const nvmoe_buffer* router_weights,
+                                    float* product, float* row_norms, float* expert_norms, float* relative, uint32_t* splits);
 /* Makes CTA 0 (enabled = 1) or CTA 1 (2) of the tensor-core expert kernels, or CTA 0 of the matrix product that a large layer
  * call's projection starts with (3), leave out its first pipeline-stage arrival, so that its consumer's bounded wait runs out: the way the give-up path (nvmoe_plan_set_wait_limit) is tested
  * without faulting or hanging anything. The call's output is incomplete and NVMOE_STATUS_WAIT_EXPIRED is

@@ -329,6 +329,21 @@ class MoePlan:
         self._call("nvmoe_plan_debug_token_tile", stage, batch_width, ctypes.byref(rows), ctypes.byref(pair))
         return rows.value, bool(pair.value)
 
+    def debug_projection(self) -> bool:
+        """Test aid: whether the last layer call made its logits by the tensor-core product and exact sums of those that matter."""
+        product = ctypes.c_uint32()
+        self._call("nvmoe_plan_debug_projection", ctypes.byref(product))
+        return bool(product.value)
+
+    def debug_router_product(self, batch_width: int, hidden, router_weights, experts: int):
+        """Test aid: that product by itself, the norms of both sides' rows, the bound's factor and the parts that the columns are
+        split into."""
+        product, rows, cols = (np.empty(n, dtype=np.float32) for n in (batch_width * experts, batch_width, experts))
+        relative, splits = ctypes.c_float(), ctypes.c_uint32()
+        self._call("nvmoe_plan_debug_router_product", batch_width, _h(hidden), _h(router_weights), _ptr(product), _ptr(rows), _ptr(cols),
+                   ctypes.byref(relative), ctypes.byref(splits))
+        return product.reshape(batch_width, experts), rows, cols, relative.value, splits.value
+
     def set_profiling(self, enabled: bool) -> None:
         self._call("nvmoe_plan_set_profiling", int(enabled))
 

@@ -3,6 +3,7 @@
 // in the other .cu files of this folder.
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -160,6 +161,7 @@ struct nvmoe_plan {
     uint32_t launches = 0;
     long long wait_cycles = 4000000000ll;  // limit of the bounded in-kernel waits of the tensor path (about 2 s)
     uint32_t debug_flags = 0;
+    bool filtered = false;       // the last layer call's projection was the matrix product
     // dense linears run as one always-selected resource of a plan of their own shape (nvmoe_dense_linear); whatever hangs
     // on a matrix (`set`: pointers, re-tiled scales, tensor map) is made anew by every call, nothing of it is kept
     struct DenseLinear {
@@ -1640,6 +1642,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
         NVMOE_TRY(post_launch(p, "router projection"));
     }
     if (projects && !filters) NVMOE_TRY(router_linear(p, T, a->hidden, logits, a->router_weights, a->router_bias, beside, start));
+    p->filtered = filters;
     mark(kStageRoute);
     // (with stage profiling on, the router keeps a launch and a time of its own)
     if (!a->routes_in && !routes_in_schedule) {
@@ -1899,6 +1902,62 @@ int nvmoe_plan_debug_token_tile(const nvmoe_plan* p, uint32_t stage, uint32_t T,
     const TokenTile tile = token_tile(p, stage == 0u, T);
     *rows = tile.rows;
     *pair = tile.pair ? 1u : 0u;
+    return NVMOE_OK;
+}
+
+int nvmoe_plan_debug_projection(const nvmoe_plan* p, uint32_t* product) {
+    if (!p || !product) return NVMOE_ERR_INVALID_ARGUMENT;
+    *product = p->filtered ? 1u : 0u;
+    return NVMOE_OK;
+}
+
+int nvmoe_plan_debug_router_product(nvmoe_plan* p, uint32_t T, const nvmoe_buffer* hidden, const nvmoe_buffer* router_weights, float* product,
+                                    float* row_norms, float* expert_norms, float* relative, uint32_t* splits) {
+    if (!p || !product || !row_norms || !expert_norms || !relative || !splits) return NVMOE_ERR_INVALID_ARGUMENT;
+    const nvmoe_geometry& g = p->g;
+    nvmoe_device* d = p->device;
+    NVMOE_TRY(check_tokens(p, T));
+    NVMOE_TRY(check_buffer(p, hidden, (size_t)T * g.hidden_size * 2u, "hidden"));
+    NVMOE_TRY(check_buffer(p, router_weights, (size_t)g.routed_experts * g.hidden_size * 2u, "router weights"));
+    if (!router_filter_form(g) || ((reinterpret_cast<uintptr_t>(hidden->ptr) | reinterpret_cast<uintptr_t>(router_weights->ptr)) & 15u) != 0u)
+        return fail(d, NVMOE_ERR_UNSUPPORTED, "no layer call of this geometry, or of such buffers, has its router's product on the tensor cores");
+    NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
+    DeviceArray scratch;
+    cudaError_t err = scratch.ensure(router_filter_floats(T, g.routed_experts) * 4u);
+    RouterLaunch router{};
+    router.g = g;
+    router.tokens = T;
+    router.status = p->status.as<uint32_t>();
+    RouterFilter filter{};
+    filter.x = (const uint16_t*)hidden->ptr;
+    filter.w = (const uint16_t*)router_weights->ptr;
+    filter.scratch = scratch.as<float>();
+    filter.hidden = g.hidden_size;
+    filter.wait_cycles = p->wait_cycles;
+    const bool launched = err == cudaSuccess && launch_router_filter(router, filter, d->stream);
+    const RouterProduct r = router_product_of(filter, T, g.routed_experts);
+    *relative = r.relative;
+    *splits = r.splits;
+    // the parts in the refinement's order
+    std::unique_ptr<float[]> part(new (std::nothrow) float[(size_t)T * r.width]), squares(new (std::nothrow) float[T]);
+    if (!part || !squares) err = cudaErrorMemoryAllocation;
+    if (err == cudaSuccess) err = cudaMemcpyAsync(expert_norms, r.w_norm, (size_t)g.routed_experts * 4u, cudaMemcpyDeviceToHost, d->stream);
+    for (uint32_t s = 0; launched && s < r.splits && err == cudaSuccess; s++) {
+        err = cudaMemcpyAsync(part.get(), r.product + (size_t)s * T * r.width, (size_t)T * r.width * 4u, cudaMemcpyDeviceToHost, d->stream);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(squares.get(), r.x_norm2 + (size_t)s * T, (size_t)T * 4u, cudaMemcpyDeviceToHost, d->stream);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);
+        for (uint32_t t = 0; t < T; t++) {
+            for (uint32_t e = 0; e < g.routed_experts; e++) {
+                const float v = part[(size_t)t * r.width + e];
+                product[(size_t)t * g.routed_experts + e] = s == 0u ? v : product[(size_t)t * g.routed_experts + e] + v;
+            }
+            row_norms[t] = s == 0u || row_norms[t] < 0.0f ? squares[t] : squares[t] < 0.0f ? row_norms[t] : row_norms[t] + squares[t];
+        }
+    }
+    cudaStreamSynchronize(d->stream);
+    scratch.release();
+    if (err != cudaSuccess || !launched) return fail(d, NVMOE_ERR_CUDA, "router product: %s", launched ? cudaGetErrorString(err) : "not launched");
+    for (uint32_t t = 0; t < T; t++) row_norms[t] = row_norms[t] < 0.0f ? 0.0f : std::sqrt(row_norms[t]);
     return NVMOE_OK;
 }
 

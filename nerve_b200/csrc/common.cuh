@@ -168,10 +168,19 @@ struct RouterFilter {
     CallStart start;
 };
 void configure_router_filter();
-bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens);  // the call, if its buffers lie on the 16-byte grid
+bool router_filter_form(const nvmoe_geometry& g);  // whether it can
+bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens);  // ... and does take the call, if its buffers lie on the 16-byte grid
 size_t router_filter_floats(uint32_t max_tokens, uint32_t experts);  // scratch of calls of up to so many tokens
 bool launch_router_filter(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream);  // false: no tensor maps here
 void launch_router_refine(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream);
+struct RouterProduct {  // what the refinement reads (diagnostics)
+    const float* product;  // [splits][tokens][width]
+    const float* x_norm2;  // [splits][tokens]
+    const float* w_norm;   // [experts]
+    uint32_t splits, width;
+    float relative;
+};
+RouterProduct router_product_of(const RouterFilter& f, uint32_t tokens, uint32_t experts);
 
 struct SortScratch {  // schedule.cu: scratch of the counting sort, sized for max_tokens
     uint32_t* block_hist;      // [blocks][buckets]

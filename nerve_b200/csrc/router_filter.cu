@@ -582,10 +582,13 @@ constexpr uint32_t kFilterSplits = 8u;  // at most
 // 2048 135.9 / 134.2; 2048 x 1024 x 32 81.4 / 80.8, 768 59.9 / 60.8; 512 x 2880 x 128 (one round) 110.7 / 113.5, 768 (two) 128.5 / 119.9, 2048 185.1 / 152.9;
 // 257 x 4096 x 64 90.6 / 89.6, 2048 191.0 / 173.3; grouped, 768 x 2048 x 64 111.3 / 115.1, 1536 157.2 / 154.0; 257 x 7168 x 256 324.9 / 320.5, 2048 788 / 673;
 // 2048 x 512 x 16 64.8 / 66.8.
-bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens) {
+bool router_filter_form(const nvmoe_geometry& g) {
     const bool form = g.router_kind == NVMOE_ROUTER_TOPK_SOFTMAX || (g.router_kind == NVMOE_ROUTER_SCORE_TOPK && g.activation == NVMOE_ACT_SIGMOID);
     const uint32_t total_k = g.routed_k + (g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? g.always_count : 0u), per = g.n_group ? g.routed_experts / g.n_group : 1u;
-    if (!form || tokens <= 256u || g.routed_experts > 256u || total_k > 32u || g.hidden_size % 64u != 0u || per > 32u || (per & (per - 1u)) != 0u) return false;
+    return form && g.routed_experts <= 256u && total_k <= 32u && g.hidden_size % 64u == 0u && per <= 32u && (per & (per - 1u)) == 0u;
+}
+bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens) {
+    if (!router_filter_form(g) || tokens <= 256u) return false;
     const uint64_t blocks = (uint64_t)((tokens + 31u) / 32u) * ((g.routed_experts + 15u) / 16u);
     return (blocks + 147u) / 148u * g.hidden_size >= 1024u + 24u * (uint64_t)g.routed_experts;
 }
@@ -643,6 +646,19 @@ bool launch_router_filter(const RouterLaunch& router, const RouterFilter& f, cud
     return true;
 }
 
+// The bound, of |x| |w| (a fiftieth for the roundings of the norms and of the bound itself, two units for those of the interval's ends).
+static float router_filter_relative(uint32_t hidden, uint32_t splits) {
+    const double chain = hidden / 64.0 + 6.0, steps = kFlushBlocks * (kFilterColumns / 16u) * kStepUnits;
+    const double flushes = (double)(hidden + kFlushBlocks * kFilterColumns - 1u) / (kFlushBlocks * kFilterColumns) + 2.0 * splits;
+    return (float)(1.02 * (chain + steps + flushes + 2.0) / (1 << 24));
+}
+
+RouterProduct router_product_of(const RouterFilter& f, uint32_t tokens, uint32_t experts) {
+    const Scratch scratch = scratch_of(f, tokens, experts);
+    const uint32_t splits = filter_splits(tokens, f.hidden);
+    return RouterProduct{scratch.product, scratch.x_norm2, scratch.w_norm, splits, router_filter_width(experts), router_filter_relative(f.hidden, splits)};
+}
+
 void launch_router_refine(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream) {
     const uint32_t E = router.g.routed_experts;
     RefineKernel r{};
@@ -657,10 +673,7 @@ void launch_router_refine(const RouterLaunch& router, const RouterFilter& f, cud
     r.hidden = f.hidden;
     r.splits = filter_splits(router.tokens, f.hidden);
     r.n = router_filter_width(E);
-    // (a fiftieth for the roundings of the norms and of the bound itself, two units for those of the interval's ends)
-    const double chain = f.hidden / 64.0 + 6.0, steps = kFlushBlocks * (kFilterColumns / 16u) * kStepUnits;
-    const double flushes = (double)(f.hidden + kFlushBlocks * kFilterColumns - 1u) / (kFlushBlocks * kFilterColumns) + 2.0 * r.splits;
-    r.relative = (float)(1.02 * (chain + steps + flushes + 2.0) / (1 << 24));
+    r.relative = router_filter_relative(f.hidden, r.splits);
     const dim3 grid((router.tokens + kRefineWarps - 1u) / kRefineWarps), block(32u * kRefineWarps);
     const bool groups = router.g.n_group != 0u;
     const auto kernel = groups ? (E <= 32u ? router_refine_kernel<1, true> : E <= 128u ? router_refine_kernel<4, true> : router_refine_kernel<8, true>)
