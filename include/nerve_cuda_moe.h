@@ -444,6 +444,9 @@ int nvmoe_plan_debug_projection(const nvmoe_plan* plan, uint32_t* product);
  * stream. No reference counterpart. */
 int nvmoe_plan_debug_router_product(nvmoe_plan* plan, uint32_t batch_width, const nvmoe_buffer* hidden, const nvmoe_buffer* router_weights,
                                     float* product, float* row_norms, float* expert_norms, float* relative, uint32_t* splits);
+/* By how many units of the last place nvmoe_silu_multiply's fast activation differs, at most, from the pinned one over all gates that it
+ * settles, and how many its check allows for. No reference counterpart. */
+int nvmoe_debug_silu_units(nvmoe_device* device, uint32_t* units, uint32_t* allowed);
 /* Makes CTA 0 (enabled = 1) or CTA 1 (2) of the tensor-core expert kernels, or CTA 0 of the matrix product that a large layer
  * call's projection starts with (3), leave out its first pipeline-stage arrival, so that its consumer's bounded wait runs out: the way the give-up path (nvmoe_plan_set_wait_limit) is tested
  * without faulting or hanging anything. The call's output is incomplete and NVMOE_STATUS_WAIT_EXPIRED is

@@ -73,6 +73,12 @@ class CudaComputeDevice:
     def synchronize(self, timeout_ns: int = 60_000_000_000) -> None:
         self._check(self._lib.nvmoe_sync(self._h, timeout_ns))
 
+    def debug_silu_units(self) -> tuple[int, int]:
+        """Test aid: units of the last place by which the fast SiLU differs from the pinned one at most, and what its check allows."""
+        units, allowed = ctypes.c_uint32(), ctypes.c_uint32()
+        self._check(self._lib.nvmoe_debug_silu_units(self._h, ctypes.byref(units), ctypes.byref(allowed)))
+        return units.value, allowed.value
+
     def probe_mma_rate(self, n_tile: int = 128, k_groups: int = 8192) -> dict:
         """Measured rate of the block-scaled tensor-core instruction of the expert kernels over all SMs."""
         r = capi.MmaProbe()

@@ -113,6 +113,7 @@ PROTOTYPES = {
     "nvmoe_plan_last_report": (c_int, [c_void_p, POINTER(WorkReport)]),
     "nvmoe_plan_launch_count": (c_uint64, [c_void_p]),
     "nvmoe_plan_debug_token_tile": (c_int, [c_void_p, c_uint32, c_uint32, POINTER(c_uint32), POINTER(c_uint32)]),
+    "nvmoe_debug_silu_units": (c_int, [c_void_p, POINTER(c_uint32), POINTER(c_uint32)]),
     "nvmoe_plan_debug_projection": (c_int, [c_void_p, POINTER(c_uint32)]),
     "nvmoe_plan_debug_router_product": (c_int, [c_void_p, c_uint32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, POINTER(c_float),
                                                 POINTER(c_uint32)]),

@@ -1905,6 +1905,22 @@ int nvmoe_plan_debug_token_tile(const nvmoe_plan* p, uint32_t stage, uint32_t T,
     return NVMOE_OK;
 }
 
+int nvmoe_debug_silu_units(nvmoe_device* d, uint32_t* units, uint32_t* allowed) {
+    if (!d || !units || !allowed) return NVMOE_ERR_INVALID_ARGUMENT;
+    NVMOE_CUDA(d, cudaSetDevice(d->ordinal));
+    DeviceArray most;
+    cudaError_t err = most.ensure(4u);
+    if (err == cudaSuccess) err = cudaMemsetAsync(most.ptr, 0, 4u, d->stream);
+    if (err == cudaSuccess) launch_silu_units(most.as<uint32_t>(), d->stream);
+    if (err == cudaSuccess) err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaMemcpyAsync(units, most.ptr, 4u, cudaMemcpyDeviceToHost, d->stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(d->stream);
+    most.release();
+    if (err != cudaSuccess) return fail(d, NVMOE_ERR_CUDA, "SiLU units: %s", cudaGetErrorString(err));
+    *allowed = silu_units_bound();
+    return NVMOE_OK;
+}
+
 int nvmoe_plan_debug_projection(const nvmoe_plan* p, uint32_t* product) {
     if (!p || !product) return NVMOE_ERR_INVALID_ARGUMENT;
     *product = p->filtered ? 1u : 0u;

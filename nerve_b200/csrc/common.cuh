@@ -363,6 +363,10 @@ void launch_sum_f32_scale_packed_bf16(const float* partials, const uint32_t* sca
                                       uint32_t participant_count, uint32_t lane_count, uint32_t elements_per_scale,
                                       uint32_t scale_bit_offset, cudaStream_t stream);
 
+// ffn_tail.cu: most (zeroed) receives by how many units the fast SiLU differs from the pinned one, of which it allows silu_units_bound
+void launch_silu_units(uint32_t* most, cudaStream_t stream);
+uint32_t silu_units_bound();
+
 // probe.cu: a run of `groups` x 8 block-scaled MMAs (128 x n_tile x 32, two alternating accumulators)
 // on every one of `ctas` CTAs; cycles[cta] = clock cycles from first issue to completion
 cudaError_t launch_mma_rate_probe(uint32_t n_tile, uint32_t groups, uint32_t ctas, long long* cycles, uint32_t* status,

@@ -129,7 +129,7 @@ __device__ __forceinline__ float silu_times(float g, float u, float limit) {
 // The same product as bf16, by the hardware's exponential and reciprocal wherever these settle the rounding: the pinned functions take a hundred
 // instructions a value and bound the node (of 24.8 us for 4096 x 2048 values memory takes 8). The argument's product with log2 e is made exact in two
 // parts, so that g / (1 + exp(-g)) by ex2.approx and rcp.approx differs from the pinned form by at most kSiluUnits units of the last place, over
-// all bf16 values g whose result is a normal number (tests/test_gpu_silu.py goes through all of them). A result whose rounding to bf16 such a difference, doubled by the
+// all gates there can be (a bf16 number or the bound) whose result is a normal number: silu_units_kernel goes through them all. A result whose rounding to bf16 such a difference, doubled by the
 // product with u, could change is made by the pinned form: one of 1700 (bounded) or 3600, besides very small and very large ones. us, pinned / this way: 777 x 2048
 // values 7.1 / 5.1, 2048 x 2048 11.4 / 9.2, 4096 x 2048 24.8 / 18.9.
 constexpr uint32_t kSiluUnits = 8u;  // (4 measured)
@@ -207,6 +207,27 @@ __global__ void __launch_bounds__(256) pairwise_kernel(const uint32_t* __restric
         i = quads * 4u + ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
     }
     for (; i < words; i += stride) out[i] = SILU ? silu_word(a[i], b[i], limit) : add_word(a[i], b[i]);
+}
+
+// By how many units of the last place silu_approx differs from the pinned form, at most, over all gates whose result is settled as a normal number: all positive f32
+// numbers (a bound that is no bf16 number can be the gate) and all negative bf16 numbers; and 2^24 if one below the exponential's range is not the zero that it is taken for.
+__global__ void __launch_bounds__(256) silu_units_kernel(uint32_t* most) {
+    uint32_t units = 0u;
+    auto look = [&](float g) {
+        if (!(fabsf(g) < 3.4e38f)) return;
+        const float a = silu_approx(g), pinned = __fdiv_rn(g, __fadd_rn(1.0f, nvmoe_expf(-g)));
+        const uint32_t bits = __float_as_uint(a), want = __float_as_uint(pinned);
+        if (g < -88.72284f) {
+            if (want != 0x80000000u) units = 1u << 24;
+        } else if ((bits & 0x7fffffffu) - 0x08000000u < 0x70000000u) {
+            units = max(units, bits > want ? bits - want : want - bits);
+        }
+    };
+    const uint32_t threads = gridDim.x * 256u, first = blockIdx.x * 256u + threadIdx.x;
+    for (uint32_t b = first; b < 0x7f800000u; b += threads) look(__uint_as_float(b));
+    for (uint32_t h = first; h < 0x8000u; h += threads) look(__uint_as_float(0x80000000u | h << 16));
+    units = __reduce_max_sync(0xffffffffu, units);
+    if ((threadIdx.x & 31u) == 0u) atomicMax(most, units);
 }
 
 // One warp per token: the first k lanes look the token's routed resources up, lane 0 sorts and counts.
@@ -364,5 +385,8 @@ void launch_route_preselected(const uint32_t* logits, const uint32_t* selections
                               const nvmoe_geometry& g, cudaStream_t stream) {
     launch_chained(route_preselected_kernel, dim3((tokens + 3u) / 4u), dim3(128), 0, stream, logits, selections, tokens, routes, status, g);
 }
+
+uint32_t silu_units_bound() { return kSiluUnits; }
+void launch_silu_units(uint32_t* most, cudaStream_t stream) { silu_units_kernel<<<148 * 8, 256, 0, stream>>>(most); }
 
 }  // namespace nvmoe

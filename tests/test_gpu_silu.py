@@ -49,3 +49,12 @@ def test_zeros(limit):
     np.testing.assert_array_equal(out.read(np.uint16).reshape(gates.shape), mo.silu_multiply(gates, ups, limit))
     plan.destroy()
     device.close()
+
+
+def test_fast_activation_errs_by_less_than_its_check_allows():
+    """Over every gate that there can be: positive f32 numbers (the bound can be any) and negative bf16 numbers."""
+    device = CudaComputeDevice(0)
+    units, allowed = device.debug_silu_units()
+    print(f"{units} units of {allowed}")
+    assert 0 < units <= allowed
+    device.close()
