@@ -156,6 +156,8 @@ bool router_is_small(const RouterLaunch& p);  // at most 128 experts, 32 selecti
 void launch_router_linear(const uint16_t* x, const uint16_t* w, const uint16_t* bias, uint32_t* logits,
                           uint32_t tokens, uint32_t hidden, uint32_t outputs, bool beside, const CallStart& start, cudaStream_t stream);  // (beside: see there)
 
+uint32_t device_sm_count();  // of the current device
+
 // router_filter.cu: projection and routing of a large call, of which only the logits that matter are made exactly.
 struct RouterFilter {
     const uint16_t* x;

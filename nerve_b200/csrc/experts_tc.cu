@@ -1096,6 +1096,8 @@ void configure_tile() {
 
 }  // namespace
 
+uint32_t device_sm_count() { return (uint32_t)sm_count(); }
+
 bool tc_shape_supported(const nvmoe_geometry& g) {
     return g.hidden_size % 32u == 0u && g.intermediate_size % 32u == 0u && g.act_block % 32u == 0u;
 }
@@ -1204,8 +1206,9 @@ bool launch_dense_prepare(const DensePrepare& p, uint32_t act_block, cudaStream_
     // A warp takes further pieces of rows, two at a time, rather than that a second wave of blocks is needed (an SM holds 10): while that asks for two rounds
     // at most. Beyond, 16 blocks an SM, which even out the rounds. Block of 2048 rows of 7168 columns, us, 16 / 10 an SM: 501 tokens 75.6 / 73.8, 777 84.4 /
     // 82.9, 1200 (1.7 rounds) 99.8 / 99.4, 2048 (2.9) 139.4 / 140.9.
-    const uint32_t wave = 148u * 10u > retile + 1u + 148u ? 148u * 10u - retile - 1u : 148u;
-    const uint32_t room = warps <= 16ull * wave ? wave : 148u * 16u > retile + 1u + 148u ? 148u * 16u - retile - 1u : 148u;
+    const uint32_t sms = (uint32_t)sm_count();
+    const uint32_t wave = sms * 10u > retile + 1u + sms ? sms * 10u - retile - 1u : sms;
+    const uint32_t room = warps <= 16ull * wave ? wave : sms * 16u > retile + 1u + sms ? sms * 16u - retile - 1u : sms;
     if (quantises && others > room) others = room;
     const auto kernel = !quantises ? dense_prepare_kernel<0u> : act_block == 32u ? dense_prepare_kernel<2u> : dense_prepare_kernel<8u>;
     launch_chained(kernel, dim3(retile + others + 1u), dim3(kDenseThreads), 0, stream, p, k_blocks, retile);
@@ -1228,6 +1231,19 @@ static EncodeFn tensor_map_encoder() {
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     return encode;
+}
+
+bool tc_encode_bf16_map(void* map128, const void* base, uint32_t rows, uint32_t cols, uint32_t box_cols, uint32_t box_rows) {
+    const EncodeFn encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {(cuuint64_t)cols * 2u};
+    const cuuint32_t box[2] = {box_cols, box_rows}, step[2] = {1u, 1u};
+    CUtensorMap map;
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    std::memcpy(map128, &map, 128);
+    return true;
 }
 
 bool tc_replace_map_address(void* map128, const void* device_address) {

@@ -26,6 +26,8 @@ bool tc_encode_activation_map(void* map128, void* base, uint32_t rows, uint32_t 
 // expert-grouped token rows, and for CTA pairs the derived scales of a set (blocks of 512 bytes, `sources` to a (row tile,
 // K block)) and the token scales [rows = K blocks][words].
 bool tc_encode_pair_weight_map(void* map128, void* any_device_address, uint32_t rows, uint32_t cols, bool bytes);
+// Rows of bf16 numbers, in 128-byte swizzled boxes.
+bool tc_encode_bf16_map(void* map128, const void* base, uint32_t rows, uint32_t cols, uint32_t box_cols, uint32_t box_rows);
 // A map encoded above, for another address. False where the driver cannot.
 bool tc_replace_map_address(void* map128, const void* device_address);
 bool tc_encode_pair_token_map(void* map128, void* base, uint32_t rows, uint32_t cols, uint32_t box_rows);

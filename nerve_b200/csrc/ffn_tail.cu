@@ -387,6 +387,6 @@ void launch_route_preselected(const uint32_t* logits, const uint32_t* selections
 }
 
 uint32_t silu_units_bound() { return kSiluUnits; }
-void launch_silu_units(uint32_t* most, cudaStream_t stream) { silu_units_kernel<<<148 * 8, 256, 0, stream>>>(most); }
+void launch_silu_units(uint32_t* most, cudaStream_t stream) { silu_units_kernel<<<device_sm_count() * 8u, 256, 0, stream>>>(most); }
 
 }  // namespace nvmoe

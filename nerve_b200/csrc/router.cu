@@ -245,14 +245,6 @@ __global__ void __launch_bounds__(128) router_reg_kernel(RouterLaunch p) {
     if (token < p.tokens) route_token<false, EPL, GROUPS>(p, token);
 }
 
-// One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the
-// instruction itself.
-__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
-    float d;
-    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
-    return d;
-}
-
 // ---- router projection ----------------------------------------------------------------------
 // The shader gives every output row 64 lanes that stride over the packed input words with two
 // f32 fma per word and then sums the lanes.  Here a block of 64 threads owns a TT x ET tile of

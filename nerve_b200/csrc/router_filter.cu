@@ -22,7 +22,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
-
+#include "experts_tc.cuh"
 #include "router_reg.cuh"
 #include "tcgen05.cuh"
 
@@ -59,13 +59,6 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, ui
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-
-// One step of a lane's sum, as in router.cu.
-__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
-    float d;
-    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
-    return d;
 }
 
 __device__ __forceinline__ float square_sum(const uint4& v, float sum) {
@@ -552,26 +545,6 @@ __global__ void __launch_bounds__(32 * kRefineWarps, EPL > 4 ? 3 : 4) router_ref
     finish_token<true>(p.router, token, found, my_e, my_v, rank);
 }
 
-typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeFn encoder() {
-    static const EncodeFn fn = [] {
-        void* found = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &found, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
-        return reinterpret_cast<EncodeFn>(ok ? found : nullptr);
-    }();
-    return fn;
-}
-bool encode_rows(CUtensorMap* map, const uint16_t* base, uint32_t rows, uint32_t cols, uint32_t box_rows) {
-    const EncodeFn encode = encoder();
-    if (!encode) return false;
-    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {(cuuint64_t)cols * 2u};
-    const cuuint32_t box[2] = {kFilterColumns, box_rows}, step[2] = {1u, 1u};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 constexpr double kStepUnits = 16.0;     // (10.5 by the above)
 constexpr uint32_t kFilterSplits = 8u;  // at most
 
@@ -590,12 +563,13 @@ bool router_filter_form(const nvmoe_geometry& g) {
 bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens) {
     if (!router_filter_form(g) || tokens <= 256u) return false;
     const uint64_t blocks = (uint64_t)((tokens + 31u) / 32u) * ((g.routed_experts + 15u) / 16u);
-    return (blocks + 147u) / 148u * g.hidden_size >= 1024u + 24u * (uint64_t)g.routed_experts;
+    const uint32_t sms = device_sm_count();
+    return (blocks + sms - 1u) / sms * g.hidden_size >= 1024u + 24u * (uint64_t)g.routed_experts;
 }
 
 static uint32_t filter_tiles(uint32_t tokens) { return (tokens + kFilterTokens - 1u) / kFilterTokens; }
 static uint32_t filter_splits(uint32_t tokens, uint32_t hidden) {
-    const uint32_t idle = 148u / filter_tiles(tokens), blocks = (hidden + kFilterColumns - 1u) / kFilterColumns;
+    const uint32_t idle = device_sm_count() / filter_tiles(tokens), blocks = (hidden + kFilterColumns - 1u) / kFilterColumns;
     const uint32_t most = blocks / 4u < kFilterSplits ? blocks / 4u : kFilterSplits;
     return idle < most ? (idle > 1u ? idle : 1u) : (most > 1u ? most : 1u);
 }
@@ -604,7 +578,7 @@ static uint32_t router_filter_width(uint32_t outputs) { return (outputs + 15u) /
 
 // Splits x tokens of any call of up to so many tokens.
 static size_t filter_rows(uint32_t max_tokens) {
-    const size_t split = (size_t)kFilterSplits * max_tokens, filled = 148u * (size_t)kFilterTokens;
+    const size_t split = (size_t)kFilterSplits * max_tokens, filled = device_sm_count() * (size_t)kFilterTokens;
     return max_tokens > (split < filled ? split : filled) ? max_tokens : (split < filled ? split : filled);
 }
 size_t router_filter_floats(uint32_t max_tokens, uint32_t experts) { return filter_rows(max_tokens) * (router_filter_width(experts) + 1u) + experts; }
@@ -622,7 +596,7 @@ static Scratch scratch_of(const RouterFilter& f, uint32_t tokens, uint32_t exper
 bool launch_router_filter(const RouterLaunch& router, const RouterFilter& f, cudaStream_t stream) {
     const uint32_t E = router.g.routed_experts, n = router_filter_width(E);
     CUtensorMap x_map, w_map;
-    if (!encode_rows(&x_map, f.x, router.tokens, f.hidden, kFilterTokens) || !encode_rows(&w_map, f.w, E, f.hidden, n)) return false;
+    if (!tc_encode_bf16_map(&x_map, f.x, router.tokens, f.hidden, kFilterColumns, kFilterTokens) || !tc_encode_bf16_map(&w_map, f.w, E, f.hidden, kFilterColumns, n)) return false;
     FilterKernel k{};
     k.w = f.w;
     const Scratch scratch = scratch_of(f, router.tokens, E);

@@ -46,6 +46,14 @@ __device__ __forceinline__ uint32_t warp_best(float s, uint32_t e) {
     return __reduce_min_sync(0xffffffffu, top != 0u && key == top ? e : kUnboundSlot);
 }
 
+// One step of a lane's sum: bf16 x bf16 (exact in f32) added with one rounding, the products' operands converted by the
+// instruction itself.
+__device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c) {
+    float d;
+    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
+    return d;
+}
+
 __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uint32_t e) {
     if (dtype == NVMOE_BIAS_F32) return reinterpret_cast<const float*>(bias)[e];
     if (dtype == NVMOE_BIAS_BF16) return nvmoe_bf16_to_f32(reinterpret_cast<const uint16_t*>(bias)[e]);

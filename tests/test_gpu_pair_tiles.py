@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, ResidentBuffer
 from oracle import moe_oracle as mo
 from oracle import sampled
 from tests.helpers import assert_close
@@ -142,5 +142,43 @@ def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, name, shape, t
     plan.layer(tokens, bank, hidden, out, router_weights=rw, bias=bias)
     assert plan.status() == 0
     np.testing.assert_array_equal(out.read(np.uint16), before)
+    plan.destroy()
+    bank.destroy()
+
+
+@pytest.mark.parametrize("rows,cols,tokens", [(288, 448, 130), (160, 2112, 40)])
+def test_outputs_off_the_word_grid(device, rows, cols, tokens):
+    """Outputs that start at an odd multiple of two bytes, which a lane stores one row of a token at a time instead of two: the same bits, nothing beside them."""
+    rng = np.random.default_rng(rows)
+    plan = MoePlan.for_config(device, synthetic.MoeConfig("odd", 256, 256, 8, 2, act_block=32), tokens)
+    plan.set_expert_path(2)
+    x = device.resident_buffer_from(synthetic.f32_to_bf16(rng.standard_normal((tokens, cols)).astype(np.float32)))
+    w, s = (device.resident_buffer_from(rng.integers(lo, hi, (rows, n), dtype=np.uint8)) for lo, hi, n in ((0, 256, cols // 2), (118, 128, cols // 32)))
+    even, odd = (device.resident_buffer_from(np.full(tokens * rows + 8, 0x7fc0, dtype=np.uint16)) for _ in range(2))
+    inner = ResidentBuffer.wrap(device, odd.device_address() + 2, tokens * rows * 2)
+    plan.dense_linear(tokens, x, even, w, s, rows, cols)
+    plan.dense_linear(tokens, x, inner, w, s, rows, cols)
+    assert plan.status() == 0
+    got, want = odd.read(np.uint16), even.read(np.uint16)
+    np.testing.assert_array_equal(got[1:tokens * rows + 1], want[:tokens * rows])
+    assert got[0] == 0x7fc0 and (got[tokens * rows + 1:] == 0x7fc0).all()
+    plan.destroy()
+
+
+def test_expert_rows_off_the_word_grid(device):
+    """The same for a layer call whose expert rows the caller gets."""
+    cfg, tokens = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 576, 320, 8), 400
+    case = synthetic.make_case(cfg, tokens, seed=17)
+    plan = MoePlan.for_config(device, cfg, tokens)
+    bank = ExpertBank.upload(device, case.w1, case.s1, case.w3, case.s3, case.w2, case.s2)
+    hidden, weights, bias = (device.resident_buffer_from(a) for a in (case.hidden, case.router_w, case.router_bias))
+    count = tokens * cfg.total_k * cfg.hidden
+    even, odd = (device.resident_buffer_from(np.full(count + 8, 0x7fc0, dtype=np.uint16)) for _ in range(2))
+    for rows in (even, ResidentBuffer.wrap(device, odd.device_address() + 2, count * 2)):
+        plan.layer(tokens, bank, hidden, None, router_weights=weights, router_bias=bias, expert_outputs=rows)
+    assert plan.status() == 0
+    got, want = odd.read(np.uint16), even.read(np.uint16)
+    np.testing.assert_array_equal(got[1:count + 1], want[:count])
+    assert got[0] == 0x7fc0 and (got[count + 1:] == 0x7fc0).all()
     plan.destroy()
     bank.destroy()
