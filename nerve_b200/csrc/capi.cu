@@ -1606,7 +1606,9 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
     rows.down.cols = g.intermediate_size;
     rows.early = projects || (!a->routes_in && !routes_in_schedule);
     const bool beside = fused_quantise && fused_schedule && !prof && places_operands(ls, routes_in_schedule, rows, g.act_block);
-    // The counters of the one launch for both expert stages are cleared two launches before it, or else it counts after its wait.
+    // The one launch for both expert stages counts before its wait. With operands beside the schedule its counters are cleared ahead of these two launches,
+    // both of which may still run then: by the projection, or, in calls without one, by the schedule, and it counts after its wait. Otherwise the
+    // schedule clears them, and the quantisation, which waits for it, stands between.
     CallStart start{clock, nullptr, 0u};
     if (one_launch && beside && projects) {
         start.clear = p->layer_sync.as<uint32_t>();
@@ -1683,7 +1685,7 @@ static int layer_call(nvmoe_plan* p, const nvmoe_layer_args* a, const HostRows* 
                                  (const uint32_t*)down_control.ptr, tensor));
     }
     mark(kStageQuantX);
-    // (this launch also keeps the one for both expert stages, which counts before it waits, apart from the schedule, which clears the counters)
+    // (where the schedule clears the counters of the one launch for both expert stages, this launch keeps the two apart)
     if (!beside) NVMOE_TRY(quantise_operands(p, true, T, a->hidden->ptr, tensor, true, fused_quantise));
     mark(kStageGateUp);
     ExpertCall call;

@@ -21,9 +21,11 @@ constexpr uint32_t kMaxExperts = 4096u;  // ids travel in the low 16 bits of a r
 // before any return, so completion still implies that all earlier kernels have completed, and before
 // touching global memory that the launch ahead of it may write or read. What stands before the call may
 // rely on the launches before that one: the kernel ahead let this one start after its own wait, when they
-// had completed. (Tensor maps and expert tables are read there, place_operands_kernel reads the tokens, the schedule behind that one does
-// all of its work, and experts_layer.cu claims its first work from a counter that a launch before the one ahead cleared: no other kernel
-// may let the next start before its wait, and a launch has to stay between those two.) Launched the ordinary way, the same kernels run unchanged.
+// had completed. (Tensor maps and expert tables are read there, place_operands_kernel reads the tokens, experts_layer.cu claims its first work
+// from a counter that an earlier launch of the call cleared.) One kernel lets the next start before its wait and does all of its work ahead of
+// it: small_schedule_kernel, right behind place_operands_kernel. Whatever it reads, and whatever the kernel behind it reads or counts before its own
+// wait, has to stand from launches before place_operands_kernel, which may still be running then, as the schedule may. No other kernel may let the next
+// start before its wait. Launched the ordinary way, the same kernels run unchanged.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_dependency_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

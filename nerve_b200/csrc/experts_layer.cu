@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
     // What is read, and counted, before the wait: what stands since earlier calls, or since a launch of this one that had completed
-    // when the kernel ahead let this one start. That one waited for all before it, the one that cleared the counters among them (the
-    // projection, or the schedule where the quantisation is a launch of its own); where it clears them itself, the claim follows the wait.
+    // when the kernel ahead let this one start: with the quantisation ahead all launches before that, the schedule, which cleared the counters, among
+    // them; with the schedule of a small call ahead, which lets this one start before its own wait, those before place_operands_kernel, the
+    // projection, which cleared them, among them. Where that schedule clears them itself, the claim follows the wait.
     uint32_t claimed = 0u;
     if (warp == 7u && lane == 0u && !p.claim_late) claimed = atomicAdd(p.sync, 1u);
     for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) {

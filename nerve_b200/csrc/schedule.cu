@@ -1419,11 +1419,12 @@ bool layer_schedule_is_fused(uint32_t tokens, uint32_t K, uint32_t num_experts, 
            three_sort_schedule_fits(count, num_experts);
 }
 
-// A warp of the one block per token, all routes in one pass. The launch saved is about a microsecond; the router's own
-// chain grows with the experts a lane holds and the warps of the one SM get in each other's way, so it stops at sixteen
-// tokens where a lane holds several. Layer of 384 x 256 in one launch / two, us: 8 tokens of 32 experts 33.0 / 34.0, 16
-// 34.2 / 35.4, 24 36.4 / 36.1, 32 37.2 / 37.1 (32 from host buffers, 1024 x 512: 71.8 / 72.6); 16 of 128 41.9 / 41.8, 24
-// of 64 39.6 / 38.7, 32 of 128 46.0 / 44.8.
+// Calls whose tokens are routed, a warp each, in the blocks that make the operands and the schedule (place_operands_kernel, small_schedule_kernel), or else in
+// the schedule's one block (route_schedule_kernel), without a launch of their own. That launch is about a microsecond; the router's own chain grows with the
+// experts a lane holds, and the warps of an SM get in each other's way. Layers, us, in these blocks / by a launch of its own, operands beside the schedule: 384 x 256,
+// 8 tokens of 32 experts 20.6 / 20.8, 16 20.9 / 20.9, 24 22.2 / 22.3, 32 23.6 / 22.8; 2880 x 2880 8 69.3 / 71.3, 16 80.5 / 81.4, 32 86.6 / 86.4; 12 of 64 22.1 /
+// 23.1, 16 22.7 / 22.8, 24 24.4 / 23.7, 32 25.6 / 23.7; 2048 x 256, 8 routes, 16 33.7 / 34.4, 24 37.2 / 34.9; 16 of 128 25.3 / 26.9, 32 27.7 / 28.6. In the schedule's
+// block alone: 8 tokens of 32 33.0 / 34.0, 16 34.2 / 35.4, 24 36.4 / 36.1, 32 37.2 / 37.1; 16 of 128 41.9 / 41.8, 24 of 64 39.6 / 38.7, 32 of 128 46.0 / 44.8.
 bool layer_routes_in_schedule(const RouterLaunch& router, uint32_t K, uint32_t num_experts) {
     const uint64_t count = (uint64_t)router.tokens * K;
     return router.tokens <= (router.g.routed_experts <= 32u ? 32u : 16u) && router_is_small(router) && count <= 1024u && rank_schedule_fits(count, num_experts);
