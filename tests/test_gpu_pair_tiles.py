@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from nerve_b200 import synthetic
-from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan, ResidentBuffer
+from nerve_b200.backend import CudaComputeDevice, ExpertBank, MoePlan
 from oracle import moe_oracle as mo
 from oracle import sampled
 from tests.helpers import assert_close
@@ -149,6 +149,8 @@ def test_waits_that_run_out_anywhere_leave_the_plan_whole(device, name, shape, t
 @pytest.mark.parametrize("rows,cols,tokens", [(288, 448, 130), (160, 2112, 40)])
 def test_outputs_off_the_word_grid(device, rows, cols, tokens):
     """Outputs that start at an odd multiple of two bytes, which a lane stores one row of a token at a time instead of two: the same bits, nothing beside them."""
+    from nerve_b200.backend import ResidentBuffer
+
     rng = np.random.default_rng(rows)
     plan = MoePlan.for_config(device, synthetic.MoeConfig("odd", 256, 256, 8, 2, act_block=32), tokens)
     plan.set_expert_path(2)
@@ -167,6 +169,8 @@ def test_outputs_off_the_word_grid(device, rows, cols, tokens):
 
 def test_expert_rows_off_the_word_grid(device):
     """The same for a layer call whose expert rows the caller gets."""
+    from nerve_b200.backend import ResidentBuffer
+
     cfg, tokens = synthetic.small_variant(synthetic.CONFIGS["gpt-oss-20b"], 576, 320, 8), 400
     case = synthetic.make_case(cfg, tokens, seed=17)
     plan = MoePlan.for_config(device, cfg, tokens)

@@ -36,8 +36,8 @@ class Layer:
         self.logit_bias = bf16(rng.standard_normal(cfg.experts, dtype=np.float32) * np.float32(0.1)) if cfg.logit_bias else None
         self.select_bias = (rng.standard_normal(cfg.experts, dtype=np.float32) * np.float32(0.05)) if cfg.bias_dtype == synthetic.BIAS_F32 else None
 
-    def both_ways(self, filtered=True):
-        """Routes, telemetry, output and status with the filter (`filtered`: whether the rule takes the call), and with logits that the caller gets."""
+    def both_ways(self):
+        """Routes, telemetry, output and status with the filter, and with logits that the caller gets."""
         buffer = lambda a: None if a is None else self.device.resident_buffer_from(a)
         cfg, T = self.cfg, self.tokens
         hidden = buffer(self.x)
@@ -48,7 +48,6 @@ class Layer:
             routes, telemetry = buffer(np.full((T, cfg.total_k), 0xdeadbeef, dtype=np.uint32)), buffer(np.zeros(self.plan.telemetry_words(), dtype=np.uint32))
             out = buffer(np.full((T, cfg.hidden), 0x7fc0, dtype=np.uint16))
             self.plan.layer(T, self.bank, hidden, out, routes_out=routes, telemetry=telemetry, **args, **extra)
-            assert self.plan.debug_projection() == (filtered and not extra)
             results.append((routes.read(np.uint32).copy(), telemetry.read(np.uint32).copy(), out.read(np.uint16).copy(), self.plan.status()))
         for got, want in zip(*results):
             np.testing.assert_array_equal(got, want)
@@ -59,10 +58,7 @@ class Layer:
         self.bank.destroy()
 
 
-# sizes that the rule leaves to the projection by itself: few columns in one round of its blocks, 256 tokens
-BELOW = [((1152, 64, 16), 300), ((2880, 64, 32), 256)]
-
-
+# (which of them the rule of router_filter_takes filters: test_which_projection_a_call_uses)
 @pytest.mark.parametrize("name,shape,tokens,changes", [
     ("gpt-oss-20b", (1152, 64, 16), 300, {}), ("gpt-oss-20b", (2880, 64, 128), 592, {}), ("gpt-oss-20b", (2880, 64, 32), 256, {}),
     ("gpt-oss-20b", (1408, 128, 16), 257, {}), ("gpt-oss-20b", (1472, 128, 17), 385, {}), ("gpt-oss-20b", (1152, 64, 5), 511, {}),
@@ -74,7 +70,7 @@ BELOW = [((1152, 64, 16), 300), ((2880, 64, 32), 256)]
     ("gpt-oss-20b", (1024, 64, 32), 19000, {})])
 def test_what_is_selected(device, name, shape, tokens, changes):
     layer = Layer(device, name, shape, tokens, **changes)
-    assert layer.both_ways((shape, tokens) not in BELOW)[3] == 0
+    assert layer.both_ways()[3] == 0
     layer.close()
 
 
@@ -97,11 +93,6 @@ def inputs(kind, layer):
     elif kind == "close experts":  # a few units of the last place between them
         w[:] = w[0]
         w *= 1 + rng.integers(-2, 3, w.shape) / 256
-    elif kind == "positive, the largest first":  # what the matrix product errs most by, experts a step or two apart
-        x, w[:] = np.abs(x) + 0.5, np.abs(w[0]) + 0.01
-        x[:, ::128] *= 8
-        x[:, 0] *= 64
-        w *= 1 + rng.integers(-1, 2, w.shape) / 256
     elif kind == "heavy":
         x, w = x ** 5, w ** 3
     elif kind == "tiny":
@@ -129,7 +120,7 @@ def inputs(kind, layer):
 
 
 @pytest.mark.parametrize("name,shape,changes", [("gpt-oss-20b", (1856, 64, 32), {}), ("gpt-oss-20b", (1728, 64, 100), {"k": 6}), ("deepseek-v3", (2560, 128, 64), {})])
-@pytest.mark.parametrize("kind", ["ties", "all the same", "cancellation", "close experts", "positive, the largest first", "heavy", "tiny", "subnormal", "huge", "overflow", "token specials",
+@pytest.mark.parametrize("kind", ["ties", "all the same", "cancellation", "close experts", "heavy", "tiny", "subnormal", "huge", "overflow", "token specials",
                                   "expert specials", "bias specials"])
 def test_inputs_that_the_product_says_little_of(device, name, shape, changes, kind):
     layer = Layer(device, name, shape, 1050, **changes)
@@ -138,8 +129,66 @@ def test_inputs_that_the_product_says_little_of(device, name, shape, changes, ki
     layer.close()
 
 
-# (a clock, some, about as many as the product takes, so that the roles give up at different places; every one that does holds its CTA two milliseconds)
-@pytest.mark.parametrize("limit", [1, 300, 1500, 5000])
+def test_a_wait_that_runs_out(device):
+    """The status says so, routes stay in range, and the next call is whole."""
+    layer = Layer(device, "gpt-oss-20b", (2880, 64, 32), 1024)
+    want = layer.both_ways()
+    layer.plan.set_wait_limit(1)
+    buffer = layer.device.resident_buffer_from
+    args = dict(router_weights=buffer(layer.w), router_bias=buffer(layer.logit_bias))
+    routes, out = buffer(np.zeros((1024, 4), dtype=np.uint32)), buffer(np.zeros((1024, 2880), dtype=np.uint16))
+    for _ in range(4):
+        layer.plan.layer(1024, layer.bank, buffer(layer.x), out, routes_out=routes, **args)
+        device.synchronize(timeout_ns=20_000_000_000)
+        assert layer.plan.status() & ~8 == 0
+        assert (routes.read(np.uint32) & 0xffff).max() < 32
+    layer.plan.set_wait_limit(0)
+    got = layer.both_ways()
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    layer.close()
+
+
+# sizes that the rule leaves to the projection by itself: few columns in one round of its blocks, 256 tokens
+BELOW = [((1152, 64, 16), 300), ((2880, 64, 32), 256)]
+SELECTED = [tuple(case) for case in test_what_is_selected.pytestmark[0].args[1]]
+UNTOLD = [(name, shape, 1050, changes) for name, shape, changes in
+          next(mark.args[1] for mark in test_inputs_that_the_product_says_little_of.pytestmark if mark.args[0] == "name,shape,changes")]
+
+
+@pytest.mark.parametrize("name,shape,tokens,changes", SELECTED + UNTOLD)
+def test_which_projection_a_call_uses(device, name, shape, tokens, changes):
+    """The calls that the tests above compare: with the filter unless the caller gets the logits, or they lie below its line."""
+    layer = Layer(device, name, shape, tokens, **changes)
+    buffer = lambda a: None if a is None else device.resident_buffer_from(a)
+    hidden, out = buffer(layer.x), device.create_resident_buffer(tokens * layer.cfg.hidden * 2)
+    logits = device.create_resident_buffer(tokens * ((layer.cfg.experts + 1) // 2) * 4)
+    args = dict(router_weights=buffer(layer.w), router_bias=buffer(layer.logit_bias), bias=buffer(layer.select_bias))
+    for extra in ({}, {"logits": logits}):
+        layer.plan.layer(tokens, layer.bank, hidden, out, **args, **extra)
+        assert layer.plan.debug_projection() == ((shape, tokens) not in BELOW and not extra)
+    assert layer.plan.status() == 0
+    layer.close()
+
+
+@pytest.mark.parametrize("name,shape,tokens,changes", UNTOLD)
+def test_rows_that_the_product_errs_most_by(device, name, shape, tokens, changes):
+    """Positive ones, the largest first, by experts a step or two apart."""
+    layer = Layer(device, name, shape, tokens, **changes)
+    rng = np.random.default_rng(11)
+    x, w = (np.abs(synthetic.bf16_to_f32(a)) for a in (layer.x, layer.w))
+    x += 0.5
+    x[:, ::128] *= 8
+    x[:, 0] *= 64
+    w[:] = w[0] + 0.01
+    w *= 1 + rng.integers(-1, 2, w.shape) / 256
+    layer.x, layer.w = synthetic.f32_to_bf16(x.astype(np.float32)), synthetic.f32_to_bf16(w.astype(np.float32))
+    layer.both_ways()
+    layer.close()
+
+
+# (some clocks, about as many as the product takes, so that the roles give up at different places; every one that does holds its CTA two milliseconds)
+@pytest.mark.parametrize("limit", [300, 1500, 5000])
 def test_waits_that_may_run_out(device, limit):
     """Whichever of the waits run out: no status but theirs, routes in range, and the next call is whole."""
     layer = Layer(device, "gpt-oss-20b", (2880, 64, 32), 1024)
@@ -154,8 +203,7 @@ def test_waits_that_may_run_out(device, limit):
         assert layer.plan.status() & ~8 == 0
         assert (routes.read(np.uint32) & 0xffff).max() < 32
     layer.plan.set_wait_limit(0)
-    got = layer.both_ways()
-    for a, b in zip(got, want):
+    for a, b in zip(layer.both_ways(), want):
         np.testing.assert_array_equal(a, b)
     layer.close()
 
