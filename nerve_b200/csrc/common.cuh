@@ -340,7 +340,7 @@ struct ExpertLaunch {  // experts_simt.cu and experts_tc.cu
     uint32_t* tile_count;        // tensor path scratch: one word
     uint32_t tokens;             // upper bound (max over what control may hold)
     long long wait_cycles;       // tensor path: clock cycles after which a bounded in-kernel wait gives up
-    uint32_t debug_flags;        // tensor path: bit n = CTA n (0 or 1) leaves out its first stage arrival (exercises the give-up path); bit 2: RouterFilter.withhold
+    uint32_t debug_flags;        // tensor path: bit n = CTA n (0 or 1) leaves out its first stage arrival (exercises the give-up path); bit 2: RouterFilter.withhold; from bit 8 on always zero
     nvmoe_geometry g;
 };
 void configure_simt_kernels();

@@ -508,13 +508,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) exp
                     const uint4 low = inbox[0], high = inbox[32];
                     other[0] = low.x, other[1] = low.y, other[2] = low.z, other[3] = low.w;
                     other[4] = high.x, other[5] = high.y, other[6] = high.z, other[7] = high.w;
-                    __syncwarp();
+                    // The place may be overwritten once the other warp hears that it was read, and an arrival there does not wait for loads that have only been
+                    // issued (chunks whose successor was under way at once came out with eight tokens of it: layers of short K, where the other CTA waits
+                    // for the place, differed from pass to pass). So its address depends on what was loaded: `none` is zero, which the compiler can't know.
+                    const uint32_t none = __reduce_or_sync(0xffffffffu, low.x | low.y | low.z | low.w | high.x | high.y | high.z | high.w) & (p.debug_flags >> 8);
                     // (the announcement of a chunk only follows the arrival of the last: one more, on a barrier whose bytes are
                     // outstanding, would be one more than it counts)
                     if (here) {
                         if (lane == 0u) {
                             mbar_arrive_expect_tx(&bars->sent[warp], 1024u);
-                            mbar_arrive_cluster(peer_taken);
+                            mbar_arrive_cluster(peer_taken + none);
                         }
                         receipts++;
                     }

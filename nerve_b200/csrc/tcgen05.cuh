@@ -132,9 +132,9 @@ __device__ __forceinline__ void cluster_sync() {
 // Arrival on a barrier of either CTA (`addr` from map_shared). It releases at CTA scope, the default: release.cluster also waits
 // for the thread's global stores, which nothing here hands over, and cost more than 1000 cycles an arrival. What the arrivals of
 // a pair do hand over is complete before them without it: scale words written in place are put before the tensor core's proxy by
-// fence.proxy.async and stay in the CTA that wrote them; accumulator columns and exchanged chunks are reads, performed in the
-// warp's order ahead of its arrival (tcgen05.wait::ld and fence::before_thread_sync; loads from its own shared memory, which
-// a release at CTA scope orders), and whoever sees the arrival overwrites them only after that.
+// fence.proxy.async and stay in the CTA that wrote them; accumulator columns and exchanged chunks are reads, whose values are there
+// ahead of the arrival (tcgen05.wait::ld and fence::before_thread_sync; for loads from shared memory an address of the arrival
+// that depends on them: the arrival overtakes loads that have only been issued), and whoever sees it overwrites them after that.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }

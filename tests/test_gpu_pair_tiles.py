@@ -186,3 +186,28 @@ def test_expert_rows_off_the_word_grid(device):
     assert got[0] == 0x7fc0 and (got[count + 1:] == 0x7fc0).all()
     plan.destroy()
     bank.destroy()
+
+
+@pytest.mark.parametrize("shape,tokens", [((960, 2752, 96), 14216), ((1216, 1920, 128), 8868), ((768, 768, 64), 12000)])
+def test_passes_agree(device, shape, tokens):
+    """Short K, where the CTAs of a pair wait for each other's chunks: a chunk that is overwritten before it was read shows as rows that differ from pass to pass."""
+    cfg = synthetic.small_variant(synthetic.CONFIGS["deepseek-v3"], *shape)
+    cfg = synthetic.replace(cfg, act_block=128 if shape[0] % 128 == 0 and shape[1] % 128 == 0 else 32)
+    rng = np.random.default_rng(shape[0])
+    (H, I), E = shape[:2], cfg.total_experts
+    mats = [m for r, c in ((I, H), (I, H), (H, I)) for m in (rng.integers(0, 256, (r, c // 2), dtype=np.uint8), rng.integers(118, 122, (r, c // 32), dtype=np.uint8))]
+    bank = ExpertBank.upload(device, *([m] * E for m in mats))
+    plan = MoePlan.for_config(device, cfg, tokens)
+    buffer = device.resident_buffer_from
+    hidden, weights = (buffer(synthetic.f32_to_bf16(rng.standard_normal(s, dtype=np.float32) * np.float32(f))) for s, f in (((tokens, H), 1), ((cfg.experts, H), 0.02)))
+    bias = buffer(rng.standard_normal(cfg.experts, dtype=np.float32) * np.float32(0.05))
+    out = device.create_resident_buffer(tokens * H * 2)
+    first = None
+    for _ in range(12):
+        plan.layer(tokens, bank, hidden, out, router_weights=weights, bias=bias)
+        got = out.read(np.uint16).reshape(tokens, H)
+        first = got.copy() if first is None else first
+        assert (got != first).any(axis=1).sum() == 0  # (rows)
+    assert plan.status() == 0
+    plan.destroy()
+    bank.destroy()
