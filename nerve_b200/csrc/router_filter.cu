@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(32 * kRefineWarps, EPL > 4 ? 3 : 4) router_ref
     float my_v;
     if (!valid) return;
     const bool found = pick_experts<EPL>(E, k, val, score, taken, my_e, my_v);
-    finish_token<true>(p.router, token, found, my_e, my_v, rank);
+    finish_token<true>(p.router, counts_of(p.router), token, found, my_e, my_v, rank);
 }
 
 constexpr double kStepUnits = 16.0;     // (10.5 by the above)

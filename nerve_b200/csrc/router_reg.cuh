@@ -64,7 +64,7 @@ __device__ __forceinline__ float read_bias(const void* bias, uint32_t dtype, uin
 // of the scores are calls, one copy for all places. Kernels that only route have them inlined. Layers, us, calls everywhere and no loop unrolled / calls in those
 // blocks only: 256 experts of 2048 x 512 in groups, 16 tokens 72.8 / 71.6, 250 151.2 / 149.1; 250 of 64 of 1024 x 512 63.7 / 63.3; 4 of 64 of 256 x 128, 32 routes a
 // token, 42.2 / 36.7; 64 of 8 of 256 x 512 23.2 / 23.1; 33 to 200 of 32 of 2880 x 2880 level. router_reg_kernel by itself, 256 experts in groups: 64 tokens
-// 8.1 / 6.7, 2048 11.5 / 10.4, 16384 50.1 / 51.6; without groups 5.9 / 4.9, 7.9 / 7.8, 35.8 / 38.5; 32 experts, 16384 9.0 / 8.5. (Loops over selections unrolled by four
+// 8.1 / 6.7, 2048 11.5 / 9.9, 4096 23.2 / 18.9, 16384 50.3 / 48.0; without groups 5.9 / 5.9, 7.9 / 7.9, 17.0 / 17.7, 36.0 / 37.6; 32 experts, 16384 7.3 / 7.0. (Loops over selections unrolled by four
 // as well: layers of 256 experts 1 to 3 us more.)
 __device__ __noinline__ float call_exp(float v) { return nvmoe_expf(v); }
 __device__ __noinline__ float call_divide(float a, float b) { return __fdiv_rn(a, b); }
@@ -212,6 +212,18 @@ __device__ __forceinline__ bool select_experts(const RouterLaunch& p, uint32_t t
     return pick_experts<EPL>(E, k, val, score, taken, my_e, my_v);
 }
 
+// How many experts every token selects besides.
+__device__ __forceinline__ uint32_t always_selected(const RouterLaunch& p) { return p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u; }
+
+// What a token's selections are counted by.
+struct RouteCounts {
+    uint32_t experts, k, kind, total_k, total_resources;
+};
+__device__ __forceinline__ RouteCounts counts_of(const RouterLaunch& p) {
+    const uint32_t always = always_selected(p);
+    return RouteCounts{p.g.routed_experts, p.g.routed_k, p.g.router_kind, p.g.routed_k + always, p.g.routed_experts + always};
+}
+
 // The places of a token's selections in ascending order of the experts: lane r < total_k holds selection r.
 __device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total_k) {
     uint32_t rank = 0u;
@@ -225,22 +237,17 @@ __device__ __forceinline__ uint32_t ascending_rank(uint32_t my_e, uint32_t total
 // Of a token whose selections the lanes hold (`found`: there are k): lane r < total_k receives the expert and the place of one of its route words, as
 // finish_token writes them.
 __device__ __forceinline__ void order_token(const RouterLaunch& p, bool found, uint32_t& my_e, uint32_t& rank) {
-    const uint32_t lane = threadIdx.x & 31u, k = p.g.routed_k, always = p.g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
+    const uint32_t lane = threadIdx.x & 31u, k = p.g.routed_k, always = always_selected(p);
     if (!found) my_e = 0u;  // words of zeros
     if (found && lane >= k) my_e = p.g.routed_experts + (lane - k);
     rank = found ? ascending_rank(my_e, k + always) : lane;
 }
 
-// Weights, route words and telemetry of such a token; my_e and rank as above.
+// Weights, route words and telemetry of such a token (n: counts_of); my_e and rank as above.
 template <bool SHORT>
-__device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t token, bool found, uint32_t& my_e, float my_v, uint32_t& rank) {
+__device__ __forceinline__ void finish_token(const RouterLaunch& p, const RouteCounts& n, uint32_t token, bool found, uint32_t& my_e, float my_v, uint32_t& rank) {
     constexpr uint32_t kFull = 0xffffffffu;
-    const uint32_t E = p.g.routed_experts;
-    const uint32_t k = p.g.routed_k;
-    const uint32_t kind = p.g.router_kind;
-    const uint32_t always = kind == NVMOE_ROUTER_SCORE_TOPK ? p.g.always_count : 0u;
-    const uint32_t total_k = k + always;
-    const uint32_t total_resources = E + always;
+    const uint32_t E = n.experts, k = n.k, kind = n.kind, total_k = n.total_k, total_resources = n.total_resources;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* out = p.routes + (size_t)token * total_k;
     if (!found) {
@@ -294,10 +301,13 @@ __device__ __forceinline__ void finish_token(const RouterLaunch& p, uint32_t tok
 
 template <bool SHORT, int EPL, bool GROUPS>
 __device__ __forceinline__ void route_token(const RouterLaunch& p, uint32_t token) {
+    // (looked up ahead of the selection: behind it, router_reg_kernel with 256 experts in groups takes 10.4 us for 2048 tokens instead of 9.9, 23.7 for 4096 instead of
+    // 18.9, 51.9 for 16384 instead of 48.0)
+    const RouteCounts n = counts_of(p);
     uint32_t my_e, rank;
     float my_v;
     const bool found = select_experts<SHORT, EPL, GROUPS>(p, token, my_e, my_v);
-    finish_token<SHORT>(p, token, found, my_e, my_v, rank);
+    finish_token<SHORT>(p, n, token, found, my_e, my_v, rank);
 }
 
 }  // namespace

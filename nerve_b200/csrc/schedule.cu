@@ -913,7 +913,7 @@ __global__ void __launch_bounds__(1024) place_operands_kernel(const __grid_const
             float v;
             const bool found = select_experts<true, EPL == 0 ? 1 : EPL, false>(router, warp, e, v);
             if (blockIdx.x == 0u) {
-                finish_token<true>(router, warp, found, e, v, rank);
+                finish_token<true>(router, counts_of(router), warp, found, e, v, rank);
             } else {
                 order_token(router, found, e, rank);
             }
