@@ -1444,20 +1444,20 @@ static size_t place_operands_smem_bytes(const LayerSchedule& s, const OperandRow
 }
 
 // Which calls. A block ranks the routes of its own tokens, each by a pass over all routes, and a warp stores a piece of a row as often as its token has routes:
-// with many routes a token and few pieces a row these take longer than what stands beside them. `steps` are a warp's passes, in 32 routes. Layers of 64
-// experts, us, in turn / beside: 16 routes a token 64 tokens of 512 columns (steps 512) 38.1 / 50.8, of 1024 (288) 42.0 / 47.3, of 2048 (160) 50.6 / 52.6, of
-// 2880 (128) 59.6 / 59.7; 25 tokens of 2048 (65) 39.1 / 40.9; 12 routes 66 tokens of 2048 (100) 47.1 / 47.4, of 2880 (75) 55.9 / 54.7; 8 routes 128 tokens
-// of 512 (256) 35.6 / 38.6, of 1024 (160) 40.1 / 38.7, 50 of 512 (104) 29.5 / 30.7, of 1024 (65) 32.0 / 31.2; 6 routes 170 of 512 (192) 35.6 / 36.9, 133 (150) 34.0 /
-// 34.5, 66 (78) 29.2 / 28.9; 4 routes 256 (128) 37.2 / 35.7, 150 (76) 30.0 / 27.9; 2 routes 512 (64) 36.1 / 32.1. By blocks of eight warps 12 routes 21 tokens of 512
-// (96) 30.6 / 30.7, of 1024 (64) 32.1 / 30.5; 9 routes 28 of 256 (72) 29.9 / 29.8. Routed in the same blocks, 32 routes 8 of 512 (256) 38.8 / 44.7, 4 of 512 (64)
-// 36.6 / 38.2, of 2048 (48) 44.2 / 43.4; 16 routes 16 of 1024 (72) 35.0 / 34.4, of 512 (128) 33.0 / 34.8, 8 of 512 (64) 30.2 / 30.8, of 1024 (40) 32.5 / 30.8; 12
-// routes 10 of 512 (32) 28.9 / 28.3.
+// with many routes a token and few pieces a row these take longer than what stands beside them. In turn, the schedule takes the longer the more experts there
+// are. `steps` are a warp's passes, in 32 routes. Layers of 64 experts, us, in turn / beside: 16 routes a token 64 tokens of 512 columns (steps 512) 38.1 / 50.8, of 1024
+// (288) 42.0 / 47.3, of 2880 (128) 59.6 / 59.7; 12 routes 66 tokens of 2048 (100) 47.1 / 47.4, of 2880 (75) 55.9 / 54.7; 8 routes 128 tokens of 512 (256) 35.6 / 38.6, of
+// 1024 (160) 40.1 / 38.7; 4 routes 256 of 512 (128) 37.2 / 35.7; 2 routes 512 (64) 36.1 / 32.1. Of 192 experts: 12 routes 49 tokens of 512 (228) 53.5 / 56.2, 38 of 960 (105)
+// 56.9 / 54.3, 20 routes 24 of 2048 (105) 70.4 / 66.9; of 256: 24 routes 9 of 384 (200) 65.3 / 67.5, 2 of 1280 (14) 55.7 / 49.6, 9 routes 90 of 768 (130) 57.2 / 50.8; of 8: 7 routes
+// 45 of 512 (70) 27.0 / 28.1. Routed in the same blocks, 64 experts, 32 routes 8 of 512 (256) 38.8 / 44.7, 4 of 2048 (48) 44.2 / 43.4; 16 routes 16 of 512 (128) 33.0 / 34.8, of 1024 (72) 35.0 /
+// 34.4; 128 experts, 20 routes 7 of 1472 (50) 42.0 / 39.2, 31 routes 2 of 320 (16) 36.8 / 38.3. Of 1920 layers drawn (1 to 32 routes, 8 to 256 experts, 256 to 4096 columns) the
+// rule takes the slower way by more than 1.5 % in 44, at most 6 %.
 static bool operands_gain(const LayerSchedule& s, const OperandRows& o, bool routed) {
     const uint32_t count = s.tokens * s.K, warps = place_operands_threads(s, routed) / 32u;
     const uint32_t most = place_words(warps, o.chunks, s.K), routes = most < count ? most : count;
     const uint32_t steps = (routes + warps - 1u) / warps * ((count + 31u) / 32u);
-    if (routed) return steps <= 48u;
-    return steps + 8u * s.K <= (warps <= 8u ? 180u : 100u + count / 8u);
+    if (routed) return steps + 2u * s.K <= 50u + s.num_experts / 2u;
+    return steps + 6u * s.K <= 60u + s.num_experts + count / 16u;
 }
 
 bool places_operands(const LayerSchedule& s, bool routed, const OperandRows& o, uint32_t block) {

@@ -85,6 +85,15 @@ def test_many_routes_a_token(device, k, hidden, tokens):
     layer.close()
 
 
+# ... which lie further out where there are many experts: routed ahead of the blocks, and in them
+@pytest.mark.parametrize("k,hidden,tokens,experts", [
+    (12, 512, 49, 192), (12, 960, 38, 192), (24, 704, 4, 256), (24, 320, 12, 256), (16, 320, 64, 256), (7, 320, 45, 8), (20, 1472, 7, 128), (31, 320, 8, 128), (7, 320, 27, 9), (31, 320, 2, 48)])
+def test_many_routes_of_many_experts(device, k, hidden, tokens, experts):
+    layer = Layer(device, "gpt-oss-20b", (hidden, 128, experts), tokens, k=k)
+    assert layer.same_both_ways() == 0
+    layer.close()
+
+
 @pytest.mark.parametrize("tokens", [5, 20, 200])
 def test_experts_that_a_stage_lacks(device, tokens):
     layer = Layer(device, "gpt-oss-20b", (1088, 192, 32), tokens)
