@@ -554,8 +554,12 @@ constexpr uint32_t kFilterSplits = 8u;  // at most
 // Which calls. Product and refinement take 13 us of latency, more with more experts a lane; the tiled projection (router.cu), in blocks of 32
 // tokens x 16 outputs, 15 us a round of the SMs at 2880 columns. Layers, us, pinned / filtered (tokens x hidden x experts): 512 x 2880 x 32 69.1 / 67.4,
 // 2048 135.9 / 134.2; 2048 x 1024 x 32 81.4 / 80.8, 768 59.9 / 60.8; 512 x 2880 x 128 (one round) 110.7 / 113.5, 768 (two) 128.5 / 119.9, 2048 185.1 / 152.9;
-// 257 x 4096 x 64 90.6 / 89.6, 2048 191.0 / 173.3; grouped, 768 x 2048 x 64 111.3 / 115.1, 1536 157.2 / 154.0; 257 x 7168 x 256 324.9 / 320.5, 2048 788 / 673;
-// 2048 x 512 x 16 64.8 / 66.8.
+// 257 x 4096 x 64 90.6 / 89.6, 2048 191.0 / 173.3; grouped, 768 x 2048 x 64 111.3 / 115.1, 1536 157.2 / 154.0; 2048 x 7168 x 256 788 / 673;
+// 2048 x 512 x 16 64.8 / 66.8. In one round of the tiled blocks that of many experts, or of groups, costs more than it gives, unless the round is nearly full, whose blocks
+// share the rows' bandwidth: 300 x 6016 x 192 141.3 / 146.0, 417 x 6976 x 160 (140 blocks) 142.5 / 134.7; grouped, 264 x 7552 x 256 120.7 / 129.4, 363 x 4480 x 128 114.2 / 121.0, 551 x
+// 5120 x 128 (144 blocks) 149.8 / 141.0, 630 x 6208 x 64 146.2 / 150.5, 1049 x 7040 x 64 (132) 162.2 / 157.7, 576 x 1792 x 32 57.6 / 58.8, 495 x 2816 x 32 59.4 / 59.8, 602 x 3840 x 16 70.0 /
+// 67.8. Of 430 layers drawn around the line the rule takes the slower way by 0.14 % in the mean (0.8 % without these), by 4 % at most.
+// (A size that is taken stays so with more tokens: a plan's scratch is sized for its largest call.)
 bool router_filter_form(const nvmoe_geometry& g) {
     const bool form = g.router_kind == NVMOE_ROUTER_TOPK_SOFTMAX || (g.router_kind == NVMOE_ROUTER_SCORE_TOPK && g.activation == NVMOE_ACT_SIGMOID);
     const uint32_t total_k = g.routed_k + (g.router_kind == NVMOE_ROUTER_SCORE_TOPK ? g.always_count : 0u), per = g.n_group ? g.routed_experts / g.n_group : 1u;
@@ -565,7 +569,14 @@ bool router_filter_takes(const nvmoe_geometry& g, uint32_t tokens) {
     if (!router_filter_form(g) || tokens <= 256u) return false;
     const uint64_t blocks = (uint64_t)((tokens + 31u) / 32u) * ((g.routed_experts + 15u) / 16u);
     const uint32_t sms = device_sm_count();
-    return (blocks + sms - 1u) / sms * g.hidden_size >= 1024u + 24u * (uint64_t)g.routed_experts;
+    const uint64_t rounds = (blocks + sms - 1u) / sms;
+    uint64_t columns = 1024u + 24u * (uint64_t)g.routed_experts;
+    if (rounds == 1u) {
+        const bool nearly_full = 10u * blocks >= 9u * (uint64_t)sms;
+        if (g.routed_experts > (g.n_group ? 32u : 128u) && !(nearly_full && (!g.n_group || g.routed_experts <= 128u))) return false;
+        if (g.n_group && g.routed_experts <= 32u) columns += 1200u;
+    }
+    return rounds * g.hidden_size >= columns;
 }
 
 static uint32_t filter_tiles(uint32_t tokens) { return (tokens + kFilterTokens - 1u) / kFilterTokens; }

@@ -149,11 +149,38 @@ def test_a_wait_that_runs_out(device):
     layer.close()
 
 
-# sizes that the rule leaves to the projection by itself: few columns in one round of its blocks, 256 tokens
-BELOW = [((1152, 64, 16), 300), ((2880, 64, 32), 256)]
+# sizes that the rule leaves to the projection by itself: few columns in one round of its blocks, 256 tokens; groups in one round
+BELOW = [((1152, 64, 16), 300), ((2880, 64, 32), 256), ((1920, 128, 32), 1029), ((1536, 128, 16), 1100), ((2560, 128, 64), 1050)]
 SELECTED = [tuple(case) for case in test_what_is_selected.pytestmark[0].args[1]]
 UNTOLD = [(name, shape, 1050, changes) for name, shape, changes in
           next(mark.args[1] for mark in test_inputs_that_the_product_says_little_of.pytestmark if mark.args[0] == "name,shape,changes")]
+
+
+# groups in one round of blocks, on either side of its lines: 32 experts or fewer by their columns, up to 128 in a round nearly full; many experts without groups
+ONE_ROUND = [("deepseek-v3", (3072, 128, 32), 1029, {"n_group": 32, "topk_group": 9}, True), ("deepseek-v3", (2944, 128, 32), 700, {}, False),
+             ("deepseek-v3", (2688, 128, 16), 1100, {"n_group": 4, "topk_group": 1, "k": 4}, True), ("deepseek-v3", (2560, 128, 64), 1057, {}, True),
+             ("deepseek-v3", (4096, 128, 128), 545, {}, True), ("deepseek-v3", (4096, 128, 128), 300, {}, False), ("deepseek-v3", (7168, 128, 256), 257, {}, False),
+             ("gpt-oss-20b", (4864, 64, 160), 417, {}, True), ("gpt-oss-20b", (4864, 64, 160), 330, {}, False)]
+
+
+@pytest.mark.parametrize("name,shape,tokens,changes,filtered", ONE_ROUND)
+def test_one_round_of_blocks(device, name, shape, tokens, changes, filtered):
+    test_what_is_selected(device, name, shape, tokens, changes)
+    layer = Layer(device, name, shape, tokens, **changes)
+    buffer = lambda a: None if a is None else device.resident_buffer_from(a)
+    layer.plan.layer(tokens, layer.bank, buffer(layer.x), device.create_resident_buffer(tokens * layer.cfg.hidden * 2), router_weights=buffer(layer.w),
+                     router_bias=buffer(layer.logit_bias), bias=buffer(layer.select_bias))
+    assert layer.plan.debug_projection() == filtered and layer.plan.status() == 0
+    layer.close()
+
+
+@pytest.mark.parametrize("kind", [kind for mark in test_inputs_that_the_product_says_little_of.pytestmark if mark.args[0] == "kind" for kind in mark.args[1]])
+def test_groups_by_a_product_that_says_little(device, kind):
+    """The inputs above, of groups in a size that the filter takes."""
+    layer = Layer(device, "deepseek-v3", (2560, 128, 64), 1057)
+    inputs(kind, layer)
+    layer.both_ways()
+    layer.close()
 
 
 @pytest.mark.parametrize("name,shape,tokens,changes", SELECTED + UNTOLD)
@@ -171,7 +198,7 @@ def test_which_projection_a_call_uses(device, name, shape, tokens, changes):
     layer.close()
 
 
-@pytest.mark.parametrize("name,shape,tokens,changes", UNTOLD)
+@pytest.mark.parametrize("name,shape,tokens,changes", [*UNTOLD[:2], ("deepseek-v3", (2560, 128, 64), 1057, {})])
 def test_rows_that_the_product_errs_most_by(device, name, shape, tokens, changes):
     """Positive ones, the largest first, by experts a step or two apart."""
     layer = Layer(device, name, shape, tokens, **changes)
