@@ -280,7 +280,8 @@ def roofline_of(cfg, tokens, bound, ms, gate_ms, down_ms, distinct, peaks, peak_
                 "kernel": "gate_up", "peak_kind": f"{peak_kind} STREAM-style copy",
                 "algorithmic_bytes_per_launch": ab["gate_up"], "kernel_ms": gate_ms,
                 # (the timed calls run gate/up and down in one launch where gate/up is more than a round of the SMs)
-                "note": "kernel times are those of a profiled call, which launches gate/up and down one by one",
+                "note": "kernel times, and stage_ms, are those of a profiled call, which launches gate/up and down one by one, a router of its own, and in small calls the schedule and "
+                        "the operands in turn that others make side by side",
                 "both_stages_traffic": traffic.get("experts") if traffic else None,
                 "down_kernel": {"achieved": ab["down"] / (down_ms * 1e-3) / 1e9, "kernel_ms": down_ms,
                                 "frac": ab["down"] / (down_ms * 1e-3) / 1e9 / hbm,

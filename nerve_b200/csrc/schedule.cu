@@ -1451,7 +1451,8 @@ static size_t place_operands_smem_bytes(const LayerSchedule& s, const OperandRow
 // 56.9 / 54.3, 20 routes 24 of 2048 (105) 70.4 / 66.9; of 256: 24 routes 9 of 384 (200) 65.3 / 67.5, 2 of 1280 (14) 55.7 / 49.6, 9 routes 90 of 768 (130) 57.2 / 50.8; of 8: 7 routes
 // 45 of 512 (70) 27.0 / 28.1. Routed in the same blocks, 64 experts, 32 routes 8 of 512 (256) 38.8 / 44.7, 4 of 2048 (48) 44.2 / 43.4; 16 routes 16 of 512 (128) 33.0 / 34.8, of 1024 (72) 35.0 /
 // 34.4; 128 experts, 20 routes 7 of 1472 (50) 42.0 / 39.2, 31 routes 2 of 320 (16) 36.8 / 38.3. Of 1920 layers drawn (1 to 32 routes, 8 to 256 experts, 256 to 4096 columns) the
-// rule takes the slower way by more than 1.5 % in 44, at most 6 %.
+// rule takes the slower way by more than 1.5 % in 44, at most 6 %. (1024 routes are what a block of the schedule has threads for, one each. 4 routes, 2880 columns, in turn /
+// beside: 900 of 32 experts 48.6 / 44.5, 1024 49.7 / 45.1; 900 of 128 102.3 / 96.5, 1024 102.8 / 96.5; in turn 1100 55.7 and 102.1, 1500 61.8 and 105.4, 2000 66.8 and 110.7.)
 static bool operands_gain(const LayerSchedule& s, const OperandRows& o, bool routed) {
     const uint32_t count = s.tokens * s.K, warps = place_operands_threads(s, routed) / 32u;
     const uint32_t most = place_words(warps, o.chunks, s.K), routes = most < count ? most : count;
