@@ -32,8 +32,9 @@ using namespace tc;
 
 // Roles, as in experts_tc.cu: warps 0-3 and 8-15 epilogue, 4 MMA, 5 weights, 6 token scales, 7 token rows and the claims.
 constexpr uint32_t kLayerThreads = 512u, kLayerGroups = 3u, kLayerEpilogueWarps = 4u * kLayerGroups;
-constexpr uint32_t kLayerMapsAhead = 64u;  // up to so many experts a block acquires the gate/up maps before its wait
-constexpr uint32_t kLayerMapWarp = 10u;    // beyond, the epilogue warp that acquires them beside the first copies
+// Who acquires the tensor maps of the weights: all threads ahead of the wait, an epilogue warp beside the first copies, or the lane that issues a tile's copies.
+enum : uint32_t { kMapsAhead = 0u, kMapsBeside = 1u, kMapsByTile = 2u };
+constexpr uint32_t kLayerMapWarp = 10u;   // the epilogue warp that does
 constexpr uint32_t kLayerWatchWarp = 2u;  // the epilogue warp that polls (not on the MMA or TMA warp's scheduler)
 constexpr uint32_t kLayerMaxSlots = 6u;
 constexpr uint32_t kLayerMaxExperts = 2u * kLayerExperts;  // of both stages together
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
     const uint32_t G = gridDim.x;
 
     const uint32_t experts = p.stage[0].work.num_experts;
-    const bool maps_beside = experts > kLayerMapsAhead;
+    const bool maps_beside = p.maps == kMapsBeside, maps_by_tile = p.maps == kMapsByTile;
 
     // ---- one-time setup ---------------------------------------------------------------------
     if (threadIdx.x >= 32u && threadIdx.x < 32u + kLayerMaxExperts / 32u) bars->bytes_form[threadIdx.x - 32u] = 0u;
@@ -151,11 +152,8 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         if (bytes) atomicOr(&bars->bytes_form[m / 32u], 1u << (m % 32u));
     }
     // (as in experts_tc.cu: a block acquires a tensor map once, while the kernel ahead still runs; 13 to 29 ns a map, one after the other, so that those of
-    // the down weights are left to epilogue warps that have nothing to do yet. With many experts one epilogue warp acquires all, a few at a time, and the lane that
-    // issues the copies goes ahead with maps that it acquires itself where that warp is not through: a block that starts late, on an SM that
-    // the kernel ahead still used, had 15 us of maps before its first copy with 257 experts. Layers, us, all ahead / beside: 256 experts of 4096 x 1024, 30
-    // tokens 142.8 / 137.4, 96 260.3 / 256.0; 128 of 2880 x 2880, 64 239.0 / 239.3, 300 315.5 / 313.6; 64 of 4096 x 2048, 50 151.8 / 152.3.)
-    if (!maps_beside)
+    // the down weights are left to epilogue warps that have nothing to do yet. With many experts: layer_maps)
+    if (p.maps == kMapsAhead)
         for (uint32_t m = threadIdx.x; m < 2u * experts; m += blockDim.x) tensormap_acquire(p.stage[0].tmaps + (size_t)m * kWeightMaps * 128u);
     if (threadIdx.x < 2u) tensormap_acquire(p.stage[threadIdx.x].act_tmap);
     __syncthreads();
@@ -190,6 +188,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         if (lane == 0u) {
             uint32_t slot = 0u, empty_parity = 1u;
             bool alive = true, maps_stand = !maps_beside;
+            uint32_t acquired = kUnboundSlot;  // by tile: whose maps were last
             auto run = [&](auto tag, uint32_t id) {
                 constexpr uint32_t phase = decltype(tag)::value;
                 // (debug) leave out the very first arrival of chunk 0 or 1: its consumer's bounded wait must then give up
@@ -198,7 +197,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
                 const ExpertLaunch& e = p.stage[phase];
                 // (the list entry of a tile is fetched a tile ahead: a load only, a thread stalls at the first instruction that needs it)
                 auto entry_of = [&](uint32_t tile) { return __ldg(e.tile_list + min(tile / s.m_tiles, e.tile_capacity - 1u)); };
-                if (phase == 1u && !mbar_wait(&bars->down_maps, 0u, abort_flag, wait_limit)) {
+                if (phase == 1u && !maps_by_tile && !mbar_wait(&bars->down_maps, 0u, abort_flag, wait_limit)) {
                     alive = false;
                     return;
                 }
@@ -218,9 +217,10 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
                     const uint8_t* scales2 = row_tile + 1u < s.row_tiles ? scales + (size_t)s.stages * scale_stride : scales;
                     const uint8_t* maps = e.tmaps + (size_t)expert * (phase == 0u ? 2u : 1u) * kWeightMaps * 128u;
                     const uint32_t box_bytes = format == 0u ? kTmaBoxBytes : 2u * kTmaBoxBytes;
-                    if (phase == 0u && !maps_stand && !(maps_stand = mbar_test(&bars->gate_maps, 0u))) {
-                        tensormap_acquire(maps);
-                        tensormap_acquire(maps + kWeightMaps * 128u);
+                    if (maps_by_tile ? form != acquired : phase == 0u && !maps_stand && !(maps_stand = mbar_test(&bars->gate_maps, 0u))) {
+                        tensormap_acquire(phase == 0u ? maps : maps + 256u);
+                        if (phase == 0u) tensormap_acquire(maps + kWeightMaps * 128u);
+                        acquired = form;
                     }
                     for (uint32_t ks = 0; ks < s.stages; ks++) {
                         if (!mbar_wait(&bars->empty[slot], empty_parity, abort_flag, wait_limit)) {
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kLayerThreads, 1) experts_layer_kernel(const _
         const bool whole_block = g.act_block == 128u;  // the scale block of the down operands is the tile's 128 rows
         uint32_t acc_it = 0u, set_it = 0u;
         bool alive = true;
-        if (!maps_beside || warp == kLayerMapWarp) {
+        if (!maps_by_tile && (!maps_beside || warp == kLayerMapWarp)) {
             const uint32_t first = maps_beside ? lane : group * 128u + quad * 32u + lane, step = maps_beside ? 32u : 32u * kLayerEpilogueWarps;
 #pragma unroll 1
             for (uint32_t m = first; m < experts; m += step) tensormap_acquire(p.stage[1].tmaps + (size_t)m * kWeightMaps * 128u + 256u);
@@ -659,7 +659,24 @@ void layer_configure_kernels() {
     configure_one<96u>();
 }
 
-void launch_experts_layer(const LayerLaunch& p, int sms, cudaStream_t stream) {
+// All maps ahead of the wait are acquired for nothing where the block would have waited anyway, but a block that starts late, on an SM that the kernel ahead still used,
+// has 15 us of them before its first copy with 257 experts. Beside the first copies they hold up an epilogue warp as long, which short K can't hide. By tile the lane that
+// issues the copies stands still for 0.4 us a tile, which costs bytes under way where K is long and a block has many tiles. Layers, us, ahead / beside / by tile: 17 tokens
+// of 257 experts of 512 x 384 39.9 / 47.0 / 39.3, 579 of 1536 x 1152 167.9 / 174.6 / 164.0; 6 of 129 of 640 x 512 34.1 / 38.7 / 33.5; 165 of 3840 x 2432 396.0 / 392.3 / 401.1; 327 of 128 of
+// 3072 x 2048 251.3 / 247.7 / 253.2; 64 tokens of 32 of 2880 x 2880 ahead. Of 420 drawn layers the rule takes the slower way by 0.15 % in the mean; beyond 64 experts it
+// is 1.9 % faster than all ahead in the mean, at most 1.7 % slower.
+static uint32_t layer_maps(const LayerLaunch& p, uint32_t sms) {
+    const nvmoe_geometry& g = p.stage[0].g;
+    const uint32_t experts = p.stage[0].work.num_experts;
+    if (experts <= 64u) return kMapsAhead;
+    const uint64_t routes = (uint64_t)p.stage[0].tokens * (g.routed_k + g.always_count), touched = routes < experts ? routes : experts;
+    const uint64_t tiles = touched * ((g.intermediate_size + kBlockM - 1u) / kBlockM + (g.hidden_size + 2u * kBlockM - 1u) / (2u * kBlockM));
+    return g.hidden_size > 2048u && tiles > 12u * (uint64_t)sms ? kMapsBeside : kMapsByTile;
+}
+
+void launch_experts_layer(const LayerLaunch& launch, int sms, cudaStream_t stream) {
+    LayerLaunch p = launch;
+    p.maps = layer_maps(p, (uint32_t)sms);
     switch (p.stage[0].token_rows) {
         case 16u: launch_one<16u>(p, sms, stream); break;
         case 32u: launch_one<32u>(p, sms, stream); break;

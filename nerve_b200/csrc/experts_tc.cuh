@@ -94,6 +94,7 @@ struct LayerLaunch {
     ExpertLaunch stage[2];
     uint32_t* sync;    // experts + 1 words, cleared earlier in the call: chunks claimed, per expert the warps done with its gate/up tiles
     bool claim_late;   // the launch right before this one clears them
+    uint32_t maps;     // who acquires the tensor maps of the weights (experts_layer.cu sets it)
 };
 constexpr uint32_t kLayerExperts = 1024u;  // at most
 void layer_configure_kernels();

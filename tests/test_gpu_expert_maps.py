@@ -26,3 +26,11 @@ def test_many_experts_in_one_launch(device, name, shape, tokens, native):  # noq
     assert plan.last_report()["kernel_launches"] == 6  # one for both stages
     plan.destroy()
     bank.destroy()
+
+
+# ... acquired tile by tile (short K, or few tiles a block) and, with long K and many, beside the first copies; one-byte weights among either
+@pytest.mark.parametrize("name,shape,tokens,native", [
+    ("gpt-oss-20b", (2176, 1152, 100), 60, 0), ("gpt-oss-20b", (2176, 1088, 90), 60, 0), ("deepseek-v3", (2304, 1280, 128), 40, 1), ("deepseek-v3", (1536, 1024, 128), 30, 1),
+    ("gpt-oss-20b", (1536, 1024, 200), 100, 0)])
+def test_maps_by_tile_and_beside(device, name, shape, tokens, native):  # noqa: F811
+    test_many_experts_in_one_launch(device, name, shape, tokens, native)
